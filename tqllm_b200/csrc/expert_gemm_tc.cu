@@ -4,24 +4,39 @@
 // (src/formats/weight/quant_u4h.inc:609-774, src/formats/weight/quant.cu:286-405) with their fused SwiGLU epilogue
 // (quant_u4h.inc:756-759): per expert Y_e = W_e . X_e^T over the expert's gathered token rows.
 //
-// One persistent block per SM; an item is (expert, tile of <= 128 of its tokens, two blocks of 128 weight rows): the same
-// 128 rows of the gate and of the up matrix, or two consecutive row blocks of the down matrix. Per row block
+// One persistent block per SM; an item is (expert, tile of up to `cap` of its tokens, block of 128 weight rows): 128 rows of the
+// down matrix, or 64 rows of the gate and the same 64 rows of the up matrix (row tiles of 16, gate and up alternating, so
+// that both rows of an output element sit in one warp's quarter of tensor memory). Per item
 //   D[128 rows][N tokens] (fp32, tensor memory) = sum over K of A[128][K] (fp16) . B[N][K] (fp16)
-//   A: the weight rows, decoded from the bank's block format to fp16 in shared memory by the CUDA cores, 64 columns per
-//      step (canonical K-major core-matrix layout, no swizzle); the raw blocks arrive through a per-warp ring of bulk
-//      copies (cp.async.bulk + mbarrier), 256 columns per copy;
-//   B: the tokens' activation rows (fp16, each row scaled by a power of two), gathered through the dispatch permutation with 16-byte cp.async;
-//   the two row blocks of an item share B (one gathered copy of the token rows serves 256 weight rows) and have an
-//   accumulator each; two accumulator sets alternate between items, so the epilogue of one item (SwiGLU, stores) overlaps
-//   the products of the next.
-// Warps: 0 issues tcgen05.mma (one lane); 1..4 epilogue (tcgen05.ld, one TMEM lane quarter each); 5..6 load B;
-// 7..22 decode A (two warps per row tile of the block: rows g and rows g + 8 of the lane-major tile). Every wait is bounded; a wait that runs out sets the plan's
+//   A: the weight rows, decoded from the bank's block format to fp16 by the CUDA cores and written to TENSOR MEMORY
+//      (tcgen05.st.16x256b: the lane-major bank tile decodes to exactly that fragment). An A operand in shared memory costs
+//      64 bytes per clock for its stores and 64 for the tensor core's reads beside 64 for B at N = 128: more than the 128 an
+//      SM has, and that was the limit. Four stages of a unit (two steps of 64 columns);
+//   B: the tokens' activation rows (fp16, each row scaled by a power of two, brought into slot order before the product), one TMA
+//      box per unit in the 128-byte swizzled form. Copies by the threads (cp.async) need a proxy fence before the tensor core
+//      may read them, and that fence waits for the copies of the later steps too: measured, the B loader then set the pace
+//      (1680 cycles per step at 80 tokens). Gathering token rows by TMA (tile::gather4) costs the issuing warp 60 to 200
+//      cycles per four rows and stays for calls whose scratch holds no rows in slot order;
+//   two accumulators of 128 columns alternate between items of up to 128 tokens, so the epilogue of one item (SwiGLU, stores)
+//   overlaps the products of the next; a wider item takes both. Products into one accumulator follow each other by at least 80
+//   cycles however few tokens they have, products into two alternating ones by 44 (measured), so an item of up to 64 tokens
+//   splits its K over the two halves of its accumulator and the epilogue adds them.
+// The control warps share their schedulers with six others, so what they execute per unit bounds the block: they walk uniform
+// loops, one elected lane issues, and the raw blocks and rows come in the largest boxes that fit. They are the first warps of the
+// block: as the last ones they were served last (c3 decode gate/up 110 us, as the first 78).
+// Warps: 0 issues tcgen05.mma; 1 streams the raw blocks (256 columns of the item's eight row tiles per ring slot: one TMA box
+// of the down bank, one each of gate and up, running ahead across items); 2 (and 3 when it gathers) loads B; 4..11 epilogue (two
+// per TMEM lane quarter, 16-token groups in turn); 12..27 decode A (warp 12 + j: lane quarter j & 3, row tile (j >> 2) & 1 of
+// it, every second 256-column chunk). One barrier per step says that its products are done (a commit costs the issuing thread
+// 60 cycles): it frees the unit's A stage and the step's B stage. Every wait is bounded; a wait that runs out sets the plan's
 // status word, and the block drains and leaves.
 //
 // Numerics: weights are rounded to fp16 after the exact fp32 decode (relative error <= 2^-11 per weight; bf16 operands
 // gave 3e-2 of the output RMS as the largest error, fp16 stays below the layer tolerance). An activation row is
 // multiplied by 2^e so that its largest magnitude lies in [2^14, 2^15) and rounded to fp16: exact for bf16 inputs down
 // to 2^-29 of the row maximum; the epilogue multiplies the sums (fp32) by 2^-e.
+#include <cuda.h>
+
 #include <type_traits>
 
 #include "common.cuh"
@@ -33,55 +48,54 @@ namespace b2 {
 namespace {
 using namespace tc;
 
-constexpr int G_ROWS = 128;                 // weight rows per item = M
-// tokens per item: template parameter NT = 128 (two accumulator sets, four B stages; the default) or 256 (one accumulator
-// set in the gate/up product, two B stages; opt-in)
-constexpr int G_KS = 64;                    // columns per pipeline step (four MMAs of K = 16 per matrix)
-constexpr int NMAT = 2;                     // row blocks per item: (gate, up) or two consecutive blocks of the down matrix
-constexpr int A_STAGES = 2;                 // stages of decoded A operand (two row blocks each)
-constexpr int MAX_A_STAGES = A_STAGES, RAW_SLOTS = 2, MAX_B_STAGES = 4;
-constexpr uint32_t DEC_BACKOFF = 60;       // ns between tries of a decode warp's waits
-constexpr int A_LBO = gdec::A_LBO;          // bytes between k cores of A
-constexpr int A_MAT = 8 * A_LBO;            // one matrix of one A stage: 128 rows x 64 columns
-#ifndef B2_LOAD_WARPS
-#define B2_LOAD_WARPS 2
-#endif
-constexpr int MMA_WARP = 0, LOAD_WARP0 = 5, LOAD_WARPS = B2_LOAD_WARPS, LOAD_THREADS = 32 * LOAD_WARPS, DEC_WARP0 = LOAD_WARP0 + LOAD_WARPS, DEC_WARPS = 16;   // warps 1..4: epilogue
+constexpr int G_KS = 64;                    // columns per step (four MMAs of K = 16); a unit is two steps
+constexpr int A_STAGES = 4, A_COLS = 64;    // stages of decoded A operand, a unit each (two chunks in all: one per decode warp of a row tile), and their columns
+constexpr int STEP_RING = 2 * A_STAGES;     // barriers "the products of step g are done"
+constexpr int ACC_COLS = 128, A_COL0 = 2 * ACC_COLS;                // the two accumulators, then the A stages: all 512 columns
+constexpr int SPLIT_COLS = ACC_COLS / 2;    // items of up to this many tokens split their K over the halves of the accumulator
+constexpr int MAX_B_STAGES = 8, RAW_SLOTS = 6, MAX_CAP = 256;
+constexpr int MMA_WARP = 0, RAW_WARP = 1, LOAD_WARP0 = 2, LOAD_WARPS = 2, EPI_WARP0 = 4, EPI_WARPS = 8, DEC_WARP0 = 12, DEC_WARPS = 16;
 constexpr int G_THREADS = (DEC_WARP0 + DEC_WARPS) * 32;
-constexpr int N_BARS = 2 * 8 * RAW_SLOTS + 2 * MAX_A_STAGES + 2 * MAX_B_STAGES + 4;
+static_assert(EPI_WARPS * 32 == MAX_CAP, "an epilogue thread looks one token up");
+static_assert(MAX_B_STAGES <= STEP_RING, "a B stage is freed by the barrier of the step that used it");
+constexpr int N_BARS = 2 * RAW_SLOTS + A_STAGES + STEP_RING + MAX_B_STAGES + 6;
 
 struct GemmArgs {
-    const uint8_t * w0, * w1;               // stacked banks (gate, up) or (down, -)
-    const uint8_t * s0, * s1;               // the shared expert's banks (may be null)
-    const float * aux0, * aux1, * saux0, * saux1;
-    size_t bank_bytes;
-    const __half * xb;                      // activation rows, fp16, row stride k, row r scaled by 1 / inv_scale[r]
-    const float * inv_scale;
+    const float * aux0, * aux1, * saux0, * saux1;      // row scales of the banks (gate, up) or (down, -) and of the shared expert's (may be null)
+    const float * inv_scale;                // per activation row (the fp16 rows themselves come through the tensor maps)
     int * plan;
     float * out;
     int rows, k, experts, topk, A;
+    int cap, b_stages, raw_slots;           // most tokens of an item; B stages; raw chunks in the ring
+    int b_pair;                             // 1: the B stages are filled and freed a unit at a time
+    int slots;                              // 1: the activation rows lie in slot order; 0: in token (row) order, and are gathered
 };
+// x[i]: the activation rows, boxes of (i + 1) cap / 4 rows (a gathering launch: x[0], one row); w: banks (gate, up) or (down, -), then the shared expert's
+struct GemmMaps { CUtensorMap x[4], w[4]; };
 
 template <uint32_t T> constexpr int chunk_tiles() { return 256 / Fmt<T>::KT; }
 template <uint32_t T> constexpr int chunk_bytes() { return chunk_tiles<T>() * Fmt<T>::TILE; }
+// a chunk of a row tile as the raw TMA boxes see it: parts of at most 256 8-byte words; rows of K may end after any part
+template <uint32_t T> constexpr int chunk_parts() { return T == T_IQ4_NL ? 4 : 2; }
+template <uint32_t T> constexpr int part_words() { return chunk_bytes<T>() / chunk_parts<T>() / 8; }
 
-template <uint32_t T, int NT>
-constexpr size_t gemm_smem(int experts) {
-    return size_t(A_STAGES) * NMAT * A_MAT + size_t(NT == 128 ? 4 : 2) * (8 * NT * 16) + size_t(8) * RAW_SLOTS * NMAT * chunk_bytes<T>() +
-           gdec::Dec<T>::TAB_BYTES + size_t(experts + 3) * 4 + 16 + size_t(N_BARS) * 8 + 16;
+// the active experts of the launch: items before it, expert, tokens, first assignment slot
+struct Info { int cum, e, cnt, off; };
+
+template <uint32_t T>
+constexpr size_t gemm_smem(int experts, int cap, int b_stages, int raw_slots) {
+    return 1024 + size_t(b_stages) * cap * 128 + size_t(8) * raw_slots * chunk_bytes<T>() + gdec::Dec<T>::TAB_BYTES +
+           size_t(experts + 2) * sizeof(Info) + 2 * MAX_CAP * sizeof(int2) + size_t(N_BARS) * 8 + 16;
 }
 
-// any activation dtype -> fp16 rows scaled by a power of two per row (one warp per row) + the inverse scales; inside every
-// 64-column step the columns are stored in the order of the format's A operand (gdec::colmap). Two passes over the row:
-// its largest magnitude with 16-byte loads, then (from the cache) two source columns per lane and step into one half2
+// One activation row of any dtype -> fp16 scaled by a power of two (largest magnitude in [2^14, 2^15)), by one warp; returns the
+// inverse scale. Inside every 64-column step the columns are stored in the order of the format's A operand (gdec::colmap).
+// Two passes over the row: its largest magnitude with 16-byte loads, then (from the cache) eight source columns per lane into
+// one 16-byte store.
 template <uint32_t T, int DT>
-__global__ void rows_to_f16_k(const typename Elem<DT>::type * __restrict__ x, int rows, int k, bool wide_loads, __half * __restrict__ out,
-                              float * __restrict__ inv_scale) {
+__device__ __forceinline__ float row_to_f16(const typename Elem<DT>::type * __restrict__ xr, int k, bool wide_loads, __half * __restrict__ orow, int lane) {
     using E = typename Elem<DT>::type;
     constexpr int V = 16 / int(sizeof(E));                              // elements per 16-byte load
-    const int lane = threadIdx.x & 31, row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (row >= rows) return;
-    const E * xr = x + size_t(row) * k;
     float mx = 0.f;
     if (wide_loads) {                                                  // rows start on 16-byte boundaries (k is a multiple of 64)
 #pragma unroll 4
@@ -98,309 +112,406 @@ __global__ void rows_to_f16_k(const typename Elem<DT>::type * __restrict__ x, in
     int ex = int((__float_as_uint(mx) >> 23) & 255u) - 127;              // floor(log2(mx)) for a normal mx
     ex = (mx > 0.f && mx < 3e38f) ? max(-100, min(100, ex)) : 14;
     const float scale = __uint_as_float(uint32_t(127 + 14 - ex) << 23);  // 2^(14 - ex)
-    if (lane == 0) inv_scale[row] = __uint_as_float(uint32_t(127 - 14 + ex) << 23);
-    const int c0 = gdec::colmap<T>(2 * lane), c1 = gdec::colmap<T>(2 * lane + 1);       // source columns of this lane's two positions
-    __half2 * orow = reinterpret_cast<__half2 *>(out + size_t(row) * k) + lane;
-#pragma unroll 4
-    for (int gb = 0; gb < k; gb += 64)
-        orow[gb >> 1] = __floats2half2_rn(Elem<DT>::to_f(xr[gb + c0]) * scale, Elem<DT>::to_f(xr[gb + c1]) * scale);
+    int col[8];                                                        // source columns of this lane's eight positions, in its 64-column group
+#pragma unroll
+    for (int i = 0; i < 8; ++i) col[i] = gdec::colmap<T>(8 * (lane & 7) + i);
+#pragma unroll 2
+    for (int gb = 64 * (lane >> 3); gb < k; gb += 256) {
+        uint32_t v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = gdec::pack_h2(Elem<DT>::to_f(xr[gb + col[2 * i]]) * scale, Elem<DT>::to_f(xr[gb + col[2 * i + 1]]) * scale);
+        *reinterpret_cast<uint4 *>(orow + gb + 8 * (lane & 7)) = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+    return __uint_as_float(uint32_t(127 - 14 + ex) << 23);
+}
+// rows in their own order: the gathered form
+template <uint32_t T, int DT>
+__global__ void rows_to_f16_k(const typename Elem<DT>::type * __restrict__ x, int rows, int k, bool wide_loads, __half * __restrict__ out,
+                              float * __restrict__ inv_scale) {
+    const int lane = threadIdx.x & 31, row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    grid_release();
+    grid_wait();
+    if (row >= rows) return;
+    const float inv = row_to_f16<T, DT>(x + size_t(row) * k, k, wide_loads, out + size_t(row) * k, lane);
+    if (lane == 0) inv_scale[row] = inv;
+}
+// rows in the order of the plan's slots (a token's row once for every assignment it has; topk = 0: row = assignment)
+template <uint32_t T, int DT>
+__global__ void rows_to_slots_k(const typename Elem<DT>::type * __restrict__ x, const int * __restrict__ plan, int experts, int A, int topk, int k,
+                                bool wide_loads, __half * __restrict__ out, float * __restrict__ inv_scale) {
+    const int lane = threadIdx.x & 31, slot = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    grid_release();
+    grid_wait();
+    if (slot >= plan[PLAN_NGROUPED]) return;
+    const int e1 = experts + 1, a = plan[PLAN_HDR + e1 + e1 + 1 + e1 + slot];
+    const int row = topk == 0 ? a : a < A ? a / topk : a - A;
+    const float inv = row_to_f16<T, DT>(x + size_t(row) * k, k, wide_loads, out + size_t(slot) * k, lane);
+    if (lane == 0) inv_scale[slot] = inv;
 }
 
 // MODE 0: act[a][r] = silu(gate_r . x_tok(a)) * (up_r . x_tok(a));  MODE 1: y[a][r] = down_r . act[a]
-template <uint32_t T, int MODE, int NT>
-__global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p) {
-    constexpr int G_NT = NT, B_LBO = NT * 16, B_STAGE = 8 * B_LBO;      // B: bytes between k cores; NT tokens x 64 columns
-    constexpr int B_STAGES = NT == 128 ? 4 : 2, B_LAG = NT == 128 ? 2 : 1;
-    constexpr uint32_t ACC_SETS = NMAT * NT * 2 <= 512 ? 2 : 1;        // accumulator sets that fit the 512 tensor-memory columns
-    constexpr int KT = Fmt<T>::KT, TILE = Fmt<T>::TILE, CT = chunk_tiles<T>(), CB = chunk_bytes<T>();
-    constexpr uint32_t TMEM_COLS = 512;
-    extern __shared__ __align__(128) uint8_t smem[];
-    uint8_t * a_st = smem;                                            // [A_STAGES][NMAT][A_MAT]
-    uint8_t * b_st = a_st + A_STAGES * NMAT * A_MAT;                  // [B_STAGES][B_STAGE]
-    uint8_t * raw = b_st + B_STAGES * B_STAGE;                        // [8 warps][RAW_SLOTS][NMAT][CB]
-    uint8_t * dec_tab = raw + 8 * RAW_SLOTS * NMAT * CB;             // the decoder's lookup table
-    int * cum = reinterpret_cast<int *>(dec_tab + gdec::Dec<T>::TAB_BYTES);                                   // [na + 1]
-    uint64_t * bars = reinterpret_cast<uint64_t *>((reinterpret_cast<uintptr_t>(cum + p.experts + 3) + 15) & ~uintptr_t(15));
+template <uint32_t T, int MODE>
+__global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, const __grid_constant__ GemmMaps maps) {
+    using D = gdec::Dec<T>;
+    constexpr int CB = chunk_bytes<T>();
+    constexpr int ITEM_TILES = MODE == 0 ? 4 : 8;                      // row tiles of one matrix that an item covers
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t * smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t * b_st = smem;                                            // [b_stages][cap][128 bytes], swizzled
+    uint8_t * raw = b_st + size_t(p.b_stages) * p.cap * 128;          // [raw_slots][8 row tiles][CB]
+    uint8_t * dec_tab = raw + size_t(8) * p.raw_slots * CB;           // the decoder's lookup table
+    Info * info = reinterpret_cast<Info *>(dec_tab + D::TAB_BYTES);   // [na + 1]
+    int2 * tok = reinterpret_cast<int2 *>(info + p.experts + 2);      // [2][MAX_CAP]: assignment (-1: none) and activation scale of an item's tokens
+    uint64_t * bars = reinterpret_cast<uint64_t *>(tok + 2 * MAX_CAP);
     uint32_t * tmem_slot = reinterpret_cast<uint32_t *>(bars + N_BARS);
     volatile int * abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    const uint32_t raw_full = saddr(bars), raw_empty = raw_full + 8 * 8 * RAW_SLOTS, a_full = raw_empty + 8 * 8 * RAW_SLOTS, a_empty = a_full + 8 * MAX_A_STAGES,
-                   b_full = a_empty + 8 * MAX_A_STAGES, b_empty = b_full + 8 * MAX_B_STAGES, acc_full = b_empty + 8 * MAX_B_STAGES,
-                   acc_empty = acc_full + 16;
+    const int S = p.raw_slots, BS = p.b_stages;
+    const uint32_t raw_full = saddr(bars), raw_empty = raw_full + 8 * RAW_SLOTS, a_full = raw_empty + 8 * RAW_SLOTS,
+                   done = a_full + 8 * A_STAGES, b_full = done + 8 * STEP_RING, acc_full = b_full + 8 * MAX_B_STAGES, acc_empty = acc_full + 16,
+                   drain = acc_empty + 16, tok_bar = drain + 8;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int e1 = p.experts + 1;
     const int * counts = p.plan + PLAN_HDR, * offsets = counts + e1, * active = offsets + e1 + 1, * perm = active + e1;
-    constexpr int ITEM_TILES = MODE == 0 ? 8 : 16;                     // row tiles of one matrix that an item covers
-    const int na = p.plan[PLAN_NACTIVE], row_tiles = (p.rows + 15) >> 4, row_blocks = (row_tiles + ITEM_TILES - 1) / ITEM_TILES;
-    const int k_tiles = p.k / KT, ksteps = p.k / G_KS, nchunks = (k_tiles + CT - 1) / CT;
+    const int row_tiles = (p.rows + 15) >> 4, row_blocks = (row_tiles + ITEM_TILES - 1) / ITEM_TILES;
+    const int ksteps = p.k / G_KS, nunits = (ksteps + 1) >> 1, nchunks = (nunits + 1) >> 1;
 
-    gdec::Dec<T>::init(dec_tab, threadIdx.x, G_THREADS);
-    if (warp == 1) {                                                  // items before active expert i: cum[i]
-        int carry = 0;
-        for (int base = 0; base < na; base += 32) {
-            const int i = base + lane;
-            int v = i < na ? ((counts[active[i]] + G_NT - 1) / G_NT) * row_blocks : 0;
-            for (int d = 1; d < 32; d <<= 1) { const int o = __shfl_up_sync(0xffffffffu, v, d); if (lane >= d) v += o; }
-            if (i < na) cum[i + 1] = carry + v;
-            carry += __shfl_sync(0xffffffffu, v, 31);
-        }
-        if (lane == 0) cum[0] = 0;
-    }
+    D::init(dec_tab, threadIdx.x, G_THREADS);
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 8 * RAW_SLOTS; ++i) { bar_init(raw_full + 8 * i, 1); bar_init(raw_empty + 8 * i, 2); }
-        for (int i = 0; i < A_STAGES; ++i) { bar_init(a_full + 8 * i, DEC_WARPS); bar_init(a_empty + 8 * i, 1); }
-        for (int i = 0; i < MAX_B_STAGES; ++i) { bar_init(b_full + 8 * i, LOAD_WARPS); bar_init(b_empty + 8 * i, 1); }
-        for (int i = 0; i < 2; ++i) { bar_init(acc_full + 8 * i, 1); bar_init(acc_empty + 8 * i, 4); }
+        for (int i = 0; i < RAW_SLOTS; ++i) { bar_init(raw_full + 8 * i, 1); bar_init(raw_empty + 8 * i, 8); }
+        for (int i = 0; i < A_STAGES; ++i) bar_init(a_full + 8 * i, 8);
+        for (int i = 0; i < STEP_RING; ++i) bar_init(done + 8 * i, 1);
+        for (int i = 0; i < MAX_B_STAGES; ++i) bar_init(b_full + 8 * i, p.slots ? 1 : LOAD_WARPS);
+        for (int i = 0; i < 2; ++i) { bar_init(acc_full + 8 * i, 1); bar_init(acc_empty + 8 * i, EPI_WARPS); }
+        bar_init(drain, 1);
+        bar_init(tok_bar, EPI_WARPS);
         *abort_flag = 0;
         bar_init_fence();
     }
-    if (warp == MMA_WARP) tmem_alloc(saddr(tmem_slot), TMEM_COLS);
+    if (warp == MMA_WARP) tmem_alloc(saddr(tmem_slot), 512);
+    grid_wait();                                                      // the plan and the activation rows come from the launches before this one
+    const int na = p.plan[PLAN_NACTIVE];
+    for (int i = threadIdx.x; i < na; i += G_THREADS) {
+        const int e = active[i];
+        info[i] = Info{0, e, counts[e], offsets[e]};
+    }
     fence_before();
     __syncthreads();
     fence_after();
+    // an expert's tokens are spread evenly over the fewest tiles of at most `cap`
+    auto tiles_of = [&](int cnt) { return (cnt + p.cap - 1) / p.cap; };
+    if (warp == 0) {                                                  // items before active expert i
+        int carry = 0;
+        for (int base = 0; base < na; base += 32) {
+            const int i = base + lane;
+            const int mine = i < na ? tiles_of(info[i].cnt) * row_blocks : 0;
+            int v = mine;
+            for (int d = 1; d < 32; d <<= 1) { const int o = __shfl_up_sync(0xffffffffu, v, d); if (lane >= d) v += o; }
+            if (i < na) info[i].cum = carry + v - mine;
+            carry += __shfl_sync(0xffffffffu, v, 31);
+        }
+        if (lane == 0) info[na].cum = carry;
+    }
+    __syncthreads();
     const uint32_t tmem = *tmem_slot;
-    const int n_items = cum[na];
+    const int n_items = info[na].cum;
 
-    // item -> expert, first token slot, token count, row block
-    struct Item { int e, off, c0, nv, rb; };
-    auto locate = [&](int it) {
-        int lo = 0, hi = na - 1;
-        while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (cum[mid] <= it) lo = mid; else hi = mid - 1; }
+    // item -> expert, first token slot, token count, row block; called by whole warps, with `at` = the active expert of the
+    // warp's previous item (items only grow: usually one round of 32 probes)
+    struct Item { int e, slot0, nv, rb; };
+    auto locate = [&](int it, int & at) {
+        while (true) {
+            const unsigned m = __ballot_sync(0xffffffffu, at + 1 + lane < na && info[min(at + 1 + lane, na)].cum <= it);
+            at += __popc(m);
+            if (m != 0xffffffffu) break;
+        }
+        const Info f = info[at];
+        const int nt = tiles_of(f.cnt), per = ((f.cnt + nt - 1) / nt + 15) & ~15, local = it - f.cum, tile = local % nt;
         Item r;
-        r.e = active[lo];
-        const int cnt = counts[r.e], nt = (cnt + G_NT - 1) / G_NT, local = it - cum[lo];
-        r.off = offsets[r.e];
+        r.e = f.e;
         r.rb = local / nt;
-        r.c0 = (local - r.rb * nt) * G_NT;
-        r.nv = min(G_NT, cnt - r.c0);
+        r.slot0 = f.off + tile * per;
+        r.nv = max(0, min(per, f.cnt - tile * per));
         return r;
     };
+    auto x_row = [&](int a) { return MODE == 0 ? (a < p.A ? a / p.topk : a - p.A) : a; };
+    // the rows' boxes come in four sizes: the smallest that holds the item's tokens
+    auto b_class = [&](int nv) { return max(nv - 1, 0) / (p.cap / 4); };
     auto give_up = [&]() { *abort_flag = 1; atomicExch(p.plan + PLAN_STATUS, 2); };
+    int at = 0;
 
-    if (warp == MMA_WARP) {
-        // ---- MMA issuer ----
-        uint32_t gk = 0, ic = 0;
-        // descriptor halves: low = address / 16 | (bytes between k cores / 16) << 16; high = (128 / 16) | the format's fixed bit 46
-        const uint32_t a_lo0 = ((saddr(a_st) & 0x3FFFFu) >> 4) | (uint32_t(A_LBO >> 4) << 16);
-        const uint32_t b_lo0 = ((saddr(b_st) & 0x3FFFFu) >> 4) | (uint32_t(B_LBO >> 4) << 16);
-        const uint32_t a_hi = (128u >> 4) | (1u << 14), b_hi = a_hi;
-        for (int it = blockIdx.x; it < n_items && !*abort_flag; it += gridDim.x, ++ic) {
-            const Item im = locate(it);
-            const uint32_t npad = uint32_t(im.nv + 15) & ~15u, id = idesc(G_ROWS, npad, 0), ab = ic % ACC_SETS;
-            if (lane == 0) {
-                if (ic >= ACC_SETS && !bar_wait(acc_empty + 8 * ab, ((ic / ACC_SETS) - 1) & 1u, 100)) give_up();
-                fence_after();
-                for (int ks = 0; ks < ksteps && !*abort_flag; ++ks, ++gk) {
-                    const uint32_t sa = gk % A_STAGES, sb = gk % B_STAGES;
-                    if (!bar_wait(a_full + 8 * sa, (gk / A_STAGES) & 1u, 40)) { give_up(); break; }
-                    if (!bar_wait(b_full + 8 * sb, (gk / B_STAGES) & 1u, 40)) { give_up(); break; }
-                    fence_after();
-                    const uint32_t a_lo = a_lo0 + sa * uint32_t((NMAT * A_MAT) >> 4), b_lo = b_lo0 + sb * uint32_t(B_STAGE >> 4);
-                    const uint32_t d0 = tmem + ab * (NMAT * G_NT);
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-#pragma unroll
-                        for (int m = 0; m < NMAT; ++m)
-                            mma_f16_lohi(d0 + m * G_NT, a_lo + uint32_t((m * A_MAT + 2 * kk * A_LBO) >> 4), a_hi,
-                                         b_lo + uint32_t((2 * kk * B_LBO) >> 4), b_hi, id, (ks | kk) != 0);
-                    }
-                    mma_commit(a_empty + 8 * sa);
-                    mma_commit(b_empty + 8 * sb);
-                }
-                mma_commit(acc_full + 8 * ab);
+    if (warp >= EPI_WARP0 && warp < DEC_WARP0) {
+        // ---- epilogue: warps q and q + 4 read TMEM lanes [32 q, 32 q + 32) = rows of the block, 16-token groups in turn.
+        // What a store needs to know about its token (assignment, activation scale) lies in a table that the warps fill one
+        // item ahead, and is read for eight tokens before their stores (the compiler may not move a load over a store that
+        // could alias it: one load per store took 100 cycles per token, and two shuffles per token before that 140, which bound
+        // every product with a short K: c3 down, 80 tokens x K = 512: 412 us, 255 with the table) ----
+        const int q = warp & 3, tid = threadIdx.x - EPI_WARP0 * 32, first = 16 * ((warp - EPI_WARP0) >> 2);
+        const bool upper = lane >= 16;
+        int2 mine;
+        auto fetch = [&](const Item & im) {                            // this thread's token of the item
+            mine = make_int2(-1, 0);
+            if (tid < im.nv) {
+                mine.x = __ldg(perm + im.slot0 + tid);
+                mine.y = __float_as_int(__ldg(p.inv_scale + (p.slots ? im.slot0 + tid : x_row(mine.x))));
             }
+        };
+        auto put = [&](uint32_t n) {                                   // the table of the block's n-th item; then a (bounded) meeting of the warps
+            tok[(n & 1u) * MAX_CAP + tid] = mine;
             __syncwarp();
-        }
-    } else if (warp < LOAD_WARP0) {
-        // ---- epilogue: warp q reads TMEM lanes [32 q, 32 q + 32) = rows of the block ----
-        const int q = warp & 3;
-        uint32_t ic = 0;
-        for (int it = blockIdx.x; it < n_items && !*abort_flag; it += gridDim.x, ++ic) {
-            const Item im = locate(it);
-            const uint32_t ab = ic % ACC_SETS;
-            if (!__all_sync(0xffffffffu, bar_wait(acc_full + 8 * ab, (ic / ACC_SETS) & 1u, 1000))) { if (lane == 0) give_up(); break; }
-            fence_after();
-            // this thread's weight row in accumulator 0 and in accumulator 1 (the up matrix's same row, or the next row block)
-            const int row = im.rb * (ITEM_TILES * 16) + 32 * q + lane, row1 = MODE == 0 ? row : row + G_ROWS;
-            float rs[NMAT];                                            // fp32 row scales of the bank (NVFP4G), else 1
-            {
+            if (lane == 0) bar_arrive(tok_bar);
+            return warp_wait(tok_bar, n & 1u);
+        };
+        uint32_t next = 0, uses0 = 0, uses1 = 0, ic = 0;
+        Item im{}, after{};
+        bool ok = true;
+        if (int(blockIdx.x) < n_items) { im = locate(blockIdx.x, at); fetch(im); ok = put(0); }
+        for (int it = blockIdx.x; it < n_items && ok && !*abort_flag; it += gridDim.x, ++ic, im = after) {
+            const bool wide = im.nv > ACC_COLS, split = im.nv <= SPLIT_COLS;
+            const uint32_t h = wide ? 0 : next;
+            next = wide ? 0 : next ^ 1u;
+            if (it + int(gridDim.x) < n_items) { after = locate(it + gridDim.x, at); fetch(after); }
+            // this lane's weight row: row tiles of a quarter are (gate, up) of the same 16 output rows, or two tiles of the down matrix
+            const int row = MODE == 0 ? 16 * (im.rb * 4 + q) + (lane & 15) : 128 * im.rb + 32 * q + lane;
+            float rs = 1.f;                                            // fp32 row scale of the bank (NVFP4G)
+            if (p.aux0 && row < p.rows) {
                 const bool shared = im.e == p.experts;
-                const size_t ai = size_t(shared ? 0 : im.e) * row_tiles * 16;
-                const float * a0 = shared ? p.saux0 : p.aux0, * a1 = MODE == 0 ? (shared ? p.saux1 : p.aux1) : a0;
-                rs[0] = (a0 && row < p.rows) ? a0[ai + row] : 1.f;
-                rs[1] = (a1 && row1 < p.rows) ? a1[ai + row1] : 1.f;
+                const float * ax = MODE == 0 && upper ? (shared ? p.saux1 : p.aux1) : (shared ? p.saux0 : p.aux0);
+                rs = ax[size_t(shared ? 0 : im.e) * row_tiles * 16 + row];
             }
-            const uint32_t taddr = tmem + (uint32_t(32 * q) << 16) + ab * (NMAT * G_NT);
-            // the item's assignments and their activation scales, 32 per round in registers: the stores below may alias any
-            // global array as far as the compiler knows, so loads inside the token loop would each wait for the one before
-            int a_of[G_NT / 32];
-            float is_of[G_NT / 32];
-#pragma unroll
-            for (int i = 0; i < G_NT / 32; ++i) {
-                const int idx = 32 * i + lane;
-                a_of[i] = idx < im.nv ? perm[im.off + im.c0 + idx] : -1;
-                is_of[i] = a_of[i] >= 0 ? p.inv_scale[MODE == 0 ? (a_of[i] < p.A ? a_of[i] / p.topk : a_of[i] - p.A) : a_of[i]] : 0.f;
-            }
-#pragma unroll
-            for (int i = 0; i < G_NT / 32; ++i) {
-                if (32 * i >= im.nv) break;
-#pragma unroll
-                for (int c2 = 0; c2 < 32; c2 += 16) {
-                    const int c = 32 * i + c2;
-                    if (c >= im.nv) break;
-                    uint32_t g[16], u[16];
-                    tmem_ld16(taddr + c, g);
-                    tmem_ld16(taddr + G_NT + c, u);
+            if (!__all_sync(0xffffffffu, bar_wait(acc_full + 8 * h, (h ? uses1 : uses0) & 1u, 200))) { ok = false; break; }
+            if (h) ++uses1; else ++uses0;
+            fence_after();
+            const uint32_t taddr = tmem + (uint32_t(32 * q) << 16) + h * ACC_COLS;
+            const int4 * t = reinterpret_cast<const int4 *>(tok + (ic & 1u) * MAX_CAP);
+            float * out = p.out + row;
+            const bool in = row < p.rows;
+            for (int c = first; c < im.nv; c += 32) {
+                uint32_t v[16];
+                tmem_ld16(taddr + c, v);
+                if (split) {
+                    uint32_t w[16];
+                    tmem_ld16(taddr + SPLIT_COLS + c, w);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const int a = __shfl_sync(0xffffffffu, a_of[i], c2 + j);
-                        const float is = __shfl_sync(0xffffffffu, is_of[i], c2 + j);
-                        if (a >= 0 && row < p.rows) {
-                            const float gv = __uint_as_float(g[j]) * (is * rs[0]), uv = __uint_as_float(u[j]) * (is * rs[1]);
-                            p.out[size_t(a) * p.rows + row] = MODE == 0 ? __fdividef(gv, 1.f + __expf(-gv)) * uv : gv;      // fast exp and divide: relative error about 2^-21
-                            if (MODE == 1 && row1 < p.rows) p.out[size_t(a) * p.rows + row1] = uv;
+                    for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
+                } else {
+                    tmem_ld_wait();
+                }
+#pragma unroll
+                for (int j0 = 0; j0 < 16; j0 += 8) {
+                    int4 two[4];                                       // tokens j, j + 1: (assignment, scale) each
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) two[i] = t[(c + j0) / 2 + i];
+                    if (MODE == 0) {
+                        // lanes l and l + 16 hold gate and up of the same row: they swap, and l finishes the even tokens, l + 16 the odd ones
+                        float res[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float v0 = __uint_as_float(v[j0 + 2 * i]) * rs, v1 = __uint_as_float(v[j0 + 2 * i + 1]) * rs;
+                            const float other = __shfl_xor_sync(0xffffffffu, upper ? v0 : v1, 16);
+                            const float is = __int_as_float(upper ? two[i].w : two[i].y);
+                            const float gv = (upper ? other : v0) * is, uv = (upper ? v1 : other) * is;
+                            res[i] = __fdividef(gv, 1.f + __expf(-gv)) * uv;      // fast exp and divide: relative error about 2^-21
+                        }
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int a = upper ? two[i].z : two[i].x;
+                            if (in && a >= 0) out[size_t(a) * p.rows] = res[i];
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            if (in && two[i].x >= 0) out[size_t(two[i].x) * p.rows] = __uint_as_float(v[j0 + 2 * i]) * (__int_as_float(two[i].y) * rs);
+                            if (in && two[i].z >= 0) out[size_t(two[i].z) * p.rows] = __uint_as_float(v[j0 + 2 * i + 1]) * (__int_as_float(two[i].w) * rs);
                         }
                     }
                 }
             }
             fence_before();
             __syncwarp();
-            if (lane == 0) bar_arrive(acc_empty + 8 * ab);
-        }
-    } else if (warp < DEC_WARP0) {
-        // ---- B loader: thread n copies the 128 bytes of token rows n, n + 64, ... of every step, B_LAG steps in flight ----
-        const int n = threadIdx.x - LOAD_WARP0 * 32;
-        uint32_t gk = 0, arrived = 0;
-        bool ok = true;
-        auto arrive_next = [&]() {
-            fence_async_smem();
-            __syncwarp();
-            if (lane == 0) bar_arrive(b_full + 8 * (arrived % B_STAGES));
-            ++arrived;
-        };
-        for (int it = blockIdx.x; it < n_items && ok && !*abort_flag; it += gridDim.x) {
-            const Item im = locate(it);
-            const int npad = (im.nv + 15) & ~15;
-            constexpr int RPT = NT / LOAD_THREADS;                      // token rows per loader thread
-            const __half * src[RPT];
-            uint32_t src_bytes[RPT];
-#pragma unroll
-            for (int h = 0; h < RPT; ++h) {
-                src[h] = p.xb;
-                src_bytes[h] = 0;
-                if (n + LOAD_THREADS * h < im.nv) {
-                    const int a = perm[im.off + im.c0 + n + LOAD_THREADS * h];
-                    src[h] = p.xb + size_t(MODE == 0 ? (a < p.A ? a / p.topk : a - p.A) : a) * p.k;
-                    src_bytes[h] = 16;
-                }
+            if (lane == 0) {
+                bar_arrive(acc_empty + 8 * h);
+                if (wide) bar_arrive(acc_empty + 8);
             }
-            const uint32_t dst0 = saddr(b_st) + (n >> 3) * 128 + (n & 7) * 16;
-            for (int ks = 0; ks < ksteps; ++ks, ++gk) {
-                const uint32_t sb = gk % B_STAGES;
-                if (gk >= B_STAGES && !__all_sync(0xffffffffu, bar_wait(b_empty + 8 * sb, ((gk / B_STAGES) - 1) & 1u, 200))) { ok = false; break; }
-#pragma unroll
-                for (int h = 0; h < RPT; ++h) {
-                    if (n + LOAD_THREADS * h < npad) {
-#pragma unroll
-                        for (int c = 0; c < 8; ++c)
-                            cp_async16(dst0 + sb * B_STAGE + c * B_LBO + h * (LOAD_THREADS * 16), src[h] + (src_bytes[h] ? ks * G_KS + c * 8 : 0), src_bytes[h]);
-                    }
-                }
-                cp_async_commit();
-                if (gk - arrived >= B_LAG) { cp_async_wait<B_LAG>(); arrive_next(); }
-            }
+            ok = put(ic + 1);                                          // the other table: every warp has left the item that used it
         }
-        cp_async_wait<0>();
-        while (arrived < gk) arrive_next();
         if (!ok && lane == 0) give_up();
-    } else {
-        // ---- A decoder: warps tw and tw + 8 own row tile tw of the block (rows g / rows g + 8 of the tile): raw chunks
-        // (256 columns) -> fp16 operand, 64 columns a step; the first warp of the pair streams the chunks ----
-        const int dwi = warp - DEC_WARP0, tw = dwi & 7, half = dwi >> 3;
-        uint8_t * my_raw = raw + tw * RAW_SLOTS * NMAT * CB;
-        const uint32_t my_full = raw_full + 8 * tw * RAW_SLOTS, my_empty = raw_empty + 8 * tw * RAW_SLOTS;
-        uint32_t gk = 0, gc = 0;
+    } else if (warp >= DEC_WARP0) {
+        // ---- A decoder: raw chunks (256 columns of one row tile) -> fp16 operand in tensor memory, a unit (128 columns) a stage ----
+        const int j = warp - DEC_WARP0, q = j & 3, m = (j >> 2) & 1, parity = j >> 3, r = 2 * q + m;      // r: row tile of the block
+        const uint8_t * my_raw = raw + size_t(MODE == 0 ? 4 * m + q : r) * CB;
+        const uint32_t a_lane = tmem + (uint32_t(32 * q + 16 * m) << 16) + A_COL0;
+        uint32_t gu = 0, gc = 0, slot = 0, phase = 0;                  // unit, chunk; ring slot and phase of the next chunk
         bool ok = true;
         for (int it = blockIdx.x; it < n_items && ok && !*abort_flag; it += gridDim.x) {
-            const Item im = locate(it);
-            // row tile of accumulator 0 and of accumulator 1: the same tile of the gate and the up matrix, or tiles tw and tw + 8 of the item's 16
-            const int rt = im.rb * ITEM_TILES + tw, rt1 = MODE == 0 ? rt : rt + 8;
-            const bool live = rt < row_tiles, live1 = rt1 < row_tiles, shared = im.e == p.experts;      // live1 implies live
-            const uint8_t * bank0 = shared ? p.s0 : p.w0 + size_t(im.e) * p.bank_bytes;
-            const uint8_t * bank1 = MODE == 0 ? (shared ? p.s1 : p.w1 + size_t(im.e) * p.bank_bytes) : bank0;
-            const uint8_t * base[NMAT] = {bank0 + size_t(rt) * k_tiles * TILE, bank1 + size_t(rt1) * k_tiles * TILE};
-            // chunk c of this row tile -> the ring slot of use number u (lane 0 of the pair's first warp); false = gave up
-            auto issue = [&](int c, uint32_t u) {
-                const uint32_t slot = u % RAW_SLOTS;
-                if (u >= RAW_SLOTS && !bar_wait(my_empty + 8 * slot, ((u / RAW_SLOTS) - 1) & 1u)) return false;   // both warps are done with it
-                const int tiles = min(CT, k_tiles - c * CT);
-                const uint32_t bytes = uint32_t(tiles) * TILE, bar = my_full + 8 * slot;
-                bar_expect_tx(bar, live1 ? 2 * bytes : bytes);
-                bulk_copy(saddr(my_raw) + (slot * NMAT + 0) * CB, base[0] + size_t(c) * CT * TILE, bytes, bar);
-                if (live1) bulk_copy(saddr(my_raw) + (slot * NMAT + 1) * CB, base[1] + size_t(c) * CT * TILE, bytes, bar);
-                return true;
-            };
-            if (live && half == 0 && lane == 0)
-                for (int c = 0; c < RAW_SLOTS && c < nchunks; ++c)
-                    if (!issue(c, gc + c)) { give_up(); break; }
-            for (int c = 0; c < nchunks && ok; ++c, gc += live ? 1u : 0u) {     // a dead row tile (past the last row) uses no slot
-                const uint32_t slot = gc % RAW_SLOTS;
-                if (live && !__all_sync(0xffffffffu, bar_wait(my_full + 8 * slot, (gc / RAW_SLOTS) & 1u, DEC_BACKOFF))) { ok = false; break; }
-                const int steps = min(4, ksteps - 4 * c);
-                typename gdec::Dec<T>::Pre pre[NMAT];                  // per-chunk constants of the decoder
-                const uint8_t * chunk0 = my_raw + (slot * NMAT + 0) * CB, * chunk1 = my_raw + (slot * NMAT + 1) * CB;
-                typename gdec::Dec<T>::Raw rw[NMAT];                   // the raw words of the step that comes next
-                if (live) { pre[0] = gdec::Dec<T>::prep(chunk0, lane, half); rw[0] = gdec::Dec<T>::template load<0>(chunk0, lane, half); }
-                if (live1) { pre[1] = gdec::Dec<T>::prep(chunk1, lane, half); rw[1] = gdec::Dec<T>::template load<0>(chunk1, lane, half); }
-                // the (up to) four 64-column steps of the chunk, written out so that every step is straight-line code with its
-                // column offset a constant and the lane's row / table / scale addresses computed once per chunk
-                auto one_step = [&](auto J) {
-                    constexpr int j = decltype(J)::value;
-                    if (j >= steps || !ok) return;
-                    const uint32_t sa = gk % A_STAGES;
-                    if (gk >= A_STAGES && !__all_sync(0xffffffffu, bar_wait(a_empty + 8 * sa, ((gk / A_STAGES) - 1) & 1u, DEC_BACKOFF))) { ok = false; return; }
-                    const int row16 = (lane >> 2) + 8 * half, tq = lane & 3;
-                    if (live) {
-                        uint4 o[2];
-                        gdec::Dec<T>::template compute<j>(rw[0], chunk0, lane, dec_tab, half, pre[0], o);
-                        uint8_t * dst = a_st + (sa * NMAT + 0) * A_MAT + 2 * tw * 128;
-                        *gdec::core_row(dst, tq, row16) = o[0];
-                        *gdec::core_row(dst, tq + 4, row16) = o[1];
-                    }
-                    if (live1) {
-                        uint4 o[2];
-                        gdec::Dec<T>::template compute<j>(rw[1], chunk1, lane, dec_tab, half, pre[1], o);
-                        uint8_t * dst = a_st + (sa * NMAT + 1) * A_MAT + 2 * tw * 128;
-                        *gdec::core_row(dst, tq, row16) = o[0];
-                        *gdec::core_row(dst, tq + 4, row16) = o[1];
-                    }
-                    if (j + 1 < 4 && j + 1 < steps) {                  // the next step's raw words, in flight across the hand-off and the next wait
-                        if (live) rw[0] = gdec::Dec<T>::template load<(j + 1) & 3>(chunk0, lane, half);
-                        if (live1) rw[1] = gdec::Dec<T>::template load<(j + 1) & 3>(chunk1, lane, half);
-                    }
-                    fence_async_smem();
-                    __syncwarp();
-                    if (lane == 0) bar_arrive(a_full + 8 * sa);
-                    ++gk;
+            const Item im = locate(it, at);
+            const bool live = (MODE == 0 ? im.rb * 4 + q : im.rb * 8 + r) < row_tiles;      // a tile past the last row is not decoded
+            for (int c = 0; c < nchunks; ++c, ++gc) {
+                const int steps = min(4, ksteps - 4 * c), units = (steps + 1) >> 1;
+                if ((gc & 1u) == uint32_t(parity)) {
+                    const uint8_t * chunk = my_raw + slot * (8 * CB);
+                    typename D::Pre pre;
+                    if (!warp_wait(raw_full + 8 * slot, phase)) { ok = false; break; }
+                    if (live) pre = D::prep(chunk, lane);
+                    auto one_unit = [&](auto U) {
+                        constexpr int u = decltype(U)::value;
+                        if (u >= units || !ok) return;
+                        const uint32_t g = gu + u, sa = g % A_STAGES, a_addr = a_lane + sa * A_COLS;
+                        uint32_t f[16];
+                        if (live) D::template step<2 * u>(chunk, lane, dec_tab, pre, f);
+                        // the unit that used the stage before: its second step's products
+                        if (g >= A_STAGES && !warp_wait(done + 8 * ((2 * g + 1) % STEP_RING), ((g / A_STAGES) - 1) & 1u)) { ok = false; return; }
+                        if (live) {
+                            fence_after();
+                            tmem_st_16x256b_x4(a_addr, f);
+                            if (2 * u + 1 < steps) {
+                                D::template step<2 * u + 1>(chunk, lane, dec_tab, pre, f);
+                                tmem_st_16x256b_x4(a_addr + A_COLS / 2, f);
+                            }
+                            tmem_st_wait();
+                            fence_before();
+                        }
+                        __syncwarp();
+                        if (lane == 0) bar_arrive(a_full + 8 * sa);
+                    };
+                    one_unit(std::integral_constant<int, 0>{});
+                    one_unit(std::integral_constant<int, 1>{});
+                    if (!ok) break;
+                    if (lane == 0) bar_arrive(raw_empty + 8 * slot);               // every lane is done with the slot (the syncwarp above)
+                }
+                gu += units;
+                if (++slot == uint32_t(S)) { slot = 0; phase ^= 1u; }
+            }
+        }
+        if (!ok && lane == 0) give_up();
+    } else if (warp == MMA_WARP) {
+        // ---- MMA issuer: the whole warp walks the loop (its values stay in uniform registers), one elected lane issues ----
+        const uint32_t b_lo0 = sw128_desc_lo(saddr(b_st)), b_step = uint32_t(p.cap * 128) >> 4;
+        uint32_t gu = 0, sb = 0, pb = 0, next = 0, uses0 = 0, uses1 = 0;
+        bool ok = true;
+        for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x) {
+            const Item im = locate(it, at);
+            const bool wide = im.nv > ACC_COLS;
+            const uint32_t h = wide ? 0 : next;
+            next = wide ? 0 : next ^ 1u;
+            const uint32_t npad = uint32_t(max(im.nv, 1) + 15) & ~15u, id = idesc(128, npad, 0), d = tmem + h * ACC_COLS;
+            const uint32_t second = im.nv <= SPLIT_COLS ? SPLIT_COLS : 0;          // columns from the accumulator of even products to that of odd ones
+            const uint32_t b_half = p.slots ? (uint32_t(b_class(im.nv) + 1) * (p.cap / 4) * 128) >> 4 : b_step;       // from the first to the second step of a pair
+            if (wide || h == 0) { if (uses0 > 0) ok = warp_wait(acc_empty, (uses0 - 1) & 1u) && ok; ++uses0; }
+            if (wide || h == 1) { if (uses1 > 0) ok = warp_wait(acc_empty + 8, (uses1 - 1) & 1u) && ok; ++uses1; }
+            fence_after();
+            for (int u = 0; u < nunits && ok; ++u, ++gu) {
+                const uint32_t sa = gu % A_STAGES;
+                if (!warp_wait(a_full + 8 * sa, (gu / A_STAGES) & 1u)) { ok = false; break; }
+                // the two steps of the unit; the second one of an odd K's last unit is empty: no products, but its barriers turn
+                const uint32_t a = tmem + A_COL0 + sa * A_COLS;
+                auto products = [&](int half, uint32_t b_lo) {
+                    if (2 * u + half >= ksteps) return;
+#pragma unroll
+                    for (uint32_t kk = 0; kk < 4; ++kk)
+                        mma_f16_ts(d + (kk & 1 ? second : 0), a + half * (A_COLS / 2) + 8 * kk, b_lo + 2 * kk, SW128_DESC_HI, id,
+                                   half > 0 || u > 0 || kk > (second ? 1 : 0));
                 };
-                one_step(std::integral_constant<int, 0>{});
-                one_step(std::integral_constant<int, 1>{});
-                one_step(std::integral_constant<int, 2>{});
-                one_step(std::integral_constant<int, 3>{});
-                if (!ok) break;
-                __syncwarp();                                          // every lane is done with the slot
-                if (live && lane == 0) {
-                    bar_arrive(my_empty + 8 * slot);
-                    if (half == 0 && c + RAW_SLOTS < nchunks && !issue(c + RAW_SLOTS, gc + RAW_SLOTS)) { give_up(); ok = false; }
+                if (!warp_wait(b_full + 8 * sb, pb)) { ok = false; break; }
+                fence_after();
+                uint32_t b_lo = b_lo0 + sb * b_step;
+                if (!p.b_pair) {
+                    if (elect_one()) {
+                        products(0, b_lo);
+                        mma_commit(done + 8 * (2 * sa));
+                    }
+                    __syncwarp();
+                    if (++sb == uint32_t(BS)) { sb = 0; pb ^= 1u; }
+                    if (!warp_wait(b_full + 8 * sb, pb)) { ok = false; break; }
+                    fence_after();
+                    b_lo = b_lo0 + sb * b_step;
                 }
-                ok = __all_sync(0xffffffffu, ok);
+                if (elect_one()) {
+                    if (p.b_pair) { products(0, b_lo); products(1, b_lo + b_half); }
+                    else products(1, b_lo);
+                    mma_commit(done + 8 * (2 * sa + 1));
+                    if (u == nunits - 1) mma_commit(acc_full + 8 * h);
+                }
+                __syncwarp();
+                sb += p.b_pair ? 2 : 1;
+                if (sb == uint32_t(BS)) { sb = 0; pb ^= 1u; }
             }
         }
         if (!ok && lane == 0) give_up();
+        // nothing may be in flight when the tensor memory is freed (after a clean run the epilogue has waited for all of it)
+        if (elect_one()) { mma_commit(drain); bar_wait(drain, 0); }
+        __syncwarp();
+    } else if (warp == RAW_WARP) {
+        // ---- raw blocks ----
+        constexpr int PARTS = chunk_parts<T>();
+        constexpr uint32_t BYTES = 8 * CB;
+        uint32_t issued = 0, slot = 0, phase = 1;                      // phase: of the empty barrier's wait (none in the first round)
+        bool ok = true;
+        for (int it = blockIdx.x; it < n_items && ok && !*abort_flag; it += gridDim.x) {
+            const Item im = locate(it, at);
+            const CUtensorMap * map = maps.w + (im.e == p.experts ? 2 : 0);
+            const int rt = (im.e == p.experts ? 0 : im.e * row_tiles) + im.rb * ITEM_TILES;        // rows past the matrix: the next expert's, never used
+            for (int c = 0; c < nchunks; ++c) {
+                if (issued >= uint32_t(S) && !warp_wait(raw_empty + 8 * slot, phase)) { ok = false; break; }
+                if (elect_one()) {
+                    const uint32_t bar = raw_full + 8 * slot, dst = saddr(raw) + slot * BYTES;
+                    bar_expect_tx(bar, BYTES);
+                    tma_load_3d(dst, map, 0, c * PARTS, rt, bar);
+                    if (MODE == 0) tma_load_3d(dst + BYTES / 2, map + 1, 0, c * PARTS, rt, bar);
+                }
+                __syncwarp();
+                ++issued;
+                if (++slot == uint32_t(S)) { slot = 0; phase ^= 1u; }
+            }
+        }
+        if (!ok && lane == 0) give_up();
+        // before leaving, every copy must have landed (after a clean run these waits return at once)
+        for (uint32_t i = issued > uint32_t(S) ? issued - S : 0; i < issued; ++i) bar_wait(raw_full + 8 * (i % S), (i / S) & 1u);
+    } else {
+        // ---- B loader: warp 2 brings a step's (or a unit's) rows with one box; a gathering launch: lane l of warp w brings rows
+        // 4 (2 l + w) .. + 3 ----
+        const int lw = warp - LOAD_WARP0, n0 = 4 * (2 * lane + lw), group = p.b_pair ? 2 : 1;      // steps that share a barrier
+        uint32_t gk = 0, sb = 0;
+        bool ok = true;
+        for (int it = blockIdx.x; it < n_items && ok && !*abort_flag && (lw == 0 || !p.slots); it += gridDim.x) {
+            const Item im = locate(it, at);
+            int row[4] = {0, 0, 0, 0};
+            if (!p.slots) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) row[i] = n0 < im.nv ? x_row(__ldg(perm + im.slot0 + min(n0 + i, im.nv - 1))) : 0;      // past the last token: repeat it (dead columns of D)
+            }
+            const int cls = b_class(im.nv), quads = (im.nv + 3) >> 2, mine = (quads + 1 - lw) >> 1;
+            const uint32_t box_bytes = uint32_t((cls + 1) * (p.cap / 4) * group) * 128u;
+            for (int ks = 0; ks < 2 * nunits; ks += group, gk += group) {
+                const uint32_t freed = gk + group - 1 - uint32_t(BS);  // the (last) step that used the stage before
+                if (gk >= uint32_t(BS) && !warp_wait(done + 8 * (freed % STEP_RING), (freed / STEP_RING) & 1u)) { ok = false; break; }
+                const uint32_t bar = b_full + 8 * sb, dst = saddr(b_st) + sb * uint32_t(p.cap * 128);
+                if (p.slots) {
+                    if (elect_one()) {
+                        bar_expect_tx(bar, box_bytes);
+                        tma_load_3d(dst, maps.x + cls, 0, im.slot0, ks, bar);      // the second step of an odd K's last unit lies outside: zeros
+                    }
+                    __syncwarp();
+                } else {
+                    const int real = min(group, ksteps - ks);
+                    if (lane == 0) bar_expect_tx(bar, uint32_t(max(real, 0) * mine) * 512u);
+                    __syncwarp();
+                    if (n0 < im.nv)
+                        for (int i = 0; i < real; ++i)
+                            tma_gather4(dst + i * uint32_t(p.cap * 128) + n0 * 128, maps.x, (ks + i) * G_KS, row[0], row[1], row[2], row[3], bar);
+                }
+                sb += group;
+                if (sb == uint32_t(BS)) sb = 0;
+            }
+        }
+        if (!ok && lane == 0) give_up();
+        // before leaving, every copy into the stages must have landed (after a clean run these waits return at once)
+        for (uint32_t g = gk > uint32_t(BS) ? gk - BS : 0; g < gk; g += group) bar_wait(b_full + 8 * (g % BS), (g / BS) & 1u);
     }
+    grid_release();
     fence_before();
     __syncthreads();
-    if (warp == MMA_WARP) tmem_free(tmem, TMEM_COLS);
+    if (warp == MMA_WARP) tmem_free(tmem, 512);
 }
 
 int gemm_sm_count() {
@@ -410,103 +521,146 @@ int gemm_sm_count() {
 }
 constexpr size_t GEMM_SMEM_LIMIT = 232448 - 1024;
 
-template <uint32_t T, int MODE, int NT>
-int32_t gemm_launch_nt(const GemmArgs & a, int sms, cudaStream_t s) {
-    const size_t smem = gemm_smem<T, NT>(a.experts);
-    if (smem > GEMM_SMEM_LIMIT) return B2MOE_ERR_SHAPE;
-    if (cudaFuncSetAttribute(gemm_tc_k<T, MODE, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return B2MOE_ERR_CUDA;
-    gemm_tc_k<T, MODE, NT><<<sms, G_THREADS, smem, s>>>(a);
+// shared-memory split of a launch: the widest items wanted first, then narrower ones (their B stages are smaller) until the raw
+// ring holds at least three chunks
+int g_item_tokens = 0;                      // test hook: 256 = 256-token items whatever the batch
+template <uint32_t T> bool gemm_fit(int experts, int cap_wanted, GemmArgs & a) {
+    constexpr int opts[4][3] = {{256, 4, 3}, {128, 8, 3}, {64, 8, 3}, {64, 4, 2}};      // tokens per item, B stages, fewest raw slots
+    for (const auto & o : opts) {
+        if (o[0] > cap_wanted) continue;
+        for (int s = RAW_SLOTS; s >= o[2]; --s)
+            if (gemm_smem<T>(experts, o[0], o[1], s) <= GEMM_SMEM_LIMIT) {
+                a.cap = o[0]; a.b_stages = o[1]; a.raw_slots = s;
+                a.b_pair = o[0] < 256;
+                return true;
+            }
+    }
+    return false;
+}
+decltype(&cuTensorMapEncodeTiled) map_encoder() {
+    static const auto encode = []() -> decltype(&cuTensorMapEncodeTiled) {
+        void * f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess) f = nullptr;
+        return reinterpret_cast<decltype(&cuTensorMapEncodeTiled)>(f);
+    }();
+    return encode;
+}
+bool encode_map(CUtensorMap & m, CUtensorMapDataType type, int rank, const void * base, const cuuint64_t * dims, const cuuint64_t * strides,
+                const cuuint32_t * box, CUtensorMapSwizzle swizzle) {
+    const cuuint32_t steps[3] = {1, 1, 1};
+    const auto encode = map_encoder();
+    return encode && encode(&m, type, rank, const_cast<void *>(base), dims, strides, box, steps, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// `rows` fp16 activation rows of length k as [k / 64][rows][64]: a box is box_rows rows of `steps` 64-column steps, one step after the other
+bool rows_map(CUtensorMap & m, const void * xb, int rows, int k, int box_rows, int steps) {
+    const cuuint64_t dims[3] = {G_KS, cuuint64_t(rows), cuuint64_t(k / G_KS)}, strides[2] = {cuuint64_t(k) * 2, G_KS * 2};
+    const cuuint32_t box[3] = {G_KS, cuuint32_t(box_rows), cuuint32_t(steps)};
+    return encode_map(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, xb, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+// the same rows for tile::gather4
+bool gather_map(CUtensorMap & m, const void * xb, int rows, int k) {
+    const cuuint64_t dims[2] = {cuuint64_t(k), cuuint64_t(rows)}, strides[1] = {cuuint64_t(k) * 2};
+    const cuuint32_t box[2] = {G_KS, 1};
+    return encode_map(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, xb, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+// a bank's tiles as [experts * row tiles][parts of a chunk][8-byte words]: a box is one 256-column chunk of `tiles` consecutive row tiles
+template <uint32_t T> bool bank_map(CUtensorMap & m, const b2moe_bank * b, int tiles) {
+    constexpr int PW = part_words<T>();
+    const cuuint64_t line = cuuint64_t(b->cols / Fmt<T>::KT) * Fmt<T>::TILE;       // bytes of a row tile
+    const cuuint64_t dims[3] = {cuuint64_t(PW), line / (PW * 8), cuuint64_t(b->experts) * ((b->rows + 15) / 16)}, strides[2] = {PW * 8, line};
+    const cuuint32_t box[3] = {PW, chunk_parts<T>(), cuuint32_t(tiles)};
+    return encode_map(m, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, b->data, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
+}
+template <uint32_t T, int DT>
+int32_t convert_rows_dt(const void * x, int rows, int k, bool slots, const GemmArgs & a, int topk, __half * out, float * inv, cudaStream_t s) {
+    using E = typename Elem<DT>::type;
+    const dim3 grid(ceil_div(rows, 8)), block(256);
+    const bool wide = aligned16(x);
+    if (slots) launch_overlapped(rows_to_slots_k<T, DT>, grid, block, 0, s, static_cast<const E *>(x), static_cast<const int *>(a.plan), a.experts, a.A, topk, k, wide, out, inv);
+    else launch_overlapped(rows_to_f16_k<T, DT>, grid, block, 0, s, static_cast<const E *>(x), rows, k, wide, out, inv);
     return launch_status();
 }
-// 128-token items. The 256-token variant (weights decoded once per 256 tokens, but one accumulator set and two B stages) is
-// correct and slower where it was measured (c5, 512 tokens per expert: 261 against 395 TFLOP/s: the gathered B loads with one
-// step of lookahead become the limit); b2moe_harness_select(.., 256) selects it for measurements
-int g_item_tokens = 128;
+// m: the banks (gate, up) or (down, null), then the shared expert's (null: none); x (rows_x rows, in token order for MODE 0, in
+// assignment order for MODE 1) -> fp16 rows in xb (in slot order: slot_rows of them), then the product
 template <uint32_t T, int MODE>
-int32_t gemm_launch_t(const GemmArgs & a, cudaStream_t s) {
+int32_t gemm_launch_t(GemmArgs a, const b2moe_bank * const * m, const void * x, int dtype, int rows_x, bool slots, int slot_rows, __half * xb, float * inv, cudaStream_t s) {
     const int sms = gemm_sm_count();
     if (sms <= 0) return B2MOE_ERR_CUDA;
-    const bool wide = g_item_tokens == 256;
-    if (wide && gemm_smem<T, 256>(a.experts) <= GEMM_SMEM_LIMIT) return gemm_launch_nt<T, MODE, 256>(a, sms, s);
-    return gemm_launch_nt<T, MODE, 128>(a, sms, s);
-}
-template <int MODE>
-int32_t gemm_launch(uint32_t type, const GemmArgs & a, cudaStream_t s) {
-    switch (type) {
-        case T_Q4_K: return gemm_launch_t<T_Q4_K, MODE>(a, s);
-        case T_IQ3_S: return gemm_launch_t<T_IQ3_S, MODE>(a, s);
-        case T_IQ3S4: return gemm_launch_t<T_IQ3S4, MODE>(a, s);
-        case T_IQ4_XS: return gemm_launch_t<T_IQ4_XS, MODE>(a, s);
-        case T_IQ4_NL: return gemm_launch_t<T_IQ4_NL, MODE>(a, s);
-        case T_NVFP4G: return gemm_launch_t<T_NVFP4G, MODE>(a, s);
-    }
-    return B2MOE_ERR_FORMAT;
-}
-size_t gemm_smem_of(uint32_t type, int experts) {
-    switch (type) {
-        case T_Q4_K: return gemm_smem<T_Q4_K, 128>(experts);
-        case T_IQ3_S: return gemm_smem<T_IQ3_S, 128>(experts);
-        case T_IQ3S4: return gemm_smem<T_IQ3S4, 128>(experts);
-        case T_IQ4_XS: return gemm_smem<T_IQ4_XS, 128>(experts);
-        case T_IQ4_NL: return gemm_smem<T_IQ4_NL, 128>(experts);
-        case T_NVFP4G: return gemm_smem<T_NVFP4G, 128>(experts);
-    }
-    return ~size_t(0);
-}
-template <uint32_t T>
-int32_t convert_rows_t(const void * x, int dtype, int rows, int k, __half * out, float * inv, cudaStream_t s) {
-    const int blocks = ceil_div(rows, 8);
-    const bool wide = aligned16(x);
-    switch (dtype) {
-        case B2MOE_F32: rows_to_f16_k<T, B2MOE_F32><<<blocks, 256, 0, s>>>(static_cast<const float *>(x), rows, k, wide, out, inv); break;
-        case B2MOE_F16: rows_to_f16_k<T, B2MOE_F16><<<blocks, 256, 0, s>>>(static_cast<const __half *>(x), rows, k, wide, out, inv); break;
-        case B2MOE_BF16: rows_to_f16_k<T, B2MOE_BF16><<<blocks, 256, 0, s>>>(static_cast<const __nv_bfloat16 *>(x), rows, k, wide, out, inv); break;
-        default: return B2MOE_ERR_SHAPE;
-    }
+    const long long per = (long long)a.A / a.experts;                 // mean tokens per expert
+    const int cap = g_item_tokens == 256 || per > 128 ? 256 : per > 24 ? 128 : 64;
+    if (!gemm_fit<T>(a.experts, cap, a)) return B2MOE_ERR_SHAPE;
+    const int rows = slots ? slot_rows : rows_x, topk = MODE == 0 ? a.topk : 0;
+    int32_t rc = B2MOE_ERR_SHAPE;
+    if (dtype == B2MOE_F32) rc = convert_rows_dt<T, B2MOE_F32>(x, rows, a.k, slots, a, topk, xb, inv, s);
+    else if (dtype == B2MOE_F16) rc = convert_rows_dt<T, B2MOE_F16>(x, rows, a.k, slots, a, topk, xb, inv, s);
+    else if (dtype == B2MOE_BF16) rc = convert_rows_dt<T, B2MOE_BF16>(x, rows, a.k, slots, a, topk, xb, inv, s);
+    if (rc) return rc;
+    a.slots = slots;
+    a.inv_scale = inv;
+    GemmMaps maps;
+    bool mapped = true;
+    if (slots) for (int i = 0; i < 4; ++i) mapped = mapped && rows_map(maps.x[i], xb, rows, a.k, (i + 1) * a.cap / 4, a.b_pair ? 2 : 1);
+    else mapped = gather_map(maps.x[0], xb, rows, a.k);
+    for (int i = 0; i < 4; ++i)
+        if (m[i]) mapped = mapped && bank_map<T>(maps.w[i], m[i], MODE == 0 ? 4 : 8);
+    if (!mapped) return B2MOE_ERR_CUDA;
+    const size_t smem = gemm_smem<T>(a.experts, a.cap, a.b_stages, a.raw_slots);
+    if (cudaFuncSetAttribute(gemm_tc_k<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return B2MOE_ERR_CUDA;
+    launch_overlapped(gemm_tc_k<T, MODE>, dim3(sms), dim3(G_THREADS), smem, s, a, maps);
     return launch_status();
 }
-int32_t convert_rows(uint32_t type, const void * x, int dtype, int rows, int k, __half * out, float * inv, cudaStream_t s) {
+template <int MODE, typename... Args>
+int32_t gemm_launch(uint32_t type, const Args &... args) {
     switch (type) {
-        case T_Q4_K: return convert_rows_t<T_Q4_K>(x, dtype, rows, k, out, inv, s);
-        case T_IQ3_S: return convert_rows_t<T_IQ3_S>(x, dtype, rows, k, out, inv, s);
-        case T_IQ3S4: return convert_rows_t<T_IQ3S4>(x, dtype, rows, k, out, inv, s);
-        case T_IQ4_XS: return convert_rows_t<T_IQ4_XS>(x, dtype, rows, k, out, inv, s);
-        case T_IQ4_NL: return convert_rows_t<T_IQ4_NL>(x, dtype, rows, k, out, inv, s);
-        case T_NVFP4G: return convert_rows_t<T_NVFP4G>(x, dtype, rows, k, out, inv, s);
+        case T_Q4_K: return gemm_launch_t<T_Q4_K, MODE>(args...);
+        case T_IQ3_S: return gemm_launch_t<T_IQ3_S, MODE>(args...);
+        case T_IQ3S4: return gemm_launch_t<T_IQ3S4, MODE>(args...);
+        case T_IQ4_XS: return gemm_launch_t<T_IQ4_XS, MODE>(args...);
+        case T_IQ4_NL: return gemm_launch_t<T_IQ4_NL, MODE>(args...);
+        case T_NVFP4G: return gemm_launch_t<T_NVFP4G, MODE>(args...);
     }
     return B2MOE_ERR_FORMAT;
+}
+bool gemm_fits(uint32_t type, int experts) {
+    GemmArgs a{};
+    switch (type) {
+        case T_Q4_K: return gemm_fit<T_Q4_K>(experts, 64, a);
+        case T_IQ3_S: return gemm_fit<T_IQ3_S>(experts, 64, a);
+        case T_IQ3S4: return gemm_fit<T_IQ3S4>(experts, 64, a);
+        case T_IQ4_XS: return gemm_fit<T_IQ4_XS>(experts, 64, a);
+        case T_IQ4_NL: return gemm_fit<T_IQ4_NL>(experts, 64, a);
+        case T_NVFP4G: return gemm_fit<T_NVFP4G>(experts, 64, a);
+    }
+    return false;
 }
 
 }  // namespace
 
-void gemm_tc_item_tokens(int tokens) { g_item_tokens = tokens == 256 ? 256 : 128; }
-// true when the tensor-core GEMM takes banks of this type with rows of length k (nmat: 2 = gate/up, 1 = down)
-bool gemm_tc_supported(uint32_t type, int k, int nmat, int experts) {
-    (void)nmat;                                                       // both products stage two row blocks per item
-    return k >= G_KS && k % G_KS == 0 && gemm_smem_of(type, experts) <= GEMM_SMEM_LIMIT;
-}
+void gemm_tc_item_tokens(int tokens) { g_item_tokens = tokens; }
+// true when the tensor-core GEMM takes banks of this type with rows of length k
+bool gemm_tc_supported(uint32_t type, int k, int experts) { return k >= G_KS && k % G_KS == 0 && gemm_fits(type, experts); }
 // scratch: the scaled fp16 copy of `rows_x` activation rows of length k and one float per row
 size_t gemm_tc_workspace_bytes(int rows_x, int k) {
     return align_up(size_t(rows_x) * k * 2, 256) + align_up(size_t(rows_x) * sizeof(float), 256);
 }
 
+// rows_buf: optional scratch for the activation rows in slot order (n * topk + shared_tokens rows of length k and their scales)
 int32_t gemm_tc_gateup(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_bank * sg, const b2moe_bank * su, const void * x,
-                       int x_dtype, const int * plan, int n, int topk, int shared_tokens, float * act, void * ws, cudaStream_t s) {
-    const int k = gate->cols;
-    __half * xb = static_cast<__half *>(ws);
-    float * inv = reinterpret_cast<float *>(static_cast<uint8_t *>(ws) + align_up(size_t(n) * k * 2, 256));
-    if (int32_t rc = convert_rows(gate->type, x, x_dtype, n, k, xb, inv, s)) return rc;
+                       int x_dtype, const int * plan, int n, int topk, int shared_tokens, float * act, void * ws, void * rows_buf,
+                       size_t rows_buf_bytes, cudaStream_t s) {
+    const int k = gate->cols, slot_rows = n * topk + shared_tokens;
+    const bool slots = rows_buf && rows_buf_bytes >= gemm_tc_workspace_bytes(slot_rows, k);
+    __half * xb = static_cast<__half *>(slots ? rows_buf : ws);
+    float * inv = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(xb) + align_up(size_t(slots ? slot_rows : n) * k * 2, 256));
     GemmArgs a{};
-    a.w0 = static_cast<const uint8_t *>(gate->data); a.w1 = static_cast<const uint8_t *>(up->data);
+    const b2moe_bank * banks[4] = {gate, up, shared_tokens ? sg : nullptr, shared_tokens ? su : nullptr};
     a.aux0 = static_cast<const float *>(gate->aux); a.aux1 = static_cast<const float *>(up->aux);
-    if (shared_tokens) {
-        a.s0 = static_cast<const uint8_t *>(sg->data); a.s1 = static_cast<const uint8_t *>(su->data);
-        a.saux0 = static_cast<const float *>(sg->aux); a.saux1 = static_cast<const float *>(su->aux);
-    }
-    a.bank_bytes = b2moe_bank_bytes(gate->type, gate->rows, gate->cols);
-    a.xb = xb; a.inv_scale = inv; a.plan = const_cast<int *>(plan); a.out = act;
+    if (shared_tokens) { a.saux0 = static_cast<const float *>(sg->aux); a.saux1 = static_cast<const float *>(su->aux); }
+    a.plan = const_cast<int *>(plan); a.out = act;
     a.rows = gate->rows; a.k = k; a.experts = gate->experts; a.topk = topk; a.A = n * topk;
-    return gemm_launch<0>(gate->type, a, s);
+    return gemm_launch<0>(gate->type, a, banks, x, x_dtype, n, slots, slot_rows, xb, inv, s);
 }
 
 int32_t gemm_tc_down(const b2moe_bank * down, const b2moe_bank * sd, const float * act, const int * plan, int n, int topk,
@@ -514,15 +668,13 @@ int32_t gemm_tc_down(const b2moe_bank * down, const b2moe_bank * sd, const float
     const int rows_x = n * topk + shared_tokens, k = down->cols;
     __half * xb = static_cast<__half *>(ws);
     float * inv = reinterpret_cast<float *>(static_cast<uint8_t *>(ws) + align_up(size_t(rows_x) * k * 2, 256));
-    if (int32_t rc = convert_rows(down->type, act, B2MOE_F32, rows_x, k, xb, inv, s)) return rc;
     GemmArgs a{};
-    a.w0 = static_cast<const uint8_t *>(down->data);
+    const b2moe_bank * banks[4] = {down, nullptr, shared_tokens ? sd : nullptr, nullptr};
     a.aux0 = static_cast<const float *>(down->aux);
-    if (shared_tokens) { a.s0 = static_cast<const uint8_t *>(sd->data); a.saux0 = static_cast<const float *>(sd->aux); }
-    a.bank_bytes = b2moe_bank_bytes(down->type, down->rows, down->cols);
-    a.xb = xb; a.inv_scale = inv; a.plan = const_cast<int *>(plan); a.out = y;
+    if (shared_tokens) a.saux0 = static_cast<const float *>(sd->aux);
+    a.plan = const_cast<int *>(plan); a.out = y;
     a.rows = down->rows; a.k = k; a.experts = down->experts; a.topk = topk; a.A = n * topk;
-    return gemm_launch<1>(down->type, a, s);
+    return gemm_launch<1>(down->type, a, banks, static_cast<const void *>(act), int(B2MOE_F32), rows_x, true, rows_x, xb, inv, s);
 }
 
 }  // namespace b2

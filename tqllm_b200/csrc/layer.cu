@@ -30,10 +30,10 @@ void dec4_ring(int nbuf, int stages, int slot_tiles);
 void dec4_ksplit_max(int ks);
 unsigned long long g_launch_count = 0;
 bool g_overlap = true;
-bool gemm_tc_supported(uint32_t type, int k, int nmat, int experts);
+bool gemm_tc_supported(uint32_t type, int k, int experts);
 size_t gemm_tc_workspace_bytes(int rows_x, int k);
 int32_t gemm_tc_gateup(const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const void *, int, const int *, int,
-                       int, int, float *, void *, cudaStream_t);
+                       int, int, float *, void *, void * rows_buf, size_t rows_buf_bytes, cudaStream_t);
 int32_t gemm_tc_down(const b2moe_bank *, const b2moe_bank *, const float *, const int *, int, int, int, float *, void *, cudaStream_t);
 void gemm_tc_item_tokens(int tokens);
 
@@ -65,9 +65,9 @@ int decode_kernel(uint32_t type, int k, int dtype) {
 // else the GEMM. b2moe_harness_select forces a family where it supports the shape (tests and benchmarks).
 constexpr int GEMM_MIN_PER = 32, GEMM_MIN_EXPERTS = 128;   // measured on the c2 shape: below either, the decode kernels' finer work items win
 int g_family = B2MOE_FAMILY_AUTO;
-int expert_path(uint32_t type, int k, int dtype, int nmat, int experts, long long assignments) {
+int expert_path(uint32_t type, int k, int dtype, int experts, long long assignments) {
     if (g_family == B2MOE_FAMILY_GENERIC) return B2MOE_FAMILY_GENERIC;
-    const bool dec = decode_kernel(type, k, dtype) != DEC_NONE, gemm = gemm_tc_supported(type, k, nmat, experts);
+    const bool dec = decode_kernel(type, k, dtype) != DEC_NONE, gemm = gemm_tc_supported(type, k, experts);
     if (g_family == B2MOE_FAMILY_DECODE) return dec ? B2MOE_FAMILY_DECODE : B2MOE_FAMILY_GENERIC;
     if (g_family == B2MOE_FAMILY_GEMM) return gemm ? B2MOE_FAMILY_GEMM : dec ? B2MOE_FAMILY_DECODE : B2MOE_FAMILY_GENERIC;
     if (dec && (!gemm || assignments < (long long)GEMM_MIN_PER * experts || experts < GEMM_MIN_EXPERTS)) return B2MOE_FAMILY_DECODE;
@@ -76,7 +76,7 @@ int expert_path(uint32_t type, int k, int dtype, int nmat, int experts, long lon
 }  // namespace
 // true when b2moe_expert_down would take the format-generic kernels (which use no scratch) for this call
 bool expert_down_is_generic(const b2moe_bank * down, int n, int topk) {
-    return expert_path(down->type, down->cols, B2MOE_F32, 1, down->experts, (long long)n * topk) == B2MOE_FAMILY_GENERIC;
+    return expert_path(down->type, down->cols, B2MOE_F32, down->experts, (long long)n * topk) == B2MOE_FAMILY_GENERIC;
 }
 }  // namespace b2
 
@@ -123,10 +123,12 @@ extern "C" B2MOE_API size_t b2moe_expert_workspace_bytes(uint32_t type, int32_t 
     return g > need ? g : need;
 }
 
-// x_staged: the caller has already written the staged form of x where the 4-bit decode kernels expect it (b2moe_layer_forward)
+// x_staged: the caller has already written the staged form of x where the 4-bit decode kernels expect it (b2moe_layer_forward);
+// rows_buf: scratch the caller has to spare for the grouped GEMM's activation rows in slot order (null: it gathers them)
 static int32_t expert_gateup(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_bank * shared_gate, const b2moe_bank * shared_up,
                              const void * x, int32_t x_dtype, const int32_t * plan, int32_t n, int32_t topk, int32_t shared_tokens, float * act,
-                             void * workspace, size_t workspace_bytes, b2moe_stream stream, bool x_staged, long long live = -1) {
+                             void * workspace, size_t workspace_bytes, b2moe_stream stream, bool x_staged, long long live = -1,
+                             void * rows_buf = nullptr, size_t rows_buf_bytes = 0) {
     if (int32_t rc = check_bank(gate)) return rc;
     if (int32_t rc = check_bank(up)) return rc;
     if (int32_t rc = same_shape(gate, up, true)) return rc;
@@ -139,14 +141,15 @@ static int32_t expert_gateup(const b2moe_bank * gate, const b2moe_bank * up, con
     }
     if (!x || !plan || !act) return B2MOE_ERR_NULL;
     if (!aligned16(x) || !aligned16(act)) return B2MOE_ERR_ALIGN;
-    const int path = expert_path(gate->type, gate->cols, x_dtype, 2, gate->experts, live >= 0 ? live : (long long)n * topk);
+    const int path = expert_path(gate->type, gate->cols, x_dtype, gate->experts, live >= 0 ? live : (long long)n * topk);
     if (path != B2MOE_FAMILY_GENERIC) {
         const size_t need = b2moe_expert_workspace_bytes(gate->type, n, gate->cols, x_dtype);
         if (need && !workspace) return B2MOE_ERR_NULL;
         if (need && !aligned16(workspace)) return B2MOE_ERR_ALIGN;
         if (workspace_bytes < need) return B2MOE_ERR_WORKSPACE;
         if (path == B2MOE_FAMILY_GEMM)
-            return gemm_tc_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, workspace, as_stream(stream));
+            return gemm_tc_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, workspace, rows_buf, rows_buf_bytes,
+                                  as_stream(stream));
         const int ma = max_active_of(gate->experts, n, topk, shared_tokens);
         if (decode_kernel(gate->type, gate->cols, x_dtype) == DEC_4BIT)
             return dec4_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, workspace, ma, as_stream(stream), x_staged);
@@ -172,7 +175,7 @@ static int32_t expert_down(const b2moe_bank * down, const b2moe_bank * shared_do
     }
     if (!act || !plan || !y) return B2MOE_ERR_NULL;
     if (!aligned16(act) || !aligned16(y)) return B2MOE_ERR_ALIGN;
-    const int path = expert_path(down->type, down->cols, B2MOE_F32, 1, down->experts, live >= 0 ? live : (long long)n * topk);
+    const int path = expert_path(down->type, down->cols, B2MOE_F32, down->experts, live >= 0 ? live : (long long)n * topk);
     if (path != B2MOE_FAMILY_GENERIC) {
         const int rows_x = n * topk + shared_tokens;
         if (!workspace) return B2MOE_ERR_NULL;
@@ -261,7 +264,7 @@ static int32_t layer_forward(const b2moe_layer * L, const void * x, int32_t x_dt
     // decode-sized call on the 4-bit decode kernels: top-k, dispatch and the staging of x in one cluster launch
     bool x_staged = false;
     if (route_cluster_fits(L->experts, L->topk, n) && es_bytes >= b2moe_expert_workspace_bytes(L->gate.type, n, L->gate.cols, x_dtype) &&
-        expert_path(L->gate.type, L->gate.cols, x_dtype, 2, L->gate.experts, (long long)n * L->topk) == B2MOE_FAMILY_DECODE &&
+        expert_path(L->gate.type, L->gate.cols, x_dtype, L->gate.experts, (long long)n * L->topk) == B2MOE_FAMILY_DECODE &&
         decode_kernel(L->gate.type, L->gate.cols, x_dtype) == DEC_4BIT && valid_dtype(x_dtype)) {
         uint8_t * rows;
         float * inv;
@@ -274,8 +277,9 @@ static int32_t layer_forward(const b2moe_layer * L, const void * x, int32_t x_dt
         if (int32_t rc = b2moe_route_dispatch(L->gating, logits, ld, L->sel_bias, ids, weights, gated_shared ? shw : nullptr, L->experts, L->topk,
                                               L->norm, L->scale, n, 0, sh, plan, base + ws.scratch, ws.expert_scratch - ws.scratch, stream))
             return rc;
-    if (int32_t rc = expert_gateup(&L->gate, &L->up, &L->sh_gate, &L->sh_up, x, x_dtype, plan, n, L->topk, sh, act, es, es_bytes, stream, x_staged))
-        return rc;
+    // y is written by the down product: until then its rows hold the gate/up product's activation rows
+    if (int32_t rc = expert_gateup(&L->gate, &L->up, &L->sh_gate, &L->sh_up, x, x_dtype, plan, n, L->topk, sh, act, es, es_bytes, stream, x_staged, -1, y,
+                                   ws.scratch - ws.y)) return rc;
     if (int32_t rc = b2moe_expert_down(&L->down, &L->sh_down, act, plan, n, L->topk, sh, y, es, es_bytes, stream)) return rc;
     if (residual) return b2moe_combine_residual(y, nullptr, weights, gated_shared ? shw : nullptr, residual, n, L->topk, L->hidden, sh, out, out_dtype, stream);
     return b2moe_combine(y, nullptr, weights, gated_shared ? shw : nullptr, n, L->topk, L->hidden, sh, out, out_dtype, stream);

@@ -41,19 +41,42 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, uint32_t
     }
     return false;
 }
-// global -> shared bulk copy (both addresses and the size multiples of 16 bytes), completion on an mbarrier
-__device__ __forceinline__ void bulk_copy(uint32_t dst, const void * src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(bar) : "memory");
+// The same for a whole converged warp, all lanes on one barrier. The first try carries no time hint: on a phase that is already
+// complete it costs a tenth of the general loop above (measured 15 against 120 cycles), and a pipeline step has several.
+__device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
 }
-// 16-byte asynchronous copy of one thread; src_bytes = 0 writes zeros
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void * src, uint32_t src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(__cvta_generic_to_global(src)), "r"(src_bytes) : "memory");
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {
+    if (__all_sync(0xffffffffu, bar_try(bar, parity))) return true;
+    for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
+        uint32_t ok;
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(ok) : "r"(bar), "r"(parity), "r"(1000u) : "memory");
+        if (__all_sync(0xffffffffu, ok)) return true;
+    }
+    return false;
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+// TMA gather: rows y0..y3, 64 16-bit columns from x (a multiple of 8), of the mapped matrix (box of one row) -> four consecutive
+// 128-byte rows at dst, 128-byte swizzled, completion on an mbarrier
+__device__ __forceinline__ void tma_gather4(uint32_t dst, const void * map, int x, int y0, int y1, int y2, int y3, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y0), "r"(y1), "r"(y2), "r"(y3), "r"(bar) : "memory");
+}
+// TMA box of a mapped 3-D array from (x, y, z), completion on an mbarrier (what lies outside the array arrives as zeros)
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const void * map, int x, int y, int z, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
+}
+// one lane of a converged warp, the same every time
+__device__ __forceinline__ bool elect_one() {
+    uint32_t ok;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(ok));
+    return ok != 0;
+}
 
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
@@ -66,28 +89,22 @@ __device__ __forceinline__ void tmem_free(uint32_t base, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols) : "memory");
 }
 
-// shared-memory matrix descriptor: K-major, no swizzle. A core matrix is 8 rows x 16 bytes, stored as 128 contiguous
-// bytes; lbo = bytes between core matrices that are neighbours along K, sbo = between neighbours along the rows.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    return uint64_t((addr & 0x3FFFFu) >> 4) | (uint64_t(lbo >> 4) << 16) | (uint64_t(sbo >> 4) << 32) | (uint64_t(1) << 46);
-}
+// shared-memory matrix descriptor, the 128-byte swizzled K-major form: a row's 64 16-bit values are 128 contiguous bytes whose
+// 16-byte pieces are XORed with the row's low three bits; eight rows (1024 bytes, aligned so) form an atom, sbo = bytes between
+// atoms. Split in halves: the low half carries the address, the high half is a constant (sbo 1024, fixed bit 46, swizzle).
+constexpr uint32_t SW128_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t sw128_desc_lo(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | (1u << 16); }
 // instruction descriptor: fp32 accumulator, K-major A and B, M x N; ab_format: 0 = E4M3 (kind::f8f6f4) / fp16 (kind::f16),
 // 1 = bf16 (kind::f16)
 __device__ __forceinline__ uint32_t idesc(uint32_t m, uint32_t n, uint32_t ab_format) {
     return (1u << 4) | (ab_format << 7) | (ab_format << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
-// D (tensor memory, fp32) (+)= A (M x 16, 16-bit) * B (N x 16)^T; one thread issues
-__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t id, uint32_t accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-                 ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(id), "r"(accumulate) : "memory");
-}
-// the same with the descriptors given as (low, high) 32-bit halves: the issuing thread keeps the high halves and the base low
-// halves in registers and adds small constants per MMA, so that its instruction stream (one thread feeds the tensor core) stays short
-__device__ __forceinline__ void mma_f16_lohi(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t id,
-                                             uint32_t accumulate) {
-    asm volatile("{\n .reg .pred p;\n .reg .b64 da, db;\n mov.b64 da, {%1, %2};\n mov.b64 db, {%3, %4};\n setp.ne.b32 p, %6, 0;\n"
-                 " tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}"
-                 ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(id), "r"(accumulate) : "memory");
+// D (tensor memory, fp32) (+)= A (128 x 16, 16-bit, in tensor memory: row in lane, two values of K per column) * B (N x 16)^T;
+// one thread issues. The descriptor comes as (low, high) halves: the issuing thread adds small constants to the low half.
+__device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t id, uint32_t accumulate) {
+    asm volatile("{\n .reg .pred p;\n .reg .b64 db;\n mov.b64 db, {%2, %3};\n setp.ne.b32 p, %5, 0;\n"
+                 " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n}"
+                 ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(id), "r"(accumulate) : "memory");
 }
 // the barrier gets one arrival when every MMA this thread issued before has completed
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
@@ -100,6 +117,14 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
                    "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                  : "r"(taddr) : "memory");
 }
+// a warp's 16 rows x 32 columns from the registers of an m16n8-style fragment: register 4 i + 2 r + c of lane 4 g + t is column
+// 8 i + 2 t + c of row g + 8 r; taddr's lane is the first of the 16 (a multiple of 16 inside the warp's quarter)
+__device__ __forceinline__ void tmem_st_16x256b_x4(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+                   "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 }  // namespace tc
