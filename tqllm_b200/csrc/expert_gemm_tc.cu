@@ -27,7 +27,7 @@
 // Warps: 0 issues tcgen05.mma; 1 streams the raw blocks (256 columns of the item's eight row tiles per ring slot: one TMA box
 // of the down bank, one each of gate and up, running ahead across items); 2 (and 3 when it gathers) loads B; 4..11 epilogue (two
 // per TMEM lane quarter, 16-token groups in turn); 12..27 decode A (warp 12 + j: lane quarter j & 3, row tile (j >> 2) & 1 of
-// it, every second 256-column chunk). One barrier per step says that its products are done (a commit costs the issuing thread
+// it, unit j >> 3 of every 256-column chunk). One barrier per step says that its products are done (a commit costs the issuing thread
 // 60 cycles): it frees the unit's A stage and the step's B stage. Every wait is bounded; a wait that runs out sets the plan's
 // status word, and the block drains and leaves.
 //
@@ -49,7 +49,7 @@ namespace {
 using namespace tc;
 
 constexpr int G_KS = 64;                    // columns per step (four MMAs of K = 16); a unit is two steps
-constexpr int A_STAGES = 4, A_COLS = 64;    // stages of decoded A operand, a unit each (two chunks in all: one per decode warp of a row tile), and their columns
+constexpr int A_STAGES = 4, A_COLS = 64;    // stages of decoded A operand, a unit each, and their columns
 constexpr int STEP_RING = 2 * A_STAGES;     // barriers "the products of step g are done"
 constexpr int ACC_COLS = 128, A_COL0 = 2 * ACC_COLS;                // the two accumulators, then the A stages: all 512 columns
 constexpr int SPLIT_COLS = ACC_COLS / 2;    // items of up to this many tokens split their K over the halves of the accumulator
@@ -66,8 +66,8 @@ struct GemmArgs {
     int * plan;
     float * out;
     int rows, k, experts, topk, A;
-    int cap, b_stages, raw_slots;           // most tokens of an item; B stages; raw chunks in the ring
-    int b_pair;                             // 1: the B stages are filled and freed a unit at a time
+    int cap, cap_log2, b_stages, raw_slots; // most tokens of an item; B stages; raw chunks in the ring
+    int b_pair;                             // 1: the B stages are filled and freed a unit at a time, beside the A stage of the unit and through its barriers (b_stages = 2 A_STAGES)
     int slots;                              // 1: the activation rows lie in slot order; 0: in token (row) order, and are gathered
 };
 // x[i]: the activation rows, boxes of (i + 1) cap / 4 rows (a gathering launch: x[0], one row); w: banks (gate, up) or (down, -), then the shared expert's
@@ -177,9 +177,13 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
 
     D::init(dec_tab, threadIdx.x, G_THREADS);
     if (threadIdx.x == 0) {
-        for (int i = 0; i < RAW_SLOTS; ++i) { bar_init(raw_full + 8 * i, 1); bar_init(raw_empty + 8 * i, 8); }
-        for (int i = 0; i < A_STAGES; ++i) bar_init(a_full + 8 * i, 8);
+#pragma unroll 1
+        for (int i = 0; i < RAW_SLOTS; ++i) { bar_init(raw_full + 8 * i, 1); bar_init(raw_empty + 8 * i, DEC_WARPS); }
+#pragma unroll 1
+        for (int i = 0; i < A_STAGES; ++i) bar_init(a_full + 8 * i, p.b_pair ? 8 + (p.slots ? 1 : LOAD_WARPS) : 8);
+#pragma unroll 1
         for (int i = 0; i < STEP_RING; ++i) bar_init(done + 8 * i, 1);
+#pragma unroll 1
         for (int i = 0; i < MAX_B_STAGES; ++i) bar_init(b_full + 8 * i, p.slots ? 1 : LOAD_WARPS);
         for (int i = 0; i < 2; ++i) { bar_init(acc_full + 8 * i, 1); bar_init(acc_empty + 8 * i, EPI_WARPS); }
         bar_init(drain, 1);
@@ -190,6 +194,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
     if (warp == MMA_WARP) tmem_alloc(saddr(tmem_slot), 512);
     grid_wait();                                                      // the plan and the activation rows come from the launches before this one
     const int na = p.plan[PLAN_NACTIVE];
+#pragma unroll 1
     for (int i = threadIdx.x; i < na; i += G_THREADS) {
         const int e = active[i];
         info[i] = Info{0, e, counts[e], offsets[e]};
@@ -198,9 +203,10 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
     __syncthreads();
     fence_after();
     // an expert's tokens are spread evenly over the fewest tiles of at most `cap`
-    auto tiles_of = [&](int cnt) { return (cnt + p.cap - 1) / p.cap; };
+    auto tiles_of = [&](int cnt) { return (cnt + p.cap - 1) >> p.cap_log2; };
     if (warp == 0) {                                                  // items before active expert i
         int carry = 0;
+#pragma unroll 1
         for (int base = 0; base < na; base += 32) {
             const int i = base + lane;
             const int mine = i < na ? tiles_of(info[i].cnt) * row_blocks : 0;
@@ -235,7 +241,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
     };
     auto x_row = [&](int a) { return MODE == 0 ? (a < p.A ? a / p.topk : a - p.A) : a; };
     // the rows' boxes come in four sizes: the smallest that holds the item's tokens
-    auto b_class = [&](int nv) { return max(nv - 1, 0) / (p.cap / 4); };
+    auto b_class = [&](int nv) { return max(nv - 1, 0) >> (p.cap_log2 - 2); };
     auto give_up = [&]() { *abort_flag = 1; atomicExch(p.plan + PLAN_STATUS, 2); };
     int at = 0;
 
@@ -261,10 +267,12 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
             if (lane == 0) bar_arrive(tok_bar);
             return warp_wait(tok_bar, n & 1u);
         };
+        const uint32_t poll_ns = uint32_t(min(1000, 100 + 25 * nunits));       // an item takes 300 ns a unit or more: polling that is seldom leaves the issue slots to the decoders
         uint32_t next = 0, uses0 = 0, uses1 = 0, ic = 0;
         Item im{}, after{};
         bool ok = true;
         if (int(blockIdx.x) < n_items) { im = locate(blockIdx.x, at); fetch(im); ok = put(0); }
+#pragma unroll 1
         for (int it = blockIdx.x; it < n_items && ok && !*abort_flag; it += gridDim.x, ++ic, im = after) {
             const bool wide = im.nv > ACC_COLS, split = im.nv <= SPLIT_COLS;
             const uint32_t h = wide ? 0 : next;
@@ -278,13 +286,14 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
                 const float * ax = MODE == 0 && upper ? (shared ? p.saux1 : p.aux1) : (shared ? p.saux0 : p.aux0);
                 rs = ax[size_t(shared ? 0 : im.e) * row_tiles * 16 + row];
             }
-            if (!__all_sync(0xffffffffu, bar_wait(acc_full + 8 * h, (h ? uses1 : uses0) & 1u, 200))) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, bar_wait(acc_full + 8 * h, (h ? uses1 : uses0) & 1u, poll_ns))) { ok = false; break; }
             if (h) ++uses1; else ++uses0;
             fence_after();
             const uint32_t taddr = tmem + (uint32_t(32 * q) << 16) + h * ACC_COLS;
             const int4 * t = reinterpret_cast<const int4 *>(tok + (ic & 1u) * MAX_CAP);
             float * out = p.out + row;
             const bool in = row < p.rows;
+#pragma unroll 1
             for (int c = first; c < im.nv; c += 32) {
                 uint32_t v[16];
                 tmem_ld16(taddr + c, v);
@@ -337,49 +346,47 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
         }
         if (!ok && lane == 0) give_up();
     } else if (warp >= DEC_WARP0) {
-        // ---- A decoder: raw chunks (256 columns of one row tile) -> fp16 operand in tensor memory, a unit (128 columns) a stage ----
-        const int j = warp - DEC_WARP0, q = j & 3, m = (j >> 2) & 1, parity = j >> 3, r = 2 * q + m;      // r: row tile of the block
+        // ---- A decoder: raw chunks (256 columns of one row tile) -> fp16 operand in tensor memory, unit `part` of every chunk.
+        // (Whole chunks in turn instead: the products then came in bursts of two units of one group, and both sides waited.) ----
+        const int j = warp - DEC_WARP0, q = j & 3, m = (j >> 2) & 1, part = j >> 3, r = 2 * q + m;      // r: row tile of the block
         const uint8_t * my_raw = raw + size_t(MODE == 0 ? 4 * m + q : r) * CB;
         const uint32_t a_lane = tmem + (uint32_t(32 * q + 16 * m) << 16) + A_COL0;
-        uint32_t gu = 0, gc = 0, slot = 0, phase = 0;                  // unit, chunk; ring slot and phase of the next chunk
+        uint32_t gu = 0, slot = 0, phase = 0;                          // units before the chunk; ring slot and phase of the chunk
         bool ok = true;
+#pragma unroll 1
         for (int it = blockIdx.x; it < n_items && ok && !*abort_flag; it += gridDim.x) {
             const Item im = locate(it, at);
             const bool live = (MODE == 0 ? im.rb * 4 + q : im.rb * 8 + r) < row_tiles;      // a tile past the last row is not decoded
-            for (int c = 0; c < nchunks; ++c, ++gc) {
-                const int steps = min(4, ksteps - 4 * c), units = (steps + 1) >> 1;
-                if ((gc & 1u) == uint32_t(parity)) {
-                    const uint8_t * chunk = my_raw + slot * (8 * CB);
+#pragma unroll 1
+            for (int left = ksteps; left > 0; left -= 4) {             // steps of the item that are left
+                const uint8_t * chunk = my_raw + slot * (8 * CB);
+                if (!warp_wait(raw_full + 8 * slot, phase)) { ok = false; break; }
+                const int steps = left - 2 * part;                     // of this unit (more than two count as two)
+                if (steps > 0) {
+                    const uint32_t g = gu + part, sa = g % A_STAGES, a_addr = a_lane + sa * A_COLS;
                     typename D::Pre pre;
-                    if (!warp_wait(raw_full + 8 * slot, phase)) { ok = false; break; }
-                    if (live) pre = D::prep(chunk, lane);
-                    auto one_unit = [&](auto U) {
-                        constexpr int u = decltype(U)::value;
-                        if (u >= units || !ok) return;
-                        const uint32_t g = gu + u, sa = g % A_STAGES, a_addr = a_lane + sa * A_COLS;
-                        uint32_t f[16];
-                        if (live) D::template step<2 * u>(chunk, lane, dec_tab, pre, f);
-                        // the unit that used the stage before: its second step's products
-                        if (g >= A_STAGES && !warp_wait(done + 8 * ((2 * g + 1) % STEP_RING), ((g / A_STAGES) - 1) & 1u)) { ok = false; return; }
-                        if (live) {
-                            fence_after();
-                            tmem_st_16x256b_x4(a_addr, f);
-                            if (2 * u + 1 < steps) {
-                                D::template step<2 * u + 1>(chunk, lane, dec_tab, pre, f);
-                                tmem_st_16x256b_x4(a_addr + A_COLS / 2, f);
-                            }
-                            tmem_st_wait();
-                            fence_before();
+                    uint32_t f[16];
+                    if (live) {
+                        pre = D::prep(chunk, lane, part);
+                        D::template step<0>(chunk, lane, part, dec_tab, pre, f);
+                    }
+                    // the unit that used the stage before: its second step's products
+                    if (g >= A_STAGES && !warp_wait(done + 8 * (2 * sa + 1), ((g / A_STAGES) - 1) & 1u)) { ok = false; break; }
+                    if (live) {
+                        fence_after();
+                        tmem_st_16x256b_x4(a_addr, f);
+                        if (steps > 1) {
+                            D::template step<1>(chunk, lane, part, dec_tab, pre, f);
+                            tmem_st_16x256b_x4(a_addr + A_COLS / 2, f);
                         }
-                        __syncwarp();
-                        if (lane == 0) bar_arrive(a_full + 8 * sa);
-                    };
-                    one_unit(std::integral_constant<int, 0>{});
-                    one_unit(std::integral_constant<int, 1>{});
-                    if (!ok) break;
-                    if (lane == 0) bar_arrive(raw_empty + 8 * slot);               // every lane is done with the slot (the syncwarp above)
+                        tmem_st_wait();
+                        fence_before();
+                    }
+                    __syncwarp();
+                    if (lane == 0) bar_arrive(a_full + 8 * sa);
                 }
-                gu += units;
+                if (lane == 0) bar_arrive(raw_empty + 8 * slot);       // every lane is done with the slot (the syncwarp above, or nothing was read)
+                gu += left > 2 ? 2 : 1;
                 if (++slot == uint32_t(S)) { slot = 0; phase ^= 1u; }
             }
         }
@@ -389,6 +396,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
         const uint32_t b_lo0 = sw128_desc_lo(saddr(b_st)), b_step = uint32_t(p.cap * 128) >> 4;
         uint32_t gu = 0, sb = 0, pb = 0, next = 0, uses0 = 0, uses1 = 0;
         bool ok = true;
+#pragma unroll 1
         for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x) {
             const Item im = locate(it, at);
             const bool wide = im.nv > ACC_COLS;
@@ -400,41 +408,29 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
             if (wide || h == 0) { if (uses0 > 0) ok = warp_wait(acc_empty, (uses0 - 1) & 1u) && ok; ++uses0; }
             if (wide || h == 1) { if (uses1 > 0) ok = warp_wait(acc_empty + 8, (uses1 - 1) & 1u) && ok; ++uses1; }
             fence_after();
-            for (int u = 0; u < nunits && ok; ++u, ++gu) {
-                const uint32_t sa = gu % A_STAGES;
+#pragma unroll 1
+            for (int u = 0; u < nunits; ++u, ++gu) {
+                const uint32_t sa = gu % A_STAGES, a = tmem + A_COL0 + sa * A_COLS, b_lo = b_lo0 + sb * b_step, freed = done + 16 * sa;
+                const uint32_t acc = u > 0, acc1 = acc | (second == 0), last = u == nunits - 1 ? acc_full + 8 * h : 0;
+                const bool both = 2 * u + 1 < ksteps;                  // the second step of an odd K's last unit is empty: no products, but its barriers turn
                 if (!warp_wait(a_full + 8 * sa, (gu / A_STAGES) & 1u)) { ok = false; break; }
-                // the two steps of the unit; the second one of an odd K's last unit is empty: no products, but its barriers turn
-                const uint32_t a = tmem + A_COL0 + sa * A_COLS;
-                auto products = [&](int half, uint32_t b_lo) {
-                    if (2 * u + half >= ksteps) return;
-#pragma unroll
-                    for (uint32_t kk = 0; kk < 4; ++kk)
-                        mma_f16_ts(d + (kk & 1 ? second : 0), a + half * (A_COLS / 2) + 8 * kk, b_lo + 2 * kk, SW128_DESC_HI, id,
-                                   half > 0 || u > 0 || kk > (second ? 1 : 0));
-                };
-                if (!warp_wait(b_full + 8 * sb, pb)) { ok = false; break; }
-                fence_after();
-                uint32_t b_lo = b_lo0 + sb * b_step;
-                if (!p.b_pair) {
-                    if (elect_one()) {
-                        products(0, b_lo);
-                        mma_commit(done + 8 * (2 * sa));
-                    }
-                    __syncwarp();
+                if (p.b_pair) {                                        // a_full stands for the unit's rows too
+                    fence_after();
+                    if (both) mma_unit(d, d + second, a, b_lo, id, acc, acc1, freed + 8, last, b_lo + b_half);
+                    else mma_step(d, d + second, a, b_lo, id, acc, acc1, freed + 8, last);
+                    sb = (sb + 2) % MAX_B_STAGES;
+                } else {
+                    if (!warp_wait(b_full + 8 * sb, pb)) { ok = false; break; }
+                    fence_after();
+                    mma_step(d, d + second, a, b_lo, id, acc, acc1, freed, 0);
                     if (++sb == uint32_t(BS)) { sb = 0; pb ^= 1u; }
                     if (!warp_wait(b_full + 8 * sb, pb)) { ok = false; break; }
                     fence_after();
-                    b_lo = b_lo0 + sb * b_step;
+                    if (both) mma_step(d, d + second, a + A_COLS / 2, b_lo0 + sb * b_step, id, 1, 1, freed + 8, last);
+                    else if (elect_one()) { mma_commit(freed + 8); mma_commit(last); }
+                    __syncwarp();
+                    if (++sb == uint32_t(BS)) { sb = 0; pb ^= 1u; }
                 }
-                if (elect_one()) {
-                    if (p.b_pair) { products(0, b_lo); products(1, b_lo + b_half); }
-                    else products(1, b_lo);
-                    mma_commit(done + 8 * (2 * sa + 1));
-                    if (u == nunits - 1) mma_commit(acc_full + 8 * h);
-                }
-                __syncwarp();
-                sb += p.b_pair ? 2 : 1;
-                if (sb == uint32_t(BS)) { sb = 0; pb ^= 1u; }
             }
         }
         if (!ok && lane == 0) give_up();
@@ -447,10 +443,12 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
         constexpr uint32_t BYTES = 8 * CB;
         uint32_t issued = 0, slot = 0, phase = 1;                      // phase: of the empty barrier's wait (none in the first round)
         bool ok = true;
+#pragma unroll 1
         for (int it = blockIdx.x; it < n_items && ok && !*abort_flag; it += gridDim.x) {
             const Item im = locate(it, at);
             const CUtensorMap * map = maps.w + (im.e == p.experts ? 2 : 0);
             const int rt = (im.e == p.experts ? 0 : im.e * row_tiles) + im.rb * ITEM_TILES;        // rows past the matrix: the next expert's, never used
+#pragma unroll 1
             for (int c = 0; c < nchunks; ++c) {
                 if (issued >= uint32_t(S) && !warp_wait(raw_empty + 8 * slot, phase)) { ok = false; break; }
                 if (elect_one()) {
@@ -466,6 +464,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
         }
         if (!ok && lane == 0) give_up();
         // before leaving, every copy must have landed (after a clean run these waits return at once)
+#pragma unroll 1
         for (uint32_t i = issued > uint32_t(S) ? issued - S : 0; i < issued; ++i) bar_wait(raw_full + 8 * (i % S), (i / S) & 1u);
     } else {
         // ---- B loader: warp 2 brings a step's (or a unit's) rows with one box; a gathering launch: lane l of warp w brings rows
@@ -473,6 +472,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
         const int lw = warp - LOAD_WARP0, n0 = 4 * (2 * lane + lw), group = p.b_pair ? 2 : 1;      // steps that share a barrier
         uint32_t gk = 0, sb = 0;
         bool ok = true;
+#pragma unroll 1
         for (int it = blockIdx.x; it < n_items && ok && !*abort_flag && (lw == 0 || !p.slots); it += gridDim.x) {
             const Item im = locate(it, at);
             int row[4] = {0, 0, 0, 0};
@@ -482,10 +482,11 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
             }
             const int cls = b_class(im.nv), quads = (im.nv + 3) >> 2, mine = (quads + 1 - lw) >> 1;
             const uint32_t box_bytes = uint32_t((cls + 1) * (p.cap / 4) * group) * 128u;
+#pragma unroll 1
             for (int ks = 0; ks < 2 * nunits; ks += group, gk += group) {
                 const uint32_t freed = gk + group - 1 - uint32_t(BS);  // the (last) step that used the stage before
                 if (gk >= uint32_t(BS) && !warp_wait(done + 8 * (freed % STEP_RING), (freed / STEP_RING) & 1u)) { ok = false; break; }
-                const uint32_t bar = b_full + 8 * sb, dst = saddr(b_st) + sb * uint32_t(p.cap * 128);
+                const uint32_t bar = p.b_pair ? a_full + 4 * sb : b_full + 8 * sb, dst = saddr(b_st) + sb * uint32_t(p.cap * 128);
                 if (p.slots) {
                     if (elect_one()) {
                         bar_expect_tx(bar, box_bytes);
@@ -497,6 +498,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
                     if (lane == 0) bar_expect_tx(bar, uint32_t(max(real, 0) * mine) * 512u);
                     __syncwarp();
                     if (n0 < im.nv)
+#pragma unroll 1
                         for (int i = 0; i < real; ++i)
                             tma_gather4(dst + i * uint32_t(p.cap * 128) + n0 * 128, maps.x, (ks + i) * G_KS, row[0], row[1], row[2], row[3], bar);
                 }
@@ -506,7 +508,9 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
         }
         if (!ok && lane == 0) give_up();
         // before leaving, every copy into the stages must have landed (after a clean run these waits return at once)
-        for (uint32_t g = gk > uint32_t(BS) ? gk - BS : 0; g < gk; g += group) bar_wait(b_full + 8 * (g % BS), (g / BS) & 1u);
+        // (b_pair: the products that read the last stages have been waited for by the MMA warp, or the unit's barrier is waited for here)
+#pragma unroll 1
+        for (uint32_t g = gk > uint32_t(BS) ? gk - BS : 0; g < gk; g += group) bar_wait(p.b_pair ? a_full + 4 * (g % BS) : b_full + 8 * (g % BS), (g / BS) & 1u);
     }
     grid_release();
     fence_before();
@@ -525,13 +529,13 @@ constexpr size_t GEMM_SMEM_LIMIT = 232448 - 1024;
 // ring holds at least three chunks
 int g_item_tokens = 0;                      // test hook: 256 = 256-token items whatever the batch
 template <uint32_t T> bool gemm_fit(int experts, int cap_wanted, GemmArgs & a) {
-    constexpr int opts[4][3] = {{256, 4, 3}, {128, 8, 3}, {64, 8, 3}, {64, 4, 2}};      // tokens per item, B stages, fewest raw slots
+    constexpr int opts[4][3] = {{256, 4, 3}, {128, 8, 3}, {64, 8, 3}, {64, 8, 2}};      // tokens per item, B stages, fewest raw slots
     for (const auto & o : opts) {
         if (o[0] > cap_wanted) continue;
         for (int s = RAW_SLOTS; s >= o[2]; --s)
             if (gemm_smem<T>(experts, o[0], o[1], s) <= GEMM_SMEM_LIMIT) {
-                a.cap = o[0]; a.b_stages = o[1]; a.raw_slots = s;
-                a.b_pair = o[0] < 256;
+                a.cap = o[0]; a.cap_log2 = o[0] == 256 ? 8 : o[0] == 128 ? 7 : 6; a.b_stages = o[1]; a.raw_slots = s;
+                a.b_pair = o[1] == 2 * A_STAGES;
                 return true;
             }
     }

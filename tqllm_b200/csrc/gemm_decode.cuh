@@ -1,4 +1,6 @@
 // Weight decoders of the tensor-core grouped GEMM: one 64-column step of one 16-row bank tile -> fp16 A operand in registers.
+// A 256-column chunk has two units of two steps; a warp decodes unit u (0 or 1) of every chunk: prep once per chunk, then
+// step<0>, step<1>.
 //
 // A warp owns a row tile; lane L = 4 g + t holds, in the bank's lane-major layout, the code words of rows g and g + 8
 // (formats.cuh). Every code word (or pair of IQ3_S grid entries) decodes to eight fp16 values, so a step leaves sixteen
@@ -64,47 +66,43 @@ template <> struct Dec<T_Q4_K> {
     __device__ __forceinline__ static uint32_t two(uint32_t nib, __half2 S, __half2 NS, __half2 MH, __half2 ML, __half2 D) {
         return h2_bits(__hadd2(__hfma2(__hfma2(bits_h2(nib | 0x64006400u), S, NS), D, MH), ML));
     }
-    // Once per 256-column chunk: lane t of a row's four lanes turns the header into S and the two terms of -dmin m of
-    // sub-blocks 2 t and 2 t + 1 of its two rows; a step fetches the sub-blocks it needs from lane J with shuffles.
-    // SM[r][b] = (S, MH), ML[r] = (ML of sub-block 2 t, of 2 t + 1), D = d of row g, d of row g + 8.
-    struct Pre { uint32_t SM[2][2], ML[2], D; };
-    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane) {
+    // Once per chunk: lane t of a row's four lanes turns the headers of its two rows into the constants of the unit's sub-block t;
+    // a step fetches its two sub-blocks from lanes 2 js and 2 js + 1. SM[r] = (S, MH), ML = the rows' ML, D = the rows' d.
+    struct Pre { uint32_t SM[2], ML, D; };
+    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, int u) {
         const int g = lane >> 2, t = lane & 3;
         Pre p;
         uint32_t d[2];
+        float ml[2];
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             const uint4 h = *reinterpret_cast<const uint4 *>(chunk + 2048 + 16 * (g + 8 * r));    // d, dmin | s[12]
             const float dmin = __half2float(__ushort_as_half((unsigned short)(h.x >> 16)));
             d[r] = h.x & 0xffffu;
-            const uint32_t sc4 = t < 2 ? h.y & 0x3F3F3F3Fu : (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u);         // scales of sub-blocks 0..3 or 4..7
-            const uint32_t mn4 = t < 2 ? h.z & 0x3F3F3F3Fu : ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u);
-            const uint32_t sc2 = sc4 >> (16 * (t & 1)), mn2 = mn4 >> (16 * (t & 1));
-            float ml[2];
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                const float sc = float((sc2 >> (8 * b)) & 255u), m = -(dmin * float((mn2 >> (8 * b)) & 255u));         // exact in fp32 (11 x 6 bits)
-                const __half mh = __float2half_rn(m);
-                p.SM[r][b] = h2_bits(__halves2half2(__float2half_rn(b ? sc * 0.0625f : sc), mh));
-                ml[b] = m - __half2float(mh);
-            }
-            p.ML[r] = pack_h2(ml[0], ml[1]);
+            const uint32_t sc4 = u == 0 ? h.y & 0x3F3F3F3Fu : (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u);         // scales of sub-blocks 0..3 or 4..7
+            const uint32_t mn4 = u == 0 ? h.z & 0x3F3F3F3Fu : ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u);
+            const float sc = float((sc4 >> (8 * t)) & 255u), m = -(dmin * float((mn4 >> (8 * t)) & 255u));              // exact in fp32 (11 x 6 bits)
+            const __half mh = __float2half_rn(m);
+            p.SM[r] = h2_bits(__halves2half2(__float2half_rn(t & 1 ? sc * 0.0625f : sc), mh));
+            ml[r] = m - __half2float(mh);
         }
+        p.ML = pack_h2(ml[0], ml[1]);
         p.D = d[0] | (d[1] << 16);
         return p;
     }
-    template <int J> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const void *, const Pre & p, uint32_t (&f)[16]) {
-        const int src = (lane & ~3) | J;
-        const uint4 w4 = plane(chunk, J, lane);
+    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void *, const Pre & p, uint32_t (&f)[16]) {
+        const int s0 = (lane & ~3) | (2 * JS), s1 = s0 + 1;
+        const uint4 w4 = plane(chunk, 2 * u + JS, lane);
         const uint32_t w[2][2] = {{w4.x, w4.y}, {w4.z, w4.w}};
         const __half2 neg1024 = __float2half2_rn(-1024.f);
+        const __half2 ml0 = bits_h2(__shfl_sync(0xffffffffu, p.ML, s0)), ml1 = bits_h2(__shfl_sync(0xffffffffu, p.ML, s1));
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-            const __half2 a0 = bits_h2(__shfl_sync(0xffffffffu, p.SM[r][0], src)), a1 = bits_h2(__shfl_sync(0xffffffffu, p.SM[r][1], src));
-            const __half2 ml = bits_h2(__shfl_sync(0xffffffffu, p.ML[r], src));
+            const __half2 a0 = bits_h2(__shfl_sync(0xffffffffu, p.SM[r], s0)), a1 = bits_h2(__shfl_sync(0xffffffffu, p.SM[r], s1));
             const __half2 D = r ? __high2half2(bits_h2(p.D)) : __low2half2(bits_h2(p.D));
             const __half2 S0 = __low2half2(a0), S1 = __low2half2(a1), N0 = __hmul2(S0, neg1024), N1 = __hmul2(S1, neg1024);
-            const __half2 MH0 = __high2half2(a0), MH1 = __high2half2(a1), ML0 = __low2half2(ml), ML1 = __high2half2(ml);
+            const __half2 MH0 = __high2half2(a0), MH1 = __high2half2(a1);
+            const __half2 ML0 = r ? __high2half2(ml0) : __low2half2(ml0), ML1 = r ? __high2half2(ml1) : __low2half2(ml1);
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
                 const uint32_t v = w[r][b], v8 = v >> 8;
@@ -130,7 +128,7 @@ template <> struct Dec<T_IQ3S4> {
         return bits_h2((s & 0x03C003C0u) | 0x3C003C00u);
     }
     struct Pre { uint32_t sc[2], D; };                                 // the rows' eight 4-bit scales; d of row g, d of row g + 8
-    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane) {
+    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, int) {
         const int g = lane >> 2;
         Pre p;
 #pragma unroll
@@ -139,14 +137,15 @@ template <> struct Dec<T_IQ3S4> {
               (uint32_t(*reinterpret_cast<const unsigned short *>(chunk + 2112 + 2 * (g + 8))) << 16);
         return p;
     }
-    template <int J> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const void *, const Pre & p, uint32_t (&f)[16]) {
-        const uint4 w4 = plane(chunk, J, lane);
+    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void *, const Pre & p, uint32_t (&f)[16]) {
+        const int j = 2 * u + JS;
+        const uint4 w4 = plane(chunk, j, lane);
         const uint32_t w[2][2] = {{w4.x, w4.y}, {w4.z, w4.w}};
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             const __half2 D = r ? __high2half2(bits_h2(p.D)) : __low2half2(bits_h2(p.D));
             // the two scale nibbles of the step side by side under the exponent of 1: (1 + s / 16, 1 + s' / 16), then 1 + 2 s exactly
-            const uint32_t sb = p.sc[r] >> (8 * J);
+            const uint32_t sb = p.sc[r] >> (8 * j);
             const __half2 s1 = __hfma2(bits_h2(((sb << 6) & 0x03C0u) | ((sb << 18) & 0x03C00000u) | 0x3C003C00u), __float2half2_rn(32.f), __float2half2_rn(-31.f));
             const __half2 SC = __hmul2(s1, __float2half2_rn(32.f)), CC = __hmul2(s1, __float2half2_rn(-47.f));
             const __half2 SC1 = __low2half2(SC), C1 = __low2half2(CC), SC2 = __high2half2(SC), C2 = __high2half2(CC);
@@ -161,76 +160,78 @@ template <> struct Dec<T_IQ3S4> {
 };
 
 // ---------------------------------------------------------------------------------------------------------------
-// The eight 4-bit codes of a word -> their kvalues (exact) times `scale`, in nibble order. The 16-entry codebook sits in four
-// registers as bytes kvalue + 128: a byte permute looks four codes up among entries 0..7 and among entries 8..15 (the three
-// low bits of each nibble select), a third one takes the right byte of each by the nibble's top bit; a byte under 0x64 is
-// the fp16 1024 + byte. 23 instructions for eight weights, none of them in the load/store unit: a 256-entry half2 table in
-// shared memory takes 16, but its reads (two bank wavefronts each) cost more there than the tensor core's own operand reads.
-struct Iq4Table { uint32_t t[4]; };
-__device__ __forceinline__ constexpr uint32_t iq4_table_word(int i) {
-    constexpr int8_t kv[16] = B2_KVALUES_IQ4NL_INIT;
-    uint32_t v = 0;
-    for (int j = 0; j < 4; ++j) v |= uint32_t(int(kv[4 * i + j]) + 128) << (8 * j);
-    return v;
+// The eight 4-bit codes of a word -> their kvalues (exact) times `scale`, in nibble order, through a 256-entry table byte ->
+// half2 in shared memory with a copy per lane (no bank conflicts: entry b of lane l at word 32 b + l). Per code byte: a byte
+// permute extracts it, a multiply-add makes the address, one load, one product by the scale. The integer pipe takes one of
+// the four: it is the one these formats fill (shift, mask and add take three: c5, 24 tokens, gate/up 332 us at 0.69 of that
+// pipe; byte permutes over a codebook in registers 23 instructions a word, fifteen of them there: 370 us).
+constexpr int LUT_BYTES = 256 * 32 * 4;
+__device__ inline void build_lut(void * tab, int tid, int nthreads) {
+    uint32_t * lut = static_cast<uint32_t *>(tab);
+    for (int i = tid; i < 256 * 32; i += nthreads) lut[i] = pack_h2(float(c_kvalues_iq4nl[(i >> 5) & 15]), float(c_kvalues_iq4nl[i >> 9]));
 }
-__device__ __forceinline__ Iq4Table iq4_table() {
-    constexpr uint32_t a = iq4_table_word(0), b = iq4_table_word(1), c = iq4_table_word(2), d = iq4_table_word(3);
-    return Iq4Table{{a, b, c, d}};
+// the lane's copy: its shared-memory address and the 128 bytes between entries, opaque so that the address stays a multiply-add
+struct Lut { uint32_t base, stride; };
+__device__ __forceinline__ Lut lut_of(const void * tab, int lane) {
+    Lut l{uint32_t(__cvta_generic_to_shared(tab)) + 4u * uint32_t(lane), 0};
+    asm volatile("mov.b32 %0, 128;" : "=r"(l.stride));
+    return l;
 }
-__device__ __forceinline__ uint4 iq4_word(const Iq4Table & k, uint32_t w, __half2 scale) {
-    const uint32_t lo = w & 0x77777777u, top = ((w >> 1) & 0x44444444u) | 0x32103210u;
-    const uint32_t r0 = __byte_perm(__byte_perm(k.t[0], k.t[1], lo), __byte_perm(k.t[2], k.t[3], lo), top);
-    const uint32_t lo1 = lo >> 16;
-    const uint32_t r1 = __byte_perm(__byte_perm(k.t[0], k.t[1], lo1), __byte_perm(k.t[2], k.t[3], lo1), top >> 16);
-    const __half2 bias = __float2half2_rn(-1152.f);                    // 1024 + 128
-    auto val = [&](uint32_t r, uint32_t sel) { return h2_bits(__hmul2(__hadd2(bits_h2(__byte_perm(r, 0x64646464u, sel)), bias), scale)); };
-    return make_uint4(val(r0, 0x4140u), val(r0, 0x4342u), val(r1, 0x4140u), val(r1, 0x4342u));
+__device__ __forceinline__ uint4 lut_word(const Lut & l, uint32_t w, __half2 scale) {
+    auto val = [&](uint32_t sel) {
+        uint32_t b, at, v;
+        asm("prmt.b32 %0, %1, 0, %2;" : "=r"(b) : "r"(w), "r"(sel));
+        asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(at) : "r"(b), "r"(l.stride), "r"(l.base));
+        asm("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(at));
+        return h2_bits(__hmul2(bits_h2(v), scale));
+    };
+    return make_uint4(val(0x4440u), val(0x4441u), val(0x4442u), val(0x4443u));
 }
 
 template <> struct Dec<T_IQ4_XS> {
-    static constexpr int TAB_BYTES = 0;
-    __device__ static void init(void *, int, int) {}
-    // once per chunk: lane t holds fp16(d (ls - 32)) of sub-blocks 2 t and 2 t + 1 of its two rows
-    struct Pre { uint32_t dl[2]; };
-    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane) {
-        const int g = lane >> 2, t = lane & 3;
-        Pre p;
+    static constexpr int TAB_BYTES = LUT_BYTES;
+    __device__ static void init(void * tab, int tid, int n) { build_lut(tab, tid, n); }
+    // once per chunk: lane t holds fp16(d (ls - 32)) of the unit's sub-block t, for its two rows
+    struct Pre { uint32_t dl; };
+    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, int u) {
+        const int g = lane >> 2, ib = 4 * u + (lane & 3);
+        float dl[2];
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             const uint2 h = *reinterpret_cast<const uint2 *>(chunk + 2048 + 8 * (g + 8 * r));       // d, scales_h | scales_l[4]
             const float d = __half2float(__ushort_as_half((unsigned short)(h.x & 0xffffu)));
-            const uint32_t sh = (h.x >> 16) >> (4 * t), sl = h.y >> (8 * t);
-            const int l0 = int(sl & 15u) | int((sh & 3u) << 4), l1 = int((sl >> 4) & 15u) | int(((sh >> 2) & 3u) << 4);
-            p.dl[r] = pack_h2(d * float(l0 - 32), d * float(l1 - 32));
+            const int ls = int((h.y >> (4 * ib)) & 15u) | int(((h.x >> (16 + 2 * ib)) & 3u) << 4);
+            dl[r] = d * float(ls - 32);
         }
-        return p;
+        return Pre{pack_h2(dl[0], dl[1])};
     }
-    template <int J> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const void *, const Pre & p, uint32_t (&f)[16]) {
-        const int src = (lane & ~3) | J;
-        const uint4 w4 = plane(chunk, J, lane);
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const __half2 d = bits_h2(__shfl_sync(0xffffffffu, p.dl[r], src));
-            put(f, r, 0, iq4_word(iq4_table(), r ? w4.z : w4.x, __low2half2(d)));
-            put(f, r, 1, iq4_word(iq4_table(), r ? w4.w : w4.y, __high2half2(d)));
-        }
+    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void * tab, const Pre & p, uint32_t (&f)[16]) {
+        const Lut lut = lut_of(tab, lane);
+        const uint4 w4 = plane(chunk, 2 * u + JS, lane);
+        const int src = (lane & ~3) | (2 * JS);
+        const __half2 d0 = bits_h2(__shfl_sync(0xffffffffu, p.dl, src)), d1 = bits_h2(__shfl_sync(0xffffffffu, p.dl, src + 1));
+        put(f, 0, 0, lut_word(lut, w4.x, __low2half2(d0)));
+        put(f, 0, 1, lut_word(lut, w4.y, __low2half2(d1)));
+        put(f, 1, 0, lut_word(lut, w4.z, __high2half2(d0)));
+        put(f, 1, 1, lut_word(lut, w4.w, __high2half2(d1)));
     }
 };
 
 template <> struct Dec<T_IQ4_NL> {
     struct Pre {};
-    __device__ __forceinline__ static Pre prep(const uint8_t *, int) { return Pre{}; }
-    static constexpr int TAB_BYTES = 0;
-    __device__ static void init(void *, int, int) {}
-    template <int J> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const void *, const Pre &, uint32_t (&f)[16]) {
+    __device__ __forceinline__ static Pre prep(const uint8_t *, int, int) { return Pre{}; }
+    static constexpr int TAB_BYTES = LUT_BYTES;
+    __device__ static void init(void * tab, int tid, int n) { build_lut(tab, tid, n); }
+    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void * tab, const Pre &, uint32_t (&f)[16]) {
+        const Lut lut = lut_of(tab, lane);
         const int g = lane >> 2;
 #pragma unroll
         for (int b = 0; b < 2; ++b) {                                   // the step's two 32-column tiles: the rows' code words and fp16 scales
-            const uint8_t * tile = chunk + (2 * J + b) * Fmt<T_IQ4_NL>::TILE;
+            const uint8_t * tile = chunk + (4 * u + 2 * JS + b) * Fmt<T_IQ4_NL>::TILE;
             const uint2 w = *reinterpret_cast<const uint2 *>(tile + 8 * lane);
             const __half d0 = *reinterpret_cast<const __half *>(tile + 256 + 2 * g), d1 = *reinterpret_cast<const __half *>(tile + 256 + 2 * (g + 8));
-            put(f, 0, b, iq4_word(iq4_table(), w.x, __half2half2(d0)));
-            put(f, 1, b, iq4_word(iq4_table(), w.y, __half2half2(d1)));
+            put(f, 0, b, lut_word(lut, w.x, __half2half2(d0)));
+            put(f, 1, b, lut_word(lut, w.y, __half2half2(d1)));
         }
     }
 };
@@ -238,7 +239,7 @@ template <> struct Dec<T_IQ4_NL> {
 // ---------------------------------------------------------------------------------------------------------------
 template <> struct Dec<T_NVFP4G> {
     struct Pre {};
-    __device__ __forceinline__ static Pre prep(const uint8_t *, int) { return Pre{}; }
+    __device__ __forceinline__ static Pre prep(const uint8_t *, int, int) { return Pre{}; }
     static constexpr int TAB_BYTES = 0;
     __device__ static void init(void *, int, int) {}
     // the eight e2m1 codes of a word -> eight fp16 values (the hardware conversion, two codes per instruction: low nibble
@@ -250,10 +251,10 @@ template <> struct Dec<T_NVFP4G> {
         return make_uint4(h2_bits(__hmul2(bits_h2(v0), scale)), h2_bits(__hmul2(bits_h2(v1), scale)), h2_bits(__hmul2(bits_h2(v2), scale)),
                           h2_bits(__hmul2(bits_h2(v3), scale)));
     }
-    template <int J> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const void *, const Pre &, uint32_t (&f)[16]) {
+    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void *, const Pre &, uint32_t (&f)[16]) {
         const int g = lane >> 2, t = lane & 3;
-        const uint8_t * tile = chunk + (J >> 1) * Fmt<T_NVFP4G>::TILE;
-        constexpr int P = J & 1;                                         // plane = sub-blocks 2 P, 2 P + 1 of the 128-column tile
+        const uint8_t * tile = chunk + u * Fmt<T_NVFP4G>::TILE;
+        constexpr int P = JS;                                            // the unit is one 128-column tile; plane = sub-blocks 2 P, 2 P + 1 of the 128-column tile
         const uint4 w4 = plane(tile, P, lane);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
@@ -270,7 +271,7 @@ template <> struct Dec<T_NVFP4G> {
 // ---------------------------------------------------------------------------------------------------------------
 template <> struct Dec<T_IQ3_S> {
     struct Pre {};
-    __device__ __forceinline__ static Pre prep(const uint8_t *, int) { return Pre{}; }
+    __device__ __forceinline__ static Pre prep(const uint8_t *, int, int) { return Pre{}; }
     // table: grid entry -> its four odd magnitudes as fp16 (8 bytes)
     static constexpr int TAB_BYTES = 512 * 8;
     __device__ static void init(void * tab, int tid, int n) {
@@ -280,7 +281,11 @@ template <> struct Dec<T_IQ3_S> {
             t2[i] = make_uint2(pack_h2(float(m & 255u), float((m >> 8) & 255u)), pack_h2(float((m >> 16) & 255u), float(m >> 24)));
         }
     }
-    template <int J> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const void * tab, const Pre &, uint32_t (&f)[16]) {
+    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void * tab, const Pre &, uint32_t (&f)[16]) {
+        if (u == 0) bits_step<JS>(chunk, lane, tab, f);                // the bit positions have to be constants
+        else bits_step<2 + JS>(chunk, lane, tab, f);
+    }
+    template <int J> __device__ __forceinline__ static void bits_step(const uint8_t * chunk, int lane, const void * tab, uint32_t (&f)[16]) {
         const int g = lane >> 2;
         const uint2 * mags = static_cast<const uint2 *>(tab);
         uint32_t w[13];
