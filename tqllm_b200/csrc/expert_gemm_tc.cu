@@ -253,6 +253,8 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
         // every product with a short K: c3 down, 80 tokens x K = 512: 412 us, 255 with the table) ----
         const int q = warp & 3, tid = threadIdx.x - EPI_WARP0 * 32, first = 16 * ((warp - EPI_WARP0) >> 2);
         const bool upper = lane >= 16;
+        constexpr bool ROW_SCALE = T == T_NVFP4G;
+        const uint32_t row_bytes = uint32_t(p.rows) * 4u;
         int2 mine;
         auto fetch = [&](const Item & im) {                            // this thread's token of the item
             mine = make_int2(-1, 0);
@@ -267,7 +269,6 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
             if (lane == 0) bar_arrive(tok_bar);
             return warp_wait(tok_bar, n & 1u);
         };
-        const uint32_t poll_ns = uint32_t(min(1000, 100 + 25 * nunits));       // an item takes 300 ns a unit or more: polling that is seldom leaves the issue slots to the decoders
         uint32_t next = 0, uses0 = 0, uses1 = 0, ic = 0;
         Item im{}, after{};
         bool ok = true;
@@ -280,19 +281,20 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
             if (it + int(gridDim.x) < n_items) { after = locate(it + gridDim.x, at); fetch(after); }
             // this lane's weight row: row tiles of a quarter are (gate, up) of the same 16 output rows, or two tiles of the down matrix
             const int row = MODE == 0 ? 16 * (im.rb * 4 + q) + (lane & 15) : 128 * im.rb + 32 * q + lane;
-            float rs = 1.f;                                            // fp32 row scale of the bank (NVFP4G)
-            if (p.aux0 && row < p.rows) {
+            [[maybe_unused]] float rs = 1.f;                           // fp32 row scale of the bank
+            if (ROW_SCALE && row < p.rows) {
                 const bool shared = im.e == p.experts;
                 const float * ax = MODE == 0 && upper ? (shared ? p.saux1 : p.aux1) : (shared ? p.saux0 : p.aux0);
                 rs = ax[size_t(shared ? 0 : im.e) * row_tiles * 16 + row];
             }
-            if (!__all_sync(0xffffffffu, bar_wait(acc_full + 8 * h, (h ? uses1 : uses0) & 1u, poll_ns))) { ok = false; break; }
+            if (!warp_wait(acc_full + 8 * h, (h ? uses1 : uses0) & 1u)) { ok = false; break; }
             if (h) ++uses1; else ++uses0;
             fence_after();
             const uint32_t taddr = tmem + (uint32_t(32 * q) << 16) + h * ACC_COLS;
             const int4 * t = reinterpret_cast<const int4 *>(tok + (ic & 1u) * MAX_CAP);
-            float * out = p.out + row;
+            char * const out = reinterpret_cast<char *>(p.out + row);
             const bool in = row < p.rows;
+            auto store = [&](int a, float y) { if (in && a >= 0) *reinterpret_cast<float *>(out + uint64_t(uint32_t(a)) * row_bytes) = y; };
 #pragma unroll 1
             for (int c = first; c < im.nv; c += 32) {
                 uint32_t v[16];
@@ -316,22 +318,21 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
                         float res[4];
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
-                            const float v0 = __uint_as_float(v[j0 + 2 * i]) * rs, v1 = __uint_as_float(v[j0 + 2 * i + 1]) * rs;
+                            float v0 = __uint_as_float(v[j0 + 2 * i]), v1 = __uint_as_float(v[j0 + 2 * i + 1]);
+                            if (ROW_SCALE) { v0 *= rs; v1 *= rs; }
                             const float other = __shfl_xor_sync(0xffffffffu, upper ? v0 : v1, 16);
                             const float is = __int_as_float(upper ? two[i].w : two[i].y);
                             const float gv = (upper ? other : v0) * is, uv = (upper ? v1 : other) * is;
                             res[i] = __fdividef(gv, 1.f + __expf(-gv)) * uv;      // fast exp and divide: relative error about 2^-21
                         }
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const int a = upper ? two[i].z : two[i].x;
-                            if (in && a >= 0) out[size_t(a) * p.rows] = res[i];
-                        }
+                        for (int i = 0; i < 4; ++i) store(upper ? two[i].z : two[i].x, res[i]);
                     } else {
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
-                            if (in && two[i].x >= 0) out[size_t(two[i].x) * p.rows] = __uint_as_float(v[j0 + 2 * i]) * (__int_as_float(two[i].y) * rs);
-                            if (in && two[i].z >= 0) out[size_t(two[i].z) * p.rows] = __uint_as_float(v[j0 + 2 * i + 1]) * (__int_as_float(two[i].w) * rs);
+                            const float is0 = __int_as_float(two[i].y), is1 = __int_as_float(two[i].w);
+                            store(two[i].x, __uint_as_float(v[j0 + 2 * i]) * (ROW_SCALE ? is0 * rs : is0));
+                            store(two[i].z, __uint_as_float(v[j0 + 2 * i + 1]) * (ROW_SCALE ? is1 * rs : is1));
                         }
                     }
                 }

@@ -6,7 +6,7 @@
 namespace b2 {
 namespace tc {
 
-constexpr uint32_t WAIT_LIMIT = 1u << 18;   // tries of about a microsecond each before a wait gives up
+constexpr uint32_t WAIT_LIMIT = 1u << 18;   // tries of four microseconds before a wait gives up: about a second
 
 __device__ __forceinline__ uint32_t saddr(const void * p) { return uint32_t(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) {
@@ -19,46 +19,25 @@ __device__ __forceinline__ void bar_arrive(uint32_t bar) {
 __device__ __forceinline__ void bar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// One phase of a barrier; false = gave up after WAIT_LIMIT tries.
-// backoff_ns = 0: the hardware's suspending try_wait (fast wake-up, for the waits on the critical path). The compiler
-// expands it into a polling loop, which takes issue slots and the integer pipe from the warps that work; so a wait
-// that is expected to last (an epilogue waiting for a whole item, a loader waiting for a free stage) passes a back-off
-// and polls with test_wait + nanosleep instead.
-__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, uint32_t backoff_ns = 0) {
-    const uint32_t limit = (backoff_ns && backoff_ns < 500) ? WAIT_LIMIT * 8 : WAIT_LIMIT;   // about a quarter of a second either way
-#pragma unroll 1
-    for (uint32_t i = 0; i < limit; ++i) {
-        uint32_t ok;
-        if (backoff_ns) {
-            asm volatile("{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-            if (ok) return true;
-            __nanosleep(backoff_ns);
-        } else {
-            asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}"
-                         : "=r"(ok) : "r"(bar), "r"(parity), "r"(1000u) : "memory");
-            if (ok) return true;
-        }
-    }
-    return false;
-}
-// The same for a whole converged warp, all lanes on one barrier. The first try carries no time hint: on a phase that is already
-// complete it costs a tenth of the general loop above (measured 15 against 120 cycles), and a pipeline step has several.
+// One try at a phase of a barrier: the hardware suspends the thread until the phase completes, four microseconds at most
 __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {
-    if (__all_sync(0xffffffffu, bar_try(bar, parity))) return true;
+// One phase of a barrier, one thread; false = gave up after WAIT_LIMIT tries
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
 #pragma unroll 1
-    for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
-        uint32_t ok;
-        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}"
-                     : "=r"(ok) : "r"(bar), "r"(parity), "r"(1000u) : "memory");
-        if (__all_sync(0xffffffffu, ok)) return true;
-    }
+    for (uint32_t i = 0; i < WAIT_LIMIT; ++i)
+        if (bar_try(bar, parity)) return true;
+    return false;
+}
+// The same for a whole converged warp, all lanes on one barrier
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < WAIT_LIMIT; ++i)
+        if (__all_sync(0xffffffffu, bar_try(bar, parity))) return true;
     return false;
 }
 // TMA gather: rows y0..y3, 64 16-bit columns from x (a multiple of 8), of the mapped matrix (box of one row) -> four consecutive
