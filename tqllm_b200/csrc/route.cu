@@ -47,11 +47,14 @@ __global__ void router_k(const float * __restrict__ w, const float * __restrict_
     }
 }
 
-// ---- tensor-core router for bf16 activations ----
-// logits = W x with W fp32 split exactly into three bf16 terms (hi + mid + lo = 24 significant bits) and x bf16 as it
-// is: every product is exact in fp32 and the sums are fp32, so the result is fp32-accurate (within 3e-6 of an fp64
-// dot) at a fraction of the instructions of the scalar loop. One block = 16 router rows x 64 tokens; its 8 warps
-// split the hidden dimension and add their partial tiles in shared memory in warp order.
+// ---- tensor-core router ----
+// logits = W x with W fp32 split exactly into three bf16 terms (hi + mid + lo = 24 significant bits) and x split into as many as
+// it has bits for (bf16: itself, fp16: two, fp32: three; of the fp32 products the three whose terms lie below 2^-24 of the
+// product are left out): every product is exact in fp32 and the sums are fp32, so the result is fp32-accurate (within 3e-6 of
+// an fp64 dot) at a fraction of the instructions of a scalar loop (fp16, 600 tokens x 256 experts x 3072: scalar 245 us).
+// One block = 16 router rows x 8 J tokens; its 16 warps split the hidden dimension and add their partial tiles in shared
+// memory in warp order. J is the smallest of 1, 2, 4, 8 that takes the batch, 8 above: with J = 8 one token pays for 64.
+template <int DT> constexpr int x_terms() { return DT == B2MOE_BF16 ? 1 : DT == B2MOE_F16 ? 2 : 3; }
 constexpr int RM_WARPS = 16, RM_PART = 8;   // warps per block (each takes a slice of the columns); partial-sum slots in shared memory
 __device__ __forceinline__ void split3(float2 w, uint32_t & hi, uint32_t & mid, uint32_t & lo) {
     const __nv_bfloat16 h0 = __float2bfloat16_rn(w.x), h1 = __float2bfloat16_rn(w.y);
@@ -66,9 +69,32 @@ __device__ __forceinline__ void mma_bf16_acc(float (&c)[4], const uint32_t (&a)[
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// (w.x, w.y) -> bf16x2 terms hi, mid, lo with hi + mid + lo = w exactly (24 significant bits); same values as split3
+__device__ __forceinline__ void split3_pair(float2 w, uint32_t & hi, uint32_t & mid, uint32_t & lo) {
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(w.y), "f"(w.x));
+    const float r0 = w.x - __uint_as_float(hi << 16), r1 = w.y - __uint_as_float(hi & 0xffff0000u);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(mid) : "f"(r1), "f"(r0));
+    const float q0 = r0 - __uint_as_float(mid << 16), q1 = r1 - __uint_as_float(mid & 0xffff0000u);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(q1), "f"(q0));
+}
+// two neighbouring activations at p -> their bf16x2 terms, the largest first
+template <int DT> __device__ __forceinline__ void x_pair(const typename Elem<DT>::type * p, uint32_t (&v)[x_terms<DT>()]) {
+    if constexpr (DT == B2MOE_BF16) {
+        v[0] = *reinterpret_cast<const uint32_t *>(p);
+    } else if constexpr (DT == B2MOE_F16) {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(p));
+        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(v[0]) : "f"(f.y), "f"(f.x));
+        const float r0 = f.x - __uint_as_float(v[0] << 16), r1 = f.y - __uint_as_float(v[0] & 0xffff0000u);      // at most 3 bits are left: exact as bf16
+        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(v[1]) : "f"(r1), "f"(r0));
+    } else {
+        split3_pair(*reinterpret_cast<const float2 *>(p), v[0], v[1], v[2]);
+    }
+}
+template <int DT, int J>
 __global__ void __launch_bounds__(RM_WARPS * 32) router_mma_k(const float * __restrict__ w, const float * __restrict__ shared,
-                                                                const __nv_bfloat16 * __restrict__ x, float * __restrict__ logits, int ld,
+                                                                const typename Elem<DT>::type * __restrict__ x, float * __restrict__ logits, int ld,
                                                                 int h, int e, int rows, int n) {
+    constexpr int XT = x_terms<DT>(), TOK = 8 * J;
     __shared__ float part[RM_PART][16][65];
     __shared__ float tile[16][65];                                      // this block's sums over its slice of the columns
     namespace cg = cooperative_groups;
@@ -76,12 +102,12 @@ __global__ void __launch_bounds__(RM_WARPS * 32) router_mma_k(const float * __re
     grid_release();
     grid_wait();                                                       // x may be the output of the launch before this one
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    const int r0 = blockIdx.x * 16, t0 = blockIdx.y * 64;
+    const int r0 = blockIdx.x * 16, t0 = blockIdx.y * TOK;
     const int ra = min(r0 + g, rows - 1), rb = min(r0 + g + 8, rows - 1);
     const float * wa = ra == e ? shared : w + size_t(ra) * h, * wb = rb == e ? shared : w + size_t(rb) * h;
-    float acc[8][4];
+    float acc[J][4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
+    for (int j = 0; j < J; ++j)
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[j][i] = 0.f;
     const int hs = h / int(gridDim.z), h_lo = int(blockIdx.z) * hs;     // this block's columns (a multiple of 16)
@@ -95,19 +121,24 @@ __global__ void __launch_bounds__(RM_WARPS * 32) router_mma_k(const float * __re
         split3(*reinterpret_cast<const float2 *>(wa + k0 + 2 * t + 8), hi[2], mid[2], lo[2]);
         split3(*reinterpret_cast<const float2 *>(wb + k0 + 2 * t + 8), hi[3], mid[3], lo[3]);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < J; ++j) {
             const int tok = min(t0 + 8 * j + g, n - 1);
-            const uint32_t * xr = reinterpret_cast<const uint32_t *>(x + size_t(tok) * h + k0 + 2 * t);
-            const uint32_t b0 = xr[0], b1 = xr[4];
-            mma_bf16_acc(acc[j], lo, b0, b1);                            // smallest terms first
-            mma_bf16_acc(acc[j], mid, b0, b1);
-            mma_bf16_acc(acc[j], hi, b0, b1);
+            const typename Elem<DT>::type * xr = x + size_t(tok) * h + k0 + 2 * t;
+            uint32_t b0[XT], b1[XT];
+            x_pair<DT>(xr, b0);
+            x_pair<DT>(xr + 8, b1);
+#pragma unroll
+            for (int xt = XT - 1; xt >= 0; --xt) {                       // smallest terms first
+                if (xt == 0 || DT == B2MOE_F16) mma_bf16_acc(acc[j], lo, b0[xt], b1[xt]);
+                if (xt < 2) mma_bf16_acc(acc[j], mid, b0[xt], b1[xt]);
+                mma_bf16_acc(acc[j], hi, b0[xt], b1[xt]);
+            }
         }
     }
     // warps 8..15 park their sums, warps 0..7 add theirs on top (always in this order: the same bits every run)
     if (warp >= RM_PART) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < J; ++j) {
             part[warp - RM_PART][g][8 * j + 2 * t] = acc[j][0]; part[warp - RM_PART][g][8 * j + 2 * t + 1] = acc[j][1];
             part[warp - RM_PART][g + 8][8 * j + 2 * t] = acc[j][2]; part[warp - RM_PART][g + 8][8 * j + 2 * t + 1] = acc[j][3];
         }
@@ -115,13 +146,13 @@ __global__ void __launch_bounds__(RM_WARPS * 32) router_mma_k(const float * __re
     __syncthreads();
     if (warp < RM_PART) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < J; ++j) {
             part[warp][g][8 * j + 2 * t] += acc[j][0]; part[warp][g][8 * j + 2 * t + 1] += acc[j][1];
             part[warp][g + 8][8 * j + 2 * t] += acc[j][2]; part[warp][g + 8][8 * j + 2 * t + 1] += acc[j][3];
         }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < 16 * 64; i += blockDim.x) {
+    for (int i = threadIdx.x; i < 16 * TOK; i += blockDim.x) {
         const int r = i & 15, c = i >> 4;
         float s = 0.f;
 #pragma unroll
@@ -132,7 +163,7 @@ __global__ void __launch_bounds__(RM_WARPS * 32) router_mma_k(const float * __re
     // distributed shared memory (the same bits every run) and writes the logits
     cluster.sync();
     if (blockIdx.z == 0) {
-        for (int i = threadIdx.x; i < 16 * 64; i += blockDim.x) {
+        for (int i = threadIdx.x; i < 16 * TOK; i += blockDim.x) {
             const int r = i & 15, c = i >> 4;
             if (r0 + r < rows && t0 + c < n) {
                 float s = tile[r][c];
@@ -145,35 +176,41 @@ __global__ void __launch_bounds__(RM_WARPS * 32) router_mma_k(const float * __re
 }
 
 // ---- the same product for many tokens (prefill): shared-memory tiles ----
-// One block = 64 router rows x 128 tokens, 8 warps of 32 x 32 outputs, 32 columns per stage: the weights are split into
-// their three bf16 terms once per block and stage (not once per 64 tokens and warp as above) and both operands reach the
-// MMAs through ldmatrix, so a stage costs a warp 16 shared loads for its 48 MMAs. Every output is summed by one warp over
-// the whole hidden dimension in ascending column order (terms lo, mid, hi per 16 columns; 256 columns per partial sum): the
-// same bits every run.
+// One block = 64 router rows x 128 tokens, 8 warps of 32 x 32 outputs, 32 columns per stage: both operands are split into
+// their bf16 terms once per block and stage (not once per 64 tokens and warp as above) and reach the MMAs through ldmatrix, so
+// a stage of bf16 rows costs a warp 16 shared loads for its 48 MMAs. Every output is summed over the hidden dimension in
+// ascending column order (terms lo, mid, hi per 16 columns; 256 columns per partial sum): the same bits every run.
+// A launch has few such tiles (2047 tokens x 256 experts: 64), and a tile alone leaves an SM waiting on its own loads: up to
+// eight blocks of a cluster take a part of a tile's 256-column partial sums each and add all of them, in column order, through
+// distributed shared memory, so the split changes no bit.
+// Measured, one block per tile against the split: 32 tiles of 2048 columns 60 -> 21 us, 64 of 3072 columns 85 -> 57, 20 of 3072
+// columns (fp16) 124 -> 32; 128 of 4096 columns 116 -> 127, 256 of 2048 columns 96 -> 118: from 100 tiles on, one block per tile.
 constexpr int RT_ROWS = 64, RT_TOK = 128, RT_K = 32, RT_THREADS = 256, RT_LD = RT_K + 8;   // row stride in shared memory: 80 bytes, conflict-free for ldmatrix
-constexpr int RT_W_STAGE = 3 * RT_ROWS * RT_LD * 2, RT_X_STAGE = RT_TOK * RT_LD * 2, RT_SMEM = 2 * (RT_W_STAGE + RT_X_STAGE);
+constexpr int RT_SPLIT_BELOW = 100, RT_MAX_PARTS = 64, RT_COLS = 256, RT_PLD = RT_ROWS + 4, RT_PART = RT_TOK * RT_PLD * 4;           // columns of a partial sum; a tile of them in shared memory, [token][row]
+constexpr int RT_W_STAGE = 3 * RT_ROWS * RT_LD * 2, RT_X_TERM = RT_TOK * RT_LD * 2;
+template <int DT> constexpr int rt_stages_bytes() { return 2 * (RT_W_STAGE + x_terms<DT>() * RT_X_TERM); }
 __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
-// (w.x, w.y) -> bf16x2 terms hi, mid, lo with hi + mid + lo = w exactly (24 significant bits); same values as split3
-__device__ __forceinline__ void split3_pair(float2 w, uint32_t & hi, uint32_t & mid, uint32_t & lo) {
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(w.y), "f"(w.x));
-    const float r0 = w.x - __uint_as_float(hi << 16), r1 = w.y - __uint_as_float(hi & 0xffff0000u);
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(mid) : "f"(r1), "f"(r0));
-    const float q0 = r0 - __uint_as_float(mid << 16), q1 = r1 - __uint_as_float(mid & 0xffff0000u);
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(q1), "f"(q0));
-}
+template <int DT, bool SPLIT>
 __global__ void __launch_bounds__(RT_THREADS) router_tile_k(const float * __restrict__ w, const float * __restrict__ shared,
-                                                             const __nv_bfloat16 * __restrict__ x, float * __restrict__ logits, int ld, int h,
+                                                             const typename Elem<DT>::type * __restrict__ x, float * __restrict__ logits, int ld, int h,
                                                              int e, int rows, int n) {
+    using E = typename Elem<DT>::type;
+    constexpr int XT = x_terms<DT>(), X_STAGE = XT * RT_X_TERM;
+    namespace cg = cooperative_groups;
     extern __shared__ __align__(128) uint8_t rt_smem[];
     uint8_t * w_sm = rt_smem;                                          // [2 stages][3 terms][64 rows][RT_LD] bf16
-    uint8_t * x_sm = rt_smem + 2 * RT_W_STAGE;                         // [2 stages][128 tokens][RT_LD] bf16
+    uint8_t * x_sm = rt_smem + 2 * RT_W_STAGE;                         // [2 stages][XT terms][128 tokens][RT_LD] bf16
     grid_release();
     grid_wait();                                                       // x may be the output of the launch before this one
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int r0 = blockIdx.x * RT_ROWS, t0 = blockIdx.y * RT_TOK;
     const int wr = warp >> 2, wc = warp & 3;                            // the warp's 32 rows x 32 tokens
+    // the block's partial sums [p_lo, p_hi) of the tile's n_part; the last one takes the stages' place in shared memory, the others follow them
+    const int n_part = (h + RT_COLS - 1) / RT_COLS, ks = gridDim.z;
+    auto first_part = [&](int z) { return n_part * z / ks; };
+    const int p_lo = first_part(blockIdx.z), p_hi = first_part(blockIdx.z + 1);
     // this thread's four float2 of a weight stage: row f / 16, columns 2 (f % 16), f = tid + 256 j
     const float * wsrc[4];
 #pragma unroll
@@ -181,21 +218,43 @@ __global__ void __launch_bounds__(RT_THREADS) router_tile_k(const float * __rest
         const int f = tid + RT_THREADS * j, row = min(r0 + (f >> 4), rows - 1);
         wsrc[j] = (row == e ? shared : w + size_t(row) * h) + 2 * (f & 15);
     }
-    // this thread's two 16-byte pieces of an activation stage: token p / 4, piece p % 4, p = tid + 256 j
-    const __nv_bfloat16 * xsrc[2];
+    // this thread's 16 values of an activation stage: 16-byte pieces p = tid + 256 j, token p / PPT, piece p % PPT
+    constexpr int V = 16 / int(sizeof(E)), PPT = RT_K / V, XJ = RT_TOK * PPT / RT_THREADS;
+    const E * xsrc[XJ];
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
+    for (int j = 0; j < XJ; ++j) {
         const int p = tid + RT_THREADS * j;
-        xsrc[j] = x + size_t(min(t0 + (p >> 2), n - 1)) * h + 8 * (p & 3);
+        xsrc[j] = x + size_t(min(t0 + p / PPT, n - 1)) * h + V * (p % PPT);
     }
-    auto load_x = [&](int stage, int k0) {
+    [[maybe_unused]] uint4 xreg[XJ];
+    auto load_x = [&](int stage, int k0) {                             // bf16 rows go straight to shared memory, the others wait in registers to be split
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int p = tid + RT_THREADS * j;
-            const uint32_t dst = uint32_t(__cvta_generic_to_shared(x_sm + stage * RT_X_STAGE + ((p >> 2) * RT_LD + 8 * (p & 3)) * 2));
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(__cvta_generic_to_global(xsrc[j] + k0)) : "memory");
+        for (int j = 0; j < XJ; ++j) {
+            if constexpr (XT == 1) {
+                const int p = tid + RT_THREADS * j;
+                const uint32_t dst = uint32_t(__cvta_generic_to_shared(x_sm + stage * X_STAGE + ((p / PPT) * RT_LD + V * (p % PPT)) * 2));
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(__cvta_generic_to_global(xsrc[j] + k0)) : "memory");
+            } else {
+                xreg[j] = *reinterpret_cast<const uint4 *>(xsrc[j] + k0);
+            }
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        if constexpr (XT == 1) asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto store_x = [&](int stage) {
+        if constexpr (XT > 1) {
+#pragma unroll
+            for (int j = 0; j < XJ; ++j) {
+                const int p = tid + RT_THREADS * j;
+                uint32_t * dst = reinterpret_cast<uint32_t *>(x_sm + stage * X_STAGE + ((p / PPT) * RT_LD + V * (p % PPT)) * 2);
+#pragma unroll
+                for (int i = 0; i < V / 2; ++i) {
+                    uint32_t v[XT];
+                    x_pair<DT>(reinterpret_cast<const E *>(&xreg[j]) + 2 * i, v);
+#pragma unroll
+                    for (int q = 0; q < XT; ++q) dst[q * (RT_X_TERM / 4) + i] = v[q];
+                }
+            }
+        }
     };
     float2 wreg[4];
     auto load_w = [&](int k0) {
@@ -214,33 +273,50 @@ __global__ void __launch_bounds__(RT_THREADS) router_tile_k(const float * __rest
             dst[2 * RT_ROWS * RT_LD / 2] = lo;
         }
     };
-    // acc sums 256 columns at a time and is then added to tot: the rounding error of a long fp32 chain grows with its
+    // acc sums 256 columns at a time and is then put away: the rounding error of a long fp32 chain grows with its
     // length, and the router's tolerance against an fp64 dot (3e-6) leaves no room for a 2048-term chain
-    float acc[2][4][4], tot[2][4][4];
+    float acc[2][4][4];
+    [[maybe_unused]] float tot[2][4][4];                               // one block per tile: it adds the partial sums up in registers
 #pragma unroll
     for (int a = 0; a < 2; ++a)
 #pragma unroll
         for (int b = 0; b < 4; ++b)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) acc[a][b][c] = tot[a][b][c] = 0.f;
+            for (int c = 0; c < 4; ++c) { acc[a][b][c] = 0.f; if (!SPLIT) tot[a][b][c] = 0.f; }
+    auto put_away = [&](uint8_t * at) {
+        float * part = reinterpret_cast<float *>(at);
+#pragma unroll
+        for (int rt = 0; rt < 2; ++rt)
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    part[(32 * wc + 8 * nt + 2 * t + (c & 1)) * RT_PLD + 32 * wr + 16 * rt + g + 8 * (c >> 1)] = acc[rt][nt][c];
+                    acc[rt][nt][c] = 0.f;
+                }
+    };
     // ldmatrix addresses of this lane inside a stage: A rows 32 wr + 16 rt + (lane % 16), columns 8 (lane / 16);
     // B tokens 32 wc + 16 pr + (lane % 8) + 8 (lane / 16), columns 8 ((lane / 8) % 2)
     const uint32_t w_base = uint32_t(__cvta_generic_to_shared(w_sm)) + ((32 * wr + (lane & 15)) * RT_LD + 8 * (lane >> 4)) * 2;
     const uint32_t x_base = uint32_t(__cvta_generic_to_shared(x_sm)) + ((32 * wc + (lane & 7) + 8 * (lane >> 4)) * RT_LD + 8 * ((lane >> 3) & 1)) * 2;
-    const int stages = h / RT_K;
-    load_x(0, 0);
-    load_w(0);
-    for (int s = 0; s < stages; ++s) {
+    const int s_lo = p_lo * (RT_COLS / RT_K), s_hi = min(h / RT_K, p_hi * (RT_COLS / RT_K));
+    load_x(s_lo & 1, s_lo * RT_K);
+    load_w(s_lo * RT_K);
+#pragma unroll 1
+    for (int s = s_lo; s < s_hi; ++s) {
         const int buf = s & 1;
         store_w(buf);
+        store_x(buf);
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();                                               // stage s is complete; every warp is done with stage s - 1
-        if (s + 1 < stages) { load_x(buf ^ 1, (s + 1) * RT_K); load_w((s + 1) * RT_K); }
+        if (s + 1 < s_hi) { load_x(buf ^ 1, (s + 1) * RT_K); load_w((s + 1) * RT_K); }
 #pragma unroll
         for (int kk = 0; kk < RT_K / 16; ++kk) {
-            uint32_t b[2][4];                                          // token tiles (0, 1) and (2, 3): b0, b1 of each
+            uint32_t b[XT][2][4];                                      // per term, token tiles (0, 1) and (2, 3): b0, b1 of each
 #pragma unroll
-            for (int pr = 0; pr < 2; ++pr) ldmatrix4(b[pr], x_base + buf * RT_X_STAGE + (16 * pr * RT_LD + 16 * kk) * 2);
+            for (int q = 0; q < XT; ++q)
+#pragma unroll
+                for (int pr = 0; pr < 2; ++pr) ldmatrix4(b[q][pr], x_base + buf * X_STAGE + q * RT_X_TERM + (16 * pr * RT_LD + 16 * kk) * 2);
 #pragma unroll
             for (int term = 2; term >= 0; --term) {                    // smallest terms first
 #pragma unroll
@@ -248,11 +324,16 @@ __global__ void __launch_bounds__(RT_THREADS) router_tile_k(const float * __rest
                     uint32_t a[4];
                     ldmatrix4(a, w_base + buf * RT_W_STAGE + ((term * RT_ROWS + 16 * rt) * RT_LD + 16 * kk) * 2);
 #pragma unroll
-                    for (int nt = 0; nt < 4; ++nt) mma_bf16_acc(acc[rt][nt], a, b[nt >> 1][2 * (nt & 1)], b[nt >> 1][2 * (nt & 1) + 1]);
+                    for (int q = XT - 1; q >= 0; --q)
+#pragma unroll
+                        for (int nt = 0; nt < 4; ++nt)
+                            if (DT != B2MOE_F32 || term + q < 3) mma_bf16_acc(acc[rt][nt], a, b[q][nt >> 1][2 * (nt & 1)], b[q][nt >> 1][2 * (nt & 1) + 1]);
                 }
             }
         }
-        if ((s & 7) == 7 || s + 1 == stages) {
+        if constexpr (SPLIT) {
+            if ((s & 7) == 7 && s + 1 < s_hi) put_away(rt_smem + rt_stages_bytes<DT>() + (s / 8 - p_lo) * RT_PART);
+        } else if ((s & 7) == 7 || s + 1 == s_hi) {
 #pragma unroll
             for (int a = 0; a < 2; ++a)
 #pragma unroll
@@ -261,15 +342,52 @@ __global__ void __launch_bounds__(RT_THREADS) router_tile_k(const float * __rest
                     for (int c = 0; c < 4; ++c) { tot[a][b][c] += acc[a][b][c]; acc[a][b][c] = 0.f; }
         }
     }
+    if constexpr (!SPLIT) {
 #pragma unroll
-    for (int rt = 0; rt < 2; ++rt)
+        for (int rt = 0; rt < 2; ++rt)
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
+            for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int row = r0 + 32 * wr + 16 * rt + g + 8 * (c >> 1), tok = t0 + 32 * wc + 8 * nt + 2 * t + (c & 1);
-                if (row < rows && tok < n) logits[size_t(tok) * ld + row] = tot[rt][nt][c];
+                for (int c = 0; c < 4; ++c) {
+                    const int row = r0 + 32 * wr + 16 * rt + g + 8 * (c >> 1), tok = t0 + 32 * wc + 8 * nt + 2 * t + (c & 1);
+                    if (row < rows && tok < n) logits[size_t(tok) * ld + row] = tot[rt][nt][c];
+                }
+        return;
+    }
+    __syncthreads();                                                   // every warp is done with the stages
+    put_away(rt_smem);
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    // every block of the cluster finishes a share of the tile's tokens; the partial sums' places in the cluster's shared memory
+    // come from a table, eight loads are in flight at a time
+    __shared__ uint32_t place[RT_MAX_PARTS];
+    if (tid < n_part) {
+        int z = 0;
+        while (first_part(z + 1) <= tid) ++z;
+        const int q = tid - first_part(z), last = first_part(z + 1) - first_part(z) - 1;
+        const uint32_t local = uint32_t(__cvta_generic_to_shared(rt_smem)) + (q < last ? rt_stages_bytes<DT>() + q * RT_PART : 0);
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(place[tid]) : "r"(local), "r"(z));
+    }
+    __syncthreads();
+    const int tk_lo = RT_TOK * int(blockIdx.z) / ks, tk_hi = RT_TOK * (int(blockIdx.z) + 1) / ks;
+    for (int i = tid; i < (tk_hi - tk_lo) * RT_ROWS; i += RT_THREADS) {
+        const int tk = tk_lo + i / RT_ROWS, r = i % RT_ROWS;
+        if (t0 + tk >= n || r0 + r >= rows) continue;
+        const uint32_t off = uint32_t(tk * RT_PLD + r) * 4u;
+        float sum = 0.f;
+        for (int q = 0; q < n_part; q += 8) {
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                v[j] = 0.f;
+                if (q + j < n_part) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[j]) : "r"(place[q + j] + off) : "memory");
             }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) if (q + j < n_part) sum += v[j];
+        }
+        logits[size_t(t0 + tk) * ld + r0 + r] = sum;
+    }
+    cluster.sync();                                                    // the blocks' tiles stay alive until every block has read them
 }
 
 __device__ __forceinline__ void argmax_merge(float & v, int & i, float ov, int oi) {
@@ -530,6 +648,53 @@ int32_t route_plan_stage(int gating, const float * logits, int ld, const float *
     *took = true;
     return launch_status();
 }
+namespace {
+template <typename... KArgs, typename... Args>
+int32_t launch_cluster_z(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t s, Args &&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = grid.z;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_overlap ? 2 : 1;
+    if (cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...) != cudaSuccess) return B2MOE_ERR_CUDA;
+    return launch_status();
+}
+template <int DT>
+int32_t router_launch(const float * w, const float * shared, const void * xv, float * logits, int ld, int h, int e, int rows, int n, cudaStream_t s) {
+    const auto * x = static_cast<const typename Elem<DT>::type *>(xv);
+    // Tiles from 256 tokens for bf16 (below, router_mma_k has more blocks and no stage hand-offs); the split operands of the other
+    // types make router_mma_k split the same token values again for every 16 rows, so they change over at 128.
+    if (h % RT_K == 0 && n >= (DT == B2MOE_BF16 ? 2 : 1) * RT_TOK) {
+        const dim3 tiles(ceil_div(rows, RT_ROWS), ceil_div(n, RT_TOK), 1);
+        const int n_part = ceil_div(h, RT_COLS), share = ceil_div(n_part, 8), ks = ceil_div(n_part, share);      // at most eight blocks, no more than the shares need
+        const size_t smem = rt_stages_bytes<DT>() + size_t(share - 1) * RT_PART;
+        static_assert(rt_stages_bytes<DT>() >= RT_PART, "the last partial sum takes the stages' place");
+        const bool split = tiles.x * tiles.y < RT_SPLIT_BELOW && n_part <= RT_MAX_PARTS && smem <= 227 * 1024;
+        const auto kernel = split ? router_tile_k<DT, true> : router_tile_k<DT, false>;
+        const size_t bytes = split ? smem : size_t(rt_stages_bytes<DT>());
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)) != cudaSuccess) return B2MOE_ERR_CUDA;
+        return launch_cluster_z(kernel, dim3(tiles.x, tiles.y, split ? ks : 1), RT_THREADS, bytes, s, w, shared, x, logits, ld, h, e, rows, n);
+    }
+    if (h % 16 == 0) {
+        // split the hidden dimension over a cluster of up to 4 blocks while every block keeps at least 256 columns
+        int ks = 1;
+        while (ks < 4 && h % (32 * ks) == 0 && h / (2 * ks) >= 256) ks *= 2;
+        auto launch = [&](auto kernel, int tokens) {
+            return launch_cluster_z(kernel, dim3(ceil_div(rows, 16), ceil_div(n, tokens), ks), RM_WARPS * 32, 0, s, w, shared, x, logits, ld, h, e, rows, n);
+        };
+        return n <= 8 ? launch(router_mma_k<DT, 1>, 8) : n <= 16 ? launch(router_mma_k<DT, 2>, 16) : n <= 32 ? launch(router_mma_k<DT, 4>, 32) : launch(router_mma_k<DT, 8>, 64);
+    }
+    router_k<DT><<<dim3(ceil_div(rows, 8), std::min(ceil_div(n, ROUTER_TOK), 64)), 256, 0, s>>>(w, shared, x, logits, ld, h, e, rows, n);
+    return launch_status();
+}
+}  // namespace
 }  // namespace b2
 
 using namespace b2;
@@ -541,39 +706,10 @@ extern "C" B2MOE_API int32_t b2moe_router(const float * router_w, const float * 
     if (!valid_dtype(x_dtype)) return B2MOE_ERR_SHAPE;
     if (!aligned16(router_w) || !aligned16(x) || (shared_gate && !aligned16(shared_gate))) return B2MOE_ERR_ALIGN;
     const int rows = experts + (shared_gate ? 1 : 0);
-    const dim3 grid(ceil_div(rows, 8), std::min(ceil_div(n, ROUTER_TOK), 64));
     cudaStream_t s = as_stream(stream);
-    if (x_dtype == B2MOE_F32)
-        router_k<B2MOE_F32><<<grid, 256, 0, s>>>(router_w, shared_gate, static_cast<const float *>(x), logits, ld, hidden, experts, rows, n);
-    else if (x_dtype == B2MOE_BF16 && hidden % RT_K == 0 && n >= 2 * RT_TOK) {
-        if (cudaFuncSetAttribute(router_tile_k, cudaFuncAttributeMaxDynamicSharedMemorySize, RT_SMEM) != cudaSuccess) return B2MOE_ERR_CUDA;
-        launch_overlapped(router_tile_k, dim3(ceil_div(rows, RT_ROWS), ceil_div(n, RT_TOK)), dim3(RT_THREADS), size_t(RT_SMEM), s, router_w, shared_gate,
-                          static_cast<const __nv_bfloat16 *>(x), logits, ld, hidden, experts, rows, n);
-    }
-    else if (x_dtype == B2MOE_BF16 && hidden % 16 == 0)
-    {
-        // split the hidden dimension over a cluster of up to 4 blocks while every block keeps at least 256 columns
-        int ks = 1;
-        while (ks < 4 && hidden % (32 * ks) == 0 && hidden / (2 * ks) >= 256) ks *= 2;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(ceil_div(rows, 16), ceil_div(n, 64), ks);
-        cfg.blockDim = dim3(RM_WARPS * 32);
-        cfg.stream = s;
-        cudaLaunchAttribute attr[2];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = ks;
-        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[1].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = g_overlap ? 2 : 1;
-        if (cudaLaunchKernelEx(&cfg, router_mma_k, router_w, shared_gate, static_cast<const __nv_bfloat16 *>(x), logits, ld, hidden, experts,
-                               rows, n) != cudaSuccess) return B2MOE_ERR_CUDA;
-    }
-    else if (x_dtype == B2MOE_BF16)
-        router_k<B2MOE_BF16><<<grid, 256, 0, s>>>(router_w, shared_gate, static_cast<const __nv_bfloat16 *>(x), logits, ld, hidden, experts, rows, n);
-    else
-        router_k<B2MOE_F16><<<grid, 256, 0, s>>>(router_w, shared_gate, static_cast<const __half *>(x), logits, ld, hidden, experts, rows, n);
-    return launch_status();
+    if (x_dtype == B2MOE_F32) return router_launch<B2MOE_F32>(router_w, shared_gate, x, logits, ld, hidden, experts, rows, n, s);
+    if (x_dtype == B2MOE_BF16) return router_launch<B2MOE_BF16>(router_w, shared_gate, x, logits, ld, hidden, experts, rows, n, s);
+    return router_launch<B2MOE_F16>(router_w, shared_gate, x, logits, ld, hidden, experts, rows, n, s);
 }
 
 extern "C" B2MOE_API int32_t b2moe_topk_softmax(const float * logits, int32_t ld, int32_t * ids, float * weights, float * shared_weights,
