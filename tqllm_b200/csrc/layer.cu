@@ -60,17 +60,18 @@ int decode_kernel(uint32_t type, int k, int dtype) {
 //   decode   every expert sees a few tokens, the product is bound by streaming the weights;
 //   GEMM     the tcgen05 grouped GEMM (all formats): the weights of an expert are decoded once per 128 tokens;
 //   generic  exact fp32 CUDA-core path: every shape, the floor under the other two.
-// Default: a type with a decode kernel takes it while the batch averages fewer than GEMM_MIN_PER assignments per expert
-// or the bank has fewer than GEMM_MIN_EXPERTS experts (too few 128-row x 128-token items to fill the SMs), everything
-// else the GEMM. b2moe_harness_select forces a family where it supports the shape (tests and benchmarks).
-constexpr int GEMM_MIN_PER = 32, GEMM_MIN_EXPERTS = 128;   // measured on the c2 shape: below either, the decode kernels' finer work items win
+// Default: a type with a decode kernel takes it while the batch averages fewer assignments per expert than the crossover
+// below, everything else the GEMM. Measured layer times, decode / GEMM, us: IQ3_S codes (512 experts) 10 per expert 400 / 502,
+// 16: 564 / 550; Q4_K (256 experts) 12: 848 / 1009, 19: 1139 / 1027, (60 experts) 15: 175 / 177, 30: 249 / 184, (32 experts of
+// 1024 x 512) 16: 70 / 70, 64: 111 / 78, (16 experts) 8: 104 / 142, 19: 156 / 148; IQ3_S in GGUF fields 10: 617 / 610. b2moe_harness_select forces a family where it supports the shape (tests and benchmarks).
+constexpr int GEMM_MIN_PER = 16, GEMM_MIN_PER_IQ3S = 10;
 int g_family = B2MOE_FAMILY_AUTO;
 int expert_path(uint32_t type, int k, int dtype, int experts, long long assignments) {
     if (g_family == B2MOE_FAMILY_GENERIC) return B2MOE_FAMILY_GENERIC;
     const bool dec = decode_kernel(type, k, dtype) != DEC_NONE, gemm = gemm_tc_supported(type, k, experts);
     if (g_family == B2MOE_FAMILY_DECODE) return dec ? B2MOE_FAMILY_DECODE : B2MOE_FAMILY_GENERIC;
     if (g_family == B2MOE_FAMILY_GEMM) return gemm ? B2MOE_FAMILY_GEMM : dec ? B2MOE_FAMILY_DECODE : B2MOE_FAMILY_GENERIC;
-    if (dec && (!gemm || assignments < (long long)GEMM_MIN_PER * experts || experts < GEMM_MIN_EXPERTS)) return B2MOE_FAMILY_DECODE;
+    if (dec && (!gemm || assignments < (long long)(type == T_IQ3_S ? GEMM_MIN_PER_IQ3S : GEMM_MIN_PER) * experts)) return B2MOE_FAMILY_DECODE;
     return gemm ? B2MOE_FAMILY_GEMM : B2MOE_FAMILY_GENERIC;
 }
 }  // namespace
