@@ -66,28 +66,32 @@ template <> struct Dec<T_Q4_K> {
     __device__ __forceinline__ static uint32_t two(uint32_t nib, __half2 S, __half2 NS, __half2 MH, __half2 ML, __half2 D) {
         return h2_bits(__hadd2(__hfma2(__hfma2(bits_h2(nib | 0x64006400u), S, NS), D, MH), ML));
     }
-    // Once per chunk: lane t of a row's four lanes turns the headers of its two rows into the constants of the unit's sub-block t;
-    // a step fetches its two sub-blocks from lanes 2 js and 2 js + 1. SM[r] = (S, MH), ML = the rows' ML, D = the rows' d.
-    struct Pre { uint32_t SM[2], ML, D; };
+    // Once per chunk: lane t of a row's four lanes turns the headers of its two rows into the constants of the unit's sub-block t,
+    // both rows in one register (row g low, row g + 8 high); a step fetches its two sub-blocks from lanes 2 js and 2 js + 1. The
+    // scales and mins are exact as fp16, MH = fp16(-dmin m), ML = the exact rest.
+    struct Pre { uint32_t S, MH, ML, D; };
     __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, int u) {
         const int g = lane >> 2, t = lane & 3;
-        Pre p;
-        uint32_t d[2];
-        float ml[2];
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const uint4 h = *reinterpret_cast<const uint4 *>(chunk + 2048 + 16 * (g + 8 * r));    // d, dmin | s[12]
-            const float dmin = __half2float(__ushort_as_half((unsigned short)(h.x >> 16)));
-            d[r] = h.x & 0xffffu;
-            const uint32_t sc4 = u == 0 ? h.y & 0x3F3F3F3Fu : (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u);         // scales of sub-blocks 0..3 or 4..7
-            const uint32_t mn4 = u == 0 ? h.z & 0x3F3F3F3Fu : ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u);
-            const float sc = float((sc4 >> (8 * t)) & 255u), m = -(dmin * float((mn4 >> (8 * t)) & 255u));              // exact in fp32 (11 x 6 bits)
-            const __half mh = __float2half_rn(m);
-            p.SM[r] = h2_bits(__halves2half2(__float2half_rn(t & 1 ? sc * 0.0625f : sc), mh));
-            ml[r] = m - __half2float(mh);
+        const uint4 h0 = *reinterpret_cast<const uint4 *>(chunk + 2048 + 16 * g), h1 = *reinterpret_cast<const uint4 *>(chunk + 2048 + 16 * (g + 8));    // d, dmin | s[12]
+        // the unit's four scales and four mins as bytes (src/formats/weight/dequant.cpp:56-64)
+        uint32_t sc0 = h0.y, mn0 = h0.z, sc1 = h1.y, mn1 = h1.z;
+        if (u) {
+            sc0 = (h0.w & 0x0F0F0F0Fu) | ((h0.y >> 2) & 0x30303030u); mn0 = ((h0.w >> 4) & 0x0F0F0F0Fu) | ((h0.z >> 2) & 0x30303030u);
+            sc1 = (h1.w & 0x0F0F0F0Fu) | ((h1.y >> 2) & 0x30303030u); mn1 = ((h1.w >> 4) & 0x0F0F0F0Fu) | ((h1.z >> 2) & 0x30303030u);
         }
-        p.ML = pack_h2(ml[0], ml[1]);
-        p.D = d[0] | (d[1] << 16);
+        const uint32_t sel = uint32_t(t) * 0x0101u + 0x0400u;               // selector nibbles 0 and 2: byte t of the first, of the second word
+        auto pick = [&](uint32_t x, uint32_t y) {                            // byte t of either word, 16 bits apart, as fp16: 1024 + byte, then - 1024
+            const uint32_t v = __byte_perm(x, y, sel);
+            return __hadd2(bits_h2((v & 0x003F003Fu) | 0x64006400u), __float2half2_rn(-1024.f));
+        };
+        const __half2 sc = pick(sc0, sc1), mn = pick(mn0, mn1);
+        const __half2 dm = bits_h2(__byte_perm(h0.x, h1.x, 0x7632) ^ 0x80008000u);       // -dmin of the two rows
+        Pre p;
+        p.S = h2_bits(t & 1 ? __hmul2(sc, __float2half2_rn(0.0625f)) : sc);
+        const __half2 mh = __hmul2(dm, mn);
+        p.MH = h2_bits(mh);
+        p.ML = h2_bits(__hfma2(dm, mn, __hneg2(mh)));
+        p.D = __byte_perm(h0.x, h1.x, 0x5410);
         return p;
     }
     template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void *, const Pre & p, uint32_t (&f)[16]) {
@@ -95,14 +99,14 @@ template <> struct Dec<T_Q4_K> {
         const uint4 w4 = plane(chunk, 2 * u + JS, lane);
         const uint32_t w[2][2] = {{w4.x, w4.y}, {w4.z, w4.w}};
         const __half2 neg1024 = __float2half2_rn(-1024.f);
-        const __half2 ml0 = bits_h2(__shfl_sync(0xffffffffu, p.ML, s0)), ml1 = bits_h2(__shfl_sync(0xffffffffu, p.ML, s1));
+        const __half2 SA = bits_h2(__shfl_sync(0xffffffffu, p.S, s0)), SB = bits_h2(__shfl_sync(0xffffffffu, p.S, s1));
+        const __half2 MHA = bits_h2(__shfl_sync(0xffffffffu, p.MH, s0)), MHB = bits_h2(__shfl_sync(0xffffffffu, p.MH, s1));
+        const __half2 MLA = bits_h2(__shfl_sync(0xffffffffu, p.ML, s0)), MLB = bits_h2(__shfl_sync(0xffffffffu, p.ML, s1));
+        const __half2 NA = __hmul2(SA, neg1024), NB = __hmul2(SB, neg1024), DD = bits_h2(p.D);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-            const __half2 a0 = bits_h2(__shfl_sync(0xffffffffu, p.SM[r], s0)), a1 = bits_h2(__shfl_sync(0xffffffffu, p.SM[r], s1));
-            const __half2 D = r ? __high2half2(bits_h2(p.D)) : __low2half2(bits_h2(p.D));
-            const __half2 S0 = __low2half2(a0), S1 = __low2half2(a1), N0 = __hmul2(S0, neg1024), N1 = __hmul2(S1, neg1024);
-            const __half2 MH0 = __high2half2(a0), MH1 = __high2half2(a1);
-            const __half2 ML0 = r ? __high2half2(ml0) : __low2half2(ml0), ML1 = r ? __high2half2(ml1) : __low2half2(ml1);
+            auto row = [&](__half2 v) { return r ? __high2half2(v) : __low2half2(v); };
+            const __half2 S0 = row(SA), S1 = row(SB), N0 = row(NA), N1 = row(NB), MH0 = row(MHA), MH1 = row(MHB), ML0 = row(MLA), ML1 = row(MLB), D = row(DD);
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
                 const uint32_t v = w[r][b], v8 = v >> 8;
