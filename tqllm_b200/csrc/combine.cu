@@ -8,9 +8,8 @@ namespace {
 
 // residual (may be null): rows [n][h] of the output's type added to the sum: the layer's skip connection in the same pass
 template <int DT>
-__global__ void combine_k(const float * __restrict__ y, const int * __restrict__ ids, const float * __restrict__ w,
-                          const float * __restrict__ sw, int n, int k, int h, int shared_tokens, const typename Elem<DT>::type * residual,
-                          typename Elem<DT>::type * out) {                 // residual may be out: no __restrict__ on the two
+__global__ void combine_k(const float * y, const int * ids, const float * w, const float * sw, int n, int k, int h, int shared_tokens,
+                          const typename Elem<DT>::type * residual, typename Elem<DT>::type * out) {
     const int t = blockIdx.x;                     // tokens on gridDim.x: any batch size
     const int j = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
     grid_release();

@@ -53,7 +53,7 @@ template <> struct RowLoad<B2MOE_F16> {
     }
 };
 template <int DT>
-__device__ inline float stage_row_lanes(const void * __restrict__ x, size_t first, int k, int bits, uint8_t * orow, int lane) {
+__device__ inline float stage_row_lanes(const void * x, size_t first, int k, int bits, uint8_t * orow, int lane) {
     float mx = 0.f;
     for (int i = lane; i < (k >> 3); i += 32) {
         float v[8];

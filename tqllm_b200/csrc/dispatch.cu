@@ -17,7 +17,7 @@ namespace {
 
 constexpr int CHUNK = 256;   // assignments per warp-chunk on the multi-block path
 
-__global__ void dispatch_small_k(const int * __restrict__ ids, int A, int e, int shared_first, int shared_tokens, int * __restrict__ plan) {
+__global__ void dispatch_small_k(const int * ids, int A, int e, int shared_first, int shared_tokens, int * __restrict__ plan) {
     extern __shared__ unsigned short hist[];       // [32 warps][e]
     grid_release();
     grid_wait();

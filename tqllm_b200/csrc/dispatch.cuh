@@ -51,7 +51,7 @@ __device__ inline void finish_plan(int * plan, const int * cs, int * os, int * a
 __host__ __device__ inline size_t dispatch_small_smem(int warps, int e) { return (size_t(warps) * e * 2 + 15) / 16 * 16 + size_t(3) * (e + 2) * 4; }
 
 // ---- single block (up to 32 warps): every phase in shared memory (decode-sized batches); hist = [warps][e] ----
-__device__ __forceinline__ void dispatch_small_body(const int * __restrict__ ids, int A, int e, int shared_first, int shared_tokens,
+__device__ __forceinline__ void dispatch_small_body(const int * ids, int A, int e, int shared_first, int shared_tokens,
                                                     int * __restrict__ plan, unsigned short * hist) {
     const int e1 = e + 1;
     int * counts = plan + PLAN_HDR, * offsets = counts + e1, * active = offsets + e1 + 1, * perm = active + e1;

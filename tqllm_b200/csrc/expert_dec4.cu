@@ -84,7 +84,7 @@ __device__ __forceinline__ void mma_i8(int (&c)[4], uint32_t a0, uint32_t a1, ui
 }
 // Activation staging (layout and row code: dec4_stage.cuh): a warp per row, four rows per block.
 constexpr int STAGE_WARPS = 4;
-__global__ void __launch_bounds__(STAGE_WARPS * 32) dec4_stage_k(const void * __restrict__ x, int dtype, int rows, int k, int bits,
+__global__ void __launch_bounds__(STAGE_WARPS * 32) dec4_stage_k(const void * x, int dtype, int rows, int k, int bits,
                                                                  uint8_t * __restrict__ out, float * __restrict__ inv_scale) {
     const int lane = threadIdx.x & 31, row = blockIdx.x * STAGE_WARPS + (threadIdx.x >> 5);
     grid_release();

@@ -92,7 +92,7 @@ template <int DT> __device__ __forceinline__ void x_pair(const typename Elem<DT>
 }
 template <int DT, int J>
 __global__ void __launch_bounds__(RM_WARPS * 32) router_mma_k(const float * __restrict__ w, const float * __restrict__ shared,
-                                                                const typename Elem<DT>::type * __restrict__ x, float * __restrict__ logits, int ld,
+                                                                const typename Elem<DT>::type * x, float * logits, int ld,
                                                                 int h, int e, int rows, int n) {
     constexpr int XT = x_terms<DT>(), TOK = 8 * J;
     __shared__ float part[RM_PART][16][65];
@@ -194,7 +194,7 @@ __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
 }
 template <int DT, bool SPLIT>
 __global__ void __launch_bounds__(RT_THREADS) router_tile_k(const float * __restrict__ w, const float * __restrict__ shared,
-                                                             const typename Elem<DT>::type * __restrict__ x, float * __restrict__ logits, int ld, int h,
+                                                             const typename Elem<DT>::type * x, float * logits, int ld, int h,
                                                              int e, int rows, int n) {
     using E = typename Elem<DT>::type;
     constexpr int XT = x_terms<DT>(), X_STAGE = XT * RT_X_TERM;
@@ -403,7 +403,7 @@ __device__ __forceinline__ uint32_t ordered_bits(float v) {          // monotoni
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 template <int GATING, int R>
-__device__ __forceinline__ void route_token_regs(const float * __restrict__ logits, int ld, const float * __restrict__ bias,
+__device__ __forceinline__ void route_token_regs(const float * logits, int ld, const float * __restrict__ bias,
                                                  int * __restrict__ ids, float * __restrict__ weights, float * __restrict__ shared_weights,
                                                  int e, int k, int norm, float scale, int token, int lane) {
     const float * x = logits + size_t(token) * ld;
@@ -462,7 +462,7 @@ __device__ __forceinline__ void route_token_regs(const float * __restrict__ logi
 // One warp per token. p[] = unbiased probabilities, key[] = selection keys (p, or p + bias), both in shared memory.
 // routes one token with one warp; p / key: e floats each of shared memory owned by the warp
 template <int GATING>
-__device__ __forceinline__ void route_token(const float * __restrict__ logits, int ld, const float * __restrict__ bias, int * __restrict__ ids,
+__device__ __forceinline__ void route_token(const float * logits, int ld, const float * __restrict__ bias, int * __restrict__ ids,
                                             float * __restrict__ weights, float * __restrict__ shared_weights, int e, int k, int norm,
                                             float scale, int token, int lane, float * p, float * key) {
     if (k <= 32 && e <= 128) return route_token_regs<GATING, 4>(logits, ld, bias, ids, weights, shared_weights, e, k, norm, scale, token, lane);
@@ -516,7 +516,7 @@ __device__ __forceinline__ void route_token(const float * __restrict__ logits, i
 }
 
 template <int GATING>
-__global__ void route_k(const float * __restrict__ logits, int ld, const float * __restrict__ bias, int * __restrict__ ids,
+__global__ void route_k(const float * logits, int ld, const float * __restrict__ bias, int * __restrict__ ids,
                         float * __restrict__ weights, float * __restrict__ shared_weights, int e, int k, int norm, float scale, int n) {
     extern __shared__ float smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -549,7 +549,7 @@ __global__ void route2_k(const RouteSet a, const RouteSet b, int ld, const float
 // 512 threads: the register-resident top-k keeps 32 values per lane, which a 1024-thread block's 64 registers would spill.
 constexpr int RD_THREADS = 512;
 template <int GATING>
-__global__ void __launch_bounds__(RD_THREADS) route_dispatch_k(const float * __restrict__ logits, int ld, const float * __restrict__ bias,
+__global__ void __launch_bounds__(RD_THREADS) route_dispatch_k(const float * logits, int ld, const float * __restrict__ bias,
                                                          int * __restrict__ ids, float * __restrict__ weights,
                                                          float * __restrict__ shared_weights, int e, int k, int norm, float scale, int n,
                                                          int shared_first, int shared_count, int * __restrict__ plan) {
@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(RD_THREADS) route_dispatch_k(const float * __r
 constexpr int RC_BLOCKS = 8;
 struct StageJob { const void * x; int dtype, k, bits; uint8_t * rows; float * inv_scale; };     // x = nullptr: nothing to stage
 template <int GATING>
-__global__ void __launch_bounds__(RD_THREADS) route_cluster_k(const float * __restrict__ logits, int ld, const float * __restrict__ bias,
+__global__ void __launch_bounds__(RD_THREADS) route_cluster_k(const float * logits, int ld, const float * __restrict__ bias,
                                                         int * __restrict__ ids, float * __restrict__ weights,
                                                         float * __restrict__ shared_weights, int e, int k, int norm, float scale, int n,
                                                         int shared_first, int shared_count, int * __restrict__ plan, const StageJob st) {
