@@ -88,65 +88,120 @@ constexpr size_t gemm_smem(int experts, int cap, int b_stages, int raw_slots) {
            size_t(experts + 2) * sizeof(Info) + 2 * MAX_CAP * sizeof(int2) + size_t(N_BARS) * 8 + 16;
 }
 
-// One activation row of any dtype -> fp16 scaled by a power of two (largest magnitude in [2^14, 2^15)), by one warp; returns the
-// inverse scale. Inside every 64-column step the columns are stored in the order of the format's A operand (gdec::colmap).
-// Two passes over the row: its largest magnitude with 16-byte loads, then (from the cache) eight source columns per lane into
-// one 16-byte store.
-template <uint32_t T, int DT>
-__device__ __forceinline__ float row_to_f16(const typename Elem<DT>::type * __restrict__ xr, int k, bool wide_loads, __half * __restrict__ orow, int lane) {
+// Eight values of an activation row, those of positions 8 l .. 8 l + 7 of a 64-column step (gdec::colmap): they lie in one, two
+// or four runs of neighbouring columns, so a lane takes them with loads of 16, 8 or 4 bytes (16-bit types; rows are 16-byte
+// aligned). xr points at the step's first column.
+template <uint32_t T, int DT> __device__ __forceinline__ void load_positions(const typename Elem<DT>::type * xr, int l, float (&v)[8]) {
+    using E = typename Elem<DT>::type;
+    constexpr int RUN = T == T_Q4_K || T == T_IQ3S4 ? 8 : T == T_IQ4_XS || T == T_IQ4_NL ? 2 : 4, BYTES = RUN * int(sizeof(E));
+    const int i = l >> 1, b = l & 1;
+    float w[8];                                                        // run after run
+#pragma unroll
+    for (int r = 0; r < 8 / RUN; ++r) {
+        const int col = RUN == 8 ? 32 * (i & 1) + 16 * (i >> 1) + 8 * b : RUN == 4 ? 8 * (2 * b + r + 4 * (i >> 1)) + 4 * (i & 1)
+                                                                                : 32 * (i >> 1) + 8 * b + 2 * (i & 1) + 16 * (r & 1) + 4 * (r >> 1);
+        uint32_t raw[BYTES / 4];
+        if constexpr (BYTES >= 16) {
+#pragma unroll
+            for (int q = 0; q < BYTES / 16; ++q) *reinterpret_cast<uint4 *>(raw + 4 * q) = reinterpret_cast<const uint4 *>(xr + col)[q];
+        } else if constexpr (BYTES == 8) {
+            *reinterpret_cast<uint2 *>(raw) = *reinterpret_cast<const uint2 *>(xr + col);
+        } else {
+            raw[0] = *reinterpret_cast<const uint32_t *>(xr + col);
+        }
+#pragma unroll
+        for (int q = 0; q < RUN; ++q) w[r * RUN + q] = Elem<DT>::to_f(reinterpret_cast<const E *>(raw)[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int half = q & 4, e = q & 3;                             // positions come in two words of four values
+        v[q] = RUN == 8 ? w[half + ((e & 1) << 1) + (e >> 1)] : RUN == 4 ? w[q] : w[half + 2 * (e & 1) + (e >> 1)];
+    }
+}
+// One activation row of any dtype -> fp16 scaled by a power of two (largest magnitude in [2^14, 2^15)), by one warp; put(step
+// column, 16 bytes) stores a lane's eight positions, the inverse scale is returned. Two passes over the row: its largest
+// magnitude, then (from the cache) the values.
+template <uint32_t T, int DT, typename Put>
+__device__ __forceinline__ float row_to_f16(const typename Elem<DT>::type * xr, int k, int lane, Put put) {
     using E = typename Elem<DT>::type;
     constexpr int V = 16 / int(sizeof(E));                              // elements per 16-byte load
     float mx = 0.f;
-    if (wide_loads) {                                                  // rows start on 16-byte boundaries (k is a multiple of 64)
 #pragma unroll 4
-        for (int j = lane * V; j < k; j += 32 * V) {
-            const uint4 q = *reinterpret_cast<const uint4 *>(xr + j);
-            const E * e = reinterpret_cast<const E *>(&q);
+    for (int j = lane * V; j < k; j += 32 * V) {
+        const uint4 q = *reinterpret_cast<const uint4 *>(xr + j);
+        const E * e = reinterpret_cast<const E *>(&q);
 #pragma unroll
-            for (int i = 0; i < V; ++i) mx = fmaxf(mx, fabsf(Elem<DT>::to_f(e[i])));
-        }
-    } else {
-        for (int j = lane; j < k; j += 32) mx = fmaxf(mx, fabsf(Elem<DT>::to_f(xr[j])));
+        for (int i = 0; i < V; ++i) mx = fmaxf(mx, fabsf(Elem<DT>::to_f(e[i])));
     }
     for (int d = 16; d; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
     int ex = int((__float_as_uint(mx) >> 23) & 255u) - 127;              // floor(log2(mx)) for a normal mx
     ex = (mx > 0.f && mx < 3e38f) ? max(-100, min(100, ex)) : 14;
     const float scale = __uint_as_float(uint32_t(127 + 14 - ex) << 23);  // 2^(14 - ex)
-    int col[8];                                                        // source columns of this lane's eight positions, in its 64-column group
-#pragma unroll
-    for (int i = 0; i < 8; ++i) col[i] = gdec::colmap<T>(8 * (lane & 7) + i);
 #pragma unroll 2
     for (int gb = 64 * (lane >> 3); gb < k; gb += 256) {
-        uint32_t v[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = gdec::pack_h2(Elem<DT>::to_f(xr[gb + col[2 * i]]) * scale, Elem<DT>::to_f(xr[gb + col[2 * i + 1]]) * scale);
-        *reinterpret_cast<uint4 *>(orow + gb + 8 * (lane & 7)) = make_uint4(v[0], v[1], v[2], v[3]);
+        float v[8];
+        load_positions<T, DT>(xr + gb, lane & 7, v);
+        put(gb + 8 * (lane & 7), make_uint4(gdec::pack_h2(v[0] * scale, v[1] * scale), gdec::pack_h2(v[2] * scale, v[3] * scale),
+                                            gdec::pack_h2(v[4] * scale, v[5] * scale), gdec::pack_h2(v[6] * scale, v[7] * scale)));
     }
     return __uint_as_float(uint32_t(127 - 14 + ex) << 23);
 }
 // rows in their own order: the gathered form
 template <uint32_t T, int DT>
-__global__ void rows_to_f16_k(const typename Elem<DT>::type * __restrict__ x, int rows, int k, bool wide_loads, __half * __restrict__ out,
-                              float * __restrict__ inv_scale) {
+__global__ void rows_to_f16_k(const typename Elem<DT>::type * x, int rows, int k, __half * out, float * inv_scale) {
     const int lane = threadIdx.x & 31, row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     grid_release();
     grid_wait();
     if (row >= rows) return;
-    const float inv = row_to_f16<T, DT>(x + size_t(row) * k, k, wide_loads, out + size_t(row) * k, lane);
+    const float inv = row_to_f16<T, DT>(x + size_t(row) * k, k, lane, [&](int c, const uint4 & v) { *reinterpret_cast<uint4 *>(out + size_t(row) * k + c) = v; });
     if (lane == 0) inv_scale[row] = inv;
 }
-// rows in the order of the plan's slots (a token's row once for every assignment it has; topk = 0: row = assignment)
+// rows in the order of the plan's slots (a token's row once for every assignment it has; topk = 0: row = assignment), a warp per slot
 template <uint32_t T, int DT>
-__global__ void rows_to_slots_k(const typename Elem<DT>::type * __restrict__ x, const int * __restrict__ plan, int experts, int A, int topk, int k,
-                                bool wide_loads, __half * __restrict__ out, float * __restrict__ inv_scale) {
+__global__ void rows_to_slots_k(const typename Elem<DT>::type * x, const int * plan, int experts, int A, int topk, int k,
+                                __half * out, float * inv_scale) {
     const int lane = threadIdx.x & 31, slot = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     grid_release();
     grid_wait();
     if (slot >= plan[PLAN_NGROUPED]) return;
     const int e1 = experts + 1, a = plan[PLAN_HDR + e1 + e1 + 1 + e1 + slot];
     const int row = topk == 0 ? a : a < A ? a / topk : a - A;
-    const float inv = row_to_f16<T, DT>(x + size_t(row) * k, k, wide_loads, out + size_t(slot) * k, lane);
+    const float inv = row_to_f16<T, DT>(x + size_t(row) * k, k, lane, [&](int c, const uint4 & v) { *reinterpret_cast<uint4 *>(out + size_t(slot) * k + c) = v; });
     if (lane == 0) inv_scale[slot] = inv;
+}
+// the slot of every grouped assignment
+__global__ void slot_of_k(const int * plan, int experts, int * slot_of) {
+    grid_release();
+    grid_wait();
+    const int slot = blockIdx.x * blockDim.x + threadIdx.x, e1 = experts + 1;
+    if (slot < plan[PLAN_NGROUPED]) slot_of[plan[PLAN_HDR + e1 + e1 + 1 + e1 + slot]] = slot;
+}
+// the same rows, a warp per token: the row is converted once and stored into the slots of all its assignments. An assignment that
+// is not grouped has no slot: what slot_of holds for it is told by the plan's own list.
+template <uint32_t T, int DT>
+__global__ void tokens_to_slots_k(const typename Elem<DT>::type * x, const int * plan, const int * slot_of,
+                                  int experts, int n, int topk, int shared, int k, __half * out, float * inv_scale) {
+    const int lane = threadIdx.x & 31, token = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    grid_release();
+    grid_wait();
+    if (token >= n) return;
+    const int e1 = experts + 1, grouped = plan[PLAN_NGROUPED];
+    const int * perm = plan + PLAN_HDR + e1 + e1 + 1 + e1;
+    int mine = -1;                                                     // lane s: the slot of the token's s-th assignment (lane topk: the shared expert's)
+    if (lane < topk + shared) {
+        const int a = lane < topk ? token * topk + lane : n * topk + token, slot = slot_of[a];
+        if (slot >= 0 && slot < grouped && perm[slot] == a) mine = slot;
+    }
+    __shared__ int list[8][32];                                        // the token's slots, for each of the block's warps
+    int * slots = list[threadIdx.x >> 5];
+    const unsigned live = __ballot_sync(0xffffffffu, mine >= 0);
+    if (mine >= 0) slots[__popc(live & ((1u << lane) - 1u))] = mine;
+    __syncwarp();
+    const int count = __popc(live);
+    const float inv = row_to_f16<T, DT>(x + size_t(token) * k, k, lane, [&](int c, const uint4 & v) {
+        for (int i = 0; i < count; ++i) *reinterpret_cast<uint4 *>(out + size_t(slots[i]) * k + c) = v;
+    });
+    if (mine >= 0) inv_scale[mine] = inv;
 }
 
 // MODE 0: act[a][r] = silu(gate_r . x_tok(a)) * (up_r . x_tok(a));  MODE 1: y[a][r] = down_r . act[a]
@@ -259,8 +314,8 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
         auto fetch = [&](const Item & im) {                            // this thread's token of the item
             mine = make_int2(-1, 0);
             if (tid < im.nv) {
-                mine.x = __ldg(perm + im.slot0 + tid);
-                mine.y = __float_as_int(__ldg(p.inv_scale + (p.slots ? im.slot0 + tid : x_row(mine.x))));
+                mine.x = perm[im.slot0 + tid];
+                mine.y = __float_as_int(p.inv_scale[p.slots ? im.slot0 + tid : x_row(mine.x)]);
             }
         };
         auto put = [&](uint32_t n) {                                   // the table of the block's n-th item; then a (bounded) meeting of the warps
@@ -479,7 +534,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
             int row[4] = {0, 0, 0, 0};
             if (!p.slots) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) row[i] = n0 < im.nv ? x_row(__ldg(perm + im.slot0 + min(n0 + i, im.nv - 1))) : 0;      // past the last token: repeat it (dead columns of D)
+                for (int i = 0; i < 4; ++i) row[i] = n0 < im.nv ? x_row(perm[im.slot0 + min(n0 + i, im.nv - 1)]) : 0;      // past the last token: repeat it (dead columns of D)
             }
             const int cls = b_class(im.nv), quads = (im.nv + 3) >> 2, mine = (quads + 1 - lw) >> 1;
             const uint32_t box_bytes = uint32_t((cls + 1) * (p.cap / 4) * group) * 128u;
@@ -578,19 +633,29 @@ template <uint32_t T> bool bank_map(CUtensorMap & m, const b2moe_bank * b, int t
     const cuuint32_t box[3] = {PW, chunk_parts<T>(), cuuint32_t(tiles)};
     return encode_map(m, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, b->data, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
+// From this many slots on, the rows of a batch are converted once per token (two launches), below once per slot (one)
+constexpr int TOKEN_WISE_SLOTS = 4096;
 template <uint32_t T, int DT>
-int32_t convert_rows_dt(const void * x, int rows, int k, bool slots, const GemmArgs & a, int topk, __half * out, float * inv, cudaStream_t s) {
-    using E = typename Elem<DT>::type;
-    const dim3 grid(ceil_div(rows, 8)), block(256);
-    const bool wide = aligned16(x);
-    if (slots) launch_overlapped(rows_to_slots_k<T, DT>, grid, block, 0, s, static_cast<const E *>(x), static_cast<const int *>(a.plan), a.experts, a.A, topk, k, wide, out, inv);
-    else launch_overlapped(rows_to_f16_k<T, DT>, grid, block, 0, s, static_cast<const E *>(x), rows, k, wide, out, inv);
+int32_t convert_rows_dt(const void * xv, int rows_x, int slot_rows, bool slots, int topk, const GemmArgs & a, __half * out, float * inv, int * slot_of, cudaStream_t s) {
+    const auto * x = static_cast<const typename Elem<DT>::type *>(xv);
+    const int * plan = a.plan;
+    const dim3 block(256);
+    if (!slots) {
+        launch_overlapped(rows_to_f16_k<T, DT>, dim3(ceil_div(rows_x, 8)), block, 0, s, x, rows_x, a.k, out, inv);
+    } else if (topk > 1 && topk < 32 && slot_rows >= TOKEN_WISE_SLOTS) {
+        launch_overlapped(slot_of_k, dim3(ceil_div(slot_rows, 256)), block, 0, s, plan, a.experts, slot_of);
+        if (int32_t rc = launch_status()) return rc;
+        launch_overlapped(tokens_to_slots_k<T, DT>, dim3(ceil_div(rows_x, 8)), block, 0, s, x, plan, slot_of, a.experts, rows_x, topk, int(slot_rows > a.A), a.k, out, inv);
+    } else {
+        launch_overlapped(rows_to_slots_k<T, DT>, dim3(ceil_div(slot_rows, 8)), block, 0, s, x, plan, a.experts, a.A, topk, a.k, out, inv);
+    }
     return launch_status();
 }
 // m: the banks (gate, up) or (down, null), then the shared expert's (null: none); x (rows_x rows, in token order for MODE 0, in
-// assignment order for MODE 1) -> fp16 rows in xb (in slot order: slot_rows of them), then the product
+// assignment order for MODE 1) -> fp16 rows in xb (in slot order: slot_rows of them; slot_of: scratch for MODE 0), then the product
 template <uint32_t T, int MODE>
-int32_t gemm_launch_t(GemmArgs a, const b2moe_bank * const * m, const void * x, int dtype, int rows_x, bool slots, int slot_rows, __half * xb, float * inv, cudaStream_t s) {
+int32_t gemm_launch_t(GemmArgs a, const b2moe_bank * const * m, const void * x, int dtype, int rows_x, bool slots, int slot_rows, __half * xb, float * inv, int * slot_of,
+                      cudaStream_t s) {
     const int sms = gemm_sm_count();
     if (sms <= 0) return B2MOE_ERR_CUDA;
     const long long per = (long long)a.A / a.experts;                 // mean tokens per expert
@@ -598,9 +663,9 @@ int32_t gemm_launch_t(GemmArgs a, const b2moe_bank * const * m, const void * x, 
     if (!gemm_fit<T>(a.experts, cap, a)) return B2MOE_ERR_SHAPE;
     const int rows = slots ? slot_rows : rows_x, topk = MODE == 0 ? a.topk : 0;
     int32_t rc = B2MOE_ERR_SHAPE;
-    if (dtype == B2MOE_F32) rc = convert_rows_dt<T, B2MOE_F32>(x, rows, a.k, slots, a, topk, xb, inv, s);
-    else if (dtype == B2MOE_F16) rc = convert_rows_dt<T, B2MOE_F16>(x, rows, a.k, slots, a, topk, xb, inv, s);
-    else if (dtype == B2MOE_BF16) rc = convert_rows_dt<T, B2MOE_BF16>(x, rows, a.k, slots, a, topk, xb, inv, s);
+    if (dtype == B2MOE_F32) rc = convert_rows_dt<T, B2MOE_F32>(x, rows_x, slot_rows, slots, topk, a, xb, inv, slot_of, s);
+    else if (dtype == B2MOE_F16) rc = convert_rows_dt<T, B2MOE_F16>(x, rows_x, slot_rows, slots, topk, a, xb, inv, slot_of, s);
+    else if (dtype == B2MOE_BF16) rc = convert_rows_dt<T, B2MOE_BF16>(x, rows_x, slot_rows, slots, topk, a, xb, inv, slot_of, s);
     if (rc) return rc;
     a.slots = slots;
     a.inv_scale = inv;
@@ -651,12 +716,13 @@ size_t gemm_tc_workspace_bytes(int rows_x, int k) {
     return align_up(size_t(rows_x) * k * 2, 256) + align_up(size_t(rows_x) * sizeof(float), 256);
 }
 
-// rows_buf: optional scratch for the activation rows in slot order (n * topk + shared_tokens rows of length k and their scales)
+// rows_buf: optional scratch for the activation rows in slot order (n * topk + shared_tokens rows of length k, their scales and an index each)
 int32_t gemm_tc_gateup(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_bank * sg, const b2moe_bank * su, const void * x,
                        int x_dtype, const int * plan, int n, int topk, int shared_tokens, float * act, void * ws, void * rows_buf,
                        size_t rows_buf_bytes, cudaStream_t s) {
     const int k = gate->cols, slot_rows = n * topk + shared_tokens;
-    const bool slots = rows_buf && rows_buf_bytes >= gemm_tc_workspace_bytes(slot_rows, k);
+    const bool slots = rows_buf && rows_buf_bytes >= gemm_tc_workspace_bytes(slot_rows, k) + size_t(slot_rows) * sizeof(int);
+    int * slot_of = slots ? reinterpret_cast<int *>(static_cast<uint8_t *>(rows_buf) + gemm_tc_workspace_bytes(slot_rows, k)) : nullptr;
     __half * xb = static_cast<__half *>(slots ? rows_buf : ws);
     float * inv = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(xb) + align_up(size_t(slots ? slot_rows : n) * k * 2, 256));
     GemmArgs a{};
@@ -665,7 +731,7 @@ int32_t gemm_tc_gateup(const b2moe_bank * gate, const b2moe_bank * up, const b2m
     if (shared_tokens) { a.saux0 = static_cast<const float *>(sg->aux); a.saux1 = static_cast<const float *>(su->aux); }
     a.plan = const_cast<int *>(plan); a.out = act;
     a.rows = gate->rows; a.k = k; a.experts = gate->experts; a.topk = topk; a.A = n * topk;
-    return gemm_launch<0>(gate->type, a, banks, x, x_dtype, n, slots, slot_rows, xb, inv, s);
+    return gemm_launch<0>(gate->type, a, banks, x, x_dtype, n, slots, slot_rows, xb, inv, slot_of, s);
 }
 
 int32_t gemm_tc_down(const b2moe_bank * down, const b2moe_bank * sd, const float * act, const int * plan, int n, int topk,
@@ -679,7 +745,7 @@ int32_t gemm_tc_down(const b2moe_bank * down, const b2moe_bank * sd, const float
     if (shared_tokens) a.saux0 = static_cast<const float *>(sd->aux);
     a.plan = const_cast<int *>(plan); a.out = y;
     a.rows = down->rows; a.k = k; a.experts = down->experts; a.topk = topk; a.A = n * topk;
-    return gemm_launch<1>(down->type, a, banks, static_cast<const void *>(act), int(B2MOE_F32), rows_x, true, rows_x, xb, inv, s);
+    return gemm_launch<1>(down->type, a, banks, static_cast<const void *>(act), int(B2MOE_F32), rows_x, true, rows_x, xb, inv, static_cast<int *>(nullptr), s);
 }
 
 }  // namespace b2
