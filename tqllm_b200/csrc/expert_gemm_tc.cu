@@ -85,7 +85,7 @@ struct Info { int cum, e, cnt, off; };
 template <uint32_t T>
 constexpr size_t gemm_smem(int experts, int cap, int b_stages, int raw_slots) {
     return 1024 + size_t(b_stages) * cap * 128 + size_t(8) * raw_slots * chunk_bytes<T>() + gdec::Dec<T>::TAB_BYTES +
-           size_t(experts + 2) * sizeof(Info) + 2 * MAX_CAP * sizeof(int2) + size_t(N_BARS) * 8 + 16;
+           DEC_WARPS * gdec::Dec<T>::SCRATCH + size_t(experts + 2) * sizeof(Info) + 2 * MAX_CAP * sizeof(int2) + size_t(N_BARS) * 8 + 16;
 }
 
 // Eight values of an activation row, those of positions 8 l .. 8 l + 7 of a 64-column step (gdec::colmap): they lie in one, two
@@ -215,7 +215,8 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
     uint8_t * b_st = smem;                                            // [b_stages][cap][128 bytes], swizzled
     uint8_t * raw = b_st + size_t(p.b_stages) * p.cap * 128;          // [raw_slots][8 row tiles][CB]
     uint8_t * dec_tab = raw + size_t(8) * p.raw_slots * CB;           // the decoder's lookup table
-    Info * info = reinterpret_cast<Info *>(dec_tab + D::TAB_BYTES);   // [na + 1]
+    uint8_t * dec_scratch = dec_tab + D::TAB_BYTES;                   // [decode warps][SCRATCH]
+    Info * info = reinterpret_cast<Info *>(dec_scratch + DEC_WARPS * D::SCRATCH);   // [na + 1]
     int2 * tok = reinterpret_cast<int2 *>(info + p.experts + 2);      // [2][MAX_CAP]: assignment (-1: none) and activation scale of an item's tokens
     uint64_t * bars = reinterpret_cast<uint64_t *>(tok + 2 * MAX_CAP);
     uint32_t * tmem_slot = reinterpret_cast<uint32_t *>(bars + N_BARS);
@@ -405,6 +406,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
         // ---- A decoder: raw chunks (256 columns of one row tile) -> fp16 operand in tensor memory, unit `part` of every chunk.
         // (Whole chunks in turn instead: the products then came in bursts of two units of one group, and both sides waited.) ----
         const int j = warp - DEC_WARP0, q = j & 3, m = (j >> 2) & 1, part = j >> 3, r = 2 * q + m;      // r: row tile of the block
+        uint8_t * my_scratch = dec_scratch + j * D::SCRATCH;
         const uint8_t * my_raw = raw + size_t(MODE == 0 ? 4 * m + q : r) * CB;
         const uint32_t a_lane = tmem + (uint32_t(32 * q + 16 * m) << 16) + A_COL0;
         uint32_t gu = 0, slot = 0, phase = 0;                          // units before the chunk; ring slot and phase of the chunk
@@ -423,8 +425,9 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
                     typename D::Pre pre;
                     uint32_t f[16];
                     if (live) {
-                        pre = D::prep(chunk, lane, part);
-                        D::template step<0>(chunk, lane, part, dec_tab, pre, f);
+                        pre = D::prep(chunk, lane, part, my_scratch);
+                        if (D::SCRATCH) __syncwarp();
+                        D::template step<0>(chunk, lane, part, dec_tab, my_scratch, pre, f);
                     }
                     // the unit that used the stage before: its second step's products
                     if (g >= A_STAGES && !warp_wait(done + 8 * (2 * sa + 1), ((g / A_STAGES) - 1) & 1u)) { ok = false; break; }
@@ -432,7 +435,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
                         fence_after();
                         tmem_st_16x256b_x4(a_addr, f);
                         if (steps > 1) {
-                            D::template step<1>(chunk, lane, part, dec_tab, pre, f);
+                            D::template step<1>(chunk, lane, part, dec_tab, my_scratch, pre, f);
                             tmem_st_16x256b_x4(a_addr + A_COLS / 2, f);
                         }
                         tmem_st_wait();

@@ -51,6 +51,19 @@ __device__ __forceinline__ void put(uint32_t (&f)[16], int r, int b, const uint4
 // the four words of plane j of a 256-column tile of nibble planes: {row g: word t, word t + 4; row g + 8: the same}
 __device__ __forceinline__ uint4 plane(const uint8_t * chunk, int j, int lane) { return *reinterpret_cast<const uint4 *>(chunk + 512 * j + 16 * lane); }
 
+// (v & mask) | bits in one instruction: it takes one constant as an immediate, so `bits` has to be in a register and look like a
+// variable (with two constants the compiler writes two instructions: 16 more per step of the formats below)
+__device__ __forceinline__ uint32_t in_register(uint32_t v) {
+    uint32_t r;
+    asm volatile("mov.b32 %0, %1;" : "=r"(r) : "r"(v));
+    return r;
+}
+__device__ __forceinline__ uint32_t and_or(uint32_t v, uint32_t mask, uint32_t bits) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(v), "r"(mask), "r"(bits));
+    return r;
+}
+
 template <uint32_t T> struct Dec;
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -63,14 +76,16 @@ template <> struct Dec<T_Q4_K> {
     // of the weight) and + ML, where MH + ML = -dmin m split into two fp16 terms. Rounding the sub-block's d sc or dmin m to
     // one fp16 constant would be cheaper, but that error is shared by the 32 weights of the sub-block and adds up along a
     // row, and rounding t d before the subtraction loses the bits that cancel (both measured: 2.5 to 3 times the output error).
-    __device__ __forceinline__ static uint32_t two(uint32_t nib, __half2 S, __half2 NS, __half2 MH, __half2 ML, __half2 D) {
-        return h2_bits(__hadd2(__hfma2(__hfma2(bits_h2(nib | 0x64006400u), S, NS), D, MH), ML));
+    __device__ __forceinline__ static uint32_t two(uint32_t n1024, __half2 S, __half2 NS, __half2 MH, __half2 ML, __half2 D) {
+        return h2_bits(__hadd2(__hfma2(__hfma2(bits_h2(n1024), S, NS), D, MH), ML));
     }
-    // Once per chunk: lane t of a row's four lanes turns the headers of its two rows into the constants of the unit's sub-block t,
-    // both rows in one register (row g low, row g + 8 high); a step fetches its two sub-blocks from lanes 2 js and 2 js + 1. The
-    // scales and mins are exact as fp16, MH = fp16(-dmin m), ML = the exact rest.
-    struct Pre { uint32_t S, MH, ML, D; };
-    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, int u) {
+    // Once per chunk: lane t of a row's four lanes turns the headers of its two rows into the constants of the unit's sub-block t
+    // and leaves them in the warp's scratch, each twice in a word as the arithmetic takes it: [row][sub-block](S, -1024 S, MH, ML).
+    // The scales and mins are exact as fp16, MH = fp16(-dmin m), ML = the exact rest. (Constants of two rows in one register,
+    // fetched with shuffles and spread with byte permutes, took 45 more instructions a step, 36 of them in the integer pipe.)
+    static constexpr int SCRATCH = 16 * 4 * 16;
+    struct Pre { uint32_t D[2], magic; };
+    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, int u, uint8_t * scratch) {
         const int g = lane >> 2, t = lane & 3;
         const uint4 h0 = *reinterpret_cast<const uint4 *>(chunk + 2048 + 16 * g), h1 = *reinterpret_cast<const uint4 *>(chunk + 2048 + 16 * (g + 8));    // d, dmin | s[12]
         // the unit's four scales and four mins as bytes (src/formats/weight/dequant.cpp:56-64)
@@ -84,36 +99,29 @@ template <> struct Dec<T_Q4_K> {
             const uint32_t v = __byte_perm(x, y, sel);
             return __hadd2(bits_h2((v & 0x003F003Fu) | 0x64006400u), __float2half2_rn(-1024.f));
         };
-        const __half2 sc = pick(sc0, sc1), mn = pick(mn0, mn1);
-        const __half2 dm = bits_h2(__byte_perm(h0.x, h1.x, 0x7632) ^ 0x80008000u);       // -dmin of the two rows
-        Pre p;
-        p.S = h2_bits(t & 1 ? __hmul2(sc, __float2half2_rn(0.0625f)) : sc);
-        const __half2 mh = __hmul2(dm, mn);
-        p.MH = h2_bits(mh);
-        p.ML = h2_bits(__hfma2(dm, mn, __hneg2(mh)));
-        p.D = __byte_perm(h0.x, h1.x, 0x5410);
-        return p;
+        __half2 sc = pick(sc0, sc1);
+        const __half2 mn = pick(mn0, mn1), dm = bits_h2(__byte_perm(h0.x, h1.x, 0x7632) ^ 0x80008000u);       // -dmin of the two rows
+        if (t & 1) sc = __hmul2(sc, __float2half2_rn(0.0625f));
+        const __half2 ns = __hmul2(sc, __float2half2_rn(-1024.f)), mh = __hmul2(dm, mn), ml = __hfma2(dm, mn, __hneg2(mh));
+        uint4 * to = reinterpret_cast<uint4 *>(scratch) + 4 * g + t;
+        to[0] = make_uint4(h2_bits(__low2half2(sc)), h2_bits(__low2half2(ns)), h2_bits(__low2half2(mh)), h2_bits(__low2half2(ml)));
+        to[32] = make_uint4(h2_bits(__high2half2(sc)), h2_bits(__high2half2(ns)), h2_bits(__high2half2(mh)), h2_bits(__high2half2(ml)));
+        return Pre{{__byte_perm(h0.x, 0u, 0x1010), __byte_perm(h1.x, 0u, 0x1010)}, in_register(0x64006400u)};
     }
-    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void *, const Pre & p, uint32_t (&f)[16]) {
-        const int s0 = (lane & ~3) | (2 * JS), s1 = s0 + 1;
+    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void *, const uint8_t * scratch, const Pre & p, uint32_t (&f)[16]) {
         const uint4 w4 = plane(chunk, 2 * u + JS, lane);
-        const uint32_t w[2][2] = {{w4.x, w4.y}, {w4.z, w4.w}};
-        const __half2 neg1024 = __float2half2_rn(-1024.f);
-        const __half2 SA = bits_h2(__shfl_sync(0xffffffffu, p.S, s0)), SB = bits_h2(__shfl_sync(0xffffffffu, p.S, s1));
-        const __half2 MHA = bits_h2(__shfl_sync(0xffffffffu, p.MH, s0)), MHB = bits_h2(__shfl_sync(0xffffffffu, p.MH, s1));
-        const __half2 MLA = bits_h2(__shfl_sync(0xffffffffu, p.ML, s0)), MLB = bits_h2(__shfl_sync(0xffffffffu, p.ML, s1));
-        const __half2 NA = __hmul2(SA, neg1024), NB = __hmul2(SB, neg1024), DD = bits_h2(p.D);
+        const uint4 * c = reinterpret_cast<const uint4 *>(scratch) + 4 * (lane >> 2) + 2 * JS;
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-            auto row = [&](__half2 v) { return r ? __high2half2(v) : __low2half2(v); };
-            const __half2 S0 = row(SA), S1 = row(SB), N0 = row(NA), N1 = row(NB), MH0 = row(MHA), MH1 = row(MHB), ML0 = row(MLA), ML1 = row(MLB), D = row(DD);
+            const uint4 c0 = c[32 * r], c1 = c[32 * r + 1];
+            const __half2 D = bits_h2(p.D[r]);
+            auto lo = [&](uint32_t w) { return two(and_or(w, 0x000F000Fu, p.magic), bits_h2(c0.x), bits_h2(c0.y), bits_h2(c0.z), bits_h2(c0.w), D); };
+            auto hi = [&](uint32_t w) { return two(and_or(w, 0x00F000F0u, p.magic), bits_h2(c1.x), bits_h2(c1.y), bits_h2(c1.z), bits_h2(c1.w), D); };
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
-                const uint32_t v = w[r][b], v8 = v >> 8;
-                put(f, r, b, make_uint4(two(v & 0x000F000Fu, S0, N0, MH0, ML0, D),       // bytes 0 and 2, low nibbles
-                                        two(v8 & 0x000F000Fu, S0, N0, MH0, ML0, D),      // bytes 1 and 3, low nibbles
-                                        two(v & 0x00F000F0u, S1, N1, MH1, ML1, D),       // bytes 0 and 2, high nibbles
-                                        two(v8 & 0x00F000F0u, S1, N1, MH1, ML1, D)));    // bytes 1 and 3, high nibbles
+                const uint32_t v = r ? (b ? w4.w : w4.z) : (b ? w4.y : w4.x), v8 = v >> 8;
+                // bytes 0 and 2, bytes 1 and 3: low nibbles, then high nibbles
+                put(f, r, b, make_uint4(lo(v), lo(v8), hi(v), hi(v8)));
             }
         }
     }
@@ -127,37 +135,39 @@ template <> struct Dec<T_IQ3S4> {
     static constexpr int TAB_BYTES = 0;
     __device__ static void init(void *, int, int) {}
     // the nibbles at bits POS and POS + 16 of w as the half2 (1 + n / 16, 1 + n' / 16)
-    template <int POS> __device__ __forceinline__ static __half2 pair(uint32_t w) {
-        const uint32_t s = POS <= 6 ? w << (6 - POS) : w >> (POS - 6);
-        return bits_h2((s & 0x03C003C0u) | 0x3C003C00u);
+    template <int POS> __device__ __forceinline__ static __half2 pair(uint32_t w, uint32_t one) {
+        return bits_h2(and_or(POS <= 6 ? w << (6 - POS) : w >> (POS - 6), 0x03C003C0u, one));
     }
-    struct Pre { uint32_t sc[2], D; };                                 // the rows' eight 4-bit scales; d of row g, d of row g + 8
-    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, int) {
-        const int g = lane >> 2;
+    // the constants of (row, sub-block) in the warp's scratch, as for Q4_K: (32 (1 + 2 s), -47 (1 + 2 s))
+    static constexpr int SCRATCH = 16 * 4 * 8;
+    struct Pre { uint32_t D[2], one; };
+    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, int u, uint8_t * scratch) {
+        const int g = lane >> 2, t = lane & 3;
         Pre p;
-#pragma unroll
-        for (int r = 0; r < 2; ++r) p.sc[r] = *reinterpret_cast<const uint32_t *>(chunk + 2048 + 4 * (g + 8 * r));
-        p.D = uint32_t(*reinterpret_cast<const unsigned short *>(chunk + 2112 + 2 * g)) |
-              (uint32_t(*reinterpret_cast<const unsigned short *>(chunk + 2112 + 2 * (g + 8))) << 16);
-        return p;
-    }
-    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void *, const Pre & p, uint32_t (&f)[16]) {
-        const int j = 2 * u + JS;
-        const uint4 w4 = plane(chunk, j, lane);
-        const uint32_t w[2][2] = {{w4.x, w4.y}, {w4.z, w4.w}};
+        p.one = in_register(0x3C003C00u);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-            const __half2 D = r ? __high2half2(bits_h2(p.D)) : __low2half2(bits_h2(p.D));
-            // the two scale nibbles of the step side by side under the exponent of 1: (1 + s / 16, 1 + s' / 16), then 1 + 2 s exactly
-            const uint32_t sb = p.sc[r] >> (8 * j);
-            const __half2 s1 = __hfma2(bits_h2(((sb << 6) & 0x03C0u) | ((sb << 18) & 0x03C00000u) | 0x3C003C00u), __float2half2_rn(32.f), __float2half2_rn(-31.f));
-            const __half2 SC = __hmul2(s1, __float2half2_rn(32.f)), CC = __hmul2(s1, __float2half2_rn(-47.f));
-            const __half2 SC1 = __low2half2(SC), C1 = __low2half2(CC), SC2 = __high2half2(SC), C2 = __high2half2(CC);
+            const uint32_t sc = *reinterpret_cast<const uint32_t *>(chunk + 2048 + 4 * (g + 8 * r)) >> (16 * u + 4 * t);
+            // the 4-bit scale under the exponent of 1: 1 + s / 16
+            const __half2 s = bits_h2(((sc & 15u) * 0x00400040u) | 0x3C003C00u);
+            reinterpret_cast<uint2 *>(scratch)[4 * (g + 8 * r) + t] = make_uint2(h2_bits(__hfma2(s, __float2half2_rn(1024.f), __float2half2_rn(-992.f))),
+                                                                               h2_bits(__hfma2(s, __float2half2_rn(-1504.f), __float2half2_rn(1457.f))));
+            p.D[r] = uint32_t(*reinterpret_cast<const unsigned short *>(chunk + 2112 + 2 * (g + 8 * r))) * 0x10001u;
+        }
+        return p;
+    }
+    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void *, const uint8_t * scratch, const Pre & p, uint32_t (&f)[16]) {
+        const uint4 w4 = plane(chunk, 2 * u + JS, lane);
+        const uint4 * c = reinterpret_cast<const uint4 *>(scratch) + 2 * (lane >> 2) + JS;       // both sub-blocks of the step
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const uint4 k = c[16 * r];
+            const __half2 D = bits_h2(p.D[r]), SC1 = bits_h2(k.x), C1 = bits_h2(k.y), SC2 = bits_h2(k.z), C2 = bits_h2(k.w);
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
-                const uint32_t v = w[r][b];
-                put(f, r, b, make_uint4(h2_bits(__hmul2(__hfma2(pair<0>(v), SC1, C1), D)), h2_bits(__hmul2(__hfma2(pair<8>(v), SC1, C1), D)),
-                                        h2_bits(__hmul2(__hfma2(pair<4>(v), SC2, C2), D)), h2_bits(__hmul2(__hfma2(pair<12>(v), SC2, C2), D))));
+                const uint32_t v = r ? (b ? w4.w : w4.z) : (b ? w4.y : w4.x);
+                put(f, r, b, make_uint4(h2_bits(__hmul2(__hfma2(pair<0>(v, p.one), SC1, C1), D)), h2_bits(__hmul2(__hfma2(pair<8>(v, p.one), SC1, C1), D)),
+                                        h2_bits(__hmul2(__hfma2(pair<4>(v, p.one), SC2, C2), D)), h2_bits(__hmul2(__hfma2(pair<12>(v, p.one), SC2, C2), D))));
             }
         }
     }
@@ -193,11 +203,12 @@ __device__ __forceinline__ uint4 lut_word(const Lut & l, uint32_t w, __half2 sca
 }
 
 template <> struct Dec<T_IQ4_XS> {
+    static constexpr int SCRATCH = 0;
     static constexpr int TAB_BYTES = LUT_BYTES;
     __device__ static void init(void * tab, int tid, int n) { build_lut(tab, tid, n); }
     // once per chunk: lane t holds fp16(d (ls - 32)) of the unit's sub-block t, for its two rows
     struct Pre { uint32_t dl; };
-    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, int u) {
+    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, int u, uint8_t *) {
         const int g = lane >> 2, ib = 4 * u + (lane & 3);
         float dl[2];
 #pragma unroll
@@ -209,7 +220,7 @@ template <> struct Dec<T_IQ4_XS> {
         }
         return Pre{pack_h2(dl[0], dl[1])};
     }
-    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void * tab, const Pre & p, uint32_t (&f)[16]) {
+    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void * tab, const uint8_t *, const Pre & p, uint32_t (&f)[16]) {
         const Lut lut = lut_of(tab, lane);
         const uint4 w4 = plane(chunk, 2 * u + JS, lane);
         const int src = (lane & ~3) | (2 * JS);
@@ -222,11 +233,12 @@ template <> struct Dec<T_IQ4_XS> {
 };
 
 template <> struct Dec<T_IQ4_NL> {
+    static constexpr int SCRATCH = 0;
     struct Pre {};
-    __device__ __forceinline__ static Pre prep(const uint8_t *, int, int) { return Pre{}; }
+    __device__ __forceinline__ static Pre prep(const uint8_t *, int, int, uint8_t *) { return Pre{}; }
     static constexpr int TAB_BYTES = LUT_BYTES;
     __device__ static void init(void * tab, int tid, int n) { build_lut(tab, tid, n); }
-    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void * tab, const Pre &, uint32_t (&f)[16]) {
+    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void * tab, const uint8_t *, const Pre &, uint32_t (&f)[16]) {
         const Lut lut = lut_of(tab, lane);
         const int g = lane >> 2;
 #pragma unroll
@@ -242,8 +254,9 @@ template <> struct Dec<T_IQ4_NL> {
 
 // ---------------------------------------------------------------------------------------------------------------
 template <> struct Dec<T_NVFP4G> {
+    static constexpr int SCRATCH = 0;
     struct Pre {};
-    __device__ __forceinline__ static Pre prep(const uint8_t *, int, int) { return Pre{}; }
+    __device__ __forceinline__ static Pre prep(const uint8_t *, int, int, uint8_t *) { return Pre{}; }
     static constexpr int TAB_BYTES = 0;
     __device__ static void init(void *, int, int) {}
     // the eight e2m1 codes of a word -> eight fp16 values (the hardware conversion, two codes per instruction: low nibble
@@ -255,7 +268,7 @@ template <> struct Dec<T_NVFP4G> {
         return make_uint4(h2_bits(__hmul2(bits_h2(v0), scale)), h2_bits(__hmul2(bits_h2(v1), scale)), h2_bits(__hmul2(bits_h2(v2), scale)),
                           h2_bits(__hmul2(bits_h2(v3), scale)));
     }
-    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void *, const Pre &, uint32_t (&f)[16]) {
+    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void *, const uint8_t *, const Pre &, uint32_t (&f)[16]) {
         const int g = lane >> 2, t = lane & 3;
         const uint8_t * tile = chunk + u * Fmt<T_NVFP4G>::TILE;
         constexpr int P = JS;                                            // the unit is one 128-column tile; plane = sub-blocks 2 P, 2 P + 1 of the 128-column tile
@@ -274,8 +287,9 @@ template <> struct Dec<T_NVFP4G> {
 
 // ---------------------------------------------------------------------------------------------------------------
 template <> struct Dec<T_IQ3_S> {
+    static constexpr int SCRATCH = 0;
     struct Pre {};
-    __device__ __forceinline__ static Pre prep(const uint8_t *, int, int) { return Pre{}; }
+    __device__ __forceinline__ static Pre prep(const uint8_t *, int, int, uint8_t *) { return Pre{}; }
     // table: grid entry -> its four odd magnitudes as fp16 (8 bytes)
     static constexpr int TAB_BYTES = 512 * 8;
     __device__ static void init(void * tab, int tid, int n) {
@@ -285,7 +299,7 @@ template <> struct Dec<T_IQ3_S> {
             t2[i] = make_uint2(pack_h2(float(m & 255u), float((m >> 8) & 255u)), pack_h2(float((m >> 16) & 255u), float(m >> 24)));
         }
     }
-    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void * tab, const Pre &, uint32_t (&f)[16]) {
+    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void * tab, const uint8_t *, const Pre &, uint32_t (&f)[16]) {
         if (u == 0) bits_step<JS>(chunk, lane, tab, f);                // the bit positions have to be constants
         else bits_step<2 + JS>(chunk, lane, tab, f);
     }
