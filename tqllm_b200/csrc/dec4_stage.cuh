@@ -1,6 +1,6 @@
 // Staged activation rows of the 4-bit decode kernels (expert_dec4.cu): layout and the device code that writes one row.
 // Rows [R][K] of any dtype -> 16-bit fixed point, the row scaled by a power of two so that the largest magnitude lies
-// in [2^(bits-2), 2^(bits-1)), split into a signed high byte and an unsigned low byte (x16 = 256 hi + lo).
+// in [2^(bits-2), 2^(bits-1)), split into a signed high and a signed low byte (x16 = 256 hi + lo, -128 <= lo < 128).
 // One staged row = K / 32 sub-blocks of 64 bytes + K / 256 records of 32 bytes:
 //   sub-block: for t = 0..3 the 16 bytes {hi of columns 4t..4t+3, hi of 16+4t..16+4t+3, lo of 4t.., lo of 16+4t..}: the
 //              B fragments of the lane with that t for the high-byte and the low-byte MMA;
@@ -75,11 +75,11 @@ __device__ inline float stage_row_lanes(const void * x, size_t first, int k, int
             int q[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) { q[j] = __float2int_rn(v[j] * scale); sum += q[j]; }
-            // byte 1 (high) and byte 0 (low) of four values, in column order
+            // high bytes (of x16 + 128, so that the low byte may count as signed) and low bytes of four values, in column order
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const uint32_t a = uint32_t(q[4 * h]), c = uint32_t(q[4 * h + 1]), d = uint32_t(q[4 * h + 2]), e = uint32_t(q[4 * h + 3]);
-                hi[2 * i + h] = __byte_perm(__byte_perm(a, c, 0x0051), __byte_perm(d, e, 0x0051), 0x5410);
+                hi[2 * i + h] = __byte_perm(__byte_perm(a + 128u, c + 128u, 0x0051), __byte_perm(d + 128u, e + 128u, 0x0051), 0x5410);
                 lo[2 * i + h] = __byte_perm(__byte_perm(a, c, 0x0040), __byte_perm(d, e, 0x0040), 0x5410);
             }
         }

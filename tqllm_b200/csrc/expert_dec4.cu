@@ -6,9 +6,11 @@
 //
 // Arithmetic. A weight of a 32-weight sub-block is an affine function of its 4-bit code n with constants of the (row,
 // sub-block): Q4_K  d sc n - dmin m;  IQ3_S  d (1 + 2 s) (2 n - 15). The activations are brought to 16-bit fixed point
-// per row (a power-of-two scale; 14 or 15 significant bits) and split into a signed high and an unsigned low byte, so
-// that  sum_k n_k x_k  is two integer tensor-core products per sub-block (mma.m16n8k32, u8 x s8 and u8 x u8 -> s32: the
-// masked code words ARE the A fragment, no conversion) and every sum up to the end of a 256-column tile is an exact
+// per row (a power-of-two scale; 14 or 15 significant bits) and split into a signed high and a signed low byte, so
+// that  sum_k n_k x_k  is two integer tensor-core products per sub-block (mma.m16n8k32, u8 x s8 -> s32: the
+// masked code words ARE the A fragment, no conversion; a pass of up to four tokens takes the high bytes as columns 0 .. 3 of
+// one product and the low bytes as columns 4 .. 7, which leaves half the products and half the scaling: most experts of a
+// decode step have one or two tokens) and every sum up to the end of a 256-column tile is an exact
 // integer: the 6-bit / 4-bit sub-block scales multiply as integers, and the offset terms (- dmin m, - 15 d (1 + 2 s))
 // times the activation sum of each sub-block, which the staging kernel takes once per activation row, are one more
 // small MMA per tile (fp16 operands that hold the integer factors and the sums exactly). Two fp32 multiply-adds per
@@ -30,6 +32,8 @@
 // down product then also has one more warp that stages its fp32 activation rows itself (no staging launch).
 // Every wait is bounded; a wait that runs out sets the plan's status word and a block-wide flag, every warp stops at
 // its next wait or item, the producer lets the copies in flight land, and the block leaves.
+#include <type_traits>
+
 #include "common.cuh"
 #include "dec4_stage.cuh"
 #include "formats.cuh"
@@ -72,15 +76,10 @@ __device__ __forceinline__ void mma_f16_zero(float (&c)[4], uint32_t a0, uint32_
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
                  : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
-// m16n8k32 integer MMA, A unsigned bytes, B signed (SB = 1) or unsigned (SB = 0) bytes, C = 0
-template <int SB>
+// m16n8k32 integer MMA, A unsigned bytes, B signed bytes, C = 0
 __device__ __forceinline__ void mma_i8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    if (SB)
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
-                     : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
-    else
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
-                     : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+                 : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
 }
 // Activation staging (layout and row code: dec4_stage.cuh): a warp per row, four rows per block.
 constexpr int STAGE_WARPS = 4;
@@ -241,6 +240,7 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
         const unsigned m1 = __ballot_sync(0xffffffffu, lane * stride < na && passes[i1] <= w);
         const int base = (31 - __clz(int(m1 | 1u))) * stride;                      // passes[0] = 0 <= w always
         int lo = base;
+#pragma unroll 1
         for (int o = 0; o < stride; o += 32) {                                     // second round: the entries of that stretch
             const int i2 = base + o + lane;
             const unsigned m2 = __ballot_sync(0xffffffffu, i2 < min(na, base + stride) && passes[min(i2, na - 1)] <= w);
@@ -254,6 +254,7 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
     // a bounded wait that also gives up when another warp of the block has
     auto wait = [&](uint32_t bar, uint32_t parity) {
         if (mbar_try(bar, parity)) return true;
+#pragma unroll 1
         for (uint32_t i = 0; i < p.wait_limit; ++i) {
             if (mbar_try(bar, parity)) return true;
             if ((i & 63) == 63 && *abort_flag) return false;
@@ -293,6 +294,7 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
         int pass, r0, r1;
         uint32_t idx = 0;
         bool first_staged = false;                         // the first segment's rows are asked for right after its first weight copies
+#pragma unroll 1
         for (long long u = u_begin; u < u_end && ok; u += r1 - r0, ++idx) {
             segment(u, pass, r0, r1);
             int e, c0;
@@ -303,11 +305,13 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
             if (u_next < u_end) segment(u_next, npass, nr0, nr1);
             bool next_staged = p.nbuf != 2 || u_next >= u_end;
             int in_seg = 0;
+#pragma unroll 1
             for (int rb = r0; rb < r1 && ok; rb += JW) {                  // JW row tiles at a time, warp w its part of its own
                 const int rt = rb + w / KSP, k_first = (w % KSP) * kpart;
                 const bool mine = lane < CTA_WARPS && rt < r1;
                 const uint8_t * b0 = (shared ? p.s0 : p.w0 + size_t(e) * p.bank_bytes) + size_t(rt) * p.k_tiles * TILE;
                 const uint8_t * b1 = NMAT == 2 ? (shared ? p.s1 : p.w1 + size_t(e) * p.bank_bytes) + size_t(rt) * p.k_tiles * TILE : b0;
+#pragma unroll 1
                 for (int j = 0; j < nslots && ok; ++j, ++in_seg) {
                     if (mine) {
                         if (issued >= uint32_t(S) && !wait(my_empty + 8 * slot, ((issued / S) - 1) & 1u)) ok = false;
@@ -336,10 +340,12 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
         // waits return at once.
         if (lane < CTA_WARPS) {
             const uint32_t first = issued > uint32_t(S) ? issued - S : 0;
+#pragma unroll 1
             for (uint32_t i = first; i < issued; ++i)
                 if (int(i) != p.drop_tile) wait(my_full + 8 * (i % S), (i / S) & 1u);
         }
         if (!in_kernel && lane == 16)       // the last copy into each activation buffer (an earlier phase of a barrier can no longer be waited for)
+#pragma unroll 1
             for (uint32_t i = xissued > uint32_t(p.nbuf) ? xissued - p.nbuf : 0; i < xissued; ++i)
                 wait(xfull + 8 * (p.nbuf == 2 ? (i & 1u) : 0u), (p.nbuf == 2 ? i >> 1 : i) & 1u);
     } else if (STAGER && warp == CTA_WARPS + 1) {
@@ -348,6 +354,7 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
         const int pass_first = u_begin < u_end ? int(u_begin / row_tiles) : 0;
         const int nseg = u_begin < u_end ? int((u_end - 1) / row_tiles) - pass_first + 1 : 0;
         bool ok = true;
+#pragma unroll 1
         for (int q = 0; q < nseg && ok; ++q) {
             const uint32_t b = p.nbuf == 2 ? (uint32_t(q) & 1u) : 0u, use = p.nbuf == 2 ? uint32_t(q) >> 1 : uint32_t(q);
             if (use > 0 && !__all_sync(0xffffffffu, wait(xempty + 8 * b, (use - 1) & 1u))) { ok = false; break; }   // the consumers are done with the buffer
@@ -355,6 +362,7 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
             locate(pass_first + q, e, c0);
             const int nv = min(PASS_TOKENS, counts[e] - c0);
             const int mine = lane < nv ? perm[offsets[e] + c0 + lane] : -1;
+#pragma unroll 1
             for (int col = 0; col < PASS_TOKENS; ++col) {
                 const int a = __shfl_sync(0xffffffffu, mine, col);
                 float inv = 0.f;
@@ -375,13 +383,16 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
         bool alive = true;
         int pass, r0, r1;
         uint32_t idx = 0;
+#pragma unroll 1
         for (long long u = u_begin; u < u_end && alive; u += r1 - r0, ++idx) {
             segment(u, pass, r0, r1);
             const uint32_t b = p.nbuf == 2 ? (idx & 1u) : 0u, use = p.nbuf == 2 ? idx >> 1 : idx;
             if (*abort_flag) break;
             if (!__all_sync(0xffffffffu, wait(xfull + 8 * b, use & 1u))) { alive = false; break; }
-            const uint8_t * xw = xs + b * xbuf + g * xrow + t * 16;          // + sub-block * 64
-            const uint8_t * rec = xs + b * xbuf + g * xrow + size_t(K) * 2 + t * 8;   // + tile * 32
+            const bool quad = meta[b].col_a[4] < 0;                          // up to four tokens: high bytes as columns 0 .. 3, low bytes as 4 .. 7
+            const int xr = quad ? g & 3 : g;
+            const uint8_t * xw = xs + b * xbuf + xr * xrow + t * 16 + (quad && g >= 4 ? 8 : 0);      // + sub-block * 64
+            const uint8_t * rec = xs + b * xbuf + xr * xrow + size_t(K) * 2 + t * 8;  // + tile * 32
             // the lane's two token columns (2t, 2t + 1): assignment index and inverse activation scale, as the producer left them
             int col_a[2];
             float col_is[2];
@@ -389,6 +400,7 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
             for (int q = 0; q < 2; ++q) { col_a[q] = meta[b].col_a[2 * t + q]; col_is[q] = meta[b].col_is[2 * t + q]; }
 
             const int grp = warp / KSP, part = warp % KSP;                  // row-job slot of this warp and its part of the columns
+#pragma unroll 1
             for (int rt = r0 + grp; rt < r1 && alive; rt += JW) {
                 float acc[NMAT][4];
 #pragma unroll
@@ -396,52 +408,76 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
 #pragma unroll
                     for (int i = 0; i < 4; ++i) acc[m][i] = 0.f;
 
-                for (int ks = part * kpart; ks < (part + 1) * kpart && alive; ++ks) {
-                    const int nt = min(SLOT_TILES, p.k_tiles - ks * SLOT_TILES);
+                auto columns = [&](auto Q) {
+                    constexpr bool QUAD = decltype(Q)::value;
+#pragma unroll 1
+                    for (int ks = part * kpart; ks < (part + 1) * kpart && alive; ++ks) {
+                        const int nt = min(SLOT_TILES, p.k_tiles - ks * SLOT_TILES);
 #pragma unroll
-                    for (int m = 0; m < NMAT; ++m) {
-                        if (!__all_sync(0xffffffffu, wait(my_full + 8 * c_slot, c_phase))) { alive = false; break; }
-                        for (int kk = 0; kk < nt; ++kk) {
-                            const int kt = ks * SLOT_TILES + kk;
-                            const uint8_t * tile = my_ring + c_slot * SLOT + kk * TILE;
-                            // the sub-block sums of this tile's columns: B fragment of the correction MMA
-                            const uint2 sp = *reinterpret_cast<const uint2 *>(rec + kt * 32);
-                            const uint4 * xk = reinterpret_cast<const uint4 *>(xw + kt * 512);
-                            Hdr4 hdr;
-                            F::load(hdr, tile, lane);
-                            int main_[4] = {0, 0, 0, 0};
+                        for (int m = 0; m < NMAT; ++m) {
+                            if (!__all_sync(0xffffffffu, wait(my_full + 8 * c_slot, c_phase))) { alive = false; break; }
+#pragma unroll 1
+                            for (int kk = 0; kk < nt; ++kk) {
+                                const int kt = ks * SLOT_TILES + kk;
+                                const uint8_t * tile = my_ring + c_slot * SLOT + kk * TILE;
+                                // the sub-block sums of this tile's columns: B fragment of the correction MMA (the low-byte columns have none)
+                                uint2 sp = *reinterpret_cast<const uint2 *>(rec + kt * 32);
+                                if (QUAD && g >= 4) sp = make_uint2(0u, 0u);
+                                const uint8_t * xk = xw + kt * 512;                // + sub-block * 64
+                                Hdr4 hdr;
+                                F::load(hdr, tile, lane);
+                                int main_[4] = {0, 0, 0, 0};
 #pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                const uint4 pl = reinterpret_cast<const uint4 *>(tile + 512 * q)[lane];
+                                for (int q = 0; q < 4; ++q) {
+                                    const uint4 pl = reinterpret_cast<const uint4 *>(tile + 512 * q)[lane];
 #pragma unroll
-                                for (int half = 0; half < 2; ++half) {                     // sub-block 2q (low nibbles), 2q + 1 (high nibbles)
-                                    const uint32_t a0 = (half ? pl.x >> 4 : pl.x) & 0x0F0F0F0Fu, a2 = (half ? pl.y >> 4 : pl.y) & 0x0F0F0F0Fu;
-                                    const uint32_t a1 = (half ? pl.z >> 4 : pl.z) & 0x0F0F0F0Fu, a3 = (half ? pl.w >> 4 : pl.w) & 0x0F0F0F0Fu;
-                                    const uint4 xv = xk[(2 * q + half) * 4];             // dead token columns read stale rows: they feed dead C columns only
-                                    int rh[4], rl[4];
-                                    mma_i8<1>(rh, a0, a1, a2, a3, xv.x, xv.y);             // high bytes of the activations (signed)
-                                    mma_i8<0>(rl, a0, a1, a2, a3, xv.z, xv.w);             // low bytes (unsigned)
-                                    const int s0 = int(__byte_perm(hdr.isc[0][half], 0u, 0x4440 + q)), s8 = int(__byte_perm(hdr.isc[1][half], 0u, 0x4440 + q));
-                                    main_[0] += s0 * (rh[0] * 256 + rl[0]); main_[1] += s0 * (rh[1] * 256 + rl[1]);
-                                    main_[2] += s8 * (rh[2] * 256 + rl[2]); main_[3] += s8 * (rh[3] * 256 + rl[3]);
+                                    for (int half = 0; half < 2; ++half) {             // sub-block 2q (low nibbles), 2q + 1 (high nibbles)
+                                        const uint32_t a0 = (half ? pl.x >> 4 : pl.x) & 0x0F0F0F0Fu, a2 = (half ? pl.y >> 4 : pl.y) & 0x0F0F0F0Fu;
+                                        const uint32_t a1 = (half ? pl.z >> 4 : pl.z) & 0x0F0F0F0Fu, a3 = (half ? pl.w >> 4 : pl.w) & 0x0F0F0F0Fu;
+                                        const int s0 = int(__byte_perm(hdr.isc[0][half], 0u, 0x4440 + q)), s8 = int(__byte_perm(hdr.isc[1][half], 0u, 0x4440 + q));
+                                        // dead token columns read stale rows: they feed dead C columns only
+                                        if constexpr (QUAD) {
+                                            const uint2 xv = *reinterpret_cast<const uint2 *>(xk + (2 * q + half) * 64);
+                                            int r[4];
+                                            mma_i8(r, a0, a1, a2, a3, xv.x, xv.y);
+                                            main_[0] += s0 * r[0]; main_[1] += s0 * r[1];
+                                            main_[2] += s8 * r[2]; main_[3] += s8 * r[3];
+                                        } else {
+                                            const uint4 xv = *reinterpret_cast<const uint4 *>(xk + (2 * q + half) * 64);
+                                            int rh[4], rl[4];
+                                            mma_i8(rh, a0, a1, a2, a3, xv.x, xv.y);        // high bytes of the activations
+                                            mma_i8(rl, a0, a1, a2, a3, xv.z, xv.w);        // low bytes
+                                            main_[0] += s0 * (rh[0] * 256 + rl[0]); main_[1] += s0 * (rh[1] * 256 + rl[1]);
+                                            main_[2] += s8 * (rh[2] * 256 + rl[2]); main_[3] += s8 * (rh[3] * 256 + rl[3]);
+                                        }
+                                    }
+                                    if (!QUAD && F::FLUSH_AT == q) {   // keep `main` inside 32 bits: hand the first half of the tile over now
+#pragma unroll
+                                        for (int i = 0; i < 4; ++i) { acc[m][i] = fmaf(hdr.f_main[i >> 1], float(main_[i]), acc[m][i]); main_[i] = 0; }
+                                    }
                                 }
-                                if (F::FLUSH_AT == q) {      // keep `main` inside 32 bits: hand the first half of the tile over now
+                                float corr[4];
+                                mma_f16_zero(corr, hdr.ca[0], hdr.ca[1], hdr.ca[2], hdr.ca[3], sp.x, sp.y);
+                                // QUAD: in units of 256 for the high-byte columns (which carry the correction), of 1 for the others
 #pragma unroll
-                                    for (int i = 0; i < 4; ++i) { acc[m][i] = fmaf(hdr.f_main[i >> 1], float(main_[i]), acc[m][i]); main_[i] = 0; }
-                                }
+                                for (int i = 0; i < 4; ++i)
+                                    acc[m][i] = fmaf(hdr.f_main[i >> 1], float(main_[i]), fmaf(QUAD ? hdr.f_corr[i >> 1] * 0x1p-8f : hdr.f_corr[i >> 1], corr[i], acc[m][i]));
                             }
-                            float corr[4];
-                            mma_f16_zero(corr, hdr.ca[0], hdr.ca[1], hdr.ca[2], hdr.ca[3], sp.x, sp.y);
-#pragma unroll
-                            for (int i = 0; i < 4; ++i)
-                                acc[m][i] = fmaf(hdr.f_main[i >> 1], float(main_[i]), fmaf(hdr.f_corr[i >> 1], corr[i], acc[m][i]));
+                            __syncwarp();             // every lane has read its words: the slot can be refilled
+                            if (lane == 0) mbar_arrive(my_empty + 8 * c_slot);
+                            c_slot = c_slot + 1 == uint32_t(S) ? 0 : c_slot + 1;
+                            c_phase ^= c_slot == 0 ? 1u : 0u;
                         }
-                        __syncwarp();             // every lane has read its words: the slot can be refilled
-                        if (lane == 0) mbar_arrive(my_empty + 8 * c_slot);
-                        c_slot = c_slot + 1 == uint32_t(S) ? 0 : c_slot + 1;
-                        c_phase ^= c_slot == 0 ? 1u : 0u;
                     }
-                }
+                    if constexpr (QUAD) {                               // lane t < 2: tokens 2 t, 2 t + 1 = 256 x (columns 2 t, 2 t + 1) + (columns 2 t + 4, 2 t + 5)
+#pragma unroll
+                        for (int m = 0; m < NMAT; ++m)
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) acc[m][i] = fmaf(256.f, acc[m][i], __shfl_xor_sync(0xffffffffu, acc[m][i], 2));
+                    }
+                };
+                if (quad) columns(std::true_type{});
+                else columns(std::false_type{});
                 if (!alive) break;
                 if (KSP > 1) {
                     // the parts of the row job meet in shared memory: every warp leaves its sums, part 0 adds them in part order
@@ -460,6 +496,7 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
                     }
                     if (lane == 0) mbar_arrive(red_full + 8 * grp);
                     if (!__all_sync(0xffffffffu, wait(red_full + 8 * grp, red_use & 1u))) { alive = false; break; }
+#pragma unroll 1
                     for (int o = 1; o < KSP; ++o)
 #pragma unroll
                         for (int m = 0; m < NMAT; ++m)
