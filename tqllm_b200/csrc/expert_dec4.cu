@@ -158,7 +158,9 @@ struct Dec4Args {
     const float * x_raw;                     // MODE 1: the fp32 activation rows [A + shared][k], staged inside the kernel
     const float * inv_scale;                 // [rows_x]
     int * plan;
-    float * out;                             // [A + shared][rows]
+    void * out;                              // [A + shared][rows] of out_dtype
+    int out_dtype;
+    int x_per_token;                         // MODE 1: the staged rows are one per token, not one per assignment
     int rows, k_tiles, experts, topk, A, nbuf, stages, slot_tiles;
     int passes_bound;                        // host: an upper bound of the plan's pass count, from the call's shape
     int ksplit;                              // consumer warps that share one row job, each taking 1 / ksplit of its columns (1, 2 or 4)
@@ -250,7 +252,7 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
         c0 = (w - passes[lo]) * PASS_TOKENS;
     };
     constexpr bool in_kernel = STAGER;                             // the down product stages its rows itself (small launches)
-    auto x_row = [&](int a) { return MODE == 0 ? size_t(a < p.A ? a / p.topk : a - p.A) : size_t(a); };
+    auto x_row = [&](int a) { return MODE == 0 || p.x_per_token ? size_t(a < p.A ? a / p.topk : a - p.A) : size_t(a); };
     // a bounded wait that also gives up when another warp of the block has
     auto wait = [&](uint32_t bar, uint32_t parity) {
         if (mbar_try(bar, parity)) return true;
@@ -410,6 +412,9 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
 
                 auto columns = [&](auto Q) {
                     constexpr bool QUAD = decltype(Q)::value;
+                    // QUAD: lane t < 2 meets the low-byte sums of its tokens, which lane t + 2 holds (whose own result means nothing), so
+                    // that a token's sums are the same integers, and its result the same bits, in a pass of either form
+                    auto whole = [&](int v) { return QUAD ? int(uint32_t(v) * 256u + uint32_t(__shfl_xor_sync(0xffffffffu, v, 2))) : v; };
 #pragma unroll 1
                     for (int ks = part * kpart; ks < (part + 1) * kpart && alive; ++ks) {
                         const int nt = min(SLOT_TILES, p.k_tiles - ks * SLOT_TILES);
@@ -420,9 +425,8 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
                             for (int kk = 0; kk < nt; ++kk) {
                                 const int kt = ks * SLOT_TILES + kk;
                                 const uint8_t * tile = my_ring + c_slot * SLOT + kk * TILE;
-                                // the sub-block sums of this tile's columns: B fragment of the correction MMA (the low-byte columns have none)
-                                uint2 sp = *reinterpret_cast<const uint2 *>(rec + kt * 32);
-                                if (QUAD && g >= 4) sp = make_uint2(0u, 0u);
+                                // the sub-block sums of this tile's columns: B fragment of the correction MMA
+                                const uint2 sp = *reinterpret_cast<const uint2 *>(rec + kt * 32);
                                 const uint8_t * xk = xw + kt * 512;                // + sub-block * 64
                                 Hdr4 hdr;
                                 F::load(hdr, tile, lane);
@@ -451,29 +455,22 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
                                             main_[2] += s8 * (rh[2] * 256 + rl[2]); main_[3] += s8 * (rh[3] * 256 + rl[3]);
                                         }
                                     }
-                                    if (!QUAD && F::FLUSH_AT == q) {   // keep `main` inside 32 bits: hand the first half of the tile over now
+                                    if (F::FLUSH_AT == q) {            // keep `main` inside 32 bits: hand the first half of the tile over now
 #pragma unroll
-                                        for (int i = 0; i < 4; ++i) { acc[m][i] = fmaf(hdr.f_main[i >> 1], float(main_[i]), acc[m][i]); main_[i] = 0; }
+                                        for (int i = 0; i < 4; ++i) { acc[m][i] = fmaf(hdr.f_main[i >> 1], float(whole(main_[i])), acc[m][i]); main_[i] = 0; }
                                     }
                                 }
                                 float corr[4];
                                 mma_f16_zero(corr, hdr.ca[0], hdr.ca[1], hdr.ca[2], hdr.ca[3], sp.x, sp.y);
-                                // QUAD: in units of 256 for the high-byte columns (which carry the correction), of 1 for the others
 #pragma unroll
                                 for (int i = 0; i < 4; ++i)
-                                    acc[m][i] = fmaf(hdr.f_main[i >> 1], float(main_[i]), fmaf(QUAD ? hdr.f_corr[i >> 1] * 0x1p-8f : hdr.f_corr[i >> 1], corr[i], acc[m][i]));
+                                    acc[m][i] = fmaf(hdr.f_main[i >> 1], float(whole(main_[i])), fmaf(hdr.f_corr[i >> 1], corr[i], acc[m][i]));
                             }
                             __syncwarp();             // every lane has read its words: the slot can be refilled
                             if (lane == 0) mbar_arrive(my_empty + 8 * c_slot);
                             c_slot = c_slot + 1 == uint32_t(S) ? 0 : c_slot + 1;
                             c_phase ^= c_slot == 0 ? 1u : 0u;
                         }
-                    }
-                    if constexpr (QUAD) {                               // lane t < 2: tokens 2 t, 2 t + 1 = 256 x (columns 2 t, 2 t + 1) + (columns 2 t + 4, 2 t + 5)
-#pragma unroll
-                        for (int m = 0; m < NMAT; ++m)
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) acc[m][i] = fmaf(256.f, acc[m][i], __shfl_xor_sync(0xffffffffu, acc[m][i], 2));
                     }
                 };
                 if (quad) columns(std::true_type{});
@@ -517,7 +514,7 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
                         const int row = 16 * rt + g + 8 * h;
                         if (row >= p.rows) continue;
                         const float v0 = acc[0][2 * h + q] * is, v1 = acc[NMAT - 1][2 * h + q] * is;
-                        p.out[size_t(a) * p.rows + row] = MODE == 0 ? (v0 / (1.f + expf(-v0))) * v1 : v0;
+                        store_act(p.out, p.out_dtype, size_t(a) * p.rows + row, MODE == 0 ? (v0 / (1.f + expf(-v0))) * v1 : v0);
                     }
                 }
             }
@@ -597,35 +594,36 @@ int32_t stage(Dec4Args & a, const void * x, int dtype, int rows_x, int k, void *
 
 template <uint32_t T>
 int32_t gateup_t(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_bank * sg, const b2moe_bank * su, const void * x, int x_dtype,
-                 const int * plan, int n, int topk, int shared_tokens, float * act, void * ws, int max_active, cudaStream_t s, bool x_staged) {
+                 const int * plan, int n, int topk, int shared_tokens, void * act, int act_dtype, void * ws, cudaStream_t s, bool x_staged) {
     const int k = gate->cols;
     Dec4Args a{};
     if (int32_t rc = stage<T>(a, x, x_dtype, n, k, ws, s, x_staged)) return rc;
     a.w0 = static_cast<const uint8_t *>(gate->data); a.w1 = static_cast<const uint8_t *>(up->data);
     if (shared_tokens) { a.s0 = static_cast<const uint8_t *>(sg->data); a.s1 = static_cast<const uint8_t *>(su->data); }
     a.bank_bytes = b2moe_bank_bytes(gate->type, gate->rows, gate->cols);
-    a.plan = const_cast<int *>(plan); a.out = act;
+    a.plan = const_cast<int *>(plan); a.out = act; a.out_dtype = act_dtype;
     a.rows = gate->rows; a.k_tiles = k / 256; a.experts = gate->experts; a.topk = topk; a.A = n * topk;
     a.passes_bound = n * topk + (shared_tokens + PASS_TOKENS - 1) / PASS_TOKENS;
     return launch_dec4<T, 0>(a, s);
 }
 template <uint32_t T>
-int32_t down_t(const b2moe_bank * down, const b2moe_bank * sd, const float * act, const int * plan, int n, int topk, int shared_tokens,
-               float * y, void * ws, int max_active, cudaStream_t s) {
-    const int rows_x = n * topk + shared_tokens, k = down->cols;
+int32_t down_t(const b2moe_bank * down, const b2moe_bank * sd, const void * x, int x_dtype, bool per_token, const int * plan, int n, int topk,
+               int shared_tokens, void * y, int y_dtype, void * ws, cudaStream_t s) {
+    const int rows_x = per_token ? n : n * topk + shared_tokens, k = down->cols;
     Dec4Args a{};
     // A launch of a few jobs per block is a chain of latencies: its rows are staged inside the kernel by a warp of their own
     // (one launch less). A full launch keeps the staging kernel: measured at 64 tokens the in-kernel staging costs 11 us more
     // than the launch it saves (the staging warp shares a scheduler with five busy warps).
     const long long jobs_bound = (long long)(n * topk + (shared_tokens + PASS_TOKENS - 1) / PASS_TOKENS) * ((down->rows + 15) / 16);
     const int sms = sm_count();
-    const bool in_kernel = sms > 0 && jobs_bound <= 24LL * sms && !g_skip_stage;
-    if (in_kernel) a.x_raw = act;
-    else if (int32_t rc = stage<T>(a, act, B2MOE_F32, rows_x, k, ws, s)) return rc;
+    const bool in_kernel = sms > 0 && jobs_bound <= 24LL * sms && !g_skip_stage && x_dtype == B2MOE_F32 && !per_token;
+    a.x_per_token = per_token;
+    if (in_kernel) a.x_raw = static_cast<const float *>(x);
+    else if (int32_t rc = stage<T>(a, x, x_dtype, rows_x, k, ws, s)) return rc;
     a.w0 = static_cast<const uint8_t *>(down->data);
     if (shared_tokens) a.s0 = static_cast<const uint8_t *>(sd->data);
     a.bank_bytes = b2moe_bank_bytes(down->type, down->rows, down->cols);
-    a.plan = const_cast<int *>(plan); a.out = y;
+    a.plan = const_cast<int *>(plan); a.out = y; a.out_dtype = y_dtype;
     a.rows = down->rows; a.k_tiles = k / 256; a.experts = down->experts; a.topk = topk; a.A = n * topk;
     a.passes_bound = n * topk + (shared_tokens + PASS_TOKENS - 1) / PASS_TOKENS;
     return in_kernel ? launch_dec4<T, 1, true>(a, s) : launch_dec4<T, 1>(a, s);
@@ -646,16 +644,16 @@ size_t dec4_workspace_bytes(int rows_x, int k) {
     return staged_bytes(rows_x, k) + align_up(size_t(rows_x) * sizeof(float), 256);
 }
 int32_t dec4_gateup(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_bank * sg, const b2moe_bank * su, const void * x,
-                    int x_dtype, const int * plan, int n, int topk, int shared_tokens, float * act, void * ws, int max_active,
+                    int x_dtype, const int * plan, int n, int topk, int shared_tokens, void * act, int act_dtype, void * ws,
                     cudaStream_t s, bool x_staged) {
-    if (gate->type == T_Q4_K) return gateup_t<T_Q4_K>(gate, up, sg, su, x, x_dtype, plan, n, topk, shared_tokens, act, ws, max_active, s, x_staged);
-    if (gate->type == T_IQ3S4) return gateup_t<T_IQ3S4>(gate, up, sg, su, x, x_dtype, plan, n, topk, shared_tokens, act, ws, max_active, s, x_staged);
+    if (gate->type == T_Q4_K) return gateup_t<T_Q4_K>(gate, up, sg, su, x, x_dtype, plan, n, topk, shared_tokens, act, act_dtype, ws, s, x_staged);
+    if (gate->type == T_IQ3S4) return gateup_t<T_IQ3S4>(gate, up, sg, su, x, x_dtype, plan, n, topk, shared_tokens, act, act_dtype, ws, s, x_staged);
     return B2MOE_ERR_FORMAT;
 }
-int32_t dec4_down(const b2moe_bank * down, const b2moe_bank * sd, const float * act, const int * plan, int n, int topk,
-                  int shared_tokens, float * y, void * ws, int max_active, cudaStream_t s) {
-    if (down->type == T_Q4_K) return down_t<T_Q4_K>(down, sd, act, plan, n, topk, shared_tokens, y, ws, max_active, s);
-    if (down->type == T_IQ3S4) return down_t<T_IQ3S4>(down, sd, act, plan, n, topk, shared_tokens, y, ws, max_active, s);
+int32_t dec4_down(const b2moe_bank * down, const b2moe_bank * sd, const void * x, int x_dtype, bool per_token, const int * plan, int n, int topk,
+                  int shared_tokens, void * y, int y_dtype, void * ws, cudaStream_t s) {
+    if (down->type == T_Q4_K) return down_t<T_Q4_K>(down, sd, x, x_dtype, per_token, plan, n, topk, shared_tokens, y, y_dtype, ws, s);
+    if (down->type == T_IQ3S4) return down_t<T_IQ3S4>(down, sd, x, x_dtype, per_token, plan, n, topk, shared_tokens, y, y_dtype, ws, s);
     return B2MOE_ERR_FORMAT;
 }
 void dec4_skip_staging(bool on) { g_skip_stage = on; }

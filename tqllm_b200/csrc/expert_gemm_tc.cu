@@ -64,7 +64,8 @@ struct GemmArgs {
     const float * aux0, * aux1, * saux0, * saux1;      // row scales of the banks (gate, up) or (down, -) and of the shared expert's (may be null)
     const float * inv_scale;                // per activation row (the fp16 rows themselves come through the tensor maps)
     int * plan;
-    float * out;
+    void * out;                             // [assignments][rows] of out_dtype
+    int out_dtype;
     int rows, k, experts, topk, A;
     int cap, cap_log2, b_stages, raw_slots; // most tokens of an item; B stages; raw chunks in the ring
     int b_pair;                             // 1: the B stages are filled and freed a unit at a time, beside the A stage of the unit and through its barriers (b_stages = 2 A_STAGES)
@@ -310,7 +311,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
         const int q = warp & 3, tid = threadIdx.x - EPI_WARP0 * 32, first = 16 * ((warp - EPI_WARP0) >> 2);
         const bool upper = lane >= 16;
         constexpr bool ROW_SCALE = T == T_NVFP4G;
-        const uint32_t row_bytes = uint32_t(p.rows) * 4u;
+        const uint32_t out_size = p.out_dtype == B2MOE_F32 ? 4u : 2u, row_bytes = uint32_t(p.rows) * out_size;
         int2 mine;
         auto fetch = [&](const Item & im) {                            // this thread's token of the item
             mine = make_int2(-1, 0);
@@ -348,9 +349,10 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
             fence_after();
             const uint32_t taddr = tmem + (uint32_t(32 * q) << 16) + h * ACC_COLS;
             const int4 * t = reinterpret_cast<const int4 *>(tok + (ic & 1u) * MAX_CAP);
-            char * const out = reinterpret_cast<char *>(p.out + row);
+            char * const out = static_cast<char *>(p.out) + row * out_size;
             const bool in = row < p.rows;
             auto store = [&](int a, float y) { if (in && a >= 0) *reinterpret_cast<float *>(out + uint64_t(uint32_t(a)) * row_bytes) = y; };
+            auto store_short = [&](int a, float y) { if (in && a >= 0) store_act(out + uint64_t(uint32_t(a)) * row_bytes, p.out_dtype, 0, y); };
 #pragma unroll 1
             for (int c = first; c < im.nv; c += 32) {
                 uint32_t v[16];
@@ -381,14 +383,20 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
                             const float gv = (upper ? other : v0) * is, uv = (upper ? v1 : other) * is;
                             res[i] = __fdividef(gv, 1.f + __expf(-gv)) * uv;      // fast exp and divide: relative error about 2^-21
                         }
+                        if (out_size == 4u) {
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) store(upper ? two[i].z : two[i].x, res[i]);
+                            for (int i = 0; i < 4; ++i) store(upper ? two[i].z : two[i].x, res[i]);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) store_short(upper ? two[i].z : two[i].x, res[i]);
+                        }
                     } else {
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             const float is0 = __int_as_float(two[i].y), is1 = __int_as_float(two[i].w);
-                            store(two[i].x, __uint_as_float(v[j0 + 2 * i]) * (ROW_SCALE ? is0 * rs : is0));
-                            store(two[i].z, __uint_as_float(v[j0 + 2 * i + 1]) * (ROW_SCALE ? is1 * rs : is1));
+                            const float y0 = __uint_as_float(v[j0 + 2 * i]) * (ROW_SCALE ? is0 * rs : is0), y1 = __uint_as_float(v[j0 + 2 * i + 1]) * (ROW_SCALE ? is1 * rs : is1);
+                            if (out_size == 4u) { store(two[i].x, y0); store(two[i].z, y1); }
+                            else { store_short(two[i].x, y0); store_short(two[i].z, y1); }
                         }
                     }
                 }
@@ -645,7 +653,7 @@ int32_t convert_rows_dt(const void * xv, int rows_x, int slot_rows, bool slots, 
     const dim3 block(256);
     if (!slots) {
         launch_overlapped(rows_to_f16_k<T, DT>, dim3(ceil_div(rows_x, 8)), block, 0, s, x, rows_x, a.k, out, inv);
-    } else if (topk > 1 && topk < 32 && slot_rows >= TOKEN_WISE_SLOTS) {
+    } else if (slot_of && topk > 1 && topk < 32 && slot_rows >= TOKEN_WISE_SLOTS) {
         launch_overlapped(slot_of_k, dim3(ceil_div(slot_rows, 256)), block, 0, s, plan, a.experts, slot_of);
         if (int32_t rc = launch_status()) return rc;
         launch_overlapped(tokens_to_slots_k<T, DT>, dim3(ceil_div(rows_x, 8)), block, 0, s, x, plan, slot_of, a.experts, rows_x, topk, int(slot_rows > a.A), a.k, out, inv);
@@ -654,17 +662,17 @@ int32_t convert_rows_dt(const void * xv, int rows_x, int slot_rows, bool slots, 
     }
     return launch_status();
 }
-// m: the banks (gate, up) or (down, null), then the shared expert's (null: none); x (rows_x rows, in token order for MODE 0, in
-// assignment order for MODE 1) -> fp16 rows in xb (in slot order: slot_rows of them; slot_of: scratch for MODE 0), then the product
+// m: the banks (gate, up) or (down, null), then the shared expert's (null: none); x (rows_x rows, in token order when map_topk > 0, in
+// assignment order otherwise) -> fp16 rows in xb (in slot order: slot_rows of them; slot_of: scratch for MODE 0), then the product
 template <uint32_t T, int MODE>
-int32_t gemm_launch_t(GemmArgs a, const b2moe_bank * const * m, const void * x, int dtype, int rows_x, bool slots, int slot_rows, __half * xb, float * inv, int * slot_of,
+int32_t gemm_launch_t(GemmArgs a, const b2moe_bank * const * m, const void * x, int dtype, int rows_x, int map_topk, bool slots, int slot_rows, __half * xb, float * inv, int * slot_of,
                       cudaStream_t s) {
     const int sms = gemm_sm_count();
     if (sms <= 0) return B2MOE_ERR_CUDA;
     const long long per = (long long)a.A / a.experts;                 // mean tokens per expert
     const int cap = g_item_tokens == 256 || per > 128 ? 256 : per > 24 ? 128 : 64;
     if (!gemm_fit<T>(a.experts, cap, a)) return B2MOE_ERR_SHAPE;
-    const int rows = slots ? slot_rows : rows_x, topk = MODE == 0 ? a.topk : 0;
+    const int rows = slots ? slot_rows : rows_x, topk = map_topk;
     int32_t rc = B2MOE_ERR_SHAPE;
     if (dtype == B2MOE_F32) rc = convert_rows_dt<T, B2MOE_F32>(x, rows_x, slot_rows, slots, topk, a, xb, inv, slot_of, s);
     else if (dtype == B2MOE_F16) rc = convert_rows_dt<T, B2MOE_F16>(x, rows_x, slot_rows, slots, topk, a, xb, inv, slot_of, s);
@@ -721,7 +729,7 @@ size_t gemm_tc_workspace_bytes(int rows_x, int k) {
 
 // rows_buf: optional scratch for the activation rows in slot order (n * topk + shared_tokens rows of length k, their scales and an index each)
 int32_t gemm_tc_gateup(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_bank * sg, const b2moe_bank * su, const void * x,
-                       int x_dtype, const int * plan, int n, int topk, int shared_tokens, float * act, void * ws, void * rows_buf,
+                       int x_dtype, const int * plan, int n, int topk, int shared_tokens, void * act, int act_dtype, void * ws, void * rows_buf,
                        size_t rows_buf_bytes, cudaStream_t s) {
     const int k = gate->cols, slot_rows = n * topk + shared_tokens;
     const bool slots = rows_buf && rows_buf_bytes >= gemm_tc_workspace_bytes(slot_rows, k) + size_t(slot_rows) * sizeof(int);
@@ -732,13 +740,14 @@ int32_t gemm_tc_gateup(const b2moe_bank * gate, const b2moe_bank * up, const b2m
     const b2moe_bank * banks[4] = {gate, up, shared_tokens ? sg : nullptr, shared_tokens ? su : nullptr};
     a.aux0 = static_cast<const float *>(gate->aux); a.aux1 = static_cast<const float *>(up->aux);
     if (shared_tokens) { a.saux0 = static_cast<const float *>(sg->aux); a.saux1 = static_cast<const float *>(su->aux); }
-    a.plan = const_cast<int *>(plan); a.out = act;
+    a.plan = const_cast<int *>(plan); a.out = act; a.out_dtype = act_dtype;
     a.rows = gate->rows; a.k = k; a.experts = gate->experts; a.topk = topk; a.A = n * topk;
-    return gemm_launch<0>(gate->type, a, banks, x, x_dtype, n, slots, slot_rows, xb, inv, slot_of, s);
+    return gemm_launch<0>(gate->type, a, banks, x, x_dtype, n, topk, slots, slot_rows, xb, inv, slot_of, s);
 }
 
-int32_t gemm_tc_down(const b2moe_bank * down, const b2moe_bank * sd, const float * act, const int * plan, int n, int topk,
-                     int shared_tokens, float * y, void * ws, cudaStream_t s) {
+// per_token: x has a row per token instead of one per assignment (shared_tokens = 0)
+int32_t gemm_tc_down(const b2moe_bank * down, const b2moe_bank * sd, const void * x, int x_dtype, bool per_token, const int * plan, int n, int topk,
+                     int shared_tokens, void * y, int y_dtype, void * ws, cudaStream_t s) {
     const int rows_x = n * topk + shared_tokens, k = down->cols;
     __half * xb = static_cast<__half *>(ws);
     float * inv = reinterpret_cast<float *>(static_cast<uint8_t *>(ws) + align_up(size_t(rows_x) * k * 2, 256));
@@ -746,9 +755,9 @@ int32_t gemm_tc_down(const b2moe_bank * down, const b2moe_bank * sd, const float
     const b2moe_bank * banks[4] = {down, nullptr, shared_tokens ? sd : nullptr, nullptr};
     a.aux0 = static_cast<const float *>(down->aux);
     if (shared_tokens) a.saux0 = static_cast<const float *>(sd->aux);
-    a.plan = const_cast<int *>(plan); a.out = y;
+    a.plan = const_cast<int *>(plan); a.out = y; a.out_dtype = y_dtype;
     a.rows = down->rows; a.k = k; a.experts = down->experts; a.topk = topk; a.A = n * topk;
-    return gemm_launch<1>(down->type, a, banks, static_cast<const void *>(act), int(B2MOE_F32), rows_x, true, rows_x, xb, inv, static_cast<int *>(nullptr), s);
+    return gemm_launch<1>(down->type, a, banks, x, x_dtype, per_token ? n : rows_x, per_token ? topk : 0, true, rows_x, xb, inv, static_cast<int *>(nullptr), s);
 }
 
 }  // namespace b2

@@ -17,13 +17,14 @@ int32_t iq3s_down(const b2moe_bank *, const b2moe_bank *, const float *, const i
 bool dec4_supported(uint32_t type, int k);
 size_t dec4_workspace_bytes(int rows_x, int k);
 int32_t dec4_gateup(const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const void *, int, const int *, int,
-                    int, int, float *, void *, int, cudaStream_t, bool x_staged);
+                    int, int, void *, int act_dtype, void *, cudaStream_t, bool x_staged);
 void dec4_stage_target(uint32_t type, void * ws, int n, int k, uint8_t ** rows, float ** inv_scale, int * bits);
 bool route_cluster_fits(int experts, int topk, int n);
 int32_t route_plan_stage(int gating, const float * logits, int ld, const float * bias, int * ids, float * weights, float * shared_weights,
                          int experts, int topk, int norm, float scale, int n, int shared_first, int shared_count, int * plan, const void * x,
                          int x_dtype, int k, int bits, uint8_t * staged_rows, float * inv_scale, cudaStream_t s, bool * took);
-int32_t dec4_down(const b2moe_bank *, const b2moe_bank *, const float *, const int *, int, int, int, float *, void *, int, cudaStream_t);
+int32_t dec4_down(const b2moe_bank *, const b2moe_bank *, const void *, int x_dtype, bool per_token, const int *, int, int, int, void *, int y_dtype, void *,
+                  cudaStream_t);
 void dec4_debug(int drop_tile, uint32_t wait_limit);
 void dec4_skip_staging(bool on);
 void dec4_ring(int nbuf, int stages, int slot_tiles);
@@ -33,8 +34,9 @@ bool g_overlap = true;
 bool gemm_tc_supported(uint32_t type, int k, int experts);
 size_t gemm_tc_workspace_bytes(int rows_x, int k);
 int32_t gemm_tc_gateup(const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const void *, int, const int *, int,
-                       int, int, float *, void *, void * rows_buf, size_t rows_buf_bytes, cudaStream_t);
-int32_t gemm_tc_down(const b2moe_bank *, const b2moe_bank *, const float *, const int *, int, int, int, float *, void *, cudaStream_t);
+                       int, int, void *, int act_dtype, void *, void * rows_buf, size_t rows_buf_bytes, cudaStream_t);
+int32_t gemm_tc_down(const b2moe_bank *, const b2moe_bank *, const void *, int x_dtype, bool per_token, const int *, int, int, int, void *, int y_dtype,
+                     void *, cudaStream_t);
 void gemm_tc_item_tokens(int tokens);
 
 namespace {
@@ -75,6 +77,30 @@ int expert_path(uint32_t type, int k, int dtype, int experts, long long assignme
     return gemm ? B2MOE_FAMILY_GEMM : B2MOE_FAMILY_GENERIC;
 }
 }  // namespace
+// One matrix over a ready plan with the caller's own row types: x [assignments or, per_token, tokens][cols] of x_dtype -> y
+// [assignments][rows] of y_dtype, without a pass to fp32 before and one back behind. *took = false: the family that serves this call
+// has no such form (b2moe_expert_down on fp32 rows does it).
+int32_t product_typed(const b2moe_bank * m, const void * x, int x_dtype, bool per_token, const int * plan, int n, int topk, void * y, int y_dtype,
+                      void * ws, cudaStream_t s, bool * took) {
+    const int path = expert_path(m->type, m->cols, B2MOE_F32, m->experts, (long long)n * topk);
+    *took = true;
+    if (path == B2MOE_FAMILY_GEMM) return gemm_tc_down(m, nullptr, x, x_dtype, per_token, plan, n, topk, 0, y, y_dtype, ws, s);
+    if (path == B2MOE_FAMILY_DECODE && decode_kernel(m->type, m->cols, B2MOE_F32) == DEC_4BIT)
+        return dec4_down(m, nullptr, x, x_dtype, per_token, plan, n, topk, 0, y, y_dtype, ws, s);
+    *took = false;
+    return B2MOE_OK;
+}
+// the same for gate / up + SwiGLU; rows_buf as in expert_gateup
+int32_t gateup_typed(const b2moe_bank * gate, const b2moe_bank * up, const void * x, int x_dtype, const int * plan, int n, int topk, void * act, int act_dtype,
+                     void * ws, void * rows_buf, size_t rows_buf_bytes, cudaStream_t s, bool * took) {
+    const int path = expert_path(gate->type, gate->cols, x_dtype, gate->experts, (long long)n * topk);
+    *took = true;
+    if (path == B2MOE_FAMILY_GEMM) return gemm_tc_gateup(gate, up, nullptr, nullptr, x, x_dtype, plan, n, topk, 0, act, act_dtype, ws, rows_buf, rows_buf_bytes, s);
+    if (path == B2MOE_FAMILY_DECODE && decode_kernel(gate->type, gate->cols, x_dtype) == DEC_4BIT)
+        return dec4_gateup(gate, up, nullptr, nullptr, x, x_dtype, plan, n, topk, 0, act, act_dtype, ws, s, false);
+    *took = false;
+    return B2MOE_OK;
+}
 // true when b2moe_expert_down would take the format-generic kernels (which use no scratch) for this call
 bool expert_down_is_generic(const b2moe_bank * down, int n, int topk) {
     return expert_path(down->type, down->cols, B2MOE_F32, down->experts, (long long)n * topk) == B2MOE_FAMILY_GENERIC;
@@ -149,12 +175,11 @@ static int32_t expert_gateup(const b2moe_bank * gate, const b2moe_bank * up, con
         if (need && !aligned16(workspace)) return B2MOE_ERR_ALIGN;
         if (workspace_bytes < need) return B2MOE_ERR_WORKSPACE;
         if (path == B2MOE_FAMILY_GEMM)
-            return gemm_tc_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, workspace, rows_buf, rows_buf_bytes,
-                                  as_stream(stream));
-        const int ma = max_active_of(gate->experts, n, topk, shared_tokens);
+            return gemm_tc_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, B2MOE_F32, workspace, rows_buf,
+                                  rows_buf_bytes, as_stream(stream));
         if (decode_kernel(gate->type, gate->cols, x_dtype) == DEC_4BIT)
-            return dec4_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, workspace, ma, as_stream(stream), x_staged);
-        return iq3s_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, workspace, ma, as_stream(stream));
+            return dec4_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, B2MOE_F32, workspace, as_stream(stream), x_staged);
+        return iq3s_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, workspace, max_active_of(gate->experts, n, topk, shared_tokens), as_stream(stream));
     }
     return generic_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, as_stream(stream));
 }
@@ -183,11 +208,10 @@ static int32_t expert_down(const b2moe_bank * down, const b2moe_bank * shared_do
         if (!aligned16(workspace)) return B2MOE_ERR_ALIGN;
         if (workspace_bytes < b2moe_expert_workspace_bytes(down->type, rows_x, down->cols, B2MOE_F32)) return B2MOE_ERR_WORKSPACE;
         if (path == B2MOE_FAMILY_GEMM)
-            return gemm_tc_down(down, shared_down, act, plan, n, topk, shared_tokens, y, workspace, as_stream(stream));
-        const int ma = max_active_of(down->experts, n, topk, shared_tokens);
+            return gemm_tc_down(down, shared_down, act, B2MOE_F32, false, plan, n, topk, shared_tokens, y, B2MOE_F32, workspace, as_stream(stream));
         if (decode_kernel(down->type, down->cols, B2MOE_F32) == DEC_4BIT)
-            return dec4_down(down, shared_down, act, plan, n, topk, shared_tokens, y, workspace, ma, as_stream(stream));
-        return iq3s_down(down, shared_down, act, plan, n, topk, shared_tokens, y, workspace, ma, as_stream(stream));
+            return dec4_down(down, shared_down, act, B2MOE_F32, false, plan, n, topk, shared_tokens, y, B2MOE_F32, workspace, as_stream(stream));
+        return iq3s_down(down, shared_down, act, plan, n, topk, shared_tokens, y, workspace, max_active_of(down->experts, n, topk, shared_tokens), as_stream(stream));
     }
     return generic_down(down, shared_down, act, plan, n, topk, shared_tokens, y, as_stream(stream));
 }
