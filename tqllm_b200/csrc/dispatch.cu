@@ -4,18 +4,21 @@
 // dedup_maps_k (src/experts/moe.cu:453-483) produce, without the O(A^2) walk of the latter or the atomics of group_k
 // (src/experts/moe.cu:168-176), whose list order is not deterministic.
 //
-// Method: the assignments are cut into chunks that one warp walks 32 at a time. __match_any_sync groups the lanes
+// Method: the assignments are cut into chunks that one warp walks 32 at a time. A vote per bit of the ids finds the lanes
 // holding the same expert, so each distinct expert of a step has one leader lane that bumps the chunk's private
 // counter by the group size (no atomics); an exclusive scan over (expert, chunk) turns the counters into each
 // chunk's first output slot per expert; a second walk in the same order hands every assignment
 // base + (number of lower lanes with the same expert), which keeps ascending order inside an expert.
+#include <algorithm>
+
 #include "common.cuh"
 #include "dispatch.cuh"
 
 namespace b2 {
 namespace {
 
-constexpr int CHUNK = 256;   // assignments per warp-chunk on the multi-block path
+constexpr int CHUNK = 256;   // assignments per warp-chunk on the multi-block path with counters in global memory
+constexpr int WALK_WARPS = 8, WALK_THREADS = WALK_WARPS * 32;
 
 __global__ void dispatch_small_k(const int * ids, int A, int e, int shared_first, int shared_tokens, int * __restrict__ plan) {
     extern __shared__ unsigned short hist[];       // [32 warps][e]
@@ -24,7 +27,92 @@ __global__ void dispatch_small_k(const int * ids, int A, int e, int shared_first
     dispatch_small_body(ids, A, e, shared_first, shared_tokens, plan, hist);
 }
 
-// ---- multi-block path: chunk counters in global scratch [chunks][e] ----
+// ---- multi-block path: two launches. Every block counts its segment of the assignments in shared memory, a private row of
+// counters per warp, and leaves the sums as its row of `rows` [blocks][e]; then every block adds up the rows (all of them: the
+// experts' totals and offsets; those below its own: its first slot per expert), counts its segment again and places it. Nothing
+// is cleared, no block waits for another, and the sums over the rows are a few batches of independent loads. Bound by latency:
+// the launch, one load of the ids, the batches of rows, the plan's header and pass list in
+// block 0. Measured on the device: 41,000 ids on 512 experts 41 us + a memset -> 20 us, 65,536 on 128 experts 15 us.
+struct WalkArgs { const int * ids; int A, e, seg, shared_first, shared_tokens; int * rows, * plan; };
+__host__ __device__ inline int row_parts(int e) { return e >= WALK_THREADS ? 1 : WALK_THREADS / e; }
+// hist [warps][e], totals and lower sums [row_parts][e], three arrays of e + 2
+inline size_t walk_smem(int e) { return (size_t(WALK_WARPS) * e + size_t(2) * row_parts(e) * e + size_t(3) * (e + 2)) * sizeof(int); }
+
+__device__ __forceinline__ void count_segment(const WalkArgs & p, int a0, int a1, int * hist, int lane, int warp) {
+    for (int i = threadIdx.x; i < WALK_WARPS * p.e; i += WALK_THREADS) hist[i] = 0;
+    __syncthreads();
+    walk_ids(p.ids, a0, a1, p.e, lane, [&](int, int id, unsigned peers) {
+        if (id >= 0 && lane == __ffs(peers) - 1) hist[warp * p.e + id] += __popc(peers);
+    });
+    __syncthreads();
+}
+__global__ void __launch_bounds__(WALK_THREADS) dispatch_count_k(const WalkArgs p) {
+    extern __shared__ int walk_mem[];
+    grid_release();
+    grid_wait();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int a0 = blockIdx.x * p.seg * WALK_WARPS + warp * p.seg;
+    count_segment(p, a0, min(p.A, a0 + p.seg), walk_mem, lane, warp);
+    for (int x = threadIdx.x; x < p.e; x += WALK_THREADS) {
+        int sum = 0;
+#pragma unroll
+        for (int w = 0; w < WALK_WARPS; ++w) sum += walk_mem[w * p.e + x];
+        p.rows[size_t(blockIdx.x) * p.e + x] = sum;
+    }
+}
+__global__ void __launch_bounds__(WALK_THREADS) dispatch_place_k(const WalkArgs p) {
+    extern __shared__ int walk_mem[];
+    grid_release();
+    grid_wait();
+    const int e = p.e, e1 = e + 1, parts = row_parts(e), blocks = gridDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int * hist = walk_mem, * total = hist + WALK_WARPS * e, * lower = total + parts * e, * cs = lower + parts * e, * os = cs + e + 2, * as = os + e + 2;
+    int * counts = p.plan + PLAN_HDR, * offsets = counts + e1, * active = offsets + e1 + 1, * perm = active + e1;
+    for (int i = threadIdx.x; i < parts * e; i += WALK_THREADS) {
+        const int x = i % e, part = i / e, per = (blocks + parts - 1) / parts, r1 = min(blocks, (part + 1) * per);
+        int sum = 0, below = 0;
+        for (int r = part * per; r < r1; r += 16) {
+            int v[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = r + j < r1 ? p.rows[size_t(r + j) * e + x] : 0;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) { sum += v[j]; below += r + j < int(blockIdx.x) ? v[j] : 0; }
+        }
+        total[i] = sum;
+        lower[i] = below;
+    }
+    const int a0 = blockIdx.x * p.seg * WALK_WARPS + warp * p.seg, a1 = min(p.A, a0 + p.seg);
+    count_segment(p, a0, a1, hist, lane, warp);
+    for (int x = threadIdx.x; x < e; x += WALK_THREADS) {
+        int sum = 0, below = 0;
+        for (int q = 0; q < parts; ++q) { sum += total[q * e + x]; below += lower[q * e + x]; }
+        cs[x] = sum;
+        lower[x] = below;
+        prefix_counters(hist + x, WALK_WARPS, e);
+        if (blockIdx.x == 0) counts[x] = sum;
+    }
+    if (threadIdx.x == 0) {
+        cs[e] = p.shared_tokens;
+        if (blockIdx.x == 0) counts[e] = p.shared_tokens;
+    }
+    __syncthreads();
+    finish_plan(p.plan, cs, os, as, offsets, active, perm + p.A + p.shared_tokens, e1, blockIdx.x == 0);
+    __syncthreads();
+    int * h = hist + warp * e;
+    walk_ids(p.ids, a0, a1, e, lane, [&](int a, int id, unsigned peers) {
+        if (id >= 0) perm[os[id] + lower[id] + h[id] + __popc(peers & ((1u << lane) - 1u))] = a;
+        __syncwarp();
+        if (id >= 0 && lane == __ffs(peers) - 1) h[id] += __popc(peers);
+    });
+    for (int t = blockIdx.x * WALK_THREADS + threadIdx.x; t < p.shared_tokens; t += blocks * WALK_THREADS) perm[os[e] + t] = p.A + p.shared_first + t;
+}
+// Assignments per warp: 128 (four steps; a block of eight warps takes 1,024) while that makes at most a block per SM, and
+// beyond that what a block per SM leaves, since every block reads every row.
+inline int walk_seg(int A) { return std::max(128, (ceil_div(A, 148 * WALK_WARPS) + 31) / 32 * 32); }
+inline int walk_blocks(int A) { return ceil_div(A, walk_seg(A) * WALK_WARPS); }
+// the counters have to fit a block's ordinary shared memory: up to about 900 experts
+inline bool walk_path(int e) { return walk_smem(e) <= 46 * 1024; }
+
+// ---- more experts than that: chunk counters in global scratch [chunks][e] ----
 __global__ void dispatch_hist_k(const int * __restrict__ ids, int A, int e, int * __restrict__ hist) {
     const int lane = threadIdx.x & 31, chunk = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int a0 = chunk * CHUNK;
@@ -40,23 +128,11 @@ __global__ void dispatch_hist_k(const int * __restrict__ ids, int A, int e, int 
 __global__ void dispatch_scan_k(int * __restrict__ hist, int chunks, int e, int A, int shared_tokens, int * __restrict__ plan) {
     const int e1 = e + 1;
     int * counts = plan + PLAN_HDR, * offsets = counts + e1, * active = offsets + e1 + 1;
-    for (int x = threadIdx.x; x < e; x += blockDim.x) {
-        int run = 0;
-        // eight chunk counters at a time: the loads of a batch are independent of its stores (one load per store would wait
-        // for the store before it, since both go to the same array)
-        for (int c0 = 0; c0 < chunks; c0 += 8) {
-            int v[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = c0 + i < chunks ? hist[size_t(c0 + i) * e + x] : 0;
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (c0 + i < chunks) { hist[size_t(c0 + i) * e + x] = run; run += v[i]; }
-        }
-        counts[x] = run;
-    }
+    for (int x = threadIdx.x; x < e; x += blockDim.x)
+        counts[x] = prefix_counters(hist + x, chunks, e);
     if (threadIdx.x == 0) counts[e] = shared_tokens;
     __syncthreads();
-    if (threadIdx.x < 32) finish_plan(plan, counts, offsets, active, offsets, active, active + e1 + A + shared_tokens, e1, threadIdx.x);
+    finish_plan(plan, counts, offsets, active, offsets, active, active + e1 + A + shared_tokens, e1, true);
 }
 __global__ void dispatch_scatter_k(const int * __restrict__ ids, int A, int e, int shared_first, int shared_tokens, int * __restrict__ hist,
                                    int * __restrict__ plan) {
@@ -111,7 +187,7 @@ extern "C" B2MOE_API void b2moe_plan_view_of(int32_t experts, int32_t assignment
 extern "C" B2MOE_API size_t b2moe_dispatch_workspace_bytes(int32_t experts, int32_t assignments) {
     if (experts <= 0 || assignments < 0) return 0;
     if (small_path(experts, assignments)) return 16;
-    return align_up(size_t(ceil_div(assignments, CHUNK)) * experts * sizeof(int), 16);
+    return align_up(size_t(walk_path(experts) ? walk_blocks(assignments) : ceil_div(assignments, CHUNK)) * experts * sizeof(int), 16);
 }
 
 extern "C" B2MOE_API int32_t b2moe_dispatch_range(const int32_t * ids, int32_t n, int32_t topk, int32_t experts, int32_t shared_first,
@@ -130,6 +206,12 @@ extern "C" B2MOE_API int32_t b2moe_dispatch_range(const int32_t * ids, int32_t n
     if (!workspace) return B2MOE_ERR_NULL;
     if (workspace_bytes < need) return B2MOE_ERR_WORKSPACE;
     int * hist = static_cast<int *>(workspace);
+    if (walk_path(experts)) {
+        const WalkArgs w{ids, A, experts, walk_seg(A), shared_first, shared_count, hist, plan};
+        launch_overlapped(dispatch_count_k, dim3(walk_blocks(A)), dim3(WALK_THREADS), walk_smem(experts), s, w);
+        launch_overlapped(dispatch_place_k, dim3(walk_blocks(A)), dim3(WALK_THREADS), walk_smem(experts), s, w);
+        return launch_status();
+    }
     const int chunks = ceil_div(A, CHUNK);
     if (cudaMemsetAsync(hist, 0, size_t(chunks) * experts * sizeof(int), s) != cudaSuccess) return B2MOE_ERR_CUDA;
     dispatch_hist_k<<<ceil_div(chunks, 8), 256, 0, s>>>(ids, A, experts, hist);
