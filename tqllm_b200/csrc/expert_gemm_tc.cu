@@ -206,7 +206,9 @@ __global__ void tokens_to_slots_k(const typename Elem<DT>::type * x, const int *
 }
 
 // MODE 0: act[a][r] = silu(gate_r . x_tok(a)) * (up_r . x_tok(a));  MODE 1: y[a][r] = down_r . act[a]
-template <uint32_t T, int MODE>
+// F32_OUT: an instance for fp32 results and one for 16-bit ones, chosen by the call's output type. A branch at the stores, or two
+// loops in one kernel, cost every fp32 caller: c3 down (80 tokens x K = 512) 262 us against 184, c5 gate/up 1305 against 1240.
+template <uint32_t T, int MODE, bool F32_OUT>
 __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, const __grid_constant__ GemmMaps maps) {
     using D = gdec::Dec<T>;
     constexpr int CB = chunk_bytes<T>();
@@ -311,7 +313,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
         const int q = warp & 3, tid = threadIdx.x - EPI_WARP0 * 32, first = 16 * ((warp - EPI_WARP0) >> 2);
         const bool upper = lane >= 16;
         constexpr bool ROW_SCALE = T == T_NVFP4G;
-        const uint32_t out_size = p.out_dtype == B2MOE_F32 ? 4u : 2u, row_bytes = uint32_t(p.rows) * out_size;
+        const uint32_t row_bytes = uint32_t(p.rows) * (F32_OUT ? 4u : 2u);
         int2 mine;
         auto fetch = [&](const Item & im) {                            // this thread's token of the item
             mine = make_int2(-1, 0);
@@ -349,10 +351,13 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
             fence_after();
             const uint32_t taddr = tmem + (uint32_t(32 * q) << 16) + h * ACC_COLS;
             const int4 * t = reinterpret_cast<const int4 *>(tok + (ic & 1u) * MAX_CAP);
-            char * const out = static_cast<char *>(p.out) + row * out_size;
+            char * const out = reinterpret_cast<char *>(static_cast<typename std::conditional<F32_OUT, float, uint16_t>::type *>(p.out) + row);
             const bool in = row < p.rows;
-            auto store = [&](int a, float y) { if (in && a >= 0) *reinterpret_cast<float *>(out + uint64_t(uint32_t(a)) * row_bytes) = y; };
-            auto store_short = [&](int a, float y) { if (in && a >= 0) store_act(out + uint64_t(uint32_t(a)) * row_bytes, p.out_dtype, 0, y); };
+            auto store = [&](int a, float y) {
+                if (!in || a < 0) return;
+                if constexpr (F32_OUT) *reinterpret_cast<float *>(out + uint64_t(uint32_t(a)) * row_bytes) = y;
+                else store_act(out + uint64_t(uint32_t(a)) * row_bytes, p.out_dtype, 0, y);
+            };
 #pragma unroll 1
             for (int c = first; c < im.nv; c += 32) {
                 uint32_t v[16];
@@ -383,20 +388,14 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
                             const float gv = (upper ? other : v0) * is, uv = (upper ? v1 : other) * is;
                             res[i] = __fdividef(gv, 1.f + __expf(-gv)) * uv;      // fast exp and divide: relative error about 2^-21
                         }
-                        if (out_size == 4u) {
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) store(upper ? two[i].z : two[i].x, res[i]);
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) store_short(upper ? two[i].z : two[i].x, res[i]);
-                        }
+                        for (int i = 0; i < 4; ++i) store(upper ? two[i].z : two[i].x, res[i]);
                     } else {
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             const float is0 = __int_as_float(two[i].y), is1 = __int_as_float(two[i].w);
-                            const float y0 = __uint_as_float(v[j0 + 2 * i]) * (ROW_SCALE ? is0 * rs : is0), y1 = __uint_as_float(v[j0 + 2 * i + 1]) * (ROW_SCALE ? is1 * rs : is1);
-                            if (out_size == 4u) { store(two[i].x, y0); store(two[i].z, y1); }
-                            else { store_short(two[i].x, y0); store_short(two[i].z, y1); }
+                            store(two[i].x, __uint_as_float(v[j0 + 2 * i]) * (ROW_SCALE ? is0 * rs : is0));
+                            store(two[i].z, __uint_as_float(v[j0 + 2 * i + 1]) * (ROW_SCALE ? is1 * rs : is1));
                         }
                     }
                 }
@@ -688,8 +687,9 @@ int32_t gemm_launch_t(GemmArgs a, const b2moe_bank * const * m, const void * x, 
         if (m[i]) mapped = mapped && bank_map<T>(maps.w[i], m[i], MODE == 0 ? 4 : 8);
     if (!mapped) return B2MOE_ERR_CUDA;
     const size_t smem = gemm_smem<T>(a.experts, a.cap, a.b_stages, a.raw_slots);
-    if (cudaFuncSetAttribute(gemm_tc_k<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return B2MOE_ERR_CUDA;
-    launch_overlapped(gemm_tc_k<T, MODE>, dim3(sms), dim3(G_THREADS), smem, s, a, maps);
+    const auto kernel = a.out_dtype == B2MOE_F32 ? gemm_tc_k<T, MODE, true> : gemm_tc_k<T, MODE, false>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return B2MOE_ERR_CUDA;
+    launch_overlapped(kernel, dim3(sms), dim3(G_THREADS), smem, s, a, maps);
     return launch_status();
 }
 template <int MODE, typename... Args>
