@@ -191,6 +191,10 @@ template <uint32_t T, int MODE, bool STAGER>
 __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4Args p) {
     using F = D4<T>;
     constexpr int NMAT = MODE == 0 ? 2 : 1, TILE = F::TILE;
+    // how the byte sums of a four-token pass meet: two shuffles and half of the fp32 steps, or four shuffles and no selects.
+    // Measured, halves against not: IQ3_S gate/up (64 tokens) 90.4 / 92.6 us, its down product 53.2 / 52.7, Q4_K (which meets
+    // twice a tile) 112.8 / 111.7 and 59.4 / 57.3.
+    constexpr bool HALVES = F::FLUSH_AT < 0 && MODE == 0;
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t * bars = reinterpret_cast<uint64_t *>(smem);
     volatile int * abort_flag = reinterpret_cast<volatile int *>(smem + (2 * CTA_WARPS * MAX_STAGES + 4) * 8);
@@ -395,11 +399,13 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
             const int xr = quad ? g & 3 : g;
             const uint8_t * xw = xs + b * xbuf + xr * xrow + t * 16 + (quad && g >= 4 ? 8 : 0);      // + sub-block * 64
             const uint8_t * rec = xs + b * xbuf + xr * xrow + size_t(K) * 2 + t * 8;  // + tile * 32
-            // the lane's two token columns (2t, 2t + 1): assignment index and inverse activation scale, as the producer left them
+            // the lane's two tokens (columns 2t, 2t + 1; of four tokens in HALVES, 2 (t & 1) and the next): assignment index and inverse
+            // activation scale, as the producer left them
+            const bool halves = HALVES && quad;
             int col_a[2];
             float col_is[2];
 #pragma unroll
-            for (int q = 0; q < 2; ++q) { col_a[q] = meta[b].col_a[2 * t + q]; col_is[q] = meta[b].col_is[2 * t + q]; }
+            for (int q = 0; q < 2; ++q) { const int c = 2 * (halves ? t & 1 : t) + q; col_a[q] = meta[b].col_a[c]; col_is[q] = meta[b].col_is[c]; }
 
             const int grp = warp / KSP, part = warp % KSP;                  // row-job slot of this warp and its part of the columns
 #pragma unroll 1
@@ -412,9 +418,26 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
 
                 auto columns = [&](auto Q) {
                     constexpr bool QUAD = decltype(Q)::value;
-                    // QUAD: lane t < 2 meets the low-byte sums of its tokens, which lane t + 2 holds (whose own result means nothing), so
-                    // that a token's sums are the same integers, and its result the same bits, in a pass of either form
-                    auto whole = [&](int v) { return QUAD ? int(uint32_t(v) * 256u + uint32_t(__shfl_xor_sync(0xffffffffu, v, 2))) : v; };
+                    // QUAD: lanes t and t + 2 hold the high- and low-byte sums of two tokens. They meet so that a token's sums are the same
+                    // integers, and its result the same bits, in a pass of either form. HALVES: lane t < 2 ends with the whole sums of
+                    // row g and lane t + 2 with those of row g + 8 (acc[.][0 .. 1] of either); else lane t < 2 ends with both rows.
+                    const bool upper = QUAD && HALVES && t >= 2;
+                    auto add_main = [&](float (&a)[4], const Hdr4 & hdr, int (&v)[4]) {
+                        if constexpr (QUAD && HALVES) {
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) {
+                                const uint32_t other = __shfl_xor_sync(0xffffffffu, uint32_t(upper ? v[i] : v[2 + i]), 2);
+                                const int sum = int(uint32_t(upper ? v[2 + i] : v[i]) * (upper ? 1u : 256u) + other * (upper ? 256u : 1u));
+                                a[i] = fmaf(upper ? hdr.f_main[1] : hdr.f_main[0], float(sum), a[i]);
+                            }
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                const int sum = QUAD ? int(uint32_t(v[i]) * 256u + uint32_t(__shfl_xor_sync(0xffffffffu, v[i], 2))) : v[i];
+                                a[i] = fmaf(hdr.f_main[i >> 1], float(sum), a[i]);
+                            }
+                        }
+                    };
 #pragma unroll 1
                     for (int ks = part * kpart; ks < (part + 1) * kpart && alive; ++ks) {
                         const int nt = min(SLOT_TILES, p.k_tiles - ks * SLOT_TILES);
@@ -456,15 +479,21 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
                                         }
                                     }
                                     if (F::FLUSH_AT == q) {            // keep `main` inside 32 bits: hand the first half of the tile over now
+                                        add_main(acc[m], hdr, main_);
 #pragma unroll
-                                        for (int i = 0; i < 4; ++i) { acc[m][i] = fmaf(hdr.f_main[i >> 1], float(whole(main_[i])), acc[m][i]); main_[i] = 0; }
+                                        for (int i = 0; i < 4; ++i) main_[i] = 0;
                                     }
                                 }
                                 float corr[4];
                                 mma_f16_zero(corr, hdr.ca[0], hdr.ca[1], hdr.ca[2], hdr.ca[3], sp.x, sp.y);
+                                if constexpr (QUAD && HALVES) {
 #pragma unroll
-                                for (int i = 0; i < 4; ++i)
-                                    acc[m][i] = fmaf(hdr.f_main[i >> 1], float(whole(main_[i])), fmaf(hdr.f_corr[i >> 1], corr[i], acc[m][i]));
+                                    for (int i = 0; i < 2; ++i) acc[m][i] = fmaf(upper ? hdr.f_corr[1] : hdr.f_corr[0], upper ? corr[2 + i] : corr[i], acc[m][i]);
+                                } else {
+#pragma unroll
+                                    for (int i = 0; i < 4; ++i) acc[m][i] = fmaf(hdr.f_corr[i >> 1], corr[i], acc[m][i]);
+                                }
+                                add_main(acc[m], hdr, main_);
                             }
                             __syncwarp();             // every lane has read its words: the slot can be refilled
                             if (lane == 0) mbar_arrive(my_empty + 8 * c_slot);
@@ -503,7 +532,7 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
                     if (lane == 0) mbar_arrive(red_free + 8 * grp);
                     ++red_use;
                 }
-                // epilogue: the lane holds rows g, g + 8 x token columns 2t, 2t + 1
+                // epilogue: the lane holds rows g, g + 8 of its two tokens, in HALVES only row g (t < 2) or g + 8
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {
                     const int a = col_a[q];
@@ -511,8 +540,8 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
                     const float is = col_is[q];
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        const int row = 16 * rt + g + 8 * h;
-                        if (row >= p.rows) continue;
+                        const int row = 16 * rt + g + 8 * (halves ? t >> 1 : h);
+                        if (row >= p.rows || (halves && h == 1)) continue;
                         const float v0 = acc[0][2 * h + q] * is, v1 = acc[NMAT - 1][2 * h + q] * is;
                         store_act(p.out, p.out_dtype, size_t(a) * p.rows + row, MODE == 0 ? (v0 / (1.f + expf(-v0))) * v1 : v0);
                     }
