@@ -24,7 +24,7 @@ __global__ void dispatch_small_k(const int * ids, int A, int e, int shared_first
     extern __shared__ unsigned short hist[];       // [32 warps][e]
     grid_release();
     grid_wait();
-    dispatch_small_body(ids, A, e, shared_first, shared_tokens, plan, hist);
+    dispatch_small_body<true>(ids, A, e, shared_first, shared_tokens, plan, hist);
 }
 
 // ---- multi-block path: two launches. Every block counts its segment of the assignments in shared memory, a private row of
@@ -41,7 +41,7 @@ inline size_t walk_smem(int e) { return (size_t(WALK_WARPS) * e + size_t(2) * ro
 __device__ __forceinline__ void count_segment(const WalkArgs & p, int a0, int a1, int * hist, int lane, int warp) {
     for (int i = threadIdx.x; i < WALK_WARPS * p.e; i += WALK_THREADS) hist[i] = 0;
     __syncthreads();
-    walk_ids(p.ids, a0, a1, p.e, lane, [&](int, int id, unsigned peers) {
+    walk_ids<true>(p.ids, a0, a1, p.e, lane, [&](int, int id, unsigned peers) {
         if (id >= 0 && lane == __ffs(peers) - 1) hist[warp * p.e + id] += __popc(peers);
     });
     __syncthreads();
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(WALK_THREADS) dispatch_place_k(const WalkArgs 
     finish_plan(p.plan, cs, os, as, offsets, active, perm + p.A + p.shared_tokens, e1, blockIdx.x == 0);
     __syncthreads();
     int * h = hist + warp * e;
-    walk_ids(p.ids, a0, a1, e, lane, [&](int a, int id, unsigned peers) {
+    walk_ids<true>(p.ids, a0, a1, e, lane, [&](int a, int id, unsigned peers) {
         if (id >= 0) perm[os[id] + lower[id] + h[id] + __popc(peers & ((1u << lane) - 1u))] = a;
         __syncwarp();
         if (id >= 0 && lane == __ffs(peers) - 1) h[id] += __popc(peers);

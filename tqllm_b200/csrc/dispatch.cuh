@@ -11,8 +11,9 @@ __device__ __forceinline__ int valid_id(const int * ids, int a, int A, int e) {
     return (v >= 0 && v < e) ? v : -1;
 }
 
-// the lanes whose id equals this lane's (meaningless where id < 0): a vote per bit of the ids (__match_any_sync queues behind the
-// other warps of the SM: 32 warps of dispatch_small_k took 18 us with it and take 14 us with the votes)
+// the lanes whose id equals this lane's (meaningless where id < 0): a vote per bit of the ids. For kernels of many steps:
+// __match_any_sync queues behind the other warps of the SM (32 warps of dispatch_small_k, 5,090 ids: 18 us with it, 13.5 with the
+// votes); in the routing launch, of two steps a warp, the shorter code wins (15.4 against 16.5 us).
 __device__ __forceinline__ unsigned same_id(int id, int bits) {
     unsigned peers = __ballot_sync(0xffffffffu, id >= 0);
 #pragma unroll 4
@@ -26,7 +27,7 @@ __device__ __forceinline__ unsigned same_id(int id, int bits) {
 // One warp walks the assignments [a0, a1) in order, 32 per step, and calls step(assignment, expert or -1, lanes with the same
 // expert): the ids of eight steps are loaded together, so that a walk waits for memory once per 256 assignments and not at
 // every step.
-template <class F>
+template <bool VOTES, class F>
 __device__ __forceinline__ void walk_ids(const int * ids, int a0, int a1, int e, int lane, F step) {
     const int bits = 32 - __clz(e - 1);
 #pragma unroll 1
@@ -37,7 +38,7 @@ __device__ __forceinline__ void walk_ids(const int * ids, int a0, int a1, int e,
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             if (b + 32 * j >= a1) break;
-            step(b + 32 * j + lane, id[j], same_id(id[j], bits));
+            step(b + 32 * j + lane, id[j], VOTES ? same_id(id[j], bits) : __match_any_sync(0xffffffffu, id[j]));
             __syncwarp();             // a step's counter updates are in place before the next step's leaders read them
         }
     }
@@ -118,6 +119,7 @@ __device__ inline void finish_plan(int * plan, const int * cs, int * os, int * a
 __host__ __device__ inline size_t dispatch_small_smem(int warps, int e) { return (size_t(warps) * e * 2 + 15) / 16 * 16 + size_t(3) * (e + 2) * 4; }
 
 // ---- single block (up to 32 warps): every phase in shared memory (decode-sized batches); hist = [warps][e] ----
+template <bool VOTES>
 __device__ __forceinline__ void dispatch_small_body(const int * ids, int A, int e, int shared_first, int shared_tokens,
                                                     int * __restrict__ plan, unsigned short * hist) {
     const int e1 = e + 1;
@@ -130,7 +132,7 @@ __device__ __forceinline__ void dispatch_small_body(const int * ids, int A, int 
     const int a0 = warp * chunk;
     const int a1 = min(A, a0 + chunk);
     unsigned short * h = hist + warp * e;
-    walk_ids(ids, a0, a1, e, lane, [&](int, int id, unsigned peers) {
+    walk_ids<VOTES>(ids, a0, a1, e, lane, [&](int, int id, unsigned peers) {
         if (id >= 0 && lane == __ffs(peers) - 1) h[id] += (unsigned short)__popc(peers);
     });
     __syncthreads();
@@ -139,7 +141,7 @@ __device__ __forceinline__ void dispatch_small_body(const int * ids, int A, int 
     __syncthreads();
     finish_plan(plan, cs, os, as, offsets, active, perm + A + shared_tokens, e1, true);
     __syncthreads();
-    walk_ids(ids, a0, a1, e, lane, [&](int a, int id, unsigned peers) {
+    walk_ids<VOTES>(ids, a0, a1, e, lane, [&](int a, int id, unsigned peers) {
         if (id >= 0) perm[os[id] + h[id] + __popc(peers & ((1u << lane) - 1u))] = a;
         __syncwarp();
         if (id >= 0 && lane == __ffs(peers) - 1) h[id] += (unsigned short)__popc(peers);

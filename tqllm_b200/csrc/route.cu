@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(RD_THREADS) route_dispatch_k(const float * log
         __syncwarp();
     }
     __syncthreads();                              // the ids are written and the routing scratch is dead
-    dispatch_small_body(ids, n * k, e, shared_first, shared_count, plan, reinterpret_cast<unsigned short *>(smem));
+    dispatch_small_body<false>(ids, n * k, e, shared_first, shared_count, plan, reinterpret_cast<unsigned short *>(smem));
 }
 
 // The same for up to RC_BLOCKS * RD_THREADS / 32 tokens, as one thread-block cluster: every block routes its share of the tokens
@@ -592,7 +592,7 @@ __global__ void __launch_bounds__(RD_THREADS) route_cluster_k(const float * logi
     __threadfence();
     cluster.sync();                               // every block's ids are written and visible
     if (rank == 0) {
-        dispatch_small_body(ids, n * k, e, shared_first, shared_count, plan, reinterpret_cast<unsigned short *>(smem));
+        dispatch_small_body<false>(ids, n * k, e, shared_first, shared_count, plan, reinterpret_cast<unsigned short *>(smem));
     } else if (st.x) {
         for (int row = (rank - 1) + (nb - 1) * warp; row < n; row += (nb - 1) * (RD_THREADS / 32))
             stage_row_warp(st.x, st.dtype, row, st.k, st.bits, st.rows, st.inv_scale, lane);
