@@ -421,9 +421,11 @@ class CudaEpLayer:
         ews = self._b("ews", (max(eg, ed, 16),), torch.uint8)
         br = lambda b: C.byref(b.c)
         shg, shu, shd = (br(L.sh[0]), br(L.sh[1]), br(L.sh[2])) if has_sh else (None, None, None)
+        # y is written by the down product: until then its memory is the gate/up product's workspace, with a row per assignment
+        gws = y if y.nbytes >= eg else ews
         live = self.live_estimate(N * k)                 # this rank owns count / experts_total of the experts: so many ids are not -1
         self.capi.check(lib.b2moe_expert_gateup_swiglu_sparse(br(L.gate), br(L.up), shg, shu, x_all.data_ptr(), dt, plan.data_ptr(), N, k,
-                                                              shared_n, live, act.data_ptr(), ews.data_ptr(), ews.numel(), self._st()), "gateup")
+                                                              shared_n, live, act.data_ptr(), gws.data_ptr(), gws.nbytes, self._st()), "gateup")
         self.capi.check(lib.b2moe_expert_down_sparse(br(L.down), shd, act.data_ptr(), plan.data_ptr(), N, k, shared_n, live, y.data_ptr(),
                                                      ews.data_ptr(), ews.numel(), self._st()), "down")
         parts = self._b("parts", (N, sh.hidden), torch.float32)
@@ -486,9 +488,10 @@ class CudaEpLayer:
         ews = torch.empty(max(eg, ed, 16), dtype=torch.uint8, device=recv.device)
         br = lambda b: C.byref(b.c)
         shg, shu, shd = (br(L.sh[0]), br(L.sh[1]), br(L.sh[2])) if has_sh else (None, None, None)
+        gws = y if y.nbytes >= eg else ews                 # as above
         live = self.live_estimate(N * k)
         self.capi.check(lib.b2moe_expert_gateup_swiglu_sparse(br(L.gate), br(L.up), shg, shu, x.data_ptr(), dt, plan.data_ptr(), N, k, shared_n,
-                                                              live, act.data_ptr(), ews.data_ptr(), ews.numel(), self._st()), "gateup")
+                                                              live, act.data_ptr(), gws.data_ptr(), gws.nbytes, self._st()), "gateup")
         self.capi.check(lib.b2moe_expert_down_sparse(br(L.down), shd, act.data_ptr(), plan.data_ptr(), N, k, shared_n, live, y.data_ptr(),
                                                      ews.data_ptr(), ews.numel(), self._st()), "down")
         parts = torch.empty(N, H, dtype=torch.float32, device=recv.device)
