@@ -62,18 +62,22 @@ int decode_kernel(uint32_t type, int k, int dtype) {
 //   decode   every expert sees a few tokens, the product is bound by streaming the weights;
 //   GEMM     the tcgen05 grouped GEMM (all formats): the weights of an expert are decoded once per 128 tokens;
 //   generic  exact fp32 CUDA-core path: every shape, the floor under the other two.
-// Default: a type with a decode kernel takes it while the batch averages fewer assignments per expert than the crossover
-// below, everything else the GEMM. Measured layer times, decode / GEMM, us: IQ3_S codes (512 experts) 10 per expert 400 / 502,
-// 16: 564 / 550; Q4_K (256 experts) 12: 848 / 1009, 19: 1139 / 1027, (60 experts) 15: 175 / 177, 30: 249 / 184, (32 experts of
-// 1024 x 512) 16: 70 / 70, 64: 111 / 78, (16 experts) 8: 104 / 142, 19: 156 / 148; IQ3_S in GGUF fields 10: 617 / 610. b2moe_harness_select forces a family where it supports the shape (tests and benchmarks).
-constexpr int GEMM_MIN_PER = 16, GEMM_MIN_PER_IQ3S = 10;
+// Default: a type with a decode kernel takes it while the batch averages fewer than GEMM_MIN_PER assignments per expert or
+// the bank has fewer than GEMM_MIN_EXPERTS experts, everything else the GEMM. The line is one of precision as much as of time: the
+// decode kernels take the weights as they are and 15-bit activations, the GEMM rounds both to 11 bits. Relative error against
+// 64-bit sums (2-norm), decode / GEMM, at any density: Q4_K act 2.5e-5 / 4.0e-4, down of it 2.0e-4 / 5.3e-4; IQ3_S codes 2.5e-5 / 3.0e-4
+// and 2.0e-4 / 4.2e-4; IQ3_S in GGUF fields 2e-7 / 3.0e-4 and 2.1e-4 / 4.2e-4. The GEMM is the faster one from about 16 per
+// expert on (layer times, decode / GEMM, us: Q4_K of 256 experts at 19 per expert 1139 / 1027, of 60 at 30 249 / 184; IQ3_S codes of 512 at
+// 16 564 / 550), but nothing below this line asked for fewer bits. b2moe_harness_select forces a family where it supports the shape
+// (tests and benchmarks).
+constexpr int GEMM_MIN_PER = 32, GEMM_MIN_EXPERTS = 128;
 int g_family = B2MOE_FAMILY_AUTO;
 int expert_path(uint32_t type, int k, int dtype, int experts, long long assignments) {
     if (g_family == B2MOE_FAMILY_GENERIC) return B2MOE_FAMILY_GENERIC;
     const bool dec = decode_kernel(type, k, dtype) != DEC_NONE, gemm = gemm_tc_supported(type, k, experts);
     if (g_family == B2MOE_FAMILY_DECODE) return dec ? B2MOE_FAMILY_DECODE : B2MOE_FAMILY_GENERIC;
     if (g_family == B2MOE_FAMILY_GEMM) return gemm ? B2MOE_FAMILY_GEMM : dec ? B2MOE_FAMILY_DECODE : B2MOE_FAMILY_GENERIC;
-    if (dec && (!gemm || assignments < (long long)(type == T_IQ3_S ? GEMM_MIN_PER_IQ3S : GEMM_MIN_PER) * experts)) return B2MOE_FAMILY_DECODE;
+    if (dec && (!gemm || assignments < (long long)GEMM_MIN_PER * experts || experts < GEMM_MIN_EXPERTS)) return B2MOE_FAMILY_DECODE;
     return gemm ? B2MOE_FAMILY_GEMM : B2MOE_FAMILY_GENERIC;
 }
 }  // namespace
