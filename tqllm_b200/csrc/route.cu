@@ -51,7 +51,12 @@ __global__ void router_k(const float * __restrict__ w, const float * __restrict_
 // logits = W x with W fp32 split exactly into three bf16 terms (hi + mid + lo = 24 significant bits) and x split into as many as
 // it has bits for (bf16: itself, fp16: two, fp32: three; of the fp32 products the three whose terms lie below 2^-24 of the
 // product are left out): every product is exact in fp32 and the sums are fp32, so the result is fp32-accurate (within 3e-6 of
-// an fp64 dot) at a fraction of the instructions of a scalar loop (fp16, 600 tokens x 256 experts x 3072: scalar 245 us).
+// an fp64 dot) at a fraction of the instructions of a scalar loop (fp16, 600 tokens x 256 experts x 3072: scalar 148 us).
+// The tensor core cuts its running sums off instead of rounding them, by up to an ulp per product and always the same way, so for fp16
+// and fp32 rows a chain of products does not carry the sum: the leading products of 16 columns start from zero and are added with
+// rounding, the others, 2^-8 of them and less, have sums of their own. Relative error against fp64 (2-norm; a scalar fp32 loop,
+// one chain for all, this): h = 768 0.88e-7, 1.7e-7, 0.81e-7; 4096 1.28e-7, 3.3e-7 (fp32 4.0e-7), 0.9e-7; in router_tile_k 1.04e-7 where one chain had
+// 1.37e-6 (fp32 1.68e-6). bf16 rows, whose products lost three bits of the fp32 chain from the start, keep their one chain (2.2e-7; 8.2e-7).
 // One block = 16 router rows x 8 J tokens; its 16 warps split the hidden dimension and add their partial tiles in shared
 // memory in warp order. J is the smallest of 1, 2, 4, 8 that takes the batch, 8 above: with J = 8 one token pays for 64.
 template <int DT> constexpr int x_terms() { return DT == B2MOE_BF16 ? 1 : DT == B2MOE_F16 ? 2 : 3; }
@@ -106,14 +111,15 @@ __global__ void __launch_bounds__(RM_WARPS * 32) router_mma_k(const float * __re
     const int ra = min(r0 + g, rows - 1), rb = min(r0 + g + 8, rows - 1);
     const float * wa = ra == e ? shared : w + size_t(ra) * h, * wb = rb == e ? shared : w + size_t(rb) * h;
     float acc[J][4];
+    [[maybe_unused]] float low[J][4];                                   // fp16, fp32: the sums of all products but the leading one
 #pragma unroll
     for (int j = 0; j < J; ++j)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) acc[j][i] = 0.f;
+        for (int i = 0; i < 4; ++i) { acc[j][i] = 0.f; if (XT > 1) low[j][i] = 0.f; }
     const int hs = h / int(gridDim.z), h_lo = int(blockIdx.z) * hs;     // this block's columns (a multiple of 16)
     const int kper = (hs / 16 + RM_WARPS - 1) / RM_WARPS * 16;          // columns per warp, a multiple of 16
     const int k_lo = h_lo + warp * kper, k_hi = min(h_lo + hs, k_lo + kper);
-#pragma unroll 4
+#pragma unroll (XT == 1 ? 4 : 2)
     for (int k0 = k_lo; k0 < k_hi; k0 += 16) {
         uint32_t hi[4], mid[4], lo[4];
         split3(*reinterpret_cast<const float2 *>(wa + k0 + 2 * t), hi[0], mid[0], lo[0]);
@@ -127,13 +133,29 @@ __global__ void __launch_bounds__(RM_WARPS * 32) router_mma_k(const float * __re
             uint32_t b0[XT], b1[XT];
             x_pair<DT>(xr, b0);
             x_pair<DT>(xr + 8, b1);
+            if constexpr (XT == 1) {                                     // smallest terms first
+                mma_bf16_acc(acc[j], lo, b0[0], b1[0]);
+                mma_bf16_acc(acc[j], mid, b0[0], b1[0]);
+                mma_bf16_acc(acc[j], hi, b0[0], b1[0]);
+            } else {
 #pragma unroll
-            for (int xt = XT - 1; xt >= 0; --xt) {                       // smallest terms first
-                if (xt == 0 || DT == B2MOE_F16) mma_bf16_acc(acc[j], lo, b0[xt], b1[xt]);
-                if (xt < 2) mma_bf16_acc(acc[j], mid, b0[xt], b1[xt]);
-                mma_bf16_acc(acc[j], hi, b0[xt], b1[xt]);
+                for (int xt = XT - 1; xt >= 0; --xt) {
+                    if (xt == 0 || DT == B2MOE_F16) mma_bf16_acc(low[j], lo, b0[xt], b1[xt]);
+                    if (xt < 2) mma_bf16_acc(low[j], mid, b0[xt], b1[xt]);
+                    if (xt > 0) mma_bf16_acc(low[j], hi, b0[xt], b1[xt]);
+                }
+                float lead[4] = {0.f, 0.f, 0.f, 0.f};
+                mma_bf16_acc(lead, hi, b0[0], b1[0]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[j][i] += lead[i];
             }
         }
+    }
+    if constexpr (XT > 1) {
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[j][i] += low[j][i];
     }
     // warps 8..15 park their sums, warps 0..7 add theirs on top (always in this order: the same bits every run)
     if (warp >= RM_PART) {
@@ -179,7 +201,8 @@ __global__ void __launch_bounds__(RM_WARPS * 32) router_mma_k(const float * __re
 // One block = 64 router rows x 128 tokens, 8 warps of 32 x 32 outputs, 32 columns per stage: both operands are split into
 // their bf16 terms once per block and stage (not once per 64 tokens and warp as above) and reach the MMAs through ldmatrix, so
 // a stage of bf16 rows costs a warp 16 shared loads for its 48 MMAs. Every output is summed over the hidden dimension in
-// ascending column order (terms lo, mid, hi per 16 columns; 256 columns per partial sum): the same bits every run.
+// ascending column order (terms lo, mid, hi per 16 columns; 256 columns per partial sum): the same bits every run. fp16 and fp32 rows:
+// the leading products of a stage's two 16-column steps are added to each other, then to the partial sum (see above for the reason).
 // A launch has few such tiles (2047 tokens x 256 experts: 64), and a tile alone leaves an SM waiting on its own loads: up to
 // eight blocks of a cluster take a part of a tile's 256-column partial sums each and add all of them, in column order, through
 // distributed shared memory, so the split changes no bit.
@@ -276,13 +299,20 @@ __global__ void __launch_bounds__(RT_THREADS) router_tile_k(const float * __rest
     // acc sums 256 columns at a time and is then put away: the rounding error of a long fp32 chain grows with its
     // length, and the router's tolerance against an fp64 dot (3e-6) leaves no room for a 2048-term chain
     float acc[2][4][4];
+    [[maybe_unused]] float low[2][4][4];                               // fp16, fp32: the sums of all products but the leading one
     [[maybe_unused]] float tot[2][4][4];                               // one block per tile: it adds the partial sums up in registers
 #pragma unroll
     for (int a = 0; a < 2; ++a)
 #pragma unroll
         for (int b = 0; b < 4; ++b)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) { acc[a][b][c] = 0.f; if (!SPLIT) tot[a][b][c] = 0.f; }
+            for (int c = 0; c < 4; ++c) { acc[a][b][c] = 0.f; if (XT > 1) low[a][b][c] = 0.f; if (!SPLIT) tot[a][b][c] = 0.f; }
+    auto part_sum = [&](int a, int b, int c) {                         // the finished partial sum, and back to zero
+        const float v = XT > 1 ? acc[a][b][c] + low[a][b][c] : acc[a][b][c];
+        acc[a][b][c] = 0.f;
+        if (XT > 1) low[a][b][c] = 0.f;
+        return v;
+    };
     auto put_away = [&](uint8_t * at) {
         float * part = reinterpret_cast<float *>(at);
 #pragma unroll
@@ -290,10 +320,8 @@ __global__ void __launch_bounds__(RT_THREADS) router_tile_k(const float * __rest
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    part[(32 * wc + 8 * nt + 2 * t + (c & 1)) * RT_PLD + 32 * wr + 16 * rt + g + 8 * (c >> 1)] = acc[rt][nt][c];
-                    acc[rt][nt][c] = 0.f;
-                }
+                for (int c = 0; c < 4; ++c)
+                    part[(32 * wc + 8 * nt + 2 * t + (c & 1)) * RT_PLD + 32 * wr + 16 * rt + g + 8 * (c >> 1)] = part_sum(rt, nt, c);
     };
     // ldmatrix addresses of this lane inside a stage: A rows 32 wr + 16 rt + (lane % 16), columns 8 (lane / 16);
     // B tokens 32 wc + 16 pr + (lane % 8) + 8 (lane / 16), columns 8 ((lane / 8) % 2)
@@ -310,6 +338,7 @@ __global__ void __launch_bounds__(RT_THREADS) router_tile_k(const float * __rest
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();                                               // stage s is complete; every warp is done with stage s - 1
         if (s + 1 < s_hi) { load_x(buf ^ 1, (s + 1) * RT_K); load_w((s + 1) * RT_K); }
+        [[maybe_unused]] float lead[2][4][4];                          // the leading products of the stage's first 16 columns
 #pragma unroll
         for (int kk = 0; kk < RT_K / 16; ++kk) {
             uint32_t b[XT][2][4];                                      // per term, token tiles (0, 1) and (2, 3): b0, b1 of each
@@ -327,7 +356,22 @@ __global__ void __launch_bounds__(RT_THREADS) router_tile_k(const float * __rest
                     for (int q = XT - 1; q >= 0; --q)
 #pragma unroll
                         for (int nt = 0; nt < 4; ++nt)
-                            if (DT != B2MOE_F32 || term + q < 3) mma_bf16_acc(acc[rt][nt], a, b[q][nt >> 1][2 * (nt & 1)], b[q][nt >> 1][2 * (nt & 1) + 1]);
+                            if (DT != B2MOE_F32 || term + q < 3) {
+                                const uint32_t b0 = b[q][nt >> 1][2 * (nt & 1)], b1 = b[q][nt >> 1][2 * (nt & 1) + 1];
+                                if constexpr (XT == 1) {
+                                    mma_bf16_acc(acc[rt][nt], a, b0, b1);
+                                } else if (term + q > 0) {
+                                    mma_bf16_acc(low[rt][nt], a, b0, b1);
+                                } else {
+                                    float v[4] = {0.f, 0.f, 0.f, 0.f};
+                                    mma_bf16_acc(v, a, b0, b1);
+#pragma unroll
+                                    for (int c = 0; c < 4; ++c) {
+                                        if (kk == 0) lead[rt][nt][c] = v[c];
+                                        else acc[rt][nt][c] += lead[rt][nt][c] + v[c];
+                                    }
+                                }
+                            }
                 }
             }
         }
@@ -339,7 +383,7 @@ __global__ void __launch_bounds__(RT_THREADS) router_tile_k(const float * __rest
 #pragma unroll
                 for (int b = 0; b < 4; ++b)
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) { tot[a][b][c] += acc[a][b][c]; acc[a][b][c] = 0.f; }
+                    for (int c = 0; c < 4; ++c) tot[a][b][c] += part_sum(a, b, c);
         }
     }
     if constexpr (!SPLIT) {
