@@ -58,7 +58,8 @@ __global__ void router_k(const float * __restrict__ w, const float * __restrict_
 // one chain for all, this): h = 768 0.88e-7, 1.7e-7, 0.81e-7; 4096 1.28e-7, 3.3e-7 (fp32 4.0e-7), 0.9e-7; in router_tile_k 1.04e-7 where one chain had
 // 1.37e-6 (fp32 1.68e-6). bf16 rows, whose products lost three bits of the fp32 chain from the start, keep their one chain (2.2e-7; 8.2e-7).
 // One block = 16 router rows x 8 J tokens; its 16 warps split the hidden dimension and add their partial tiles in shared
-// memory in warp order. J is the smallest of 1, 2, 4, 8 that takes the batch, 8 above: with J = 8 one token pays for 64.
+// memory in warp order (a token's bits do not depend on J). J is the smallest of 1, 2, 4, 8 that takes the batch in one block or leaves
+// at most a block per SM: with J = 8 one token pays for 64.
 template <int DT> constexpr int x_terms() { return DT == B2MOE_BF16 ? 1 : DT == B2MOE_F16 ? 2 : 3; }
 constexpr int RM_WARPS = 16, RM_PART = 8;   // warps per block (each takes a slice of the columns); partial-sum slots in shared memory
 __device__ __forceinline__ void split3(float2 w, uint32_t & hi, uint32_t & mid, uint32_t & lo) {
@@ -693,6 +694,7 @@ int32_t route_plan_stage(int gating, const float * logits, int ld, const float *
     return launch_status();
 }
 namespace {
+constexpr int ROUTER_SMS = 148;
 template <typename... KArgs, typename... Args>
 int32_t launch_cluster_z(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t s, Args &&... args) {
     cudaLaunchConfig_t cfg = {};
@@ -713,27 +715,32 @@ int32_t launch_cluster_z(void (*kernel)(KArgs...), dim3 grid, int threads, size_
 template <int DT>
 int32_t router_launch(const float * w, const float * shared, const void * xv, float * logits, int ld, int h, int e, int rows, int n, cudaStream_t s) {
     const auto * x = static_cast<const typename Elem<DT>::type *>(xv);
-    // Tiles from 256 tokens for bf16 (below, router_mma_k has more blocks and no stage hand-offs); the split operands of the other
-    // types make router_mma_k split the same token values again for every 16 rows, so they change over at 128.
-    if (h % RT_K == 0 && n >= (DT == B2MOE_BF16 ? 2 : 1) * RT_TOK) {
+    // router_mma_k splits the hidden dimension over a cluster of up to 4 blocks while every block keeps at least 256 columns
+    int ks = 1;
+    while (ks < 4 && h % (32 * ks) == 0 && h / (2 * ks) >= 256) ks *= 2;
+    auto mma_blocks = [&](int tokens) { return (long long)ceil_div(rows, 16) * ceil_div(n, tokens) * ks; };
+    // Tiles from 256 tokens for bf16 (below, router_mma_k has more blocks and no stage hand-offs). fp16 and fp32 rows: once router_mma_k
+    // with its 64 tokens a block has more than two blocks per SM. router_mma_k / tiles, us: 1024 columns x 32 experts, fp16,
+    // 600 tokens 8.9 / 17.7, 2047 (256 blocks) 16.8 / 18.0, 4096 (512 blocks) 32 / 18; 2560 x 60, 600 tokens (160) 22.8 / 31, 2047 (512) 46 / 32;
+    // 3072 x 256, 256 tokens (256) 25 / 31, 300 (320) 36 / 31; 256 x 32 4096 tokens (128) 8.3 / 22.
+    if (h % RT_K == 0 && (DT == B2MOE_BF16 ? n >= 2 * RT_TOK : mma_blocks(64) > 2 * ROUTER_SMS)) {
         const dim3 tiles(ceil_div(rows, RT_ROWS), ceil_div(n, RT_TOK), 1);
         const int n_part = ceil_div(h, RT_COLS), share = ceil_div(n_part, 8), ks = ceil_div(n_part, share);      // at most eight blocks, no more than the shares need
         const size_t smem = rt_stages_bytes<DT>() + size_t(share - 1) * RT_PART;
         static_assert(rt_stages_bytes<DT>() >= RT_PART, "the last partial sum takes the stages' place");
-        const bool split = tiles.x * tiles.y < RT_SPLIT_BELOW && n_part <= RT_MAX_PARTS && smem <= 227 * 1024;
+        const bool split = n_part > 1 && tiles.x * tiles.y < RT_SPLIT_BELOW && n_part <= RT_MAX_PARTS && smem <= 227 * 1024;
         const auto kernel = split ? router_tile_k<DT, true> : router_tile_k<DT, false>;
         const size_t bytes = split ? smem : size_t(rt_stages_bytes<DT>());
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)) != cudaSuccess) return B2MOE_ERR_CUDA;
         return launch_cluster_z(kernel, dim3(tiles.x, tiles.y, split ? ks : 1), RT_THREADS, bytes, s, w, shared, x, logits, ld, h, e, rows, n);
     }
     if (h % 16 == 0) {
-        // split the hidden dimension over a cluster of up to 4 blocks while every block keeps at least 256 columns
-        int ks = 1;
-        while (ks < 4 && h % (32 * ks) == 0 && h / (2 * ks) >= 256) ks *= 2;
         auto launch = [&](auto kernel, int tokens) {
             return launch_cluster_z(kernel, dim3(ceil_div(rows, 16), ceil_div(n, tokens), ks), RM_WARPS * 32, 0, s, w, shared, x, logits, ld, h, e, rows, n);
         };
-        return n <= 8 ? launch(router_mma_k<DT, 1>, 8) : n <= 16 ? launch(router_mma_k<DT, 2>, 16) : n <= 32 ? launch(router_mma_k<DT, 4>, 32) : launch(router_mma_k<DT, 8>, 64);
+        // the fewest tokens a block that leave at most a block per SM: with 64, 64 tokens of 768 columns x 64 experts were 8 blocks
+        auto fits = [&](int tokens) { return n <= tokens || mma_blocks(tokens) <= ROUTER_SMS; };
+        return fits(8) ? launch(router_mma_k<DT, 1>, 8) : fits(16) ? launch(router_mma_k<DT, 2>, 16) : fits(32) ? launch(router_mma_k<DT, 4>, 32) : launch(router_mma_k<DT, 8>, 64);
     }
     router_k<DT><<<dim3(ceil_div(rows, 8), std::min(ceil_div(n, ROUTER_TOK), 64)), 256, 0, s>>>(w, shared, x, logits, ld, h, e, rows, n);
     return launch_status();
