@@ -96,6 +96,22 @@ template <int DT> __device__ __forceinline__ void x_pair(const typename Elem<DT>
         split3_pair(*reinterpret_cast<const float2 *>(p), v[0], v[1], v[2]);
     }
 }
+// A logit whose split products did not give a number: an infinity (or a value that rounds to one as bf16) leaves infinity minus
+// infinity behind when it is split, and meets zero terms of the other operand. In a plain loop one infinite activation gives
+// infinite logits of the weights' signs, as it should. A NaN ends the loop, so that rows of garbage cost little.
+template <int DT> __device__ __noinline__ float plain_logit(const float * w, const typename Elem<DT>::type * x, int h) {
+    float s = 0.f;
+    for (int j = 0; j < h && s == s; j += 4) {
+        const float4 v = *reinterpret_cast<const float4 *>(w + j);
+        s += v.x * Elem<DT>::to_f(x[j]) + v.y * Elem<DT>::to_f(x[j + 1]) + v.z * Elem<DT>::to_f(x[j + 2]) + v.w * Elem<DT>::to_f(x[j + 3]);
+    }
+    return s;
+}
+// the logit to store: the sum s of (router row, token), looked at again where fp16 or fp32 rows were split
+template <int DT> __device__ __forceinline__ float checked_logit(float s, const float * w, const float * shared, const typename Elem<DT>::type * x, int row, int tok, int e, int h) {
+    if (x_terms<DT>() > 1 && !isfinite(s)) return plain_logit<DT>(row == e ? shared : w + size_t(row) * h, x + size_t(tok) * h, h);
+    return s;
+}
 template <int DT, int J>
 __global__ void __launch_bounds__(RM_WARPS * 32) router_mma_k(const float * __restrict__ w, const float * __restrict__ shared,
                                                                 const typename Elem<DT>::type * x, float * logits, int ld,
@@ -191,7 +207,7 @@ __global__ void __launch_bounds__(RM_WARPS * 32) router_mma_k(const float * __re
             if (r0 + r < rows && t0 + c < n) {
                 float s = tile[r][c];
                 for (unsigned z = 1; z < gridDim.z; ++z) s += cluster.map_shared_rank(&tile[0][0], z)[r * 65 + c];
-                logits[size_t(t0 + c) * ld + r0 + r] = s;
+                logits[size_t(t0 + c) * ld + r0 + r] = checked_logit<DT>(s, w, shared, x, r0 + r, t0 + c, e, h);
             }
         }
     }
@@ -395,7 +411,7 @@ __global__ void __launch_bounds__(RT_THREADS) router_tile_k(const float * __rest
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const int row = r0 + 32 * wr + 16 * rt + g + 8 * (c >> 1), tok = t0 + 32 * wc + 8 * nt + 2 * t + (c & 1);
-                    if (row < rows && tok < n) logits[size_t(tok) * ld + row] = tot[rt][nt][c];
+                    if (row < rows && tok < n) logits[size_t(tok) * ld + row] = checked_logit<DT>(tot[rt][nt][c], w, shared, x, row, tok, e, h);
                 }
         return;
     }
@@ -430,7 +446,7 @@ __global__ void __launch_bounds__(RT_THREADS) router_tile_k(const float * __rest
 #pragma unroll
             for (int j = 0; j < 8; ++j) if (q + j < n_part) sum += v[j];
         }
-        logits[size_t(t0 + tk) * ld + r0 + r] = sum;
+        logits[size_t(t0 + tk) * ld + r0 + r] = checked_logit<DT>(sum, w, shared, x, r0 + r, t0 + tk, e, h);
     }
     cluster.sync();                                                    // the blocks' tiles stay alive until every block has read them
 }
