@@ -18,7 +18,7 @@ namespace b2 {
 namespace {
 
 constexpr int CHUNK = 256;   // assignments per warp-chunk on the multi-block path with counters in global memory
-constexpr int WALK_WARPS = 8, WALK_THREADS = WALK_WARPS * 32;
+constexpr int WALK_WARPS = 8, WALK_THREADS = WALK_WARPS * 32, WALK_MAX_BLOCKS = 148;
 
 __global__ void dispatch_small_k(const int * ids, int A, int e, int shared_first, int shared_tokens, int * __restrict__ plan) {
     extern __shared__ unsigned short hist[];       // [32 warps][e]
@@ -107,8 +107,8 @@ __global__ void __launch_bounds__(WALK_THREADS) dispatch_place_k(const WalkArgs 
 }
 // Assignments per warp: 128 (four steps; a block of eight warps takes 1,024) while that makes at most a block per SM, and
 // beyond that what a block per SM leaves, since every block reads every row.
-inline int walk_seg(int A) { return std::max(128, (ceil_div(A, 148 * WALK_WARPS) + 31) / 32 * 32); }
-inline int walk_blocks(int A) { return ceil_div(A, walk_seg(A) * WALK_WARPS); }
+inline int walk_seg(int A) { return std::max(128, (ceil_div(A, WALK_MAX_BLOCKS * WALK_WARPS) + 31) / 32 * 32); }
+inline int walk_blocks(int A) { return ceil_div(A, walk_seg(A) * WALK_WARPS); }         // at most WALK_MAX_BLOCKS
 // the counters have to fit a block's ordinary shared memory: up to about 900 experts
 inline bool walk_path(int e) { return walk_smem(e) <= 46 * 1024; }
 
@@ -187,7 +187,10 @@ extern "C" B2MOE_API void b2moe_plan_view_of(int32_t experts, int32_t assignment
 extern "C" B2MOE_API size_t b2moe_dispatch_workspace_bytes(int32_t experts, int32_t assignments) {
     if (experts <= 0 || assignments < 0) return 0;
     if (small_path(experts, assignments)) return 16;
-    return align_up(size_t(walk_path(experts) ? walk_blocks(assignments) : ceil_div(assignments, CHUNK)) * experts * sizeof(int), 16);
+    // a size that grows with the assignments, so that scratch for the largest batch serves every smaller one: the number of blocks does
+    // not (151,552 ids take 148 blocks, one more 119)
+    const int rows = walk_path(experts) ? std::min(ceil_div(assignments, 128 * WALK_WARPS), WALK_MAX_BLOCKS) : ceil_div(assignments, CHUNK);
+    return align_up(size_t(rows) * experts * sizeof(int), 16);
 }
 
 extern "C" B2MOE_API int32_t b2moe_dispatch_range(const int32_t * ids, int32_t n, int32_t topk, int32_t experts, int32_t shared_first,
