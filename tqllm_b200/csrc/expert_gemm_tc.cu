@@ -662,13 +662,16 @@ int32_t convert_rows_dt(const void * xv, int rows_x, int slot_rows, bool slots, 
     return launch_status();
 }
 // m: the banks (gate, up) or (down, null), then the shared expert's (null: none); x (rows_x rows, in token order when map_topk > 0, in
-// assignment order otherwise) -> fp16 rows in xb (in slot order: slot_rows of them; slot_of: scratch for MODE 0), then the product
+// assignment order otherwise), live: how many of the a.A assignments are expected to be grouped -> fp16 rows in xb (in slot order: slot_rows of them; slot_of: scratch for MODE 0), then the product
 template <uint32_t T, int MODE>
-int32_t gemm_launch_t(GemmArgs a, const b2moe_bank * const * m, const void * x, int dtype, int rows_x, int map_topk, bool slots, int slot_rows, __half * xb, float * inv, int * slot_of,
+int32_t gemm_launch_t(GemmArgs a, long long live, const b2moe_bank * const * m, const void * x, int dtype, int rows_x, int map_topk, bool slots, int slot_rows, __half * xb, float * inv, int * slot_of,
                       cudaStream_t s) {
     const int sms = gemm_sm_count();
     if (sms <= 0) return B2MOE_ERR_CUDA;
-    const long long per = (long long)a.A / a.experts;                 // mean tokens per expert
+    const long long per = live / a.experts;                           // mean tokens per expert
+    // The width of the items. Gate/up with items of 64 / 128 / 256 tokens, us: NVFP4 (512 experts) 24 per expert 235 / 235 / 279, 64: 342 / 265 / 315,
+    // 112: 488 / 339 / 374, 144: 674 / 553 / 464; IQ4 (128 experts) 24: 317 / 317 / 366, 64: 496 / 388 / 431, 112: 702 / 469 / 486, 144: 998 / 800 / 585; Q4_K (256
+    // experts) 24: 651 / 652 / 646, 64: 978 / 711 / 718, 112: 1385 / 908 / 881, 144: 1932 / 1427 / 993. The narrow ones leave room for more raw slots.
     const int cap = g_item_tokens == 256 || per > 128 ? 256 : per > 24 ? 128 : 64;
     if (!gemm_fit<T>(a.experts, cap, a)) return B2MOE_ERR_SHAPE;
     const int rows = slots ? slot_rows : rows_x, topk = map_topk;
@@ -729,8 +732,8 @@ size_t gemm_tc_workspace_bytes(int rows_x, int k) {
 
 // rows_buf: optional scratch for the activation rows in slot order (n * topk + shared_tokens rows of length k, their scales and an index each)
 int32_t gemm_tc_gateup(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_bank * sg, const b2moe_bank * su, const void * x,
-                       int x_dtype, const int * plan, int n, int topk, int shared_tokens, void * act, int act_dtype, void * ws, void * rows_buf,
-                       size_t rows_buf_bytes, cudaStream_t s) {
+                       int x_dtype, const int * plan, int n, int topk, int shared_tokens, long long live, void * act, int act_dtype, void * ws,
+                       void * rows_buf, size_t rows_buf_bytes, cudaStream_t s) {
     const int k = gate->cols, slot_rows = n * topk + shared_tokens;
     const bool slots = rows_buf && rows_buf_bytes >= gemm_tc_workspace_bytes(slot_rows, k) + size_t(slot_rows) * sizeof(int);
     int * slot_of = slots ? reinterpret_cast<int *>(static_cast<uint8_t *>(rows_buf) + gemm_tc_workspace_bytes(slot_rows, k)) : nullptr;
@@ -742,12 +745,12 @@ int32_t gemm_tc_gateup(const b2moe_bank * gate, const b2moe_bank * up, const b2m
     if (shared_tokens) { a.saux0 = static_cast<const float *>(sg->aux); a.saux1 = static_cast<const float *>(su->aux); }
     a.plan = const_cast<int *>(plan); a.out = act; a.out_dtype = act_dtype;
     a.rows = gate->rows; a.k = k; a.experts = gate->experts; a.topk = topk; a.A = n * topk;
-    return gemm_launch<0>(gate->type, a, banks, x, x_dtype, n, topk, slots, slot_rows, xb, inv, slot_of, s);
+    return gemm_launch<0>(gate->type, a, live, banks, x, x_dtype, n, topk, slots, slot_rows, xb, inv, slot_of, s);
 }
 
 // per_token: x has a row per token instead of one per assignment (shared_tokens = 0)
 int32_t gemm_tc_down(const b2moe_bank * down, const b2moe_bank * sd, const void * x, int x_dtype, bool per_token, const int * plan, int n, int topk,
-                     int shared_tokens, void * y, int y_dtype, void * ws, cudaStream_t s) {
+                     int shared_tokens, long long live, void * y, int y_dtype, void * ws, cudaStream_t s) {
     const int rows_x = n * topk + shared_tokens, k = down->cols;
     __half * xb = static_cast<__half *>(ws);
     float * inv = reinterpret_cast<float *>(static_cast<uint8_t *>(ws) + align_up(size_t(rows_x) * k * 2, 256));
@@ -757,7 +760,7 @@ int32_t gemm_tc_down(const b2moe_bank * down, const b2moe_bank * sd, const void 
     if (shared_tokens) a.saux0 = static_cast<const float *>(sd->aux);
     a.plan = const_cast<int *>(plan); a.out = y; a.out_dtype = y_dtype;
     a.rows = down->rows; a.k = k; a.experts = down->experts; a.topk = topk; a.A = n * topk;
-    return gemm_launch<1>(down->type, a, banks, x, x_dtype, per_token ? n : rows_x, per_token ? topk : 0, true, rows_x, xb, inv, static_cast<int *>(nullptr), s);
+    return gemm_launch<1>(down->type, a, live, banks, x, x_dtype, per_token ? n : rows_x, per_token ? topk : 0, true, rows_x, xb, inv, static_cast<int *>(nullptr), s);
 }
 
 }  // namespace b2

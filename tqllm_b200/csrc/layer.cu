@@ -34,9 +34,9 @@ bool g_overlap = true;
 bool gemm_tc_supported(uint32_t type, int k, int experts);
 size_t gemm_tc_workspace_bytes(int rows_x, int k);
 int32_t gemm_tc_gateup(const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const void *, int, const int *, int,
-                       int, int, void *, int act_dtype, void *, void * rows_buf, size_t rows_buf_bytes, cudaStream_t);
-int32_t gemm_tc_down(const b2moe_bank *, const b2moe_bank *, const void *, int x_dtype, bool per_token, const int *, int, int, int, void *, int y_dtype,
-                     void *, cudaStream_t);
+                       int, int, long long live, void *, int act_dtype, void *, void * rows_buf, size_t rows_buf_bytes, cudaStream_t);
+int32_t gemm_tc_down(const b2moe_bank *, const b2moe_bank *, const void *, int x_dtype, bool per_token, const int *, int, int, int, long long live, void *,
+                     int y_dtype, void *, cudaStream_t);
 void gemm_tc_item_tokens(int tokens);
 
 namespace {
@@ -88,7 +88,7 @@ int32_t product_typed(const b2moe_bank * m, const void * x, int x_dtype, bool pe
                       void * ws, cudaStream_t s, bool * took) {
     const int path = expert_path(m->type, m->cols, B2MOE_F32, m->experts, (long long)n * topk);
     *took = true;
-    if (path == B2MOE_FAMILY_GEMM) return gemm_tc_down(m, nullptr, x, x_dtype, per_token, plan, n, topk, 0, y, y_dtype, ws, s);
+    if (path == B2MOE_FAMILY_GEMM) return gemm_tc_down(m, nullptr, x, x_dtype, per_token, plan, n, topk, 0, (long long)n * topk, y, y_dtype, ws, s);
     if (path == B2MOE_FAMILY_DECODE && decode_kernel(m->type, m->cols, B2MOE_F32) == DEC_4BIT)
         return dec4_down(m, nullptr, x, x_dtype, per_token, plan, n, topk, 0, y, y_dtype, ws, s);
     *took = false;
@@ -99,7 +99,8 @@ int32_t gateup_typed(const b2moe_bank * gate, const b2moe_bank * up, const void 
                      void * ws, void * rows_buf, size_t rows_buf_bytes, cudaStream_t s, bool * took) {
     const int path = expert_path(gate->type, gate->cols, x_dtype, gate->experts, (long long)n * topk);
     *took = true;
-    if (path == B2MOE_FAMILY_GEMM) return gemm_tc_gateup(gate, up, nullptr, nullptr, x, x_dtype, plan, n, topk, 0, act, act_dtype, ws, rows_buf, rows_buf_bytes, s);
+    if (path == B2MOE_FAMILY_GEMM) return gemm_tc_gateup(gate, up, nullptr, nullptr, x, x_dtype, plan, n, topk, 0, (long long)n * topk, act, act_dtype, ws, rows_buf,
+                                                               rows_buf_bytes, s);
     if (path == B2MOE_FAMILY_DECODE && decode_kernel(gate->type, gate->cols, x_dtype) == DEC_4BIT)
         return dec4_gateup(gate, up, nullptr, nullptr, x, x_dtype, plan, n, topk, 0, act, act_dtype, ws, s, false);
     *took = false;
@@ -172,7 +173,8 @@ static int32_t expert_gateup(const b2moe_bank * gate, const b2moe_bank * up, con
     }
     if (!x || !plan || !act) return B2MOE_ERR_NULL;
     if (!aligned16(x) || !aligned16(act)) return B2MOE_ERR_ALIGN;
-    const int path = expert_path(gate->type, gate->cols, x_dtype, gate->experts, live >= 0 ? live : (long long)n * topk);
+    if (live < 0) live = (long long)n * topk;
+    const int path = expert_path(gate->type, gate->cols, x_dtype, gate->experts, live);
     if (path != B2MOE_FAMILY_GENERIC) {
         const size_t need = b2moe_expert_workspace_bytes(gate->type, n, gate->cols, x_dtype);
         if (need && !workspace) return B2MOE_ERR_NULL;
@@ -181,7 +183,7 @@ static int32_t expert_gateup(const b2moe_bank * gate, const b2moe_bank * up, con
         // a workspace larger than it has to be may hold the rows in slot order itself (gemm_tc_gateup looks at its size): IQ4 banks,
         // 8192 tokens of 8, gate/up alone 4020 us with gathered rows and 1430 with slot order
         if (path == B2MOE_FAMILY_GEMM)
-            return gemm_tc_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, B2MOE_F32, workspace,
+            return gemm_tc_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, live, act, B2MOE_F32, workspace,
                                   rows_buf ? rows_buf : workspace, rows_buf ? rows_buf_bytes : workspace_bytes, as_stream(stream));
         if (decode_kernel(gate->type, gate->cols, x_dtype) == DEC_4BIT)
             return dec4_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, B2MOE_F32, workspace, as_stream(stream), x_staged);
@@ -207,14 +209,15 @@ static int32_t expert_down(const b2moe_bank * down, const b2moe_bank * shared_do
     }
     if (!act || !plan || !y) return B2MOE_ERR_NULL;
     if (!aligned16(act) || !aligned16(y)) return B2MOE_ERR_ALIGN;
-    const int path = expert_path(down->type, down->cols, B2MOE_F32, down->experts, live >= 0 ? live : (long long)n * topk);
+    if (live < 0) live = (long long)n * topk;
+    const int path = expert_path(down->type, down->cols, B2MOE_F32, down->experts, live);
     if (path != B2MOE_FAMILY_GENERIC) {
         const int rows_x = n * topk + shared_tokens;
         if (!workspace) return B2MOE_ERR_NULL;
         if (!aligned16(workspace)) return B2MOE_ERR_ALIGN;
         if (workspace_bytes < b2moe_expert_workspace_bytes(down->type, rows_x, down->cols, B2MOE_F32)) return B2MOE_ERR_WORKSPACE;
         if (path == B2MOE_FAMILY_GEMM)
-            return gemm_tc_down(down, shared_down, act, B2MOE_F32, false, plan, n, topk, shared_tokens, y, B2MOE_F32, workspace, as_stream(stream));
+            return gemm_tc_down(down, shared_down, act, B2MOE_F32, false, plan, n, topk, shared_tokens, live, y, B2MOE_F32, workspace, as_stream(stream));
         if (decode_kernel(down->type, down->cols, B2MOE_F32) == DEC_4BIT)
             return dec4_down(down, shared_down, act, B2MOE_F32, false, plan, n, topk, shared_tokens, y, B2MOE_F32, workspace, as_stream(stream));
         return iq3s_down(down, shared_down, act, plan, n, topk, shared_tokens, y, workspace, max_active_of(down->experts, n, topk, shared_tokens), as_stream(stream));
