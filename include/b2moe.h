@@ -160,8 +160,8 @@ B2MOE_API int32_t b2moe_plan_to_groups(const int32_t * plan, int32_t n, int32_t 
  * Scratch: the tensor-core kernels first bring the activation rows into operand form (one fp16 term per value, the row
  * scaled by a power of two, + that scale) inside a caller-provided workspace of b2moe_expert_workspace_bytes(type, rows_x, k, x_dtype) bytes (16-byte aligned), where
  * rows_x = n for the gate/up product (k = hidden) and n*topk + shared_tokens for the down product (k = ff, x_dtype
- * B2MOE_F32). The workspace may be NULL only where the size is 0. Prefill-sized gate/up calls are faster (up to three
- * times) with a larger one: that of rows_x = n*topk + shared_tokens rows and 4 bytes more for each of them. */
+ * B2MOE_F32). The workspace may be NULL only where the size is 0. Gate/up calls of many tokens per
+ * expert are faster (up to one and a half times) with a larger one: that of rows_x = n*topk + shared_tokens rows and 4 bytes more for each of them. */
 B2MOE_API size_t b2moe_expert_workspace_bytes(uint32_t type, int32_t rows_x, int32_t k, int32_t x_dtype);
 /* act[a][f] = silu(gate_e(a)[f] . x[token(a)]) * (up_e(a)[f] . x[token(a)]) for every grouped assignment a: the
  * paired gate/up product with the SwiGLU fused (replaces expert_matvec2 / expert_matvec_dedup2 / expert_gemm_gateup +

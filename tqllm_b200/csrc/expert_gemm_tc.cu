@@ -25,9 +25,9 @@
 // loops, one elected lane issues, and the raw blocks and rows come in the largest boxes that fit. They are the first warps of the
 // block: as the last ones they were served last (c3 decode gate/up 110 us, as the first 78).
 // Warps: 0 issues tcgen05.mma; 1 streams the raw blocks (256 columns of the item's eight row tiles per ring slot: one TMA box
-// of the down bank, one each of gate and up, running ahead across items); 2 (and 3 when it gathers) loads B; 4..11 epilogue (two
-// per TMEM lane quarter, 16-token groups in turn); 12..27 decode A (warp 12 + j: lane quarter j & 3, row tile (j >> 2) & 1 of
-// it, unit j >> 3 of every 256-column chunk). One barrier per step says that its products are done (a commit costs the issuing thread
+// of the down bank, one each of gate and up, running ahead across items); 2 (when it gathers 2..7) loads B; then from 4 (8) on
+// eight epilogue warps (two per TMEM lane quarter, 16-token groups in turn) and sixteen that decode A (the j-th: lane quarter j & 3, row tile
+// (j >> 2) & 1 of it, unit j >> 3 of every 256-column chunk). One barrier per step says that its products are done (a commit costs the issuing thread
 // 60 cycles): it frees the unit's A stage and the step's B stage. Every wait is bounded; a wait that runs out sets the plan's
 // status word, and the block drains and leaves.
 //
@@ -54,8 +54,10 @@ constexpr int STEP_RING = 2 * A_STAGES;     // barriers "the products of step g 
 constexpr int ACC_COLS = 128, A_COL0 = 2 * ACC_COLS;                // the two accumulators, then the A stages: all 512 columns
 constexpr int SPLIT_COLS = ACC_COLS / 2;    // items of up to this many tokens split their K over the halves of the accumulator
 constexpr int MAX_B_STAGES = 8, RAW_SLOTS = 6, MAX_CAP = 256;
-constexpr int MMA_WARP = 0, RAW_WARP = 1, LOAD_WARP0 = 2, LOAD_WARPS = 2, EPI_WARP0 = 4, EPI_WARPS = 8, DEC_WARP0 = 12, DEC_WARPS = 16;
-constexpr int G_THREADS = (DEC_WARP0 + DEC_WARPS) * 32;
+constexpr int MMA_WARP = 0, RAW_WARP = 1, LOAD_WARP0 = 2, EPI_WARPS = 8, DEC_WARPS = 16;
+// warps that load rows: one with boxes (and one idle: the roles behind start at a multiple of four, a TMEM lane quarter each), six gather
+constexpr int load_warps(bool gather) { return gather ? 6 : 2; }
+constexpr int g_threads(bool gather) { return (LOAD_WARP0 + load_warps(gather) + EPI_WARPS + DEC_WARPS) * 32; }
 static_assert(EPI_WARPS * 32 == MAX_CAP, "an epilogue thread looks one token up");
 static_assert(MAX_B_STAGES <= STEP_RING, "a B stage is freed by the barrier of the step that used it");
 constexpr int N_BARS = 2 * RAW_SLOTS + A_STAGES + STEP_RING + MAX_B_STAGES + 6;
@@ -69,7 +71,6 @@ struct GemmArgs {
     int rows, k, experts, topk, A;
     int cap, cap_log2, b_stages, raw_slots; // most tokens of an item; B stages; raw chunks in the ring
     int b_pair;                             // 1: the B stages are filled and freed a unit at a time, beside the A stage of the unit and through its barriers (b_stages = 2 A_STAGES)
-    int slots;                              // 1: the activation rows lie in slot order; 0: in token (row) order, and are gathered
 };
 // x[i]: the activation rows, boxes of (i + 1) cap / 4 rows (a gathering launch: x[0], one row); w: banks (gate, up) or (down, -), then the shared expert's
 struct GemmMaps { CUtensorMap x[4], w[4]; };
@@ -208,11 +209,14 @@ __global__ void tokens_to_slots_k(const typename Elem<DT>::type * x, const int *
 // MODE 0: act[a][r] = silu(gate_r . x_tok(a)) * (up_r . x_tok(a));  MODE 1: y[a][r] = down_r . act[a]
 // F32_OUT: an instance for fp32 results and one for 16-bit ones, chosen by the call's output type. A branch at the stores, or two
 // loops in one kernel, cost every fp32 caller: c3 down (80 tokens x K = 512) 262 us against 184, c5 gate/up 1305 against 1240.
-template <uint32_t T, int MODE, bool F32_OUT>
-__global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, const __grid_constant__ GemmMaps maps) {
+// GATHER: the activation rows lie in token order.
+template <uint32_t T, int MODE, bool F32_OUT, bool GATHER>
+__global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs p, const __grid_constant__ GemmMaps maps) {
     using D = gdec::Dec<T>;
     constexpr int CB = chunk_bytes<T>();
     constexpr int ITEM_TILES = MODE == 0 ? 4 : 8;                      // row tiles of one matrix that an item covers
+    constexpr int LOAD_WARPS = load_warps(GATHER), EPI_WARP0 = LOAD_WARP0 + LOAD_WARPS, DEC_WARP0 = EPI_WARP0 + EPI_WARPS, G_THREADS = g_threads(GATHER);
+    static_assert(EPI_WARP0 % 4 == 0 && DEC_WARP0 % 4 == 0, "warp w reaches the tensor-memory lanes of quarter w % 4");
     extern __shared__ uint8_t smem_raw[];
     uint8_t * smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t * b_st = smem;                                            // [b_stages][cap][128 bytes], swizzled
@@ -239,11 +243,11 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
 #pragma unroll 1
         for (int i = 0; i < RAW_SLOTS; ++i) { bar_init(raw_full + 8 * i, 1); bar_init(raw_empty + 8 * i, DEC_WARPS); }
 #pragma unroll 1
-        for (int i = 0; i < A_STAGES; ++i) bar_init(a_full + 8 * i, p.b_pair ? 8 + (p.slots ? 1 : LOAD_WARPS) : 8);
+        for (int i = 0; i < A_STAGES; ++i) bar_init(a_full + 8 * i, p.b_pair ? 8 + (GATHER ? LOAD_WARPS : 1) : 8);
 #pragma unroll 1
         for (int i = 0; i < STEP_RING; ++i) bar_init(done + 8 * i, 1);
 #pragma unroll 1
-        for (int i = 0; i < MAX_B_STAGES; ++i) bar_init(b_full + 8 * i, p.slots ? 1 : LOAD_WARPS);
+        for (int i = 0; i < MAX_B_STAGES; ++i) bar_init(b_full + 8 * i, GATHER ? LOAD_WARPS : 1);
         for (int i = 0; i < 2; ++i) { bar_init(acc_full + 8 * i, 1); bar_init(acc_empty + 8 * i, EPI_WARPS); }
         bar_init(drain, 1);
         bar_init(tok_bar, EPI_WARPS);
@@ -319,7 +323,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
             mine = make_int2(-1, 0);
             if (tid < im.nv) {
                 mine.x = perm[im.slot0 + tid];
-                mine.y = __float_as_int(p.inv_scale[p.slots ? im.slot0 + tid : x_row(mine.x)]);
+                mine.y = __float_as_int(p.inv_scale[GATHER ? x_row(mine.x) : im.slot0 + tid]);
             }
         };
         auto put = [&](uint32_t n) {                                   // the table of the block's n-th item; then a (bounded) meeting of the warps
@@ -470,7 +474,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
             next = wide ? 0 : next ^ 1u;
             const uint32_t npad = uint32_t(max(im.nv, 1) + 15) & ~15u, id = idesc(128, npad, 0), d = tmem + h * ACC_COLS;
             const uint32_t second = im.nv <= SPLIT_COLS ? SPLIT_COLS : 0;          // columns from the accumulator of even products to that of odd ones
-            const uint32_t b_half = p.slots ? (uint32_t(b_class(im.nv) + 1) * (p.cap / 4) * 128) >> 4 : b_step;       // from the first to the second step of a pair
+            const uint32_t b_half = GATHER ? b_step : uint32_t(b_class(im.nv) + 1) * (b_step >> 2);       // from the first to the second step of a pair
             if (wide || h == 0) { if (uses0 > 0) ok = warp_wait(acc_empty, (uses0 - 1) & 1u) && ok; ++uses0; }
             if (wide || h == 1) { if (uses1 > 0) ok = warp_wait(acc_empty + 8, (uses1 - 1) & 1u) && ok; ++uses1; }
             fence_after();
@@ -533,27 +537,29 @@ __global__ void __launch_bounds__(G_THREADS, 1) gemm_tc_k(const GemmArgs p, cons
 #pragma unroll 1
         for (uint32_t i = issued > uint32_t(S) ? issued - S : 0; i < issued; ++i) bar_wait(raw_full + 8 * (i % S), (i / S) & 1u);
     } else {
-        // ---- B loader: warp 2 brings a step's (or a unit's) rows with one box; a gathering launch: lane l of warp w brings rows
-        // 4 (2 l + w) .. + 3 ----
-        const int lw = warp - LOAD_WARP0, n0 = 4 * (2 * lane + lw), group = p.b_pair ? 2 : 1;      // steps that share a barrier
+        // ---- B loader: warp 2 brings a step's (or a unit's) rows with one box; a gathering launch: lane l of loader w brings rows
+        // 4 (6 l + w) .. + 3. Issuing sets the pace of a gather (90 to 120 cycles per four rows and warp), so it takes
+        // all the threads that a block may have, with 64 registers. With two loaders / with six / from slot order, us: NVFP4 of 2048 columns, 10 tokens per
+        // expert 260 / 252 / 228, 80: 571 / 375 / 309; IQ4 of 4096 columns, 512: 3680 / 2050 / 1415; Q4_K of 3072 columns, 64: 1050 / 788 / 653 ----
+        const int lw = warp - LOAD_WARP0, n0 = 4 * (LOAD_WARPS * lane + lw), group = p.b_pair ? 2 : 1;      // steps that share a barrier
         uint32_t gk = 0, sb = 0;
         bool ok = true;
 #pragma unroll 1
-        for (int it = blockIdx.x; it < n_items && ok && !*abort_flag && (lw == 0 || !p.slots); it += gridDim.x) {
+        for (int it = blockIdx.x; it < n_items && ok && !*abort_flag && (lw == 0 || GATHER); it += gridDim.x) {
             const Item im = locate(it, at);
             int row[4] = {0, 0, 0, 0};
-            if (!p.slots) {
+            if constexpr (GATHER) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) row[i] = n0 < im.nv ? x_row(perm[im.slot0 + min(n0 + i, im.nv - 1)]) : 0;      // past the last token: repeat it (dead columns of D)
             }
-            const int cls = b_class(im.nv), quads = (im.nv + 3) >> 2, mine = (quads + 1 - lw) >> 1;
+            const int cls = b_class(im.nv), quads = (im.nv + 3) >> 2, mine = (quads + LOAD_WARPS - 1 - lw) / LOAD_WARPS;
             const uint32_t box_bytes = uint32_t((cls + 1) * (p.cap / 4) * group) * 128u;
 #pragma unroll 1
             for (int ks = 0; ks < 2 * nunits; ks += group, gk += group) {
                 const uint32_t freed = gk + group - 1 - uint32_t(BS);  // the (last) step that used the stage before
                 if (gk >= uint32_t(BS) && !warp_wait(done + 8 * (freed % STEP_RING), (freed / STEP_RING) & 1u)) { ok = false; break; }
                 const uint32_t bar = p.b_pair ? a_full + 4 * sb : b_full + 8 * sb, dst = saddr(b_st) + sb * uint32_t(p.cap * 128);
-                if (p.slots) {
+                if constexpr (!GATHER) {
                     if (elect_one()) {
                         bar_expect_tx(bar, box_bytes);
                         tma_load_3d(dst, maps.x + cls, 0, im.slot0, ks, bar);      // the second step of an odd K's last unit lies outside: zeros
@@ -680,7 +686,6 @@ int32_t gemm_launch_t(GemmArgs a, long long live, const b2moe_bank * const * m, 
     else if (dtype == B2MOE_F16) rc = convert_rows_dt<T, B2MOE_F16>(x, rows_x, slot_rows, slots, topk, a, xb, inv, slot_of, s);
     else if (dtype == B2MOE_BF16) rc = convert_rows_dt<T, B2MOE_BF16>(x, rows_x, slot_rows, slots, topk, a, xb, inv, slot_of, s);
     if (rc) return rc;
-    a.slots = slots;
     a.inv_scale = inv;
     GemmMaps maps;
     bool mapped = true;
@@ -690,9 +695,14 @@ int32_t gemm_launch_t(GemmArgs a, long long live, const b2moe_bank * const * m, 
         if (m[i]) mapped = mapped && bank_map<T>(maps.w[i], m[i], MODE == 0 ? 4 : 8);
     if (!mapped) return B2MOE_ERR_CUDA;
     const size_t smem = gemm_smem<T>(a.experts, a.cap, a.b_stages, a.raw_slots);
-    const auto kernel = a.out_dtype == B2MOE_F32 ? gemm_tc_k<T, MODE, true> : gemm_tc_k<T, MODE, false>;
+    auto kernel = a.out_dtype == B2MOE_F32 ? gemm_tc_k<T, MODE, true, false> : gemm_tc_k<T, MODE, false, false>;
+    if constexpr (MODE == 0)
+        if (!slots) {
+            if (a.out_dtype != B2MOE_F32) return B2MOE_ERR_SHAPE;      // calls with 16-bit results bring scratch for the rows in slot order
+            kernel = gemm_tc_k<T, MODE, true, true>;
+        }
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return B2MOE_ERR_CUDA;
-    launch_overlapped(kernel, dim3(sms), dim3(G_THREADS), smem, s, a, maps);
+    launch_overlapped(kernel, dim3(sms), dim3(g_threads(!slots)), smem, s, a, maps);
     return launch_status();
 }
 template <int MODE, typename... Args>
