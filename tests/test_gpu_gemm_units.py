@@ -1,6 +1,8 @@
 """GPU: the grouped GEMM where its unit of two 64-column steps does not divide the rows: odd numbers of units, a last unit of one
-step, several items per block, at the three item widths (64, 128, 192 tokens), rows in slot order and gathered. Against the
+step, several items per block, at the three item widths (64, 128, 256 tokens), rows in slot order and gathered. Against the
 exact fp32 kernels of the library; bound as in test_gpu_gemm.py (weights and activations rounded to fp16: 1e-2 of the RMS)."""
+import ctypes as C
+
 import pytest
 import torch
 
@@ -28,9 +30,15 @@ def test_ragged_units(types, hidden, ff, tokens):
         art = dev.artefacts()
         assert art["status"] == 0, "a bounded wait ran out"
     assert rel_err(out["gemm"], out["generic"]) <= TOL
-    # the product alone has no room for the rows in slot order and gathers them
+    # the product alone with the smallest workspace has no room for the rows in slot order and gathers them
     plan = moe.dispatch(art["ids"].clone(), 16, tokens)
+    slots, t = tokens * 4 + tokens, types[0]
+    small = capi.lib.b2moe_expert_workspace_bytes(t, tokens, hidden, capi.BF16)
+    assert small < slots * (2 * hidden + 8)
+    act, ws = torch.zeros(slots, ff, device="cuda"), torch.empty(small, dtype=torch.uint8, device="cuda")
+    ref = lambda b: C.byref(b.c)
     with capi.family("gemm"):
-        act = moe.expert_gateup_swiglu(dev.gate, dev.up, x, plan, dev.sh[0], dev.sh[1])
+        capi.check(capi.lib.b2moe_expert_gateup_swiglu(ref(dev.gate), ref(dev.up), ref(dev.sh[0]), ref(dev.sh[1]), x.data_ptr(), capi.BF16, plan.buf.data_ptr(),
+                                                       tokens, 4, tokens, act.data_ptr(), ws.data_ptr(), small, torch.cuda.current_stream().cuda_stream), "gateup")
     assert int(plan.buf[3]) == 0
-    assert torch.equal(act, dev.artefacts()["act"])
+    assert torch.equal(act, art["act"])
