@@ -15,7 +15,7 @@
 
 namespace b2 {
 int32_t check_bank(const b2moe_bank * b);
-size_t gemm_tc_workspace_bytes(int rows_x, int k);
+size_t gemm_tc_slot_bytes(int slot_rows, int k);
 int32_t product_typed(const b2moe_bank * m, const void * x, int x_dtype, bool per_token, const int * plan, int n, int topk, void * y, int y_dtype,
                       void * ws, cudaStream_t s, bool * took);
 int32_t gateup_typed(const b2moe_bank * gate, const b2moe_bank * up, const void * x, int x_dtype, const int * plan, int n, int topk, void * act, int act_dtype,
@@ -130,7 +130,7 @@ Parts carve(void * ws, size_t bytes, const b2moe_bank * b, int A, int rows_x, in
     p.dws = c.take(p.dws_bytes);
     p.x32 = static_cast<float *>(c.take(size_t(rows_x) * b->cols * sizeof(float)));
     p.y32_bytes = size_t(A) * out_cols * sizeof(float);
-    if (slot_rows) p.y32_bytes = std::max(p.y32_bytes, gemm_tc_workspace_bytes(slot_rows, b->cols) + size_t(slot_rows) * sizeof(int));
+    if (slot_rows) p.y32_bytes = std::max(p.y32_bytes, gemm_tc_slot_bytes(slot_rows, b->cols));
     p.y32 = static_cast<float *>(c.take(p.y32_bytes));
     p.ews_bytes = ews_bytes;
     p.ews = c.take(ews_bytes);
@@ -222,7 +222,9 @@ extern "C" B2MOE_API int32_t b2moe_expert_gemm_gateup(const b2moe_bank * gate, c
     if (!x || !act || !counts || !groups || !workspace) return B2MOE_ERR_NULL;
     if (!aligned16(x) || !aligned16(act) || !aligned16(workspace)) return B2MOE_ERR_ALIGN;
     const int A = n * topk;
-    const Parts p = carve(workspace, workspace_bytes, gate, A, 0, gate->rows, b2moe_expert_workspace_bytes(gate->type, n, gate->cols, x_dtype), A);
+    const size_t product = b2moe_expert_workspace_bytes(gate->type, n, gate->cols, x_dtype);
+    Parts p = carve(workspace, workspace_bytes, gate, A, 0, gate->rows, product, A);
+    if (p.total > workspace_bytes) p = carve(workspace, workspace_bytes, gate, A, 0, gate->rows, product);       // without the rows in slot order the call still works
     if (p.total > workspace_bytes) return B2MOE_ERR_WORKSPACE;
     cudaStream_t s = as_stream(stream);
     if (int32_t rc = plan_from_groups(counts, groups, capacity, gate->experts, A, p.plan, s)) return rc;

@@ -739,13 +739,15 @@ bool gemm_tc_supported(uint32_t type, int k, int experts) { return k >= G_KS && 
 size_t gemm_tc_workspace_bytes(int rows_x, int k) {
     return align_up(size_t(rows_x) * k * 2, 256) + align_up(size_t(rows_x) * sizeof(float), 256);
 }
+// the same for rows in slot order that come from token rows: an index per row in addition
+size_t gemm_tc_slot_bytes(int slot_rows, int k) { return gemm_tc_workspace_bytes(slot_rows, k) + size_t(slot_rows) * sizeof(int); }
 
 // rows_buf: optional scratch for the activation rows in slot order (n * topk + shared_tokens rows of length k, their scales and an index each)
 int32_t gemm_tc_gateup(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_bank * sg, const b2moe_bank * su, const void * x,
                        int x_dtype, const int * plan, int n, int topk, int shared_tokens, long long live, void * act, int act_dtype, void * ws,
                        void * rows_buf, size_t rows_buf_bytes, cudaStream_t s) {
     const int k = gate->cols, slot_rows = n * topk + shared_tokens;
-    const bool slots = rows_buf && rows_buf_bytes >= gemm_tc_workspace_bytes(slot_rows, k) + size_t(slot_rows) * sizeof(int);
+    const bool slots = rows_buf && rows_buf_bytes >= gemm_tc_slot_bytes(slot_rows, k);
     int * slot_of = slots ? reinterpret_cast<int *>(static_cast<uint8_t *>(rows_buf) + gemm_tc_workspace_bytes(slot_rows, k)) : nullptr;
     __half * xb = static_cast<__half *>(slots ? rows_buf : ws);
     float * inv = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(xb) + align_up(size_t(slots ? slot_rows : n) * k * 2, 256));

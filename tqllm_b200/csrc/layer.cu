@@ -33,6 +33,7 @@ unsigned long long g_launch_count = 0;
 bool g_overlap = true;
 bool gemm_tc_supported(uint32_t type, int k, int experts);
 size_t gemm_tc_workspace_bytes(int rows_x, int k);
+size_t gemm_tc_slot_bytes(int slot_rows, int k);
 int32_t gemm_tc_gateup(const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const void *, int, const int *, int,
                        int, int, long long live, void *, int act_dtype, void *, void * rows_buf, size_t rows_buf_bytes, cudaStream_t);
 int32_t gemm_tc_down(const b2moe_bank *, const b2moe_bank *, const void *, int x_dtype, bool per_token, const int *, int, int, int, long long live, void *,
@@ -94,12 +95,12 @@ int32_t product_typed(const b2moe_bank * m, const void * x, int x_dtype, bool pe
     *took = false;
     return B2MOE_OK;
 }
-// the same for gate / up + SwiGLU; rows_buf as in expert_gateup
+// the same for gate / up + SwiGLU; rows_buf as in expert_gateup (the GEMM stores 16-bit results only from rows in slot order)
 int32_t gateup_typed(const b2moe_bank * gate, const b2moe_bank * up, const void * x, int x_dtype, const int * plan, int n, int topk, void * act, int act_dtype,
                      void * ws, void * rows_buf, size_t rows_buf_bytes, cudaStream_t s, bool * took) {
     const int path = expert_path(gate->type, gate->cols, x_dtype, gate->experts, (long long)n * topk);
     *took = true;
-    if (path == B2MOE_FAMILY_GEMM) return gemm_tc_gateup(gate, up, nullptr, nullptr, x, x_dtype, plan, n, topk, 0, (long long)n * topk, act, act_dtype, ws, rows_buf,
+    if (path == B2MOE_FAMILY_GEMM && gemm_tc_slot_bytes(n * topk, gate->cols) <= rows_buf_bytes) return gemm_tc_gateup(gate, up, nullptr, nullptr, x, x_dtype, plan, n, topk, 0, (long long)n * topk, act, act_dtype, ws, rows_buf,
                                                                rows_buf_bytes, s);
     if (path == B2MOE_FAMILY_DECODE && decode_kernel(gate->type, gate->cols, x_dtype) == DEC_4BIT)
         return dec4_gateup(gate, up, nullptr, nullptr, x, x_dtype, plan, n, topk, 0, act, act_dtype, ws, s, false);
