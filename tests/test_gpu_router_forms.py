@@ -57,3 +57,14 @@ def test_split_tiles_give_the_bits_of_whole_ones(dtype, h):
     w, gate, x = inputs(2048, h, 511, dtype)              # 128 tiles: one block each
     full = held(w, gate, x)
     assert torch.equal(moe.router(w, x[:600].contiguous(), gate), full[:600])        # 40 tiles: split
+
+
+@pytest.mark.parametrize("dtype", (torch.float16, torch.float32), ids=("f16", "f32"))
+@pytest.mark.parametrize("n,h", ((65535 * 128 + 3, 32), (65535 * 64 + 3, 16)))
+def test_more_tokens_than_a_grid_has_blocks(dtype, n, h):
+    from tqllm_b200 import moe
+    w, gate, x = inputs(1000, h, 3, dtype)
+    many = x.repeat(-(-n // 1000), 1)[:n]
+    got, want = moe.router(w, many, gate), x.double() @ torch.cat([w, gate[None]]).double().T
+    assert float((got[-1003:-3] - want.roll(-((n - 1003) % 1000), 0)).abs().max()) < 3e-6
+    assert float((got[:1000] - want).abs().max()) < 3e-6

@@ -739,7 +739,9 @@ int32_t router_launch(const float * w, const float * shared, const void * xv, fl
     // with its 64 tokens a block has more than two blocks per SM. router_mma_k / tiles, us: 1024 columns x 32 experts, fp16,
     // 600 tokens 8.9 / 17.7, 2047 (256 blocks) 16.8 / 18.0, 4096 (512 blocks) 32 / 18; 2560 x 60, 600 tokens (160) 22.8 / 31, 2047 (512) 46 / 32;
     // 3072 x 256, 256 tokens (256) 25 / 31, 300 (320) 36 / 31; 256 x 32 4096 tokens (128) 8.3 / 22.
-    if (h % RT_K == 0 && (DT == B2MOE_BF16 ? n >= 2 * RT_TOK : mma_blocks(64) > 2 * ROUTER_SMS)) {
+    // A grid holds 65,535 blocks of tokens; what is more than that many takes the scalar loop, as everything else that does not fit.
+    constexpr int GRID_Y = 65535;
+    if (h % RT_K == 0 && (DT == B2MOE_BF16 ? n >= 2 * RT_TOK : mma_blocks(64) > 2 * ROUTER_SMS) && ceil_div(n, RT_TOK) <= GRID_Y) {
         const dim3 tiles(ceil_div(rows, RT_ROWS), ceil_div(n, RT_TOK), 1);
         const int n_part = ceil_div(h, RT_COLS), share = ceil_div(n_part, 8), ks = ceil_div(n_part, share);      // at most eight blocks, no more than the shares need
         const size_t smem = rt_stages_bytes<DT>() + size_t(share - 1) * RT_PART;
@@ -750,7 +752,7 @@ int32_t router_launch(const float * w, const float * shared, const void * xv, fl
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)) != cudaSuccess) return B2MOE_ERR_CUDA;
         return launch_cluster_z(kernel, dim3(tiles.x, tiles.y, split ? ks : 1), RT_THREADS, bytes, s, w, shared, x, logits, ld, h, e, rows, n);
     }
-    if (h % 16 == 0) {
+    if (h % 16 == 0 && ceil_div(n, 64) <= GRID_Y) {
         auto launch = [&](auto kernel, int tokens) {
             return launch_cluster_z(kernel, dim3(ceil_div(rows, 16), ceil_div(n, tokens), ks), RM_WARPS * 32, 0, s, w, shared, x, logits, ld, h, e, rows, n);
         };
