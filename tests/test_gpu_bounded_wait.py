@@ -1,5 +1,6 @@
-"""GPU: a try of the grouped GEMM's waits lasts as long as its source says, so that a wait that runs out does so in about a second: a
-thousand tries of a barrier that nobody arrives at, at most 4 us each by the hint they carry; twice that is allowed for the loop."""
+"""GPU: a bounded wait of the grouped GEMM that runs out does so soon. How long a try suspends its thread is the hardware's choice, so it is
+measured: a thousand tries of a barrier that nobody arrives at. 2.0 us a try was seen (the limit of tries then is half a second); up to
+8 us, two seconds a wait, is what the launches around it can bear."""
 import ctypes
 import os
 import subprocess
@@ -24,4 +25,4 @@ def test_a_wait_ends_in_time():
     assert lib.run_wait(1000, out.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
     ns, passed = out.tolist()
     assert passed == 0 and ns < 1000 * 8000
-    assert ns / 1000 * lib.wait_limit() < 3e9
+    assert ns / 1000 * lib.wait_limit() < 2.1e9
