@@ -458,7 +458,7 @@ __device__ __forceinline__ void argmax_merge(float & v, int & i, float ov, int o
 // ---- register-resident routing of one token by one warp (experts <= 32 R) ----
 // Lane l keeps experts l, l + 32, ... in registers; a round is a local scan, one warp-wide max of an order-preserving
 // integer image of the key and one warp-wide min over the indices that hold it (ties -> lowest index), so the ten
-// rounds of a top-10 cost about a microsecond instead of a chain of shared-memory scans and shuffle ladders.
+// rounds of a top-10 are ten short chains of register operations instead of shared-memory scans and shuffle ladders.
 __device__ __forceinline__ uint32_t ordered_bits(float v) {          // monotonic float -> uint (taken entries use 0)
     const uint32_t u = __float_as_uint(v);
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
@@ -822,8 +822,8 @@ extern "C" B2MOE_API int32_t b2moe_route_dispatch(int32_t gating, const float * 
     if (!logits || !ids || !weights || !plan) return B2MOE_ERR_NULL;
     const size_t smem = size_t(RD_THREADS / 32) * 2 * experts * sizeof(float);
     // one launch only while every token has a warp of its own: the single block routes its tokens RD_THREADS / 32 at a time,
-    // and a token's ten selection rounds are a dependent chain of about ten microseconds (measured: 64 tokens, 512 experts:
-    // 53 us fused against 12 + 10 us as two launches)
+    // and a token's selection rounds are a dependent chain (measured: 64 tokens, 512 experts: 53 us fused against 12 + 10 us as
+    // two launches)
     if (n <= RD_THREADS / 32 && dispatch_small_path(experts, n * topk) && smem <= 160 * 1024) {
         cudaStream_t s = as_stream(stream);
         if (gating == B2MOE_SOFTMAX) {
