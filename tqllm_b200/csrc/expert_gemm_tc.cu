@@ -462,9 +462,12 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
         }
         if (!ok && lane == 0) give_up();
     } else if (warp == MMA_WARP) {
-        // ---- MMA issuer: the whole warp walks the loop (its values stay in uniform registers), one elected lane issues ----
+        // ---- MMA issuer: the whole warp looks the items up, one elected lane issues an item's products. What an issue costs decides
+        // the pace of narrow items: the tensor core takes N / 2 cycles a product (at least 16), the issuing thread beside busy
+        // decoders 43 with its operands' addresses constant but for one addend (the loop is unrolled over the A stages) and 58 with
+        // addresses of a running stage (microbenchmark, N = 64, cycles a product with its share of the unit's wait and commit) ----
         const uint32_t b_lo0 = sw128_desc_lo(saddr(b_st)), b_step = uint32_t(p.cap * 128) >> 4;
-        uint32_t gu = 0, sb = 0, pb = 0, next = 0, uses0 = 0, uses1 = 0;
+        uint32_t gu = 0, next = 0, uses0 = 0, uses1 = 0;
         bool ok = true;
 #pragma unroll 1
         for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x) {
@@ -474,34 +477,41 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
             next = wide ? 0 : next ^ 1u;
             const uint32_t npad = uint32_t(max(im.nv, 1) + 15) & ~15u, id = idesc(128, npad, 0), d = tmem + h * ACC_COLS;
             const uint32_t second = im.nv <= SPLIT_COLS ? SPLIT_COLS : 0;          // columns from the accumulator of even products to that of odd ones
-            const uint32_t b_half = GATHER ? b_step : uint32_t(b_class(im.nv) + 1) * (b_step >> 2);       // from the first to the second step of a pair
             if (wide || h == 0) { if (uses0 > 0) ok = warp_wait(acc_empty, (uses0 - 1) & 1u) && ok; ++uses0; }
             if (wide || h == 1) { if (uses1 > 0) ok = warp_wait(acc_empty + 8, (uses1 - 1) & 1u) && ok; ++uses1; }
             fence_after();
+            auto products = [&](auto PAIR) {
+                // from the first to the second step of a unit: with b_pair one box holds both; else B stages in turn
+                const uint32_t b_half = PAIR && !GATHER ? uint32_t(b_class(im.nv) + 1) * (b_step >> 2) : b_step;
+                uint32_t left = nunits, first = gu % A_STAGES, turn = gu / A_STAGES, acc = 0;
 #pragma unroll 1
-            for (int u = 0; u < nunits; ++u, ++gu) {
-                const uint32_t sa = gu % A_STAGES, a = tmem + A_COL0 + sa * A_COLS, b_lo = b_lo0 + sb * b_step, freed = done + 16 * sa;
-                const uint32_t acc = u > 0, acc1 = acc | (second == 0), last = u == nunits - 1 ? acc_full + 8 * h : 0;
-                const bool both = 2 * u + 1 < ksteps;                  // the second step of an odd K's last unit is empty: no products, but its barriers turn
-                if (!warp_wait(a_full + 8 * sa, (gu / A_STAGES) & 1u)) { ok = false; break; }
-                if (p.b_pair) {                                        // a_full stands for the unit's rows too
-                    fence_after();
-                    if (both) mma_unit(d, d + second, a, b_lo, id, acc, acc1, freed + 8, last, b_lo + b_half);
-                    else mma_step(d, d + second, a, b_lo, id, acc, acc1, freed + 8, last);
-                    sb = (sb + 2) % MAX_B_STAGES;
-                } else {
-                    if (!warp_wait(b_full + 8 * sb, pb)) { ok = false; break; }
-                    fence_after();
-                    mma_step(d, d + second, a, b_lo, id, acc, acc1, freed, 0);
-                    if (++sb == uint32_t(BS)) { sb = 0; pb ^= 1u; }
-                    if (!warp_wait(b_full + 8 * sb, pb)) { ok = false; break; }
-                    fence_after();
-                    if (both) mma_step(d, d + second, a + A_COLS / 2, b_lo0 + sb * b_step, id, 1, 1, freed + 8, last);
-                    else if (elect_one()) { mma_commit(freed + 8); mma_commit(last); }
-                    __syncwarp();
-                    if (++sb == uint32_t(BS)) { sb = 0; pb ^= 1u; }
+                while (true) {
+#pragma unroll
+                    for (uint32_t s = 0; s < A_STAGES; ++s) {
+                        if (s < first) continue;                       // an item's units begin at any stage
+                        const uint32_t a = tmem + A_COL0 + s * A_COLS, sb = PAIR ? 2 * s : 2 * (s & 1), b = b_lo0 + sb * b_step;
+                        const bool both = left > 1 || !(ksteps & 1);   // the second step of an odd K's last unit is empty: no products, but its barriers turn
+                        if (!bar_wait(a_full + 8 * s, turn & 1u)) return false;
+                        if (!PAIR && !bar_wait(b_full + 8 * sb, (2 * turn + (s >> 1)) & 1u)) return false;      // with b_pair a_full stands for the unit's rows too
+                        fence_after();
+                        mma_step(d, d + second, a, b, id, acc, acc | (second == 0));
+                        if constexpr (!PAIR) {
+                            mma_commit(done + 16 * s);
+                            if (!bar_wait(b_full + 8 * (sb + 1), (2 * turn + (s >> 1)) & 1u)) return false;
+                            fence_after();
+                        }
+                        if (both) mma_step(d, d + second, a + A_COLS / 2, b + b_half, id, 1, 1);
+                        mma_commit(done + 16 * s + 8);
+                        acc = 1;
+                        if (--left == 0) { mma_commit(acc_full + 8 * h); return true; }
+                    }
+                    first = 0;
+                    ++turn;
                 }
-            }
+            };
+            if (elect_one()) ok = ok && (p.b_pair ? products(std::true_type{}) : products(std::false_type{}));
+            ok = __all_sync(0xffffffffu, ok);
+            gu += nunits;
         }
         if (!ok && lane == 0) give_up();
         // nothing may be in flight when the tensor memory is freed (after a clean run the epilogue has waited for all of it)

@@ -81,32 +81,18 @@ __device__ __forceinline__ uint32_t sw128_desc_lo(uint32_t addr) { return ((addr
 __device__ __forceinline__ uint32_t idesc(uint32_t m, uint32_t n, uint32_t ab_format) {
     return (1u << 4) | (ab_format << 7) | (ab_format << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
-// Products with A (128 x 16 per product, fp16) in tensor memory (row in lane, two values of K per column) and B (N x 16 each) in
-// shared memory, fp32 sums in tensor memory: one 64-column step is four of them, even ones into d0 (added to what is there when
-// acc0), odd ones into d1 (acc1); the two may be the same. Then `bar` gets one arrival when every product issued so far has
-// completed, and `bar2` too when it is not 0. Called by a whole converged warp; one elected lane issues. One statement with
-// predicates: as separate calls inside a branch each product cost the warp 48 cycles, the commit 60.
-#define B2_MMA(D, A, B, P) " @pe tcgen05.mma.cta_group::1.kind::f16 [" D "], [" A "], " B ", id, " P ";\n"
-#define B2_MMA_STEP(BLO, A0, A1, A2, A3, P0, P1, P2)                                                                                  \
-    " mov.b64 db, {" BLO ", bh};\n" B2_MMA("%0", A0, "db", P0) " add.u32 t, " BLO ", 2;\n mov.b64 db, {t, bh};\n" B2_MMA("%1", A1, "db", P1)  \
-    " add.u32 t, " BLO ", 4;\n mov.b64 db, {t, bh};\n" B2_MMA("%0", A2, "db", P2) " add.u32 t, " BLO ", 6;\n mov.b64 db, {t, bh};\n" B2_MMA("%1", A3, "db", P2)
-#define B2_MMA_HEAD                                                                                                                  \
-    "{\n .reg .pred pe, p0, p1, pt, pb, pc;\n .reg .b64 db;\n .reg .b32 t, a1, a2, a3, a4, a5, a6, a7, id, bh;\n"                        \
-    " elect.sync _|pe, 0xffffffff;\n setp.ne.b32 p0, %5, 0;\n setp.ne.b32 p1, %6, 0;\n setp.eq.b32 pt, 0, 0;\n setp.ne.and.b32 pb, %8, 0, pe;\n" \
-    " mov.b32 id, %4;\n mov.b32 bh, %9;\n add.u32 a1, %2, 8;\n add.u32 a2, %2, 16;\n add.u32 a3, %2, 24;\n"
-#define B2_MMA_TAIL                                                                                                                  \
-    " @pe tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%7];\n"                                               \
-    " @pb tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%8];\n}"
-__device__ __forceinline__ void mma_step(uint32_t d0, uint32_t d1, uint32_t a, uint32_t b_lo, uint32_t id, uint32_t acc0, uint32_t acc1, uint32_t bar, uint32_t bar2) {
-    asm volatile(B2_MMA_HEAD B2_MMA_STEP("%3", "%2", "a1", "a2", "a3", "p0", "p1", "pt") B2_MMA_TAIL
-                 ::"r"(d0), "r"(d1), "r"(a), "r"(b_lo), "r"(id), "r"(acc0), "r"(acc1), "r"(bar), "r"(bar2), "r"(SW128_DESC_HI) : "memory");
+// One product with A (128 x 16, fp16) in tensor memory (row in lane, two values of K per column) and B (N x 16) in shared memory,
+// fp32 sums in tensor memory, added to what is there when acc != 0. One thread issues.
+__device__ __forceinline__ void mma_f16(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t id, uint32_t acc) {
+    asm volatile("{\n .reg .pred p;\n .reg .b64 db;\n setp.ne.b32 p, %4, 0;\n mov.b64 db, {%2, %5};\n"
+                 " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n}" ::"r"(d), "r"(a), "r"(b_lo), "r"(id), "r"(acc), "r"(SW128_DESC_HI) : "memory");
 }
-// two steps whose A operands follow each other (32 columns each) and whose B operands start at b_lo and b_lo2
-__device__ __forceinline__ void mma_unit(uint32_t d0, uint32_t d1, uint32_t a, uint32_t b_lo, uint32_t id, uint32_t acc0, uint32_t acc1, uint32_t bar, uint32_t bar2,
-                                         uint32_t b_lo2) {
-    asm volatile(B2_MMA_HEAD " add.u32 a4, %2, 32;\n add.u32 a5, %2, 40;\n add.u32 a6, %2, 48;\n add.u32 a7, %2, 56;\n"
-                 B2_MMA_STEP("%3", "%2", "a1", "a2", "a3", "p0", "p1", "pt") B2_MMA_STEP("%10", "a4", "a5", "a6", "a7", "pt", "pt", "pt") B2_MMA_TAIL
-                 ::"r"(d0), "r"(d1), "r"(a), "r"(b_lo), "r"(id), "r"(acc0), "r"(acc1), "r"(bar), "r"(bar2), "r"(SW128_DESC_HI), "r"(b_lo2) : "memory");
+// a 64-column step: four products, even ones into d0 (added when acc0), odd ones into d1 (acc1); the two may be the same
+__device__ __forceinline__ void mma_step(uint32_t d0, uint32_t d1, uint32_t a, uint32_t b_lo, uint32_t id, uint32_t acc0, uint32_t acc1) {
+    mma_f16(d0, a, b_lo, id, acc0);
+    mma_f16(d1, a + 8, b_lo + 2, id, acc1);
+    mma_f16(d0, a + 16, b_lo + 4, id, 1);
+    mma_f16(d1, a + 24, b_lo + 6, id, 1);
 }
 // the barrier gets one arrival when every MMA this thread issued before has completed
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
