@@ -236,12 +236,12 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
     const int e1 = p.experts + 1;
     const int * counts = p.plan + PLAN_HDR, * offsets = counts + e1, * active = offsets + e1 + 1, * perm = active + e1;
     const int row_tiles = (p.rows + 15) >> 4, row_blocks = (row_tiles + ITEM_TILES - 1) / ITEM_TILES;
-    const int ksteps = p.k / G_KS, nunits = (ksteps + 1) >> 1, nchunks = (nunits + 1) >> 1;
+    const int ksteps = p.k / G_KS, nchunks = (ksteps + 3) >> 2;             // a last chunk may lack steps: they bring no products, but their barriers turn
 
     D::init(dec_tab, threadIdx.x, G_THREADS);
     if (threadIdx.x == 0) {
 #pragma unroll 1
-        for (int i = 0; i < RAW_SLOTS; ++i) { bar_init(raw_full + 8 * i, 1); bar_init(raw_empty + 8 * i, DEC_WARPS); }
+        for (int i = 0; i < RAW_SLOTS; ++i) { bar_init(raw_full + 8 * i, 1); bar_init(raw_empty + 8 * i, DEC_WARPS / 2); }
 #pragma unroll 1
         for (int i = 0; i < A_STAGES; ++i) bar_init(a_full + 8 * i, p.b_pair ? 8 + (GATHER ? LOAD_WARPS : 1) : 8);
 #pragma unroll 1
@@ -414,50 +414,54 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
         }
         if (!ok && lane == 0) give_up();
     } else if (warp >= DEC_WARP0) {
-        // ---- A decoder: raw chunks (256 columns of one row tile) -> fp16 operand in tensor memory, unit `part` of every chunk.
-        // (Whole chunks in turn instead: the products then came in bursts of two units of one group, and both sides waited.) ----
-        const int j = warp - DEC_WARP0, q = j & 3, m = (j >> 2) & 1, part = j >> 3, r = 2 * q + m;      // r: row tile of the block
+        // ---- A decoder: raw chunks (256 columns of one row tile) -> fp16 operand in tensor memory. The warps j < 8 and j >= 8 take
+        // the block's chunks in turn, a chunk's two units in the A stages 2 (j >> 3) and the next: what a warp does once per chunk
+        // (waits, scales, addresses) took as many instructions as the conversion itself when it took a unit of every chunk.
+        // Steps past the end of K and units without steps are decoded from zeros and not multiplied ----
+        const int j = warp - DEC_WARP0, q = j & 3, m = (j >> 2) & 1, group = j >> 3, r = 2 * q + m;      // r: row tile of the block
         uint8_t * my_scratch = dec_scratch + j * D::SCRATCH;
         const uint8_t * my_raw = raw + size_t(MODE == 0 ? 4 * m + q : r) * CB;
-        const uint32_t a_lane = tmem + (uint32_t(32 * q + 16 * m) << 16) + A_COL0;
-        uint32_t gu = 0, slot = 0, phase = 0;                          // units before the chunk; ring slot and phase of the chunk
+        const uint32_t a_addr = tmem + (uint32_t(32 * q + 16 * m) << 16) + A_COL0 + 2 * group * A_COLS;
+        const uint32_t full = a_full + 16 * group, freed = done + 8 * (4 * group + 1);      // the stages' second steps: their products free them
+        uint32_t turn = 0, slot = group, phase = 0;                    // chunks of this warp so far; ring slot and phase of the next
+        int pos = group;                                               // the next chunk, in the current item
         bool ok = true;
 #pragma unroll 1
-        for (int it = blockIdx.x; it < n_items && ok && !*abort_flag; it += gridDim.x) {
+        for (int it = blockIdx.x; it < n_items && ok && !*abort_flag; it += gridDim.x, pos -= nchunks) {
             const Item im = locate(it, at);
             const bool live = (MODE == 0 ? im.rb * 4 + q : im.rb * 8 + r) < row_tiles;      // a tile past the last row is not decoded
 #pragma unroll 1
-            for (int left = ksteps; left > 0; left -= 4) {             // steps of the item that are left
+            for (; pos < nchunks; pos += 2, ++turn) {
                 const uint8_t * chunk = my_raw + slot * (8 * CB);
                 if (!warp_wait(raw_full + 8 * slot, phase)) { ok = false; break; }
-                const int steps = left - 2 * part;                     // of this unit (more than two count as two)
-                if (steps > 0) {
-                    const uint32_t g = gu + part, sa = g % A_STAGES, a_addr = a_lane + sa * A_COLS;
+                auto unit = [&](auto U) {
+                    constexpr int u = decltype(U)::value;
                     typename D::Pre pre;
                     uint32_t f[16];
                     if (live) {
-                        pre = D::prep(chunk, lane, part, my_scratch);
+                        pre = D::template prep<u>(chunk, lane, my_scratch);
                         if (D::SCRATCH) __syncwarp();
-                        D::template step<0>(chunk, lane, part, dec_tab, my_scratch, pre, f);
+                        D::template step<u, 0>(chunk, lane, dec_tab, my_scratch, pre, f);
                     }
-                    // the unit that used the stage before: its second step's products
-                    if (g >= A_STAGES && !warp_wait(done + 8 * (2 * sa + 1), ((g / A_STAGES) - 1) & 1u)) { ok = false; break; }
+                    if (turn > 0 && !warp_wait(freed + 16 * u, (turn - 1) & 1u)) return false;
                     if (live) {
                         fence_after();
-                        tmem_st_16x256b_x4(a_addr, f);
-                        if (steps > 1) {
-                            D::template step<1>(chunk, lane, part, dec_tab, my_scratch, pre, f);
-                            tmem_st_16x256b_x4(a_addr + A_COLS / 2, f);
-                        }
+                        tmem_st_16x256b_x4(a_addr + u * A_COLS, f);
+                        D::template step<u, 1>(chunk, lane, dec_tab, my_scratch, pre, f);
+                        tmem_st_16x256b_x4(a_addr + u * A_COLS + A_COLS / 2, f);
                         tmem_st_wait();
                         fence_before();
                     }
                     __syncwarp();
-                    if (lane == 0) bar_arrive(a_full + 8 * sa);
-                }
-                if (lane == 0) bar_arrive(raw_empty + 8 * slot);       // every lane is done with the slot (the syncwarp above, or nothing was read)
-                gu += left > 2 ? 2 : 1;
-                if (++slot == uint32_t(S)) { slot = 0; phase ^= 1u; }
+                    if (lane == 0) {
+                        bar_arrive(full + 8 * u);
+                        if (u == 1) bar_arrive(raw_empty + 8 * slot);  // every lane is done with the slot (the syncwarp above)
+                    }
+                    return true;
+                };
+                if (!unit(std::integral_constant<int, 0>{}) || !unit(std::integral_constant<int, 1>{})) { ok = false; break; }
+                slot += 2;
+                if (slot >= uint32_t(S)) { slot -= S; phase ^= 1u; }
             }
         }
         if (!ok && lane == 0) give_up();
@@ -483,27 +487,28 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
             auto products = [&](auto PAIR) {
                 // from the first to the second step of a unit: with b_pair one box holds both; else B stages in turn
                 const uint32_t b_half = PAIR && !GATHER ? uint32_t(b_class(im.nv) + 1) * (b_step >> 2) : b_step;
-                uint32_t left = nunits, first = gu % A_STAGES, turn = gu / A_STAGES, acc = 0;
+                uint32_t first = gu % A_STAGES, turn = gu / A_STAGES, acc = 0;
+                int left = ksteps, units = 2 * nchunks;
 #pragma unroll 1
                 while (true) {
 #pragma unroll
                     for (uint32_t s = 0; s < A_STAGES; ++s) {
                         if (s < first) continue;                       // an item's units begin at any stage
                         const uint32_t a = tmem + A_COL0 + s * A_COLS, sb = PAIR ? 2 * s : 2 * (s & 1), b = b_lo0 + sb * b_step;
-                        const bool both = left > 1 || !(ksteps & 1);   // the second step of an odd K's last unit is empty: no products, but its barriers turn
                         if (!bar_wait(a_full + 8 * s, turn & 1u)) return false;
                         if (!PAIR && !bar_wait(b_full + 8 * sb, (2 * turn + (s >> 1)) & 1u)) return false;      // with b_pair a_full stands for the unit's rows too
                         fence_after();
-                        mma_step(d, d + second, a, b, id, acc, acc | (second == 0));
+                        if (left > 0) mma_step(d, d + second, a, b, id, acc, acc | (second == 0));
                         if constexpr (!PAIR) {
                             mma_commit(done + 16 * s);
                             if (!bar_wait(b_full + 8 * (sb + 1), (2 * turn + (s >> 1)) & 1u)) return false;
                             fence_after();
                         }
-                        if (both) mma_step(d, d + second, a + A_COLS / 2, b + b_half, id, 1, 1);
+                        if (left > 1) mma_step(d, d + second, a + A_COLS / 2, b + b_half, id, 1, 1);
                         mma_commit(done + 16 * s + 8);
                         acc = 1;
-                        if (--left == 0) { mma_commit(acc_full + 8 * h); return true; }
+                        left -= 2;
+                        if (--units == 0) { mma_commit(acc_full + 8 * h); return true; }
                     }
                     first = 0;
                     ++turn;
@@ -511,7 +516,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
             };
             if (elect_one()) ok = ok && (p.b_pair ? products(std::true_type{}) : products(std::false_type{}));
             ok = __all_sync(0xffffffffu, ok);
-            gu += nunits;
+            gu += 2 * nchunks;
         }
         if (!ok && lane == 0) give_up();
         // nothing may be in flight when the tensor memory is freed (after a clean run the epilogue has waited for all of it)
@@ -565,14 +570,14 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
             const int cls = b_class(im.nv), quads = (im.nv + 3) >> 2, mine = (quads + LOAD_WARPS - 1 - lw) / LOAD_WARPS;
             const uint32_t box_bytes = uint32_t((cls + 1) * (p.cap / 4) * group) * 128u;
 #pragma unroll 1
-            for (int ks = 0; ks < 2 * nunits; ks += group, gk += group) {
+            for (int ks = 0; ks < 4 * nchunks; ks += group, gk += group) {
                 const uint32_t freed = gk + group - 1 - uint32_t(BS);  // the (last) step that used the stage before
                 if (gk >= uint32_t(BS) && !warp_wait(done + 8 * (freed % STEP_RING), (freed / STEP_RING) & 1u)) { ok = false; break; }
                 const uint32_t bar = p.b_pair ? a_full + 4 * sb : b_full + 8 * sb, dst = saddr(b_st) + sb * uint32_t(p.cap * 128);
                 if constexpr (!GATHER) {
                     if (elect_one()) {
                         bar_expect_tx(bar, box_bytes);
-                        tma_load_3d(dst, maps.x + cls, 0, im.slot0, ks, bar);      // the second step of an odd K's last unit lies outside: zeros
+                        tma_load_3d(dst, maps.x + cls, 0, im.slot0, ks, bar);      // steps past K lie outside: zeros
                     }
                     __syncwarp();
                 } else {

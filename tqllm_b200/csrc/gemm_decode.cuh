@@ -1,6 +1,6 @@
 // Weight decoders of the tensor-core grouped GEMM: one 64-column step of one 16-row bank tile -> fp16 A operand in registers.
-// A 256-column chunk has two units of two steps; a warp decodes unit u (0 or 1) of every chunk: prep once per chunk, then
-// step<0>, step<1>.
+// A 256-column chunk has two units of two steps; a warp decodes both units of every other chunk: for u = 0, 1 prep<u>, then
+// step<u, 0>, step<u, 1>.
 //
 // A warp owns a row tile; lane L = 4 g + t holds, in the bank's lane-major layout, the code words of rows g and g + 8
 // (formats.cuh). Every code word (or pair of IQ3_S grid entries) decodes to eight fp16 values, so a step leaves sixteen
@@ -85,7 +85,7 @@ template <> struct Dec<T_Q4_K> {
     // fetched with shuffles and spread with byte permutes, took 45 more instructions a step, 36 of them in the integer pipe.)
     static constexpr int SCRATCH = 16 * 4 * 16;
     struct Pre { uint32_t D[2], magic; };
-    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, int u, uint8_t * scratch) {
+    template <int u> __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t * scratch) {
         const int g = lane >> 2, t = lane & 3;
         const uint4 h0 = *reinterpret_cast<const uint4 *>(chunk + 2048 + 16 * g), h1 = *reinterpret_cast<const uint4 *>(chunk + 2048 + 16 * (g + 8));    // d, dmin | s[12]
         // the unit's four scales and four mins as bytes (src/formats/weight/dequant.cpp:56-64)
@@ -108,7 +108,7 @@ template <> struct Dec<T_Q4_K> {
         to[32] = make_uint4(h2_bits(__high2half2(sc)), h2_bits(__high2half2(ns)), h2_bits(__high2half2(mh)), h2_bits(__high2half2(ml)));
         return Pre{{__byte_perm(h0.x, 0u, 0x1010), __byte_perm(h1.x, 0u, 0x1010)}, in_register(0x64006400u)};
     }
-    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void *, const uint8_t * scratch, const Pre & p, uint32_t (&f)[16]) {
+    template <int u, int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const void *, const uint8_t * scratch, const Pre & p, uint32_t (&f)[16]) {
         const uint4 w4 = plane(chunk, 2 * u + JS, lane);
         const uint4 * c = reinterpret_cast<const uint4 *>(scratch) + 4 * (lane >> 2) + 2 * JS;
 #pragma unroll
@@ -141,7 +141,7 @@ template <> struct Dec<T_IQ3S4> {
     // the constants of (row, sub-block) in the warp's scratch, as for Q4_K: (32 (1 + 2 s), -47 (1 + 2 s))
     static constexpr int SCRATCH = 16 * 4 * 8;
     struct Pre { uint32_t D[2], one; };
-    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, int u, uint8_t * scratch) {
+    template <int u> __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t * scratch) {
         const int g = lane >> 2, t = lane & 3;
         Pre p;
         p.one = in_register(0x3C003C00u);
@@ -156,7 +156,7 @@ template <> struct Dec<T_IQ3S4> {
         }
         return p;
     }
-    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void *, const uint8_t * scratch, const Pre & p, uint32_t (&f)[16]) {
+    template <int u, int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const void *, const uint8_t * scratch, const Pre & p, uint32_t (&f)[16]) {
         const uint4 w4 = plane(chunk, 2 * u + JS, lane);
         const uint4 * c = reinterpret_cast<const uint4 *>(scratch) + 2 * (lane >> 2) + JS;       // both sub-blocks of the step
 #pragma unroll
@@ -208,7 +208,7 @@ template <> struct Dec<T_IQ4_XS> {
     __device__ static void init(void * tab, int tid, int n) { build_lut(tab, tid, n); }
     // once per chunk: lane t holds fp16(d (ls - 32)) of the unit's sub-block t, for its two rows
     struct Pre { uint32_t dl; };
-    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, int u, uint8_t *) {
+    template <int u> __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t *) {
         const int g = lane >> 2, ib = 4 * u + (lane & 3);
         float dl[2];
 #pragma unroll
@@ -220,7 +220,7 @@ template <> struct Dec<T_IQ4_XS> {
         }
         return Pre{pack_h2(dl[0], dl[1])};
     }
-    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void * tab, const uint8_t *, const Pre & p, uint32_t (&f)[16]) {
+    template <int u, int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const void * tab, const uint8_t *, const Pre & p, uint32_t (&f)[16]) {
         const Lut lut = lut_of(tab, lane);
         const uint4 w4 = plane(chunk, 2 * u + JS, lane);
         const int src = (lane & ~3) | (2 * JS);
@@ -235,10 +235,10 @@ template <> struct Dec<T_IQ4_XS> {
 template <> struct Dec<T_IQ4_NL> {
     static constexpr int SCRATCH = 0;
     struct Pre {};
-    __device__ __forceinline__ static Pre prep(const uint8_t *, int, int, uint8_t *) { return Pre{}; }
+    template <int u> __device__ __forceinline__ static Pre prep(const uint8_t *, int, uint8_t *) { return Pre{}; }
     static constexpr int TAB_BYTES = LUT_BYTES;
     __device__ static void init(void * tab, int tid, int n) { build_lut(tab, tid, n); }
-    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void * tab, const uint8_t *, const Pre &, uint32_t (&f)[16]) {
+    template <int u, int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const void * tab, const uint8_t *, const Pre &, uint32_t (&f)[16]) {
         const Lut lut = lut_of(tab, lane);
         const int g = lane >> 2;
 #pragma unroll
@@ -256,7 +256,7 @@ template <> struct Dec<T_IQ4_NL> {
 template <> struct Dec<T_NVFP4G> {
     static constexpr int SCRATCH = 0;
     struct Pre {};
-    __device__ __forceinline__ static Pre prep(const uint8_t *, int, int, uint8_t *) { return Pre{}; }
+    template <int u> __device__ __forceinline__ static Pre prep(const uint8_t *, int, uint8_t *) { return Pre{}; }
     static constexpr int TAB_BYTES = 0;
     __device__ static void init(void *, int, int) {}
     // the eight e2m1 codes of a word -> eight fp16 values (the hardware conversion, two codes per instruction: low nibble
@@ -268,7 +268,7 @@ template <> struct Dec<T_NVFP4G> {
         return make_uint4(h2_bits(__hmul2(bits_h2(v0), scale)), h2_bits(__hmul2(bits_h2(v1), scale)), h2_bits(__hmul2(bits_h2(v2), scale)),
                           h2_bits(__hmul2(bits_h2(v3), scale)));
     }
-    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void *, const uint8_t *, const Pre &, uint32_t (&f)[16]) {
+    template <int u, int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const void *, const uint8_t *, const Pre &, uint32_t (&f)[16]) {
         const int g = lane >> 2, t = lane & 3;
         const uint8_t * tile = chunk + u * Fmt<T_NVFP4G>::TILE;
         constexpr int P = JS;                                            // the unit is one 128-column tile; plane = sub-blocks 2 P, 2 P + 1 of the 128-column tile
@@ -289,7 +289,7 @@ template <> struct Dec<T_NVFP4G> {
 template <> struct Dec<T_IQ3_S> {
     static constexpr int SCRATCH = 0;
     struct Pre {};
-    __device__ __forceinline__ static Pre prep(const uint8_t *, int, int, uint8_t *) { return Pre{}; }
+    template <int u> __device__ __forceinline__ static Pre prep(const uint8_t *, int, uint8_t *) { return Pre{}; }
     // table: grid entry -> its four odd magnitudes as fp16 (8 bytes)
     static constexpr int TAB_BYTES = 512 * 8;
     __device__ static void init(void * tab, int tid, int n) {
@@ -299,9 +299,8 @@ template <> struct Dec<T_IQ3_S> {
             t2[i] = make_uint2(pack_h2(float(m & 255u), float((m >> 8) & 255u)), pack_h2(float((m >> 16) & 255u), float(m >> 24)));
         }
     }
-    template <int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, int u, const void * tab, const uint8_t *, const Pre &, uint32_t (&f)[16]) {
-        if (u == 0) bits_step<JS>(chunk, lane, tab, f);                // the bit positions have to be constants
-        else bits_step<2 + JS>(chunk, lane, tab, f);
+    template <int u, int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const void * tab, const uint8_t *, const Pre &, uint32_t (&f)[16]) {
+        bits_step<2 * u + JS>(chunk, lane, tab, f);
     }
     template <int J> __device__ __forceinline__ static void bits_step(const uint8_t * chunk, int lane, const void * tab, uint32_t (&f)[16]) {
         const int g = lane >> 2;
