@@ -18,16 +18,16 @@
 //      (1680 cycles per step at 80 tokens). Gathering token rows by TMA (tile::gather4) costs the issuing warp 60 to 200
 //      cycles per four rows and stays for calls whose scratch holds no rows in slot order;
 //   two accumulators of 128 columns alternate between items of up to 128 tokens, so the epilogue of one item (SwiGLU, stores)
-//   overlaps the products of the next; a wider item takes both. Products into one accumulator follow each other by at least 80
-//   cycles however few tokens they have, products into two alternating ones by 44 (measured), so an item of up to 64 tokens
-//   splits its K over the two halves of its accumulator and the epilogue adds them.
+//   overlaps the products of the next; a wider item takes both. An item of up to 64 tokens splits its K over the two halves of
+//   its accumulator and the epilogue adds them: half as long a chain of truncated sums (NVFP4 gate/up, relative error against
+//   64 bits 3.7e-7 and 8.3e-7 in one chain); the products' pace is the same either way.
 // The control warps share their schedulers with six others, so what they execute per unit bounds the block: they walk uniform
 // loops, one elected lane issues, and the raw blocks and rows come in the largest boxes that fit. They are the first warps of the
 // block: as the last ones they were served last (c3 decode gate/up 110 us, as the first 78).
 // Warps: 0 issues tcgen05.mma; 1 streams the raw blocks (256 columns of the item's eight row tiles per ring slot: one TMA box
 // of the down bank, one each of gate and up, running ahead across items); 2 (when it gathers 2..7) loads B; then from 4 (8) on
 // eight epilogue warps (two per TMEM lane quarter, 16-token groups in turn) and sixteen that decode A (the j-th: lane quarter j & 3, row tile
-// (j >> 2) & 1 of it, unit j >> 3 of every 256-column chunk). One barrier per step says that its products are done (a commit costs the issuing thread
+// (j >> 2) & 1 of it, every other 256-column chunk). One barrier per step says that its products are done (a commit costs the issuing thread
 // 60 cycles): it frees the unit's A stage and the step's B stage. Every wait is bounded; a wait that runs out sets the plan's
 // status word, and the block drains and leaves.
 //
@@ -218,7 +218,9 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
     constexpr int LOAD_WARPS = load_warps(GATHER), EPI_WARP0 = LOAD_WARP0 + LOAD_WARPS, DEC_WARP0 = EPI_WARP0 + EPI_WARPS, G_THREADS = g_threads(GATHER);
     static_assert(EPI_WARP0 % 4 == 0 && DEC_WARP0 % 4 == 0, "warp w reaches the tensor-memory lanes of quarter w % 4");
     extern __shared__ uint8_t smem_raw[];
-    uint8_t * smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    // aligned by an offset and not by a cast of the rounded address: that one loses the pointer's address space, and every read of
+    // the block's shared memory became a generic load with 64-bit addresses
+    uint8_t * smem = smem_raw + (-saddr(smem_raw) & 1023u);
     uint8_t * b_st = smem;                                            // [b_stages][cap][128 bytes], swizzled
     uint8_t * raw = b_st + size_t(p.b_stages) * p.cap * 128;          // [raw_slots][8 row tiles][CB]
     uint8_t * dec_tab = raw + size_t(8) * p.raw_slots * CB;           // the decoder's lookup table
@@ -294,10 +296,16 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
             if (m != 0xffffffffu) break;
         }
         const Info f = info[at];
-        const int nt = tiles_of(f.cnt), per = ((f.cnt + nt - 1) / nt + 15) & ~15, local = it - f.cum, tile = local % nt;
+        const int nt = tiles_of(f.cnt), local = it - f.cum;
         Item r;
         r.e = f.e;
-        r.rb = local / nt;
+        int per = (f.cnt + 15) & ~15, tile = 0;
+        r.rb = local;
+        if (nt > 1) {                                                  // (three divisions: as many instructions as a warp's conversion of half a chunk, in every warp)
+            per = ((f.cnt + nt - 1) / nt + 15) & ~15;
+            r.rb = local / nt;
+            tile = local - r.rb * nt;
+        }
         r.slot0 = f.off + tile * per;
         r.nv = max(0, min(per, f.cnt - tile * per));
         return r;
@@ -428,30 +436,23 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
         bool ok = true;
 #pragma unroll 1
         for (int it = blockIdx.x; it < n_items && ok && !*abort_flag; it += gridDim.x, pos -= nchunks) {
-            const Item im = locate(it, at);
-            const bool live = (MODE == 0 ? im.rb * 4 + q : im.rb * 8 + r) < row_tiles;      // a tile past the last row is not decoded
 #pragma unroll 1
             for (; pos < nchunks; pos += 2, ++turn) {
                 const uint8_t * chunk = my_raw + slot * (8 * CB);
                 if (!warp_wait(raw_full + 8 * slot, phase)) { ok = false; break; }
                 auto unit = [&](auto U) {
                     constexpr int u = decltype(U)::value;
-                    typename D::Pre pre;
                     uint32_t f[16];
-                    if (live) {
-                        pre = D::template prep<u>(chunk, lane, my_scratch);
-                        if (D::SCRATCH) __syncwarp();
-                        D::template step<u, 0>(chunk, lane, dec_tab, my_scratch, pre, f);
-                    }
+                    const typename D::Pre pre = D::template prep<u>(chunk, lane, my_scratch);
+                    if (D::SCRATCH) __syncwarp();
+                    D::template step<u, 0>(chunk, lane, dec_tab, my_scratch, pre, f);
                     if (turn > 0 && !warp_wait(freed + 16 * u, (turn - 1) & 1u)) return false;
-                    if (live) {
-                        fence_after();
-                        tmem_st_16x256b_x4(a_addr + u * A_COLS, f);
-                        D::template step<u, 1>(chunk, lane, dec_tab, my_scratch, pre, f);
-                        tmem_st_16x256b_x4(a_addr + u * A_COLS + A_COLS / 2, f);
-                        tmem_st_wait();
-                        fence_before();
-                    }
+                    fence_after();
+                    tmem_st_16x256b_x4(a_addr + u * A_COLS, f);
+                    D::template step<u, 1>(chunk, lane, dec_tab, my_scratch, pre, f);
+                    tmem_st_16x256b_x4(a_addr + u * A_COLS + A_COLS / 2, f);
+                    tmem_st_wait();
+                    fence_before();
                     __syncwarp();
                     if (lane == 0) {
                         bar_arrive(full + 8 * u);

@@ -79,11 +79,12 @@ template <> struct Dec<T_Q4_K> {
     __device__ __forceinline__ static uint32_t two(uint32_t n1024, __half2 S, __half2 NS, __half2 MH, __half2 ML, __half2 D) {
         return h2_bits(__hadd2(__hfma2(__hfma2(bits_h2(n1024), S, NS), D, MH), ML));
     }
-    // Once per chunk: lane t of a row's four lanes turns the headers of its two rows into the constants of the unit's sub-block t
-    // and leaves them in the warp's scratch, each twice in a word as the arithmetic takes it: [row][sub-block](S, -1024 S, MH, ML).
+    // Once per unit: lane t of a row's four lanes turns the headers of its two rows into the constants of the unit's sub-block t
+    // and leaves them in the warp's scratch, two in a word (the arithmetic takes either half of a register twice at no
+    // cost; spread there, they took twice the registers and loads): [row][sub-block]((S, -1024 S), (MH, ML)).
     // The scales and mins are exact as fp16, MH = fp16(-dmin m), ML = the exact rest. (Constants of two rows in one register,
     // fetched with shuffles and spread with byte permutes, took 45 more instructions a step, 36 of them in the integer pipe.)
-    static constexpr int SCRATCH = 16 * 4 * 16;
+    static constexpr int SCRATCH = 16 * 4 * 8;
     struct Pre { uint32_t D[2], magic; };
     template <int u> __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t * scratch) {
         const int g = lane >> 2, t = lane & 3;
@@ -103,20 +104,20 @@ template <> struct Dec<T_Q4_K> {
         const __half2 mn = pick(mn0, mn1), dm = bits_h2(__byte_perm(h0.x, h1.x, 0x7632) ^ 0x80008000u);       // -dmin of the two rows
         if (t & 1) sc = __hmul2(sc, __float2half2_rn(0.0625f));
         const __half2 ns = __hmul2(sc, __float2half2_rn(-1024.f)), mh = __hmul2(dm, mn), ml = __hfma2(dm, mn, __hneg2(mh));
-        uint4 * to = reinterpret_cast<uint4 *>(scratch) + 4 * g + t;
-        to[0] = make_uint4(h2_bits(__low2half2(sc)), h2_bits(__low2half2(ns)), h2_bits(__low2half2(mh)), h2_bits(__low2half2(ml)));
-        to[32] = make_uint4(h2_bits(__high2half2(sc)), h2_bits(__high2half2(ns)), h2_bits(__high2half2(mh)), h2_bits(__high2half2(ml)));
+        uint2 * to = reinterpret_cast<uint2 *>(scratch) + 4 * g + t;
+        to[0] = make_uint2(h2_bits(__lows2half2(sc, ns)), h2_bits(__lows2half2(mh, ml)));
+        to[32] = make_uint2(h2_bits(__highs2half2(sc, ns)), h2_bits(__highs2half2(mh, ml)));
         return Pre{{__byte_perm(h0.x, 0u, 0x1010), __byte_perm(h1.x, 0u, 0x1010)}, in_register(0x64006400u)};
     }
     template <int u, int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const void *, const uint8_t * scratch, const Pre & p, uint32_t (&f)[16]) {
         const uint4 w4 = plane(chunk, 2 * u + JS, lane);
-        const uint4 * c = reinterpret_cast<const uint4 *>(scratch) + 4 * (lane >> 2) + 2 * JS;
+        const uint4 * c = reinterpret_cast<const uint4 *>(scratch) + 2 * (lane >> 2) + JS;
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-            const uint4 c0 = c[32 * r], c1 = c[32 * r + 1];
+            const uint4 cc = c[16 * r];
             const __half2 D = bits_h2(p.D[r]);
-            auto lo = [&](uint32_t w) { return two(and_or(w, 0x000F000Fu, p.magic), bits_h2(c0.x), bits_h2(c0.y), bits_h2(c0.z), bits_h2(c0.w), D); };
-            auto hi = [&](uint32_t w) { return two(and_or(w, 0x00F000F0u, p.magic), bits_h2(c1.x), bits_h2(c1.y), bits_h2(c1.z), bits_h2(c1.w), D); };
+            auto lo = [&](uint32_t w) { return two(and_or(w, 0x000F000Fu, p.magic), __low2half2(bits_h2(cc.x)), __high2half2(bits_h2(cc.x)), __low2half2(bits_h2(cc.y)), __high2half2(bits_h2(cc.y)), D); };
+            auto hi = [&](uint32_t w) { return two(and_or(w, 0x00F000F0u, p.magic), __low2half2(bits_h2(cc.z)), __high2half2(bits_h2(cc.z)), __low2half2(bits_h2(cc.w)), __high2half2(bits_h2(cc.w)), D); };
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
                 const uint32_t v = r ? (b ? w4.w : w4.z) : (b ? w4.y : w4.x), v8 = v >> 8;
