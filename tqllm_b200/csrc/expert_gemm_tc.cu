@@ -60,7 +60,7 @@ constexpr int load_warps(bool gather) { return gather ? 6 : 2; }
 constexpr int g_threads(bool gather) { return (LOAD_WARP0 + load_warps(gather) + EPI_WARPS + DEC_WARPS) * 32; }
 static_assert(EPI_WARPS * 32 == MAX_CAP, "an epilogue thread looks one token up");
 static_assert(MAX_B_STAGES <= STEP_RING, "a B stage is freed by the barrier of the step that used it");
-constexpr int N_BARS = 2 * RAW_SLOTS + A_STAGES + STEP_RING + MAX_B_STAGES + 6;
+constexpr int N_BARS = 3 * RAW_SLOTS + A_STAGES + STEP_RING + MAX_B_STAGES + 6;
 
 struct GemmArgs {
     const float * aux0, * aux1, * saux0, * saux1;      // row scales of the banks (gate, up) or (down, -) and of the shared expert's (may be null)
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
     uint32_t * tmem_slot = reinterpret_cast<uint32_t *>(bars + N_BARS);
     volatile int * abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     const int S = p.raw_slots, BS = p.b_stages;
-    const uint32_t raw_full = saddr(bars), raw_empty = raw_full + 8 * RAW_SLOTS, a_full = raw_empty + 8 * RAW_SLOTS,
+    const uint32_t raw_full = saddr(bars), raw_empty = raw_full + 16 * RAW_SLOTS, a_full = raw_empty + 8 * RAW_SLOTS,
                    done = a_full + 8 * A_STAGES, b_full = done + 8 * STEP_RING, acc_full = b_full + 8 * MAX_B_STAGES, acc_empty = acc_full + 16,
                    drain = acc_empty + 16, tok_bar = drain + 8;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
     D::init(dec_tab, threadIdx.x, G_THREADS);
     if (threadIdx.x == 0) {
 #pragma unroll 1
-        for (int i = 0; i < RAW_SLOTS; ++i) { bar_init(raw_full + 8 * i, 1); bar_init(raw_empty + 8 * i, DEC_WARPS / 2); }
+        for (int i = 0; i < RAW_SLOTS; ++i) { bar_init(raw_full + 8 * i, 1); bar_init(raw_full + 8 * (RAW_SLOTS + i), 1); bar_init(raw_empty + 8 * i, DEC_WARPS / 2); }
 #pragma unroll 1
         for (int i = 0; i < A_STAGES; ++i) bar_init(a_full + 8 * i, p.b_pair ? 8 + (GATHER ? LOAD_WARPS : 1) : 8);
 #pragma unroll 1
@@ -431,15 +431,18 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
         const uint8_t * my_raw = raw + size_t(MODE == 0 ? 4 * m + q : r) * CB;
         const uint32_t a_addr = tmem + (uint32_t(32 * q + 16 * m) << 16) + A_COL0 + 2 * group * A_COLS;
         const uint32_t full = a_full + 16 * group, freed = done + 8 * (4 * group + 1);      // the stages' second steps: their products free them
-        uint32_t turn = 0, slot = group, phase = 0;                    // chunks of this warp so far; ring slot and phase of the next
+        // Chunk c lies in slot c % S and is announced by barrier c % 2 S: a ring of S barriers with an odd S would bring a group to every other
+        // phase of each, and a phase that two chunks back has completed looks like the one that the group waits for
+        uint32_t turn = 0, next = group, phase = 0;                    // chunks of this warp so far; the next one's barrier and its phase
         int pos = group;                                               // the next chunk, in the current item
         bool ok = true;
 #pragma unroll 1
         for (int it = blockIdx.x; it < n_items && ok && !*abort_flag; it += gridDim.x, pos -= nchunks) {
 #pragma unroll 1
             for (; pos < nchunks; pos += 2, ++turn) {
+                const uint32_t slot = next >= uint32_t(S) ? next - S : next;
                 const uint8_t * chunk = my_raw + slot * (8 * CB);
-                if (!warp_wait(raw_full + 8 * slot, phase)) { ok = false; break; }
+                if (!warp_wait(raw_full + 8 * next, phase)) { ok = false; break; }
                 auto unit = [&](auto U) {
                     constexpr int u = decltype(U)::value;
                     uint32_t f[16];
@@ -461,8 +464,8 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                     return true;
                 };
                 if (!unit(std::integral_constant<int, 0>{}) || !unit(std::integral_constant<int, 1>{})) { ok = false; break; }
-                slot += 2;
-                if (slot >= uint32_t(S)) { slot -= S; phase ^= 1u; }
+                next += 2;
+                if (next >= 2 * uint32_t(S)) { next -= 2 * S; phase ^= 1u; }
             }
         }
         if (!ok && lane == 0) give_up();
@@ -538,7 +541,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
             for (int c = 0; c < nchunks; ++c) {
                 if (issued >= uint32_t(S) && !warp_wait(raw_empty + 8 * slot, phase)) { ok = false; break; }
                 if (elect_one()) {
-                    const uint32_t bar = raw_full + 8 * slot, dst = saddr(raw) + slot * BYTES;
+                    const uint32_t bar = raw_full + 8 * (issued % (2 * uint32_t(S))), dst = saddr(raw) + slot * BYTES;
                     bar_expect_tx(bar, BYTES);
                     tma_load_3d(dst, map, 0, c * PARTS, rt, bar);
                     if (MODE == 0) tma_load_3d(dst + BYTES / 2, map + 1, 0, c * PARTS, rt, bar);
@@ -551,7 +554,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
         if (!ok && lane == 0) give_up();
         // before leaving, every copy must have landed (after a clean run these waits return at once)
 #pragma unroll 1
-        for (uint32_t i = issued > uint32_t(S) ? issued - S : 0; i < issued; ++i) bar_wait(raw_full + 8 * (i % S), (i / S) & 1u);
+        for (uint32_t i = issued > uint32_t(S) ? issued - S : 0; i < issued; ++i) bar_wait(raw_full + 8 * (i % (2 * uint32_t(S))), (i / (2 * uint32_t(S))) & 1u);
     } else {
         // ---- B loader: warp 2 brings a step's (or a unit's) rows with one box; a gathering launch: lane l of loader w brings rows
         // 4 (6 l + w) .. + 3. Issuing sets the pace of a gather (90 to 120 cycles per four rows and warp), so it takes
