@@ -353,7 +353,8 @@ B2MOE_API int32_t b2moe_place_experts(const uint64_t * counts, int32_t experts, 
  * For tests and benchmarks, not for engines: process-wide switches, not thread-safe, to be set while no call of this
  * library is running. They have no counterpart in the reference.
  * b2moe_harness_select: family = the kernel family every later expert product takes where it supports the shape
- * (AUTO = the library's own choice by tokens per expert, the default); gemm_item_tokens = 256: work items of 256 tokens
+ * (AUTO = the library's own choice by tokens per expert, the default; DECODE for banks of 4-bit codes: the decode kernels or,
+ * from nine assignments per expert on, the exact grouped product that takes their place there); gemm_item_tokens = 256: work items of 256 tokens
  * in the grouped GEMM; any other value (0 = the default): the library's own choice of 64, 128 or 256 by tokens per expert.
  * b2moe_harness_wait_probe: the 4-bit decode kernels skip the copy of weight tile number drop_tile of every warp
  * (-1 = none, the default) and bound each wait by wait_limit polls (0 = default), so that a test can watch a bounded

@@ -17,7 +17,7 @@ namespace b2 {
 int32_t check_bank(const b2moe_bank * b);
 size_t gemm_tc_slot_bytes(int slot_rows, int k);
 int32_t product_typed(const b2moe_bank * m, const void * x, int x_dtype, bool per_token, const int * plan, int n, int topk, void * y, int y_dtype,
-                      void * ws, cudaStream_t s, bool * took);
+                      void * ws, void * rows_buf, size_t rows_buf_bytes, cudaStream_t s, bool * took);
 int32_t gateup_typed(const b2moe_bank * gate, const b2moe_bank * up, const void * x, int x_dtype, const int * plan, int n, int topk, void * act, int act_dtype,
                      void * ws, void * rows_buf, size_t rows_buf_bytes, cudaStream_t s, bool * took);
 
@@ -119,7 +119,10 @@ struct Carve {
     void * take(size_t bytes) { const size_t o = at; at = align_up(at + bytes, 256); return base ? base + o : nullptr; }
     bool fits() const { return at <= cap; }
 };
-struct Parts { int32_t * plan; void * dws; size_t dws_bytes; float * x32, * y32; size_t y32_bytes; void * ews; size_t ews_bytes; size_t total; };
+struct Parts {
+    int32_t * plan; void * dws; size_t dws_bytes; float * x32, * y32; size_t y32_bytes; void * ews; size_t ews_bytes; size_t total; const char * base;
+    size_t from(const void * part) const { return total - size_t(static_cast<const char *>(part) - base); }      // bytes from a part to the end: a product that takes typed rows uses no part but the plan
+};
 // rows_x: rows of the product's fp32 input copy (0: the product reads the caller's x directly); out_cols: row length of the fp32 output
 // slot_rows: the output rows' place must also hold that many of the GEMM's activation rows in slot order (gate/up)
 Parts carve(void * ws, size_t bytes, const b2moe_bank * b, int A, int rows_x, int out_cols, size_t ews_bytes, int slot_rows = 0) {
@@ -135,6 +138,7 @@ Parts carve(void * ws, size_t bytes, const b2moe_bank * b, int A, int rows_x, in
     p.ews_bytes = ews_bytes;
     p.ews = c.take(ews_bytes);
     p.total = c.at;
+    p.base = c.base;
     return p;
 }
 int32_t plan_from_groups(const int32_t * counts, const int32_t * groups, int capacity, int experts, int A, int32_t * plan, cudaStream_t s) {
@@ -150,7 +154,7 @@ int32_t single_product(const b2moe_bank * m, const void * x, int x_dtype, void *
                        int per_expert_input, cudaStream_t s) {
     const int A = n * topk;
     bool took;
-    if (int32_t rc = product_typed(m, x, x_dtype, !per_expert_input, p.plan, n, topk, y, y_dtype, p.ews, s, &took)) return rc;
+    if (int32_t rc = product_typed(m, x, x_dtype, !per_expert_input, p.plan, n, topk, y, y_dtype, p.ews, p.x32, p.from(p.x32), s, &took)) return rc;
     if (took) return B2MOE_OK;
     launch_overlapped(rows_expand_k, dim3(A), dim3(128), 0, s, x, x_dtype, A, m->cols, topk, per_expert_input, p.x32);
     if (int32_t rc = launch_status()) return rc;
@@ -230,7 +234,7 @@ extern "C" B2MOE_API int32_t b2moe_expert_gemm_gateup(const b2moe_bank * gate, c
     if (int32_t rc = plan_from_groups(counts, groups, capacity, gate->experts, A, p.plan, s)) return rc;
     bool took = false;
     if (gate->type == up->type && gate->rows == up->rows && gate->cols == up->cols && gate->experts == up->experts)      // else the call below rejects them
-        if (int32_t rc = gateup_typed(gate, up, x, x_dtype, p.plan, n, topk, act, act_dtype, p.ews, p.y32, p.y32_bytes, s, &took)) return rc;
+        if (int32_t rc = gateup_typed(gate, up, x, x_dtype, p.plan, n, topk, act, act_dtype, p.ews, p.y32, p.from(p.y32), s, &took)) return rc;
     if (took) return B2MOE_OK;
     if (int32_t rc = b2moe_expert_gateup_swiglu(gate, up, nullptr, nullptr, x, x_dtype, p.plan, n, topk, 0, p.y32, p.ews, p.ews_bytes, stream)) return rc;
     launch_overlapped(rows_convert_k, dim3(A), dim3(128), 0, s, p.y32, p.plan, gate->experts, gate->rows, act, act_dtype);

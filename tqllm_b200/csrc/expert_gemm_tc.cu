@@ -30,8 +30,13 @@
 // (j >> 2) & 1 of it, every other 256-column chunk). One barrier per step says that its products are done (a commit costs the issuing thread
 // 60 cycles): it frees the unit's A stage and the step's B stage. Every wait is bounded; a wait that runs out sets the plan's
 // status word, and the block drains and leaves.
+// The exact form (TERMS > 0; Q4_K and IQ3_S codes, where the decode kernels' precision is asked for and their eight tokens a pass are too few): A
+// holds the integers sc q or (1 + 2 s)(2 n - 15), B the activations in one or two fp16 terms, every 256-column chunk has accumulators of
+// its own (two sets in turn), and the epilogue warps scale a chunk's sums by the rows' d in fp32 while the next one is multiplied. The mins of Q4_K
+// meet the sub-block sums of the activations in one more product a chunk. Items have up to 32 tokens. Decoding costs two instructions
+// less a pair of weights than with the scales in the operand, reading the sums back about 150 a scheduler and chunk.
 //
-// Numerics: weights are rounded to fp16 after the exact fp32 decode (relative error <= 2^-11 per weight; bf16 operands
+// Numerics of the other form: weights are rounded to fp16 after the exact fp32 decode (relative error <= 2^-11 per weight; bf16 operands
 // gave 3e-2 of the output RMS as the largest error, fp16 stays below the layer tolerance). An activation row is
 // multiplied by 2^e so that its largest magnitude lies in [2^14, 2^15) and rounded to fp16: exact for bf16 inputs down
 // to 2^-29 of the row maximum; the epilogue multiplies the sums (fp32) by 2^-e.
@@ -60,7 +65,11 @@ constexpr int load_warps(bool gather) { return gather ? 6 : 2; }
 constexpr int g_threads(bool gather) { return (LOAD_WARP0 + load_warps(gather) + EPI_WARPS + DEC_WARPS) * 32; }
 static_assert(EPI_WARPS * 32 == MAX_CAP, "an epilogue thread looks one token up");
 static_assert(MAX_B_STAGES <= STEP_RING, "a B stage is freed by the barrier of the step that used it");
-constexpr int N_BARS = 3 * RAW_SLOTS + A_STAGES + STEP_RING + MAX_B_STAGES + 6;
+// The exact form (TERMS > 0): items of up to X_CAP tokens; two sets of sums, a chunk's each: X_CAP columns per term of the activations, then X_CAP
+// of the mins; after both the mins' A operand of either chunk. X_RING: chunks whose row constants the epilogue may still need
+constexpr int X_CAP = 32, X_SET = 3 * X_CAP, X_MINS = 2 * X_CAP, X_AMINS = 2 * X_SET, X_RING = 4;
+static_assert(X_AMINS + 2 * 8 <= A_COL0, "two sets of sums and two operands of mins below the A stages");
+constexpr int N_BARS = 3 * RAW_SLOTS + A_STAGES + STEP_RING + MAX_B_STAGES + X_RING + 6;
 
 struct GemmArgs {
     const float * aux0, * aux1, * saux0, * saux1;      // row scales of the banks (gate, up) or (down, -) and of the shared expert's (may be null)
@@ -84,9 +93,11 @@ template <uint32_t T> constexpr int part_words() { return chunk_bytes<T>() / chu
 // the active experts of the launch: items before it, expert, tokens, first assignment slot
 struct Info { int cum, e, cnt, off; };
 
+// what the exact form keeps beside the operands: the mins' B tiles (32 bytes a row) and the rows' constants
+constexpr size_t exact_smem(int terms) { return terms ? size_t(A_STAGES) * X_CAP * 32 + size_t(X_RING) * 128 * sizeof(float2) : 0; }
 template <uint32_t T>
-constexpr size_t gemm_smem(int experts, int cap, int b_stages, int raw_slots) {
-    return 1024 + size_t(b_stages) * cap * 128 + size_t(8) * raw_slots * chunk_bytes<T>() + gdec::Dec<T>::TAB_BYTES +
+constexpr size_t gemm_smem(int experts, int cap, int b_stages, int raw_slots, int terms = 0) {
+    return 1024 + size_t(b_stages) * cap * 128 * (terms ? terms : 1) + exact_smem(terms) + size_t(8) * raw_slots * chunk_bytes<T>() + gdec::Dec<T>::TAB_BYTES +
            DEC_WARPS * gdec::Dec<T>::SCRATCH + size_t(experts + 2) * sizeof(Info) + 2 * MAX_CAP * sizeof(int2) + size_t(N_BARS) * 8 + 16;
 }
 
@@ -120,11 +131,11 @@ template <uint32_t T, int DT> __device__ __forceinline__ void load_positions(con
         v[q] = RUN == 8 ? w[half + ((e & 1) << 1) + (e >> 1)] : RUN == 4 ? w[q] : w[half + 2 * (e & 1) + (e >> 1)];
     }
 }
-// One activation row of any dtype -> fp16 scaled by a power of two (largest magnitude in [2^14, 2^15)), by one warp; put(step
-// column, 16 bytes) stores a lane's eight positions, the inverse scale is returned. Two passes over the row: its largest
+// One activation row of any dtype scaled by a power of two (largest magnitude in [2^14, 2^15)), by one warp; put(step
+// column, values) gets a lane's eight positions, the inverse scale is returned. Two passes over the row: its largest
 // magnitude, then (from the cache) the values.
 template <uint32_t T, int DT, typename Put>
-__device__ __forceinline__ float row_to_f16(const typename Elem<DT>::type * xr, int k, int lane, Put put) {
+__device__ __forceinline__ float row_scaled(const typename Elem<DT>::type * xr, int k, int lane, Put put) {
     using E = typename Elem<DT>::type;
     constexpr int V = 16 / int(sizeof(E));                              // elements per 16-byte load
     float mx = 0.f;
@@ -143,10 +154,18 @@ __device__ __forceinline__ float row_to_f16(const typename Elem<DT>::type * xr, 
     for (int gb = 64 * (lane >> 3); gb < k; gb += 256) {
         float v[8];
         load_positions<T, DT>(xr + gb, lane & 7, v);
-        put(gb + 8 * (lane & 7), make_uint4(gdec::pack_h2(v[0] * scale, v[1] * scale), gdec::pack_h2(v[2] * scale, v[3] * scale),
-                                            gdec::pack_h2(v[4] * scale, v[5] * scale), gdec::pack_h2(v[6] * scale, v[7] * scale)));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] *= scale;
+        put(gb + 8 * (lane & 7), v);
     }
     return __uint_as_float(uint32_t(127 - 14 + ex) << 23);
+}
+__device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
+    return make_uint4(gdec::pack_h2(v[0], v[1]), gdec::pack_h2(v[2], v[3]), gdec::pack_h2(v[4], v[5]), gdec::pack_h2(v[6], v[7]));
+}
+template <uint32_t T, int DT, typename Put>
+__device__ __forceinline__ float row_to_f16(const typename Elem<DT>::type * xr, int k, int lane, Put put) {
+    return row_scaled<T, DT>(xr, k, lane, [&](int c, const float (&v)[8]) { put(c, pack8(v)); });
 }
 // rows in their own order: the gathered form
 template <uint32_t T, int DT>
@@ -205,14 +224,69 @@ __global__ void tokens_to_slots_k(const typename Elem<DT>::type * x, const int *
     });
     if (mine >= 0) inv_scale[mine] = inv;
 }
+// Rows of the exact form: [TERMS][rows][k] fp16, a value as one term (16-bit activations: exact) or as two (fp32: 22 bits), and for the mins of
+// Q4_K the sums of the row's 32-column sub-blocks, divided by 32, as [rows][k / 256][16]: eight leading fp16 terms, then the eight rests.
+// A lane holds eight columns of one sub-block, lanes l, l ^ 1, l ^ 4, l ^ 5 all of it.
+template <uint32_t T, int DT, int TERMS, typename Slots>
+__device__ __forceinline__ float exact_row(const typename Elem<DT>::type * xr, int k, int lane, __half * out, size_t plane, __half * mins, Slots each) {
+    return row_scaled<T, DT>(xr, k, lane, [&](int c, const float (&v)[8]) {
+        const uint4 hi = pack8(v);
+        uint4 lo;
+        if (TERMS == 2) {
+            float r[8];
+            const __half * h = reinterpret_cast<const __half *>(&hi);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) r[i] = v[i] - __half2float(h[i]);
+            lo = pack8(r);
+        }
+        __half s0, s1;
+        if (gdec::Exact<T>::MINS) {
+            float s = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s = (s + __shfl_xor_sync(0xffffffffu, s, 4)) * 0.03125f;
+            s0 = __float2half_rn(s);
+            s1 = __float2half_rn(s - __half2float(s0));
+        }
+        each([&](size_t slot) {
+            *reinterpret_cast<uint4 *>(out + slot * k + c) = hi;
+            if (TERMS == 2) *reinterpret_cast<uint4 *>(out + plane + slot * k + c) = lo;
+            if (gdec::Exact<T>::MINS && (lane & 5) == 0) {
+                __half * m = mins + slot * (k / 16) + 16 * (c >> 8) + 2 * (lane >> 3) + ((lane >> 1) & 1);
+                m[0] = s0;
+                m[8] = s1;
+            }
+        });
+    });
+}
+template <uint32_t T, int DT, int TERMS>
+__global__ void exact_rows_k(const typename Elem<DT>::type * x, const int * plan, int experts, int A, int topk, int k, __half * out, size_t plane,
+                             __half * mins, float * inv_scale) {
+    const int lane = threadIdx.x & 31, slot = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    grid_release();
+    grid_wait();
+    int row = slot;                                                    // no plan: A rows in their own order, the gathered form
+    if (plan) {
+        if (slot >= plan[PLAN_NGROUPED]) return;
+        const int e1 = experts + 1, a = plan[PLAN_HDR + e1 + e1 + 1 + e1 + slot];
+        row = topk == 0 ? a : a < A ? a / topk : a - A;
+    } else if (slot >= A) {
+        return;
+    }
+    const float inv = exact_row<T, DT, TERMS>(x + size_t(row) * k, k, lane, out, plane, mins, [&](auto store) { store(size_t(slot)); });
+    if (lane == 0) inv_scale[slot] = inv;
+}
 
 // MODE 0: act[a][r] = silu(gate_r . x_tok(a)) * (up_r . x_tok(a));  MODE 1: y[a][r] = down_r . act[a]
+// TERMS > 0: the exact form: no rounding but that of the activations to TERMS fp16 terms and of the fp32 sums
 // F32_OUT: an instance for fp32 results and one for 16-bit ones, chosen by the call's output type. A branch at the stores, or two
 // loops in one kernel, cost every fp32 caller: c3 down (80 tokens x K = 512) 262 us against 184, c5 gate/up 1305 against 1240.
 // GATHER: the activation rows lie in token order.
-template <uint32_t T, int MODE, bool F32_OUT, bool GATHER>
+template <uint32_t T, int MODE, bool F32_OUT, bool GATHER, int TERMS = 0>
 __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs p, const __grid_constant__ GemmMaps maps) {
     using D = gdec::Dec<T>;
+    constexpr bool EXACT = TERMS > 0;
+    using X = gdec::Exact<EXACT ? T : uint32_t(T_Q4_K)>;
+    constexpr int PLANES = EXACT ? TERMS : 1;                          // rows of B per token
     constexpr int CB = chunk_bytes<T>();
     constexpr int ITEM_TILES = MODE == 0 ? 4 : 8;                      // row tiles of one matrix that an item covers
     constexpr int LOAD_WARPS = load_warps(GATHER), EPI_WARP0 = LOAD_WARP0 + LOAD_WARPS, DEC_WARP0 = EPI_WARP0 + EPI_WARPS, G_THREADS = g_threads(GATHER);
@@ -222,7 +296,9 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
     // the block's shared memory became a generic load with 64-bit addresses
     uint8_t * smem = smem_raw + (-saddr(smem_raw) & 1023u);
     uint8_t * b_st = smem;                                            // [b_stages][cap][128 bytes], swizzled
-    uint8_t * raw = b_st + size_t(p.b_stages) * p.cap * 128;          // [raw_slots][8 row tiles][CB]
+    uint8_t * mins_st = b_st + size_t(p.b_stages) * p.cap * 128 * PLANES;       // exact: [A stages][X_CAP][32 bytes], swizzled; then the row constants, [X_RING][128]
+    float2 * consts = reinterpret_cast<float2 *>(mins_st + A_STAGES * X_CAP * 32);
+    uint8_t * raw = mins_st + exact_smem(TERMS);                      // [raw_slots][8 row tiles][CB]
     uint8_t * dec_tab = raw + size_t(8) * p.raw_slots * CB;           // the decoder's lookup table
     uint8_t * dec_scratch = dec_tab + D::TAB_BYTES;                   // [decode warps][SCRATCH]
     Info * info = reinterpret_cast<Info *>(dec_scratch + DEC_WARPS * D::SCRATCH);   // [na + 1]
@@ -233,7 +309,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
     const int S = p.raw_slots, BS = p.b_stages;
     const uint32_t raw_full = saddr(bars), raw_empty = raw_full + 16 * RAW_SLOTS, a_full = raw_empty + 8 * RAW_SLOTS,
                    done = a_full + 8 * A_STAGES, b_full = done + 8 * STEP_RING, acc_full = b_full + 8 * MAX_B_STAGES, acc_empty = acc_full + 16,
-                   drain = acc_empty + 16, tok_bar = drain + 8;
+                   drain = acc_empty + 16, tok_bar = drain + 8, const_full = tok_bar + 8;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int e1 = p.experts + 1;
     const int * counts = p.plan + PLAN_HDR, * offsets = counts + e1, * active = offsets + e1 + 1, * perm = active + e1;
@@ -253,6 +329,8 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
         for (int i = 0; i < 2; ++i) { bar_init(acc_full + 8 * i, 1); bar_init(acc_empty + 8 * i, EPI_WARPS); }
         bar_init(drain, 1);
         bar_init(tok_bar, EPI_WARPS);
+#pragma unroll 1
+        for (int i = 0; i < X_RING; ++i) bar_init(const_full + 8 * i, 8);
         *abort_flag = 0;
         bar_init_fence();
     }
@@ -312,7 +390,8 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
     };
     auto x_row = [&](int a) { return MODE == 0 ? (a < p.A ? a / p.topk : a - p.A) : a; };
     // the rows' boxes come in four sizes: the smallest that holds the item's tokens
-    auto b_class = [&](int nv) { return max(nv - 1, 0) >> (p.cap_log2 - 2); };
+    auto b_class = [&](int nv) { return max(nv - 1, 0) >> (EXACT ? 4 : p.cap_log2 - 2); };
+    const int class_rows = EXACT ? 16 : p.cap / 4;
     auto give_up = [&]() { *abort_flag = 1; atomicExch(p.plan + PLAN_STATUS, 2); };
     int at = 0;
 
@@ -358,9 +437,11 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                 const float * ax = MODE == 0 && upper ? (shared ? p.saux1 : p.aux1) : (shared ? p.saux0 : p.aux0);
                 rs = ax[size_t(shared ? 0 : im.e) * row_tiles * 16 + row];
             }
-            if (!warp_wait(acc_full + 8 * h, (h ? uses1 : uses0) & 1u)) { ok = false; break; }
-            if (h) ++uses1; else ++uses0;
-            fence_after();
+            if constexpr (!EXACT) {
+                if (!warp_wait(acc_full + 8 * h, (h ? uses1 : uses0) & 1u)) { ok = false; break; }
+                if (h) ++uses1; else ++uses0;
+                fence_after();
+            }
             const uint32_t taddr = tmem + (uint32_t(32 * q) << 16) + h * ACC_COLS;
             const int4 * t = reinterpret_cast<const int4 *>(tok + (ic & 1u) * MAX_CAP);
             char * const out = reinterpret_cast<char *>(static_cast<typename std::conditional<F32_OUT, float, uint16_t>::type *>(p.out) + row);
@@ -370,6 +451,62 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                 if constexpr (F32_OUT) *reinterpret_cast<float *>(out + uint64_t(uint32_t(a)) * row_bytes) = y;
                 else store_act(out + uint64_t(uint32_t(a)) * row_bytes, p.out_dtype, 0, y);
             };
+            if constexpr (EXACT) {
+                // the sums of every chunk are scaled by the row's d (and the mins' sums by its dmin) and added in fp32, 8-token groups in turn
+                const int g0 = 8 * ((warp - EPI_WARP0) >> 2), lo = 16 * (b_class(im.nv) + 1);       // the second term's columns
+                float sum[2][8];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) sum[i >> 3][i & 7] = 0.f;
+#pragma unroll 1
+                for (int c = 0; c < nchunks; ++c, ++uses0) {
+                    const uint32_t set = uses0 & 1u, at_set = tmem + (uint32_t(32 * q) << 16) + set * X_SET;
+                    if (!warp_wait(const_full + 8 * (uses0 % X_RING), (uses0 / X_RING) & 1u)) { ok = false; break; }
+                    const float2 k = consts[(uses0 % X_RING) * 128 + 32 * q + lane];
+                    if (!warp_wait(acc_full + 8 * set, (uses0 >> 1) & 1u)) { ok = false; break; }
+                    fence_after();
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        if (g0 + 16 * i >= im.nv) break;
+                        uint32_t v[8], w[8], z[8];
+                        tmem_ld8(at_set + g0 + 16 * i, v);
+                        if constexpr (TERMS == 2) tmem_ld8(at_set + lo + g0 + 16 * i, w);
+                        if constexpr (X::MINS) tmem_ld8(at_set + X_MINS + g0 + 16 * i, z);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            float m = __uint_as_float(v[j]);
+                            if constexpr (TERMS == 2) m += __uint_as_float(w[j]);
+                            sum[i][j] = fmaf(k.x, m, sum[i][j]);
+                            if constexpr (X::MINS) sum[i][j] = fmaf(k.y, __uint_as_float(z[j]), sum[i][j]);
+                        }
+                    }
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) bar_arrive(acc_empty + 8 * set);
+                }
+                if (!ok) break;
+#pragma unroll
+                for (int g = 0; g < 2; ++g) {
+                    const int c = g0 + 16 * g;
+                    if (c >= im.nv) break;
+                    int4 two[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) two[i] = t[c / 2 + i];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float v0 = sum[g][2 * i], v1 = sum[g][2 * i + 1];
+                        if (MODE == 0) {
+                            const float other = __shfl_xor_sync(0xffffffffu, upper ? v0 : v1, 16);
+                            const float is = __int_as_float(upper ? two[i].w : two[i].y);
+                            const float gv = (upper ? other : v0) * is, uv = (upper ? v1 : other) * is;
+                            store(upper ? two[i].z : two[i].x, gv / (1.f + expf(-gv)) * uv);
+                        } else {
+                            store(two[i].x, v0 * __int_as_float(two[i].y));
+                            store(two[i].z, v1 * __int_as_float(two[i].w));
+                        }
+                    }
+                }
+            } else {
 #pragma unroll 1
             for (int c = first; c < im.nv; c += 32) {
                 uint32_t v[16];
@@ -418,6 +555,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                 bar_arrive(acc_empty + 8 * h);
                 if (wide) bar_arrive(acc_empty + 8);
             }
+            }
             ok = put(ic + 1);                                          // the other table: every warp has left the item that used it
         }
         if (!ok && lane == 0) give_up();
@@ -446,19 +584,32 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                 auto unit = [&](auto U) {
                     constexpr int u = decltype(U)::value;
                     uint32_t f[16];
-                    const typename D::Pre pre = D::template prep<u>(chunk, lane, my_scratch);
-                    if (D::SCRATCH) __syncwarp();
-                    D::template step<u, 0>(chunk, lane, dec_tab, my_scratch, pre, f);
+                    using P = typename std::conditional<EXACT, X, D>::type;
+                    const typename P::Pre pre = P::template prep<u>(chunk, lane, my_scratch);
+                    if (P::SCRATCH) __syncwarp();
+                    if constexpr (EXACT) X::template step<u, 0>(chunk, lane, my_scratch, pre, f);
+                    else D::template step<u, 0>(chunk, lane, dec_tab, my_scratch, pre, f);
                     if (turn > 0 && !warp_wait(freed + 16 * u, (turn - 1) & 1u)) return false;
                     fence_after();
                     tmem_st_16x256b_x4(a_addr + u * A_COLS, f);
-                    D::template step<u, 1>(chunk, lane, dec_tab, my_scratch, pre, f);
+                    if constexpr (EXACT && u == 0) {
+                        // the chunk's mins and row constants: what used their places belongs to chunks whose sums are read (the wait above)
+                        if constexpr (X::MINS) {
+                            uint32_t mn[4];
+                            X::mins(chunk, lane, mn);
+                            tmem_st_16x256b_x1(tmem + (uint32_t(32 * q + 16 * m) << 16) + X_AMINS + 8 * group, mn);
+                        }
+                        if (lane < 16) consts[(group + 2 * (turn & 1u)) * 128 + 32 * q + 16 * m + lane] = X::consts(chunk, lane);
+                    }
+                    if constexpr (EXACT) X::template step<u, 1>(chunk, lane, my_scratch, pre, f);
+                    else D::template step<u, 1>(chunk, lane, dec_tab, my_scratch, pre, f);
                     tmem_st_16x256b_x4(a_addr + u * A_COLS + A_COLS / 2, f);
                     tmem_st_wait();
                     fence_before();
                     __syncwarp();
                     if (lane == 0) {
                         bar_arrive(full + 8 * u);
+                        if (EXACT && u == 0) bar_arrive(const_full + 8 * (group + 2 * (turn & 1u)));
                         if (u == 1) bar_arrive(raw_empty + 8 * slot);  // every lane is done with the slot (the syncwarp above)
                     }
                     return true;
@@ -474,7 +625,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
         // the pace of narrow items: the tensor core takes N / 2 cycles a product (at least 16), the issuing thread beside busy
         // decoders 43 with its operands' addresses constant but for one addend (the loop is unrolled over the A stages) and 58 with
         // addresses of a running stage (microbenchmark, N = 64, cycles a product with its share of the unit's wait and commit) ----
-        const uint32_t b_lo0 = sw128_desc_lo(saddr(b_st)), b_step = uint32_t(p.cap * 128) >> 4;
+        const uint32_t b_lo0 = sw128_desc_lo(saddr(b_st)), b_step = uint32_t(p.cap * 128 * PLANES) >> 4;
         uint32_t gu = 0, next = 0, uses0 = 0, uses1 = 0;
         bool ok = true;
 #pragma unroll 1
@@ -483,14 +634,16 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
             const bool wide = im.nv > ACC_COLS;
             const uint32_t h = wide ? 0 : next;
             next = wide ? 0 : next ^ 1u;
-            const uint32_t npad = uint32_t(max(im.nv, 1) + 15) & ~15u, id = idesc(128, npad, 0), d = tmem + h * ACC_COLS;
-            const uint32_t second = im.nv <= SPLIT_COLS ? SPLIT_COLS : 0;          // columns from the accumulator of even products to that of odd ones
+            const uint32_t npad = uint32_t(max(im.nv, 1) + 15) & ~15u, id = idesc(128, npad * PLANES, 0), d = tmem + h * ACC_COLS;
+            const uint32_t second = !EXACT && im.nv <= SPLIT_COLS ? SPLIT_COLS : 0;          // columns from the accumulator of even products to that of odd ones
+            if constexpr (!EXACT) {
             if (wide || h == 0) { if (uses0 > 0) ok = warp_wait(acc_empty, (uses0 - 1) & 1u) && ok; ++uses0; }
             if (wide || h == 1) { if (uses1 > 0) ok = warp_wait(acc_empty + 8, (uses1 - 1) & 1u) && ok; ++uses1; }
             fence_after();
+            }
             auto products = [&](auto PAIR) {
                 // from the first to the second step of a unit: with b_pair one box holds both; else B stages in turn
-                const uint32_t b_half = PAIR && !GATHER ? uint32_t(b_class(im.nv) + 1) * (b_step >> 2) : b_step;
+                const uint32_t b_half = PAIR && !GATHER ? uint32_t(b_class(im.nv) + 1) * (uint32_t(class_rows * 128 * PLANES) >> 4) : b_step;
                 uint32_t first = gu % A_STAGES, turn = gu / A_STAGES, acc = 0;
                 int left = ksteps, units = 2 * nchunks;
 #pragma unroll 1
@@ -501,6 +654,20 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                         const uint32_t a = tmem + A_COL0 + s * A_COLS, sb = PAIR ? 2 * s : 2 * (s & 1), b = b_lo0 + sb * b_step;
                         if (!bar_wait(a_full + 8 * s, turn & 1u)) return false;
                         if (!PAIR && !bar_wait(b_full + 8 * sb, (2 * turn + (s >> 1)) & 1u)) return false;      // with b_pair a_full stands for the unit's rows too
+                        if constexpr (EXACT) {                         // a chunk's units are the stages 0, 1 or 2, 3, its sums a set of their own
+                            const uint32_t set = s >> 1, ds = tmem + set * X_SET;
+                            if ((s & 1) == 0 && turn > 0 && !bar_wait(acc_empty + 8 * set, (turn - 1) & 1u)) return false;
+                            fence_after();
+                            mma_step(ds, ds, a, b, id, s & 1, 1);
+                            mma_step(ds, ds, a + A_COLS / 2, b + b_half, id, 1, 1);
+                            if constexpr (X::MINS)
+                                if ((s & 1) == 0)
+                                    mma_f16<SW32_DESC_HI>(ds + X_MINS, tmem + X_AMINS + 8 * set, sw128_desc_lo(saddr(mins_st) + s * (X_CAP * 32)), idesc(128, npad, 0), 0);
+                            mma_commit(done + 16 * s + 8);
+                            if (s & 1) mma_commit(acc_full + 8 * set);
+                            if (--units == 0) return true;
+                            continue;
+                        }
                         fence_after();
                         if (left > 0) mma_step(d, d + second, a, b, id, acc, acc | (second == 0));
                         if constexpr (!PAIR) {
@@ -518,7 +685,10 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                     ++turn;
                 }
             };
-            if (elect_one()) ok = ok && (p.b_pair ? products(std::true_type{}) : products(std::false_type{}));
+            if (elect_one()) {
+                if constexpr (EXACT) ok = ok && products(std::true_type{});
+                else ok = ok && (p.b_pair ? products(std::true_type{}) : products(std::false_type{}));
+            }
             ok = __all_sync(0xffffffffu, ok);
             gu += 2 * nchunks;
         }
@@ -572,13 +742,21 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                 for (int i = 0; i < 4; ++i) row[i] = n0 < im.nv ? x_row(perm[im.slot0 + min(n0 + i, im.nv - 1)]) : 0;      // past the last token: repeat it (dead columns of D)
             }
             const int cls = b_class(im.nv), quads = (im.nv + 3) >> 2, mine = (quads + LOAD_WARPS - 1 - lw) / LOAD_WARPS;
-            const uint32_t box_bytes = uint32_t((cls + 1) * (p.cap / 4) * group) * 128u;
+            const uint32_t box_bytes = uint32_t((cls + 1) * class_rows * group * PLANES) * 128u;
 #pragma unroll 1
             for (int ks = 0; ks < 4 * nchunks; ks += group, gk += group) {
                 const uint32_t freed = gk + group - 1 - uint32_t(BS);  // the (last) step that used the stage before
                 if (gk >= uint32_t(BS) && !warp_wait(done + 8 * (freed % STEP_RING), (freed / STEP_RING) & 1u)) { ok = false; break; }
-                const uint32_t bar = p.b_pair ? a_full + 4 * sb : b_full + 8 * sb, dst = saddr(b_st) + sb * uint32_t(p.cap * 128);
-                if constexpr (!GATHER) {
+                const uint32_t bar = p.b_pair ? a_full + 4 * sb : b_full + 8 * sb, dst = saddr(b_st) + sb * uint32_t(p.cap * 128 * PLANES);
+                if constexpr (EXACT && !GATHER) {
+                    if (elect_one()) {
+                        const bool mins = X::MINS && (ks & 2) == 0;    // a chunk's first unit brings the tokens' sub-block sums too
+                        bar_expect_tx(bar, box_bytes + (mins ? uint32_t((cls + 1) * 16 * 32) : 0u));
+                        tma_load_4d(dst, maps.x + cls, 0, im.slot0, 0, ks, bar);
+                        if (mins) tma_load_3d(saddr(mins_st) + (sb >> 1) * (X_CAP * 32), maps.x + 2 + cls, 0, im.slot0, ks >> 2, bar);
+                    }
+                    __syncwarp();
+                } else if constexpr (!GATHER) {
                     if (elect_one()) {
                         bar_expect_tx(bar, box_bytes);
                         tma_load_3d(dst, maps.x + cls, 0, im.slot0, ks, bar);      // steps past K lie outside: zeros
@@ -586,8 +764,10 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                     __syncwarp();
                 } else {
                     const int real = min(group, ksteps - ks);
-                    if (lane == 0) bar_expect_tx(bar, uint32_t(max(real, 0) * mine) * 512u);
+                    const bool mins = EXACT && X::MINS && (ks & 2) == 0;
+                    if (lane == 0) bar_expect_tx(bar, uint32_t(max(real, 0) * mine) * 512u + (mins ? uint32_t(mine) * 128u : 0u));
                     __syncwarp();
+                    if (mins && n0 < im.nv) tma_gather4(saddr(mins_st) + (sb >> 1) * (X_CAP * 32) + n0 * 32, maps.x + 2, ks * 4, row[0], row[1], row[2], row[3], bar);
                     if (n0 < im.nv)
 #pragma unroll 1
                         for (int i = 0; i < real; ++i)
@@ -643,7 +823,7 @@ decltype(&cuTensorMapEncodeTiled) map_encoder() {
 }
 bool encode_map(CUtensorMap & m, CUtensorMapDataType type, int rank, const void * base, const cuuint64_t * dims, const cuuint64_t * strides,
                 const cuuint32_t * box, CUtensorMapSwizzle swizzle) {
-    const cuuint32_t steps[3] = {1, 1, 1};
+    const cuuint32_t steps[4] = {1, 1, 1, 1};
     const auto encode = map_encoder();
     return encode && encode(&m, type, rank, const_cast<void *>(base), dims, strides, box, steps, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
@@ -659,6 +839,23 @@ bool gather_map(CUtensorMap & m, const void * xb, int rows, int k) {
     const cuuint64_t dims[2] = {cuuint64_t(k), cuuint64_t(rows)}, strides[1] = {cuuint64_t(k) * 2};
     const cuuint32_t box[2] = {G_KS, 1};
     return encode_map(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, xb, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+// the exact form's sub-block sums for tile::gather4: rows of k / 16 values, sixteen a chunk
+bool gather_mins_map(CUtensorMap & m, const void * mins, int rows, int k) {
+    const cuuint64_t dims[2] = {cuuint64_t(k / 16), cuuint64_t(rows)}, strides[1] = {cuuint64_t(k) / 8};
+    const cuuint32_t box[2] = {16, 1};
+    return encode_map(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, mins, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_32B);
+}
+// the exact form's rows as [k / 64][TERMS][rows][64], boxes of two steps, and its sub-block sums as [k / 256][rows][16]
+bool exact_rows_map(CUtensorMap & m, const void * xb, int rows, int k, int box_rows, int terms) {
+    const cuuint64_t dims[4] = {G_KS, cuuint64_t(rows), cuuint64_t(terms), cuuint64_t(k / G_KS)}, strides[3] = {cuuint64_t(k) * 2, cuuint64_t(rows) * k * 2, G_KS * 2};
+    const cuuint32_t box[4] = {G_KS, cuuint32_t(box_rows), cuuint32_t(terms), 2};
+    return encode_map(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, xb, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+bool mins_map(CUtensorMap & m, const void * mins, int rows, int k, int box_rows) {
+    const cuuint64_t dims[3] = {16, cuuint64_t(rows), cuuint64_t(k / 256)}, strides[2] = {cuuint64_t(k) / 8, 32};
+    const cuuint32_t box[3] = {16, cuuint32_t(box_rows), 1};
+    return encode_map(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, mins, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_32B);
 }
 // a bank's tiles as [experts * row tiles][parts of a chunk][8-byte words]: a box is one 256-column chunk of `tiles` consecutive row tiles
 template <uint32_t T> bool bank_map(CUtensorMap & m, const b2moe_bank * b, int tiles) {
@@ -724,6 +921,63 @@ int32_t gemm_launch_t(GemmArgs a, long long live, const b2moe_bank * const * m, 
     launch_overlapped(kernel, dim3(sms), dim3(g_threads(!slots)), smem, s, a, maps);
     return launch_status();
 }
+// The exact form: x (a row per token when topk > 0, per assignment otherwise) -> rows in slot order in `rows` (or, gathered: in their own order), then the product
+template <uint32_t T> bool exact_fit(int experts, int terms, GemmArgs & a) {
+    a.cap = X_CAP; a.cap_log2 = 5; a.b_stages = 2 * A_STAGES; a.b_pair = 1;
+    static_assert(X_CAP == 1 << 5);
+    for (a.raw_slots = RAW_SLOTS; a.raw_slots >= 3; --a.raw_slots)
+        if (gemm_smem<T>(experts, X_CAP, a.b_stages, a.raw_slots, terms) <= GEMM_SMEM_LIMIT) return true;
+    return false;
+}
+size_t exact_rows_bytes(int slot_rows, int k, int terms) { return align_up(size_t(slot_rows) * (size_t(k) * 2 * terms + k / 8), 256); }
+template <uint32_t T, int MODE, int DT>
+int32_t exact_launch_t(GemmArgs a, const b2moe_bank * const * m, const void * x, int topk, int slot_rows, bool slots, void * rows, cudaStream_t s) {
+    constexpr int TERMS = DT == B2MOE_F32 ? 2 : 1;
+    const int sms = gemm_sm_count();
+    if (sms <= 0) return B2MOE_ERR_CUDA;
+    if (!exact_fit<T>(a.experts, TERMS, a)) return B2MOE_ERR_SHAPE;
+    __half * xb = static_cast<__half *>(rows), * mins = xb + size_t(slot_rows) * a.k * TERMS;
+    float * inv = reinterpret_cast<float *>(static_cast<uint8_t *>(rows) + exact_rows_bytes(slot_rows, a.k, TERMS));
+    launch_overlapped(exact_rows_k<T, DT, TERMS>, dim3(ceil_div(slot_rows, 8)), dim3(256), 0, s, static_cast<const typename Elem<DT>::type *>(x), static_cast<const int *>(slots ? a.plan : nullptr), a.experts, slots ? a.A : slot_rows, topk,
+                      a.k, xb, size_t(slot_rows) * a.k, mins, inv);
+    if (int32_t rc = launch_status()) return rc;
+    a.inv_scale = inv;
+    GemmMaps maps;
+    bool mapped = true;
+    if (!slots) {
+        mapped = gather_map(maps.x[0], xb, slot_rows, a.k);
+        if (gdec::Exact<T>::MINS) mapped = mapped && gather_mins_map(maps.x[2], mins, slot_rows, a.k);
+    } else for (int i = 0; i < 2; ++i) {
+        mapped = mapped && exact_rows_map(maps.x[i], xb, slot_rows, a.k, 16 * (i + 1), TERMS);
+        if (gdec::Exact<T>::MINS) mapped = mapped && mins_map(maps.x[2 + i], mins, slot_rows, a.k, 16 * (i + 1));
+    }
+    for (int i = 0; i < 4; ++i)
+        if (m[i]) mapped = mapped && bank_map<T>(maps.w[i], m[i], MODE == 0 ? 4 : 8);
+    if (!mapped) return B2MOE_ERR_CUDA;
+    const size_t smem = gemm_smem<T>(a.experts, a.cap, a.b_stages, a.raw_slots, TERMS);
+    auto kernel = a.out_dtype == B2MOE_F32 ? gemm_tc_k<T, MODE, true, false, TERMS> : gemm_tc_k<T, MODE, false, false, TERMS>;
+    if (!slots) {
+        if constexpr (MODE == 0 && TERMS == 1) {
+            if (a.out_dtype != B2MOE_F32) return B2MOE_ERR_SHAPE;
+            kernel = gemm_tc_k<T, MODE, true, true, TERMS>;
+        } else {
+            return B2MOE_ERR_SHAPE;
+        }
+    }
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return B2MOE_ERR_CUDA;
+    launch_overlapped(kernel, dim3(sms), dim3(g_threads(!slots)), smem, s, a, maps);
+    return launch_status();
+}
+template <int MODE>
+int32_t exact_launch(uint32_t type, const GemmArgs & a, const b2moe_bank * const * m, const void * x, int dtype, int topk, int slot_rows, bool slots, void * rows, cudaStream_t s) {
+    if (type == T_Q4_K) return dtype == B2MOE_F32 ? exact_launch_t<T_Q4_K, MODE, B2MOE_F32>(a, m, x, topk, slot_rows, slots, rows, s)
+                             : dtype == B2MOE_F16 ? exact_launch_t<T_Q4_K, MODE, B2MOE_F16>(a, m, x, topk, slot_rows, slots, rows, s)
+                                                  : exact_launch_t<T_Q4_K, MODE, B2MOE_BF16>(a, m, x, topk, slot_rows, slots, rows, s);
+    if (type == T_IQ3S4) return dtype == B2MOE_F32 ? exact_launch_t<T_IQ3S4, MODE, B2MOE_F32>(a, m, x, topk, slot_rows, slots, rows, s)
+                              : dtype == B2MOE_F16 ? exact_launch_t<T_IQ3S4, MODE, B2MOE_F16>(a, m, x, topk, slot_rows, slots, rows, s)
+                                                   : exact_launch_t<T_IQ3S4, MODE, B2MOE_BF16>(a, m, x, topk, slot_rows, slots, rows, s);
+    return B2MOE_ERR_FORMAT;
+}
 template <int MODE, typename... Args>
 int32_t gemm_launch(uint32_t type, const Args &... args) {
     switch (type) {
@@ -760,6 +1014,30 @@ size_t gemm_tc_workspace_bytes(int rows_x, int k) {
 }
 // the same for rows in slot order that come from token rows: an index per row in addition
 size_t gemm_tc_slot_bytes(int slot_rows, int k) { return gemm_tc_workspace_bytes(slot_rows, k) + size_t(slot_rows) * sizeof(int); }
+
+// The exact form takes Q4_K banks and IQ3_S codes; its scratch: the rows in slot order (two terms a value for fp32 rows), their
+// sub-block sums and scales. slots = false: gate/up on 16-bit rows with fp32 results from a scratch for the n rows of the tokens
+bool gemm_exact_supported(uint32_t type, int k, int experts) {
+    GemmArgs a{};
+    return k > 0 && k % 256 == 0 && (type == T_Q4_K ? exact_fit<T_Q4_K>(experts, 2, a) : type == T_IQ3S4 && exact_fit<T_IQ3S4>(experts, 2, a));
+}
+size_t gemm_exact_bytes(int slot_rows, int k, int dtype) { return exact_rows_bytes(slot_rows, k, dtype == B2MOE_F32 ? 2 : 1) + size_t(slot_rows) * sizeof(float); }
+int32_t gemm_exact_gateup(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_bank * sg, const b2moe_bank * su, const void * x, int x_dtype,
+                          const int * plan, int n, int topk, int shared_tokens, void * act, int act_dtype, void * rows, bool slots, cudaStream_t s) {
+    GemmArgs a{};
+    const b2moe_bank * banks[4] = {gate, up, shared_tokens ? sg : nullptr, shared_tokens ? su : nullptr};
+    a.plan = const_cast<int *>(plan); a.out = act; a.out_dtype = act_dtype;
+    a.rows = gate->rows; a.k = gate->cols; a.experts = gate->experts; a.topk = topk; a.A = n * topk;
+    return exact_launch<0>(gate->type, a, banks, x, x_dtype, topk, slots ? n * topk + shared_tokens : n, slots, rows, s);
+}
+int32_t gemm_exact_down(const b2moe_bank * down, const b2moe_bank * sd, const void * x, int x_dtype, bool per_token, const int * plan, int n, int topk,
+                        int shared_tokens, void * y, int y_dtype, void * rows, cudaStream_t s) {
+    GemmArgs a{};
+    const b2moe_bank * banks[4] = {down, nullptr, shared_tokens ? sd : nullptr, nullptr};
+    a.plan = const_cast<int *>(plan); a.out = y; a.out_dtype = y_dtype;
+    a.rows = down->rows; a.k = down->cols; a.experts = down->experts; a.topk = topk; a.A = n * topk;
+    return exact_launch<1>(down->type, a, banks, x, x_dtype, per_token ? topk : 0, n * topk + shared_tokens, true, rows, s);
+}
 
 // rows_buf: optional scratch for the activation rows in slot order (n * topk + shared_tokens rows of length k, their scales and an index each)
 int32_t gemm_tc_gateup(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_bank * sg, const b2moe_bank * su, const void * x,

@@ -175,6 +175,103 @@ template <> struct Dec<T_IQ3S4> {
 };
 
 // ---------------------------------------------------------------------------------------------------------------
+// The same tiles without a rounding, for the GEMM that scales its sums itself once per 256 columns: the operand is the integer
+// sc q (Q4_K, at most 945) or (1 + 2 s)(2 n - 15) (IQ3_S codes, at most 465), exact in fp16, one logic operation and one
+// multiply-add for two weights. consts: what a row's sums of the chunk are multiplied with, fp32 (d, and for Q4_K -32 dmin
+// for the sums over the mins: the activation sums that these meet come divided by 32); mins: the fragment of the eight mins of
+// a row (16x256b.x1: lane 4 g + t holds positions 4 t .. 4 t + 3 of rows g, g + 8), twice: for the leading and the low halves of the
+// activation sums.
+template <uint32_t T> struct Exact;
+template <> struct Exact<T_Q4_K> {
+    static constexpr bool MINS = true;
+    static constexpr int SCRATCH = 16 * 4 * 4;
+    struct Pre { uint32_t magic; };
+    template <int u> __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t * scratch) {
+        const int g = lane >> 2, t = lane & 3;
+        const uint32_t * h0 = reinterpret_cast<const uint32_t *>(chunk + 2048 + 16 * g), * h1 = h0 + 32;       // d, dmin | s[12]
+        uint32_t sc0 = h0[1], sc1 = h1[1];
+        if (u) {
+            sc0 = (h0[3] & 0x0F0F0F0Fu) | ((sc0 >> 2) & 0x30303030u);
+            sc1 = (h1[3] & 0x0F0F0F0Fu) | ((sc1 >> 2) & 0x30303030u);
+        }
+        const uint32_t v = __byte_perm(sc0, sc1, uint32_t(t) * 0x0101u + 0x0400u);      // byte t of either row's word, 16 bits apart
+        __half2 sc = __hadd2(bits_h2((v & 0x003F003Fu) | 0x64006400u), __float2half2_rn(-1024.f));
+        if (t & 1) sc = __hmul2(sc, __float2half2_rn(0.0625f));
+        const __half2 ns = __hmul2(sc, __float2half2_rn(-1024.f));
+        uint32_t * to = reinterpret_cast<uint32_t *>(scratch) + lane;
+        to[0] = h2_bits(__lows2half2(sc, ns));
+        to[32] = h2_bits(__highs2half2(sc, ns));
+        return Pre{in_register(0x64006400u)};
+    }
+    template <int u, int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const uint8_t * scratch, const Pre & p, uint32_t (&f)[16]) {
+        const uint4 w4 = plane(chunk, 2 * u + JS, lane);
+        const uint2 * c = reinterpret_cast<const uint2 *>(scratch) + 2 * (lane >> 2) + JS;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const uint2 k = c[16 * r];
+            const __half2 S0 = __low2half2(bits_h2(k.x)), N0 = __high2half2(bits_h2(k.x)), S1 = __low2half2(bits_h2(k.y)), N1 = __high2half2(bits_h2(k.y));
+            auto lo = [&](uint32_t w) { return h2_bits(__hfma2(bits_h2(and_or(w, 0x000F000Fu, p.magic)), S0, N0)); };
+            auto hi = [&](uint32_t w) { return h2_bits(__hfma2(bits_h2(and_or(w, 0x00F000F0u, p.magic)), S1, N1)); };
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                const uint32_t v = r ? (b ? w4.w : w4.z) : (b ? w4.y : w4.x), v8 = v >> 8;
+                put(f, r, b, make_uint4(lo(v), lo(v8), hi(v), hi(v8)));
+            }
+        }
+    }
+    __device__ __forceinline__ static float2 consts(const uint8_t * chunk, int row) {
+        const __half2 h = *reinterpret_cast<const __half2 *>(chunk + 2048 + 16 * row);
+        return make_float2(__low2float(h), -32.f * __high2float(h));
+    }
+    __device__ __forceinline__ static void mins(const uint8_t * chunk, int lane, uint32_t (&f)[4]) {
+        const int g = lane >> 2;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const uint4 h = *reinterpret_cast<const uint4 *>(chunk + 2048 + 16 * (g + 8 * r));
+            // mins of sub-blocks 0 .. 3 (lanes t = 0, 2) or 4 .. 7 as bytes (src/formats/weight/dequant.cpp:56-64)
+            const uint32_t m = lane & 1 ? ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u) : h.z & 0x3F3F3F3Fu;
+            f[2 * r] = h2_bits(__hadd2(bits_h2(__byte_perm(m, 0x64646464u, 0x4140)), __float2half2_rn(-1024.f)));
+            f[2 * r + 1] = h2_bits(__hadd2(bits_h2(__byte_perm(m, 0x64646464u, 0x4342)), __float2half2_rn(-1024.f)));
+        }
+    }
+};
+template <> struct Exact<T_IQ3S4> {
+    static constexpr bool MINS = false;
+    static constexpr int SCRATCH = 16 * 4 * 4;
+    struct Pre { uint32_t one; };
+    template <int u> __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t * scratch) {
+        const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const uint32_t sc = *reinterpret_cast<const uint32_t *>(chunk + 2048 + 4 * (g + 8 * r)) >> (16 * u + 4 * t);
+            const __half2 s = bits_h2(((sc & 15u) * 0x00400040u) | 0x3C003C00u);        // 1 + s / 16 -> 32 (1 + 2 s), -47 (1 + 2 s)
+            reinterpret_cast<uint32_t *>(scratch)[lane + 32 * r] = h2_bits(__hfma2(s, __floats2half2_rn(1024.f, -1504.f), __floats2half2_rn(-992.f, 1457.f)));
+        }
+        return Pre{in_register(0x3C003C00u)};
+    }
+    template <int u, int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const uint8_t * scratch, const Pre & p, uint32_t (&f)[16]) {
+        using D = Dec<T_IQ3S4>;
+        const uint4 w4 = plane(chunk, 2 * u + JS, lane);
+        const uint2 * c = reinterpret_cast<const uint2 *>(scratch) + 2 * (lane >> 2) + JS;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const uint2 k = c[16 * r];
+            const __half2 S0 = __low2half2(bits_h2(k.x)), C0 = __high2half2(bits_h2(k.x)), S1 = __low2half2(bits_h2(k.y)), C1 = __high2half2(bits_h2(k.y));
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                const uint32_t v = r ? (b ? w4.w : w4.z) : (b ? w4.y : w4.x);
+                put(f, r, b, make_uint4(h2_bits(__hfma2(D::pair<0>(v, p.one), S0, C0)), h2_bits(__hfma2(D::pair<8>(v, p.one), S0, C0)),
+                                        h2_bits(__hfma2(D::pair<4>(v, p.one), S1, C1)), h2_bits(__hfma2(D::pair<12>(v, p.one), S1, C1))));
+            }
+        }
+    }
+    __device__ __forceinline__ static float2 consts(const uint8_t * chunk, int row) {
+        return make_float2(__half2float(*reinterpret_cast<const __half *>(chunk + 2112 + 2 * row)), 0.f);
+    }
+    __device__ __forceinline__ static void mins(const uint8_t *, int, uint32_t (&)[4]) {}
+};
+
+// ---------------------------------------------------------------------------------------------------------------
 // The eight 4-bit codes of a word -> their kvalues (exact) times `scale`, in nibble order, through a 256-entry table byte ->
 // half2 in shared memory with a copy per lane (no bank conflicts: entry b of lane l at word 32 b + l). Per code byte: a byte
 // permute extracts it, a multiply-add makes the address, one load, one product by the scale. The integer pipe takes one of

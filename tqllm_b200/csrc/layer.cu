@@ -1,6 +1,8 @@
 // C entry points of the expert products and the whole-layer sequence (router -> top-k -> dispatch -> gate/up + SwiGLU
 // -> down -> combine): the launch order of qwen35_forward.cpp:1121-1252 / fn_layer_forward.cpp:311-336,504-522 /
 // minimax.cpp:1083-1131 with every step stream-ordered on the device and no host read-back of the routing.
+#include <algorithm>
+
 #include "common.cuh"
 #include "formats.cuh"
 
@@ -39,6 +41,11 @@ int32_t gemm_tc_gateup(const b2moe_bank *, const b2moe_bank *, const b2moe_bank 
 int32_t gemm_tc_down(const b2moe_bank *, const b2moe_bank *, const void *, int x_dtype, bool per_token, const int *, int, int, int, long long live, void *,
                      int y_dtype, void *, cudaStream_t);
 void gemm_tc_item_tokens(int tokens);
+bool gemm_exact_supported(uint32_t type, int k, int experts);
+size_t gemm_exact_bytes(int slot_rows, int k, int dtype);
+int32_t gemm_exact_gateup(const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const void *, int, const int *, int, int, int, void *, int act_dtype,
+                          void * rows, bool slots, cudaStream_t);
+int32_t gemm_exact_down(const b2moe_bank *, const b2moe_bank *, const void *, int, bool per_token, const int *, int, int, int, void *, int y_dtype, void * rows, cudaStream_t);
 
 namespace {
 int32_t same_shape(const b2moe_bank * a, const b2moe_bank * b, bool same_experts) {
@@ -63,9 +70,9 @@ int decode_kernel(uint32_t type, int k, int dtype) {
 //   decode   every expert sees a few tokens, the product is bound by streaming the weights;
 //   GEMM     the tcgen05 grouped GEMM (all formats): the weights of an expert are decoded once per 128 tokens;
 //   generic  exact fp32 CUDA-core path: every shape, the floor under the other two.
-// Default: a type with a decode kernel takes it while the batch averages fewer than GEMM_MIN_PER assignments per expert or
-// the bank has fewer than GEMM_MIN_EXPERTS experts, everything else the GEMM. The line is one of precision as much as of time: the
-// decode kernels take the weights as they are and 15-bit activations, the GEMM rounds both to 11 bits. Relative error against
+// Default: a type with a decode kernel takes that family (for 4-bit codes in either of its forms, see exact_path) while the batch averages
+// fewer than GEMM_MIN_PER assignments per expert or the bank has fewer than GEMM_MIN_EXPERTS experts, everything else the GEMM. The line is one
+// of precision as much as of time: the decode kernels take the weights as they are and 15-bit activations, the GEMM rounds both to 11 bits. Relative error against
 // 64-bit sums (2-norm), decode / GEMM, at any density: Q4_K act 2.5e-5 / 4.0e-4, down of it 2.0e-4 / 5.3e-4; IQ3_S codes 2.5e-5 / 3.0e-4
 // and 2.0e-4 / 4.2e-4; IQ3_S in GGUF fields 2e-7 / 3.0e-4 and 2.1e-4 / 4.2e-4. The GEMM is the faster one from about 16 per
 // expert on (layer times, decode / GEMM, us: Q4_K of 256 experts at 19 per expert 1139 / 1027, of 60 at 30 249 / 184; IQ3_S codes of 512 at
@@ -73,22 +80,35 @@ int decode_kernel(uint32_t type, int k, int dtype) {
 // (tests and benchmarks).
 constexpr int GEMM_MIN_PER = 32, GEMM_MIN_EXPERTS = 128;
 int g_family = B2MOE_FAMILY_AUTO;
-int expert_path(uint32_t type, int k, int dtype, int experts, long long assignments) {
-    if (g_family == B2MOE_FAMILY_GENERIC) return B2MOE_FAMILY_GENERIC;
+int expert_path(uint32_t type, int k, int dtype, int experts, long long assignments, int family = g_family) {
+    if (family == B2MOE_FAMILY_GENERIC) return B2MOE_FAMILY_GENERIC;
     const bool dec = decode_kernel(type, k, dtype) != DEC_NONE, gemm = gemm_tc_supported(type, k, experts);
-    if (g_family == B2MOE_FAMILY_DECODE) return dec ? B2MOE_FAMILY_DECODE : B2MOE_FAMILY_GENERIC;
-    if (g_family == B2MOE_FAMILY_GEMM) return gemm ? B2MOE_FAMILY_GEMM : dec ? B2MOE_FAMILY_DECODE : B2MOE_FAMILY_GENERIC;
+    if (family == B2MOE_FAMILY_DECODE) return dec ? B2MOE_FAMILY_DECODE : B2MOE_FAMILY_GENERIC;
+    if (family == B2MOE_FAMILY_GEMM) return gemm ? B2MOE_FAMILY_GEMM : dec ? B2MOE_FAMILY_DECODE : B2MOE_FAMILY_GENERIC;
     if (dec && (!gemm || assignments < (long long)GEMM_MIN_PER * experts || experts < GEMM_MIN_EXPERTS)) return B2MOE_FAMILY_DECODE;
     return gemm ? B2MOE_FAMILY_GEMM : B2MOE_FAMILY_GENERIC;
+}
+// Where the rule above says DECODE, banks of 4-bit codes have a second form: the grouped GEMM with integer operands and scales
+// applied to its sums in fp32 (gemm_exact_*), which loses less precision than the decode kernels and reads an expert's weights once per 32
+// tokens instead of once per eight. It takes over from EXACT_MIN_PER assignments per expert on. Layer times, decode / this form, us: Q4_K of 256
+// experts at 7.8 per expert 629 / 685, 19 1237 / 797, 31 1920 / 1116; of 60 at 7.7 106 / 109, 10 124 / 111, 100 577 / 315; of 32 in fp32 at 8 45 / 43, 1000 838 / 491; IQ3_S
+// codes of 512 at 7 307 / 336, 8 339 / 344, 10 390 / 355. Relative error of both products against 64 bits 2.0e-4 / 1.0e-6. Gate/up on 16-bit rows runs
+// from any scratch that the call accepts; fp32 rows (two terms each) take the decode kernels where the scratch has no room for them.
+constexpr int EXACT_MIN_PER = 9;
+bool exact_path(uint32_t type, int k, int dtype, int experts, long long live, int family = g_family) {
+    return (family == B2MOE_FAMILY_AUTO || family == B2MOE_FAMILY_DECODE) && decode_kernel(type, k, dtype) == DEC_4BIT && live >= (long long)EXACT_MIN_PER * experts &&
+           expert_path(type, k, dtype, experts, live, family) == B2MOE_FAMILY_DECODE && gemm_exact_supported(type, k, experts);
 }
 }  // namespace
 // One matrix over a ready plan with the caller's own row types: x [assignments or, per_token, tokens][cols] of x_dtype -> y
 // [assignments][rows] of y_dtype, without a pass to fp32 before and one back behind. *took = false: the family that serves this call
 // has no such form (b2moe_expert_down on fp32 rows does it).
 int32_t product_typed(const b2moe_bank * m, const void * x, int x_dtype, bool per_token, const int * plan, int n, int topk, void * y, int y_dtype,
-                      void * ws, cudaStream_t s, bool * took) {
+                      void * ws, void * rows_buf, size_t rows_buf_bytes, cudaStream_t s, bool * took) {
     const int path = expert_path(m->type, m->cols, B2MOE_F32, m->experts, (long long)n * topk);
     *took = true;
+    if (exact_path(m->type, m->cols, x_dtype, m->experts, (long long)n * topk) && rows_buf_bytes >= gemm_exact_bytes(n * topk, m->cols, x_dtype))
+        return gemm_exact_down(m, nullptr, x, x_dtype, per_token, plan, n, topk, 0, y, y_dtype, rows_buf, s);
     if (path == B2MOE_FAMILY_GEMM) return gemm_tc_down(m, nullptr, x, x_dtype, per_token, plan, n, topk, 0, (long long)n * topk, y, y_dtype, ws, s);
     if (path == B2MOE_FAMILY_DECODE && decode_kernel(m->type, m->cols, B2MOE_F32) == DEC_4BIT)
         return dec4_down(m, nullptr, x, x_dtype, per_token, plan, n, topk, 0, y, y_dtype, ws, s);
@@ -100,6 +120,12 @@ int32_t gateup_typed(const b2moe_bank * gate, const b2moe_bank * up, const void 
                      void * ws, void * rows_buf, size_t rows_buf_bytes, cudaStream_t s, bool * took) {
     const int path = expert_path(gate->type, gate->cols, x_dtype, gate->experts, (long long)n * topk);
     *took = true;
+    if (exact_path(gate->type, gate->cols, x_dtype, gate->experts, (long long)n * topk)) {
+        if (rows_buf_bytes >= gemm_exact_bytes(n * topk, gate->cols, x_dtype))
+            return gemm_exact_gateup(gate, up, nullptr, nullptr, x, x_dtype, plan, n, topk, 0, act, act_dtype, rows_buf, true, s);
+        *took = x_dtype == B2MOE_F32;                                  // 16-bit rows: the call with fp32 results gathers them, for the same bits
+        if (!*took) return B2MOE_OK;
+    }
     if (path == B2MOE_FAMILY_GEMM && gemm_tc_slot_bytes(n * topk, gate->cols) <= rows_buf_bytes) return gemm_tc_gateup(gate, up, nullptr, nullptr, x, x_dtype, plan, n, topk, 0, (long long)n * topk, act, act_dtype, ws, rows_buf,
                                                                rows_buf_bytes, s);
     if (path == B2MOE_FAMILY_DECODE && decode_kernel(gate->type, gate->cols, x_dtype) == DEC_4BIT)
@@ -181,11 +207,18 @@ static int32_t expert_gateup(const b2moe_bank * gate, const b2moe_bank * up, con
         if (need && !workspace) return B2MOE_ERR_NULL;
         if (need && !aligned16(workspace)) return B2MOE_ERR_ALIGN;
         if (workspace_bytes < need) return B2MOE_ERR_WORKSPACE;
+        void * const spare = rows_buf ? rows_buf : workspace;
+        const size_t spare_bytes = rows_buf ? rows_buf_bytes : workspace_bytes;
+        if (exact_path(gate->type, gate->cols, x_dtype, gate->experts, live)) {
+            const bool slots = spare_bytes >= gemm_exact_bytes(n * topk + shared_tokens, gate->cols, x_dtype);
+            if (slots || x_dtype != B2MOE_F32)
+                return gemm_exact_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, B2MOE_F32, slots ? spare : workspace, slots, as_stream(stream));
+        }
         // a workspace larger than it has to be may hold the rows in slot order itself (gemm_tc_gateup looks at its size): IQ4 banks,
         // 8192 tokens of 8, gate/up alone 2050 us with gathered rows and 1415 with slot order
         if (path == B2MOE_FAMILY_GEMM)
-            return gemm_tc_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, live, act, B2MOE_F32, workspace,
-                                  rows_buf ? rows_buf : workspace, rows_buf ? rows_buf_bytes : workspace_bytes, as_stream(stream));
+            return gemm_tc_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, live, act, B2MOE_F32, workspace, spare, spare_bytes,
+                                  as_stream(stream));
         if (decode_kernel(gate->type, gate->cols, x_dtype) == DEC_4BIT)
             return dec4_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, B2MOE_F32, workspace, as_stream(stream), x_staged);
         return iq3s_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, workspace, max_active_of(gate->experts, n, topk, shared_tokens), as_stream(stream));
@@ -217,6 +250,8 @@ static int32_t expert_down(const b2moe_bank * down, const b2moe_bank * shared_do
         if (!workspace) return B2MOE_ERR_NULL;
         if (!aligned16(workspace)) return B2MOE_ERR_ALIGN;
         if (workspace_bytes < b2moe_expert_workspace_bytes(down->type, rows_x, down->cols, B2MOE_F32)) return B2MOE_ERR_WORKSPACE;
+        if (exact_path(down->type, down->cols, B2MOE_F32, down->experts, live) && workspace_bytes >= gemm_exact_bytes(rows_x, down->cols, B2MOE_F32))
+            return gemm_exact_down(down, shared_down, act, B2MOE_F32, false, plan, n, topk, shared_tokens, y, B2MOE_F32, workspace, as_stream(stream));
         if (path == B2MOE_FAMILY_GEMM)
             return gemm_tc_down(down, shared_down, act, B2MOE_F32, false, plan, n, topk, shared_tokens, live, y, B2MOE_F32, workspace, as_stream(stream));
         if (decode_kernel(down->type, down->cols, B2MOE_F32) == DEC_4BIT)
@@ -248,7 +283,7 @@ extern "C" B2MOE_API int32_t b2moe_expert_down_sparse(const b2moe_bank * down, c
     return expert_down(down, shared_down, act, plan, n, topk, shared_tokens, y, workspace, workspace_bytes, stream, live_assignments);
 }
 
-extern "C" B2MOE_API int32_t b2moe_layer_workspace(const b2moe_layer * L, int32_t n, b2moe_layer_ws * ws) {
+static int32_t layer_layout(const b2moe_layer * L, int32_t n, b2moe_layer_ws * ws) {
     if (!L || !ws) return B2MOE_ERR_NULL;
     if (n <= 0 || L->hidden <= 0 || L->experts <= 0 || L->topk <= 0 || L->topk > L->experts || L->ff <= 0) return B2MOE_ERR_SHAPE;
     if ((long long)n * L->topk > 0x3fffffffLL) return B2MOE_ERR_SHAPE;
@@ -269,11 +304,19 @@ extern "C" B2MOE_API int32_t b2moe_layer_workspace(const b2moe_layer * L, int32_
     ws->total = at;
     return B2MOE_OK;
 }
+// The caller is asked for what the exact form of the down product takes where it would be chosen; layer_forward needs no more than layer_layout says
+extern "C" B2MOE_API int32_t b2moe_layer_workspace(const b2moe_layer * L, int32_t n, b2moe_layer_ws * ws) {
+    if (int32_t rc = layer_layout(L, n, ws)) return rc;
+    const int At = n * L->topk + (L->has_shared ? n : 0);
+    const size_t exact = gemm_exact_bytes(At, L->ff, B2MOE_F32);
+    if (exact_path(L->down.type, L->ff, B2MOE_F32, L->experts, (long long)n * L->topk, B2MOE_FAMILY_AUTO)) ws->total = std::max(ws->total, ws->expert_scratch + align_up(exact, 256));
+    return B2MOE_OK;
+}
 
 static int32_t layer_forward(const b2moe_layer * L, const void * x, int32_t x_dtype, int32_t n, const void * residual, void * out,
                              int32_t out_dtype, void * workspace, size_t workspace_bytes, b2moe_stream stream) {
     b2moe_layer_ws ws;
-    if (int32_t rc = b2moe_layer_workspace(L, n, &ws)) return rc;
+    if (int32_t rc = layer_layout(L, n, &ws)) return rc;
     if (!x || !out || !workspace || !L->router_w) return B2MOE_ERR_NULL;
     if (workspace_bytes < ws.total) return B2MOE_ERR_WORKSPACE;
     if (!aligned16(workspace)) return B2MOE_ERR_ALIGN;
@@ -295,7 +338,7 @@ static int32_t layer_forward(const b2moe_layer * L, const void * x, int32_t x_dt
                                   n, stream)) return rc;
     if (L->gating == B2MOE_SIGMOID && gated_shared) return B2MOE_ERR_SHAPE;   // the sigmoid family adds its shared expert unscaled (moe_common.cu:191)
     void * es = base + ws.expert_scratch;
-    const size_t es_bytes = ws.total - ws.expert_scratch;
+    const size_t es_bytes = workspace_bytes - ws.expert_scratch;
     // decode-sized call on the 4-bit decode kernels: top-k, dispatch and the staging of x in one cluster launch
     bool x_staged = false;
     if (route_cluster_fits(L->experts, L->topk, n) && es_bytes >= b2moe_expert_workspace_bytes(L->gate.type, n, L->gate.cols, x_dtype) &&
@@ -312,9 +355,10 @@ static int32_t layer_forward(const b2moe_layer * L, const void * x, int32_t x_dt
         if (int32_t rc = b2moe_route_dispatch(L->gating, logits, ld, L->sel_bias, ids, weights, gated_shared ? shw : nullptr, L->experts, L->topk,
                                               L->norm, L->scale, n, 0, sh, plan, base + ws.scratch, ws.expert_scratch - ws.scratch, stream))
             return rc;
-    // y is written by the down product: until then its rows hold the gate/up product's activation rows
+    // y is written by the down product: until then its rows (and what lies behind them: the dispatch is done, and a product that
+    // converts its rows into y takes no other scratch) hold the gate/up product's activation rows
     if (int32_t rc = expert_gateup(&L->gate, &L->up, &L->sh_gate, &L->sh_up, x, x_dtype, plan, n, L->topk, sh, act, es, es_bytes, stream, x_staged, -1, y,
-                                   ws.scratch - ws.y)) return rc;
+                                   workspace_bytes - ws.y)) return rc;
     if (int32_t rc = b2moe_expert_down(&L->down, &L->sh_down, act, plan, n, L->topk, sh, y, es, es_bytes, stream)) return rc;
     if (residual) return b2moe_combine_residual(y, nullptr, weights, gated_shared ? shw : nullptr, residual, n, L->topk, L->hidden, sh, out, out_dtype, stream);
     return b2moe_combine(y, nullptr, weights, gated_shared ? shw : nullptr, n, L->topk, L->hidden, sh, out, out_dtype, stream);

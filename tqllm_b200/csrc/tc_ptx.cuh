@@ -52,6 +52,10 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const void * map, int 
     asm volatile("cp.async.bulk.tensor.3d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                  ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
 }
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const void * map, int x, int y, int z, int w, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar) : "memory");
+}
 // one lane of a converged warp, the same every time
 __device__ __forceinline__ bool elect_one() {
     uint32_t ok;
@@ -76,6 +80,8 @@ __device__ __forceinline__ void tmem_free(uint32_t base, uint32_t cols) {
 // atoms. Split in halves: the low half carries the address, the high half is a constant (sbo 1024, fixed bit 46, swizzle).
 constexpr uint32_t SW128_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t sw128_desc_lo(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | (1u << 16); }
+// the same for rows of 32 bytes (sixteen 16-bit values), 32-byte swizzle: eight rows are 256 bytes
+constexpr uint32_t SW32_DESC_HI = (256u >> 4) | (1u << 14) | (6u << 29);
 // instruction descriptor: fp32 accumulator, K-major A and B, M x N; ab_format: 0 = E4M3 (kind::f8f6f4) / fp16 (kind::f16),
 // 1 = bf16 (kind::f16)
 __device__ __forceinline__ uint32_t idesc(uint32_t m, uint32_t n, uint32_t ab_format) {
@@ -83,9 +89,10 @@ __device__ __forceinline__ uint32_t idesc(uint32_t m, uint32_t n, uint32_t ab_fo
 }
 // One product with A (128 x 16, fp16) in tensor memory (row in lane, two values of K per column) and B (N x 16) in shared memory,
 // fp32 sums in tensor memory, added to what is there when acc != 0. One thread issues.
+template <uint32_t DESC_HI = SW128_DESC_HI>
 __device__ __forceinline__ void mma_f16(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t id, uint32_t acc) {
     asm volatile("{\n .reg .pred p;\n .reg .b64 db;\n setp.ne.b32 p, %4, 0;\n mov.b64 db, {%2, %5};\n"
-                 " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n}" ::"r"(d), "r"(a), "r"(b_lo), "r"(id), "r"(acc), "r"(SW128_DESC_HI) : "memory");
+                 " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n}" ::"r"(d), "r"(a), "r"(b_lo), "r"(id), "r"(acc), "r"(DESC_HI) : "memory");
 }
 // a 64-column step: four products, even ones into d0 (added when acc0), odd ones into d1 (acc1); the two may be the same
 __device__ __forceinline__ void mma_step(uint32_t d0, uint32_t d1, uint32_t a, uint32_t b_lo, uint32_t id, uint32_t acc0, uint32_t acc1) {
@@ -104,6 +111,14 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
                    "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                  : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+}
+// 16 rows x 8 columns, as the first four registers of the next one
+__device__ __forceinline__ void tmem_st_16x256b_x1(uint32_t taddr, const uint32_t (&r)[4]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x1.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
 }
 // a warp's 16 rows x 32 columns from the registers of an m16n8-style fragment: register 4 i + 2 r + c of lane 4 g + t is column
 // 8 i + 2 t + c of row g + 8 r; taddr's lane is the first of the 16 (a multiple of 16 inside the warp's quarter)
