@@ -361,7 +361,9 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
         if (lane == 0) info[na].cum = carry;
     }
     __syncthreads();
-    const uint32_t tmem = *tmem_slot;
+    // All 512 columns are this block's, so they begin at column 0 of lane 0. As a constant the base saves the issuing thread an addition and
+    // a move into the uniform registers per product: c5 decode 24 gate/up 196.6 -> 194.5 us, down 119 -> 115
+    constexpr uint32_t tmem = 0;
     const int n_items = info[na].cum;
 
     // item -> expert, first token slot, token count, row block; called by whole warps, with `at` = the active expert of the
