@@ -33,7 +33,7 @@ __global__ void groups_head_k(const int * counts_in, int experts, int capacity, 
     for (int x = threadIdx.x; x < experts; x += blockDim.x) counts[x] = max(0, min(counts_in[x], capacity));
     if (threadIdx.x == 0) counts[experts] = 0;
     __syncthreads();
-    finish_plan(plan, counts, offsets, active, offsets, active, perm + assignments, e1, true);
+    finish_plan(plan, counts, offsets, offsets, active, perm + assignments, e1, true);
 }
 __global__ void groups_perm_k(const int * groups, int experts, int capacity, int * plan) {
     grid_release();

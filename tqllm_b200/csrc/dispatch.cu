@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(WALK_THREADS) dispatch_place_k(const WalkArgs 
     grid_release();
     grid_wait();
     const int e = p.e, e1 = e + 1, parts = row_parts(e), blocks = gridDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int * hist = walk_mem, * total = hist + WALK_WARPS * e, * lower = total + parts * e, * cs = lower + parts * e, * os = cs + e + 2, * as = os + e + 2;
+    int * hist = walk_mem, * total = hist + WALK_WARPS * e, * lower = total + parts * e, * cs = lower + parts * e, * os = cs + e + 2;
     int * counts = p.plan + PLAN_HDR, * offsets = counts + e1, * active = offsets + e1 + 1, * perm = active + e1;
     for (int i = threadIdx.x; i < parts * e; i += WALK_THREADS) {
         const int x = i % e, part = i / e, per = (blocks + parts - 1) / parts, r1 = min(blocks, (part + 1) * per);
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(WALK_THREADS) dispatch_place_k(const WalkArgs 
         if (blockIdx.x == 0) counts[e] = p.shared_tokens;
     }
     __syncthreads();
-    finish_plan(p.plan, cs, os, as, offsets, active, perm + p.A + p.shared_tokens, e1, blockIdx.x == 0);
+    finish_plan(p.plan, cs, os, offsets, active, perm + p.A + p.shared_tokens, e1, blockIdx.x == 0);
     __syncthreads();
     int * h = hist + warp * e;
     walk_ids<true>(p.ids, a0, a1, e, lane, [&](int a, int id, unsigned peers) {
@@ -132,7 +132,7 @@ __global__ void dispatch_scan_k(int * __restrict__ hist, int chunks, int e, int 
         counts[x] = prefix_counters(hist + x, chunks, e);
     if (threadIdx.x == 0) counts[e] = shared_tokens;
     __syncthreads();
-    finish_plan(plan, counts, offsets, active, offsets, active, active + e1 + A + shared_tokens, e1, true);
+    finish_plan(plan, counts, offsets, offsets, active, active + e1 + A + shared_tokens, e1, true);
 }
 __global__ void dispatch_scatter_k(const int * __restrict__ ids, int A, int e, int shared_first, int shared_tokens, int * __restrict__ hist,
                                    int * __restrict__ plan) {

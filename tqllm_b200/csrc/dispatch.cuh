@@ -60,59 +60,62 @@ __device__ __forceinline__ int prefix_counters(C * h, int n, int stride) {
     return run;
 }
 
-// exclusive prefix sums of (a, b) over the threads of a block of whole warps, and their totals; w: 32 entries of shared memory
-__device__ __forceinline__ int2 block_scan(int a, int b, int2 * w, int2 & total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    int pa = a, pb = b;
-    for (int d = 1; d < 32; d <<= 1) {
-        const int oa = __shfl_up_sync(0xffffffffu, pa, d), ob = __shfl_up_sync(0xffffffffu, pb, d);
-        if (lane >= d) { pa += oa; pb += ob; }
+// exclusive prefix sums of (x, y, z) over the threads of a block's first `used` warps, and their totals, for those warps; w: 32
+// entries of shared memory; one barrier for the whole block
+__device__ __forceinline__ int3 block_scan(int3 v, int used, int3 * w, int3 & total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int3 p = v;
+    if (warp < used) {
+#pragma unroll 1
+        for (int d = 1; d < 32; d <<= 1) {
+            const int ox = __shfl_up_sync(0xffffffffu, p.x, d), oy = __shfl_up_sync(0xffffffffu, p.y, d), oz = __shfl_up_sync(0xffffffffu, p.z, d);
+            if (lane >= d) { p.x += ox; p.y += oy; p.z += oz; }
+        }
+        if (lane == 31) w[warp] = p;
     }
-    if (lane == 31) w[warp] = make_int2(pa, pb);
     __syncthreads();
-    const int2 own = lane < nw ? w[lane] : make_int2(0, 0);
-    int wa = own.x, wb = own.y;
+    if (warp >= used) return p;
+    const int3 own = lane < used ? w[lane] : make_int3(0, 0, 0);
+    int3 q = own;
+#pragma unroll 1
     for (int d = 1; d < 32; d <<= 1) {
-        const int oa = __shfl_up_sync(0xffffffffu, wa, d), ob = __shfl_up_sync(0xffffffffu, wb, d);
-        if (lane >= d) { wa += oa; wb += ob; }
+        const int ox = __shfl_up_sync(0xffffffffu, q.x, d), oy = __shfl_up_sync(0xffffffffu, q.y, d), oz = __shfl_up_sync(0xffffffffu, q.z, d);
+        if (lane >= d) { q.x += ox; q.y += oy; q.z += oz; }
     }
-    total = make_int2(__shfl_sync(0xffffffffu, wa, 31), __shfl_sync(0xffffffffu, wb, 31));
-    const int la = __shfl_sync(0xffffffffu, wa - own.x, warp), lb = __shfl_sync(0xffffffffu, wb - own.y, warp);
-    return make_int2(la + pa - a, lb + pb - b);
+    total = make_int3(__shfl_sync(0xffffffffu, q.x, 31), __shfl_sync(0xffffffffu, q.y, 31), __shfl_sync(0xffffffffu, q.z, 31));
+    return make_int3(__shfl_sync(0xffffffffu, q.x - own.x, warp) + p.x - v.x, __shfl_sync(0xffffffffu, q.y - own.y, warp) + p.y - v.y,
+                     __shfl_sync(0xffffffffu, q.z - own.z, warp) + p.z - v.z);
 }
 
-// counts cs[0..e1) -> offsets[0..e1], active list, pass list and the header words, by all threads of the block, each with a
-// contiguous span of the experts (one warp for all of them was a chain of e1 / 32 dependent steps, three times over: 2 us of dispatch_place_k at 512 experts).
-// cs, os and as are shared-memory copies; with `write` every result also goes to the plan in global memory. The caller
-// synchronises before (cs) and after (os).
-__device__ inline void finish_plan(int * plan, const int * cs, int * os, int * as, int * offsets, int * active, int * passes, int e1, bool write) {
-    __shared__ int2 wsum[2][32];
+// counts cs[0..e1) -> offsets os[0..e1] and, with `write`, the plan's offsets, active list, pass list and header words, by the threads of
+// the block, each with a contiguous span of the experts (one warp for all of them was a chain of e1 / 32 dependent steps, three times
+// over: 2 us of dispatch_place_k at 512 experts). The pass list runs over the active experts from the last (the shared expert, the heaviest) to the
+// first, cut into passes of PASS_TOKENS tokens: passes[i] = passes before the i-th expert of that order = all of them but those up to
+// that expert, so tokens, experts and passes take one scan and one barrier together (a scan for the passes alone, behind the list that it read, was half of
+// the 3.6 to 8 thousand cycles that this took in a routing launch). cs and os are shared-memory copies, or the plan's own arrays.
+// The caller synchronises before (cs) and after (os).
+__device__ inline void finish_plan(int * plan, const int * cs, int * os, int * offsets, int * active, int * passes, int e1, bool write) {
+    __shared__ int3 wsum[32];
     const int nt = blockDim.x, span = (e1 + nt - 1) / nt, lo = min(e1, int(threadIdx.x) * span), hi = min(e1, lo + span);
-    int sum = 0, act = 0;
-    for (int i = lo; i < hi; ++i) { sum += cs[i]; act += cs[i] > 0; }
-    int2 total, at = block_scan(sum, act, wsum[0], total);
+    const int used = ((e1 + span - 1) / span + 31) >> 5;
+    int3 v = make_int3(0, 0, 0), total;
+    for (int i = lo; i < hi; ++i) { const int c = cs[i]; v.x += c; v.y += c > 0; v.z += (c + PASS_TOKENS - 1) / PASS_TOKENS; }
+    int3 at = block_scan(v, used, wsum, total);
     for (int i = lo; i < hi; ++i) {
         const int c = cs[i];
         os[i] = at.x;
         if (write) offsets[i] = at.x;
+        at.x += c;
         if (c > 0) {
-            as[at.y] = i;
-            if (write) active[at.y] = i;
+            at.z += (c + PASS_TOKENS - 1) / PASS_TOKENS;
+            if (write) { active[at.y] = i; passes[total.y - 1 - at.y] = total.z - at.z; }
             ++at.y;
         }
-        at.x += c;
     }
-    if (!write) return;
-    if (threadIdx.x == 0) { offsets[e1] = total.x; os[e1] = total.x; plan[PLAN_NGROUPED] = total.x; plan[PLAN_NACTIVE] = total.y; plan[PLAN_STATUS] = 0; }
-    __syncthreads();
-    // pass list: active experts from the last (the shared expert, the heaviest) to the first, cut into passes of
-    // PASS_TOKENS tokens; passes[i] = number of passes before the i-th expert of that order
-    const int na = total.y, sp = (na + nt - 1) / nt, l2 = min(na, int(threadIdx.x) * sp), h2 = min(na, l2 + sp);
-    int mine = 0;
-    for (int i = l2; i < h2; ++i) mine += (cs[as[na - 1 - i]] + PASS_TOKENS - 1) / PASS_TOKENS;
-    int rp = block_scan(mine, 0, wsum[1], total).x;
-    for (int i = l2; i < h2; ++i) { passes[i] = rp; rp += (cs[as[na - 1 - i]] + PASS_TOKENS - 1) / PASS_TOKENS; }
-    if (threadIdx.x == 0) { passes[na] = total.x; plan[PLAN_NPASS] = total.x; }
+    if (write && threadIdx.x == 0) {
+        offsets[e1] = total.x; os[e1] = total.x; passes[total.y] = total.z;
+        plan[PLAN_NGROUPED] = total.x; plan[PLAN_NACTIVE] = total.y; plan[PLAN_NPASS] = total.z; plan[PLAN_STATUS] = 0;
+    }
 }
 
 // shared memory of dispatch_small_body for a block of `warps` warps: hist [warps][e] (16-bit) + three int arrays of e + 2
@@ -125,27 +128,44 @@ __device__ __forceinline__ void dispatch_small_body(const int * ids, int A, int 
     const int e1 = e + 1;
     int * counts = plan + PLAN_HDR, * offsets = counts + e1, * active = offsets + e1 + 1, * perm = active + e1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    int * cs = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(hist) + (size_t(nw) * e * 2 + 15) / 16 * 16), * os = cs + e + 2, * as = os + e + 2;
+    int * cs = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(hist) + (size_t(nw) * e * 2 + 15) / 16 * 16), * os = cs + e + 2;
     const int chunk = ((A + nw - 1) / nw + 31) / 32 * 32;   // per warp, a multiple of 32
-    for (int i = threadIdx.x; i < nw * e; i += blockDim.x) hist[i] = 0;
-    __syncthreads();
+    const int used = (A + chunk - 1) / chunk;               // warps that have assignments: a decode step's ids fill a few of them
     const int a0 = warp * chunk;
     const int a1 = min(A, a0 + chunk);
     unsigned short * h = hist + warp * e;
-    walk_ids<VOTES>(ids, a0, a1, e, lane, [&](int, int id, unsigned peers) {
-        if (id >= 0 && lane == __ffs(peers) - 1) h[id] += (unsigned short)__popc(peers);
-    });
+    // one step a warp: its id and the lanes that share it stay in registers for the second walk
+    int id1 = -1;
+    unsigned peers1 = 0;
+    const bool one = chunk == 32;
+    if (one && warp < used) id1 = valid_id(ids, a0 + lane, a1, e);          // asked for before the counters are cleared
+    if (warp < used) for (int i = lane; i < e; i += 32) h[i] = 0;
+    __syncwarp();
+    if (one) {
+        if (warp < used) {
+            peers1 = VOTES ? same_id(id1, 32 - __clz(e - 1)) : __match_any_sync(0xffffffffu, id1);
+            if (id1 >= 0 && lane == __ffs(peers1) - 1) h[id1] = (unsigned short)__popc(peers1);
+        }
+    } else if (warp < used) {
+        walk_ids<VOTES>(ids, a0, a1, e, lane, [&](int, int id, unsigned peers) {
+            if (id >= 0 && lane == __ffs(peers) - 1) h[id] += (unsigned short)__popc(peers);
+        });
+    }
     __syncthreads();
-    for (int x = threadIdx.x; x < e; x += blockDim.x) counts[x] = cs[x] = prefix_counters(hist + x, nw, e);
+    for (int x = threadIdx.x; x < e; x += blockDim.x) counts[x] = cs[x] = prefix_counters(hist + x, used, e);
     if (threadIdx.x == 0) { counts[e] = shared_tokens; cs[e] = shared_tokens; }
     __syncthreads();
-    finish_plan(plan, cs, os, as, offsets, active, perm + A + shared_tokens, e1, true);
+    finish_plan(plan, cs, os, offsets, active, perm + A + shared_tokens, e1, true);
     __syncthreads();
-    walk_ids<VOTES>(ids, a0, a1, e, lane, [&](int a, int id, unsigned peers) {
-        if (id >= 0) perm[os[id] + h[id] + __popc(peers & ((1u << lane) - 1u))] = a;
-        __syncwarp();
-        if (id >= 0 && lane == __ffs(peers) - 1) h[id] += (unsigned short)__popc(peers);
-    });
+    if (one) {
+        if (id1 >= 0) perm[os[id1] + h[id1] + __popc(peers1 & ((1u << lane) - 1u))] = a0 + lane;
+    } else if (warp < used) {
+        walk_ids<VOTES>(ids, a0, a1, e, lane, [&](int a, int id, unsigned peers) {
+            if (id >= 0) perm[os[id] + h[id] + __popc(peers & ((1u << lane) - 1u))] = a;
+            __syncwarp();
+            if (id >= 0 && lane == __ffs(peers) - 1) h[id] += (unsigned short)__popc(peers);
+        });
+    }
     for (int t = threadIdx.x; t < shared_tokens; t += blockDim.x) perm[os[e] + t] = A + shared_first + t;
 }
 
