@@ -187,8 +187,13 @@ template <bool STAGER> constexpr int threads_of() { return (CTA_WARPS + (STAGER 
 template <bool STAGER> constexpr int bound_threads() { return STAGER ? 640 : threads_of<false>(); }
 
 // MODE 0: out = act[a][row] = silu(gate . x) * (up . x);   MODE 1: out = y[a][row] = down . act[a]
-template <uint32_t T, int MODE, bool STAGER>
-__global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4Args p) {
+// FEW: the instances of small launches (a few jobs per block): chains of latencies more than streams, so the way from the plan to the first copy is
+// shorter there and a block's share lies in one pass where that costs no round. The other instances keep their plain walk: these
+// lines in them cost the compiler registers and every large launch 2.5 % (64 tokens of 512 IQ3_S experts, gate/up 87.6 -> 90 us).
+template <uint32_t T, int MODE, bool FEW>
+__global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(const Dec4Args p) {
+    constexpr bool STAGER = FEW && MODE == 1;
+    using Job = typename std::conditional<FEW, int, long long>::type;
     using F = D4<T>;
     constexpr int NMAT = MODE == 0 ? 2 : 1, TILE = F::TILE;
     // how the byte sums of a four-token pass meet: two shuffles and half of the fp32 steps, or four shuffles and no selects.
@@ -230,17 +235,46 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
     const int na = p.plan[PLAN_NACTIVE], row_tiles = (p.rows + 15) >> 4;
     // the block's share of the launch: jobs [u_begin, u_end) of the pass-major list of (pass, row tile) jobs; it walks the
     // share as segments = runs of row tiles [r0, r1) of one pass
-    const long long n_jobs = (long long)p.plan[PLAN_NPASS] * row_tiles;
-    const long long u_begin = n_jobs * blockIdx.x / gridDim.x, u_end = n_jobs * (blockIdx.x + 1) / gridDim.x;
-    auto segment = [&](long long u, int & pass, int & r0, int & r1) {
+    const int n_pass = p.plan[PLAN_NPASS];
+    const Job n_jobs = Job(n_pass) * row_tiles;
+    Job u_begin, u_end;
+    if constexpr (FEW) {
+        // n_jobs b / blocks = q b + r b / blocks with n_jobs = q blocks + r: 32-bit divisions
+        const int blocks = int(gridDim.x), q = n_jobs / blocks, r = n_jobs - q * blocks;
+        u_begin = q * int(blockIdx.x) + r * int(blockIdx.x) / blocks;
+        u_end = q * int(blockIdx.x + 1) + r * int(blockIdx.x + 1) / blocks;
+        // Few passes: every pass on blocks of its own, where a block's share is then still one round of JW jobs. A share that runs into a
+        // second pass waits for that one's plan entries, activation rows and products in turn: one token of 512 IQ3_S experts, gate/up 9.2 us where 6.6
+        // do. Larger shares hide that behind their rounds, and whole passes leave them uneven (8 tokens, 75 passes: 73.5 us a layer with equal shares, 80).
+        const int per_pass = blocks / max(n_pass, 1);
+        if (per_pass > 0 && (row_tiles + per_pass - 1) / per_pass <= JW) {
+            const int pass = int(blockIdx.x) / per_pass, part = int(blockIdx.x) - pass * per_pass;
+            u_begin = u_end = 0;
+            if (pass < n_pass) {
+                u_begin = pass * row_tiles + row_tiles * part / per_pass;
+                u_end = pass * row_tiles + row_tiles * (part + 1) / per_pass;
+            }
+        }
+    } else {
+        u_begin = n_jobs * blockIdx.x / gridDim.x;
+        u_end = n_jobs * (blockIdx.x + 1) / gridDim.x;
+    }
+    auto segment = [&](Job u, int & pass, int & r0, int & r1) {
         pass = int(u / row_tiles);
-        r0 = int(u - (long long)pass * row_tiles);
-        r1 = int(min((long long)row_tiles, r0 + (u_end - u)));
+        r0 = int(u - Job(pass) * row_tiles);
+        r1 = int(min(Job(row_tiles), r0 + (u_end - u)));
     };
 
     // pass w -> (expert, first token slot); the pass list runs over the active experts from the last to the first. Called by
     // all lanes of the producer warp together: two rounds of 32 probes instead of a ten-step chain of dependent loads.
     auto locate = [&](int w, int & e, int & c0) {
+        if (FEW && na <= 32) {                                                     // one round, which brings the experts along
+            const int i = min(lane, na - 1), at = passes[i], expert = active[na - 1 - i];
+            const int src = 31 - __clz(int(__ballot_sync(0xffffffffu, lane < na && at <= w) | 1u));
+            e = __shfl_sync(0xffffffffu, expert, src);
+            c0 = (w - __shfl_sync(0xffffffffu, at, src)) * PASS_TOKENS;
+            return;
+        }
         const int stride = (na + 31) >> 5;                                         // first round: every stride-th entry
         const int i1 = min(lane * stride, na - 1);
         const unsigned m1 = __ballot_sync(0xffffffffu, lane * stride < na && passes[i1] <= w);
@@ -301,12 +335,12 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
         uint32_t idx = 0;
         bool first_staged = false;                         // the first segment's rows are asked for right after its first weight copies
 #pragma unroll 1
-        for (long long u = u_begin; u < u_end && ok; u += r1 - r0, ++idx) {
+        for (Job u = u_begin; u < u_end && ok; u += r1 - r0, ++idx) {
             segment(u, pass, r0, r1);
             int e, c0;
             locate(pass, e, c0);
             const bool shared = e == p.experts;
-            const long long u_next = u + (r1 - r0);
+            const Job u_next = u + (r1 - r0);
             int npass = 0, nr0, nr1;
             if (u_next < u_end) segment(u_next, npass, nr0, nr1);
             bool next_staged = p.nbuf != 2 || u_next >= u_end;
@@ -390,7 +424,7 @@ __global__ void __launch_bounds__(bound_threads<STAGER>(), 1) dec4_k(const Dec4A
         int pass, r0, r1;
         uint32_t idx = 0;
 #pragma unroll 1
-        for (long long u = u_begin; u < u_end && alive; u += r1 - r0, ++idx) {
+        for (Job u = u_begin; u < u_end && alive; u += r1 - r0, ++idx) {
             segment(u, pass, r0, r1);
             const uint32_t b = p.nbuf == 2 ? (idx & 1u) : 0u, use = p.nbuf == 2 ? idx >> 1 : idx;
             if (*abort_flag) break;
@@ -588,7 +622,7 @@ int g_drop_tile = -1;                 // test hooks (b2moe_harness_wait_probe, b
 bool g_skip_stage = false;
 uint32_t g_wait_limit = WAIT_LIMIT;
 
-template <uint32_t T, int MODE, bool STAGER = false>
+template <uint32_t T, int MODE, bool FEW>
 int32_t launch_dec4(Dec4Args a, cudaStream_t s) {
     const int sms = sm_count(), k = a.k_tiles * 256;
     if (sms <= 0) return B2MOE_ERR_CUDA;
@@ -603,12 +637,15 @@ int32_t launch_dec4(Dec4Args a, cudaStream_t s) {
         if (per_block <= CTA_WARPS / ks && kslots % ks == 0 && g_ksplit_max >= ks &&
             dec4_smem<T>(k, a.nbuf, a.stages, a.slot_tiles) + RED_BYTES <= SMEM_LIMIT) { a.ksplit = ks; break; }
     const size_t smem = dec4_smem<T>(k, a.nbuf, a.stages, a.slot_tiles) + (a.ksplit > 1 ? RED_BYTES : 0);
-    if (cudaFuncSetAttribute(dec4_k<T, MODE, STAGER>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return B2MOE_ERR_CUDA;
+    if (cudaFuncSetAttribute(dec4_k<T, MODE, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return B2MOE_ERR_CUDA;
     a.wait_limit = g_wait_limit;
     a.drop_tile = g_drop_tile;
-    launch_overlapped(dec4_k<T, MODE, STAGER>, dim3(sms), dim3(threads_of<STAGER>()), smem, s, a);       // every block takes an equal share of the (pass, row tile) jobs
+    launch_overlapped(dec4_k<T, MODE, FEW>, dim3(sms), dim3(threads_of<FEW && MODE == 1>()), smem, s, a);       // every block takes an equal share of the (pass, row tile) jobs
     return launch_status();
 }
+
+// up to 24 jobs per block, from the call's shape
+bool few_jobs(int passes_bound, int rows) { const int sms = sm_count(); return sms > 0 && (long long)passes_bound * ((rows + 15) / 16) <= 24LL * sms; }
 
 template <uint32_t T>
 int32_t stage(Dec4Args & a, const void * x, int dtype, int rows_x, int k, void * ws, cudaStream_t s, bool already = false) {
@@ -633,7 +670,7 @@ int32_t gateup_t(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_ban
     a.plan = const_cast<int *>(plan); a.out = act; a.out_dtype = act_dtype;
     a.rows = gate->rows; a.k_tiles = k / 256; a.experts = gate->experts; a.topk = topk; a.A = n * topk;
     a.passes_bound = n * topk + (shared_tokens + PASS_TOKENS - 1) / PASS_TOKENS;
-    return launch_dec4<T, 0>(a, s);
+    return few_jobs(a.passes_bound, a.rows) ? launch_dec4<T, 0, true>(a, s) : launch_dec4<T, 0, false>(a, s);
 }
 template <uint32_t T>
 int32_t down_t(const b2moe_bank * down, const b2moe_bank * sd, const void * x, int x_dtype, bool per_token, const int * plan, int n, int topk,
@@ -643,9 +680,7 @@ int32_t down_t(const b2moe_bank * down, const b2moe_bank * sd, const void * x, i
     // A launch of a few jobs per block is a chain of latencies: its rows are staged inside the kernel by a warp of their own
     // (one launch less). A full launch keeps the staging kernel: measured at 64 tokens the in-kernel staging costs 11 us more
     // than the launch it saves (the staging warp shares a scheduler with five busy warps).
-    const long long jobs_bound = (long long)(n * topk + (shared_tokens + PASS_TOKENS - 1) / PASS_TOKENS) * ((down->rows + 15) / 16);
-    const int sms = sm_count();
-    const bool in_kernel = sms > 0 && jobs_bound <= 24LL * sms && !g_skip_stage && x_dtype == B2MOE_F32 && !per_token;
+    const bool few = few_jobs(n * topk + (shared_tokens + PASS_TOKENS - 1) / PASS_TOKENS, down->rows), in_kernel = few && !g_skip_stage && x_dtype == B2MOE_F32 && !per_token;
     a.x_per_token = per_token;
     if (in_kernel) a.x_raw = static_cast<const float *>(x);
     else if (int32_t rc = stage<T>(a, x, x_dtype, rows_x, k, ws, s)) return rc;
@@ -655,7 +690,7 @@ int32_t down_t(const b2moe_bank * down, const b2moe_bank * sd, const void * x, i
     a.plan = const_cast<int *>(plan); a.out = y; a.out_dtype = y_dtype;
     a.rows = down->rows; a.k_tiles = k / 256; a.experts = down->experts; a.topk = topk; a.A = n * topk;
     a.passes_bound = n * topk + (shared_tokens + PASS_TOKENS - 1) / PASS_TOKENS;
-    return in_kernel ? launch_dec4<T, 1, true>(a, s) : launch_dec4<T, 1>(a, s);
+    return in_kernel ? launch_dec4<T, 1, true>(a, s) : launch_dec4<T, 1, false>(a, s);
 }
 
 }  // namespace
