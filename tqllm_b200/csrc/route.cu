@@ -6,8 +6,6 @@
 #include <cooperative_groups.h>
 #include <math_constants.h>
 
-#include <type_traits>
-
 #include "common.cuh"
 #include "dec4_stage.cuh"
 #include "dispatch.cuh"
@@ -493,59 +491,25 @@ __device__ __forceinline__ void route_token_regs(const float * logits, int ld, c
             key[r] = in ? ordered_bits(bias ? p[r] + bias[lane + 32 * r] : p[r]) : 0u;
         }
     }
-    // Lane q keeps the q-th selection (k <= 32 on this path): one coalesced store of ids and weights at the end instead of a
-    // store per round and a read-modify-write pass of lane 0 over global memory. A round takes a lane's best over groups of four
-    // keys, of which only the group that lost one is searched again (the same group in every lane); the probabilities are taken
-    // back from the keys, or from the logits where a bias is in the keys, after the rounds. One search over all keys and a pick
-    // of the probability in every round: twice the time (512 experts, ten rounds: 4 thousand cycles of the routing launch)
-    constexpr int G = R / 4;
-    uint32_t gk[G];                                                    // the groups' best keys and their places: ascending places, the lowest keeps a tie
-    int gr[G];
-    auto search = [&](auto C) {
-        constexpr int g = decltype(C)::value;
-        const bool b1 = key[4 * g + 1] > key[4 * g], b3 = key[4 * g + 3] > key[4 * g + 2];
-        const uint32_t v1 = b1 ? key[4 * g + 1] : key[4 * g], v3 = b3 ? key[4 * g + 3] : key[4 * g + 2];
-        gk[g] = v3 > v1 ? v3 : v1;
-        gr[g] = 4 * g + (v3 > v1 ? (b3 ? 3 : 2) : (b1 ? 1 : 0));
-    };
-    auto groups = [&](auto what) {
-        what(std::integral_constant<int, 0>{});
-        if constexpr (G > 1) what(std::integral_constant<int, 1>{});
-        if constexpr (G > 2) { what(std::integral_constant<int, 2>{}); what(std::integral_constant<int, 3>{}); }
-    };
-    static_assert(G == 1 || G == 2 || G == 4, "groups of four keys");
-    groups(search);
-    uint32_t my_key = 0;
+    // lane q keeps the q-th selection (k <= 32 on this path): one coalesced store of ids and weights at the end instead of a
+    // store per round and a read-modify-write pass of lane 0 over global memory
+    float sel_sum = 0.f, my_p = 0.f;
     int my_idx = 0;
-#pragma unroll 1
     for (int q = 0; q < k; ++q) {
-        uint32_t best = gk[0];
-        int br = gr[0];
-        if constexpr (G == 2) { if (gk[1] > best) { best = gk[1]; br = gr[1]; } }
-        if constexpr (G == 4) {
-            const bool b1 = gk[1] > gk[0], b3 = gk[3] > gk[2];
-            const uint32_t v1 = b1 ? gk[1] : gk[0], v3 = b3 ? gk[3] : gk[2];
-            best = v3 > v1 ? v3 : v1;
-            br = v3 > v1 ? (b3 ? gr[3] : gr[2]) : (b1 ? gr[1] : gr[0]);
-        }
+        uint32_t best = 0;
+        int br = 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) if (key[r] > best) { best = key[r]; br = r; }     // ascending r: the lowest index keeps a tie
         const uint32_t top = __reduce_max_sync(0xffffffffu, best);
         const int idx = int(__reduce_min_sync(0xffffffffu, (best == top && best != 0u) ? uint32_t(lane + 32 * br) : 0x7fffffffu));
-        if (lane == q) { my_idx = idx == 0x7fffffff ? 0 : idx; my_key = top; }
-        if (idx == 0x7fffffff) continue;                               // no key is left
-        const int orow = idx >> 5;
-        const bool mine = lane == (idx & 31);
-        groups([&](auto C) {
-            constexpr int g = decltype(C)::value;
-            if ((orow >> 2) != g) return;
+        const int owner = idx & 31, orow = idx >> 5;
+        float pv = 0.f;
 #pragma unroll
-            for (int r = 0; r < 4; ++r) if (mine && (orow & 3) == r) key[4 * g + r] = 0u;
-            search(C);
-        });
+        for (int r = 0; r < R; ++r) if (r == orow) { pv = p[r]; if (lane == owner) key[r] = 0u; }
+        pv = __shfl_sync(0xffffffffu, pv, owner);
+        if (lane == q) { my_idx = idx == 0x7fffffff ? 0 : idx; my_p = pv; }
+        sel_sum += pv;
     }
-    float my_p = my_key == 0u ? 0.f : __uint_as_float(my_key & 0x80000000u ? my_key & 0x7fffffffu : ~my_key);
-    if (GATING == B2MOE_SIGMOID && lane < k && my_key != 0u) my_p = 1.f / (1.f + expf(-x[my_idx]));
-    float sel_sum = 0.f;                                               // in the order of the selections
-    for (int q = 0; q < k; ++q) sel_sum += __shfl_sync(0xffffffffu, my_p, q);
     if (lane < k) {
         float w = my_p;
         if (norm) w = w / fmaxf(sel_sum, 6.103515625e-5f);
@@ -669,34 +633,25 @@ __global__ void __launch_bounds__(RD_THREADS) route_dispatch_k(const float * log
 // alone. One launch instead of three (top-k, dispatch, staging) on the critical path of a decode-sized layer call.
 constexpr int RC_BLOCKS = 8;
 struct StageJob { const void * x; int dtype, k, bits; uint8_t * rows; float * inv_scale; };     // x = nullptr: nothing to stage
-// ALONE: up to ROUTE_ALONE tokens: block 0 routes them all, on a warp each, the other blocks stage rows meanwhile and nobody waits for
-// another block (the cluster's barrier, 0.7 us; one token 36.8 -> 35.8 us per layer, eight 73.2 -> 72.0); more would queue for the block's schedulers.
-constexpr int ROUTE_ALONE = 8;
-template <int GATING, bool ALONE>
+template <int GATING>
 __global__ void __launch_bounds__(RD_THREADS) route_cluster_k(const float * logits, int ld, const float * __restrict__ bias,
                                                         int * __restrict__ ids, float * __restrict__ weights,
                                                         float * __restrict__ shared_weights, int e, int k, int norm, float scale, int n,
                                                         int shared_first, int shared_count, int * __restrict__ plan, const StageJob st) {
     extern __shared__ float smem[];
     namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int rank = int(blockIdx.x), nb = int(gridDim.x);            // the grid is one cluster (ALONE: no cluster)
+    const int rank = int(cluster.block_rank()), nb = int(cluster.num_blocks());
     float * p = smem + size_t(warp) * 2 * e;
     grid_release();
     grid_wait();
-    if constexpr (ALONE) {
-        if (rank == 0) {
-            if (warp < n) route_token<GATING>(logits, ld, bias, ids, weights, shared_weights, e, k, norm, scale, warp, lane, p, p + e);
-            __syncthreads();                      // the ids are written and the routing scratch is dead
-        }
-    } else {
-        for (int token = rank + nb * warp; token < n; token += nb * (RD_THREADS / 32)) {
-            route_token<GATING>(logits, ld, bias, ids, weights, shared_weights, e, k, norm, scale, token, lane, p, p + e);
-            __syncwarp();
-        }
-        __threadfence();
-        cg::this_cluster().sync();                // every block's ids are written and visible
+    for (int token = rank + nb * warp; token < n; token += nb * (RD_THREADS / 32)) {
+        route_token<GATING>(logits, ld, bias, ids, weights, shared_weights, e, k, norm, scale, token, lane, p, p + e);
+        __syncwarp();
     }
+    __threadfence();
+    cluster.sync();                               // every block's ids are written and visible
     if (rank == 0) {
         dispatch_small_body<false>(ids, n * k, e, shared_first, shared_count, plan, reinterpret_cast<unsigned short *>(smem));
     } else if (st.x) {
@@ -736,19 +691,21 @@ int32_t route_plan_stage(int gating, const float * logits, int ld, const float *
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = g_overlap;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = RC_BLOCKS; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = RC_BLOCKS; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    const bool alone = n <= ROUTE_ALONE;
-    cfg.numAttrs = alone ? 1 : 2;
-    const bool softmax = gating == B2MOE_SOFTMAX;
-    auto kernel = softmax ? (alone ? route_cluster_k<B2MOE_SOFTMAX, true> : route_cluster_k<B2MOE_SOFTMAX, false>)
-                          : (alone ? route_cluster_k<B2MOE_SIGMOID, true> : route_cluster_k<B2MOE_SIGMOID, false>);
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return B2MOE_ERR_CUDA;
-    cudaLaunchKernelEx(&cfg, kernel, logits, ld, softmax ? (const float *)nullptr : bias, ids, weights, softmax ? shared_weights : (float *)nullptr, experts, topk,
-                       softmax ? 1 : norm, scale, n, shared_first, shared_count, plan, st);
+    cfg.numAttrs = g_overlap ? 2 : 1;
+    if (gating == B2MOE_SOFTMAX) {
+        if (cudaFuncSetAttribute(route_cluster_k<B2MOE_SOFTMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return B2MOE_ERR_CUDA;
+        cudaLaunchKernelEx(&cfg, route_cluster_k<B2MOE_SOFTMAX>, logits, ld, (const float *)nullptr, ids, weights, shared_weights, experts, topk, 1, scale, n,
+                           shared_first, shared_count, plan, st);
+    } else {
+        if (cudaFuncSetAttribute(route_cluster_k<B2MOE_SIGMOID>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return B2MOE_ERR_CUDA;
+        cudaLaunchKernelEx(&cfg, route_cluster_k<B2MOE_SIGMOID>, logits, ld, bias, ids, weights, (float *)nullptr, experts, topk, norm, scale, n,
+                           shared_first, shared_count, plan, st);
+    }
     *took = true;
     return launch_status();
 }
