@@ -91,8 +91,9 @@ __device__ __forceinline__ int3 block_scan(int3 v, int used, int3 * w, int3 & to
 // the block, each with a contiguous span of the experts (one warp for all of them was a chain of e1 / 32 dependent steps, three times
 // over: 2 us of dispatch_place_k at 512 experts). The pass list runs over the active experts from the last (the shared expert, the heaviest) to the
 // first, cut into passes of PASS_TOKENS tokens: passes[i] = passes before the i-th expert of that order = all of them but those up to
-// that expert, so tokens, experts and passes take one scan and one barrier together (a scan for the passes alone, behind the list that it read, was half of
-// the 3.6 to 8 thousand cycles that this took in a routing launch). cs and os are shared-memory copies, or the plan's own arrays.
+// that expert, so tokens, experts and passes take one scan and one barrier together. (Two scans, the second behind
+// the list that it read, took 3.6 to 8 thousand cycles of a routing launch. The loops are rolled: the code runs once a launch, and with unrolled ones its fetch
+// took longer than the scan: 2.4 to 3 us against 1.3 at 8 to 64 tokens.) cs and os are shared-memory copies, or the plan's own arrays.
 // The caller synchronises before (cs) and after (os).
 __device__ inline void finish_plan(int * plan, const int * cs, int * os, int * offsets, int * active, int * passes, int e1, bool write) {
     __shared__ int3 wsum[32];

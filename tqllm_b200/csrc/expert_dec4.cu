@@ -244,8 +244,8 @@ __global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(c
         u_begin = q * int(blockIdx.x) + r * int(blockIdx.x) / blocks;
         u_end = q * int(blockIdx.x + 1) + r * int(blockIdx.x + 1) / blocks;
         // Few passes: every pass on blocks of its own, where a block's share is then still one round of JW jobs. A share that runs into a
-        // second pass waits for that one's plan entries, activation rows and products in turn: one token of 512 IQ3_S experts, gate/up 9.2 us where 6.6
-        // do. Larger shares hide that behind their rounds, and whole passes leave them uneven (8 tokens, 75 passes: 73.5 us a layer with equal shares, 80).
+        // second pass waits for that one's plan entries, activation rows and products in turn: one token of 512 IQ3_S experts, gate/up: done after 9.2 us, blocks with one
+        // pass after 6.6. Larger shares hide that behind their rounds, and whole passes leave them uneven (8 tokens, 75 passes: 73.5 us a layer with equal shares, 80).
         const int per_pass = blocks / max(n_pass, 1);
         if (per_pass > 0 && (row_tiles + per_pass - 1) / per_pass <= JW) {
             const int pass = int(blockIdx.x) / per_pass, part = int(blockIdx.x) - pass * per_pass;

@@ -74,9 +74,9 @@ int decode_kernel(uint32_t type, int k, int dtype) {
 // fewer than GEMM_MIN_PER assignments per expert or the bank has fewer than GEMM_MIN_EXPERTS experts, everything else the GEMM. The line is one
 // of precision as much as of time: the decode kernels take the weights as they are and 15-bit activations, the GEMM rounds both to 11 bits. Relative error against
 // 64-bit sums (2-norm), decode / GEMM, at any density: Q4_K act 2.5e-5 / 4.0e-4, down of it 2.0e-4 / 5.3e-4; IQ3_S codes 2.5e-5 / 3.0e-4
-// and 2.0e-4 / 4.2e-4; IQ3_S in GGUF fields 2e-7 / 3.0e-4 and 2.1e-4 / 4.2e-4. The GEMM is the faster one from about 16 per
-// expert on (layer times, decode / GEMM, us: Q4_K of 256 experts at 19 per expert 1139 / 1027, of 60 at 30 249 / 184; IQ3_S codes of 512 at
-// 16 564 / 550), but nothing below this line asked for fewer bits. b2moe_harness_select forces a family where it supports the shape
+// and 2.0e-4 / 4.2e-4; IQ3_S in GGUF fields 2e-7 / 3.0e-4 and 2.1e-4 / 4.2e-4. The GEMM is the faster one from about 20 per
+// expert on (layer times, decode family / GEMM, us: IQ3_S codes of 512 experts at 20 per expert 416 / 412, Q4_K of 256 at 31 1116 / 879, of 60 at 100
+// 315 / 169), but nothing below this line asked for fewer bits. b2moe_harness_select forces a family where it supports the shape
 // (tests and benchmarks).
 constexpr int GEMM_MIN_PER = 32, GEMM_MIN_EXPERTS = 128;
 int g_family = B2MOE_FAMILY_AUTO;
