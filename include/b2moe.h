@@ -405,7 +405,7 @@ typedef struct b2moe_layer_ws {
     size_t y;              /* f32 [n*topk + shared][hidden] */
     size_t scratch;        /* dispatch scratch */
     size_t expert_scratch; /* scratch of the expert products */
-    size_t total;          /* workspace bytes needed */
+    size_t total;          /* workspace bytes to provide: they grow with n, and a workspace for the largest batch gives every smaller one the same results as its own */
 } b2moe_layer_ws;
 B2MOE_API int32_t b2moe_layer_workspace(const b2moe_layer * layer, int32_t n, b2moe_layer_ws * ws);
 B2MOE_API int32_t b2moe_layer_forward(const b2moe_layer * layer, const void * x, int32_t x_dtype, int32_t n, void * out,

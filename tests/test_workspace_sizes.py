@@ -26,3 +26,20 @@ def test_product_scratch(type_id, experts, rows, cols, topk):
                  lambda n: lib.b2moe_expert_workspace_bytes(type_id, n, cols, capi.BF16)):
         sizes = [size(a // topk + 1) for a in EDGES]
         assert sizes == sorted(sizes) and sizes[0] > 0
+
+
+@pytest.mark.parametrize("gate,down,experts,topk,hidden,ff,shared", ((12, 12, 256, 8, 3072, 1536, 0), (0x1015, 0x1015, 512, 10, 2048, 512, 1), (12, 20, 128, 4, 1024, 512, 0),
+                                                                     (12, 12, 60, 6, 2560, 768, 0), (12, 20, 48, 32, 4096, 64, 1), (323, 323, 512, 10, 2048, 512, 1)))
+def test_layer_workspace(gate, down, experts, topk, hidden, ff, shared):
+    """every batch up to past the lines of nine and 32 assignments per expert; where the exact form serves the down product its rows of two fp16 terms are in it"""
+    L = capi.Layer(hidden=hidden, experts=experts, topk=topk, ff=ff, has_shared=shared)
+    L.gate = L.up = capi.Bank(16, None, gate, experts, ff, hidden)
+    L.down = capi.Bank(16, None, down, experts, hidden, ff)
+    before = 0
+    for n in range(1, 40 * experts // topk):
+        v = capi.LayerWs()
+        capi.check(lib.b2moe_layer_workspace(C.byref(L), n, C.byref(v)), "b2moe_layer_workspace")
+        assert v.total >= before, n
+        before = v.total
+        if down in (12, 0x1015) and 9 * experts <= n * topk < (32 * experts if experts >= 128 else 1 << 30):
+            assert v.total - v.expert_scratch >= n * (topk + shared) * (4 * ff + ff // 8 + 4)

@@ -304,12 +304,27 @@ static int32_t layer_layout(const b2moe_layer * L, int32_t n, b2moe_layer_ws * w
     ws->total = at;
     return B2MOE_OK;
 }
-// The caller is asked for what the exact form of the down product takes where it would be chosen; layer_forward needs no more than layer_layout says
+// The end of what layer_forward uses where it takes the exact form: gate/up's rows from y on, the down product's in the expert scratch
+static size_t layer_exact_end(const b2moe_layer * L, int32_t n, const b2moe_layer_ws & ws) {
+    const long long live = (long long)n * L->topk;
+    const int At = n * L->topk + (L->has_shared ? n : 0);
+    size_t end = 0;
+    if (exact_path(L->gate.type, L->hidden, B2MOE_F32, L->experts, live, B2MOE_FAMILY_AUTO)) end = ws.y + align_up(gemm_exact_bytes(At, L->hidden, B2MOE_F32), 256);
+    if (exact_path(L->down.type, L->ff, B2MOE_F32, L->experts, live, B2MOE_FAMILY_AUTO)) end = std::max(end, ws.expert_scratch + align_up(gemm_exact_bytes(At, L->ff, B2MOE_F32), 256));
+    return end;
+}
+// The caller is asked for what the exact form takes (layer_forward itself needs no more than layer_layout says), and for no less above the
+// line from which the other form serves the call: the size grows with n, so that an arena for the largest batch gives every smaller one
+// the kernels, and the bits, that an arena of its own would.
 extern "C" B2MOE_API int32_t b2moe_layer_workspace(const b2moe_layer * L, int32_t n, b2moe_layer_ws * ws) {
     if (int32_t rc = layer_layout(L, n, ws)) return rc;
-    const int At = n * L->topk + (L->has_shared ? n : 0);
-    const size_t exact = gemm_exact_bytes(At, L->ff, B2MOE_F32);
-    if (exact_path(L->down.type, L->ff, B2MOE_F32, L->experts, (long long)n * L->topk, B2MOE_FAMILY_AUTO)) ws->total = std::max(ws->total, ws->expert_scratch + align_up(exact, 256));
+    ws->total = std::max(ws->total, layer_exact_end(L, n, *ws));
+    const long long below = ((long long)GEMM_MIN_PER * L->experts - 1) / L->topk;          // the last batch below that line
+    if (n > below) {
+        b2moe_layer_ws w;
+        if (int32_t rc = layer_layout(L, int32_t(below), &w)) return rc;
+        ws->total = std::max(ws->total, layer_exact_end(L, int32_t(below), w));
+    }
     return B2MOE_OK;
 }
 
