@@ -336,8 +336,8 @@ def expert_products(torch, moe, lib, C, lay, x, shape, stream):
     XDT = {torch.bfloat16: 2, torch.float16: 1, torch.float32: 0}[x.dtype]
     act = torch.zeros(A + ST, shape.ff, dtype=torch.float32, device=x.device)
     y = torch.zeros(A + ST, shape.hidden, dtype=torch.float32, device=x.device)
-    gws = torch.empty(max(lib.b2moe_expert_workspace_bytes(lay.gate.type, A + ST, shape.hidden, XDT) + 4 * (A + ST), 16), dtype=torch.uint8, device=x.device)
-    dws = torch.empty(max(lib.b2moe_expert_workspace_bytes(lay.down.type, A + ST, shape.ff, 0), 16), dtype=torch.uint8, device=x.device)
+    gws = torch.empty(max(lib.b2moe_expert_slot_workspace_bytes(C.byref(lay.gate.c), A + ST, XDT), 16), dtype=torch.uint8, device=x.device)
+    dws = torch.empty(max(lib.b2moe_expert_slot_workspace_bytes(C.byref(lay.down.c), A + ST, 0), 16), dtype=torch.uint8, device=x.device)
     shp = lambda i: C.byref(lay.sh[i].c) if shape.shared else None
     st = stream.cuda_stream
 

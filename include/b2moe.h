@@ -160,9 +160,14 @@ B2MOE_API int32_t b2moe_plan_to_groups(const int32_t * plan, int32_t n, int32_t 
  * Scratch: the tensor-core kernels first bring the activation rows into operand form (one fp16 term per value, the row
  * scaled by a power of two, + that scale) inside a caller-provided workspace of b2moe_expert_workspace_bytes(type, rows_x, k, x_dtype) bytes (16-byte aligned), where
  * rows_x = n for the gate/up product (k = hidden) and n*topk + shared_tokens for the down product (k = ff, x_dtype
- * B2MOE_F32). The workspace may be NULL only where the size is 0. Gate/up calls of many tokens per
- * expert are faster (up to one and a half times) with a larger one: that of rows_x = n*topk + shared_tokens rows and 4 bytes more for each of them. */
+ * B2MOE_F32). The workspace may be NULL only where the size is 0.
+ * That size is what the products accept. b2moe_expert_slot_workspace_bytes(bank, rows, x_dtype), with rows = n*topk + shared_tokens for
+ * either product, is the size from which they choose among all their forms, which a larger one does not change any more: gate/up calls of
+ * many tokens per expert are up to one and a half times as fast (their rows lie in slot order), and banks of 4-bit codes (Q4_K, B2MOE_IQ3_S_X4) at nine and
+ * more assignments per expert reach the form that b2moe_layer_forward uses there (fp32 rows as two fp16 terms, relative error 1e-6
+ * instead of 2e-4). Both sizes grow with the rows. */
 B2MOE_API size_t b2moe_expert_workspace_bytes(uint32_t type, int32_t rows_x, int32_t k, int32_t x_dtype);
+B2MOE_API size_t b2moe_expert_slot_workspace_bytes(const b2moe_bank * bank, int32_t slot_rows, int32_t x_dtype);
 /* act[a][f] = silu(gate_e(a)[f] . x[token(a)]) * (up_e(a)[f] . x[token(a)]) for every grouped assignment a: the
  * paired gate/up product with the SwiGLU fused (replaces expert_matvec2 / expert_matvec_dedup2 / expert_gemm_gateup +
  * moe_swiglu: src/formats/weight/weight_format.hpp:58-73, src/formats/weight/quant.cu:167-233,384-405,
@@ -198,7 +203,8 @@ B2MOE_API int32_t b2moe_expert_down_sparse(const b2moe_bank * down, const b2moe_
  * all calls on a device share the array, so calls that overlap on the GPU (different streams) race on it. The first
  * call on each device looks the array's device address up (with that device current) and should come before any
  * stream capture; later calls only launch (the cached address does not survive a cudaDeviceReset). A call that
- * resolves to the format-generic kernels uses no scratch and is not limited. Results are those of b2moe_expert_down. */
+ * resolves to the format-generic kernels uses no scratch and is not limited. Results are those of b2moe_expert_down with the array as its
+ * workspace: those of the larger size above while it fits the array. */
 #define B2MOE_STATIC_SCRATCH_BYTES (16u << 20)
 B2MOE_API size_t b2moe_static_scratch_bytes(void);
 B2MOE_API int32_t b2moe_expert_down_static(const b2moe_bank * down, const b2moe_bank * shared_down, const float * act,

@@ -104,3 +104,24 @@ def test_where_it_begins_and_small_workspaces():
             dev.forward(x)
             art = dev.artefacts()
             assert err(art["act"], act) < TOL and 1e-5 < err(art["y"], y) < 1e-3
+
+
+@pytest.mark.parametrize("dtype", (torch.bfloat16, torch.float32), ids=("bf16", "f32"))
+@pytest.mark.parametrize("types", ((Q4_K,) * 3, (IQ3_S,) * 3), ids=("q4k", "iq3s"))
+def test_plan_driven_products(types, dtype):
+    """the products over a ready plan, with skipped ids and a shared expert, in scratch of the size with a row per assignment: this form for both"""
+    from tqllm_b200 import moe
+    n, experts, topk = 130, 12, 3
+    dev = moe.MoeLayer.from_synth(synth.make_layer(synth.LayerShape("plan", 768, experts, topk, 512, shared=True, types=types), 6, "cuda"))
+    g = torch.Generator().manual_seed(3)
+    ids = torch.rand(n, experts, generator=g).argsort(1)[:, :topk].to(torch.int32)
+    ids[torch.rand(n, topk, generator=g) < 0.3] = -1
+    ids = ids.cuda()
+    x = torch.randn(n, 768, generator=g).cuda().to(dtype)
+    plan = moe.dispatch(ids, experts, n)
+    act = moe.expert_gateup_swiglu(dev.gate, dev.up, x, plan, dev.sh[0], dev.sh[1])
+    y = moe.expert_down(dev.down, act, plan, dev.sh[2])
+    want = products(dev, x, ids.long(), True)
+    assert int(plan.buf[3]) == 0 and err(act, want[0]) < TOL and err(y, want[1]) < TOL
+    skipped = (ids.reshape(-1) < 0).nonzero().flatten()
+    assert len(skipped) > 50 and not act[skipped].any() and not y[skipped].any()

@@ -23,9 +23,24 @@ def test_product_scratch(type_id, experts, rows, cols, topk):
     bank = capi.Bank(16, None, type_id, experts, rows, cols)
     for size in (lambda n: lib.b2moe_expert_matvec_workspace_bytes(C.byref(bank), n, topk),
                  lambda n: lib.b2moe_expert_gemm_gateup_workspace_bytes(C.byref(bank), n, topk, capi.F16),
-                 lambda n: lib.b2moe_expert_workspace_bytes(type_id, n, cols, capi.BF16)):
+                 lambda n: lib.b2moe_expert_workspace_bytes(type_id, n, cols, capi.BF16),
+                 lambda n: lib.b2moe_expert_slot_workspace_bytes(C.byref(bank), n, capi.F32)):
         sizes = [size(a // topk + 1) for a in EDGES]
         assert sizes == sorted(sizes) and sizes[0] > 0
+
+
+def test_product_scratch_with_a_row_per_assignment():
+    """never below the size that the products accept; for banks of 4-bit codes fp32 rows as two fp16 terms with their sub-block sums and a scale fit"""
+    for type_id in (12, 20, 21, 23, 323, 0x1015):
+        bank = capi.Bank(16, None, type_id, 60, 512, 1024)
+        for dt in (capi.F32, capi.F16, capi.BF16):
+            for rows in (1, 7, 600, 5000):
+                size = lib.b2moe_expert_slot_workspace_bytes(C.byref(bank), rows, dt)
+                assert size >= lib.b2moe_expert_workspace_bytes(type_id, rows, 1024, dt)
+                if type_id in (12, 0x1015):
+                    assert size >= rows * (1024 * (4 if dt == capi.F32 else 2) + 128 + 4)
+    assert lib.b2moe_expert_slot_workspace_bytes(None, 4, 0) == 0 and lib.b2moe_expert_slot_workspace_bytes(C.byref(bank), 0, 0) == 0
+    assert lib.b2moe_expert_slot_workspace_bytes(C.byref(bank), 4, 7) == 0
 
 
 @pytest.mark.parametrize("gate,down,experts,topk,hidden,ff,shared", ((12, 12, 256, 8, 3072, 1536, 0), (0x1015, 0x1015, 512, 10, 2048, 512, 1), (12, 20, 128, 4, 1024, 512, 0),

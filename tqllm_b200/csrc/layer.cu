@@ -181,6 +181,12 @@ extern "C" B2MOE_API size_t b2moe_expert_workspace_bytes(uint32_t type, int32_t 
     const size_t g = gemm_tc_workspace_bytes(rows_x, k);
     return g > need ? g : need;
 }
+extern "C" B2MOE_API size_t b2moe_expert_slot_workspace_bytes(const b2moe_bank * bank, int32_t slot_rows, int32_t x_dtype) {
+    const size_t base = bank ? b2moe_expert_workspace_bytes(bank->type, slot_rows, bank->cols, x_dtype) : 0;
+    if (!base) return 0;
+    const bool exact = dec4_supported(bank->type, bank->cols) && gemm_exact_supported(bank->type, bank->cols, bank->experts);
+    return std::max({base, gemm_tc_slot_bytes(slot_rows, bank->cols), exact ? gemm_exact_bytes(slot_rows, bank->cols, x_dtype) : size_t(0)});
+}
 
 // x_staged: the caller has already written the staged form of x where the 4-bit decode kernels expect it (b2moe_layer_forward);
 // rows_buf: scratch the caller has to spare for the grouped GEMM's activation rows in slot order (null: it gathers them)

@@ -73,5 +73,5 @@ extern "C" B2MOE_API int32_t b2moe_expert_down_static(const b2moe_bank * down, c
     if (need) {
         if (int32_t rc = static_scratch(&scratch)) return rc;
     }
-    return b2moe_expert_down(down, shared_down, act, plan, n, topk, shared_tokens, y, scratch, need, stream);      // no more than that call asks for: the same kernels
+    return b2moe_expert_down(down, shared_down, act, plan, n, topk, shared_tokens, y, scratch, need ? B2MOE_STATIC_SCRATCH_BYTES : 0, stream);
 }

@@ -416,13 +416,14 @@ class CudaEpLayer:
         act = self._b("act", (A + shared_n, sh.ff), torch.float32)
         y = self._b("y", (A + shared_n, sh.hidden), torch.float32)
         dt = moe._DT[x_all.dtype]
-        eg = lib.b2moe_expert_workspace_bytes(L.gate.type, N, sh.hidden, dt)
-        ed = lib.b2moe_expert_workspace_bytes(L.down.type, A + shared_n, sh.ff, self.capi.F32)
-        ews = self._b("ews", (max(eg, ed, 16),), torch.uint8)
         br = lambda b: C.byref(b.c)
-        shg, shu, shd = (br(L.sh[0]), br(L.sh[1]), br(L.sh[2])) if has_sh else (None, None, None)
-        # y is written by the down product: until then its memory is the gate/up product's workspace, with a row per assignment
+        # sizes with a row per assignment: the forms of the products that an unsplit layer call takes. y is written by the down product:
+        # until then its memory is the gate/up product's workspace where it is large enough
+        eg = lib.b2moe_expert_slot_workspace_bytes(br(L.gate), A + shared_n, dt)
+        ed = lib.b2moe_expert_slot_workspace_bytes(br(L.down), A + shared_n, self.capi.F32)
+        ews = self._b("ews", (max(ed, 0 if y.nbytes >= eg else eg, 16),), torch.uint8)
         gws = y if y.nbytes >= eg else ews
+        shg, shu, shd = (br(L.sh[0]), br(L.sh[1]), br(L.sh[2])) if has_sh else (None, None, None)
         live = self.live_estimate(N * k)                 # this rank owns count / experts_total of the experts: so many ids are not -1
         self.capi.check(lib.b2moe_expert_gateup_swiglu_sparse(br(L.gate), br(L.up), shg, shu, x_all.data_ptr(), dt, plan.data_ptr(), N, k,
                                                               shared_n, live, act.data_ptr(), gws.data_ptr(), gws.nbytes, self._st()), "gateup")
@@ -483,12 +484,12 @@ class CudaEpLayer:
         act = torch.empty(A + shared_n, sh.ff, dtype=torch.float32, device=recv.device)
         y = torch.empty(A + shared_n, H, dtype=torch.float32, device=recv.device)
         dt = moe._DT[x_dtype]
-        eg = lib.b2moe_expert_workspace_bytes(L.gate.type, N, H, dt)
-        ed = lib.b2moe_expert_workspace_bytes(L.down.type, A + shared_n, sh.ff, self.capi.F32)
-        ews = torch.empty(max(eg, ed, 16), dtype=torch.uint8, device=recv.device)
         br = lambda b: C.byref(b.c)
+        eg = lib.b2moe_expert_slot_workspace_bytes(br(L.gate), A + shared_n, dt)               # as above
+        ed = lib.b2moe_expert_slot_workspace_bytes(br(L.down), A + shared_n, self.capi.F32)
+        ews = torch.empty(max(ed, 0 if y.nbytes >= eg else eg, 16), dtype=torch.uint8, device=recv.device)
+        gws = y if y.nbytes >= eg else ews
         shg, shu, shd = (br(L.sh[0]), br(L.sh[1]), br(L.sh[2])) if has_sh else (None, None, None)
-        gws = y if y.nbytes >= eg else ews                 # as above
         live = self.live_estimate(N * k)
         self.capi.check(lib.b2moe_expert_gateup_swiglu_sparse(br(L.gate), br(L.up), shg, shu, x.data_ptr(), dt, plan.data_ptr(), N, k, shared_n,
                                                               live, act.data_ptr(), gws.data_ptr(), gws.nbytes, self._st()), "gateup")

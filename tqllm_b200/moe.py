@@ -172,7 +172,7 @@ def expert_gateup_swiglu(gate, up, x, plan: Plan, sh_gate=None, sh_up=None):
     total = plan.n * plan.topk + plan.shared_tokens
     act = torch.zeros(total, gate.rows, dtype=torch.float32, device=x.device)
     # room for a row per assignment: the grouped GEMM reads the rows of an expert as boxes then and does not gather them
-    ws = _scratch(lib.b2moe_expert_workspace_bytes(gate.type, total, gate.cols, _DT[x.dtype]) + 4 * total, x.device)
+    ws = _scratch(lib.b2moe_expert_slot_workspace_bytes(_bref(gate), total, _DT[x.dtype]), x.device)
     check(lib.b2moe_expert_gateup_swiglu(_bref(gate), _bref(up), _bref(sh_gate), _bref(sh_up), x.data_ptr(), _DT[x.dtype],
                                          plan.buf.data_ptr(), plan.n, plan.topk, plan.shared_tokens, act.data_ptr(),
                                          _ptr(ws), 0 if ws is None else ws.numel(), _stream()), "b2moe_expert_gateup_swiglu")
@@ -181,7 +181,7 @@ def expert_gateup_swiglu(gate, up, x, plan: Plan, sh_gate=None, sh_up=None):
 
 def expert_down(down, act, plan: Plan, sh_down=None):
     y = torch.zeros(act.shape[0], down.rows, dtype=torch.float32, device=act.device)
-    ws = _scratch(lib.b2moe_expert_workspace_bytes(down.type, act.shape[0], down.cols, capi.F32), act.device)
+    ws = _scratch(lib.b2moe_expert_slot_workspace_bytes(_bref(down), act.shape[0], capi.F32), act.device)
     check(lib.b2moe_expert_down(_bref(down), _bref(sh_down), act.data_ptr(), plan.buf.data_ptr(), plan.n, plan.topk,
                                 plan.shared_tokens, y.data_ptr(), _ptr(ws), 0 if ws is None else ws.numel(), _stream()),
           "b2moe_expert_down")
