@@ -99,6 +99,11 @@ bool exact_path(uint32_t type, int k, int dtype, int experts, long long live, in
     return (family == B2MOE_FAMILY_AUTO || family == B2MOE_FAMILY_DECODE) && decode_kernel(type, k, dtype) == DEC_4BIT && live >= (long long)EXACT_MIN_PER * experts &&
            expert_path(type, k, dtype, experts, live, family) == B2MOE_FAMILY_DECODE && gemm_exact_supported(type, k, experts);
 }
+// gate/up takes that form: its `rows` activation rows fit the scratch in slot order (*slots), or they are 16-bit rows, which it gathers
+bool exact_gateup(const b2moe_bank * gate, int x_dtype, long long live, int rows, size_t scratch_bytes, bool * slots) {
+    *slots = scratch_bytes >= gemm_exact_bytes(rows, gate->cols, x_dtype);
+    return exact_path(gate->type, gate->cols, x_dtype, gate->experts, live) && (*slots || x_dtype != B2MOE_F32);
+}
 }  // namespace
 // One matrix over a ready plan with the caller's own row types: x [assignments or, per_token, tokens][cols] of x_dtype -> y
 // [assignments][rows] of y_dtype, without a pass to fp32 before and one back behind. *took = false: the family that serves this call
@@ -215,11 +220,9 @@ static int32_t expert_gateup(const b2moe_bank * gate, const b2moe_bank * up, con
         if (workspace_bytes < need) return B2MOE_ERR_WORKSPACE;
         void * const spare = rows_buf ? rows_buf : workspace;
         const size_t spare_bytes = rows_buf ? rows_buf_bytes : workspace_bytes;
-        if (exact_path(gate->type, gate->cols, x_dtype, gate->experts, live)) {
-            const bool slots = spare_bytes >= gemm_exact_bytes(n * topk + shared_tokens, gate->cols, x_dtype);
-            if (slots || x_dtype != B2MOE_F32)
-                return gemm_exact_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, B2MOE_F32, slots ? spare : workspace, slots, as_stream(stream));
-        }
+        bool slots;
+        if (exact_gateup(gate, x_dtype, live, n * topk + shared_tokens, spare_bytes, &slots))
+            return gemm_exact_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, B2MOE_F32, slots ? spare : workspace, slots, as_stream(stream));
         // a workspace larger than it has to be may hold the rows in slot order itself (gemm_tc_gateup looks at its size): IQ4 banks,
         // 8192 tokens of 8, gate/up alone 2050 us with gathered rows and 1415 with slot order
         if (path == B2MOE_FAMILY_GEMM)
@@ -360,11 +363,12 @@ static int32_t layer_forward(const b2moe_layer * L, const void * x, int32_t x_dt
     if (L->gating == B2MOE_SIGMOID && gated_shared) return B2MOE_ERR_SHAPE;   // the sigmoid family adds its shared expert unscaled (moe_common.cu:191)
     void * es = base + ws.expert_scratch;
     const size_t es_bytes = workspace_bytes - ws.expert_scratch;
-    // decode-sized call on the 4-bit decode kernels: top-k, dispatch and the staging of x in one cluster launch
-    bool x_staged = false;
+    // decode-sized call whose gate/up runs on the 4-bit decode kernels: top-k, dispatch and the staging of x in one cluster launch
+    bool x_staged = false, slots;
     if (route_cluster_fits(L->experts, L->topk, n) && es_bytes >= b2moe_expert_workspace_bytes(L->gate.type, n, L->gate.cols, x_dtype) &&
         expert_path(L->gate.type, L->gate.cols, x_dtype, L->gate.experts, (long long)n * L->topk) == B2MOE_FAMILY_DECODE &&
-        decode_kernel(L->gate.type, L->gate.cols, x_dtype) == DEC_4BIT && valid_dtype(x_dtype)) {
+        decode_kernel(L->gate.type, L->gate.cols, x_dtype) == DEC_4BIT && valid_dtype(x_dtype) &&
+        !exact_gateup(&L->gate, x_dtype, (long long)n * L->topk, n * L->topk + sh, workspace_bytes - ws.y, &slots)) {
         uint8_t * rows;
         float * inv;
         int bits;
