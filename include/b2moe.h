@@ -360,7 +360,8 @@ B2MOE_API int32_t b2moe_place_experts(const uint64_t * counts, int32_t experts, 
  * library is running. They have no counterpart in the reference.
  * b2moe_harness_select: family = the kernel family every later expert product takes where it supports the shape
  * (AUTO = the library's own choice by tokens per expert, the default; DECODE for banks of 4-bit codes: the decode kernels or,
- * from nine assignments per expert on, the exact grouped product that takes their place there); gemm_item_tokens = 256: work items of 256 tokens
+ * from nine assignments per expert on, the exact grouped product that takes their place there; DECODE_KERNELS: the decode kernels at
+ * any density); gemm_item_tokens = 256: work items of 256 tokens
  * in the grouped GEMM; any other value (0 = the default): the library's own choice of 64, 128 or 256 by tokens per expert.
  * b2moe_harness_wait_probe: the 4-bit decode kernels skip the copy of weight tile number drop_tile of every warp
  * (-1 = none, the default) and bound each wait by wait_limit polls (0 = default), so that a test can watch a bounded
@@ -375,7 +376,7 @@ B2MOE_API int32_t b2moe_place_experts(const uint64_t * counts, int32_t experts, 
  * b2moe_harness_column_split: the most warps (1, 2 or 4; default 4) that the 4-bit decode kernels let share one row job
  * when a launch has only a few jobs per block; 1 switches the split off.
  * b2moe_harness_launches: kernel launches the library has made in this process so far. */
-enum b2moe_family { B2MOE_FAMILY_AUTO = 0, B2MOE_FAMILY_GENERIC = 1, B2MOE_FAMILY_DECODE = 2, B2MOE_FAMILY_GEMM = 3 };
+enum b2moe_family { B2MOE_FAMILY_AUTO = 0, B2MOE_FAMILY_GENERIC = 1, B2MOE_FAMILY_DECODE = 2, B2MOE_FAMILY_GEMM = 3, B2MOE_FAMILY_DECODE_KERNELS = 4 };
 B2MOE_API void b2moe_harness_select(int32_t family, int32_t gemm_item_tokens);
 B2MOE_API void b2moe_harness_wait_probe(int32_t drop_tile, uint32_t wait_limit);
 B2MOE_API void b2moe_harness_skip_staging(int32_t on);

@@ -125,3 +125,16 @@ def test_plan_driven_products(types, dtype):
     assert int(plan.buf[3]) == 0 and err(act, want[0]) < TOL and err(y, want[1]) < TOL
     skipped = (ids.reshape(-1) < 0).nonzero().flatten()
     assert len(skipped) > 50 and not act[skipped].any() and not y[skipped].any()
+
+
+def test_decode_kernels_can_be_pinned():
+    """the harness reaches the decode kernels at a density where a call takes this form, and they keep their precision there"""
+    from tqllm_b200 import capi, moe
+    dev = moe.MoeLayer.from_synth(synth.make_layer(synth.LayerShape("pin", 1024, 8, 2, 512, types=(IQ3_S,) * 3), 5, "cuda"))
+    x = synth.make_tokens(dev.shape, 120, 6, "cuda")
+    for family, exact in (("auto", True), ("decode", True), ("decode_kernels", False)):
+        with capi.family(family):
+            dev.forward(x)
+        art = dev.artefacts()
+        act, y = products(dev, x, art["ids"].long(), False)
+        assert (err(art["act"], act) < TOL) == exact and (err(art["y"], y) < TOL) == exact and err(art["y"], y) < 1e-3

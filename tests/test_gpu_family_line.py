@@ -1,5 +1,6 @@
-"""GPU: the line between the decode kernels and the grouped GEMM. Below it (fewer than 32 assignments per expert, or a bank of fewer than
-128 experts) a call has the decode kernels' bits and their precision, from it on the GEMM's: the library's own choice is
+"""GPU: the line between the decode family and the grouped GEMM. Below it (fewer than 32 assignments per expert, or a bank of fewer than
+128 experts) a call has the decode family's bits (the decode kernels', or at these densities for 4-bit codes those of the exact grouped
+product) and at least their precision, from it on the GEMM's: the library's own choice is
 compared, bit for bit, with either family forced. The decode kernels round the activations to 15 bits of a row's largest magnitude (about
 four standard deviations of a normal row: 1e-4 of the values' RMS) and the weights not at all; the GEMM's 11 bits of both give at least 2.9e-4."""
 import pytest

@@ -241,11 +241,11 @@ def test_errors_reach_the_caller():
 @pytest.mark.parametrize("layout", ("codes", "gguf"))
 @pytest.mark.parametrize("act_dtype,experts,tokens,topk", (("f32", 4, 40, 2), ("bf16", 4, 70, 3), ("bf16", 24, 3, 8), ("f32", 16, 1, 4)))
 def test_iq3s_decode_kernels(orc, act_dtype, experts, tokens, topk, layout):
-    """the IQ3_S decode kernels of both bank layouts (pinned: batches this dense default to the grouped GEMM): fp32 and
+    """the IQ3_S decode kernels of both bank layouts (pinned: batches this dense take grouped products otherwise): fp32 and
     bf16 activations, experts holding many more tokens than one pass takes, experts holding one token, a shared expert"""
     from tqllm_b200 import capi
     shape = synth.LayerShape("iq3s-dec", 512, experts, topk, 256, shared=True, types=(21, 21, 21), act_dtype=act_dtype)
-    with capi.family("decode"):
+    with capi.family("decode_kernels"):
         err = run_case(orc, shape, experts, tokens, 4242 + tokens, iq3s_layout=layout)
     assert err < 2e-3
 
@@ -259,7 +259,7 @@ def test_q4k_decode_kernels(orc, gating, shared, hidden, ff, experts, tokens, to
     down = 12 if ff % 256 == 0 else 20                       # Q4_K needs 256-column blocks; IQ4_NL down otherwise
     shape = synth.LayerShape("q4k-dec", hidden, experts, topk, ff, gating=gating, sel_bias=gating == 2, shared=shared,
                              types=(12, 12, down))
-    with capi.family("decode"):
+    with capi.family("decode_kernels"):
         err = run_case(orc, shape, experts, tokens, 99 + tokens)
     assert err < 2e-3
 

@@ -16,7 +16,7 @@ OK, ERR_SHAPE, ERR_ALIGN, ERR_FORMAT, ERR_NULL, ERR_WORKSPACE, ERR_CUDA, ERR_CAP
 F32, F16, BF16 = 0, 1, 2
 Q4_K, IQ4_NL, IQ3_S, IQ4_XS, NVFP4G = 12, 20, 21, 23, 323
 IQ3_S_X4 = 0x1015        # bank layout of IQ3_S blocks as 4-bit codes (b2moe_type)
-FAMILY = {"auto": 0, "generic": 1, "decode": 2, "gemm": 3}
+FAMILY = {"auto": 0, "generic": 1, "decode": 2, "gemm": 3, "decode_kernels": 4}
 SOFTMAX, SIGMOID = 1, 2
 
 
@@ -147,8 +147,8 @@ def codebooks():
 
 
 class family:
-    """Every expert product inside the block takes the named kernel family ("generic", "decode", "gemm") where it supports
-    the shape; `item_tokens` = 256 selects the wide work items of the grouped GEMM. Harness hook: process-wide."""
+    """Every expert product inside the block takes the named kernel family ("generic", "decode", "gemm", or "decode_kernels": the
+    decode family without its exact grouped product) where it supports the shape; `item_tokens` = 256 selects the wide work items of the grouped GEMM. Harness hook: process-wide."""
 
     def __init__(self, name: str, item_tokens: int = 0):
         self.name, self.item_tokens = name, item_tokens

@@ -83,7 +83,7 @@ int g_family = B2MOE_FAMILY_AUTO;
 int expert_path(uint32_t type, int k, int dtype, int experts, long long assignments, int family = g_family) {
     if (family == B2MOE_FAMILY_GENERIC) return B2MOE_FAMILY_GENERIC;
     const bool dec = decode_kernel(type, k, dtype) != DEC_NONE, gemm = gemm_tc_supported(type, k, experts);
-    if (family == B2MOE_FAMILY_DECODE) return dec ? B2MOE_FAMILY_DECODE : B2MOE_FAMILY_GENERIC;
+    if (family == B2MOE_FAMILY_DECODE || family == B2MOE_FAMILY_DECODE_KERNELS) return dec ? B2MOE_FAMILY_DECODE : B2MOE_FAMILY_GENERIC;
     if (family == B2MOE_FAMILY_GEMM) return gemm ? B2MOE_FAMILY_GEMM : dec ? B2MOE_FAMILY_DECODE : B2MOE_FAMILY_GENERIC;
     if (dec && (!gemm || assignments < (long long)GEMM_MIN_PER * experts || experts < GEMM_MIN_EXPERTS)) return B2MOE_FAMILY_DECODE;
     return gemm ? B2MOE_FAMILY_GEMM : B2MOE_FAMILY_GENERIC;
@@ -166,7 +166,7 @@ extern "C" B2MOE_API void b2moe_codebooks(uint32_t * grid, int8_t * kv) {
 }
 
 extern "C" B2MOE_API void b2moe_harness_select(int32_t family, int32_t gemm_item_tokens) {
-    g_family = family >= B2MOE_FAMILY_AUTO && family <= B2MOE_FAMILY_GEMM ? family : B2MOE_FAMILY_AUTO;
+    g_family = family >= B2MOE_FAMILY_AUTO && family <= B2MOE_FAMILY_DECODE_KERNELS ? family : B2MOE_FAMILY_AUTO;
     gemm_tc_item_tokens(gemm_item_tokens);
 }
 extern "C" B2MOE_API void b2moe_harness_wait_probe(int32_t drop_tile, uint32_t wait_limit) { dec4_debug(drop_tile, wait_limit); }
