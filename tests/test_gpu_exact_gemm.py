@@ -127,6 +127,35 @@ def test_plan_driven_products(types, dtype):
     assert len(skipped) > 50 and not act[skipped].any() and not y[skipped].any()
 
 
+@pytest.mark.parametrize("dtype", (torch.bfloat16, torch.float16), ids=("bf16", "f16"))
+@pytest.mark.parametrize("types,hidden", (((Q4_K,) * 3, 1280), ((IQ3_S,) * 3, 768)), ids=("q4k", "iq3s"))
+@pytest.mark.parametrize("n,skip,skew", ((37, 0., False), (77, .2, True), (331, .4, False)))
+def test_gathered_rows_change_no_bit(types, hidden, n, skip, skew, dtype):
+    """gate/up from the scratch that it accepts, where it gathers token rows, and from a larger one with the rows in slot order: the same rows in
+    the same order; a shared expert, skipped ids, counts that do not divide by the loaders' four rows, an expert with most of the tokens"""
+    from tqllm_b200 import capi, moe
+    lib, experts, topk = capi.lib, 16, 4
+    dev = moe.MoeLayer.from_synth(synth.make_layer(synth.LayerShape("gather", hidden, experts, topk, 512, shared=True, types=types), 3, "cuda"))
+    g = torch.Generator().manual_seed(n)
+    order = torch.rand(n, experts, generator=g)
+    if skew:
+        order[:, 11] -= 0.9
+    ids = order.argsort(1)[:, :topk].to(torch.int32).contiguous()
+    ids[torch.rand(n, topk, generator=g) < skip] = -1
+    x = torch.randn(n, hidden, generator=g).cuda().to(dtype)
+    plan, slots, code = moe.dispatch(ids.cuda(), experts, n), n * topk + n, capi.BF16 if dtype == torch.bfloat16 else capi.F16
+    small, large = lib.b2moe_expert_workspace_bytes(dev.gate.type, n, hidden, code), lib.b2moe_expert_slot_workspace_bytes(C.byref(dev.gate.c), slots, code)
+    assert small < slots * (2 * hidden + hidden // 8)
+    out = []
+    for nbytes in (small, large):
+        act, ws = torch.zeros(slots, 512, device="cuda"), torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+        capi.check(lib.b2moe_expert_gateup_swiglu(*(C.byref(b.c) for b in (dev.gate, dev.up, dev.sh[0], dev.sh[1])), x.data_ptr(), code, plan.buf.data_ptr(), n, topk,
+                                                  n, act.data_ptr(), ws.data_ptr(), nbytes, torch.cuda.current_stream().cuda_stream), "gateup")
+        assert int(plan.buf[3]) == 0
+        out.append(act)
+    assert torch.equal(out[0], out[1]) and err(out[0], products(dev, x, ids.cuda().long(), True)[0]) < TOL
+
+
 def test_decode_kernels_can_be_pinned():
     """the harness reaches the decode kernels at a density where a call takes this form, and they keep their precision there"""
     from tqllm_b200 import capi, moe
