@@ -50,6 +50,16 @@ def test_large_path(orc, n, k, e):
     check(orc, ids, e, False)
 
 
+@pytest.mark.parametrize("e", (619, 620, 654, 655, 981, 982))
+@pytest.mark.parametrize("n,k", ((70, 8), (512, 8), (513, 8), (1024, 8), (1500, 6)))
+def test_edges_of_the_paths(orc, n, k, e):
+    """the last expert counts whose counters fit the single block (654; beyond 4,096 ids 619) and the two-launch form (981), and one more"""
+    rng = np.random.default_rng(n + e)
+    ids = rng.integers(-1, e, size=(n, k)).astype(np.int32)
+    ids[:4] = (e - 1, 0, e - 2, 1, -1, 2, e - 1, 0)[:k]
+    check(orc, ids, e, n % 4 == 0)
+
+
 def test_skipped_and_degenerate(orc):
     rng = np.random.default_rng(0)
     ids = rng.integers(-1, 9, size=(50, 4)).astype(np.int32)

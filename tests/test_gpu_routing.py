@@ -113,3 +113,22 @@ def test_sigmoid_known_answers(orc):
     assert np.isfinite(w.cpu().numpy()).all() and list(ids[0].cpu().numpy()) == [0, 1, 2, 3]
     ids, _ = moe.route_sigmoid(torch.full((1, 8), 0.5).cuda(), 8, 3, None, False, 0.0)
     assert list(ids[0].cpu().numpy()) == [0, 1, 2]
+
+
+@pytest.mark.parametrize("gating", (1, 2))
+@pytest.mark.parametrize("e,k,n", ((512, 10, 64), (620, 8, 1), (640, 8, 16), (654, 10, 17), (654, 8, 128), (655, 8, 20), (640, 8, 600)))
+def test_route_dispatch_equals_separate_calls(gating, e, k, n):
+    """one launch or several: the ids, weights and plan of the separate routing and dispatch calls, where the one-launch forms end"""
+    from tqllm_b200 import capi, moe
+    logits = torch.randn(n, e + 1, device="cuda", generator=torch.Generator("cuda").manual_seed(n + e))
+    if gating == 1:
+        ids, w, _ = moe.topk_softmax(logits, e, k)
+    else:
+        ids, w = moe.route_sigmoid(logits, e, k)
+    want = moe.dispatch(ids, e, n)
+    got, ids2, w2 = moe.Plan(e, n, k, n, "cuda"), torch.empty_like(ids), torch.empty_like(w)
+    ws = torch.empty(max(16, capi.lib.b2moe_dispatch_workspace_bytes(e, n * k)), dtype=torch.uint8, device="cuda")
+    capi.check(capi.lib.b2moe_route_dispatch(gating, logits.data_ptr(), e + 1, None, ids2.data_ptr(), w2.data_ptr(), None, e, k, 1, 0.0, n, 0, n, got.buf.data_ptr(),
+                                             ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream), "route_dispatch")
+    assert torch.equal(ids, ids2) and torch.equal(w, w2) and torch.equal(got.counts, want.counts) and torch.equal(got.offsets, want.offsets)
+    assert torch.equal(got.perm, want.perm) and int(got.buf[2]) == int(want.buf[2])

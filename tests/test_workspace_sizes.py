@@ -7,10 +7,10 @@ import pytest
 from tqllm_b200 import capi
 from tqllm_b200.capi import lib
 
-EDGES = sorted({max(1, e + d) for e in (1, 1024, 8192, 37888, 65536, 151552, 303104, 1 << 20, 5 << 20) for d in (-1025, -1, 0, 1, 33, 1025)})
+EDGES = sorted({max(1, e + d) for e in (1, 1024, 4096, 8192, 37888, 65536, 151552, 303104, 1 << 20, 5 << 20) for d in (-1025, -1, 0, 1, 33, 1025)})
 
 
-@pytest.mark.parametrize("experts", (1, 8, 128, 512, 900, 1000, 4096))
+@pytest.mark.parametrize("experts", (1, 8, 128, 512, 640, 900, 1000, 4096))
 def test_dispatch_scratch(experts):
     sizes = [lib.b2moe_dispatch_workspace_bytes(experts, a) for a in EDGES]
     assert all(s % 16 == 0 and s >= 16 for s in sizes)

@@ -35,8 +35,8 @@ __global__ void dispatch_small_k(const int * ids, int A, int e, int shared_first
 // block 0. Measured on the device: 41,000 ids on 512 experts 41 us + a memset -> 20 us, 65,536 on 128 experts 15 us.
 struct WalkArgs { const int * ids; int A, e, seg, shared_first, shared_tokens; int * rows, * plan; };
 __host__ __device__ inline int row_parts(int e) { return e >= WALK_THREADS ? 1 : WALK_THREADS / e; }
-// hist [warps][e], totals and lower sums [row_parts][e], three arrays of e + 2
-inline size_t walk_smem(int e) { return (size_t(WALK_WARPS) * e + size_t(2) * row_parts(e) * e + size_t(3) * (e + 2)) * sizeof(int); }
+// hist [warps][e], totals and lower sums [row_parts][e], counts and offsets of e + 2 each
+inline size_t walk_smem(int e) { return (size_t(WALK_WARPS) * e + size_t(2) * row_parts(e) * e + size_t(2) * (e + 2)) * sizeof(int); }
 
 __device__ __forceinline__ void count_segment(const WalkArgs & p, int a0, int a1, int * hist, int lane, int warp) {
     for (int i = threadIdx.x; i < WALK_WARPS * p.e; i += WALK_THREADS) hist[i] = 0;
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(WALK_THREADS) dispatch_place_k(const WalkArgs 
 // beyond that what a block per SM leaves, since every block reads every row.
 inline int walk_seg(int A) { return std::max(128, (ceil_div(A, WALK_MAX_BLOCKS * WALK_WARPS) + 31) / 32 * 32); }
 inline int walk_blocks(int A) { return ceil_div(A, walk_seg(A) * WALK_WARPS); }         // at most WALK_MAX_BLOCKS
-// the counters have to fit a block's ordinary shared memory: up to about 900 experts
+// the counters have to fit a block's ordinary shared memory: up to 981 experts
 inline bool walk_path(int e) { return walk_smem(e) <= 46 * 1024; }
 
 // ---- more experts than that: chunk counters in global scratch [chunks][e] ----

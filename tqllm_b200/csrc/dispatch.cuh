@@ -119,8 +119,8 @@ __device__ inline void finish_plan(int * plan, const int * cs, int * os, int * o
     }
 }
 
-// shared memory of dispatch_small_body for a block of `warps` warps: hist [warps][e] (16-bit) + three int arrays of e + 2
-__host__ __device__ inline size_t dispatch_small_smem(int warps, int e) { return (size_t(warps) * e * 2 + 15) / 16 * 16 + size_t(3) * (e + 2) * 4; }
+// shared memory of dispatch_small_body for a block of `warps` warps: hist [warps][e] (16-bit) + counts and offsets, e + 2 ints each
+__host__ __device__ inline size_t dispatch_small_smem(int warps, int e) { return (size_t(warps) * e * 2 + 15) / 16 * 16 + size_t(2) * (e + 2) * 4; }
 
 // ---- single block (up to 32 warps): every phase in shared memory (decode-sized batches); hist = [warps][e] ----
 template <bool VOTES>
@@ -170,7 +170,9 @@ __device__ __forceinline__ void dispatch_small_body(const int * ids, int A, int 
     for (int t = threadIdx.x; t < shared_tokens; t += blockDim.x) perm[os[e] + t] = A + shared_first + t;
 }
 
-
-inline bool dispatch_small_path(int e, int A) { return A <= 32 * 2048 / 8 && dispatch_small_smem(32, e) <= 46 * 1024; }
+// One block while its counters fit a block's ordinary shared memory: up to 654 experts. Beyond 4,096 ids two launches over many blocks are the
+// faster form (640 experts: 640 ids 4.8 us in one block and 10.5 in two launches, 4,000 ids 10.7 and 11.0, 8,000 ids 15.7 and 11.2). Up to 619 experts
+// the line stays at 8,192 ids: callers have sized their scratch by it, and two launches need some.
+inline bool dispatch_small_path(int e, int A) { return A <= (e <= 619 ? 8192 : 4096) && dispatch_small_smem(32, e) <= 46 * 1024; }
 
 }  // namespace b2
