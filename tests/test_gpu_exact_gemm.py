@@ -1,5 +1,5 @@
 """GPU: the exact form of the grouped GEMM (banks of 4-bit codes from nine assignments per expert on): integer operands, activations in one
-fp16 term (16-bit rows: no rounding at all) or two (fp32 rows: 2^-22), sums scaled and added in fp32. Against products in 64 bits. Bound: the
+fp16 term (16-bit rows: no rounding above 2^-29 of the row's largest value) or two (fp32 rows: 2^-22), sums scaled and added in fp32. Against products in 64 bits. Bound: the
 tensor core's truncated fp32 sums of up to 256 columns and their fp32 total, about sqrt(256) 2^-24 = 1e-6 of a row's result in the
 2-norm, twice through both products; the decode kernels, which a wrong choice of the family would give, lie above 1.6e-5."""
 import ctypes as C

@@ -640,7 +640,7 @@ int32_t launch_dec4(Dec4Args a, cudaStream_t s) {
     if (cudaFuncSetAttribute(dec4_k<T, MODE, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return B2MOE_ERR_CUDA;
     a.wait_limit = g_wait_limit;
     a.drop_tile = g_drop_tile;
-    launch_overlapped(dec4_k<T, MODE, FEW>, dim3(sms), dim3(threads_of<FEW && MODE == 1>()), smem, s, a);       // every block takes an equal share of the (pass, row tile) jobs
+    launch_overlapped(dec4_k<T, MODE, FEW>, dim3(sms), dim3(threads_of<FEW && MODE == 1>()), smem, s, a);       // a block's share of the (pass, row tile) jobs: an equal one, or (FEW) whole passes
     return launch_status();
 }
 

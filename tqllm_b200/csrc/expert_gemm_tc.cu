@@ -65,7 +65,8 @@ constexpr int load_warps(bool gather) { return gather ? 6 : 2; }
 constexpr int g_threads(bool gather) { return (LOAD_WARP0 + load_warps(gather) + EPI_WARPS + DEC_WARPS) * 32; }
 static_assert(EPI_WARPS * 32 == MAX_CAP, "an epilogue thread looks one token up");
 static_assert(MAX_B_STAGES <= STEP_RING, "a B stage is freed by the barrier of the step that used it");
-// The exact form (TERMS > 0): items of up to X_CAP tokens; two sets of sums, a chunk's each: X_CAP columns per term of the activations, then X_CAP
+// The exact form (TERMS > 0): items of up to X_CAP tokens at every density (an expert of 100 tokens is decoded four times: 1000 tokens on 60 experts 311 us,
+// 168 with the other form's items of 128); two sets of sums, a chunk's each: X_CAP columns per term of the activations, then X_CAP
 // of the mins; after both the mins' A operand of either chunk. X_RING: chunks whose row constants the epilogue may still need
 constexpr int X_CAP = 32, X_SET = 3 * X_CAP, X_MINS = 2 * X_CAP, X_AMINS = 2 * X_SET, X_RING = 4;
 static_assert(X_AMINS + 2 * 8 <= A_COL0, "two sets of sums and two operands of mins below the A stages");
@@ -224,7 +225,7 @@ __global__ void tokens_to_slots_k(const typename Elem<DT>::type * x, const int *
     });
     if (mine >= 0) inv_scale[mine] = inv;
 }
-// Rows of the exact form: [TERMS][rows][k] fp16, a value as one term (16-bit activations: exact) or as two (fp32: 22 bits), and for the mins of
+// Rows of the exact form: [TERMS][rows][k] fp16, a value as one term (16-bit activations: exact down to 2^-29 of the row's largest magnitude) or as two (fp32: 22 bits), and for the mins of
 // Q4_K the sums of the row's 32-column sub-blocks, divided by 32, as [rows][k / 256][16]: eight leading fp16 terms, then the eight rests.
 // A lane holds eight columns of one sub-block, lanes l, l ^ 1, l ^ 4, l ^ 5 all of it.
 template <uint32_t T, int DT, int TERMS, typename Slots>
@@ -277,7 +278,7 @@ __global__ void exact_rows_k(const typename Elem<DT>::type * x, const int * plan
 }
 
 // MODE 0: act[a][r] = silu(gate_r . x_tok(a)) * (up_r . x_tok(a));  MODE 1: y[a][r] = down_r . act[a]
-// TERMS > 0: the exact form: no rounding but that of the activations to TERMS fp16 terms and of the fp32 sums
+// TERMS > 0: the exact form: no rounding but that of the activations to TERMS fp16 terms (16-bit ones: none above 2^-29 of the row's largest) and of the fp32 sums
 // F32_OUT: an instance for fp32 results and one for 16-bit ones, chosen by the call's output type. A branch at the stores, or two
 // loops in one kernel, cost every fp32 caller: c3 down (80 tokens x K = 512) 262 us against 184, c5 gate/up 1305 against 1240.
 // GATHER: the activation rows lie in token order.

@@ -75,8 +75,8 @@ int decode_kernel(uint32_t type, int k, int dtype) {
 // of precision as much as of time: the decode kernels take the weights as they are and 15-bit activations, the GEMM rounds both to 11 bits. Relative error against
 // 64-bit sums (2-norm), decode / GEMM, at any density: Q4_K act 2.5e-5 / 4.0e-4, down of it 2.0e-4 / 5.3e-4; IQ3_S codes 2.5e-5 / 3.0e-4
 // and 2.0e-4 / 4.2e-4; IQ3_S in GGUF fields 2e-7 / 3.0e-4 and 2.1e-4 / 4.2e-4. The GEMM is the faster one from about 20 per
-// expert on (layer times, decode family / GEMM, us: IQ3_S codes of 512 experts at 20 per expert 416 / 412, Q4_K of 256 at 31 1116 / 879, of 60 at 100
-// 315 / 169), but nothing below this line asked for fewer bits. b2moe_harness_select forces a family where it supports the shape
+// expert on (layer times, decode family / GEMM, us: IQ3_S codes of 512 experts at 20 per expert 417 / 405, Q4_K of 256 at 19 797 / 785, at 31 1074 / 843, of 60 at 100
+// 311 / 168), but nothing below this line asked for fewer bits. b2moe_harness_select forces a family where it supports the shape
 // (tests and benchmarks).
 constexpr int GEMM_MIN_PER = 32, GEMM_MIN_EXPERTS = 128;
 int g_family = B2MOE_FAMILY_AUTO;
@@ -90,10 +90,11 @@ int expert_path(uint32_t type, int k, int dtype, int experts, long long assignme
 }
 // Where the rule above says DECODE, banks of 4-bit codes have a second form: the grouped GEMM with integer operands and scales
 // applied to its sums in fp32 (gemm_exact_*), which loses less precision than the decode kernels and reads an expert's weights once per 32
-// tokens instead of once per eight. It takes over from EXACT_MIN_PER assignments per expert on. Layer times, decode / this form, us: Q4_K of 256
-// experts at 7.8 per expert 629 / 685, 19 1237 / 797, 31 1920 / 1116; of 60 at 7.7 106 / 109, 10 124 / 111, 100 577 / 315; of 32 in fp32 at 8 45 / 43, 1000 838 / 491; IQ3_S
-// codes of 512 at 7 307 / 336, 8 339 / 344, 10 390 / 355. Relative error of both products against 64 bits 2.0e-4 / 1.0e-6. Gate/up on 16-bit rows runs
-// from any scratch that the call accepts; fp32 rows (two terms each) take the decode kernels where the scratch has no room for them.
+// tokens instead of once per eight. It takes over from EXACT_MIN_PER assignments per expert on. Layer times, decode kernels / this form, us: Q4_K of 256
+// experts at 7.8 per expert 622 / 687, 9 662 / 677, 10 716 / 665, 19 1219 / 797, 31 1926 / 1074; of 60 at 7.7 103 / 105, 9 109 / 106, 10 115 / 109, 100 567 / 311; of 32 in fp32 at 6
+// 38 / 41, 8 43 / 42, 1000 837 / 485; IQ3_S codes of 512 at 7 307 / 340, 8 339 / 347, 9 361 / 347, 10 389 / 350. At nine itself, over 42 shapes of 2 to 127 experts,
+// this form takes 0.57 to 1.08 of the decode kernels' time, 0.9 on average; at twelve 0.69 to 1.03. Relative error of both products against 64 bits 2.0e-4 / 1.0e-6. Gate/up on
+// 16-bit rows runs from any scratch that the call accepts; fp32 rows (two terms each) take the decode kernels where the scratch has no room for them.
 constexpr int EXACT_MIN_PER = 9;
 bool exact_path(uint32_t type, int k, int dtype, int experts, long long live, int family = g_family) {
     return (family == B2MOE_FAMILY_AUTO || family == B2MOE_FAMILY_DECODE) && decode_kernel(type, k, dtype) == DEC_4BIT && live >= (long long)EXACT_MIN_PER * experts &&
