@@ -40,14 +40,13 @@
 // gave 3e-2 of the output RMS as the largest error, fp16 stays below the layer tolerance). An activation row is
 // multiplied by 2^e so that its largest magnitude lies in [2^14, 2^15) and rounded to fp16: exact for bf16 inputs down
 // to 2^-29 of the row maximum; the epilogue multiplies the sums (fp32) by 2^-e.
-#include <cuda.h>
-
 #include <type_traits>
 
 #include "common.cuh"
 #include "formats.cuh"
 #include "gemm_decode.cuh"
 #include "tc_ptx.cuh"
+#include "tensor_map.cuh"
 
 namespace b2 {
 namespace {
@@ -814,22 +813,6 @@ template <uint32_t T> bool gemm_fit(int experts, int cap_wanted, GemmArgs & a) {
             }
     }
     return false;
-}
-decltype(&cuTensorMapEncodeTiled) map_encoder() {
-    static const auto encode = []() -> decltype(&cuTensorMapEncodeTiled) {
-        void * f = nullptr;
-        cudaDriverEntryPointQueryResult found;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess) f = nullptr;
-        return reinterpret_cast<decltype(&cuTensorMapEncodeTiled)>(f);
-    }();
-    return encode;
-}
-bool encode_map(CUtensorMap & m, CUtensorMapDataType type, int rank, const void * base, const cuuint64_t * dims, const cuuint64_t * strides,
-                const cuuint32_t * box, CUtensorMapSwizzle swizzle) {
-    const cuuint32_t steps[4] = {1, 1, 1, 1};
-    const auto encode = map_encoder();
-    return encode && encode(&m, type, rank, const_cast<void *>(base), dims, strides, box, steps, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
-                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 // `rows` fp16 activation rows of length k as [k / 64][rows][64]: a box is box_rows rows of `steps` 64-column steps, one step after the other
 bool rows_map(CUtensorMap & m, const void * xb, int rows, int k, int box_rows, int steps) {

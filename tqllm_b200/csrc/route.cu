@@ -214,17 +214,15 @@ __global__ void __launch_bounds__(RM_WARPS * 32) router_mma_k(const float * __re
     cluster.sync();                                                     // the other blocks' tiles stay alive until block 0 has read them
 }
 
-// ---- the same product for many tokens (prefill): shared-memory tiles ----
+// ---- the same product for many tokens (prefill) of fp32, and of short fp16 rows: shared-memory tiles ----
 // One block = 64 router rows x 128 tokens, 8 warps of 32 x 32 outputs, 32 columns per stage: both operands are split into
-// their bf16 terms once per block and stage (not once per 64 tokens and warp as above) and reach the MMAs through ldmatrix, so
-// a stage of bf16 rows costs a warp 16 shared loads for its 48 MMAs. Every output is summed over the hidden dimension in
-// ascending column order (terms lo, mid, hi per 16 columns; 256 columns per partial sum): the same bits every run. fp16 and fp32 rows:
-// the leading products of a stage's two 16-column steps are added to each other, then to the partial sum (see above for the reason).
+// their bf16 terms once per block and stage (not once per 64 tokens and warp as above) and reach the MMAs through ldmatrix. Every output is summed over the hidden dimension in
+// ascending column order (terms lo, mid, hi per 16 columns; 256 columns per partial sum): the same bits every run; the leading products of a stage's two 16-column steps are added to each other, then to the partial sum (see above for the reason).
 // A launch has few such tiles (2047 tokens x 256 experts: 64), and a tile alone leaves an SM waiting on its own loads: up to
 // eight blocks of a cluster take a part of a tile's 256-column partial sums each and add all of them, in column order, through
 // distributed shared memory, so the split changes no bit.
-// Measured, one block per tile against the split: 32 tiles of 2048 columns 60 -> 21 us, 64 of 3072 columns 85 -> 57, 20 of 3072
-// columns (fp16) 124 -> 32; 128 of 4096 columns 116 -> 127, 256 of 2048 columns 96 -> 118: from 100 tiles on, one block per tile.
+// Measured, one block per tile against the split: 20 of 3072 columns (fp16) 124 -> 32; (bf16, since served by router_tc_k) 32 tiles of 2048 columns
+// 60 -> 21 us, 128 of 4096 columns 116 -> 127, 256 of 2048 columns 96 -> 118: from 100 tiles on, one block per tile.
 constexpr int RT_ROWS = 64, RT_TOK = 128, RT_K = 32, RT_THREADS = 256, RT_LD = RT_K + 8;   // row stride in shared memory: 80 bytes, conflict-free for ldmatrix
 constexpr int RT_SPLIT_BELOW = 100, RT_MAX_PARTS = 64, RT_COLS = 256, RT_PLD = RT_ROWS + 4, RT_PART = RT_TOK * RT_PLD * 4;           // columns of a partial sum; a tile of them in shared memory, [token][row]
 constexpr int RT_W_STAGE = 3 * RT_ROWS * RT_LD * 2, RT_X_TERM = RT_TOK * RT_LD * 2;
@@ -266,33 +264,22 @@ __global__ void __launch_bounds__(RT_THREADS) router_tile_k(const float * __rest
         const int p = tid + RT_THREADS * j;
         xsrc[j] = x + size_t(min(t0 + p / PPT, n - 1)) * h + V * (p % PPT);
     }
-    [[maybe_unused]] uint4 xreg[XJ];
-    auto load_x = [&](int stage, int k0) {                             // bf16 rows go straight to shared memory, the others wait in registers to be split
+    uint4 xreg[XJ];
+    auto load_x = [&](int k0) {                                        // the values wait in registers to be split
 #pragma unroll
-        for (int j = 0; j < XJ; ++j) {
-            if constexpr (XT == 1) {
-                const int p = tid + RT_THREADS * j;
-                const uint32_t dst = uint32_t(__cvta_generic_to_shared(x_sm + stage * X_STAGE + ((p / PPT) * RT_LD + V * (p % PPT)) * 2));
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(__cvta_generic_to_global(xsrc[j] + k0)) : "memory");
-            } else {
-                xreg[j] = *reinterpret_cast<const uint4 *>(xsrc[j] + k0);
-            }
-        }
-        if constexpr (XT == 1) asm volatile("cp.async.commit_group;" ::: "memory");
+        for (int j = 0; j < XJ; ++j) xreg[j] = *reinterpret_cast<const uint4 *>(xsrc[j] + k0);
     };
     auto store_x = [&](int stage) {
-        if constexpr (XT > 1) {
 #pragma unroll
-            for (int j = 0; j < XJ; ++j) {
-                const int p = tid + RT_THREADS * j;
-                uint32_t * dst = reinterpret_cast<uint32_t *>(x_sm + stage * X_STAGE + ((p / PPT) * RT_LD + V * (p % PPT)) * 2);
+        for (int j = 0; j < XJ; ++j) {
+            const int p = tid + RT_THREADS * j;
+            uint32_t * dst = reinterpret_cast<uint32_t *>(x_sm + stage * X_STAGE + ((p / PPT) * RT_LD + V * (p % PPT)) * 2);
 #pragma unroll
-                for (int i = 0; i < V / 2; ++i) {
-                    uint32_t v[XT];
-                    x_pair<DT>(reinterpret_cast<const E *>(&xreg[j]) + 2 * i, v);
+            for (int i = 0; i < V / 2; ++i) {
+                uint32_t v[XT];
+                x_pair<DT>(reinterpret_cast<const E *>(&xreg[j]) + 2 * i, v);
 #pragma unroll
-                    for (int q = 0; q < XT; ++q) dst[q * (RT_X_TERM / 4) + i] = v[q];
-                }
+                for (int q = 0; q < XT; ++q) dst[q * (RT_X_TERM / 4) + i] = v[q];
             }
         }
     };
@@ -316,18 +303,17 @@ __global__ void __launch_bounds__(RT_THREADS) router_tile_k(const float * __rest
     // acc sums 256 columns at a time and is then put away: the rounding error of a long fp32 chain grows with its
     // length, and the router's tolerance against an fp64 dot (3e-6) leaves no room for a 2048-term chain
     float acc[2][4][4];
-    [[maybe_unused]] float low[2][4][4];                               // fp16, fp32: the sums of all products but the leading one
+    float low[2][4][4];                                                // the sums of all products but the leading one
     [[maybe_unused]] float tot[2][4][4];                               // one block per tile: it adds the partial sums up in registers
 #pragma unroll
     for (int a = 0; a < 2; ++a)
 #pragma unroll
         for (int b = 0; b < 4; ++b)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) { acc[a][b][c] = 0.f; if (XT > 1) low[a][b][c] = 0.f; if (!SPLIT) tot[a][b][c] = 0.f; }
+            for (int c = 0; c < 4; ++c) { acc[a][b][c] = low[a][b][c] = 0.f; if (!SPLIT) tot[a][b][c] = 0.f; }
     auto part_sum = [&](int a, int b, int c) {                         // the finished partial sum, and back to zero
-        const float v = XT > 1 ? acc[a][b][c] + low[a][b][c] : acc[a][b][c];
-        acc[a][b][c] = 0.f;
-        if (XT > 1) low[a][b][c] = 0.f;
+        const float v = acc[a][b][c] + low[a][b][c];
+        acc[a][b][c] = low[a][b][c] = 0.f;
         return v;
     };
     auto put_away = [&](uint8_t * at) {
@@ -345,17 +331,16 @@ __global__ void __launch_bounds__(RT_THREADS) router_tile_k(const float * __rest
     const uint32_t w_base = uint32_t(__cvta_generic_to_shared(w_sm)) + ((32 * wr + (lane & 15)) * RT_LD + 8 * (lane >> 4)) * 2;
     const uint32_t x_base = uint32_t(__cvta_generic_to_shared(x_sm)) + ((32 * wc + (lane & 7) + 8 * (lane >> 4)) * RT_LD + 8 * ((lane >> 3) & 1)) * 2;
     const int s_lo = p_lo * (RT_COLS / RT_K), s_hi = min(h / RT_K, p_hi * (RT_COLS / RT_K));
-    load_x(s_lo & 1, s_lo * RT_K);
+    load_x(s_lo * RT_K);
     load_w(s_lo * RT_K);
 #pragma unroll 1
     for (int s = s_lo; s < s_hi; ++s) {
         const int buf = s & 1;
         store_w(buf);
         store_x(buf);
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();                                               // stage s is complete; every warp is done with stage s - 1
-        if (s + 1 < s_hi) { load_x(buf ^ 1, (s + 1) * RT_K); load_w((s + 1) * RT_K); }
-        [[maybe_unused]] float lead[2][4][4];                          // the leading products of the stage's first 16 columns
+        if (s + 1 < s_hi) { load_x((s + 1) * RT_K); load_w((s + 1) * RT_K); }
+        float lead[2][4][4];                          // the leading products of the stage's first 16 columns
 #pragma unroll
         for (int kk = 0; kk < RT_K / 16; ++kk) {
             uint32_t b[XT][2][4];                                      // per term, token tiles (0, 1) and (2, 3): b0, b1 of each
@@ -375,9 +360,7 @@ __global__ void __launch_bounds__(RT_THREADS) router_tile_k(const float * __rest
                         for (int nt = 0; nt < 4; ++nt)
                             if (DT != B2MOE_F32 || term + q < 3) {
                                 const uint32_t b0 = b[q][nt >> 1][2 * (nt & 1)], b1 = b[q][nt >> 1][2 * (nt & 1) + 1];
-                                if constexpr (XT == 1) {
-                                    mma_bf16_acc(acc[rt][nt], a, b0, b1);
-                                } else if (term + q > 0) {
+                                if (term + q > 0) {
                                     mma_bf16_acc(low[rt][nt], a, b0, b1);
                                 } else {
                                     float v[4] = {0.f, 0.f, 0.f, 0.f};
@@ -728,6 +711,11 @@ int32_t launch_cluster_z(void (*kernel)(KArgs...), dim3 grid, int threads, size_
     if (cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...) != cudaSuccess) return B2MOE_ERR_CUDA;
     return launch_status();
 }
+}  // namespace
+}  // namespace b2
+#include "router_tc.cuh"
+namespace b2 {
+namespace {
 template <int DT>
 int32_t router_launch(const float * w, const float * shared, const void * xv, float * logits, int ld, int h, int e, int rows, int n, cudaStream_t s) {
     const auto * x = static_cast<const typename Elem<DT>::type *>(xv);
@@ -735,13 +723,19 @@ int32_t router_launch(const float * w, const float * shared, const void * xv, fl
     int ks = 1;
     while (ks < 4 && h % (32 * ks) == 0 && h / (2 * ks) >= 256) ks *= 2;
     auto mma_blocks = [&](int tokens) { return (long long)ceil_div(rows, 16) * ceil_div(n, tokens) * ks; };
-    // Tiles from 256 tokens for bf16 (below, router_mma_k has more blocks and no stage hand-offs). fp16 and fp32 rows: once router_mma_k
-    // with its 64 tokens a block has more than two blocks per SM. router_mma_k / tiles, us: 1024 columns x 32 experts, fp16,
+    // 16-bit rows go to router_tc_k where router_mma_k, with its 64 tokens a block, has more than two blocks per SM, or more than one and enough rows to fill most of a tile of
+    // 128. Before / router_tc_k, us: bf16 2048 columns x 512 experts, 256 tokens 17.8 / 10.1, 509 23.5 / 11.2, 4096 87 / 32; 4096 x 128, 8192 tokens 163 / 40; 3072 x 256, 2047
+    // tokens 57 / 20; fp16 600 x 3072 x 256 32 / 16.5, 4096 x 2048 x 512 187 / 77, 600 x 2560 x 60 (160 blocks) 21.9 / 14.7, 4096 x 5120 x 16 (256 blocks of 16 rows) 31 / 72. Not where
+    // the other kernels are more precise (2-norm against fp64): bf16 below 256 tokens (1.3e-7 to 2.2e-7, here 4.7e-7), fp16 below 768 columns (6.9e-8, here 8.0e-8; from there on 8.1e-8 to 1.04e-7).
+    // Rows of fp32, and short ones of fp16: tiles once router_mma_k has more than two blocks per SM. router_mma_k / tiles, us: 1024 columns x 32 experts, fp16,
     // 600 tokens 8.9 / 17.7, 2047 (256 blocks) 16.8 / 18.0, 4096 (512 blocks) 32 / 18; 2560 x 60, 600 tokens (160) 22.8 / 31, 2047 (512) 46 / 32;
     // 3072 x 256, 256 tokens (256) 25 / 31, 300 (320) 36 / 31; 256 x 32 4096 tokens (128) 8.3 / 22.
     // A grid holds 65,535 blocks of tokens; what is more than that many takes the scalar loop, as everything else that does not fit.
     constexpr int GRID_Y = 65535;
-    if (h % RT_K == 0 && (DT == B2MOE_BF16 ? n >= 2 * RT_TOK : mma_blocks(64) > 2 * ROUTER_SMS) && ceil_div(n, RT_TOK) <= GRID_Y) {
+    if constexpr (DT != B2MOE_F32)
+        if (h % RT_K == 0 && (mma_blocks(64) > 2 * ROUTER_SMS || (mma_blocks(64) > ROUTER_SMS && rows > 48)) && (DT == B2MOE_F16 ? h >= 768 : n >= 256))
+            return rtc::launch<DT>(w, shared, x, logits, ld, h, e, rows, n, s);
+    if constexpr (DT != B2MOE_BF16) if (h % RT_K == 0 && mma_blocks(64) > 2 * ROUTER_SMS && ceil_div(n, RT_TOK) <= GRID_Y) {
         const dim3 tiles(ceil_div(rows, RT_ROWS), ceil_div(n, RT_TOK), 1);
         const int n_part = ceil_div(h, RT_COLS), share = ceil_div(n_part, 8), ks = ceil_div(n_part, share);      // at most eight blocks, no more than the shares need
         const size_t smem = rt_stages_bytes<DT>() + size_t(share - 1) * RT_PART;

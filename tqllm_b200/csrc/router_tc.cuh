@@ -1,0 +1,424 @@
+// Router logits of many 16-bit rows on the 5th-generation tensor cores (included by route.cu).
+//
+// logits[t][r] = sum_k W[r][k] x[t][k], W fp32. A block takes 128 router rows (M) x NT tokens (N):
+//   B: the activation rows as they are (bf16 or fp16), 64 columns a step, one TMA box in the 128-byte swizzled form;
+//   A: the router rows split exactly into three 16-bit terms, written to TENSOR MEMORY. TMA brings 64 fp32 columns of them a step, a thread splits half a row
+//      of it. bf16 rows: hi + mid + lo are bf16. fp16 rows: fp16 terms of the 32 values times a power of two that brings their largest magnitude into
+//      [2^14, 2^15) (what is below 2^-39 of it is lost), and the sums of the half step times its inverse.
+// So every product is exact in fp32 and three products do for either type (two bf16 terms of an fp16 activation would take six).
+//
+// Numerics. The tensor core cuts its running sums off, always towards zero: 1.7e-8 of the sum per product that meets it. bf16 rows: the leading products of a part of 512 columns
+// are one chain of 32, the others (2^-8 of them and less) have sums of their own; the parts are added in column order. fp16 rows: one chain per half
+// step, smallest terms first (two of its six products meet a sum of full size); half steps and parts are added in fp32 with the rounding errors carried along.
+//
+// What bounds it: the chain from a step's copy over its split to the products, 1650 cycles a step of 128 bf16 tokens, 1080 of 64, 2100 of 64 fp16 tokens (most of it the split by two warps a
+// scheduler), where the products alone take 768 and 516. Two groups of splitting warps on steps in turn: 34.2 us against 31.9 (4096 x 2048 x 512 bf16; three stages instead of four for it); the
+// router rows loaded straight from global memory into fragments, no shared memory: 39.0; one accumulator for all terms: 24.9, at 1.65e-6 (this 4.7e-7).
+// A launch with few tiles would leave SMs idle: the blocks of a cluster take parts of a tile's columns each, and
+// add them in column order through distributed shared memory, so neither the split nor NT changes a bit.
+// Every wait is bounded; where one runs out, the logits of the tile become NaN (fp16 rows: are summed again in a plain loop).
+#pragma once
+#include "tc_ptx.cuh"
+#include "tensor_map.cuh"
+
+namespace b2 {
+namespace {
+namespace rtc {
+using namespace tc;
+
+constexpr int ROWS = 128, STEP = 64, PART_STEPS = 8, MAX_PARTS = 16;
+// Warps: 0 copies, 1 issues, 4 .. 11 split, the others read the sums; roles begin at multiples of four: a TMEM lane quarter each
+constexpr int TMA_WARP = 0, MMA_WARP = 1, CONV_WARP0 = 4, EPI_WARP0 = 12, EPI_WARPS = 16, THREADS = (EPI_WARP0 + EPI_WARPS) * 32;
+// Tensor memory. bf16: the sums of the leading products, those of the others; fp16: two sets of two (the halves of a step), a step each in turn. Then A, two steps of two
+// halves: three terms of 32 columns (16 of tensor memory) each
+constexpr int ACC = 128, A_COL0 = 2 * ACC, A_TERM = 16, A_HALF = 3 * A_TERM, A_STAGE = 2 * A_HALF;
+constexpr int SCALE_STEPS = 4;                                         // steps whose scales the epilogue may still need
+constexpr int W_BYTES = ROWS * STEP * 4, GATE_BYTES = STEP * 4;
+constexpr int stage_bytes(int nt) { return W_BYTES + nt * STEP * 2; }
+constexpr int part_bytes(int nt) { return nt * ROWS * 4; }                       // a tile's sums, [token][row]
+// Tiles of sums beside the stages. SPLIT: the first of a block's two parts; else bf16: none (totals in registers), fp16: the parts so far. fp16: behind a tile what its sums lack
+template <int DT, bool SPLIT> constexpr int part_tiles() { return DT == B2MOE_F16 ? 2 : SPLIT ? 1 : 0; }
+template <int DT, bool SPLIT> constexpr int stages() { return part_tiles<DT, SPLIT>() ? 3 : 4; }
+constexpr int N_BARS = 2 * 4 + 2 + 2 + 2 + SCALE_STEPS + 1;
+template <int DT, bool SPLIT> constexpr size_t smem_bytes(int nt) {
+    return 1024 + size_t(stages<DT, SPLIT>()) * (stage_bytes(nt) + GATE_BYTES) + part_tiles<DT, SPLIT>() * part_bytes(nt) + SCALE_STEPS * 2 * ROWS * 4 + N_BARS * 8 + 16;
+}
+static_assert(smem_bytes<B2MOE_BF16, false>(128) <= 227 * 1024 && smem_bytes<B2MOE_BF16, true>(128) <= 227 * 1024 && smem_bytes<B2MOE_F16, true>(64) <= 227 * 1024 &&
+              3 * stage_bytes(64) >= 2 * part_bytes(64) && 3 * stage_bytes(128) >= part_bytes(128));
+
+// two fp32 operations in one instruction
+__device__ __forceinline__ unsigned long long bits2(float2 v) { return (unsigned long long)(__float_as_uint(v.y)) << 32 | __float_as_uint(v.x); }
+__device__ __forceinline__ float2 pair_of(uint32_t x, uint32_t y) { return make_float2(__uint_as_float(x), __uint_as_float(y)); }
+__device__ __forceinline__ float2 of_bits2(unsigned long long v) { return pair_of(uint32_t(v), uint32_t(v >> 32)); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { unsigned long long r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits2(a)), "l"(bits2(b))); return of_bits2(r); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { unsigned long long r; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits2(a)), "l"(bits2(b))); return of_bits2(r); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { unsigned long long r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits2(a)), "l"(bits2(b))); return of_bits2(r); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { unsigned long long r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(bits2(a)), "l"(bits2(b)), "l"(bits2(c))); return of_bits2(r); }
+
+// the two values' terms, largest first, as a pair of 16-bit values each
+template <int DT> __device__ __forceinline__ void split_terms(float2 w, uint32_t (&v)[3]) {
+    if constexpr (DT == B2MOE_BF16) {
+        // by cutting off: 8 of the 24 bits each (an infinity leaves NaN behind, as rounding would)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const uint32_t a = __float_as_uint(w.x), b = __float_as_uint(w.y);
+            v[i] = __byte_perm(a, b, 0x7632);
+            if (i < 2) w = sub2(w, pair_of(a & 0xffff0000u, b & 0xffff0000u));
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const __half2 h = __floats2half2_rn(w.x, w.y);
+            v[i] = *reinterpret_cast<const uint32_t *>(&h);
+            if (i < 2) w = sub2(w, __half22float2(h));
+        }
+    }
+}
+// (v, lack) += (sum, lack_sum), the sums so far: plainly, or with the addition's rounding error put into what the sum lacks
+template <bool EXACT> __device__ __forceinline__ void add_part(float & v, float & lack, float sum, float lack_sum) {
+    const float t = sum + v;
+    if (EXACT) {
+        const float z = t - sum;
+        lack += ((sum - (t - z)) + (v - z)) + lack_sum;
+    }
+    v = t;
+}
+struct Maps { CUtensorMap w, x, gate; };
+
+template <int DT, int NT, bool SPLIT>
+__global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const float * shared, const typename Elem<DT>::type * x, float * logits, int ld, int h, int e, int rows,
+                                                          int n, const __grid_constant__ Maps maps) {
+    namespace cg = cooperative_groups;
+    constexpr bool F16 = DT == B2MOE_F16;
+    constexpr int S = stages<DT, SPLIT>();
+    extern __shared__ uint8_t rtc_raw[];
+    uint8_t * smem = rtc_raw + (-saddr(rtc_raw) & 1023u);
+    const int ks = gridDim.z, n_part = (h + STEP * PART_STEPS - 1) / (STEP * PART_STEPS);
+    auto first_part = [&](int z) { return n_part * z / ks; };
+    const int p_lo = first_part(blockIdx.z), np = first_part(blockIdx.z + 1) - p_lo;
+    const int s_lo = p_lo * PART_STEPS, steps = min((h + STEP - 1) / STEP, (p_lo + np) * PART_STEPS) - s_lo;      // this block's steps
+    // see part_tiles; SPLIT: the last part takes the stages' place
+    uint8_t * parts = smem + S * stage_bytes(NT);
+    float * gate = reinterpret_cast<float *>(parts + part_tiles<DT, SPLIT>() * part_bytes(NT));      // [stages][64]: the shared expert's gate, router row e
+    float * scales = gate + S * STEP;                                   // [steps][halves][row]
+    const uint32_t full = saddr(scales + SCALE_STEPS * 2 * ROWS), done = full + 8 * S, a_full = done + 8 * S, acc_full = a_full + 16,
+                   acc_empty = acc_full + 16, sc_full = acc_empty + 16, drain = sc_full + 8 * SCALE_STEPS;
+    uint32_t * tmem_slot = reinterpret_cast<uint32_t *>(scales + SCALE_STEPS * 2 * ROWS) + 2 * N_BARS;
+    volatile int * gave_up = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int r0 = blockIdx.y * ROWS, t0 = blockIdx.x * NT;                  // tokens on gridDim.x: any batch size
+    const bool has_gate = rows > e && r0 + ROWS > e;                    // the tile holds row e
+
+    if (tid == 0) {
+#pragma unroll 1
+        for (int i = 0; i < S; ++i) { bar_init(full + 8 * i, 1); bar_init(done + 8 * i, 1); }
+#pragma unroll 1
+        for (int i = 0; i < 2; ++i) { bar_init(a_full + 8 * i, 8); bar_init(acc_full + 8 * i, 1); bar_init(acc_empty + 8 * i, EPI_WARPS); }
+#pragma unroll 1
+        for (int i = 0; i < SCALE_STEPS; ++i) bar_init(sc_full + 8 * i, 8);
+        bar_init(drain, 1);
+        *gave_up = 0;
+        bar_init_fence();
+    }
+    if (warp == MMA_WARP) tmem_alloc(saddr(tmem_slot), 512);            // all columns: they begin at column 0
+    grid_release();
+    grid_wait();                                                       // x may be the output of the launch before this one
+    fence_before();
+    __syncthreads();
+    fence_after();
+    constexpr uint32_t tmem = 0;
+
+    if (warp == TMA_WARP) {
+        if (elect_one()) {
+            bool ok = true;
+            int g = 0;
+#pragma unroll 1
+            for (; g < steps; ++g) {
+                if (g >= S && !bar_wait(done + 8 * ((g - S) % S), uint32_t((g - S) / S) & 1u)) { ok = false; break; }
+                const uint32_t bar = full + 8 * (g % S), dst = saddr(smem) + (g % S) * stage_bytes(NT);
+                const int k0 = (s_lo + g) * STEP;
+                bar_expect_tx(bar, stage_bytes(NT) + (has_gate ? GATE_BYTES : 0));
+                tma_load_2d(dst, &maps.w, k0, r0, bar);                 // what lies outside (rows, columns, tokens) arrives as zeros
+                tma_load_2d(dst + W_BYTES / 2, &maps.w, k0 + 32, r0, bar);
+                tma_load_2d(dst + W_BYTES, &maps.x, k0, t0, bar);
+                if (has_gate) tma_load_2d(saddr(gate) + (g % S) * GATE_BYTES, &maps.gate, k0, 0, bar);
+            }
+            if (!ok) *gave_up = 1;
+            // before leaving, every copy must have landed (after a clean run these waits return at once)
+#pragma unroll 1
+            for (int i = max(0, g - S); i < g; ++i) bar_wait(full + 8 * (i % S), uint32_t(i / S) & 1u);
+        }
+        __syncwarp();
+    } else if (warp == MMA_WARP) {
+        if (elect_one()) {
+            bool ok = true;
+            const uint32_t id = idesc(128, NT, F16 ? 0 : 1);
+#pragma unroll 1
+            for (int g = 0; g < steps; ++g) {
+                const int set = g & 1;
+                const uint32_t a = tmem + A_COL0 + set * A_STAGE, b = sw128_desc_lo(saddr(smem) + (g % S) * stage_bytes(NT) + W_BYTES);
+                // half hf's product number k with term t
+                auto mma = [&](uint32_t d, int hf, int t, int k, bool acc) { mma_f16(d, a + hf * A_HALF + t * A_TERM + 8 * k, b + 4 * hf + 2 * k, id, acc); };
+                if (!bar_wait(full + 8 * (g % S), uint32_t(g / S) & 1u) || !bar_wait(a_full + 8 * set, uint32_t(g >> 1) & 1u)) { ok = false; break; }
+                if constexpr (F16) {
+                    if (g > 1 && !bar_wait(acc_empty + 8 * set, uint32_t((g >> 1) - 1) & 1u)) { ok = false; break; }
+                    fence_after();
+#pragma unroll
+                    for (int hf = 0; hf < 2; ++hf)                     // a half step has sums of its own
+#pragma unroll
+                        for (int t = 2; t >= 0; --t) { mma(tmem + set * ACC + hf * NT, hf, t, 0, t < 2); mma(tmem + set * ACC + hf * NT, hf, t, 1, true); }
+                    mma_commit(acc_full + 8 * set);
+                } else {
+                    const int p = g / PART_STEPS;
+                    const bool more = g % PART_STEPS > 0;
+                    if (!more && p > 0 && !bar_wait(acc_empty, uint32_t(p - 1) & 1u)) { ok = false; break; }
+                    fence_after();
+#pragma unroll
+                    for (int hf = 0; hf < 2; ++hf) {
+                        mma(tmem + ACC, hf, 2, 0, more || hf > 0); mma(tmem + ACC, hf, 1, 0, true); mma(tmem + ACC, hf, 2, 1, true); mma(tmem + ACC, hf, 1, 1, true);
+                        mma(tmem, hf, 0, 0, more || hf > 0); mma(tmem, hf, 0, 1, true);
+                    }
+                    if (g % PART_STEPS == PART_STEPS - 1 || g + 1 == steps) mma_commit(acc_full);
+                }
+                mma_commit(done + 8 * (g % S));
+            }
+            if (!ok) *gave_up = 1;
+            mma_commit(drain);                                         // nothing may be in flight when the tensor memory is freed
+            bar_wait(drain, 0);
+        }
+        __syncwarp();
+    } else if (warp >= CONV_WARP0 && warp < EPI_WARP0) {
+        // ---- warps (half, quarter q): rows 32 q .. + 31 of the tile, a lane each; that half of every step ----
+        const int q = warp & 3, hf = (warp - CONV_WARP0) >> 2, row = 32 * q + lane;
+        const bool is_gate = has_gate && r0 + row == e;
+        const uint32_t xr = is_gate ? 0u : uint32_t(row & 7) << 4;      // the 128-byte swizzle of the row's 16-byte pieces
+        const uint32_t src0 = is_gate ? saddr(gate) + 128 * hf : saddr(smem) + hf * (W_BYTES / 2) + row * 128, src_step = is_gate ? GATE_BYTES : stage_bytes(NT);
+        bool ok = true;
+#pragma unroll 1
+        for (int g = 0; g < steps; ++g) {
+            const int s = g % S;
+            const uint32_t to = tmem + (uint32_t(32 * q) << 16) + A_COL0 + (g & 1) * A_STAGE + hf * A_HALF;
+            if (!warp_wait(full + 8 * (g % S), uint32_t(g / S) & 1u)) { ok = false; break; }
+            float v[32];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[4 * i]), "=f"(v[4 * i + 1]), "=f"(v[4 * i + 2]), "=f"(v[4 * i + 3])
+                             : "r"(src0 + s * src_step + (uint32_t(16 * i) ^ xr)) : "memory");
+            [[maybe_unused]] float up = 1.f;
+            if constexpr (F16) {
+                float most = 0.f;
+#pragma unroll
+                for (int i = 0; i < 32; ++i) most = fmaxf(most, fabsf(v[i]));
+                int ex = int(__float_as_uint(most) >> 23) - 127;        // floor(log2(most)) for a normal number
+                ex = most > 0.f && most < 3e38f ? max(-100, min(100, ex)) : 14;
+                up = __uint_as_float(uint32_t(127 + 14 - ex) << 23);
+            }
+            uint32_t t[3][16];
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+                uint32_t u[3];
+                split_terms<DT>(F16 ? mul2(make_float2(v[2 * c], v[2 * c + 1]), make_float2(up, up)) : make_float2(v[2 * c], v[2 * c + 1]), u);
+                t[0][c] = u[0]; t[1][c] = u[1]; t[2][c] = u[2];
+            }
+            if (g > 1 && !warp_wait(done + 8 * ((g - 2) % S), uint32_t((g - 2) / S) & 1u)) { ok = false; break; }      // the products of the step that had the place
+            fence_after();
+            // (the scale's place was that of four steps before: the products of two before have waited until the epilogue was done with those)
+            if (F16) scales[((g & (SCALE_STEPS - 1)) * 2 + hf) * ROWS + row] = __uint_as_float(0x7F000000u - __float_as_uint(up));      // 1 / up
+#pragma unroll
+            for (int c = 0; c < 3; ++c) tmem_st16(to + c * A_TERM, t[c]);
+            tmem_st_wait();
+            fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                bar_arrive(a_full + 8 * (g & 1));
+                if (F16) bar_arrive(sc_full + 8 * (g & (SCALE_STEPS - 1)));
+            }
+        }
+        if (!ok && lane == 0) *gave_up = 1;
+    } else if (warp >= EPI_WARP0) {
+        // ---- warps q, q + 4, ..: the sums of rows 32 q .. + 31, a lane each; a share of the tokens ----
+        constexpr int TOK = NT / (EPI_WARPS / 4);
+        const int q = warp & 3, tk0 = TOK * ((warp - EPI_WARP0) >> 2), row = 32 * q + lane;
+        const uint32_t from = tmem + (uint32_t(32 * q) << 16) + tk0;
+        float * const so_far = reinterpret_cast<float *>(parts) + tk0 * ROWS + row, * const last = reinterpret_cast<float *>(smem) + tk0 * ROWS + row;
+        const bool in = r0 + row < rows;
+        [[maybe_unused]] float tot[TOK];
+        bool ok = true;
+#pragma unroll 1
+        for (int p = 0; p < np && ok; ++p) {
+            const bool is_last = p + 1 == np;
+            // the finished sum of the part's i-th token (and what it lacks): SPLIT: put away; else added to those before it
+            auto put = [&](int i, float v, float lack = 0.f) {
+                if (SPLIT) {
+                    (is_last ? last : so_far)[i * ROWS] = v;
+                    if (F16) (is_last ? last : so_far)[(NT + i) * ROWS] = lack;
+                    return;
+                }
+                if (F16) {
+                    if (p > 0) add_part<true>(v, lack, so_far[i * ROWS], so_far[(NT + i) * ROWS]);
+                    if (!is_last) { so_far[i * ROWS] = v; so_far[(NT + i) * ROWS] = lack; }
+                } else {
+                    if (p > 0) v = tot[i] + v;
+                    tot[i] = v;
+                }
+                const int tok = t0 + tk0 + i;
+                if (is_last && in && tok < n) logits[size_t(tok) * ld + r0 + row] = checked_logit<DT>(F16 ? v + lack : v, w, shared, x, r0 + row, tok, e, h);
+            };
+            if constexpr (F16) {
+                // The steps' sums are added with their rounding errors carried along (Kahan; lost: what the sum lacks): the plain additions of a part would be the largest error
+                float2 sum[TOK / 2], lost[TOK / 2];
+#pragma unroll
+                for (int i = 0; i < TOK / 2; ++i) sum[i] = lost[i] = make_float2(0.f, 0.f);
+                const int g_hi = min(steps, (p + 1) * PART_STEPS);
+#pragma unroll 1
+                for (int g = p * PART_STEPS; g < g_hi; ++g) {
+                    const int set = g & 1;
+                    if (!warp_wait(sc_full + 8 * (g & (SCALE_STEPS - 1)), uint32_t(g / SCALE_STEPS) & 1u)) { ok = false; break; }
+                    const float * sc = scales + (g & (SCALE_STEPS - 1)) * 2 * ROWS + row;
+                    const float2 sc0 = make_float2(sc[0], sc[0]), sc1 = make_float2(sc[ROWS], sc[ROWS]);
+                    if (!warp_wait(acc_full + 8 * set, uint32_t(g >> 1) & 1u)) { ok = false; break; }
+                    fence_after();
+#pragma unroll
+                    for (int c = 0; c < TOK; c += 8) {
+                        uint32_t v0[8], v1[8];
+                        tmem_ld8(from + set * ACC + c, v0);
+                        tmem_ld8(from + set * ACC + NT + c, v1);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            float2 & s2 = sum[c / 2 + i], & l2 = lost[c / 2 + i];
+                            const float2 y = fma2(pair_of(v0[2 * i], v0[2 * i + 1]), sc0, fma2(pair_of(v1[2 * i], v1[2 * i + 1]), sc1, l2)), t = add2(s2, y);
+                            l2 = sub2(y, sub2(t, s2));
+                            s2 = t;
+                        }
+                    }
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) bar_arrive(acc_empty + 8 * set);
+                }
+                if (!ok) break;
+#pragma unroll
+                for (int i = 0; i < TOK; ++i) put(i, i & 1 ? sum[i / 2].y : sum[i / 2].x, i & 1 ? lost[i / 2].y : lost[i / 2].x);
+            } else {
+                if (!warp_wait(acc_full, uint32_t(p) & 1u)) { ok = false; break; }
+                fence_after();
+#pragma unroll
+                for (int c = 0; c < TOK; c += 8) {
+                    uint32_t v0[8], v1[8];
+                    tmem_ld8(from + c, v0);
+                    tmem_ld8(from + ACC + c, v1);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) put(c + i, __uint_as_float(v0[i]) + __uint_as_float(v1[i]));
+                }
+                fence_before();
+                __syncwarp();
+                if (lane == 0) bar_arrive(acc_empty);
+            }
+        }
+        if (!ok) {
+            if (lane == 0) *gave_up = 1;
+            if (!SPLIT)
+#pragma unroll 1
+                for (int i = 0; i < TOK; ++i)
+                    if (in && t0 + tk0 + i < n) logits[size_t(t0 + tk0 + i) * ld + r0 + row] = checked_logit<DT>(CUDART_NAN_F, w, shared, x, r0 + row, t0 + tk0 + i, e, h);
+        }
+    }
+    fence_before();
+    __syncthreads();
+    if (warp == MMA_WARP) tmem_free(tmem, 512);
+    if constexpr (SPLIT) {
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();
+        // every block of the cluster finishes a share of the tile's tokens; where the parts lie in the cluster's shared memory comes from a table
+        __shared__ uint32_t place[MAX_PARTS];
+        __shared__ int bad;
+        if (tid == 0) bad = 0;
+        __syncthreads();
+        if (tid < n_part) {
+            int z = 0;
+            while (first_part(z + 1) <= tid) ++z;
+            const int i = tid - first_part(z), last = first_part(z + 1) - first_part(z) - 1;
+            const uint32_t local = i < last ? saddr(parts) : saddr(smem);
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(place[tid]) : "r"(local), "r"(z));
+            uint32_t flag;
+            int v;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(flag) : "r"(saddr(const_cast<const int *>(gave_up))), "r"(z));
+            asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(flag) : "memory");
+            if (v) bad = 1;
+        }
+        __syncthreads();
+        const int lo = NT * int(blockIdx.z) / ks, hi = NT * (int(blockIdx.z) + 1) / ks;
+#pragma unroll 1
+        for (int i = tid; i < (hi - lo) * ROWS; i += THREADS) {
+            const int tk = lo + i / ROWS, r = i % ROWS;
+            if (t0 + tk >= n || r0 + r >= rows) continue;
+            const uint32_t off = uint32_t(tk * ROWS + r) * 4u;
+            float sum = 0.f, lack = 0.f;
+#pragma unroll 1
+            for (int q = 0; q < n_part; q += 4) {
+                float v[4], l[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    v[j] = l[j] = 0.f;
+                    if (q + j < n_part) {
+                        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[j]) : "r"(place[q + j] + off) : "memory");
+                        if (F16) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(l[j]) : "r"(place[q + j] + off + part_bytes(NT)) : "memory");
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (q + j < n_part) {
+                        if (q + j > 0) add_part<F16>(v[j], l[j], sum, lack);
+                        sum = v[j];
+                        lack = l[j];
+                    }
+            }
+            logits[size_t(t0 + tk) * ld + r0 + r] = checked_logit<DT>(bad ? CUDART_NAN_F : F16 ? sum + lack : sum, w, shared, x, r0 + r, t0 + tk, e, h);
+        }
+        cluster.sync();                                                // the blocks' tiles stay alive until every block has read them
+    }
+}
+
+// The shape of a launch: tokens a block and blocks a tile's columns are split over, the pair with the fewest cycles
+struct Shape { int nt, ks, share; };
+template <int DT> Shape shape_of(int rows, int n, int h) {
+    const int parts = ceil_div(h, STEP * PART_STEPS);
+    Shape best{0, 1, parts};
+    long long least = 0;
+    for (int nt = DT == B2MOE_F16 ? 64 : 128; nt >= 64; nt -= 64) {
+        const long long tiles = (long long)ceil_div(rows, ROWS) * ceil_div(n, nt);
+        for (int share = parts; share >= 1; --share) {
+            const int ks = ceil_div(parts, share);
+            if (ks > 8 || (ks > 1 && (share > 2 || parts > MAX_PARTS))) continue;
+            // cycles of a part (measured), of a block's start and end, and of the meeting in a cluster
+            const long long part = PART_STEPS * (DT == B2MOE_F16 ? 2100 : nt == 128 ? 1650 : 1080), cost = (tiles * ks + 147) / 148 * (share * part + 6000) + (ks > 1 ? 2000 : 0);
+            if (best.nt == 0 || cost < least) { best = Shape{nt, ks, share}; least = cost; }
+        }
+    }
+    return best;
+}
+template <int DT, int NT> int32_t launch_nt(const Shape & p, const float * w, const float * shared, const typename Elem<DT>::type * x, float * logits, int ld, int h, int e,
+                                            int rows, int n, cudaStream_t s) {
+    Maps maps;
+    const cuuint64_t xd[2] = {cuuint64_t(h), cuuint64_t(n)}, wd[2] = {cuuint64_t(h), cuuint64_t(e)}, gd[2] = {cuuint64_t(h), 1}, xs[1] = {cuuint64_t(h) * 2}, ws[1] = {cuuint64_t(h) * 4};
+    const cuuint32_t xb[2] = {STEP, NT}, wb[2] = {STEP / 2, ROWS}, gb[2] = {STEP, 1};
+    if (!encode_map(maps.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x, xd, xs, xb, CU_TENSOR_MAP_SWIZZLE_128B) ||       // (copied as they are: bf16 is as good)
+        !encode_map(maps.w, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, w, wd, ws, wb, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !encode_map(maps.gate, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, shared ? shared : w, gd, ws, gb, CU_TENSOR_MAP_SWIZZLE_NONE)) return B2MOE_ERR_CUDA;
+    const size_t smem = p.ks > 1 ? smem_bytes<DT, true>(NT) : smem_bytes<DT, false>(NT);
+    const auto kernel = p.ks > 1 ? router_tc_k<DT, NT, true> : router_tc_k<DT, NT, false>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return B2MOE_ERR_CUDA;
+    return launch_cluster_z(kernel, dim3(ceil_div(n, NT), ceil_div(rows, ROWS), p.ks), THREADS, smem, s, w, shared, x, logits, ld, h, e, rows, n, maps);
+}
+// 16-bit rows; h a multiple of 8 (strides of the maps)
+template <int DT> int32_t launch(const float * w, const float * shared, const typename Elem<DT>::type * x, float * logits, int ld, int h, int e, int rows, int n, cudaStream_t s) {
+    const Shape p = shape_of<DT>(rows, n, h);
+    if constexpr (DT == B2MOE_BF16)
+        if (p.nt == 128) return launch_nt<DT, 128>(p, w, shared, x, logits, ld, h, e, rows, n, s);
+    return launch_nt<DT, 64>(p, w, shared, x, logits, ld, h, e, rows, n, s);
+}
+
+}  // namespace rtc
+}  // namespace
+}  // namespace b2
