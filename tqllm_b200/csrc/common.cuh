@@ -20,7 +20,8 @@ inline int32_t launch_status() {
 // memory setup, no global access) and then every thread calls grid_wait(), which returns once the earlier launches have
 // completed and their writes are visible. grid_release() lets the launch after this one do the same. A kernel that is
 // launched this way must call grid_wait() in every thread before its first global access and before any early return,
-// so that completion stays transitive along the chain. What an earlier launch writes is read through plain pointers there: a load
+// so that completion stays transitive along the chain (the expert products read the plan and the weights above it where they can know both to be complete: expert_down in
+// layer.cu, rows_begin in expert_gemm_tc.cu). What an earlier launch writes is read through plain pointers there: a load
 // from a `const T * __restrict__` parameter counts as a load of memory that nobody changes, and the compiler moves it above the
 // wait (seen: a whole index array read before it was written). g_overlap = false (b2moe_harness_overlap) falls back to plain launches.
 extern bool g_overlap;

@@ -26,7 +26,7 @@ int32_t route_plan_stage(int gating, const float * logits, int ld, const float *
                          int experts, int topk, int norm, float scale, int n, int shared_first, int shared_count, int * plan, const void * x,
                          int x_dtype, int k, int bits, uint8_t * staged_rows, float * inv_scale, cudaStream_t s, bool * took);
 int32_t dec4_down(const b2moe_bank *, const b2moe_bank *, const void *, int x_dtype, bool per_token, const int *, int, int, int, void *, int y_dtype, void *,
-                  cudaStream_t);
+                  cudaStream_t, bool plan_ready);
 void dec4_debug(int drop_tile, uint32_t wait_limit);
 void dec4_skip_staging(bool on);
 void dec4_ring(int nbuf, int stages, int slot_tiles);
@@ -39,13 +39,13 @@ size_t gemm_tc_slot_bytes(int slot_rows, int k);
 int32_t gemm_tc_gateup(const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const void *, int, const int *, int,
                        int, int, long long live, void *, int act_dtype, void *, void * rows_buf, size_t rows_buf_bytes, cudaStream_t);
 int32_t gemm_tc_down(const b2moe_bank *, const b2moe_bank *, const void *, int x_dtype, bool per_token, const int *, int, int, int, long long live, void *,
-                     int y_dtype, void *, cudaStream_t);
+                     int y_dtype, void *, bool plan_ready, cudaStream_t);
 void gemm_tc_item_tokens(int tokens);
 bool gemm_exact_supported(uint32_t type, int k, int experts);
 size_t gemm_exact_bytes(int slot_rows, int k, int dtype);
 int32_t gemm_exact_gateup(const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const void *, int, const int *, int, int, int, void *, int act_dtype,
                           void * rows, bool slots, cudaStream_t);
-int32_t gemm_exact_down(const b2moe_bank *, const b2moe_bank *, const void *, int, bool per_token, const int *, int, int, int, void *, int y_dtype, void * rows, cudaStream_t);
+int32_t gemm_exact_down(const b2moe_bank *, const b2moe_bank *, const void *, int, bool per_token, const int *, int, int, int, void *, int y_dtype, void * rows, bool plan_ready, cudaStream_t);
 
 namespace {
 int32_t same_shape(const b2moe_bank * a, const b2moe_bank * b, bool same_experts) {
@@ -114,10 +114,10 @@ int32_t product_typed(const b2moe_bank * m, const void * x, int x_dtype, bool pe
     const int path = expert_path(m->type, m->cols, B2MOE_F32, m->experts, (long long)n * topk);
     *took = true;
     if (exact_path(m->type, m->cols, x_dtype, m->experts, (long long)n * topk) && rows_buf_bytes >= gemm_exact_bytes(n * topk, m->cols, x_dtype))
-        return gemm_exact_down(m, nullptr, x, x_dtype, per_token, plan, n, topk, 0, y, y_dtype, rows_buf, s);
-    if (path == B2MOE_FAMILY_GEMM) return gemm_tc_down(m, nullptr, x, x_dtype, per_token, plan, n, topk, 0, (long long)n * topk, y, y_dtype, ws, s);
+        return gemm_exact_down(m, nullptr, x, x_dtype, per_token, plan, n, topk, 0, y, y_dtype, rows_buf, false, s);
+    if (path == B2MOE_FAMILY_GEMM) return gemm_tc_down(m, nullptr, x, x_dtype, per_token, plan, n, topk, 0, (long long)n * topk, y, y_dtype, ws, false, s);
     if (path == B2MOE_FAMILY_DECODE && decode_kernel(m->type, m->cols, B2MOE_F32) == DEC_4BIT)
-        return dec4_down(m, nullptr, x, x_dtype, per_token, plan, n, topk, 0, y, y_dtype, ws, s);
+        return dec4_down(m, nullptr, x, x_dtype, per_token, plan, n, topk, 0, y, y_dtype, ws, s, false);
     *took = false;
     return B2MOE_OK;
 }
@@ -243,8 +243,10 @@ extern "C" B2MOE_API int32_t b2moe_expert_gateup_swiglu(const b2moe_bank * gate,
     return expert_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, workspace, workspace_bytes, stream, false);
 }
 
+// plan_ready: the launch before this call's is a gate/up product over the same plan. Every kernel of that product waits for the launches before it and only then (when
+// its own work is done) lets the next one begin, so whatever begins here finds the plan complete and may ask for weights before it waits
 static int32_t expert_down(const b2moe_bank * down, const b2moe_bank * shared_down, const float * act, const int32_t * plan, int32_t n, int32_t topk,
-                           int32_t shared_tokens, float * y, void * workspace, size_t workspace_bytes, b2moe_stream stream, long long live) {
+                           int32_t shared_tokens, float * y, void * workspace, size_t workspace_bytes, b2moe_stream stream, long long live, bool plan_ready = false) {
     if (int32_t rc = check_bank(down)) return rc;
     if (n <= 0 || topk <= 0 || (shared_tokens != 0 && shared_tokens != n)) return B2MOE_ERR_SHAPE;
     if (shared_tokens) {
@@ -261,11 +263,11 @@ static int32_t expert_down(const b2moe_bank * down, const b2moe_bank * shared_do
         if (!aligned16(workspace)) return B2MOE_ERR_ALIGN;
         if (workspace_bytes < b2moe_expert_workspace_bytes(down->type, rows_x, down->cols, B2MOE_F32)) return B2MOE_ERR_WORKSPACE;
         if (exact_path(down->type, down->cols, B2MOE_F32, down->experts, live) && workspace_bytes >= gemm_exact_bytes(rows_x, down->cols, B2MOE_F32))
-            return gemm_exact_down(down, shared_down, act, B2MOE_F32, false, plan, n, topk, shared_tokens, y, B2MOE_F32, workspace, as_stream(stream));
+            return gemm_exact_down(down, shared_down, act, B2MOE_F32, false, plan, n, topk, shared_tokens, y, B2MOE_F32, workspace, plan_ready, as_stream(stream));
         if (path == B2MOE_FAMILY_GEMM)
-            return gemm_tc_down(down, shared_down, act, B2MOE_F32, false, plan, n, topk, shared_tokens, live, y, B2MOE_F32, workspace, as_stream(stream));
+            return gemm_tc_down(down, shared_down, act, B2MOE_F32, false, plan, n, topk, shared_tokens, live, y, B2MOE_F32, workspace, plan_ready, as_stream(stream));
         if (decode_kernel(down->type, down->cols, B2MOE_F32) == DEC_4BIT)
-            return dec4_down(down, shared_down, act, B2MOE_F32, false, plan, n, topk, shared_tokens, y, B2MOE_F32, workspace, as_stream(stream));
+            return dec4_down(down, shared_down, act, B2MOE_F32, false, plan, n, topk, shared_tokens, y, B2MOE_F32, workspace, as_stream(stream), plan_ready);
         return iq3s_down(down, shared_down, act, plan, n, topk, shared_tokens, y, workspace, max_active_of(down->experts, n, topk, shared_tokens), as_stream(stream));
     }
     return generic_down(down, shared_down, act, plan, n, topk, shared_tokens, y, as_stream(stream));
@@ -385,7 +387,7 @@ static int32_t layer_forward(const b2moe_layer * L, const void * x, int32_t x_dt
     // converts its rows into y takes no other scratch) hold the gate/up product's activation rows
     if (int32_t rc = expert_gateup(&L->gate, &L->up, &L->sh_gate, &L->sh_up, x, x_dtype, plan, n, L->topk, sh, act, es, es_bytes, stream, x_staged, -1, y,
                                    workspace_bytes - ws.y)) return rc;
-    if (int32_t rc = b2moe_expert_down(&L->down, &L->sh_down, act, plan, n, L->topk, sh, y, es, es_bytes, stream)) return rc;
+    if (int32_t rc = expert_down(&L->down, &L->sh_down, act, plan, n, L->topk, sh, y, es, es_bytes, stream, -1, true)) return rc;
     if (residual) return b2moe_combine_residual(y, nullptr, weights, gated_shared ? shw : nullptr, residual, n, L->topk, L->hidden, sh, out, out_dtype, stream);
     return b2moe_combine(y, nullptr, weights, gated_shared ? shw : nullptr, n, L->topk, L->hidden, sh, out, out_dtype, stream);
 }
