@@ -1,6 +1,6 @@
 // Weight decoders of the tensor-core grouped GEMM: one 64-column step of one 16-row bank tile -> fp16 A operand in registers.
-// A 256-column chunk has two units of two steps; a warp decodes both units of every other chunk: for u = 0, 1 prep<u>, then
-// step<u, 0>, step<u, 1>.
+// A 256-column chunk has four steps (two units of two); a warp decodes all of every other chunk: prep once, then for J = 0 .. 3 load<J> (what the
+// step needs from shared memory; the caller asks for it a step ahead) and step<J>.
 //
 // A warp owns a row tile; lane L = 4 g + t holds, in the bank's lane-major layout, the code words of rows g and g + 8
 // (formats.cuh). Every code word (or pair of IQ3_S grid entries) decodes to eight fp16 values, so a step leaves sixteen
@@ -79,48 +79,51 @@ template <> struct Dec<T_Q4_K> {
     __device__ __forceinline__ static uint32_t two(uint32_t n1024, __half2 S, __half2 NS, __half2 MH, __half2 ML, __half2 D) {
         return h2_bits(__hadd2(__hfma2(__hfma2(bits_h2(n1024), S, NS), D, MH), ML));
     }
-    // Once per unit: lane t of a row's four lanes turns the headers of its two rows into the constants of the unit's sub-block t
+    // Once per chunk: lane t of a row's four lanes turns the headers of its two rows into the constants of sub-blocks t and 4 + t
     // and leaves them in the warp's scratch, two in a word (the arithmetic takes either half of a register twice at no
-    // cost; spread there, they took twice the registers and loads): [row][sub-block]((S, -1024 S), (MH, ML)).
+    // cost; spread there, they took twice the registers and loads): [unit][row][sub-block]((S, -1024 S), (MH, ML)).
     // The scales and mins are exact as fp16, MH = fp16(-dmin m), ML = the exact rest. (Constants of two rows in one register,
     // fetched with shuffles and spread with byte permutes, took 45 more instructions a step, 36 of them in the integer pipe.)
-    static constexpr int SCRATCH = 16 * 4 * 8;
+    static constexpr int SCRATCH = 2 * 16 * 4 * 8;
     struct Pre { uint32_t D[2], magic; };
-    template <int u> __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t * scratch) {
+    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t * scratch) {
         const int g = lane >> 2, t = lane & 3;
         const uint4 h0 = *reinterpret_cast<const uint4 *>(chunk + 2048 + 16 * g), h1 = *reinterpret_cast<const uint4 *>(chunk + 2048 + 16 * (g + 8));    // d, dmin | s[12]
-        // the unit's four scales and four mins as bytes (src/formats/weight/dequant.cpp:56-64)
-        uint32_t sc0 = h0.y, mn0 = h0.z, sc1 = h1.y, mn1 = h1.z;
-        if (u) {
-            sc0 = (h0.w & 0x0F0F0F0Fu) | ((h0.y >> 2) & 0x30303030u); mn0 = ((h0.w >> 4) & 0x0F0F0F0Fu) | ((h0.z >> 2) & 0x30303030u);
-            sc1 = (h1.w & 0x0F0F0F0Fu) | ((h1.y >> 2) & 0x30303030u); mn1 = ((h1.w >> 4) & 0x0F0F0F0Fu) | ((h1.z >> 2) & 0x30303030u);
-        }
+        const __half2 dm = bits_h2(__byte_perm(h0.x, h1.x, 0x7632) ^ 0x80008000u);       // -dmin of the two rows
         const uint32_t sel = uint32_t(t) * 0x0101u + 0x0400u;               // selector nibbles 0 and 2: byte t of the first, of the second word
         auto pick = [&](uint32_t x, uint32_t y) {                            // byte t of either word, 16 bits apart, as fp16: 1024 + byte, then - 1024
             const uint32_t v = __byte_perm(x, y, sel);
             return __hadd2(bits_h2((v & 0x003F003Fu) | 0x64006400u), __float2half2_rn(-1024.f));
         };
-        __half2 sc = pick(sc0, sc1);
-        const __half2 mn = pick(mn0, mn1), dm = bits_h2(__byte_perm(h0.x, h1.x, 0x7632) ^ 0x80008000u);       // -dmin of the two rows
-        if (t & 1) sc = __hmul2(sc, __float2half2_rn(0.0625f));
-        const __half2 ns = __hmul2(sc, __float2half2_rn(-1024.f)), mh = __hmul2(dm, mn), ml = __hfma2(dm, mn, __hneg2(mh));
         uint2 * to = reinterpret_cast<uint2 *>(scratch) + 4 * g + t;
-        to[0] = make_uint2(h2_bits(__lows2half2(sc, ns)), h2_bits(__lows2half2(mh, ml)));
-        to[32] = make_uint2(h2_bits(__highs2half2(sc, ns)), h2_bits(__highs2half2(mh, ml)));
+        auto unit = [&](int u, uint32_t sc0, uint32_t mn0, uint32_t sc1, uint32_t mn1) {      // a unit's four scales and four mins as bytes
+            __half2 sc = pick(sc0, sc1);
+            const __half2 mn = pick(mn0, mn1);
+            if (t & 1) sc = __hmul2(sc, __float2half2_rn(0.0625f));
+            const __half2 ns = __hmul2(sc, __float2half2_rn(-1024.f)), mh = __hmul2(dm, mn), ml = __hfma2(dm, mn, __hneg2(mh));
+            to[64 * u] = make_uint2(h2_bits(__lows2half2(sc, ns)), h2_bits(__lows2half2(mh, ml)));
+            to[64 * u + 32] = make_uint2(h2_bits(__highs2half2(sc, ns)), h2_bits(__highs2half2(mh, ml)));
+        };
+        unit(0, h0.y, h0.z, h1.y, h1.z);                                     // (src/formats/weight/dequant.cpp:56-64)
+        unit(1, (h0.w & 0x0F0F0F0Fu) | ((h0.y >> 2) & 0x30303030u), ((h0.w >> 4) & 0x0F0F0F0Fu) | ((h0.z >> 2) & 0x30303030u),
+             (h1.w & 0x0F0F0F0Fu) | ((h1.y >> 2) & 0x30303030u), ((h1.w >> 4) & 0x0F0F0F0Fu) | ((h1.z >> 2) & 0x30303030u));
         return Pre{{__byte_perm(h0.x, 0u, 0x1010), __byte_perm(h1.x, 0u, 0x1010)}, in_register(0x64006400u)};
     }
-    template <int u, int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const void *, const uint8_t * scratch, const Pre & p, uint32_t (&f)[16]) {
-        const uint4 w4 = plane(chunk, 2 * u + JS, lane);
-        const uint4 * c = reinterpret_cast<const uint4 *>(scratch) + 2 * (lane >> 2) + JS;
+    struct Raw { uint4 w, c[2]; };                                           // code words; constants of both sub-blocks of row g, of row g + 8
+    template <int J> __device__ __forceinline__ static Raw load(const uint8_t * chunk, int lane, const uint8_t * scratch) {
+        const uint4 * c = reinterpret_cast<const uint4 *>(scratch) + 32 * (J >> 1) + 2 * (lane >> 2) + (J & 1);
+        return Raw{plane(chunk, J, lane), {c[0], c[16]}};
+    }
+    template <int J> __device__ __forceinline__ static void step(const Raw & raw, int, const void *, const Pre & p, uint32_t (&f)[16]) {
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-            const uint4 cc = c[16 * r];
+            const uint4 cc = raw.c[r];
             const __half2 D = bits_h2(p.D[r]);
             auto lo = [&](uint32_t w) { return two(and_or(w, 0x000F000Fu, p.magic), __low2half2(bits_h2(cc.x)), __high2half2(bits_h2(cc.x)), __low2half2(bits_h2(cc.y)), __high2half2(bits_h2(cc.y)), D); };
             auto hi = [&](uint32_t w) { return two(and_or(w, 0x00F000F0u, p.magic), __low2half2(bits_h2(cc.z)), __high2half2(bits_h2(cc.z)), __low2half2(bits_h2(cc.w)), __high2half2(bits_h2(cc.w)), D); };
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
-                const uint32_t v = r ? (b ? w4.w : w4.z) : (b ? w4.y : w4.x), v8 = v >> 8;
+                const uint32_t v = r ? (b ? raw.w.w : raw.w.z) : (b ? raw.w.y : raw.w.x), v8 = v >> 8;
                 // bytes 0 and 2, bytes 1 and 3: low nibbles, then high nibbles
                 put(f, r, b, make_uint4(lo(v), lo(v8), hi(v), hi(v8)));
             }
@@ -140,33 +143,39 @@ template <> struct Dec<T_IQ3S4> {
         return bits_h2(and_or(POS <= 6 ? w << (6 - POS) : w >> (POS - 6), 0x03C003C0u, one));
     }
     // the constants of (row, sub-block) in the warp's scratch, as for Q4_K: (32 (1 + 2 s), -47 (1 + 2 s))
-    static constexpr int SCRATCH = 16 * 4 * 8;
+    static constexpr int SCRATCH = 2 * 16 * 4 * 8;
     struct Pre { uint32_t D[2], one; };
-    template <int u> __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t * scratch) {
+    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t * scratch) {
         const int g = lane >> 2, t = lane & 3;
         Pre p;
         p.one = in_register(0x3C003C00u);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-            const uint32_t sc = *reinterpret_cast<const uint32_t *>(chunk + 2048 + 4 * (g + 8 * r)) >> (16 * u + 4 * t);
-            // the 4-bit scale under the exponent of 1: 1 + s / 16
-            const __half2 s = bits_h2(((sc & 15u) * 0x00400040u) | 0x3C003C00u);
-            reinterpret_cast<uint2 *>(scratch)[4 * (g + 8 * r) + t] = make_uint2(h2_bits(__hfma2(s, __float2half2_rn(1024.f), __float2half2_rn(-992.f))),
-                                                                               h2_bits(__hfma2(s, __float2half2_rn(-1504.f), __float2half2_rn(1457.f))));
+            const uint32_t sc = *reinterpret_cast<const uint32_t *>(chunk + 2048 + 4 * (g + 8 * r)) >> (4 * t);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                // the 4-bit scale under the exponent of 1: 1 + s / 16
+                const __half2 s = bits_h2((((sc >> (16 * u)) & 15u) * 0x00400040u) | 0x3C003C00u);
+                reinterpret_cast<uint2 *>(scratch)[64 * u + 4 * (g + 8 * r) + t] = make_uint2(h2_bits(__hfma2(s, __float2half2_rn(1024.f), __float2half2_rn(-992.f))),
+                                                                                            h2_bits(__hfma2(s, __float2half2_rn(-1504.f), __float2half2_rn(1457.f))));
+            }
             p.D[r] = uint32_t(*reinterpret_cast<const unsigned short *>(chunk + 2112 + 2 * (g + 8 * r))) * 0x10001u;
         }
         return p;
     }
-    template <int u, int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const void *, const uint8_t * scratch, const Pre & p, uint32_t (&f)[16]) {
-        const uint4 w4 = plane(chunk, 2 * u + JS, lane);
-        const uint4 * c = reinterpret_cast<const uint4 *>(scratch) + 2 * (lane >> 2) + JS;       // both sub-blocks of the step
+    struct Raw { uint4 w, c[2]; };
+    template <int J> __device__ __forceinline__ static Raw load(const uint8_t * chunk, int lane, const uint8_t * scratch) {
+        const uint4 * c = reinterpret_cast<const uint4 *>(scratch) + 32 * (J >> 1) + 2 * (lane >> 2) + (J & 1);       // both sub-blocks of the step
+        return Raw{plane(chunk, J, lane), {c[0], c[16]}};
+    }
+    template <int J> __device__ __forceinline__ static void step(const Raw & raw, int, const void *, const Pre & p, uint32_t (&f)[16]) {
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-            const uint4 k = c[16 * r];
+            const uint4 k = raw.c[r];
             const __half2 D = bits_h2(p.D[r]), SC1 = bits_h2(k.x), C1 = bits_h2(k.y), SC2 = bits_h2(k.z), C2 = bits_h2(k.w);
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
-                const uint32_t v = r ? (b ? w4.w : w4.z) : (b ? w4.y : w4.x);
+                const uint32_t v = r ? (b ? raw.w.w : raw.w.z) : (b ? raw.w.y : raw.w.x);
                 put(f, r, b, make_uint4(h2_bits(__hmul2(__hfma2(pair<0>(v, p.one), SC1, C1), D)), h2_bits(__hmul2(__hfma2(pair<8>(v, p.one), SC1, C1), D)),
                                         h2_bits(__hmul2(__hfma2(pair<4>(v, p.one), SC2, C2), D)), h2_bits(__hmul2(__hfma2(pair<12>(v, p.one), SC2, C2), D))));
             }
@@ -184,37 +193,40 @@ template <> struct Dec<T_IQ3S4> {
 template <uint32_t T> struct Exact;
 template <> struct Exact<T_Q4_K> {
     static constexpr bool MINS = true;
-    static constexpr int SCRATCH = 16 * 4 * 4;
+    static constexpr int SCRATCH = 2 * 16 * 4 * 4;
     struct Pre { uint32_t magic; };
-    template <int u> __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t * scratch) {
+    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t * scratch) {
         const int g = lane >> 2, t = lane & 3;
         const uint32_t * h0 = reinterpret_cast<const uint32_t *>(chunk + 2048 + 16 * g), * h1 = h0 + 32;       // d, dmin | s[12]
-        uint32_t sc0 = h0[1], sc1 = h1[1];
-        if (u) {
-            sc0 = (h0[3] & 0x0F0F0F0Fu) | ((sc0 >> 2) & 0x30303030u);
-            sc1 = (h1[3] & 0x0F0F0F0Fu) | ((sc1 >> 2) & 0x30303030u);
-        }
-        const uint32_t v = __byte_perm(sc0, sc1, uint32_t(t) * 0x0101u + 0x0400u);      // byte t of either row's word, 16 bits apart
-        __half2 sc = __hadd2(bits_h2((v & 0x003F003Fu) | 0x64006400u), __float2half2_rn(-1024.f));
-        if (t & 1) sc = __hmul2(sc, __float2half2_rn(0.0625f));
-        const __half2 ns = __hmul2(sc, __float2half2_rn(-1024.f));
+        const uint32_t s0 = h0[1], s1 = h1[1], l0 = h0[3], l1 = h1[3], sel = uint32_t(t) * 0x0101u + 0x0400u;
         uint32_t * to = reinterpret_cast<uint32_t *>(scratch) + lane;
-        to[0] = h2_bits(__lows2half2(sc, ns));
-        to[32] = h2_bits(__highs2half2(sc, ns));
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const uint32_t sc0 = u ? (l0 & 0x0F0F0F0Fu) | ((s0 >> 2) & 0x30303030u) : s0, sc1 = u ? (l1 & 0x0F0F0F0Fu) | ((s1 >> 2) & 0x30303030u) : s1;
+            const uint32_t v = __byte_perm(sc0, sc1, sel);                  // byte t of either row's word, 16 bits apart
+            __half2 sc = __hadd2(bits_h2((v & 0x003F003Fu) | 0x64006400u), __float2half2_rn(-1024.f));
+            if (t & 1) sc = __hmul2(sc, __float2half2_rn(0.0625f));
+            const __half2 ns = __hmul2(sc, __float2half2_rn(-1024.f));
+            to[64 * u] = h2_bits(__lows2half2(sc, ns));
+            to[64 * u + 32] = h2_bits(__highs2half2(sc, ns));
+        }
         return Pre{in_register(0x64006400u)};
     }
-    template <int u, int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const uint8_t * scratch, const Pre & p, uint32_t (&f)[16]) {
-        const uint4 w4 = plane(chunk, 2 * u + JS, lane);
-        const uint2 * c = reinterpret_cast<const uint2 *>(scratch) + 2 * (lane >> 2) + JS;
+    struct Raw { uint4 w; uint2 c[2]; };
+    template <int J> __device__ __forceinline__ static Raw load(const uint8_t * chunk, int lane, const uint8_t * scratch) {
+        const uint2 * c = reinterpret_cast<const uint2 *>(scratch) + 32 * (J >> 1) + 2 * (lane >> 2) + (J & 1);
+        return Raw{plane(chunk, J, lane), {c[0], c[16]}};
+    }
+    template <int J> __device__ __forceinline__ static void step(const Raw & raw, int, const void *, const Pre & p, uint32_t (&f)[16]) {
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-            const uint2 k = c[16 * r];
+            const uint2 k = raw.c[r];
             const __half2 S0 = __low2half2(bits_h2(k.x)), N0 = __high2half2(bits_h2(k.x)), S1 = __low2half2(bits_h2(k.y)), N1 = __high2half2(bits_h2(k.y));
             auto lo = [&](uint32_t w) { return h2_bits(__hfma2(bits_h2(and_or(w, 0x000F000Fu, p.magic)), S0, N0)); };
             auto hi = [&](uint32_t w) { return h2_bits(__hfma2(bits_h2(and_or(w, 0x00F000F0u, p.magic)), S1, N1)); };
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
-                const uint32_t v = r ? (b ? w4.w : w4.z) : (b ? w4.y : w4.x), v8 = v >> 8;
+                const uint32_t v = r ? (b ? raw.w.w : raw.w.z) : (b ? raw.w.y : raw.w.x), v8 = v >> 8;
                 put(f, r, b, make_uint4(lo(v), lo(v8), hi(v), hi(v8)));
             }
         }
@@ -237,29 +249,35 @@ template <> struct Exact<T_Q4_K> {
 };
 template <> struct Exact<T_IQ3S4> {
     static constexpr bool MINS = false;
-    static constexpr int SCRATCH = 16 * 4 * 4;
+    static constexpr int SCRATCH = 2 * 16 * 4 * 4;
     struct Pre { uint32_t one; };
-    template <int u> __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t * scratch) {
+    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t * scratch) {
         const int g = lane >> 2, t = lane & 3;
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-            const uint32_t sc = *reinterpret_cast<const uint32_t *>(chunk + 2048 + 4 * (g + 8 * r)) >> (16 * u + 4 * t);
-            const __half2 s = bits_h2(((sc & 15u) * 0x00400040u) | 0x3C003C00u);        // 1 + s / 16 -> 32 (1 + 2 s), -47 (1 + 2 s)
-            reinterpret_cast<uint32_t *>(scratch)[lane + 32 * r] = h2_bits(__hfma2(s, __floats2half2_rn(1024.f, -1504.f), __floats2half2_rn(-992.f, 1457.f)));
+            const uint32_t sc = *reinterpret_cast<const uint32_t *>(chunk + 2048 + 4 * (g + 8 * r)) >> (4 * t);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const __half2 s = bits_h2((((sc >> (16 * u)) & 15u) * 0x00400040u) | 0x3C003C00u);        // 1 + s / 16 -> 32 (1 + 2 s), -47 (1 + 2 s)
+                reinterpret_cast<uint32_t *>(scratch)[64 * u + lane + 32 * r] = h2_bits(__hfma2(s, __floats2half2_rn(1024.f, -1504.f), __floats2half2_rn(-992.f, 1457.f)));
+            }
         }
         return Pre{in_register(0x3C003C00u)};
     }
-    template <int u, int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const uint8_t * scratch, const Pre & p, uint32_t (&f)[16]) {
+    struct Raw { uint4 w; uint2 c[2]; };
+    template <int J> __device__ __forceinline__ static Raw load(const uint8_t * chunk, int lane, const uint8_t * scratch) {
+        const uint2 * c = reinterpret_cast<const uint2 *>(scratch) + 32 * (J >> 1) + 2 * (lane >> 2) + (J & 1);
+        return Raw{plane(chunk, J, lane), {c[0], c[16]}};
+    }
+    template <int J> __device__ __forceinline__ static void step(const Raw & raw, int, const void *, const Pre & p, uint32_t (&f)[16]) {
         using D = Dec<T_IQ3S4>;
-        const uint4 w4 = plane(chunk, 2 * u + JS, lane);
-        const uint2 * c = reinterpret_cast<const uint2 *>(scratch) + 2 * (lane >> 2) + JS;
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-            const uint2 k = c[16 * r];
+            const uint2 k = raw.c[r];
             const __half2 S0 = __low2half2(bits_h2(k.x)), C0 = __high2half2(bits_h2(k.x)), S1 = __low2half2(bits_h2(k.y)), C1 = __high2half2(bits_h2(k.y));
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
-                const uint32_t v = r ? (b ? w4.w : w4.z) : (b ? w4.y : w4.x);
+                const uint32_t v = r ? (b ? raw.w.w : raw.w.z) : (b ? raw.w.y : raw.w.x);
                 put(f, r, b, make_uint4(h2_bits(__hfma2(D::pair<0>(v, p.one), S0, C0)), h2_bits(__hfma2(D::pair<8>(v, p.one), S0, C0)),
                                         h2_bits(__hfma2(D::pair<4>(v, p.one), S1, C1)), h2_bits(__hfma2(D::pair<12>(v, p.one), S1, C1))));
             }
@@ -304,48 +322,61 @@ template <> struct Dec<T_IQ4_XS> {
     static constexpr int SCRATCH = 0;
     static constexpr int TAB_BYTES = LUT_BYTES;
     __device__ static void init(void * tab, int tid, int n) { build_lut(tab, tid, n); }
-    // once per chunk: lane t holds fp16(d (ls - 32)) of the unit's sub-block t, for its two rows
-    struct Pre { uint32_t dl; };
-    template <int u> __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t *) {
-        const int g = lane >> 2, ib = 4 * u + (lane & 3);
-        float dl[2];
+    // once per chunk: lane t holds fp16(d (ls - 32)) of sub-blocks t and 4 + t, for its two rows
+    struct Pre { uint32_t dl[2]; };
+    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t *) {
+        const int g = lane >> 2, t = lane & 3;
+        float dl[2][2];
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             const uint2 h = *reinterpret_cast<const uint2 *>(chunk + 2048 + 8 * (g + 8 * r));       // d, scales_h | scales_l[4]
             const float d = __half2float(__ushort_as_half((unsigned short)(h.x & 0xffffu)));
-            const int ls = int((h.y >> (4 * ib)) & 15u) | int(((h.x >> (16 + 2 * ib)) & 3u) << 4);
-            dl[r] = d * float(ls - 32);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int ib = 4 * u + t, ls = int((h.y >> (4 * ib)) & 15u) | int(((h.x >> (16 + 2 * ib)) & 3u) << 4);
+                dl[u][r] = d * float(ls - 32);
+            }
         }
-        return Pre{pack_h2(dl[0], dl[1])};
+        return Pre{{pack_h2(dl[0][0], dl[0][1]), pack_h2(dl[1][0], dl[1][1])}};
     }
-    template <int u, int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const void * tab, const uint8_t *, const Pre & p, uint32_t (&f)[16]) {
+    struct Raw { uint4 w; };
+    template <int J> __device__ __forceinline__ static Raw load(const uint8_t * chunk, int lane, const uint8_t *) { return Raw{plane(chunk, J, lane)}; }
+    template <int J> __device__ __forceinline__ static void step(const Raw & raw, int lane, const void * tab, const Pre & p, uint32_t (&f)[16]) {
         const Lut lut = lut_of(tab, lane);
-        const uint4 w4 = plane(chunk, 2 * u + JS, lane);
-        const int src = (lane & ~3) | (2 * JS);
-        const __half2 d0 = bits_h2(__shfl_sync(0xffffffffu, p.dl, src)), d1 = bits_h2(__shfl_sync(0xffffffffu, p.dl, src + 1));
-        put(f, 0, 0, lut_word(lut, w4.x, __low2half2(d0)));
-        put(f, 0, 1, lut_word(lut, w4.y, __low2half2(d1)));
-        put(f, 1, 0, lut_word(lut, w4.z, __high2half2(d0)));
-        put(f, 1, 1, lut_word(lut, w4.w, __high2half2(d1)));
+        const int src = (lane & ~3) | (2 * (J & 1));
+        const __half2 d0 = bits_h2(__shfl_sync(0xffffffffu, p.dl[J >> 1], src)), d1 = bits_h2(__shfl_sync(0xffffffffu, p.dl[J >> 1], src + 1));
+        put(f, 0, 0, lut_word(lut, raw.w.x, __low2half2(d0)));
+        put(f, 0, 1, lut_word(lut, raw.w.y, __low2half2(d1)));
+        put(f, 1, 0, lut_word(lut, raw.w.z, __high2half2(d0)));
+        put(f, 1, 1, lut_word(lut, raw.w.w, __high2half2(d1)));
     }
 };
 
 template <> struct Dec<T_IQ4_NL> {
     static constexpr int SCRATCH = 0;
     struct Pre {};
-    template <int u> __device__ __forceinline__ static Pre prep(const uint8_t *, int, uint8_t *) { return Pre{}; }
+    __device__ __forceinline__ static Pre prep(const uint8_t *, int, uint8_t *) { return Pre{}; }
     static constexpr int TAB_BYTES = LUT_BYTES;
     __device__ static void init(void * tab, int tid, int n) { build_lut(tab, tid, n); }
-    template <int u, int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const void * tab, const uint8_t *, const Pre &, uint32_t (&f)[16]) {
-        const Lut lut = lut_of(tab, lane);
+    struct Raw { uint2 w[2]; __half d[2][2]; };
+    template <int J> __device__ __forceinline__ static Raw load(const uint8_t * chunk, int lane, const uint8_t *) {
         const int g = lane >> 2;
+        Raw raw;
 #pragma unroll
         for (int b = 0; b < 2; ++b) {                                   // the step's two 32-column tiles: the rows' code words and fp16 scales
-            const uint8_t * tile = chunk + (4 * u + 2 * JS + b) * Fmt<T_IQ4_NL>::TILE;
-            const uint2 w = *reinterpret_cast<const uint2 *>(tile + 8 * lane);
-            const __half d0 = *reinterpret_cast<const __half *>(tile + 256 + 2 * g), d1 = *reinterpret_cast<const __half *>(tile + 256 + 2 * (g + 8));
-            put(f, 0, b, lut_word(lut, w.x, __half2half2(d0)));
-            put(f, 1, b, lut_word(lut, w.y, __half2half2(d1)));
+            const uint8_t * tile = chunk + (2 * J + b) * Fmt<T_IQ4_NL>::TILE;
+            raw.w[b] = *reinterpret_cast<const uint2 *>(tile + 8 * lane);
+            raw.d[b][0] = *reinterpret_cast<const __half *>(tile + 256 + 2 * g);
+            raw.d[b][1] = *reinterpret_cast<const __half *>(tile + 256 + 2 * (g + 8));
+        }
+        return raw;
+    }
+    template <int J> __device__ __forceinline__ static void step(const Raw & raw, int lane, const void * tab, const Pre &, uint32_t (&f)[16]) {
+        const Lut lut = lut_of(tab, lane);
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            put(f, 0, b, lut_word(lut, raw.w[b].x, __half2half2(raw.d[b][0])));
+            put(f, 1, b, lut_word(lut, raw.w[b].y, __half2half2(raw.d[b][1])));
         }
     }
 };
@@ -354,7 +385,7 @@ template <> struct Dec<T_IQ4_NL> {
 template <> struct Dec<T_NVFP4G> {
     static constexpr int SCRATCH = 0;
     struct Pre {};
-    template <int u> __device__ __forceinline__ static Pre prep(const uint8_t *, int, uint8_t *) { return Pre{}; }
+    __device__ __forceinline__ static Pre prep(const uint8_t *, int, uint8_t *) { return Pre{}; }
     static constexpr int TAB_BYTES = 0;
     __device__ static void init(void *, int, int) {}
     // the eight e2m1 codes of a word -> eight fp16 values (the hardware conversion, two codes per instruction: low nibble
@@ -366,19 +397,22 @@ template <> struct Dec<T_NVFP4G> {
         return make_uint4(h2_bits(__hmul2(bits_h2(v0), scale)), h2_bits(__hmul2(bits_h2(v1), scale)), h2_bits(__hmul2(bits_h2(v2), scale)),
                           h2_bits(__hmul2(bits_h2(v3), scale)));
     }
-    template <int u, int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const void *, const uint8_t *, const Pre &, uint32_t (&f)[16]) {
-        const int g = lane >> 2, t = lane & 3;
-        const uint8_t * tile = chunk + u * Fmt<T_NVFP4G>::TILE;
-        constexpr int P = JS;                                            // the unit is one 128-column tile; plane = sub-blocks 2 P, 2 P + 1 of the 128-column tile
-        const uint4 w4 = plane(tile, P, lane);
+    struct Raw { uint4 w; uint32_t sc[2]; };
+    template <int J> __device__ __forceinline__ static Raw load(const uint8_t * chunk, int lane, const uint8_t *) {
+        const uint8_t * tile = chunk + (J >> 1) * Fmt<T_NVFP4G>::TILE;      // a unit is one 128-column tile; plane P = sub-blocks 2 P, 2 P + 1 of it
+        constexpr int P = J & 1;
+        const uint8_t * sc = tile + 1024 + 8 * (lane >> 2) + 4 * P;
+        return Raw{plane(tile, P, lane), {*reinterpret_cast<const uint32_t *>(sc), *reinterpret_cast<const uint32_t *>(sc + 64)}};
+    }
+    template <int J> __device__ __forceinline__ static void step(const Raw & raw, int lane, const void *, const Pre &, uint32_t (&f)[16]) {
+        const uint32_t sel = (lane & 3) < 2 ? 0x4420u : 0x4431u;
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             // E4M3 scales of sub-blocks 2 P (bytes 0, 1) and 2 P + 1 (bytes 2, 3); the 16-weight group of word t is t / 2
-            const uint32_t scw = *reinterpret_cast<const uint32_t *>(tile + 1024 + 8 * (g + 8 * r) + 4 * P);
-            const uint32_t two = __byte_perm(scw, 0u, t < 2 ? 0x4420u : 0x4431u);
+            const uint32_t two = __byte_perm(raw.sc[r], 0u, sel);
             const __half2 s = __half2(__nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)two, __NV_E4M3));
-            put(f, r, 0, word(r ? w4.z : w4.x, __low2half2(s)));
-            put(f, r, 1, word(r ? w4.w : w4.y, __high2half2(s)));
+            put(f, r, 0, word(r ? raw.w.z : raw.w.x, __low2half2(s)));
+            put(f, r, 1, word(r ? raw.w.w : raw.w.y, __high2half2(s)));
         }
     }
 };
@@ -387,7 +421,7 @@ template <> struct Dec<T_NVFP4G> {
 template <> struct Dec<T_IQ3_S> {
     static constexpr int SCRATCH = 0;
     struct Pre {};
-    template <int u> __device__ __forceinline__ static Pre prep(const uint8_t *, int, uint8_t *) { return Pre{}; }
+    __device__ __forceinline__ static Pre prep(const uint8_t *, int, uint8_t *) { return Pre{}; }
     // table: grid entry -> its four odd magnitudes as fp16 (8 bytes)
     static constexpr int TAB_BYTES = 512 * 8;
     __device__ static void init(void * tab, int tid, int n) {
@@ -397,10 +431,10 @@ template <> struct Dec<T_IQ3_S> {
             t2[i] = make_uint2(pack_h2(float(m & 255u), float((m >> 8) & 255u)), pack_h2(float((m >> 16) & 255u), float(m >> 24)));
         }
     }
-    template <int u, int JS> __device__ __forceinline__ static void step(const uint8_t * chunk, int lane, const void * tab, const uint8_t *, const Pre &, uint32_t (&f)[16]) {
-        bits_step<2 * u + JS>(chunk, lane, tab, f);
-    }
-    template <int J> __device__ __forceinline__ static void bits_step(const uint8_t * chunk, int lane, const void * tab, uint32_t (&f)[16]) {
+    struct Raw { const uint8_t * chunk; };                               // (a step's words would take thirteen registers)
+    template <int J> __device__ __forceinline__ static Raw load(const uint8_t * chunk, int, const uint8_t *) { return Raw{chunk}; }
+    template <int J> __device__ __forceinline__ static void step(const Raw & raw, int lane, const void * tab, const Pre &, uint32_t (&f)[16]) {
+        const uint8_t * chunk = raw.chunk;
         const int g = lane >> 2;
         const uint2 * mags = static_cast<const uint2 *>(tab);
         uint32_t w[13];
