@@ -37,6 +37,7 @@
 #include "common.cuh"
 #include "dec4_stage.cuh"
 #include "formats.cuh"
+#include "route_token.cuh"
 
 namespace b2 {
 namespace {
@@ -151,6 +152,26 @@ template <> struct D4<T_IQ3S4> {
     }
 };
 
+// What a gate/up launch needs to route for itself (dec4_k, ROUTED): the router's logits, where the routing's results go, the rows of the tokens
+struct Dec4Route {
+    const float * logits, * bias;            // bias: selection bias of the sigmoid family, may be null
+    int * ids;
+    float * weights, * shared_weights;       // shared_weights may be null
+    const void * x;
+    int ld, gating, norm, n, shared_first, shared_count, x_dtype;
+    float scale;
+};
+struct NoRoute {};
+// a block's own copy of the plan: its slots, and the passes in the order of their experts (expert, first slot, tokens), taken from the last
+constexpr int ROUTED_MAX = 128;              // assignments
+struct Routed {
+    int ids[ROUTED_MAX];
+    float weights[ROUTED_MAX];
+    short perm[ROUTED_MAX + PASS_TOKENS], e[ROUTED_MAX + 1], off[ROUTED_MAX + 1];
+    signed char cnt[ROUTED_MAX + 1], flags[ROUTED_MAX];      // flags of an assignment: 1: the first of its expert, 2: the first of a pass
+    float inv[PASS_TOKENS];                  // inverse scales of the staged rows
+    int row[2][PASS_TOKENS];                 // the staged row of a segment's token columns
+};
 struct Dec4Args {
     const uint8_t * w0, * w1, * s0, * s1;   // stacked banks (gate, up | down, -) and the shared expert's
     size_t bank_bytes;
@@ -187,12 +208,96 @@ constexpr size_t RED_BYTES = size_t(CTA_WARPS) * 8 * 32 * sizeof(float);     // 
 template <bool STAGER> constexpr int threads_of() { return (CTA_WARPS + (STAGER ? 2 : 1)) * 32; }
 template <bool STAGER> constexpr int bound_threads() { return STAGER ? 640 : threads_of<false>(); }
 
+// The prologue of a ROUTED block, all of its threads; returns its passes
+template <int GATING> __device__ __noinline__ void route_warp(const Dec4Route & r, int experts, int topk, int * ids, float * weights, float * shared_weights, int token, int lane) {
+    const float * bias = GATING == B2MOE_SOFTMAX ? nullptr : r.bias;
+    if (experts <= 128) route_token_regs<GATING, 4>(r.logits, r.ld, bias, ids, weights, shared_weights, experts, topk, r.norm, r.scale, token, lane);
+    else if (experts <= 256) route_token_regs<GATING, 8>(r.logits, r.ld, bias, ids, weights, shared_weights, experts, topk, r.norm, r.scale, token, lane);
+    else route_token_regs<GATING, 16>(r.logits, r.ld, bias, ids, weights, shared_weights, experts, topk, r.norm, r.scale, token, lane);
+}
+__device__ __forceinline__ int route_and_plan(const Dec4Args & p, const Dec4Route & in, Routed & r, uint8_t * rows, uint32_t xrow, int bits) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, A = p.A, e1 = p.experts + 1;
+    int * counts = p.plan + PLAN_HDR, * offsets = counts + e1, * active = offsets + e1 + 1, * perm = active + e1;
+    const bool lead = blockIdx.x == 0;                                 // writes what is not spread over the blocks
+    if (warp < in.n) {                                                 // n <= PASS_TOKENS: warps 0 .. 7 route, 8 .. 15 stage
+        float * sw = lead ? in.shared_weights : nullptr;
+        if (in.gating == B2MOE_SOFTMAX) route_warp<B2MOE_SOFTMAX>(in, p.experts, p.topk, r.ids, r.weights, sw, warp, lane);
+        else route_warp<B2MOE_SIGMOID>(in, p.experts, p.topk, r.ids, r.weights, nullptr, warp, lane);
+    } else if (warp >= PASS_TOKENS && warp < PASS_TOKENS + in.n) {
+        const int row = warp - PASS_TOKENS, k = p.k_tiles * 256;
+        const float inv = stage_row_lanes(in.x, in.x_dtype, size_t(row) * k, k, bits, rows + row * xrow, lane);
+        if (lane == 0) r.inv[row] = inv;
+    }
+    __syncthreads();
+    // an assignment's place: those of smaller experts and the earlier ones of its own (the stable order of a dispatch)
+    int below = 0, same = 0, before = 0;
+    const int e = tid < A ? r.ids[tid] : -1;
+    if (tid < A) {
+#pragma unroll 1
+        for (int a = 0; a < A; ++a) {
+            const int o = r.ids[a];
+            below += o < e;
+            same += o == e;
+            before += o == e && a < tid;
+        }
+        r.perm[below + before] = short(tid);
+        r.flags[tid] = (before == 0) | (before % PASS_TOKENS == 0) << 1;
+    }
+    const bool first = tid < A && before == 0, begins = tid < A && before % PASS_TOKENS == 0;
+    const int experts = __syncthreads_count(first), passes = __syncthreads_count(begins), shared = in.shared_count > 0;
+    int * const pass_list = perm + A + in.shared_count;
+    if (begins) {
+        int expert_at = 0, at = before / PASS_TOKENS, behind = shared;   // active experts before this one, passes before this one, passes of the experts behind
+#pragma unroll 1
+        for (int a = 0; a < A; ++a) {
+            const int o = r.ids[a], f = r.flags[a];
+            expert_at += (f & 1) && o < e;
+            at += (f & 2) && o < e;
+            behind += (f & 2) && o > e;
+        }
+        r.e[at] = short(e); r.off[at] = short(below + before); r.cnt[at] = (signed char)min(PASS_TOKENS, same - before);
+        if (lead && first) { active[expert_at] = e; pass_list[experts + shared - 1 - expert_at] = behind; }
+    }
+    if (shared) {                                                      // its tokens are one pass
+        if (tid < in.shared_count) r.perm[A + tid] = short(A + in.shared_first + tid);
+        if (tid == 0) {
+            r.e[passes] = short(p.experts); r.off[passes] = short(A); r.cnt[passes] = (signed char)in.shared_count;
+            if (lead) { active[experts] = p.experts; pass_list[0] = 0; }
+        }
+    }
+    // the plan for the launches behind: counts and offsets of a few experts a block, the rest by the first one
+    if (warp >= 4 && warp < 12) {
+        for (int x = int(blockIdx.x) + int(gridDim.x) * (warp - 4); x < e1; x += int(gridDim.x) * 8) {
+            int c = 0, b = 0;
+            for (int a = lane; a < A; a += 32) { c += r.ids[a] == x; b += r.ids[a] < x; }
+            c = __reduce_add_sync(0xffffffffu, c);
+            b = __reduce_add_sync(0xffffffffu, b);
+            if (lane == 0) { counts[x] = x < p.experts ? c : in.shared_count; offsets[x] = x < p.experts ? b : A; }
+        }
+    }
+    __syncthreads();
+    if (lead) {
+        if (tid < A) { in.ids[tid] = e; in.weights[tid] = r.weights[tid]; }
+        for (int i = tid; i < A + in.shared_count; i += blockDim.x) perm[i] = r.perm[i];
+        if (tid == 0) {
+            offsets[e1] = A + in.shared_count;
+            pass_list[experts + shared] = passes + shared;
+            p.plan[PLAN_NGROUPED] = A + in.shared_count; p.plan[PLAN_NACTIVE] = experts + shared; p.plan[PLAN_NPASS] = passes + shared; p.plan[PLAN_STATUS] = 0;
+        }
+    }
+    return passes + shared;
+}
+
 // MODE 0: out = act[a][row] = silu(gate . x) * (up . x);   MODE 1: out = y[a][row] = down . act[a]
 // FEW: the instances of small launches (a few jobs per block): chains of latencies more than streams, so the way from the plan to the first copy is
 // shorter there and a block's share lies in one pass where that costs no round. The other instances keep their plain walk: these
 // lines in them cost the compiler registers and every large launch 2.5 % (64 tokens of 512 IQ3_S experts, gate/up 87.6 -> 90 us).
-template <uint32_t T, int MODE, bool FEW>
-__global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(const Dec4Args p) {
+// ROUTED (gate/up of up to eight tokens): there is no routing launch. Every block routes all tokens for itself, a warp each, while others bring the tokens' rows into the staged form,
+// and takes its passes from a plan in shared memory; together the blocks write the plan and the routing's results for the launches behind. What that saves is a launch, the cluster's meeting, the
+// scan of all experts and seven dependent loads from the plan before the first rows: a layer of one token on 512 IQ3_S experts 32.9 -> 29.3 us, seven fp32 tokens on 32 Q4_K experts 29.3 -> 27.0.
+template <uint32_t T, int MODE, bool FEW, bool ROUTED = false>
+__global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(const Dec4Args p, const typename std::conditional<ROUTED, Dec4Route, NoRoute>::type route) {
+    static_assert(!ROUTED || (FEW && MODE == 0));
     constexpr bool STAGER = FEW && MODE == 1;
     using Job = typename std::conditional<FEW, int, long long>::type;
     using F = D4<T>;
@@ -236,11 +341,14 @@ __global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(c
     __syncthreads();
 
     const int * counts = p.plan + PLAN_HDR, * offsets = counts + e1, * active = offsets + e1 + 1, * perm = active + e1;
-    const int * passes = perm + p.A + counts[p.experts];     // the plan's own count of always-on rows (a range of the tokens under expert parallelism)
-    const int na = p.plan[PLAN_NACTIVE], row_tiles = (p.rows + 15) >> 4;
+    __shared__ typename std::conditional<ROUTED, Routed, int>::type routed;
+    int routed_passes = 0;
+    if constexpr (ROUTED) routed_passes = route_and_plan(p, route, routed, xs, xrow, F::BITS);
+    const int * passes = ROUTED ? nullptr : perm + p.A + counts[p.experts];     // the plan's own count of always-on rows (a range of the tokens under expert parallelism)
+    const int na = ROUTED ? routed_passes : p.plan[PLAN_NACTIVE], row_tiles = (p.rows + 15) >> 4;
     // the block's share of the launch: jobs [u_begin, u_end) of the pass-major list of (pass, row tile) jobs; it walks the
     // share as segments = runs of row tiles [r0, r1) of one pass
-    const int n_pass = p.plan[PLAN_NPASS];
+    const int n_pass = ROUTED ? routed_passes : p.plan[PLAN_NPASS];
     const Job n_jobs = Job(n_pass) * row_tiles;
     Job u_begin, u_end;
     if constexpr (FEW) {
@@ -273,6 +381,11 @@ __global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(c
     // pass w -> (expert, first token slot); the pass list runs over the active experts from the last to the first. Called by
     // all lanes of the producer warp together: two rounds of 32 probes instead of a ten-step chain of dependent loads.
     auto locate = [&](int w, int & e, int & c0) {
+        if constexpr (ROUTED) {
+            e = routed.e[na - 1 - w];
+            c0 = 0;
+            return;
+        }
         if (FEW && na <= 32) {                                                     // one round, which brings the experts along
             const int i = min(lane, na - 1), at = passes[i], expert = active[na - 1 - i];
             const int src = 31 - __clz(int(__ballot_sync(0xffffffffu, lane < na && at <= w) | 1u));
@@ -321,9 +434,23 @@ __global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(c
             if (!ok) return;
             int e = e_in, c0 = c0_in;
             if (!known) locate(pass, e, c0);
-            const int nv = min(PASS_TOKENS, counts[e] - c0);
             const int col = lane - 16;                                        // lanes 16 .. 23: one token column each
             int a = -1;
+            if constexpr (ROUTED) {                                           // the rows are in shared memory already
+                const int at = na - 1 - pass;
+                if (col >= 0 && col < PASS_TOKENS) {
+                    if (col < routed.cnt[at]) a = routed.perm[routed.off[at] + col];
+                    const int row = a >= 0 ? int(x_row(a)) : 0;
+                    routed.row[b][col] = row;
+                    meta[b].col_a[col] = a;
+                    meta[b].col_is[col] = a >= 0 ? routed.inv[row] : 0.f;
+                }
+                __syncwarp();
+                if (lane == 16) mbar_arrive(xfull + 8 * b);
+                ++xissued;
+                return;
+            }
+            const int nv = min(PASS_TOKENS, counts[e] - c0);
             if (col >= 0 && col < PASS_TOKENS) {
                 if (col < nv) a = perm[offsets[e] + c0 + col];
                 // the row's copy leaves first; its bytes count against the phase that lane 16's arrival below opens (the
@@ -451,6 +578,10 @@ __global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(c
             const int xr = quad ? g & 3 : g;
             const uint8_t * xw = xs + b * xbuf + xr * xrow + t * 16 + (quad && g >= 4 ? 8 : 0);      // + sub-block * 64
             const uint8_t * rec = xs + b * xbuf + xr * xrow + size_t(K) * 2 + t * 8;  // + tile * 32
+            if constexpr (ROUTED) {                                          // the row of the column's token
+                xw = xs + routed.row[b][xr] * xrow + t * 16 + (quad && g >= 4 ? 8 : 0);
+                rec = xs + routed.row[b][xr] * xrow + size_t(K) * 2 + t * 8;
+            }
             // the lane's two tokens (columns 2t, 2t + 1; of four tokens in HALVES, 2 (t & 1) and the next): assignment index and inverse
             // activation scale, as the producer left them
             const bool halves = HALVES && quad;
@@ -640,8 +771,9 @@ int g_drop_tile = -1;                 // test hooks (b2moe_harness_wait_probe, b
 bool g_skip_stage = false;
 uint32_t g_wait_limit = WAIT_LIMIT;
 
-template <uint32_t T, int MODE, bool FEW>
-int32_t launch_dec4(Dec4Args a, cudaStream_t s) {
+// took != null: the ROUTED instance, where its shared memory fits
+template <uint32_t T, int MODE, bool FEW, bool ROUTED = false>
+int32_t launch_dec4(Dec4Args a, cudaStream_t s, typename std::conditional<ROUTED, Dec4Route, NoRoute>::type route = {}, bool * took = nullptr) {
     const int sms = sm_count(), k = a.k_tiles * 256;
     if (sms <= 0) return B2MOE_ERR_CUDA;
     if (!dec4_fit<T>(k, a.nbuf, a.stages, a.slot_tiles)) return B2MOE_ERR_SHAPE;
@@ -655,10 +787,14 @@ int32_t launch_dec4(Dec4Args a, cudaStream_t s) {
         if (per_block <= CTA_WARPS / ks && kslots % ks == 0 && g_ksplit_max >= ks &&
             dec4_smem<T>(k, a.nbuf, a.stages, a.slot_tiles) + RED_BYTES <= SMEM_LIMIT) { a.ksplit = ks; break; }
     const size_t smem = dec4_smem<T>(k, a.nbuf, a.stages, a.slot_tiles) + (a.ksplit > 1 ? RED_BYTES : 0);
-    if (cudaFuncSetAttribute(dec4_k<T, MODE, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return B2MOE_ERR_CUDA;
+    if (ROUTED) {
+        if (smem + sizeof(Routed) > SMEM_LIMIT + 1024) return B2MOE_OK;
+        *took = true;
+    }
+    if (cudaFuncSetAttribute(dec4_k<T, MODE, FEW, ROUTED>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return B2MOE_ERR_CUDA;
     a.wait_limit = g_wait_limit;
     a.drop_tile = g_drop_tile;
-    launch_overlapped(dec4_k<T, MODE, FEW>, dim3(sms), dim3(threads_of<FEW && MODE == 1>()), smem, s, a);       // a block's share of the (pass, row tile) jobs: an equal one, or (FEW) whole passes
+    launch_overlapped(dec4_k<T, MODE, FEW, ROUTED>, dim3(sms), dim3(threads_of<FEW && MODE == 1>()), smem, s, a, route);       // a block's share of the (pass, row tile) jobs: an equal one, or (FEW) whole passes
     return launch_status();
 }
 
@@ -678,16 +814,18 @@ int32_t stage(Dec4Args & a, const void * x, int dtype, int rows_x, int k, void *
 
 template <uint32_t T>
 int32_t gateup_t(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_bank * sg, const b2moe_bank * su, const void * x, int x_dtype,
-                 const int * plan, int n, int topk, int shared_tokens, void * act, int act_dtype, void * ws, cudaStream_t s, bool x_staged) {
+                 const int * plan, int n, int topk, int shared_tokens, void * act, int act_dtype, void * ws, cudaStream_t s, bool x_staged, const Dec4Route * route = nullptr, bool * took = nullptr) {
     const int k = gate->cols;
     Dec4Args a{};
-    if (int32_t rc = stage<T>(a, x, x_dtype, n, k, ws, s, x_staged)) return rc;
+    if (!route)
+        if (int32_t rc = stage<T>(a, x, x_dtype, n, k, ws, s, x_staged)) return rc;
     a.w0 = static_cast<const uint8_t *>(gate->data); a.w1 = static_cast<const uint8_t *>(up->data);
     if (shared_tokens) { a.s0 = static_cast<const uint8_t *>(sg->data); a.s1 = static_cast<const uint8_t *>(su->data); }
     a.bank_bytes = b2moe_bank_bytes(gate->type, gate->rows, gate->cols);
     a.plan = const_cast<int *>(plan); a.out = act; a.out_dtype = act_dtype;
     a.rows = gate->rows; a.k_tiles = k / 256; a.experts = gate->experts; a.topk = topk; a.A = n * topk;
     a.passes_bound = n * topk + (shared_tokens + PASS_TOKENS - 1) / PASS_TOKENS;
+    if (route) return few_jobs(a.passes_bound, a.rows) ? launch_dec4<T, 0, true, true>(a, s, *route, took) : B2MOE_OK;
     return few_jobs(a.passes_bound, a.rows) ? launch_dec4<T, 0, true>(a, s) : launch_dec4<T, 0, false>(a, s);
 }
 template <uint32_t T>
@@ -732,6 +870,17 @@ int32_t dec4_gateup(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_
     if (gate->type == T_Q4_K) return gateup_t<T_Q4_K>(gate, up, sg, su, x, x_dtype, plan, n, topk, shared_tokens, act, act_dtype, ws, s, x_staged);
     if (gate->type == T_IQ3S4) return gateup_t<T_IQ3S4>(gate, up, sg, su, x, x_dtype, plan, n, topk, shared_tokens, act, act_dtype, ws, s, x_staged);
     return B2MOE_ERR_FORMAT;
+}
+// gate/up that routes for itself (dec4_k, ROUTED): up to eight tokens, a launch of a few jobs per block, experts that a warp keeps in registers. *took = false and B2MOE_OK: the shape does
+// not fit, the caller takes a routing launch and dec4_gateup
+int32_t dec4_gateup_routed(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_bank * sg, const b2moe_bank * su, const void * x, int x_dtype, int gating, const float * logits, int ld,
+                           const float * bias, int norm, float scale, int * ids, float * weights, float * shared_weights, int * plan, int n, int topk, int shared_tokens, void * act, cudaStream_t s, bool * took) {
+    *took = false;
+    if (n > PASS_TOKENS || topk > 32 || n * topk > ROUTED_MAX || gate->experts > 512 || g_skip_stage) return B2MOE_OK;
+    const Dec4Route r{logits, bias, ids, weights, shared_weights, x, ld, gating, gating == B2MOE_SOFTMAX ? 1 : norm, n, 0, shared_tokens, x_dtype, scale};
+    if (gate->type == T_Q4_K) return gateup_t<T_Q4_K>(gate, up, sg, su, x, x_dtype, plan, n, topk, shared_tokens, act, B2MOE_F32, nullptr, s, false, &r, took);
+    if (gate->type == T_IQ3S4) return gateup_t<T_IQ3S4>(gate, up, sg, su, x, x_dtype, plan, n, topk, shared_tokens, act, B2MOE_F32, nullptr, s, false, &r, took);
+    return B2MOE_OK;
 }
 int32_t dec4_down(const b2moe_bank * down, const b2moe_bank * sd, const void * x, int x_dtype, bool per_token, const int * plan, int n, int topk,
                   int shared_tokens, void * y, int y_dtype, void * ws, cudaStream_t s, bool plan_ready) {

@@ -25,6 +25,8 @@ bool route_cluster_fits(int experts, int topk, int n);
 int32_t route_plan_stage(int gating, const float * logits, int ld, const float * bias, int * ids, float * weights, float * shared_weights,
                          int experts, int topk, int norm, float scale, int n, int shared_first, int shared_count, int * plan, const void * x,
                          int x_dtype, int k, int bits, uint8_t * staged_rows, float * inv_scale, cudaStream_t s, bool * took);
+int32_t dec4_gateup_routed(const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const void *, int x_dtype, int gating, const float * logits, int ld, const float * bias,
+                           int norm, float scale, int * ids, float * weights, float * shared_weights, int * plan, int n, int topk, int shared_tokens, void * act, cudaStream_t, bool * took);
 int32_t dec4_down(const b2moe_bank *, const b2moe_bank *, const void *, int x_dtype, bool per_token, const int *, int, int, int, void *, int y_dtype, void *,
                   cudaStream_t, bool plan_ready);
 void dec4_debug(int drop_tile, uint32_t wait_limit);
@@ -194,12 +196,8 @@ extern "C" B2MOE_API size_t b2moe_expert_slot_workspace_bytes(const b2moe_bank *
     return std::max({base, gemm_tc_slot_bytes(slot_rows, bank->cols), exact ? gemm_exact_bytes(slot_rows, bank->cols, x_dtype) : size_t(0)});
 }
 
-// x_staged: the caller has already written the staged form of x where the 4-bit decode kernels expect it (b2moe_layer_forward);
-// rows_buf: scratch the caller has to spare for the grouped GEMM's activation rows in slot order (null: it gathers them)
-static int32_t expert_gateup(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_bank * shared_gate, const b2moe_bank * shared_up,
-                             const void * x, int32_t x_dtype, const int32_t * plan, int32_t n, int32_t topk, int32_t shared_tokens, float * act,
-                             void * workspace, size_t workspace_bytes, b2moe_stream stream, bool x_staged, long long live = -1,
-                             void * rows_buf = nullptr, size_t rows_buf_bytes = 0) {
+static int32_t check_gateup(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_bank * shared_gate, const b2moe_bank * shared_up, const void * x, int32_t x_dtype,
+                            const int32_t * plan, int32_t n, int32_t topk, int32_t shared_tokens, const float * act) {
     if (int32_t rc = check_bank(gate)) return rc;
     if (int32_t rc = check_bank(up)) return rc;
     if (int32_t rc = same_shape(gate, up, true)) return rc;
@@ -212,6 +210,15 @@ static int32_t expert_gateup(const b2moe_bank * gate, const b2moe_bank * up, con
     }
     if (!x || !plan || !act) return B2MOE_ERR_NULL;
     if (!aligned16(x) || !aligned16(act)) return B2MOE_ERR_ALIGN;
+    return B2MOE_OK;
+}
+// x_staged: the caller has already written the staged form of x where the 4-bit decode kernels expect it (b2moe_layer_forward);
+// rows_buf: scratch the caller has to spare for the grouped GEMM's activation rows in slot order (null: it gathers them)
+static int32_t expert_gateup(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_bank * shared_gate, const b2moe_bank * shared_up,
+                             const void * x, int32_t x_dtype, const int32_t * plan, int32_t n, int32_t topk, int32_t shared_tokens, float * act,
+                             void * workspace, size_t workspace_bytes, b2moe_stream stream, bool x_staged, long long live = -1,
+                             void * rows_buf = nullptr, size_t rows_buf_bytes = 0) {
+    if (int32_t rc = check_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act)) return rc;
     if (live < 0) live = (long long)n * topk;
     const int path = expert_path(gate->type, gate->cols, x_dtype, gate->experts, live);
     if (path != B2MOE_FAMILY_GENERIC) {
@@ -243,7 +250,7 @@ extern "C" B2MOE_API int32_t b2moe_expert_gateup_swiglu(const b2moe_bank * gate,
     return expert_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, workspace, workspace_bytes, stream, false);
 }
 
-// plan_ready: the launch before this call's is a gate/up product over the same plan. Every kernel of that product waits for the launches before it and only then (when
+// plan_ready: the launch before this call's is a gate/up product over the same plan, which another launch made. Every kernel of that product waits for the launches before it and only then (when
 // its own work is done) lets the next one begin, so whatever begins here finds the plan complete and may ask for weights before it waits
 static int32_t expert_down(const b2moe_bank * down, const b2moe_bank * shared_down, const float * act, const int32_t * plan, int32_t n, int32_t topk,
                            int32_t shared_tokens, float * y, void * workspace, size_t workspace_bytes, b2moe_stream stream, long long live, bool plan_ready = false) {
@@ -367,27 +374,34 @@ static int32_t layer_forward(const b2moe_layer * L, const void * x, int32_t x_dt
     void * es = base + ws.expert_scratch;
     const size_t es_bytes = workspace_bytes - ws.expert_scratch;
     // decode-sized call whose gate/up runs on the 4-bit decode kernels: top-k, dispatch and the staging of x in one cluster launch
-    bool x_staged = false, slots;
+    bool x_staged = false, routed = false, slots;
     if (route_cluster_fits(L->experts, L->topk, n) && es_bytes >= b2moe_expert_workspace_bytes(L->gate.type, n, L->gate.cols, x_dtype) &&
         expert_path(L->gate.type, L->gate.cols, x_dtype, L->gate.experts, (long long)n * L->topk) == B2MOE_FAMILY_DECODE &&
         decode_kernel(L->gate.type, L->gate.cols, x_dtype) == DEC_4BIT && valid_dtype(x_dtype) &&
         !exact_gateup(&L->gate, x_dtype, (long long)n * L->topk, n * L->topk + sh, workspace_bytes - ws.y, &slots)) {
-        uint8_t * rows;
-        float * inv;
-        int bits;
-        dec4_stage_target(L->gate.type, es, n, L->gate.cols, &rows, &inv, &bits);
-        if (int32_t rc = route_plan_stage(L->gating, logits, ld, L->sel_bias, ids, weights, gated_shared ? shw : nullptr, L->experts, L->topk, L->norm,
-                                          L->scale, n, 0, sh, plan, x, x_dtype, L->gate.cols, bits, rows, inv, as_stream(stream), &x_staged)) return rc;
+        // a few tokens: the gate/up launch routes for itself
+        if (int32_t rc = check_gateup(&L->gate, &L->up, &L->sh_gate, &L->sh_up, x, x_dtype, plan, n, L->topk, sh, act)) return rc;
+        if (int32_t rc = dec4_gateup_routed(&L->gate, &L->up, &L->sh_gate, &L->sh_up, x, x_dtype, L->gating, logits, ld, L->sel_bias, L->norm, L->scale, ids, weights,
+                                            gated_shared ? shw : nullptr, plan, n, L->topk, sh, act, as_stream(stream), &routed)) return rc;
+        if (!routed) {
+            uint8_t * rows;
+            float * inv;
+            int bits;
+            dec4_stage_target(L->gate.type, es, n, L->gate.cols, &rows, &inv, &bits);
+            if (int32_t rc = route_plan_stage(L->gating, logits, ld, L->sel_bias, ids, weights, gated_shared ? shw : nullptr, L->experts, L->topk, L->norm,
+                                              L->scale, n, 0, sh, plan, x, x_dtype, L->gate.cols, bits, rows, inv, as_stream(stream), &x_staged)) return rc;
+        }
     }
-    if (!x_staged)
+    if (!x_staged && !routed)
         if (int32_t rc = b2moe_route_dispatch(L->gating, logits, ld, L->sel_bias, ids, weights, gated_shared ? shw : nullptr, L->experts, L->topk,
                                               L->norm, L->scale, n, 0, sh, plan, base + ws.scratch, ws.expert_scratch - ws.scratch, stream))
             return rc;
     // y is written by the down product: until then its rows (and what lies behind them: the dispatch is done, and a product that
     // converts its rows into y takes no other scratch) hold the gate/up product's activation rows
-    if (int32_t rc = expert_gateup(&L->gate, &L->up, &L->sh_gate, &L->sh_up, x, x_dtype, plan, n, L->topk, sh, act, es, es_bytes, stream, x_staged, -1, y,
-                                   workspace_bytes - ws.y)) return rc;
-    if (int32_t rc = expert_down(&L->down, &L->sh_down, act, plan, n, L->topk, sh, y, es, es_bytes, stream, -1, true)) return rc;
+    if (!routed)
+        if (int32_t rc = expert_gateup(&L->gate, &L->up, &L->sh_gate, &L->sh_up, x, x_dtype, plan, n, L->topk, sh, act, es, es_bytes, stream, x_staged, -1, y,
+                                       workspace_bytes - ws.y)) return rc;
+    if (int32_t rc = expert_down(&L->down, &L->sh_down, act, plan, n, L->topk, sh, y, es, es_bytes, stream, -1, !routed)) return rc;
     if (residual) return b2moe_combine_residual(y, nullptr, weights, gated_shared ? shw : nullptr, residual, n, L->topk, L->hidden, sh, out, out_dtype, stream);
     return b2moe_combine(y, nullptr, weights, gated_shared ? shw : nullptr, n, L->topk, L->hidden, sh, out, out_dtype, stream);
 }
