@@ -661,8 +661,8 @@ int32_t router_launch(const float * w, const float * shared, const void * xv, fl
     auto mma_blocks = [&](int tokens) { return (long long)ceil_div(rows, 16) * ceil_div(n, tokens) * ks; };
     // 16-bit rows go to router_tc_k where router_mma_k, with its 64 tokens a block, has more than two blocks per SM, or more than one and enough rows to fill most of a tile of
     // 128. Before / router_tc_k, us: bf16 2048 columns x 512 experts, 256 tokens 17.8 / 10.1, 509 23.5 / 11.2, 4096 87 / 32; 4096 x 128, 8192 tokens 163 / 40; 3072 x 256, 2047
-    // tokens 57 / 20; fp16 600 x 3072 x 256 32 / 16.5, 4096 x 2048 x 512 187 / 77, 600 x 2560 x 60 (160 blocks) 21.9 / 14.7, 4096 x 5120 x 16 (256 blocks of 16 rows) 31 / 72. Not where
-    // the other kernels are more precise (2-norm against fp64): bf16 below 256 tokens (1.3e-7 to 2.2e-7, here 4.7e-7), fp16 below 768 columns (6.9e-8, here 8.0e-8; from there on 8.1e-8 to 1.04e-7).
+    // tokens 57 / 20; fp16 600 x 3072 x 256 32 / 15.5, 4096 x 2048 x 512 187 / 73, 600 x 2560 x 60 (160 blocks) 21.9 / 13.7, 4096 x 5120 x 16 (256 blocks of 16 rows) 31 / 64. Not where
+    // the other kernels are more precise (2-norm against fp64): bf16 below 256 tokens (1.3e-7 to 2.2e-7, here 4.7e-7), fp16 below 768 columns (6.9e-8, here 7.2e-8; from there on 8.1e-8 to 1.04e-7).
     // Rows of fp32, and short ones of fp16: tiles once router_mma_k has more than two blocks per SM. router_mma_k / tiles, us: 1024 columns x 32 experts, fp16,
     // 600 tokens 8.9 / 17.7, 2047 (256 blocks) 16.8 / 18.0, 4096 (512 blocks) 32 / 18; 2560 x 60, 600 tokens (160) 22.8 / 31, 2047 (512) 46 / 32;
     // 3072 x 256, 256 tokens (256) 25 / 31, 300 (320) 36 / 31; 256 x 32 4096 tokens (128) 8.3 / 22.

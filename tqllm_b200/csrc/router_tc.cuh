@@ -1,18 +1,19 @@
 // Router logits of many 16-bit rows on the 5th-generation tensor cores (included by route.cu).
 //
 // logits[t][r] = sum_k W[r][k] x[t][k], W fp32. A block takes 128 router rows (M) x NT tokens (N):
-//   B: the activation rows as they are (bf16 or fp16), 64 columns a step, one TMA box in the 128-byte swizzled form;
-//   A: the router rows split exactly into three 16-bit terms, written to TENSOR MEMORY. TMA brings 64 fp32 columns of them a step, a thread splits half a row
-//      of it. bf16 rows: hi + mid + lo are bf16. fp16 rows: fp16 terms of the 32 values times a power of two that brings their largest magnitude into
-//      [2^14, 2^15) (what is below 2^-39 of it is lost), and the sums of the half step times its inverse.
-// So every product is exact in fp32 and three products do for either type (two bf16 terms of an fp16 activation would take six).
+//   A: the router rows split exactly into three bf16 terms (hi + mid + lo: the 24 bits of any fp32 value), written to TENSOR MEMORY. TMA brings 64 fp32 columns of them a step, a
+//      thread splits half a row of it;
+//   B: the activation rows, 64 columns a step, one TMA box in the 128-byte swizzled form. bf16 rows as they are; fp16 rows are split exactly into two bf16 terms in shared memory by
+//      the warps that read the sums, a 16-byte piece a thread and step: the first term takes the place of the piece, so the swizzle stays what it was.
+// So every product is exact in fp32: three products of terms for bf16 rows, six for fp16 rows. (fp16 terms of the weights times a power of two per 32 columns would take three there, but lose
+// what lies far below the largest of the 32: weights of 1e-6 beside one of 1 whose activation is 0 gave an error of 1e-6.)
 //
 // Numerics. The tensor core cuts its running sums off, always towards zero: 1.7e-8 of the sum per product that meets it. bf16 rows: the leading products of a part of 512 columns
 // are one chain of 32, the others (2^-8 of them and less) have sums of their own; the parts are added in column order. fp16 rows: one chain per half
-// step, smallest terms first (two of its six products meet a sum of full size); half steps and parts are added in fp32 with the rounding errors carried along.
+// step, smallest terms first (two of its twelve products meet a sum of full size); half steps and parts are added in fp32 with the rounding errors carried along.
 //
-// What bounds it: the chain from a step's copy over its split to the products, 1650 cycles a step of 128 bf16 tokens, 1080 of 64, 2100 of 64 fp16 tokens (most of it the split by two warps a
-// scheduler), where the products alone take 768 and 516. Two groups of splitting warps on steps in turn: 34.2 us against 31.9 (4096 x 2048 x 512 bf16; three stages instead of four for it); the
+// What bounds it: the chain from a step's copy over its split to the products, 1650 cycles a step of 128 bf16 tokens, 1080 of 64 (most of it the split by two warps a
+// scheduler), where the products alone take 768 and 516; 2000 of 64 fp16 tokens, whose products take twice as long and whose sums are read at every step. Two groups of splitting warps on steps in turn: 34.2 us against 31.9 (4096 x 2048 x 512 bf16; three stages instead of four for it); the
 // router rows loaded straight from global memory into fragments, no shared memory: 39.0; one accumulator for all terms: 24.9, at 1.65e-6 (this 4.7e-7).
 // A launch with few tiles would leave SMs idle: the blocks of a cluster take parts of a tile's columns each, and
 // add them in column order through distributed shared memory, so neither the split nor NT changes a bit.
@@ -32,16 +33,17 @@ constexpr int TMA_WARP = 0, MMA_WARP = 1, CONV_WARP0 = 4, EPI_WARP0 = 12, EPI_WA
 // Tensor memory. bf16: the sums of the leading products, those of the others; fp16: two sets of two (the halves of a step), a step each in turn. Then A, two steps of two
 // halves: three terms of 32 columns (16 of tensor memory) each
 constexpr int ACC = 128, A_COL0 = 2 * ACC, A_TERM = 16, A_HALF = 3 * A_TERM, A_STAGE = 2 * A_HALF;
-constexpr int SCALE_STEPS = 4;                                         // steps whose scales the epilogue may still need
 constexpr int W_BYTES = ROWS * STEP * 4, GATE_BYTES = STEP * 4;
 constexpr int stage_bytes(int nt) { return W_BYTES + nt * STEP * 2; }
 constexpr int part_bytes(int nt) { return nt * ROWS * 4; }                       // a tile's sums, [token][row]
 // Tiles of sums beside the stages. SPLIT: the first of a block's two parts; else bf16: none (totals in registers), fp16: the parts so far. fp16: behind a tile what its sums lack
 template <int DT, bool SPLIT> constexpr int part_tiles() { return DT == B2MOE_F16 ? 2 : SPLIT ? 1 : 0; }
 template <int DT, bool SPLIT> constexpr int stages() { return part_tiles<DT, SPLIT>() ? 3 : 4; }
-constexpr int N_BARS = 2 * 4 + 2 + 2 + 2 + SCALE_STEPS + 1;
+// fp16: the second terms of a stage's rows, behind the stages
+template <int DT> constexpr int low_bytes(int nt) { return DT == B2MOE_F16 ? nt * STEP * 2 : 0; }
+constexpr int N_BARS = 3 * 4 + 2 + 2 + 2 + 1;
 template <int DT, bool SPLIT> constexpr size_t smem_bytes(int nt) {
-    return 1024 + size_t(stages<DT, SPLIT>()) * (stage_bytes(nt) + GATE_BYTES) + part_tiles<DT, SPLIT>() * part_bytes(nt) + SCALE_STEPS * 2 * ROWS * 4 + N_BARS * 8 + 16;
+    return 1024 + size_t(stages<DT, SPLIT>()) * (stage_bytes(nt) + low_bytes<DT>(nt) + GATE_BYTES) + part_tiles<DT, SPLIT>() * part_bytes(nt) + N_BARS * 8 + 16;
 }
 static_assert(smem_bytes<B2MOE_BF16, false>(128) <= 227 * 1024 && smem_bytes<B2MOE_BF16, true>(128) <= 227 * 1024 && smem_bytes<B2MOE_F16, true>(64) <= 227 * 1024 &&
               3 * stage_bytes(64) >= 2 * part_bytes(64) && 3 * stage_bytes(128) >= part_bytes(128));
@@ -52,26 +54,14 @@ __device__ __forceinline__ float2 pair_of(uint32_t x, uint32_t y) { return make_
 __device__ __forceinline__ float2 of_bits2(unsigned long long v) { return pair_of(uint32_t(v), uint32_t(v >> 32)); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { unsigned long long r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits2(a)), "l"(bits2(b))); return of_bits2(r); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { unsigned long long r; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits2(a)), "l"(bits2(b))); return of_bits2(r); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { unsigned long long r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits2(a)), "l"(bits2(b))); return of_bits2(r); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { unsigned long long r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(bits2(a)), "l"(bits2(b)), "l"(bits2(c))); return of_bits2(r); }
 
-// the two values' terms, largest first, as a pair of 16-bit values each
-template <int DT> __device__ __forceinline__ void split_terms(float2 w, uint32_t (&v)[3]) {
-    if constexpr (DT == B2MOE_BF16) {
-        // by cutting off: 8 of the 24 bits each (an infinity leaves NaN behind, as rounding would)
+// the two values' bf16 terms, largest first, as a pair of 16-bit values each: by cutting off, 8 bits each (an infinity leaves NaN behind, as rounding would)
+template <int N> __device__ __forceinline__ void split_terms(float2 w, uint32_t (&v)[N]) {
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const uint32_t a = __float_as_uint(w.x), b = __float_as_uint(w.y);
-            v[i] = __byte_perm(a, b, 0x7632);
-            if (i < 2) w = sub2(w, pair_of(a & 0xffff0000u, b & 0xffff0000u));
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const __half2 h = __floats2half2_rn(w.x, w.y);
-            v[i] = *reinterpret_cast<const uint32_t *>(&h);
-            if (i < 2) w = sub2(w, __half22float2(h));
-        }
+    for (int i = 0; i < N; ++i) {
+        const uint32_t a = __float_as_uint(w.x), b = __float_as_uint(w.y);
+        v[i] = __byte_perm(a, b, 0x7632);
+        if (i < N - 1) w = sub2(w, pair_of(a & 0xffff0000u, b & 0xffff0000u));
     }
 }
 // (v, lack) += (sum, lack_sum), the sums so far: plainly, or with the addition's rounding error put into what the sum lacks
@@ -98,12 +88,11 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
     const int p_lo = first_part(blockIdx.z), np = first_part(blockIdx.z + 1) - p_lo;
     const int s_lo = p_lo * PART_STEPS, steps = min((h + STEP - 1) / STEP, (p_lo + np) * PART_STEPS) - s_lo;      // this block's steps
     // see part_tiles; SPLIT: the last part takes the stages' place
-    uint8_t * parts = smem + S * stage_bytes(NT);
+    uint8_t * x_low = smem + S * stage_bytes(NT), * parts = x_low + S * low_bytes<DT>(NT);
     float * gate = reinterpret_cast<float *>(parts + part_tiles<DT, SPLIT>() * part_bytes(NT));      // [stages][64]: the shared expert's gate, router row e
-    float * scales = gate + S * STEP;                                   // [steps][halves][row]
-    const uint32_t full = saddr(scales + SCALE_STEPS * 2 * ROWS), done = full + 8 * S, a_full = done + 8 * S, acc_full = a_full + 16,
-                   acc_empty = acc_full + 16, sc_full = acc_empty + 16, drain = sc_full + 8 * SCALE_STEPS;
-    uint32_t * tmem_slot = reinterpret_cast<uint32_t *>(scales + SCALE_STEPS * 2 * ROWS) + 2 * N_BARS;
+    const uint32_t full = saddr(gate + S * STEP), done = full + 8 * S, x_full = done + 8 * S, a_full = x_full + 8 * S, acc_full = a_full + 16,
+                   acc_empty = acc_full + 16, drain = acc_empty + 16;
+    uint32_t * tmem_slot = reinterpret_cast<uint32_t *>(gate + S * STEP) + 2 * N_BARS;
     volatile int * gave_up = reinterpret_cast<volatile int *>(tmem_slot + 1);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int r0 = blockIdx.y * ROWS, t0 = blockIdx.x * NT;                  // tokens on gridDim.x: any batch size
@@ -111,11 +100,9 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
 
     if (tid == 0) {
 #pragma unroll 1
-        for (int i = 0; i < S; ++i) { bar_init(full + 8 * i, 1); bar_init(done + 8 * i, 1); }
+        for (int i = 0; i < S; ++i) { bar_init(full + 8 * i, 1); bar_init(done + 8 * i, 1); bar_init(x_full + 8 * i, EPI_WARPS); }
 #pragma unroll 1
         for (int i = 0; i < 2; ++i) { bar_init(a_full + 8 * i, 8); bar_init(acc_full + 8 * i, 1); bar_init(acc_empty + 8 * i, EPI_WARPS); }
-#pragma unroll 1
-        for (int i = 0; i < SCALE_STEPS; ++i) bar_init(sc_full + 8 * i, 8);
         bar_init(drain, 1);
         *gave_up = 0;
         bar_init_fence();
@@ -152,21 +139,28 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
     } else if (warp == MMA_WARP) {
         if (elect_one()) {
             bool ok = true;
-            const uint32_t id = idesc(128, NT, F16 ? 0 : 1);
+            const uint32_t id = idesc(128, NT, 1);
 #pragma unroll 1
             for (int g = 0; g < steps; ++g) {
                 const int set = g & 1;
                 const uint32_t a = tmem + A_COL0 + set * A_STAGE, b = sw128_desc_lo(saddr(smem) + (g % S) * stage_bytes(NT) + W_BYTES);
-                // half hf's product number k with term t
-                auto mma = [&](uint32_t d, int hf, int t, int k, bool acc) { mma_f16(d, a + hf * A_HALF + t * A_TERM + 8 * k, b + 4 * hf + 2 * k, id, acc); };
-                if (!bar_wait(full + 8 * (g % S), uint32_t(g / S) & 1u) || !bar_wait(a_full + 8 * set, uint32_t(g >> 1) & 1u)) { ok = false; break; }
+                [[maybe_unused]] const uint32_t bl = sw128_desc_lo(saddr(x_low) + (g % S) * low_bytes<DT>(NT));
+                // half hf's product number k of the weights' term t with the activations' first term (low: the second)
+                auto mma = [&](uint32_t d, int hf, int t, int k, bool acc, bool low = false) { mma_f16(d, a + hf * A_HALF + t * A_TERM + 8 * k, (low ? bl : b) + 4 * hf + 2 * k, id, acc); };
+                if (!bar_wait((F16 ? x_full : full) + 8 * (g % S), uint32_t(g / S) & 1u) || !bar_wait(a_full + 8 * set, uint32_t(g >> 1) & 1u)) { ok = false; break; }
                 if constexpr (F16) {
                     if (g > 1 && !bar_wait(acc_empty + 8 * set, uint32_t((g >> 1) - 1) & 1u)) { ok = false; break; }
                     fence_after();
 #pragma unroll
-                    for (int hf = 0; hf < 2; ++hf)                     // a half step has sums of its own
+                    for (int hf = 0; hf < 2; ++hf) {                   // a half step has sums of its own
+                        const uint32_t d = tmem + set * ACC + hf * NT;
 #pragma unroll
-                        for (int t = 2; t >= 0; --t) { mma(tmem + set * ACC + hf * NT, hf, t, 0, t < 2); mma(tmem + set * ACC + hf * NT, hf, t, 1, true); }
+                        for (int t = 2; t >= 0; --t) {                 // terms t + 1 of the one and t of the other are about as large: 2^-24, 2^-16, 2^-16, 2^-8, 2^-8, 1
+                            mma(d, hf, t, 0, t < 2, true); mma(d, hf, t, 1, true, true);
+                            if (t > 0) { mma(d, hf, t, 0, true); mma(d, hf, t, 1, true); }
+                        }
+                        mma(d, hf, 0, 0, true); mma(d, hf, 0, 1, true);
+                    }
                     mma_commit(acc_full + 8 * set);
                 } else {
                     const int p = g / PART_STEPS;
@@ -204,35 +198,21 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
             for (int i = 0; i < 8; ++i)
                 asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[4 * i]), "=f"(v[4 * i + 1]), "=f"(v[4 * i + 2]), "=f"(v[4 * i + 3])
                              : "r"(src0 + s * src_step + (uint32_t(16 * i) ^ xr)) : "memory");
-            [[maybe_unused]] float up = 1.f;
-            if constexpr (F16) {
-                float most = 0.f;
-#pragma unroll
-                for (int i = 0; i < 32; ++i) most = fmaxf(most, fabsf(v[i]));
-                int ex = int(__float_as_uint(most) >> 23) - 127;        // floor(log2(most)) for a normal number
-                ex = most > 0.f && most < 3e38f ? max(-100, min(100, ex)) : 14;
-                up = __uint_as_float(uint32_t(127 + 14 - ex) << 23);
-            }
             uint32_t t[3][16];
 #pragma unroll
             for (int c = 0; c < 16; ++c) {
                 uint32_t u[3];
-                split_terms<DT>(F16 ? mul2(make_float2(v[2 * c], v[2 * c + 1]), make_float2(up, up)) : make_float2(v[2 * c], v[2 * c + 1]), u);
+                split_terms(make_float2(v[2 * c], v[2 * c + 1]), u);
                 t[0][c] = u[0]; t[1][c] = u[1]; t[2][c] = u[2];
             }
             if (g > 1 && !warp_wait(done + 8 * ((g - 2) % S), uint32_t((g - 2) / S) & 1u)) { ok = false; break; }      // the products of the step that had the place
             fence_after();
-            // (the scale's place was that of four steps before: the products of two before have waited until the epilogue was done with those)
-            if (F16) scales[((g & (SCALE_STEPS - 1)) * 2 + hf) * ROWS + row] = __uint_as_float(0x7F000000u - __float_as_uint(up));      // 1 / up
 #pragma unroll
             for (int c = 0; c < 3; ++c) tmem_st16(to + c * A_TERM, t[c]);
             tmem_st_wait();
             fence_before();
             __syncwarp();
-            if (lane == 0) {
-                bar_arrive(a_full + 8 * (g & 1));
-                if (F16) bar_arrive(sc_full + 8 * (g & (SCALE_STEPS - 1)));
-            }
+            if (lane == 0) bar_arrive(a_full + 8 * (g & 1));
         }
         if (!ok && lane == 0) *gave_up = 1;
     } else if (warp >= EPI_WARP0) {
@@ -243,7 +223,29 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
         float * const so_far = reinterpret_cast<float *>(parts) + tk0 * ROWS + row, * const last = reinterpret_cast<float *>(smem) + tk0 * ROWS + row;
         const bool in = r0 + row < rows;
         [[maybe_unused]] float tot[TOK];
+        // fp16: step g's activations as two terms, a piece of eight a thread. What a stage's second terms replace was read by products that were done when the stage was filled again
+        static_assert(!F16 || NT * STEP == EPI_WARPS * 32 * 8);
+        auto split_x = [&](int g) {
+            if (!warp_wait(full + 8 * (g % S), uint32_t(g / S) & 1u)) return false;
+            const uint32_t piece = 16 * ((warp - EPI_WARP0) * 32 + lane), at = saddr(smem) + (g % S) * stage_bytes(NT) + W_BYTES + piece;
+            uint32_t v[4], u0[4], u1[4];
+            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(at) : "memory");
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                uint32_t u[2];
+                split_terms(__half22float2(*reinterpret_cast<const __half2 *>(&v[i])), u);
+                u0[i] = u[0]; u1[i] = u[1];
+            }
+            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(u0[0]), "r"(u0[1]), "r"(u0[2]), "r"(u0[3]) : "memory");
+            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(saddr(x_low) + (g % S) * low_bytes<DT>(NT) + piece), "r"(u1[0]), "r"(u1[1]), "r"(u1[2]), "r"(u1[3]) : "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) bar_arrive(x_full + 8 * (g % S));
+            return true;
+        };
         bool ok = true;
+        if constexpr (F16)
+            for (int g = 0; g < min(2, steps) && ok; ++g) ok = split_x(g);
 #pragma unroll 1
         for (int p = 0; p < np && ok; ++p) {
             const bool is_last = p + 1 == np;
@@ -273,9 +275,8 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
 #pragma unroll 1
                 for (int g = p * PART_STEPS; g < g_hi; ++g) {
                     const int set = g & 1;
-                    if (!warp_wait(sc_full + 8 * (g & (SCALE_STEPS - 1)), uint32_t(g / SCALE_STEPS) & 1u)) { ok = false; break; }
-                    const float * sc = scales + (g & (SCALE_STEPS - 1)) * 2 * ROWS + row;
-                    const float2 sc0 = make_float2(sc[0], sc[0]), sc1 = make_float2(sc[ROWS], sc[ROWS]);
+                    // two steps ahead: the stage is filled once the products of step g - 1 are done
+                    if (g + 2 < steps && !split_x(g + 2)) { ok = false; break; }
                     if (!warp_wait(acc_full + 8 * set, uint32_t(g >> 1) & 1u)) { ok = false; break; }
                     fence_after();
 #pragma unroll
@@ -287,7 +288,7 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             float2 & s2 = sum[c / 2 + i], & l2 = lost[c / 2 + i];
-                            const float2 y = fma2(pair_of(v0[2 * i], v0[2 * i + 1]), sc0, fma2(pair_of(v1[2 * i], v1[2 * i + 1]), sc1, l2)), t = add2(s2, y);
+                            const float2 y = add2(pair_of(v0[2 * i], v0[2 * i + 1]), add2(pair_of(v1[2 * i], v1[2 * i + 1]), l2)), t = add2(s2, y);
                             l2 = sub2(y, sub2(t, s2));
                             s2 = t;
                         }
@@ -392,7 +393,7 @@ template <int DT> Shape shape_of(int rows, int n, int h) {
             const int ks = ceil_div(parts, share);
             if (ks > 8 || (ks > 1 && (share > 2 || parts > MAX_PARTS))) continue;
             // cycles of a part (measured), of a block's start and end, and of the meeting in a cluster
-            const long long part = PART_STEPS * (DT == B2MOE_F16 ? 2100 : nt == 128 ? 1650 : 1080), cost = (tiles * ks + 147) / 148 * (share * part + 6000) + (ks > 1 ? 2000 : 0);
+            const long long part = PART_STEPS * (DT == B2MOE_F16 ? 2000 : nt == 128 ? 1650 : 1080), cost = (tiles * ks + 147) / 148 * (share * part + 6000) + (ks > 1 ? 2000 : 0);
             if (best.nt == 0 || cost < least) { best = Shape{nt, ks, share}; least = cost; }
         }
     }
