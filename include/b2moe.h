@@ -375,6 +375,8 @@ B2MOE_API int32_t b2moe_place_experts(const uint64_t * counts, int32_t experts, 
  * stages 2-4, tiles per slot 1-2) where it fits; zeros = the library's own order of preference.
  * b2moe_harness_column_split: the most warps (1, 2 or 4; default 4) that the 4-bit decode kernels let share one row job
  * when a launch has only a few jobs per block; 1 switches the split off.
+ * b2moe_harness_gemm_fit: what the shared memory of a block of the grouped GEMM holds for banks of this many experts where items of item_tokens (64, 128,
+ * 256; 32: the exact form on fp32 rows) are wanted: 16 x the item's tokens + the chunks in the ring of raw weights; 0: nothing fits.
  * b2moe_harness_launches: kernel launches the library has made in this process so far. */
 enum b2moe_family { B2MOE_FAMILY_AUTO = 0, B2MOE_FAMILY_GENERIC = 1, B2MOE_FAMILY_DECODE = 2, B2MOE_FAMILY_GEMM = 3, B2MOE_FAMILY_DECODE_KERNELS = 4 };
 B2MOE_API void b2moe_harness_select(int32_t family, int32_t gemm_item_tokens);
@@ -383,6 +385,7 @@ B2MOE_API void b2moe_harness_skip_staging(int32_t on);
 B2MOE_API void b2moe_harness_overlap(int32_t on);
 B2MOE_API void b2moe_harness_ring(int32_t activation_buffers, int32_t stages, int32_t slot_tiles);
 B2MOE_API void b2moe_harness_column_split(int32_t max_warps_per_job);
+B2MOE_API int32_t b2moe_harness_gemm_fit(uint32_t type, int32_t experts, int32_t item_tokens);
 B2MOE_API uint64_t b2moe_harness_launches(void);
 
 /* ---- whole layer ----------------------------------------------------------------------------------------------

@@ -290,6 +290,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
     using D = gdec::Dec<T>;
     constexpr bool EXACT = TERMS > 0;
     using X = gdec::Exact<EXACT ? T : uint32_t(T_Q4_K)>;
+    static_assert(!EXACT || X::SCRATCH <= D::SCRATCH);
     constexpr int PLANES = EXACT ? TERMS : 1;                          // rows of B per token
     constexpr int CB = chunk_bytes<T>();
     constexpr int ITEM_TILES = MODE == 0 ? 4 : 8;                      // row tiles of one matrix that an item covers
@@ -627,7 +628,14 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                     }
                     if (lane < 16) consts[(group + 2 * (turn & 1u)) * 128 + 32 * q + 16 * m + lane] = X::consts(chunk, lane);
                 }
-                if constexpr (AHEAD) first = P::template load<2>(chunk, lane, my_scratch);
+                if constexpr (AHEAD) {
+                    if constexpr (P::SCRATCH > 0) {                     // every lane has read the first unit's constants
+                        __syncwarp();
+                        P::second_unit(pre, lane, my_scratch);
+                        __syncwarp();
+                    }
+                    first = P::template load<2>(chunk, lane, my_scratch);
+                }
                 else second = P::template load<1>(chunk, lane, my_scratch);
                 P::template step<1>(second, lane, dec_tab, pre, f);
                 tmem_st_16x256b_x4(a_addr + A_COLS / 2, f);
@@ -1006,15 +1014,14 @@ int32_t gemm_launch(uint32_t type, const Args &... args) {
     }
     return B2MOE_ERR_FORMAT;
 }
-bool gemm_fits(uint32_t type, int experts) {
-    GemmArgs a{};
+bool gemm_fits(uint32_t type, int experts, int cap, GemmArgs & a) {
     switch (type) {
-        case T_Q4_K: return gemm_fit<T_Q4_K>(experts, 64, a);
-        case T_IQ3_S: return gemm_fit<T_IQ3_S>(experts, 64, a);
-        case T_IQ3S4: return gemm_fit<T_IQ3S4>(experts, 64, a);
-        case T_IQ4_XS: return gemm_fit<T_IQ4_XS>(experts, 64, a);
-        case T_IQ4_NL: return gemm_fit<T_IQ4_NL>(experts, 64, a);
-        case T_NVFP4G: return gemm_fit<T_NVFP4G>(experts, 64, a);
+        case T_Q4_K: return gemm_fit<T_Q4_K>(experts, cap, a);
+        case T_IQ3_S: return gemm_fit<T_IQ3_S>(experts, cap, a);
+        case T_IQ3S4: return gemm_fit<T_IQ3S4>(experts, cap, a);
+        case T_IQ4_XS: return gemm_fit<T_IQ4_XS>(experts, cap, a);
+        case T_IQ4_NL: return gemm_fit<T_IQ4_NL>(experts, cap, a);
+        case T_NVFP4G: return gemm_fit<T_NVFP4G>(experts, cap, a);
     }
     return false;
 }
@@ -1023,7 +1030,10 @@ bool gemm_fits(uint32_t type, int experts) {
 
 void gemm_tc_item_tokens(int tokens) { g_item_tokens = tokens; }
 // true when the tensor-core GEMM takes banks of this type with rows of length k
-bool gemm_tc_supported(uint32_t type, int k, int experts) { return k >= G_KS && k % G_KS == 0 && gemm_fits(type, experts); }
+bool gemm_tc_supported(uint32_t type, int k, int experts) {
+    GemmArgs a{};
+    return k >= G_KS && k % G_KS == 0 && gemm_fits(type, experts, 64, a);
+}
 // scratch: the scaled fp16 copy of `rows_x` activation rows of length k and one float per row
 size_t gemm_tc_workspace_bytes(int rows_x, int k) {
     return align_up(size_t(rows_x) * k * 2, 256) + align_up(size_t(rows_x) * sizeof(float), 256);
@@ -1036,6 +1046,11 @@ size_t gemm_tc_slot_bytes(int slot_rows, int k) { return gemm_tc_workspace_bytes
 bool gemm_exact_supported(uint32_t type, int k, int experts) {
     GemmArgs a{};
     return k > 0 && k % 256 == 0 && (type == T_Q4_K ? exact_fit<T_Q4_K>(experts, 2, a) : type == T_IQ3S4 && exact_fit<T_IQ3S4>(experts, 2, a));
+}
+int32_t gemm_tc_fit(uint32_t type, int experts, int item_tokens) {
+    GemmArgs a{};
+    const bool fits = item_tokens != X_CAP ? gemm_fits(type, experts, item_tokens, a) : type == T_Q4_K ? exact_fit<T_Q4_K>(experts, 2, a) : type == T_IQ3S4 && exact_fit<T_IQ3S4>(experts, 2, a);
+    return fits ? 16 * a.cap + a.raw_slots : 0;
 }
 size_t gemm_exact_bytes(int slot_rows, int k, int dtype) { return exact_rows_bytes(slot_rows, k, dtype == B2MOE_F32 ? 2 : 1) + size_t(slot_rows) * sizeof(float); }
 int32_t gemm_exact_gateup(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_bank * sg, const b2moe_bank * su, const void * x, int x_dtype,

@@ -65,6 +65,12 @@ __device__ __forceinline__ uint32_t and_or(uint32_t v, uint32_t mask, uint32_t b
 }
 
 template <uint32_t T> struct Dec;
+// the constants of sub-block t of a unit, rows g and g + 8, in the warp's scratch
+__device__ __forceinline__ void put_constants(const uint2 (&c)[2], int lane, uint8_t * scratch) {
+    uint2 * to = reinterpret_cast<uint2 *>(scratch) + lane;
+    to[0] = c[0];
+    to[32] = c[1];
+}
 
 // ---------------------------------------------------------------------------------------------------------------
 template <> struct Dec<T_Q4_K> {
@@ -81,11 +87,13 @@ template <> struct Dec<T_Q4_K> {
     }
     // Once per chunk: lane t of a row's four lanes turns the headers of its two rows into the constants of sub-blocks t and 4 + t
     // and leaves them in the warp's scratch, two in a word (the arithmetic takes either half of a register twice at no
-    // cost; spread there, they took twice the registers and loads): [unit][row][sub-block]((S, -1024 S), (MH, ML)).
+    // cost; spread there, they took twice the registers and loads): [row][sub-block]((S, -1024 S), (MH, ML)). The scratch holds a unit; the second one's words wait in registers (Pre::late)
+    // until the first one's are read. With scratch for both, items of 128 and 256 tokens had a raw slot less (294 to 805 experts: 3 instead of 4):
+    // a layer on 512 experts, 50 tokens each 527 us, with it 514; 128 each 980, 964; on 384, 125 each 711, 699.
     // The scales and mins are exact as fp16, MH = fp16(-dmin m), ML = the exact rest. (Constants of two rows in one register,
     // fetched with shuffles and spread with byte permutes, took 45 more instructions a step, 36 of them in the integer pipe.)
-    static constexpr int SCRATCH = 2 * 16 * 4 * 8;
-    struct Pre { uint32_t D[2], magic; };
+    static constexpr int SCRATCH = 16 * 4 * 8;
+    struct Pre { uint32_t D[2], magic; uint2 late[2]; };
     __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t * scratch) {
         const int g = lane >> 2, t = lane & 3;
         const uint4 h0 = *reinterpret_cast<const uint4 *>(chunk + 2048 + 16 * g), h1 = *reinterpret_cast<const uint4 *>(chunk + 2048 + 16 * (g + 8));    // d, dmin | s[12]
@@ -95,23 +103,26 @@ template <> struct Dec<T_Q4_K> {
             const uint32_t v = __byte_perm(x, y, sel);
             return __hadd2(bits_h2((v & 0x003F003Fu) | 0x64006400u), __float2half2_rn(-1024.f));
         };
-        uint2 * to = reinterpret_cast<uint2 *>(scratch) + 4 * g + t;
-        auto unit = [&](int u, uint32_t sc0, uint32_t mn0, uint32_t sc1, uint32_t mn1) {      // a unit's four scales and four mins as bytes
+        Pre p{{__byte_perm(h0.x, 0u, 0x1010), __byte_perm(h1.x, 0u, 0x1010)}, in_register(0x64006400u)};
+        auto unit = [&](uint2 * to, uint32_t sc0, uint32_t mn0, uint32_t sc1, uint32_t mn1) {      // a unit's four scales and four mins as bytes -> (row g, row g + 8)
             __half2 sc = pick(sc0, sc1);
             const __half2 mn = pick(mn0, mn1);
             if (t & 1) sc = __hmul2(sc, __float2half2_rn(0.0625f));
             const __half2 ns = __hmul2(sc, __float2half2_rn(-1024.f)), mh = __hmul2(dm, mn), ml = __hfma2(dm, mn, __hneg2(mh));
-            to[64 * u] = make_uint2(h2_bits(__lows2half2(sc, ns)), h2_bits(__lows2half2(mh, ml)));
-            to[64 * u + 32] = make_uint2(h2_bits(__highs2half2(sc, ns)), h2_bits(__highs2half2(mh, ml)));
+            to[0] = make_uint2(h2_bits(__lows2half2(sc, ns)), h2_bits(__lows2half2(mh, ml)));
+            to[1] = make_uint2(h2_bits(__highs2half2(sc, ns)), h2_bits(__highs2half2(mh, ml)));
         };
-        unit(0, h0.y, h0.z, h1.y, h1.z);                                     // (src/formats/weight/dequant.cpp:56-64)
-        unit(1, (h0.w & 0x0F0F0F0Fu) | ((h0.y >> 2) & 0x30303030u), ((h0.w >> 4) & 0x0F0F0F0Fu) | ((h0.z >> 2) & 0x30303030u),
+        uint2 now[2];
+        unit(now, h0.y, h0.z, h1.y, h1.z);                                     // (src/formats/weight/dequant.cpp:56-64)
+        unit(p.late, (h0.w & 0x0F0F0F0Fu) | ((h0.y >> 2) & 0x30303030u), ((h0.w >> 4) & 0x0F0F0F0Fu) | ((h0.z >> 2) & 0x30303030u),
              (h1.w & 0x0F0F0F0Fu) | ((h1.y >> 2) & 0x30303030u), ((h1.w >> 4) & 0x0F0F0F0Fu) | ((h1.z >> 2) & 0x30303030u));
-        return Pre{{__byte_perm(h0.x, 0u, 0x1010), __byte_perm(h1.x, 0u, 0x1010)}, in_register(0x64006400u)};
+        put_constants(now, lane, scratch);
+        return p;
     }
+    __device__ __forceinline__ static void second_unit(const Pre & p, int lane, uint8_t * scratch) { put_constants(p.late, lane, scratch); }
     struct Raw { uint4 w, c[2]; };                                           // code words; constants of both sub-blocks of row g, of row g + 8
     template <int J> __device__ __forceinline__ static Raw load(const uint8_t * chunk, int lane, const uint8_t * scratch) {
-        const uint4 * c = reinterpret_cast<const uint4 *>(scratch) + 32 * (J >> 1) + 2 * (lane >> 2) + (J & 1);
+        const uint4 * c = reinterpret_cast<const uint4 *>(scratch) + 2 * (lane >> 2) + (J & 1);
         return Raw{plane(chunk, J, lane), {c[0], c[16]}};
     }
     template <int J> __device__ __forceinline__ static void step(const Raw & raw, int, const void *, const Pre & p, uint32_t (&f)[16]) {
@@ -143,11 +154,12 @@ template <> struct Dec<T_IQ3S4> {
         return bits_h2(and_or(POS <= 6 ? w << (6 - POS) : w >> (POS - 6), 0x03C003C0u, one));
     }
     // the constants of (row, sub-block) in the warp's scratch, as for Q4_K: (32 (1 + 2 s), -47 (1 + 2 s))
-    static constexpr int SCRATCH = 2 * 16 * 4 * 8;
-    struct Pre { uint32_t D[2], one; };
+    static constexpr int SCRATCH = 16 * 4 * 8;
+    struct Pre { uint32_t D[2], one; uint2 late[2]; };
     __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t * scratch) {
         const int g = lane >> 2, t = lane & 3;
         Pre p;
+        uint2 now[2];
         p.one = in_register(0x3C003C00u);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
@@ -156,16 +168,18 @@ template <> struct Dec<T_IQ3S4> {
             for (int u = 0; u < 2; ++u) {
                 // the 4-bit scale under the exponent of 1: 1 + s / 16
                 const __half2 s = bits_h2((((sc >> (16 * u)) & 15u) * 0x00400040u) | 0x3C003C00u);
-                reinterpret_cast<uint2 *>(scratch)[64 * u + 4 * (g + 8 * r) + t] = make_uint2(h2_bits(__hfma2(s, __float2half2_rn(1024.f), __float2half2_rn(-992.f))),
-                                                                                            h2_bits(__hfma2(s, __float2half2_rn(-1504.f), __float2half2_rn(1457.f))));
+                (u ? p.late : now)[r] = make_uint2(h2_bits(__hfma2(s, __float2half2_rn(1024.f), __float2half2_rn(-992.f))),
+                                                 h2_bits(__hfma2(s, __float2half2_rn(-1504.f), __float2half2_rn(1457.f))));
             }
             p.D[r] = uint32_t(*reinterpret_cast<const unsigned short *>(chunk + 2112 + 2 * (g + 8 * r))) * 0x10001u;
         }
+        put_constants(now, lane, scratch);
         return p;
     }
+    __device__ __forceinline__ static void second_unit(const Pre & p, int lane, uint8_t * scratch) { put_constants(p.late, lane, scratch); }
     struct Raw { uint4 w, c[2]; };
     template <int J> __device__ __forceinline__ static Raw load(const uint8_t * chunk, int lane, const uint8_t * scratch) {
-        const uint4 * c = reinterpret_cast<const uint4 *>(scratch) + 32 * (J >> 1) + 2 * (lane >> 2) + (J & 1);       // both sub-blocks of the step
+        const uint4 * c = reinterpret_cast<const uint4 *>(scratch) + 2 * (lane >> 2) + (J & 1);       // both sub-blocks of the step
         return Raw{plane(chunk, J, lane), {c[0], c[16]}};
     }
     template <int J> __device__ __forceinline__ static void step(const Raw & raw, int, const void *, const Pre & p, uint32_t (&f)[16]) {

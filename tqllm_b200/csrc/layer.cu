@@ -43,6 +43,7 @@ int32_t gemm_tc_gateup(const b2moe_bank *, const b2moe_bank *, const b2moe_bank 
 int32_t gemm_tc_down(const b2moe_bank *, const b2moe_bank *, const void *, int x_dtype, bool per_token, const int *, int, int, int, long long live, void *,
                      int y_dtype, void *, bool plan_ready, cudaStream_t);
 void gemm_tc_item_tokens(int tokens);
+int32_t gemm_tc_fit(uint32_t type, int experts, int item_tokens);
 bool gemm_exact_supported(uint32_t type, int k, int experts);
 size_t gemm_exact_bytes(int slot_rows, int k, int dtype);
 int32_t gemm_exact_gateup(const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const void *, int, const int *, int, int, int, void *, int act_dtype,
@@ -177,6 +178,7 @@ extern "C" B2MOE_API void b2moe_harness_skip_staging(int32_t on) { dec4_skip_sta
 extern "C" B2MOE_API void b2moe_harness_ring(int32_t nbuf, int32_t stages, int32_t slot_tiles) { dec4_ring(nbuf, stages, slot_tiles); }
 extern "C" B2MOE_API void b2moe_harness_column_split(int32_t max_warps_per_job) { dec4_ksplit_max(max_warps_per_job); }
 extern "C" B2MOE_API void b2moe_harness_overlap(int32_t on) { g_overlap = on != 0; }
+extern "C" B2MOE_API int32_t b2moe_harness_gemm_fit(uint32_t type, int32_t experts, int32_t item_tokens) { return gemm_tc_fit(type, experts, item_tokens); }
 extern "C" B2MOE_API uint64_t b2moe_harness_launches(void) { return g_launch_count; }
 
 extern "C" B2MOE_API size_t b2moe_expert_workspace_bytes(uint32_t type, int32_t rows_x, int32_t k, int32_t x_dtype) {
