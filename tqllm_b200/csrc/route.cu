@@ -57,7 +57,7 @@ __global__ void router_k(const float * __restrict__ w, const float * __restrict_
 // and fp32 rows a chain of products does not carry the sum: the leading products of 16 columns start from zero and are added with
 // rounding, the others, 2^-8 of them and less, have sums of their own. Relative error against fp64 (2-norm; a scalar fp32 loop,
 // one chain for all, this): h = 768 0.88e-7, 1.7e-7, 0.81e-7; 4096 1.28e-7, 3.3e-7 (fp32 4.0e-7), 0.9e-7; in router_tile_k 1.04e-7 where one chain had
-// 1.37e-6 (fp32 1.68e-6). bf16 rows, whose products lost three bits of the fp32 chain from the start, keep their one chain (2.2e-7; 8.2e-7).
+// 1.37e-6 (fp32 1.68e-6). bf16 rows, whose products lost three bits of the fp32 chain from the start, keep their one chain (2.2e-7).
 // One block = 16 router rows x 8 J tokens; its 16 warps split the hidden dimension and add their partial tiles in shared
 // memory in warp order (a token's bits do not depend on J). J is the smallest of 1, 2, 4, 8 that takes the batch in one block or leaves
 // at most a block per SM: with J = 8 one token pays for 64.
@@ -661,17 +661,32 @@ int32_t router_launch(const float * w, const float * shared, const void * xv, fl
     auto mma_blocks = [&](int tokens) { return (long long)ceil_div(rows, 16) * ceil_div(n, tokens) * ks; };
     // 16-bit rows go to router_tc_k where router_mma_k, with its 64 tokens a block, has more than two blocks per SM, or more than one and enough rows to fill most of a tile of
     // 128. Before / router_tc_k, us: bf16 2048 columns x 512 experts, 256 tokens 17.8 / 10.1, 509 23.5 / 11.2, 4096 87 / 32; 4096 x 128, 8192 tokens 163 / 40; 3072 x 256, 2047
-    // tokens 57 / 20; fp16 600 x 3072 x 256 32 / 15.5, 4096 x 2048 x 512 187 / 73, 600 x 2560 x 60 (160 blocks) 21.9 / 13.7, 4096 x 5120 x 16 (256 blocks of 16 rows) 31 / 64. Not where
-    // the other kernels are more precise (2-norm against fp64): bf16 below 256 tokens (1.3e-7 to 2.2e-7, here 4.7e-7), fp16 below 768 columns (6.9e-8, here 7.2e-8; from there on 8.1e-8 to 1.04e-7).
+    // tokens 57 / 20; fp16 600 x 3072 x 256 32 / 15.5, 4096 x 2048 x 512 187 / 73, 600 x 2560 x 60 (160 blocks) 21.9 / 13.7. Not where the other kernels are more precise (2-norm against
+    // fp64): bf16 below 256 tokens (1.3e-7 to 2.2e-7, here 4.7e-7), fp16 below 768 columns (6.9e-8, here 7.2e-8; from there on 8.1e-8 to 1.04e-7).
+    // bf16 rows between one and two blocks per SM and up to 48 router rows: the fine form (7.2e-8; router_mma_k up to 2.7e-7) where it costs fewer cycles. router_tile_k, which served them once at
+    // 8.2e-7 / router_mma_k / fine, us: 2048 x 48, 1024 tokens 12.7 / 17.6 / 12.3; 1536 x 48, 1500 14.1 / 23.9 / 12.5; 1024 x 32, 2047 13.9 / 14.9 / 12.7; 256 x 32, 8192 10.5 / 12.1 / 7.8; dearer:
+    // 5120 x 32, 2047 55 / 26.6 / 39. Up to 16 rows a tile of 128 stays empty: router_mma_k (1.3e-7 and more exact than the chains) where it costs less than they: 3072 x 8, 6000 tokens
+    // 29 / 37, 5120 x 8, 4096 (256 blocks) 25 / 36, but 2048 x 16, 8192 35 / 19. Cycles of router_mma_k: fitted to 300 sizes of 256 to 5120 columns, to 10 % (2-norm).
+    // fp16 rows stay here with few rows too, as it is the most exact (8 rows x 3072, 8192 tokens: 70 us, router_mma_k 45 at 8.9e-8; router_tile_k 93 at 9.7e-8).
     // Rows of fp32, and short ones of fp16: tiles once router_mma_k has more than two blocks per SM. router_mma_k / tiles, us: 1024 columns x 32 experts, fp16,
     // 600 tokens 8.9 / 17.7, 2047 (256 blocks) 16.8 / 18.0, 4096 (512 blocks) 32 / 18; 2560 x 60, 600 tokens (160) 22.8 / 31, 2047 (512) 46 / 32;
     // 3072 x 256, 256 tokens (256) 25 / 31, 300 (320) 36 / 31; 256 x 32 4096 tokens (128) 8.3 / 22.
     // A grid holds 65,535 blocks of tokens; what is more than that many takes the scalar loop, as everything else that does not fit.
     constexpr int GRID_Y = 65535;
-    if constexpr (DT != B2MOE_F32)
-        if (h % RT_K == 0 && (mma_blocks(64) > 2 * ROUTER_SMS || (mma_blocks(64) > ROUTER_SMS && rows > 48)) && (DT == B2MOE_F16 ? h >= 768 : n >= 256))
-            return rtc::launch<DT>(w, shared, x, logits, ld, h, e, rows, n, s);
-    if constexpr (DT != B2MOE_BF16) if (h % RT_K == 0 && mma_blocks(64) > 2 * ROUTER_SMS && ceil_div(n, RT_TOK) <= GRID_Y) {
+    const long long blocks = mma_blocks(64);
+    if constexpr (DT == B2MOE_F16)
+        if (h % RT_K == 0 && h >= 768 && (blocks > 2 * ROUTER_SMS || (blocks > ROUTER_SMS && rows > 48)))
+            return rtc::launch<DT, true>(w, shared, x, logits, ld, h, e, rows, n, s);
+    if constexpr (DT == B2MOE_BF16)
+        if (h % RT_K == 0 && n >= 256 && blocks > ROUTER_SMS) {
+            const long long mma_cycles = 5000 + blocks * (8900 + 156LL * (h / ks) / 10) / ROUTER_SMS;
+            auto below_mma = [&](const rtc::Shape & p) { return p.cycles < mma_cycles || ceil_div(n, 64) > GRID_Y; };
+            if (rows > 48 || (blocks > 2 * ROUTER_SMS && (rows > 16 || below_mma(rtc::shape_of<DT, false>(rows, n, h)))))
+                return rtc::launch<DT, false>(w, shared, x, logits, ld, h, e, rows, n, s);
+            if (blocks <= 2 * ROUTER_SMS && rows > 16 && below_mma(rtc::shape_of<DT, true>(rows, n, h)))
+                return rtc::launch<DT, true>(w, shared, x, logits, ld, h, e, rows, n, s);
+        }
+    if constexpr (DT != B2MOE_BF16) if (h % RT_K == 0 && blocks > 2 * ROUTER_SMS && ceil_div(n, RT_TOK) <= GRID_Y) {
         const dim3 tiles(ceil_div(rows, RT_ROWS), ceil_div(n, RT_TOK), 1);
         const int n_part = ceil_div(h, RT_COLS), share = ceil_div(n_part, 8), ks = ceil_div(n_part, share);      // at most eight blocks, no more than the shares need
         const size_t smem = rt_stages_bytes<DT>() + size_t(share - 1) * RT_PART;

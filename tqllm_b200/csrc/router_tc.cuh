@@ -12,6 +12,8 @@
 // are one chain of 32, the others (2^-8 of them and less) have sums of their own; the parts are added in column order. fp16 rows: one chain per half
 // step, smallest terms first (two of its twelve products meet a sum of full size); half steps and parts are added in fp32 with the rounding errors carried along.
 //
+// FINE: the sums of half steps with compensation, as for fp16 rows, for bf16 ones: 7.2e-8 where the chains of a part give 4.7e-7, and 1500 cycles a step of 64 tokens.
+//
 // What bounds it: the chain from a step's copy over its split to the products, 1650 cycles a step of 128 bf16 tokens, 1080 of 64 (most of it the split by two warps a
 // scheduler), where the products alone take 768 and 516; 2000 of 64 fp16 tokens, whose products take twice as long and whose sums are read at every step. Two groups of splitting warps on steps in turn: 34.2 us against 31.9 (4096 x 2048 x 512 bf16; three stages instead of four for it); the
 // router rows loaded straight from global memory into fragments, no shared memory: 39.0; one accumulator for all terms: 24.9, at 1.65e-6 (this 4.7e-7).
@@ -37,15 +39,15 @@ constexpr int W_BYTES = ROWS * STEP * 4, GATE_BYTES = STEP * 4;
 constexpr int stage_bytes(int nt) { return W_BYTES + nt * STEP * 2; }
 constexpr int part_bytes(int nt) { return nt * ROWS * 4; }                       // a tile's sums, [token][row]
 // Tiles of sums beside the stages. SPLIT: the first of a block's two parts; else bf16: none (totals in registers), fp16: the parts so far. fp16: behind a tile what its sums lack
-template <int DT, bool SPLIT> constexpr int part_tiles() { return DT == B2MOE_F16 ? 2 : SPLIT ? 1 : 0; }
-template <int DT, bool SPLIT> constexpr int stages() { return part_tiles<DT, SPLIT>() ? 3 : 4; }
+template <bool FINE, bool SPLIT> constexpr int part_tiles() { return FINE ? 2 : SPLIT ? 1 : 0; }
+template <bool FINE, bool SPLIT> constexpr int stages() { return part_tiles<FINE, SPLIT>() ? 3 : 4; }
 // fp16: the second terms of a stage's rows, behind the stages
 template <int DT> constexpr int low_bytes(int nt) { return DT == B2MOE_F16 ? nt * STEP * 2 : 0; }
 constexpr int N_BARS = 3 * 4 + 2 + 2 + 2 + 1;
-template <int DT, bool SPLIT> constexpr size_t smem_bytes(int nt) {
-    return 1024 + size_t(stages<DT, SPLIT>()) * (stage_bytes(nt) + low_bytes<DT>(nt) + GATE_BYTES) + part_tiles<DT, SPLIT>() * part_bytes(nt) + N_BARS * 8 + 16;
+template <int DT, bool FINE, bool SPLIT> constexpr size_t smem_bytes(int nt) {
+    return 1024 + size_t(stages<FINE, SPLIT>()) * (stage_bytes(nt) + low_bytes<DT>(nt) + GATE_BYTES) + part_tiles<FINE, SPLIT>() * part_bytes(nt) + N_BARS * 8 + 16;
 }
-static_assert(smem_bytes<B2MOE_BF16, false>(128) <= 227 * 1024 && smem_bytes<B2MOE_BF16, true>(128) <= 227 * 1024 && smem_bytes<B2MOE_F16, true>(64) <= 227 * 1024 &&
+static_assert(smem_bytes<B2MOE_BF16, false, false>(128) <= 227 * 1024 && smem_bytes<B2MOE_BF16, false, true>(128) <= 227 * 1024 && smem_bytes<B2MOE_F16, true, true>(64) <= 227 * 1024 &&
               3 * stage_bytes(64) >= 2 * part_bytes(64) && 3 * stage_bytes(128) >= part_bytes(128));
 
 // two fp32 operations in one instruction
@@ -75,12 +77,13 @@ template <bool EXACT> __device__ __forceinline__ void add_part(float & v, float 
 }
 struct Maps { CUtensorMap w, x, gate; };
 
-template <int DT, int NT, bool SPLIT>
+template <int DT, int NT, bool SPLIT, bool FINE>
 __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const float * shared, const typename Elem<DT>::type * x, float * logits, int ld, int h, int e, int rows,
                                                           int n, const __grid_constant__ Maps maps) {
     namespace cg = cooperative_groups;
     constexpr bool F16 = DT == B2MOE_F16;
-    constexpr int S = stages<DT, SPLIT>();
+    static_assert(!F16 || FINE);
+    constexpr int S = stages<FINE, SPLIT>();
     extern __shared__ uint8_t rtc_raw[];
     uint8_t * smem = rtc_raw + (-saddr(rtc_raw) & 1023u);
     const int ks = gridDim.z, n_part = (h + STEP * PART_STEPS - 1) / (STEP * PART_STEPS);
@@ -89,7 +92,7 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
     const int s_lo = p_lo * PART_STEPS, steps = min((h + STEP - 1) / STEP, (p_lo + np) * PART_STEPS) - s_lo;      // this block's steps
     // see part_tiles; SPLIT: the last part takes the stages' place
     uint8_t * x_low = smem + S * stage_bytes(NT), * parts = x_low + S * low_bytes<DT>(NT);
-    float * gate = reinterpret_cast<float *>(parts + part_tiles<DT, SPLIT>() * part_bytes(NT));      // [stages][64]: the shared expert's gate, router row e
+    float * gate = reinterpret_cast<float *>(parts + part_tiles<FINE, SPLIT>() * part_bytes(NT));      // [stages][64]: the shared expert's gate, router row e
     const uint32_t full = saddr(gate + S * STEP), done = full + 8 * S, x_full = done + 8 * S, a_full = x_full + 8 * S, acc_full = a_full + 16,
                    acc_empty = acc_full + 16, drain = acc_empty + 16;
     uint32_t * tmem_slot = reinterpret_cast<uint32_t *>(gate + S * STEP) + 2 * N_BARS;
@@ -148,7 +151,7 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
                 // half hf's product number k of the weights' term t with the activations' first term (low: the second)
                 auto mma = [&](uint32_t d, int hf, int t, int k, bool acc, bool low = false) { mma_f16(d, a + hf * A_HALF + t * A_TERM + 8 * k, (low ? bl : b) + 4 * hf + 2 * k, id, acc); };
                 if (!bar_wait((F16 ? x_full : full) + 8 * (g % S), uint32_t(g / S) & 1u) || !bar_wait(a_full + 8 * set, uint32_t(g >> 1) & 1u)) { ok = false; break; }
-                if constexpr (F16) {
+                if constexpr (FINE) {
                     if (g > 1 && !bar_wait(acc_empty + 8 * set, uint32_t((g >> 1) - 1) & 1u)) { ok = false; break; }
                     fence_after();
 #pragma unroll
@@ -156,8 +159,8 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
                         const uint32_t d = tmem + set * ACC + hf * NT;
 #pragma unroll
                         for (int t = 2; t >= 0; --t) {                 // terms t + 1 of the one and t of the other are about as large: 2^-24, 2^-16, 2^-16, 2^-8, 2^-8, 1
-                            mma(d, hf, t, 0, t < 2, true); mma(d, hf, t, 1, true, true);
-                            if (t > 0) { mma(d, hf, t, 0, true); mma(d, hf, t, 1, true); }
+                            if (F16) { mma(d, hf, t, 0, t < 2, true); mma(d, hf, t, 1, true, true); }
+                            if (t > 0) { mma(d, hf, t, 0, F16 || t < 2); mma(d, hf, t, 1, true); }
                         }
                         mma(d, hf, 0, 0, true); mma(d, hf, 0, 1, true);
                     }
@@ -253,10 +256,10 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
             auto put = [&](int i, float v, float lack = 0.f) {
                 if (SPLIT) {
                     (is_last ? last : so_far)[i * ROWS] = v;
-                    if (F16) (is_last ? last : so_far)[(NT + i) * ROWS] = lack;
+                    if (FINE) (is_last ? last : so_far)[(NT + i) * ROWS] = lack;
                     return;
                 }
-                if (F16) {
+                if (FINE) {
                     if (p > 0) add_part<true>(v, lack, so_far[i * ROWS], so_far[(NT + i) * ROWS]);
                     if (!is_last) { so_far[i * ROWS] = v; so_far[(NT + i) * ROWS] = lack; }
                 } else {
@@ -264,9 +267,9 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
                     tot[i] = v;
                 }
                 const int tok = t0 + tk0 + i;
-                if (is_last && in && tok < n) logits[size_t(tok) * ld + r0 + row] = checked_logit<DT>(F16 ? v + lack : v, w, shared, x, r0 + row, tok, e, h);
+                if (is_last && in && tok < n) logits[size_t(tok) * ld + r0 + row] = checked_logit<DT>(FINE ? v + lack : v, w, shared, x, r0 + row, tok, e, h);
             };
-            if constexpr (F16) {
+            if constexpr (FINE) {
                 // The steps' sums are added with their rounding errors carried along (Kahan; lost: what the sum lacks): the plain additions of a part would be the largest error
                 float2 sum[TOK / 2], lost[TOK / 2];
 #pragma unroll
@@ -276,7 +279,7 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
                 for (int g = p * PART_STEPS; g < g_hi; ++g) {
                     const int set = g & 1;
                     // two steps ahead: the stage is filled once the products of step g - 1 are done
-                    if (g + 2 < steps && !split_x(g + 2)) { ok = false; break; }
+                    if (F16 && g + 2 < steps && !split_x(g + 2)) { ok = false; break; }
                     if (!warp_wait(acc_full + 8 * set, uint32_t(g >> 1) & 1u)) { ok = false; break; }
                     fence_after();
 #pragma unroll
@@ -364,42 +367,44 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
                     v[j] = l[j] = 0.f;
                     if (q + j < n_part) {
                         asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[j]) : "r"(place[q + j] + off) : "memory");
-                        if (F16) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(l[j]) : "r"(place[q + j] + off + part_bytes(NT)) : "memory");
+                        if (FINE) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(l[j]) : "r"(place[q + j] + off + part_bytes(NT)) : "memory");
                     }
                 }
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
                     if (q + j < n_part) {
-                        if (q + j > 0) add_part<F16>(v[j], l[j], sum, lack);
+                        if (q + j > 0) add_part<FINE>(v[j], l[j], sum, lack);
                         sum = v[j];
                         lack = l[j];
                     }
             }
-            logits[size_t(t0 + tk) * ld + r0 + r] = checked_logit<DT>(bad ? CUDART_NAN_F : F16 ? sum + lack : sum, w, shared, x, r0 + r, t0 + tk, e, h);
+            logits[size_t(t0 + tk) * ld + r0 + r] = checked_logit<DT>(bad ? CUDART_NAN_F : FINE ? sum + lack : sum, w, shared, x, r0 + r, t0 + tk, e, h);
         }
         cluster.sync();                                                // the blocks' tiles stay alive until every block has read them
     }
 }
 
-// The shape of a launch: tokens a block and blocks a tile's columns are split over, the pair with the fewest cycles
-struct Shape { int nt, ks, share; };
-template <int DT> Shape shape_of(int rows, int n, int h) {
+// The shape of a launch: tokens a block and blocks a tile's columns are split over, the pair with the fewest cycles. Clusters of such blocks that a B200 holds at once, by size
+// (cudaOccupancyMaxActiveClusters; a cluster stays inside a GPC): 16 clusters of 8 take two rounds. With 148 blocks of any cluster: bf16 4096 x 128, 1024 tokens 21.7 us, 12.7; fp16 1536 x 256, 3000 42, 29
+constexpr int CLUSTERS[9] = {0, ROUTER_SMS, 74, 45, 33, 26, 22, 15, 15};
+struct Shape { int nt, ks; long long cycles; };
+template <int DT, bool FINE> Shape shape_of(int rows, int n, int h) {
     const int parts = ceil_div(h, STEP * PART_STEPS);
-    Shape best{0, 1, parts};
-    long long least = 0;
-    for (int nt = DT == B2MOE_F16 ? 64 : 128; nt >= 64; nt -= 64) {
+    Shape best{0, 1, 0};
+    for (int nt = FINE ? 64 : 128; nt >= 64; nt -= 64) {
         const long long tiles = (long long)ceil_div(rows, ROWS) * ceil_div(n, nt);
         for (int share = parts; share >= 1; --share) {
             const int ks = ceil_div(parts, share);
             if (ks > 8 || (ks > 1 && (share > 2 || parts > MAX_PARTS))) continue;
-            // cycles of a part (measured), of a block's start and end, and of the meeting in a cluster
-            const long long part = PART_STEPS * (DT == B2MOE_F16 ? 2000 : nt == 128 ? 1650 : 1080), cost = (tiles * ks + 147) / 148 * (share * part + 6000) + (ks > 1 ? 2000 : 0);
-            if (best.nt == 0 || cost < least) { best = Shape{nt, ks, share}; least = cost; }
+            // cycles of a step (measured), of a block's start and end, and of the meeting in a cluster
+            const int step = DT == B2MOE_F16 ? 2000 : FINE ? 1500 : nt == 128 ? 1650 : 1080;
+            const long long cost = (tiles + CLUSTERS[ks] - 1) / CLUSTERS[ks] * (share * PART_STEPS * step + 6000) + (ks > 1 ? 2000 : 0);
+            if (best.nt == 0 || cost < best.cycles) best = Shape{nt, ks, cost};
         }
     }
     return best;
 }
-template <int DT, int NT> int32_t launch_nt(const Shape & p, const float * w, const float * shared, const typename Elem<DT>::type * x, float * logits, int ld, int h, int e,
+template <int DT, int NT, bool FINE> int32_t launch_nt(const Shape & p, const float * w, const float * shared, const typename Elem<DT>::type * x, float * logits, int ld, int h, int e,
                                             int rows, int n, cudaStream_t s) {
     Maps maps;
     const cuuint64_t xd[2] = {cuuint64_t(h), cuuint64_t(n)}, wd[2] = {cuuint64_t(h), cuuint64_t(e)}, gd[2] = {cuuint64_t(h), 1}, xs[1] = {cuuint64_t(h) * 2}, ws[1] = {cuuint64_t(h) * 4};
@@ -407,17 +412,17 @@ template <int DT, int NT> int32_t launch_nt(const Shape & p, const float * w, co
     if (!encode_map(maps.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x, xd, xs, xb, CU_TENSOR_MAP_SWIZZLE_128B) ||       // (copied as they are: bf16 is as good)
         !encode_map(maps.w, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, w, wd, ws, wb, CU_TENSOR_MAP_SWIZZLE_128B) ||
         !encode_map(maps.gate, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, shared ? shared : w, gd, ws, gb, CU_TENSOR_MAP_SWIZZLE_NONE)) return B2MOE_ERR_CUDA;
-    const size_t smem = p.ks > 1 ? smem_bytes<DT, true>(NT) : smem_bytes<DT, false>(NT);
-    const auto kernel = p.ks > 1 ? router_tc_k<DT, NT, true> : router_tc_k<DT, NT, false>;
+    const size_t smem = p.ks > 1 ? smem_bytes<DT, FINE, true>(NT) : smem_bytes<DT, FINE, false>(NT);
+    const auto kernel = p.ks > 1 ? router_tc_k<DT, NT, true, FINE> : router_tc_k<DT, NT, false, FINE>;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return B2MOE_ERR_CUDA;
     return launch_cluster_z(kernel, dim3(ceil_div(n, NT), ceil_div(rows, ROWS), p.ks), THREADS, smem, s, w, shared, x, logits, ld, h, e, rows, n, maps);
 }
 // 16-bit rows; h a multiple of 8 (strides of the maps)
-template <int DT> int32_t launch(const float * w, const float * shared, const typename Elem<DT>::type * x, float * logits, int ld, int h, int e, int rows, int n, cudaStream_t s) {
-    const Shape p = shape_of<DT>(rows, n, h);
-    if constexpr (DT == B2MOE_BF16)
-        if (p.nt == 128) return launch_nt<DT, 128>(p, w, shared, x, logits, ld, h, e, rows, n, s);
-    return launch_nt<DT, 64>(p, w, shared, x, logits, ld, h, e, rows, n, s);
+template <int DT, bool FINE> int32_t launch(const float * w, const float * shared, const typename Elem<DT>::type * x, float * logits, int ld, int h, int e, int rows, int n, cudaStream_t s) {
+    const Shape p = shape_of<DT, FINE>(rows, n, h);
+    if constexpr (!FINE)
+        if (p.nt == 128) return launch_nt<DT, 128, FINE>(p, w, shared, x, logits, ld, h, e, rows, n, s);
+    return launch_nt<DT, 64, FINE>(p, w, shared, x, logits, ld, h, e, rows, n, s);
 }
 
 }  // namespace rtc
