@@ -282,7 +282,7 @@ __device__ __forceinline__ int route_and_plan(const Dec4Args & p, const Dec4Rout
         if (tid == 0) {
             offsets[e1] = A + in.shared_count;
             pass_list[experts + shared] = passes + shared;
-            p.plan[PLAN_NGROUPED] = A + in.shared_count; p.plan[PLAN_NACTIVE] = experts + shared; p.plan[PLAN_NPASS] = passes + shared; p.plan[PLAN_STATUS] = 0;
+            p.plan[PLAN_NGROUPED] = A + in.shared_count; p.plan[PLAN_NACTIVE] = experts + shared; p.plan[PLAN_NPASS] = passes + shared;      // (its status word: cleared by the launch before)
         }
     }
     return passes + shared;
@@ -870,7 +870,7 @@ int32_t dec4_gateup(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_
     return B2MOE_ERR_FORMAT;
 }
 // gate/up that routes for itself (dec4_k, ROUTED): up to eight tokens, a launch of a few jobs per block, experts that a warp keeps in registers. *took = false and B2MOE_OK: the shape does
-// not fit, the caller takes a routing launch and dec4_gateup
+// not fit, the caller takes a routing launch and dec4_gateup. The plan's status word has been cleared by an earlier launch
 int32_t dec4_gateup_routed(const b2moe_bank * gate, const b2moe_bank * up, const b2moe_bank * sg, const b2moe_bank * su, const void * x, int x_dtype, int gating, const float * logits, int ld,
                            const float * bias, int norm, float scale, int * ids, float * weights, float * shared_weights, int * plan, int n, int topk, int shared_tokens, void * act, cudaStream_t s, bool * took) {
     *took = false;

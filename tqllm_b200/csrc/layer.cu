@@ -21,6 +21,7 @@ size_t dec4_workspace_bytes(int rows_x, int k);
 int32_t dec4_gateup(const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const b2moe_bank *, const void *, int, const int *, int,
                     int, int, void *, int act_dtype, void *, cudaStream_t, bool x_staged);
 void dec4_stage_target(uint32_t type, void * ws, int n, int k, uint8_t ** rows, float ** inv_scale, int * bits);
+int32_t router_logits(const float * router_w, const float * shared_gate, const void * x, int32_t x_dtype, float * logits, int32_t ld, int32_t hidden, int32_t experts, int32_t n, int * clear, bool * cleared, cudaStream_t);
 bool route_cluster_fits(int experts, int topk, int n);
 int32_t route_plan_stage(int gating, const float * logits, int ld, const float * bias, int * ids, float * weights, float * shared_weights,
                          int experts, int topk, int norm, float scale, int n, int shared_first, int shared_count, int * plan, const void * x,
@@ -370,8 +371,9 @@ static int32_t layer_forward(const b2moe_layer * L, const void * x, int32_t x_dt
     const int ld = L->experts + 1, sh = L->has_shared ? n : 0;
     const bool gated_shared = L->has_shared && L->shared_gate_vec;
 
-    if (int32_t rc = b2moe_router(L->router_w, gated_shared ? L->shared_gate_vec : nullptr, x, x_dtype, logits, ld, L->hidden, L->experts,
-                                  n, stream)) return rc;
+    // the plan's status word is cleared here for the gate/up launch that routes for itself: there, any block may report a wait that ran out before another one has begun
+    bool cleared;
+    if (int32_t rc = router_logits(L->router_w, gated_shared ? L->shared_gate_vec : nullptr, x, x_dtype, logits, ld, L->hidden, L->experts, n, plan + PLAN_STATUS, &cleared, as_stream(stream))) return rc;
     if (L->gating == B2MOE_SIGMOID && gated_shared) return B2MOE_ERR_SHAPE;   // the sigmoid family adds its shared expert unscaled (moe_common.cu:191)
     void * es = base + ws.expert_scratch;
     const size_t es_bytes = workspace_bytes - ws.expert_scratch;
@@ -383,8 +385,9 @@ static int32_t layer_forward(const b2moe_layer * L, const void * x, int32_t x_dt
         !exact_gateup(&L->gate, x_dtype, (long long)n * L->topk, n * L->topk + sh, workspace_bytes - ws.y, &slots)) {
         // a few tokens: the gate/up launch routes for itself
         if (int32_t rc = check_gateup(&L->gate, &L->up, &L->sh_gate, &L->sh_up, x, x_dtype, plan, n, L->topk, sh, act)) return rc;
-        if (int32_t rc = dec4_gateup_routed(&L->gate, &L->up, &L->sh_gate, &L->sh_up, x, x_dtype, L->gating, logits, ld, L->sel_bias, L->norm, L->scale, ids, weights,
-                                            gated_shared ? shw : nullptr, plan, n, L->topk, sh, act, as_stream(stream), &routed)) return rc;
+        if (cleared)
+            if (int32_t rc = dec4_gateup_routed(&L->gate, &L->up, &L->sh_gate, &L->sh_up, x, x_dtype, L->gating, logits, ld, L->sel_bias, L->norm, L->scale, ids, weights,
+                                                gated_shared ? shw : nullptr, plan, n, L->topk, sh, act, as_stream(stream), &routed)) return rc;
         if (!routed) {
             uint8_t * rows;
             float * inv;

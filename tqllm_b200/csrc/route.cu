@@ -116,7 +116,7 @@ template <int DT> __device__ __forceinline__ float checked_logit(float s, const 
 template <int DT, int J>
 __global__ void __launch_bounds__(RM_WARPS * 32) router_mma_k(const float * __restrict__ w, const float * __restrict__ shared,
                                                                 const typename Elem<DT>::type * x, float * logits, int ld,
-                                                                int h, int e, int rows, int n) {
+                                                                int h, int e, int rows, int n, int * clear) {
     constexpr int XT = x_terms<DT>(), TOK = 8 * J;
     __shared__ float part[RM_PART][16][65];
     __shared__ float tile[16][65];                                      // this block's sums over its slice of the columns
@@ -211,6 +211,7 @@ __global__ void __launch_bounds__(RM_WARPS * 32) router_mma_k(const float * __re
                 logits[size_t(t0 + c) * ld + r0 + r] = checked_logit<DT>(s, w, shared, x, r0 + r, t0 + c, e, h);
             }
         }
+        if (clear && blockIdx.x + blockIdx.y == 0 && threadIdx.x == blockDim.x - 1) *clear = 0;
     }
     cluster.sync();                                                     // the other blocks' tiles stay alive until block 0 has read them
 }
@@ -652,8 +653,9 @@ int32_t launch_cluster_z(void (*kernel)(KArgs...), dim3 grid, int threads, size_
 #include "router_tc.cuh"
 namespace b2 {
 namespace {
+// clear (may be null): a word that router_mma_k sets to 0; *cleared tells whether that kernel took the call
 template <int DT>
-int32_t router_launch(const float * w, const float * shared, const void * xv, float * logits, int ld, int h, int e, int rows, int n, cudaStream_t s) {
+int32_t router_launch(const float * w, const float * shared, const void * xv, float * logits, int ld, int h, int e, int rows, int n, int * clear, bool * cleared, cudaStream_t s) {
     const auto * x = static_cast<const typename Elem<DT>::type *>(xv);
     // router_mma_k splits the hidden dimension over a cluster of up to 4 blocks while every block keeps at least 256 columns
     int ks = 1;
@@ -698,8 +700,9 @@ int32_t router_launch(const float * w, const float * shared, const void * xv, fl
         return launch_cluster_z(kernel, dim3(tiles.x, tiles.y, split ? ks : 1), RT_THREADS, bytes, s, w, shared, x, logits, ld, h, e, rows, n);
     }
     if (h % 16 == 0 && ceil_div(n, 64) <= GRID_Y) {
+        if (cleared) *cleared = clear != nullptr;
         auto launch = [&](auto kernel, int tokens) {
-            return launch_cluster_z(kernel, dim3(ceil_div(rows, 16), ceil_div(n, tokens), ks), RM_WARPS * 32, 0, s, w, shared, x, logits, ld, h, e, rows, n);
+            return launch_cluster_z(kernel, dim3(ceil_div(rows, 16), ceil_div(n, tokens), ks), RM_WARPS * 32, 0, s, w, shared, x, logits, ld, h, e, rows, n, clear);
         };
         // the fewest tokens a block that leave at most a block per SM: with 64, 64 tokens of 768 columns x 64 experts were 8 blocks
         auto fits = [&](int tokens) { return n <= tokens || mma_blocks(tokens) <= ROUTER_SMS; };
@@ -709,21 +712,27 @@ int32_t router_launch(const float * w, const float * shared, const void * xv, fl
     return launch_status();
 }
 }  // namespace
+
+// b2moe_router; where it can (*cleared), the launch also sets *clear to 0, in order before every launch behind it
+int32_t router_logits(const float * router_w, const float * shared_gate, const void * x, int32_t x_dtype, float * logits, int32_t ld, int32_t hidden, int32_t experts, int32_t n, int * clear, bool * cleared,
+                      cudaStream_t s) {
+    if (cleared) *cleared = false;
+    if (hidden <= 0 || experts <= 0 || n <= 0 || hidden % 8 || ld < experts + (shared_gate ? 1 : 0)) return B2MOE_ERR_SHAPE;
+    if (!router_w || !x || !logits) return B2MOE_ERR_NULL;
+    if (!valid_dtype(x_dtype)) return B2MOE_ERR_SHAPE;
+    if (!aligned16(router_w) || !aligned16(x) || (shared_gate && !aligned16(shared_gate))) return B2MOE_ERR_ALIGN;
+    const int rows = experts + (shared_gate ? 1 : 0);
+    if (x_dtype == B2MOE_F32) return router_launch<B2MOE_F32>(router_w, shared_gate, x, logits, ld, hidden, experts, rows, n, clear, cleared, s);
+    if (x_dtype == B2MOE_BF16) return router_launch<B2MOE_BF16>(router_w, shared_gate, x, logits, ld, hidden, experts, rows, n, clear, cleared, s);
+    return router_launch<B2MOE_F16>(router_w, shared_gate, x, logits, ld, hidden, experts, rows, n, clear, cleared, s);
+}
 }  // namespace b2
 
 using namespace b2;
 
 extern "C" B2MOE_API int32_t b2moe_router(const float * router_w, const float * shared_gate, const void * x, int32_t x_dtype, float * logits,
                                 int32_t ld, int32_t hidden, int32_t experts, int32_t n, b2moe_stream stream) {
-    if (hidden <= 0 || experts <= 0 || n <= 0 || hidden % 8 || ld < experts + (shared_gate ? 1 : 0)) return B2MOE_ERR_SHAPE;
-    if (!router_w || !x || !logits) return B2MOE_ERR_NULL;
-    if (!valid_dtype(x_dtype)) return B2MOE_ERR_SHAPE;
-    if (!aligned16(router_w) || !aligned16(x) || (shared_gate && !aligned16(shared_gate))) return B2MOE_ERR_ALIGN;
-    const int rows = experts + (shared_gate ? 1 : 0);
-    cudaStream_t s = as_stream(stream);
-    if (x_dtype == B2MOE_F32) return router_launch<B2MOE_F32>(router_w, shared_gate, x, logits, ld, hidden, experts, rows, n, s);
-    if (x_dtype == B2MOE_BF16) return router_launch<B2MOE_BF16>(router_w, shared_gate, x, logits, ld, hidden, experts, rows, n, s);
-    return router_launch<B2MOE_F16>(router_w, shared_gate, x, logits, ld, hidden, experts, rows, n, s);
+    return router_logits(router_w, shared_gate, x, x_dtype, logits, ld, hidden, experts, n, nullptr, nullptr, as_stream(stream));
 }
 
 extern "C" B2MOE_API int32_t b2moe_topk_softmax(const float * logits, int32_t ld, int32_t * ids, float * weights, float * shared_weights,
