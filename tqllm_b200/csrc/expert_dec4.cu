@@ -168,7 +168,7 @@ struct Routed {
     int ids[ROUTED_MAX];
     float weights[ROUTED_MAX];
     short perm[ROUTED_MAX + PASS_TOKENS], e[ROUTED_MAX + 1], off[ROUTED_MAX + 1];
-    signed char cnt[ROUTED_MAX + 1], flags[ROUTED_MAX];      // flags of an assignment: 1: the first of its expert, 2: the first of a pass
+    signed char cnt[ROUTED_MAX + 1], first[ROUTED_MAX];      // first: the assignment is its expert's first
     float inv[PASS_TOKENS];                  // inverse scales of the staged rows
     int row[2][PASS_TOKENS];                 // the staged row of a segment's token columns
 };
@@ -229,7 +229,8 @@ __device__ __forceinline__ int route_and_plan(const Dec4Args & p, const Dec4Rout
         if (lane == 0) r.inv[row] = inv;
     }
     __syncthreads();
-    // an assignment's place: those of smaller experts and the earlier ones of its own (the stable order of a dispatch)
+    // An assignment's place: those of smaller experts and the earlier ones of its own (the stable order of a dispatch). A token's experts are all different (topk <= experts; a
+    // selected key is never taken again), so an expert has at most n <= PASS_TOKENS assignments and one pass
     int below = 0, same = 0, before = 0;
     const int e = tid < A ? r.ids[tid] : -1;
     if (tid < A) {
@@ -241,27 +242,22 @@ __device__ __forceinline__ int route_and_plan(const Dec4Args & p, const Dec4Rout
             before += o == e && a < tid;
         }
         r.perm[below + before] = short(tid);
-        r.flags[tid] = (before == 0) | (before % PASS_TOKENS == 0) << 1;
+        r.first[tid] = before == 0;
     }
-    const bool first = tid < A && before == 0, begins = tid < A && before % PASS_TOKENS == 0;
-    const int experts = __syncthreads_count(first), passes = __syncthreads_count(begins), shared = in.shared_count > 0;
+    const bool first = tid < A && before == 0;
+    const int experts = __syncthreads_count(first), shared = in.shared_count > 0;
     int * const pass_list = perm + A + in.shared_count;
-    if (begins) {
-        int expert_at = 0, at = before / PASS_TOKENS, behind = shared;   // active experts before this one, passes before this one, passes of the experts behind
+    if (first) {
+        int at = 0;                                                     // active experts before this one
 #pragma unroll 1
-        for (int a = 0; a < A; ++a) {
-            const int o = r.ids[a], f = r.flags[a];
-            expert_at += (f & 1) && o < e;
-            at += (f & 2) && o < e;
-            behind += (f & 2) && o > e;
-        }
-        r.e[at] = short(e); r.off[at] = short(below + before); r.cnt[at] = (signed char)min(PASS_TOKENS, same - before);
-        if (lead && first) { active[expert_at] = e; pass_list[experts + shared - 1 - expert_at] = behind; }
+        for (int a = 0; a < A; ++a) at += r.first[a] && r.ids[a] < e;
+        r.e[at] = short(e); r.off[at] = short(below); r.cnt[at] = (signed char)same;
+        if (lead) { active[at] = e; pass_list[experts + shared - 1 - at] = experts + shared - 1 - at; }
     }
     if (shared) {                                                      // its tokens are one pass
         if (tid < in.shared_count) r.perm[A + tid] = short(A + in.shared_first + tid);
         if (tid == 0) {
-            r.e[passes] = short(p.experts); r.off[passes] = short(A); r.cnt[passes] = (signed char)in.shared_count;
+            r.e[experts] = short(p.experts); r.off[experts] = short(A); r.cnt[experts] = (signed char)in.shared_count;
             if (lead) { active[experts] = p.experts; pass_list[0] = 0; }
         }
     }
@@ -281,11 +277,11 @@ __device__ __forceinline__ int route_and_plan(const Dec4Args & p, const Dec4Rout
         for (int i = tid; i < A + in.shared_count; i += blockDim.x) perm[i] = r.perm[i];
         if (tid == 0) {
             offsets[e1] = A + in.shared_count;
-            pass_list[experts + shared] = passes + shared;
-            p.plan[PLAN_NGROUPED] = A + in.shared_count; p.plan[PLAN_NACTIVE] = experts + shared; p.plan[PLAN_NPASS] = passes + shared;      // (its status word: cleared by the launch before)
+            pass_list[experts + shared] = experts + shared;
+            p.plan[PLAN_NGROUPED] = A + in.shared_count; p.plan[PLAN_NACTIVE] = experts + shared; p.plan[PLAN_NPASS] = experts + shared;      // (its status word: cleared by the launch before)
         }
     }
-    return passes + shared;
+    return experts + shared;
 }
 
 // MODE 0: out = act[a][row] = silu(gate . x) * (up . x);   MODE 1: out = y[a][row] = down . act[a]
