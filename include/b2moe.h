@@ -365,7 +365,8 @@ B2MOE_API int32_t b2moe_place_experts(const uint64_t * counts, int32_t experts, 
  * in the grouped GEMM; any other value (0 = the default): the library's own choice of 64, 128 or 256 by tokens per expert.
  * b2moe_harness_wait_probe: the 4-bit decode kernels skip the copy of weight tile number drop_tile of every warp
  * (-1 = none, the default) and bound each wait by wait_limit polls (0 = default), so that a test can watch a bounded
- * wait run out: the launch then sets plan word [3] and returns, its outputs invalid.
+ * wait run out: the launch then sets plan word [3] and returns, its outputs invalid. The tcgen05 router leaves out the copies of
+ * column step number drop_tile of every block; its waits keep their limit, and it sums the logits in a plain loop after it.
  * b2moe_harness_skip_staging: while on, the 4-bit decode kernels skip their activation staging launch and read the
  * staged rows the previous call left in the same workspace (a benchmark times the product kernel alone this way).
  * b2moe_harness_overlap: on (the default), the launches of a layer call are chained by programmatic dependent launch: a

@@ -31,6 +31,7 @@ int32_t dec4_gateup_routed(const b2moe_bank *, const b2moe_bank *, const b2moe_b
 int32_t dec4_down(const b2moe_bank *, const b2moe_bank *, const void *, int x_dtype, bool per_token, const int *, int, int, int, void *, int y_dtype, void *,
                   cudaStream_t, bool plan_ready);
 void dec4_debug(int drop_tile, uint32_t wait_limit);
+void router_drop_step(int step);
 void dec4_skip_staging(bool on);
 void dec4_ring(int nbuf, int stages, int slot_tiles);
 void dec4_ksplit_max(int ks);
@@ -174,7 +175,7 @@ extern "C" B2MOE_API void b2moe_harness_select(int32_t family, int32_t gemm_item
     g_family = family >= B2MOE_FAMILY_AUTO && family <= B2MOE_FAMILY_DECODE_KERNELS ? family : B2MOE_FAMILY_AUTO;
     gemm_tc_item_tokens(gemm_item_tokens);
 }
-extern "C" B2MOE_API void b2moe_harness_wait_probe(int32_t drop_tile, uint32_t wait_limit) { dec4_debug(drop_tile, wait_limit); }
+extern "C" B2MOE_API void b2moe_harness_wait_probe(int32_t drop_tile, uint32_t wait_limit) { dec4_debug(drop_tile, wait_limit); router_drop_step(drop_tile); }
 extern "C" B2MOE_API void b2moe_harness_skip_staging(int32_t on) { dec4_skip_staging(on != 0); }
 extern "C" B2MOE_API void b2moe_harness_ring(int32_t nbuf, int32_t stages, int32_t slot_tiles) { dec4_ring(nbuf, stages, slot_tiles); }
 extern "C" B2MOE_API void b2moe_harness_column_split(int32_t max_warps_per_job) { dec4_ksplit_max(max_warps_per_job); }

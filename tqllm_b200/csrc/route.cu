@@ -108,9 +108,9 @@ template <int DT> __device__ __noinline__ float plain_logit(const float * w, con
     }
     return s;
 }
-// the logit to store: the sum s of (router row, token), looked at again where fp16 or fp32 rows were split
-template <int DT> __device__ __forceinline__ float checked_logit(float s, const float * w, const float * shared, const typename Elem<DT>::type * x, int row, int tok, int e, int h) {
-    if (x_terms<DT>() > 1 && !isfinite(s)) return plain_logit<DT>(row == e ? shared : w + size_t(row) * h, x + size_t(tok) * h, h);
+// the logit to store: the sum s of (router row, token), looked at again where fp16 or fp32 rows were split; lost: there is no sum
+template <int DT> __device__ __forceinline__ float checked_logit(float s, const float * w, const float * shared, const typename Elem<DT>::type * x, int row, int tok, int e, int h, bool lost = false) {
+    if (lost || (x_terms<DT>() > 1 && !isfinite(s))) return plain_logit<DT>(row == e ? shared : w + size_t(row) * h, x + size_t(tok) * h, h);
     return s;
 }
 template <int DT, int J>
@@ -712,6 +712,8 @@ int32_t router_launch(const float * w, const float * shared, const void * xv, fl
     return launch_status();
 }
 }  // namespace
+
+void router_drop_step(int step) { rtc::g_drop_step = step; }
 
 // b2moe_router; where it can (*cleared), the launch also sets *clear to 0, in order before every launch behind it
 int32_t router_logits(const float * router_w, const float * shared_gate, const void * x, int32_t x_dtype, float * logits, int32_t ld, int32_t hidden, int32_t experts, int32_t n, int * clear, bool * cleared,

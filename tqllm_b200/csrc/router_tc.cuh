@@ -19,7 +19,7 @@
 // router rows loaded straight from global memory into fragments, no shared memory: 39.0; one accumulator for all terms: 24.9, at 1.65e-6 (this 4.7e-7).
 // A launch with few tiles would leave SMs idle: the blocks of a cluster take parts of a tile's columns each, and
 // add them in column order through distributed shared memory, so neither the split nor NT changes a bit.
-// Every wait is bounded; where one runs out, the logits of the tile become NaN (fp16 rows: are summed again in a plain loop).
+// Every wait is bounded; where one runs out, the tile's logits are summed in a plain loop.
 #pragma once
 #include "tc_ptx.cuh"
 #include "tensor_map.cuh"
@@ -76,10 +76,11 @@ template <bool EXACT> __device__ __forceinline__ void add_part(float & v, float 
     v = t;
 }
 struct Maps { CUtensorMap w, x, gate; };
+int g_drop_step = -1;                       // test hook (b2moe_harness_wait_probe): every block leaves out the copies of this step of its own
 
 template <int DT, int NT, bool SPLIT, bool FINE>
 __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const float * shared, const typename Elem<DT>::type * x, float * logits, int ld, int h, int e, int rows,
-                                                          int n, const __grid_constant__ Maps maps) {
+                                                          int n, int drop_step, const __grid_constant__ Maps maps) {
     namespace cg = cooperative_groups;
     constexpr bool F16 = DT == B2MOE_F16;
     static_assert(!F16 || FINE);
@@ -127,6 +128,7 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
                 if (g >= S && !bar_wait(done + 8 * ((g - S) % S), uint32_t((g - S) / S) & 1u)) { ok = false; break; }
                 const uint32_t bar = full + 8 * (g % S), dst = saddr(smem) + (g % S) * stage_bytes(NT);
                 const int k0 = (s_lo + g) * STEP;
+                if (g == drop_step) continue;                           // test hook
                 bar_expect_tx(bar, stage_bytes(NT) + (has_gate ? GATE_BYTES : 0));
                 tma_load_2d(dst, &maps.w, k0, r0, bar);                 // what lies outside (rows, columns, tokens) arrives as zeros
                 tma_load_2d(dst + W_BYTES / 2, &maps.w, k0 + 32, r0, bar);
@@ -136,7 +138,7 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
             if (!ok) *gave_up = 1;
             // before leaving, every copy must have landed (after a clean run these waits return at once)
 #pragma unroll 1
-            for (int i = max(0, g - S); i < g; ++i) bar_wait(full + 8 * (i % S), uint32_t(i / S) & 1u);
+            for (int i = max(0, g - S); i < g; ++i) if (i != drop_step) bar_wait(full + 8 * (i % S), uint32_t(i / S) & 1u);
         }
         __syncwarp();
     } else if (warp == MMA_WARP) {
@@ -325,7 +327,7 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
             if (!SPLIT)
 #pragma unroll 1
                 for (int i = 0; i < TOK; ++i)
-                    if (in && t0 + tk0 + i < n) logits[size_t(t0 + tk0 + i) * ld + r0 + row] = checked_logit<DT>(CUDART_NAN_F, w, shared, x, r0 + row, t0 + tk0 + i, e, h);
+                    if (in && t0 + tk0 + i < n) logits[size_t(t0 + tk0 + i) * ld + r0 + row] = checked_logit<DT>(0.f, w, shared, x, r0 + row, t0 + tk0 + i, e, h, true);
         }
     }
     fence_before();
@@ -378,7 +380,7 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
                         lack = l[j];
                     }
             }
-            logits[size_t(t0 + tk) * ld + r0 + r] = checked_logit<DT>(bad ? CUDART_NAN_F : FINE ? sum + lack : sum, w, shared, x, r0 + r, t0 + tk, e, h);
+            logits[size_t(t0 + tk) * ld + r0 + r] = checked_logit<DT>(FINE ? sum + lack : sum, w, shared, x, r0 + r, t0 + tk, e, h, bad != 0);
         }
         cluster.sync();                                                // the blocks' tiles stay alive until every block has read them
     }
@@ -415,7 +417,7 @@ template <int DT, int NT, bool FINE> int32_t launch_nt(const Shape & p, const fl
     const size_t smem = p.ks > 1 ? smem_bytes<DT, FINE, true>(NT) : smem_bytes<DT, FINE, false>(NT);
     const auto kernel = p.ks > 1 ? router_tc_k<DT, NT, true, FINE> : router_tc_k<DT, NT, false, FINE>;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return B2MOE_ERR_CUDA;
-    return launch_cluster_z(kernel, dim3(ceil_div(n, NT), ceil_div(rows, ROWS), p.ks), THREADS, smem, s, w, shared, x, logits, ld, h, e, rows, n, maps);
+    return launch_cluster_z(kernel, dim3(ceil_div(n, NT), ceil_div(rows, ROWS), p.ks), THREADS, smem, s, w, shared, x, logits, ld, h, e, rows, n, g_drop_step, maps);
 }
 // 16-bit rows; h a multiple of 8 (strides of the maps)
 template <int DT, bool FINE> int32_t launch(const float * w, const float * shared, const typename Elem<DT>::type * x, float * logits, int ld, int h, int e, int rows, int n, cudaStream_t s) {
