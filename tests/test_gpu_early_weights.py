@@ -1,6 +1,6 @@
 """GPU: the down product of a layer call asks for its weights before the launches before it are done, the grouped GEMM's products read the plan before their rows are converted. Forward
 passes launched back to back over other tokens, through one arena, give the bits of the separate entry points with a synchronisation after each of them, down to a first segment of fewer
-copies than a ring holds (K = 256), blocks without work, and with rows staged inside the down kernel (one token) or by a launch (70)."""
+copies than a ring holds (K = 256), blocks without work. (The decode kernels' early form: test_gpu_early_decode.py; here they meet up to three tokens, whose gate/up launch makes the plan, so that down waits.)"""
 import dataclasses
 
 import pytest

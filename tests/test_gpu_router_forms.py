@@ -1,6 +1,6 @@
 """GPU: the forms of the tensor-core routers and the rules between them. A token's logits have the same bits in every form of a kernel:
-in router_mma_k whatever the number of tokens a block takes (8, 16, 32, 64), in router_tile_k whether a tile's columns are split over a
-cluster (fewer than 100 tiles) or not. All are held to fp64, to 3e-6 of the largest logit as in test_gpu_routing.py, at the sizes where
+in router_mma_k whatever the number of tokens a block takes (8, 16, 32, 64), in router_tile_k (fp32; short fp16 rows: test_gpu_router_tiles.py) and
+router_tc_k (16-bit rows) whether a tile's columns are split over a cluster (few tiles) or not. All are held to fp64, to 3e-6 of the largest logit as in test_gpu_routing.py, at the sizes where
 they begin and end: one partial sum of 256 columns, several per block (more than 2048 columns), a ragged last one, ragged rows and tokens."""
 import pytest
 import torch
@@ -40,7 +40,7 @@ def test_small_routers_of_many_tokens(dtype):
     from tqllm_b200 import moe
     w, gate, x = inputs(700, 1024, 40, dtype)
     full = held(w, gate, x)
-    if dtype != torch.bfloat16:                          # fp16 and fp32 rows go to tiles only above two blocks per SM
+    if dtype != torch.bfloat16:                          # fp16 and fp32 rows leave router_mma_k only above two blocks per SM here
         assert torch.equal(moe.router(w, x[:9].contiguous(), gate), full[:9])
 
 
