@@ -168,8 +168,8 @@ __device__ __forceinline__ float row_to_f16(const typename Elem<DT>::type * xr, 
     return row_scaled<T, DT>(xr, k, lane, [&](int c, const float (&v)[8]) { put(c, pack8(v)); });
 }
 // The product behind a conversion reads the plan and the weights without waiting for the rows (gemm_tc_k), so a conversion lets it begin only once the launches
-// before are complete; or at once (late = false) where its caller knows that the plan is. A layer of 8 tokens on 512 NVFP4 experts 74.8 -> 70.5 us, a chunk of 509
-// on IQ3_S codes 356.6 -> 349.7 (with the router's part, 5).
+// before are complete; or at once (late = false) where its caller knows that the plan is. A layer of 8 tokens on 512 NVFP4 experts 73.3 -> 70.0 us
+// (four preparations of weights and tokens: 3 to 6 % each).
 __device__ __forceinline__ void rows_begin(bool late) {
     if (!late) grid_release();
     grid_wait();
@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                     if (lane < 16) consts[(group + 2 * (turn & 1u)) * 128 + 32 * q + 16 * m + lane] = X::consts(chunk, lane);
                 }
                 if constexpr (AHEAD) {
-                    if constexpr (P::SCRATCH > 0) {                     // every lane has read the first unit's constants
+                    if constexpr (T == T_Q4_K) {                        // every lane has read the first unit's constants
                         __syncwarp();
                         P::second_unit(pre, lane, my_scratch);
                         __syncwarp();

@@ -153,45 +153,43 @@ template <> struct Dec<T_IQ3S4> {
     template <int POS> __device__ __forceinline__ static __half2 pair(uint32_t w, uint32_t one) {
         return bits_h2(and_or(POS <= 6 ? w << (6 - POS) : w >> (POS - 6), 0x03C003C0u, one));
     }
-    // the constants of (row, sub-block) in the warp's scratch, as for Q4_K: (32 (1 + 2 s), -47 (1 + 2 s))
-    static constexpr int SCRATCH = 16 * 4 * 8;
-    struct Pre { uint32_t D[2], one; uint2 late[2]; };
-    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t * scratch) {
+    // The constants of (row, sub-block) in the warp's scratch, as for Q4_K but of both units: (32 (1 + 2 s), -47 (1 + 2 s)) in a word. Spread over two they took twice the scratch, and a raw slot
+    // from items of 128 and 256 tokens (614 to 1125 experts: 3 instead of 4); a unit's at a time took longer. Layers on 512 experts, us, spread / a unit at a time / this:
+    // 2000 tokens 473 / 478 / 466, 4210 686 / 686 / 675, 8192 1202 / 1204 / 1199
+    static constexpr int SCRATCH = 2 * 16 * 4 * 4;
+    __device__ __forceinline__ static void constants(const uint8_t * chunk, int lane, uint8_t * scratch) {
         const int g = lane >> 2, t = lane & 3;
-        Pre p;
-        uint2 now[2];
-        p.one = in_register(0x3C003C00u);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             const uint32_t sc = *reinterpret_cast<const uint32_t *>(chunk + 2048 + 4 * (g + 8 * r)) >> (4 * t);
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
-                // the 4-bit scale under the exponent of 1: 1 + s / 16
-                const __half2 s = bits_h2((((sc >> (16 * u)) & 15u) * 0x00400040u) | 0x3C003C00u);
-                (u ? p.late : now)[r] = make_uint2(h2_bits(__hfma2(s, __float2half2_rn(1024.f), __float2half2_rn(-992.f))),
-                                                 h2_bits(__hfma2(s, __float2half2_rn(-1504.f), __float2half2_rn(1457.f))));
+                const __half2 s = bits_h2((((sc >> (16 * u)) & 15u) * 0x00400040u) | 0x3C003C00u);        // the 4-bit scale under the exponent of 1: 1 + s / 16
+                reinterpret_cast<uint32_t *>(scratch)[64 * u + lane + 32 * r] = h2_bits(__hfma2(s, __floats2half2_rn(1024.f, -1504.f), __floats2half2_rn(-992.f, 1457.f)));
             }
-            p.D[r] = uint32_t(*reinterpret_cast<const unsigned short *>(chunk + 2112 + 2 * (g + 8 * r))) * 0x10001u;
         }
-        put_constants(now, lane, scratch);
-        return p;
     }
-    __device__ __forceinline__ static void second_unit(const Pre & p, int lane, uint8_t * scratch) { put_constants(p.late, lane, scratch); }
-    struct Raw { uint4 w, c[2]; };
+    struct Pre { uint32_t D[2], one; };
+    __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t * scratch) {
+        constants(chunk, lane, scratch);
+        auto d = [&](int row) { return uint32_t(*reinterpret_cast<const unsigned short *>(chunk + 2112 + 2 * row)) * 0x10001u; };
+        return Pre{{d(lane >> 2), d((lane >> 2) + 8)}, in_register(0x3C003C00u)};
+    }
+    struct Raw { uint4 w; uint2 c[2]; };
     template <int J> __device__ __forceinline__ static Raw load(const uint8_t * chunk, int lane, const uint8_t * scratch) {
-        const uint4 * c = reinterpret_cast<const uint4 *>(scratch) + 2 * (lane >> 2) + (J & 1);       // both sub-blocks of the step
+        const uint2 * c = reinterpret_cast<const uint2 *>(scratch) + 32 * (J >> 1) + 2 * (lane >> 2) + (J & 1);       // both sub-blocks of the step
         return Raw{plane(chunk, J, lane), {c[0], c[16]}};
     }
     template <int J> __device__ __forceinline__ static void step(const Raw & raw, int, const void *, const Pre & p, uint32_t (&f)[16]) {
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-            const uint4 k = raw.c[r];
-            const __half2 D = bits_h2(p.D[r]), SC1 = bits_h2(k.x), C1 = bits_h2(k.y), SC2 = bits_h2(k.z), C2 = bits_h2(k.w);
+            const uint2 k = raw.c[r];
+            const __half2 D = bits_h2(p.D[r]), S0 = __low2half2(bits_h2(k.x)), C0 = __high2half2(bits_h2(k.x)), S1 = __low2half2(bits_h2(k.y)), C1 = __high2half2(bits_h2(k.y));
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
                 const uint32_t v = r ? (b ? raw.w.w : raw.w.z) : (b ? raw.w.y : raw.w.x);
-                put(f, r, b, make_uint4(h2_bits(__hmul2(__hfma2(pair<0>(v, p.one), SC1, C1), D)), h2_bits(__hmul2(__hfma2(pair<8>(v, p.one), SC1, C1), D)),
-                                        h2_bits(__hmul2(__hfma2(pair<4>(v, p.one), SC2, C2), D)), h2_bits(__hmul2(__hfma2(pair<12>(v, p.one), SC2, C2), D))));
+                put(f, r, b, make_uint4(h2_bits(__hmul2(__hfma2(pair<0>(v, p.one), S0, C0), D)), h2_bits(__hmul2(__hfma2(pair<8>(v, p.one), S0, C0), D)),
+                                        h2_bits(__hmul2(__hfma2(pair<4>(v, p.one), S1, C1), D)), h2_bits(__hmul2(__hfma2(pair<12>(v, p.one), S1, C1), D))));
             }
         }
     }
@@ -262,29 +260,17 @@ template <> struct Exact<T_Q4_K> {
     }
 };
 template <> struct Exact<T_IQ3S4> {
+    using D = Dec<T_IQ3S4>;
     static constexpr bool MINS = false;
-    static constexpr int SCRATCH = 2 * 16 * 4 * 4;
+    static constexpr int SCRATCH = D::SCRATCH;
     struct Pre { uint32_t one; };
     __device__ __forceinline__ static Pre prep(const uint8_t * chunk, int lane, uint8_t * scratch) {
-        const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const uint32_t sc = *reinterpret_cast<const uint32_t *>(chunk + 2048 + 4 * (g + 8 * r)) >> (4 * t);
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const __half2 s = bits_h2((((sc >> (16 * u)) & 15u) * 0x00400040u) | 0x3C003C00u);        // 1 + s / 16 -> 32 (1 + 2 s), -47 (1 + 2 s)
-                reinterpret_cast<uint32_t *>(scratch)[64 * u + lane + 32 * r] = h2_bits(__hfma2(s, __floats2half2_rn(1024.f, -1504.f), __floats2half2_rn(-992.f, 1457.f)));
-            }
-        }
+        D::constants(chunk, lane, scratch);
         return Pre{in_register(0x3C003C00u)};
     }
-    struct Raw { uint4 w; uint2 c[2]; };
-    template <int J> __device__ __forceinline__ static Raw load(const uint8_t * chunk, int lane, const uint8_t * scratch) {
-        const uint2 * c = reinterpret_cast<const uint2 *>(scratch) + 32 * (J >> 1) + 2 * (lane >> 2) + (J & 1);
-        return Raw{plane(chunk, J, lane), {c[0], c[16]}};
-    }
+    using Raw = D::Raw;
+    template <int J> __device__ __forceinline__ static Raw load(const uint8_t * chunk, int lane, const uint8_t * scratch) { return D::load<J>(chunk, lane, scratch); }
     template <int J> __device__ __forceinline__ static void step(const Raw & raw, int, const void *, const Pre & p, uint32_t (&f)[16]) {
-        using D = Dec<T_IQ3S4>;
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             const uint2 k = raw.c[r];
