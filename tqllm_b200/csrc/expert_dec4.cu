@@ -331,8 +331,8 @@ __global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(c
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     // The plan and the staged rows come from the launches before this one: no global access above this line. With plan_ready only the rows are awaited, by the
     // warps that read them (and by the others before they leave): the producer fills the rings with weights meanwhile. Layers, us: IQ3_S codes, 64 tokens 161.5 -> 159.2 (four preparations of weights and
-    // tokens, 1.1 to 1.6 % each), 24 tokens 100.4 -> 98.5. Not in the large launches of Q4_K, whose consumers and not the first copies bound them and whose rows then come later: over
-    // twelve preparations 77 tokens on 60 experts 105.6 (1.000) -> 106.2 (median 0.992), 16 on 256 188.9 -> 189.0 (0.997); 40 on 256 312.1 -> 311.5 (1.004).
+    // tokens, 1.1 to 1.6 % each), 24 tokens 100.4 -> 98.5. Not in the large launches of Q4_K, whose consumers and not the first copies bound them and whose rows then come later: over eight and
+    // twelve preparations the speed of 77 tokens on 60 experts changes by the factor 0.994 and 1.002, that of 16 to 150 on 256 by 0.997 to 1.004.
     const bool early = MODE == 1 && (FEW || T != T_Q4_K) && p.plan_ready;
     if (!early) grid_wait();
     __syncthreads();
@@ -462,9 +462,7 @@ __global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(c
         };
         int pass, r0, r1;
         uint32_t idx = 0;
-        // The first segment's rows are asked for right after its first weight copies, or (early) once the copies are as far as they go without a consumer: the rings hold S slots.
-        // One place for both: with a second copy of stage_x behind the segment the Q4_K down product took 31.6 us instead of 31.1 (77 tokens on 60 experts, ncu)
-        int stage_at = 0;
+        bool first_staged = false;                         // the first segment's rows are asked for right after its first weight copies, or (early) after the last that the rings hold
 #pragma unroll 1
         for (Job u = u_begin; u < u_end && ok; u += r1 - r0, ++idx) {
             segment(u, pass, r0, r1);
@@ -476,7 +474,6 @@ __global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(c
             if (u_next < u_end) segment(u_next, npass, nr0, nr1);
             bool next_staged = p.nbuf != 2 || u_next >= u_end;
             int in_seg = 0;
-            if (!in_kernel && early && idx == 0) stage_at = min(S, (r1 - r0 + JW - 1) / JW * nslots) - 1;
 #pragma unroll 1
             for (int rb = r0; rb < r1 && ok; rb += JW) {                  // JW row tiles at a time, warp w its part of its own
                 const int rt = rb + w / KSP, k_first = (w % KSP) * kpart;
@@ -498,14 +495,20 @@ __global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(c
                         slot = slot + 1 == uint32_t(S) ? 0 : slot + 1;
                     }
                     ok = __all_sync(0xffffffffu, ok);
-                    if (!in_kernel && in_seg == stage_at) {
+                    if (!in_kernel && !first_staged && (!early || in_seg == S - 1)) {
                         if (early) grid_wait();
                         stage_x(pass, 0, true, e, c0);
-                        stage_at = -1;
+                        first_staged = true;
                     }
                     // once every consumer is S slots into this segment, the previous segment's buffer is free: bring the next one's rows
                     if (!in_kernel && !next_staged && in_seg == S) { stage_x(npass, idx + 1); next_staged = true; }
                 }
+            }
+            // a first segment of less than S slots (only where a launch may begin early: a second copy of stage_x here costs the Q4_K down product 0.5 us of 31, 77 tokens on 60 experts)
+            if (early && !in_kernel && !first_staged && ok) {
+                grid_wait();
+                stage_x(pass, 0, true, e, c0);
+                first_staged = true;
             }
             if (!in_kernel && !next_staged && ok) stage_x(npass, idx + 1);
             if (!in_kernel && p.nbuf == 1 && u_next < u_end && ok) stage_x(npass, idx + 1);
