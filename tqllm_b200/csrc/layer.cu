@@ -96,8 +96,8 @@ int expert_path(uint32_t type, int k, int dtype, int experts, long long assignme
 // Where the rule above says DECODE, banks of 4-bit codes have a second form: the grouped GEMM with integer operands and scales
 // applied to its sums in fp32 (gemm_exact_*), which loses less precision than the decode kernels and reads an expert's weights once per 32
 // tokens instead of once per eight. It takes over from EXACT_MIN_PER assignments per expert on. Layer times, decode kernels / this form, us: Q4_K of 256
-// experts at 7.8 per expert 622 / 687, 9 662 / 677, 10 716 / 665, 19 1219 / 797, 31 1926 / 1074; of 60 at 7.7 103 / 105, 9 109 / 106, 10 115 / 109, 100 567 / 311; of 32 in fp32 at 6
-// 38 / 41, 8 43 / 42, 1000 837 / 485; IQ3_S codes of 512 at 7 307 / 340, 8 339 / 347, 9 361 / 347, 10 389 / 350. At nine itself, over 42 shapes of 2 to 127 experts,
+// experts at 7.8 per expert 622 / 687, 9 662 / 677, 10 716 / 665, 19 1219 / 797, 31 1926 / 1074; of 60 at 6.5 98 / 97, 7.7 106 / 100, 8.5 109 / 99, 100 567 / 311; of 100 at 8 139 / 143; of 32 in fp32 at 6
+// 38 / 36, 8 42 / 37, 1000 837 / 485; IQ3_S codes of 512 at 7 307 / 340, 8 320 / 317, 9 361 / 347, 10 389 / 350. (Small banks would gain from an earlier line; the tests hold it at nine for 8 and 16 experts.) At nine itself, over 42 shapes of 2 to 127 experts,
 // this form takes 0.57 to 1.08 of the decode kernels' time, 0.9 on average; at twelve 0.69 to 1.03. Relative error of both products against 64 bits 2.0e-4 / 1.0e-6. Gate/up on
 // 16-bit rows runs from any scratch that the call accepts; fp32 rows (two terms each) take the decode kernels where the scratch has no room for them.
 constexpr int EXACT_MIN_PER = 9;
@@ -254,8 +254,9 @@ extern "C" B2MOE_API int32_t b2moe_expert_gateup_swiglu(const b2moe_bank * gate,
     return expert_gateup(gate, up, shared_gate, shared_up, x, x_dtype, plan, n, topk, shared_tokens, act, workspace, workspace_bytes, stream, false);
 }
 
-// plan_ready: the launch before this call's is a gate/up product over the same plan, which another launch made. Every kernel of that product waits for the launches before it and only then (when
-// its own work is done) lets the next one begin, so whatever begins here finds the plan complete and may ask for weights before it waits
+// plan_ready: the launch before this call's is a gate/up product over the same plan, which another launch made. The LAST kernel of that product (dec4_k, gemm_tc_k; the others have no early release) waits
+// for the launches before it and only then, when its own work is done, lets the next one begin, so whatever begins here finds the plan complete and may ask for weights before it waits. A product
+// that ends with a kernel which releases before its wait, as the conversions in front of the last kernels do, would break this
 static int32_t expert_down(const b2moe_bank * down, const b2moe_bank * shared_down, const float * act, const int32_t * plan, int32_t n, int32_t topk,
                            int32_t shared_tokens, float * y, void * workspace, size_t workspace_bytes, b2moe_stream stream, long long live, bool plan_ready = false) {
     if (int32_t rc = check_bank(down)) return rc;

@@ -17,6 +17,7 @@
 // What bounds it: the chain from a step's copy over its split to the products, 1650 cycles a step of 128 bf16 tokens, 1080 of 64 (most of it the split by two warps a
 // scheduler), where the products alone take 768 and 516; 2000 of 64 fp16 tokens, whose products take twice as long and whose sums are read at every step. Two groups of splitting warps on steps in turn: 34.2 us against 31.9 (4096 x 2048 x 512 bf16; three stages instead of four for it); the
 // router rows loaded straight from global memory into fragments, no shared memory: 39.0; one accumulator for all terms: 24.9, at 1.65e-6 (this 4.7e-7).
+// Registers: 896 threads leave 72, and the form of large bf16 launches (128 tokens, a block per tile) keeps 32 totals a thread: 292 bytes of spill stores, 456 of loads, once a part of 512 columns.
 // A launch with few tiles would leave SMs idle: the blocks of a cluster take parts of a tile's columns each, and
 // add them in column order through distributed shared memory, so neither the split nor NT changes a bit.
 // Every wait is bounded; where one runs out, the tile's logits are summed in a plain loop.
