@@ -315,7 +315,10 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
     const uint32_t raw_full = saddr(bars), raw_empty = raw_full + 16 * RAW_SLOTS, a_full = raw_empty + 8 * RAW_SLOTS,
                    done = a_full + 8 * A_STAGES, b_full = done + 8 * STEP_RING, acc_full = b_full + 8 * MAX_B_STAGES, acc_empty = acc_full + 16,
                    drain = acc_empty + 16, tok_bar = drain + 8, const_full = tok_bar + 8;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // The warp's number as a shuffle's result: the compiler then knows it, and with it the roles' branches, their loops and addresses, to be the same in the whole warp, and
+    // keeps them in uniform registers: fewer instructions in every role, and products issued without moving their operands there one by one.
+    // c3 decode 8 73.0 -> 66.9 us, c5 decode 24 308 -> 292 (309 with the issuing branch taken by one lane), c2 509 tokens 351 -> 323, c4 600 745 -> 685
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0);
     const int e1 = p.experts + 1;
     const int * counts = p.plan + PLAN_HDR, * offsets = counts + e1, * active = offsets + e1 + 1, * perm = active + e1;
     const int row_tiles = (p.rows + 15) >> 4, row_blocks = (row_tiles + ITEM_TILES - 1) / ITEM_TILES;
@@ -393,7 +396,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
             tile = local - r.rb * nt;
         }
         r.slot0 = f.off + tile * per;
-        r.nv = max(0, min(per, f.cnt - tile * per));
+        r.nv = __shfl_sync(0xffffffffu, max(0, min(per, f.cnt - tile * per)), 0);      // uniform, for the products' descriptors
         return r;
     };
     auto x_row = [&](int a) { return MODE == 0 ? (a < p.A ? a / p.topk : a - p.A) : a; };
@@ -659,11 +662,13 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
         }
         if (!ok && lane == 0) give_up();
     } else if (warp == MMA_WARP) {
-        // ---- MMA issuer: the whole warp looks the items up, one elected lane issues an item's products. What an issue costs decides
-        // the pace of narrow items: the tensor core takes N / 2 cycles a product (at least 16), the issuing thread beside busy
-        // decoders 43 with its operands' addresses constant but for one addend (the loop is unrolled over the A stages) and 58 with
-        // addresses of a running stage (microbenchmark, N = 64, cycles a product with its share of the unit's wait and commit) ----
+        // ---- MMA issuer: the whole warp walks the loops, one elected lane issues (a predicate on the instruction, not a branch: in a
+        // branch of one lane every operand is moved to the uniform registers first). What an issue costs decides the pace of narrow items: the
+        // tensor core takes N / 2 cycles a product (at least 16), the issuing thread beside busy decoders 43 when it was a branch, with its operands'
+        // addresses constant but for one addend (the loop is unrolled over the A stages) and 58 with addresses of a running stage
+        // (microbenchmark, N = 64, cycles a product with its share of the unit's wait and commit); a unit now 260 cycles beside its waits, 430 before ----
         const uint32_t b_lo0 = sw128_desc_lo(saddr(b_st)), b_step = uint32_t(p.cap * 128 * PLANES) >> 4;
+        const bool lead = elect_one();
         uint32_t gu = 0, next = 0, uses0 = 0, uses1 = 0;
         bool ok = true;
 #pragma unroll 1
@@ -690,50 +695,47 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                     for (uint32_t s = 0; s < A_STAGES; ++s) {
                         if (s < first) continue;                       // an item's units begin at any stage
                         const uint32_t a = tmem + A_COL0 + s * A_COLS, sb = PAIR ? 2 * s : 2 * (s & 1), b = b_lo0 + sb * b_step;
-                        if (!bar_wait(a_full + 8 * s, turn & 1u)) return false;
-                        if (!PAIR && !bar_wait(b_full + 8 * sb, (2 * turn + (s >> 1)) & 1u)) return false;      // with b_pair a_full stands for the unit's rows too
+                        if (!warp_wait(a_full + 8 * s, turn & 1u)) return false;
+                        if (!PAIR && !warp_wait(b_full + 8 * sb, (2 * turn + (s >> 1)) & 1u)) return false;      // with b_pair a_full stands for the unit's rows too
                         if constexpr (EXACT) {                         // a chunk's units are the stages 0, 1 or 2, 3, its sums a set of their own
                             const uint32_t set = s >> 1, ds = tmem + set * X_SET;
-                            if ((s & 1) == 0 && turn > 0 && !bar_wait(acc_empty + 8 * set, (turn - 1) & 1u)) return false;
+                            if ((s & 1) == 0 && turn > 0 && !warp_wait(acc_empty + 8 * set, (turn - 1) & 1u)) return false;
                             fence_after();
-                            mma_step(ds, ds, a, b, id, s & 1, 1);
-                            mma_step(ds, ds, a + A_COLS / 2, b + b_half, id, 1, 1);
+                            mma_step(lead, ds, ds, a, b, id, s & 1, 1);
+                            mma_step(lead, ds, ds, a + A_COLS / 2, b + b_half, id, 1, 1);
                             if constexpr (X::MINS)
                                 if ((s & 1) == 0)
-                                    mma_f16<SW32_DESC_HI>(ds + X_MINS, tmem + X_AMINS + 8 * set, sw128_desc_lo(saddr(mins_st) + s * (X_CAP * 32)), idesc(128, npad, 0), 0);
-                            mma_commit(done + 16 * s + 8);
-                            if (s & 1) mma_commit(acc_full + 8 * set);
+                                    mma_f16<SW32_DESC_HI>(lead, ds + X_MINS, tmem + X_AMINS + 8 * set, sw128_desc_lo(saddr(mins_st) + s * (X_CAP * 32)), idesc(128, npad, 0), 0);
+                            mma_commit(lead, done + 16 * s + 8);
+                            if (s & 1) mma_commit(lead, acc_full + 8 * set);
                             if (--units == 0) return true;
                             continue;
                         }
                         fence_after();
-                        if (left > 0) mma_step(d, d + second, a, b, id, acc, acc | (second == 0));
+                        if (left > 0) mma_step(lead, d, d + second, a, b, id, acc, acc | (second == 0));
                         if constexpr (!PAIR) {
-                            mma_commit(done + 16 * s);
-                            if (!bar_wait(b_full + 8 * (sb + 1), (2 * turn + (s >> 1)) & 1u)) return false;
+                            mma_commit(lead, done + 16 * s);
+                            if (!warp_wait(b_full + 8 * (sb + 1), (2 * turn + (s >> 1)) & 1u)) return false;
                             fence_after();
                         }
-                        if (left > 1) mma_step(d, d + second, a + A_COLS / 2, b + b_half, id, 1, 1);
-                        mma_commit(done + 16 * s + 8);
+                        if (left > 1) mma_step(lead, d, d + second, a + A_COLS / 2, b + b_half, id, 1, 1);
+                        mma_commit(lead, done + 16 * s + 8);
                         acc = 1;
                         left -= 2;
-                        if (--units == 0) { mma_commit(acc_full + 8 * h); return true; }
+                        if (--units == 0) { mma_commit(lead, acc_full + 8 * h); return true; }
                     }
                     first = 0;
                     ++turn;
                 }
             };
-            if (elect_one()) {
-                if constexpr (EXACT) ok = ok && products(std::true_type{});
-                else ok = ok && (p.b_pair ? products(std::true_type{}) : products(std::false_type{}));
-            }
-            ok = __all_sync(0xffffffffu, ok);
+            if constexpr (EXACT) ok = ok && products(std::true_type{});
+            else ok = ok && (p.b_pair ? products(std::true_type{}) : products(std::false_type{}));
             gu += 2 * nchunks;
         }
         if (!ok && lane == 0) give_up();
         // nothing may be in flight when the tensor memory is freed (after a clean run the epilogue has waited for all of it)
-        if (elect_one()) { mma_commit(drain); bar_wait(drain, 0); }
-        __syncwarp();
+        mma_commit(lead, drain);
+        warp_wait(drain, 0);
     } else if (warp == RAW_WARP) {
         // ---- raw blocks ----
         constexpr int PARTS = chunk_parts<T>();

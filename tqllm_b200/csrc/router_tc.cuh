@@ -143,7 +143,8 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
         }
         __syncwarp();
     } else if (warp == MMA_WARP) {
-        if (elect_one()) {
+        {
+            const bool lead = elect_one();
             bool ok = true;
             const uint32_t id = idesc(128, NT, 1);
 #pragma unroll 1
@@ -152,10 +153,10 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
                 const uint32_t a = tmem + A_COL0 + set * A_STAGE, b = sw128_desc_lo(saddr(smem) + (g % S) * stage_bytes(NT) + W_BYTES);
                 [[maybe_unused]] const uint32_t bl = sw128_desc_lo(saddr(x_low) + (g % S) * low_bytes<DT>(NT));
                 // half hf's product number k of the weights' term t with the activations' first term (low: the second)
-                auto mma = [&](uint32_t d, int hf, int t, int k, bool acc, bool low = false) { mma_f16(d, a + hf * A_HALF + t * A_TERM + 8 * k, (low ? bl : b) + 4 * hf + 2 * k, id, acc); };
-                if (!bar_wait((F16 ? x_full : full) + 8 * (g % S), uint32_t(g / S) & 1u) || !bar_wait(a_full + 8 * set, uint32_t(g >> 1) & 1u)) { ok = false; break; }
+                auto mma = [&](uint32_t d, int hf, int t, int k, bool acc, bool low = false) { mma_f16(lead, d, a + hf * A_HALF + t * A_TERM + 8 * k, (low ? bl : b) + 4 * hf + 2 * k, id, acc); };
+                if (!warp_wait((F16 ? x_full : full) + 8 * (g % S), uint32_t(g / S) & 1u) || !warp_wait(a_full + 8 * set, uint32_t(g >> 1) & 1u)) { ok = false; break; }
                 if constexpr (FINE) {
-                    if (g > 1 && !bar_wait(acc_empty + 8 * set, uint32_t((g >> 1) - 1) & 1u)) { ok = false; break; }
+                    if (g > 1 && !warp_wait(acc_empty + 8 * set, uint32_t((g >> 1) - 1) & 1u)) { ok = false; break; }
                     fence_after();
 #pragma unroll
                     for (int hf = 0; hf < 2; ++hf) {                   // a half step has sums of its own
@@ -167,24 +168,24 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
                         }
                         mma(d, hf, 0, 0, true); mma(d, hf, 0, 1, true);
                     }
-                    mma_commit(acc_full + 8 * set);
+                    mma_commit(lead, acc_full + 8 * set);
                 } else {
                     const int p = g / PART_STEPS;
                     const bool more = g % PART_STEPS > 0;
-                    if (!more && p > 0 && !bar_wait(acc_empty, uint32_t(p - 1) & 1u)) { ok = false; break; }
+                    if (!more && p > 0 && !warp_wait(acc_empty, uint32_t(p - 1) & 1u)) { ok = false; break; }
                     fence_after();
 #pragma unroll
                     for (int hf = 0; hf < 2; ++hf) {
                         mma(tmem + ACC, hf, 2, 0, more || hf > 0); mma(tmem + ACC, hf, 1, 0, true); mma(tmem + ACC, hf, 2, 1, true); mma(tmem + ACC, hf, 1, 1, true);
                         mma(tmem, hf, 0, 0, more || hf > 0); mma(tmem, hf, 0, 1, true);
                     }
-                    if (g % PART_STEPS == PART_STEPS - 1 || g + 1 == steps) mma_commit(acc_full);
+                    if (g % PART_STEPS == PART_STEPS - 1 || g + 1 == steps) mma_commit(lead, acc_full);
                 }
-                mma_commit(done + 8 * (g % S));
+                mma_commit(lead, done + 8 * (g % S));
             }
             if (!ok) *gave_up = 1;
-            mma_commit(drain);                                         // nothing may be in flight when the tensor memory is freed
-            bar_wait(drain, 0);
+            mma_commit(lead, drain);                                         // nothing may be in flight when the tensor memory is freed
+            warp_wait(drain, 0);
         }
         __syncwarp();
     } else if (warp >= CONV_WARP0 && warp < EPI_WARP0) {

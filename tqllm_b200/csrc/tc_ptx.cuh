@@ -93,22 +93,23 @@ __device__ __forceinline__ uint32_t idesc(uint32_t m, uint32_t n, uint32_t ab_fo
     return (1u << 4) | (ab_format << 7) | (ab_format << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
 // One product with A (128 x 16, fp16) in tensor memory (row in lane, two values of K per column) and B (N x 16) in shared memory,
-// fp32 sums in tensor memory, added to what is there when acc != 0. One thread issues.
+// fp32 sums in tensor memory, added to what is there when acc != 0. The thread with `lead` set issues it: the loop around it can
+// then be walked by the whole converged warp, whose addresses the compiler keeps in uniform registers.
 template <uint32_t DESC_HI = SW128_DESC_HI>
-__device__ __forceinline__ void mma_f16(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t id, uint32_t acc) {
-    asm volatile("{\n .reg .pred p;\n .reg .b64 db;\n setp.ne.b32 p, %4, 0;\n mov.b64 db, {%2, %5};\n"
-                 " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n}" ::"r"(d), "r"(a), "r"(b_lo), "r"(id), "r"(acc), "r"(DESC_HI) : "memory");
+__device__ __forceinline__ void mma_f16(bool lead, uint32_t d, uint32_t a, uint32_t b_lo, uint32_t id, uint32_t acc) {
+    asm volatile("{\n .reg .pred p, q;\n .reg .b64 db;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %6, 0;\n mov.b64 db, {%2, %5};\n"
+                 " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n}" ::"r"(d), "r"(a), "r"(b_lo), "r"(id), "r"(acc), "r"(DESC_HI), "r"(uint32_t(lead)) : "memory");
 }
 // a 64-column step: four products, even ones into d0 (added when acc0), odd ones into d1 (acc1); the two may be the same
-__device__ __forceinline__ void mma_step(uint32_t d0, uint32_t d1, uint32_t a, uint32_t b_lo, uint32_t id, uint32_t acc0, uint32_t acc1) {
-    mma_f16(d0, a, b_lo, id, acc0);
-    mma_f16(d1, a + 8, b_lo + 2, id, acc1);
-    mma_f16(d0, a + 16, b_lo + 4, id, 1);
-    mma_f16(d1, a + 24, b_lo + 6, id, 1);
+__device__ __forceinline__ void mma_step(bool lead, uint32_t d0, uint32_t d1, uint32_t a, uint32_t b_lo, uint32_t id, uint32_t acc0, uint32_t acc1) {
+    mma_f16(lead, d0, a, b_lo, id, acc0);
+    mma_f16(lead, d1, a + 8, b_lo + 2, id, acc1);
+    mma_f16(lead, d0, a + 16, b_lo + 4, id, 1);
+    mma_f16(lead, d1, a + 24, b_lo + 6, id, 1);
 }
 // the barrier gets one arrival when every MMA this thread issued before has completed
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+__device__ __forceinline__ void mma_commit(bool lead, uint32_t bar) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(bar), "r"(uint32_t(lead)) : "memory");
 }
 // 16 consecutive fp32 columns of this thread's lane (lane = 32 * (warp & 3) + lane id)
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
