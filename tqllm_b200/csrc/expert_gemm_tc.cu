@@ -19,12 +19,13 @@
 //      cycles per four rows and stays for calls whose scratch holds no rows in slot order;
 //   two accumulators of 128 columns alternate between items of up to 128 tokens, so the epilogue of one item (SwiGLU, stores)
 //   overlaps the products of the next; a wider item takes both. An item of up to 64 tokens splits its K over the two halves of
-//   its accumulator and the epilogue adds them: half as long a chain of truncated sums (NVFP4 gate/up, relative error against
-//   64 bits 3.7e-7 and 8.3e-7 in one chain); the products' pace is the same either way.
+//   its accumulator (products in turn), and the epilogue adds them: half as long a chain of truncated sums (NVFP4 gate/up, relative error against
+//   64 bits 3.7e-7 and 8.3e-7 in one chain); the products' pace is the same either way. In launches of narrow items (by_chunk) the halves take an even
+//   number of chunks in turn, and an item of up to 32 tokens has a quarter each for their even and odd products (NVFP4, K = 2048: 1.9e-7 in halves, 1.1e-7 in quarters).
 // The control warps share their schedulers with six others, so what they execute per unit bounds the block: they walk uniform
 // loops, one elected lane issues, and the raw blocks and rows come in the largest boxes that fit. They are the first warps of the
 // block: as the last ones they were served last (c3 decode gate/up 110 us, as the first 78).
-// Warps: 0 issues tcgen05.mma; 1 streams the raw blocks (256 columns of the item's eight row tiles per ring slot: one TMA box
+// Warps: 0 issues tcgen05.mma, and so does 3 unless it gathers rows; 1 streams the raw blocks (256 columns of the item's eight row tiles per ring slot: one TMA box
 // of the down bank, one each of gate and up, running ahead across items); 2 (when it gathers 2..7) loads B; then from 4 (8) on
 // eight epilogue warps (two per TMEM lane quarter, 16-token groups in turn) and sixteen that decode A (the j-th: lane quarter j & 3, row tile
 // (j >> 2) & 1 of it, every other 256-column chunk). One barrier per step says that its products are done (a commit costs the issuing thread
@@ -57,9 +58,10 @@ constexpr int A_STAGES = 4, A_COLS = 64;    // stages of decoded A operand, a un
 constexpr int STEP_RING = 2 * A_STAGES;     // barriers "the products of step g are done"
 constexpr int ACC_COLS = 128, A_COL0 = 2 * ACC_COLS;                // the two accumulators, then the A stages: all 512 columns
 constexpr int SPLIT_COLS = ACC_COLS / 2;    // items of up to this many tokens split their K over the halves of the accumulator
+constexpr int QUARTER_COLS = SPLIT_COLS / 2;  // those of up to this many over its quarters (GemmArgs::by_chunk)
 constexpr int MAX_B_STAGES = 8, RAW_SLOTS = 6, MAX_CAP = 256;
-constexpr int MMA_WARP = 0, RAW_WARP = 1, LOAD_WARP0 = 2, EPI_WARPS = 8, DEC_WARPS = 16;
-// warps that load rows: one with boxes (and one idle: the roles behind start at a multiple of four, a TMEM lane quarter each), six gather
+constexpr int MMA_WARP = 0, RAW_WARP = 1, LOAD_WARP0 = 2, MMA_WARP1 = 3, EPI_WARPS = 8, DEC_WARPS = 16;
+// warps that load rows: one with boxes (behind it the second issuer: the other roles start at a multiple of four, a TMEM lane quarter each), six gather
 constexpr int load_warps(bool gather) { return gather ? 6 : 2; }
 constexpr int g_threads(bool gather) { return (LOAD_WARP0 + load_warps(gather) + EPI_WARPS + DEC_WARPS) * 32; }
 static_assert(EPI_WARPS * 32 == MAX_CAP, "an epilogue thread looks one token up");
@@ -79,6 +81,7 @@ struct GemmArgs {
     int out_dtype;
     int rows, k, experts, topk, A;
     int cap, cap_log2, b_stages, raw_slots; // most tokens of an item; B stages; raw chunks in the ring
+    int by_chunk;                           // items of up to SPLIT_COLS tokens split their K by chunks (and products), not by products: cap <= 64, an even number of chunks
     int b_pair;                             // 1: the B stages are filled and freed a unit at a time, beside the A stage of the unit and through its barriers (b_stages = 2 A_STAGES)
 };
 // x[i]: the activation rows, boxes of (i + 1) cap / 4 rows (a gathering launch: x[0], one row); w: banks (gate, up) or (down, -), then the shared expert's
@@ -285,10 +288,12 @@ __global__ void exact_rows_k(const typename Elem<DT>::type * x, const int * plan
 // F32_OUT: an instance for fp32 results and one for 16-bit ones, chosen by the call's output type. A branch at the stores, or two
 // loops in one kernel, cost every fp32 caller: c3 down (80 tokens x K = 512) 262 us against 184, c5 gate/up 1305 against 1240.
 // GATHER: the activation rows lie in token order.
-template <uint32_t T, int MODE, bool F32_OUT, bool GATHER, int TERMS = 0>
+// NARROW: two issuers (launches of items of up to 64 tokens, GemmArgs::by_chunk). What the others do not use would cost them 1 % (c3 prefill 625 -> 633 us).
+template <uint32_t T, int MODE, bool F32_OUT, bool GATHER, int TERMS = 0, bool NARROW = false>
 __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs p, const __grid_constant__ GemmMaps maps) {
     using D = gdec::Dec<T>;
-    constexpr bool EXACT = TERMS > 0;
+    constexpr bool EXACT = TERMS > 0, TWO = !GATHER && (NARROW || EXACT);            // TWO: two issuers
+    static_assert(!NARROW || (!GATHER && !EXACT));
     using X = gdec::Exact<EXACT ? T : uint32_t(T_Q4_K)>;
     static_assert(!EXACT || X::SCRATCH <= D::SCRATCH);
     constexpr int PLANES = EXACT ? TERMS : 1;                          // rows of B per token
@@ -334,7 +339,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
         for (int i = 0; i < STEP_RING; ++i) bar_init(done + 8 * i, 1);
 #pragma unroll 1
         for (int i = 0; i < MAX_B_STAGES; ++i) bar_init(b_full + 8 * i, GATHER ? LOAD_WARPS : 1);
-        for (int i = 0; i < 2; ++i) { bar_init(acc_full + 8 * i, 1); bar_init(acc_empty + 8 * i, EPI_WARPS); }
+        for (int i = 0; i < 2; ++i) { bar_init(acc_full + 8 * i, NARROW ? 2 : 1); bar_init(acc_empty + 8 * i, EPI_WARPS); }
         bar_init(drain, 1);
         bar_init(tok_bar, EPI_WARPS);
 #pragma unroll 1
@@ -437,7 +442,8 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
         if (int(blockIdx.x) < n_items) { im = locate(blockIdx.x, at); fetch(im); ok = put(0); }
 #pragma unroll 1
         for (int it = blockIdx.x; it < n_items && ok && !*abort_flag; it += gridDim.x, ++ic, im = after) {
-            const bool wide = im.nv > ACC_COLS, split = im.nv <= SPLIT_COLS;
+            const bool wide = im.nv > ACC_COLS;
+            const int parts = im.nv > SPLIT_COLS ? 1 : (NARROW || (GATHER && p.by_chunk)) && im.nv <= QUARTER_COLS ? 4 : 2;      // sums that an item's K is split into
             const uint32_t h = wide ? 0 : next;
             next = wide ? 0 : next ^ 1u;
             if (it + int(gridDim.x) < n_items) { after = locate(it + gridDim.x, at); fetch(after); }
@@ -522,16 +528,29 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
 #pragma unroll 1
             for (int c = first; c < im.nv; c += 32) {
                 uint32_t v[16];
-                tmem_ld16(taddr + c, v);
-                if (split) {
+                if ((NARROW || GATHER) && parts == 4) {
+                    // pairs first: which of a block's chunks an item begins with must not show in the sum
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        uint32_t w[4][8];
+#pragma unroll
+                        for (int q4 = 0; q4 < 4; ++q4) tmem_ld8(taddr + q4 * QUARTER_COLS + c + 8 * i, w[q4]);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            v[8 * i + j] = __float_as_uint((__uint_as_float(w[0][j]) + __uint_as_float(w[1][j])) + (__uint_as_float(w[2][j]) + __uint_as_float(w[3][j])));
+                    }
+                } else {
+                    tmem_ld16(taddr + c, v);
+                }
+                if (parts == 2) {
                     uint32_t w[16];
                     tmem_ld16(taddr + SPLIT_COLS + c, w);
                     tmem_ld_wait();
 #pragma unroll
                     for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
-                } else {
-                    tmem_ld_wait();
                 }
+                tmem_ld_wait();
 #pragma unroll
                 for (int j0 = 0; j0 < 16; j0 += 8) {
                     int4 two[4];                                       // tokens j, j + 1: (assignment, scale) each
@@ -661,14 +680,15 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
             }
         }
         if (!ok && lane == 0) give_up();
-    } else if (warp == MMA_WARP) {
-        // ---- MMA issuer: the whole warp walks the loops, one elected lane issues (a predicate on the instruction, not a branch: in a
-        // branch of one lane every operand is moved to the uniform registers first). What an issue costs decides the pace of narrow items: the
-        // tensor core takes N / 2 cycles a product (at least 16), the issuing thread beside busy decoders 43 when it was a branch, with its operands'
-        // addresses constant but for one addend (the loop is unrolled over the A stages) and 58 with addresses of a running stage
-        // (microbenchmark, N = 64, cycles a product with its share of the unit's wait and commit); a unit now 260 cycles beside its waits, 430 before ----
-        const uint32_t b_lo0 = sw128_desc_lo(saddr(b_st)), b_step = uint32_t(p.cap * 128 * PLANES) >> 4;
+    } else if (warp == MMA_WARP || (TWO && warp == MMA_WARP1)) {
+        // ---- MMA issuers: the whole warp walks the loops, one elected lane issues (a predicate on the instruction, not a branch: in a
+        // branch of one lane every operand is moved to the uniform registers first: 43 cycles a product beside busy decoders). What an issue costs decides the pace of
+        // narrow items, whose products take the tensor core 16 to 32 cycles each: with its waits, commits and the walk it is 300 to 450 cycles a unit of eight. So those
+        // have two issuers, each for the chunks of one group of decoders, in stages, sums and barriers of their own; a gathering launch has the same sums from one. One / two issuers, us a layer: c3 decode 8 66.9 / 65.2, c5 decode 24 309 / 292,
+        // c2 509 tokens 323 / 315, c4 600 685 / 666 ----
         const bool lead = elect_one();
+        const uint32_t me = TWO && warp == MMA_WARP1 ? 1 : 0;
+        const uint32_t b_lo0 = sw128_desc_lo(saddr(b_st)), b_step = uint32_t(p.cap * 128 * PLANES) >> 4;
         uint32_t gu = 0, next = 0, uses0 = 0, uses1 = 0;
         bool ok = true;
 #pragma unroll 1
@@ -678,16 +698,51 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
             const uint32_t h = wide ? 0 : next;
             next = wide ? 0 : next ^ 1u;
             const uint32_t npad = uint32_t(max(im.nv, 1) + 15) & ~15u, id = idesc(128, npad * PLANES, 0), d = tmem + h * ACC_COLS;
-            const uint32_t second = !EXACT && im.nv <= SPLIT_COLS ? SPLIT_COLS : 0;          // columns from the accumulator of even products to that of odd ones
             if constexpr (!EXACT) {
             if (wide || h == 0) { if (uses0 > 0) ok = warp_wait(acc_empty, (uses0 - 1) & 1u) && ok; ++uses0; }
             if (wide || h == 1) { if (uses1 > 0) ok = warp_wait(acc_empty + 8, (uses1 - 1) & 1u) && ok; ++uses1; }
             fence_after();
             }
+            // from the first to the second step of a unit: with b_pair one box holds both; else B stages in turn
+            const uint32_t b_unit = !GATHER ? uint32_t(b_class(im.nv) + 1) * (uint32_t(class_rows * 128 * PLANES) >> 4) : b_step;
+            // this issuer's chunks of the item
+            auto chunks = [&](auto ME) {
+                constexpr uint32_t s0 = 2 * decltype(ME)::value;
+                const uint32_t c0 = gu >> 1, d0 = d + decltype(ME)::value * SPLIT_COLS, d1 = im.nv <= QUARTER_COLS ? d0 + QUARTER_COLS : d0;
+                uint32_t acc = 0;
+#pragma unroll 1
+                for (uint32_t c = c0 + ((c0 ^ decltype(ME)::value) & 1u); c < c0 + uint32_t(nchunks); c += 2) {
+                    const uint32_t turn = c >> 1;
+                    const int left = ksteps - 4 * int(c - c0);
+                    if constexpr (EXACT) { if (turn > 0 && !warp_wait(acc_empty + 8 * decltype(ME)::value, (turn - 1) & 1u)) return false; }
+#pragma unroll
+                    for (uint32_t u = 0; u < 2; ++u) {
+                        const uint32_t s = s0 + u, a = tmem + A_COL0 + s * A_COLS, b = b_lo0 + 2 * s * b_step;
+                        if (!warp_wait(a_full + 8 * s, turn & 1u)) return false;
+                        fence_after();
+                        if constexpr (EXACT) {
+                            const uint32_t ds = tmem + decltype(ME)::value * X_SET;
+                            mma_step(lead, ds, ds, a, b, id, u, 1);
+                            mma_step(lead, ds, ds, a + A_COLS / 2, b + b_unit, id, 1, 1);
+                            if constexpr (X::MINS)
+                                if (u == 0) mma_f16<SW32_DESC_HI>(lead, ds + X_MINS, tmem + X_AMINS + 8 * decltype(ME)::value, sw128_desc_lo(saddr(mins_st) + s * (X_CAP * 32)), idesc(128, npad, 0), 0);
+                        } else {
+                            if (left > 2 * int(u)) mma_step(lead, d0, d1, a, b, id, acc, acc | uint32_t(d1 == d0));
+                            if (left > 2 * int(u) + 1) mma_step(lead, d0, d1, a + A_COLS / 2, b + b_unit, id, 1, 1);
+                            acc = 1;
+                        }
+                        mma_commit(lead, done + 16 * s + 8);
+                    }
+                    if constexpr (EXACT) mma_commit(lead, acc_full + 8 * decltype(ME)::value);
+                }
+                if constexpr (!EXACT) mma_commit(lead, acc_full + 8 * h);
+                return true;
+            };
             auto products = [&](auto PAIR) {
-                // from the first to the second step of a unit: with b_pair one box holds both; else B stages in turn
-                const uint32_t b_half = PAIR && !GATHER ? uint32_t(b_class(im.nv) + 1) * (uint32_t(class_rows * 128 * PLANES) >> 4) : b_step;
-                uint32_t first = gu % A_STAGES, turn = gu / A_STAGES, acc = 0;
+                const bool by_chunk = GATHER && p.by_chunk && im.nv <= SPLIT_COLS;      // (rows in slot order: chunks())
+                const uint32_t second = im.nv > SPLIT_COLS ? 0 : !by_chunk ? SPLIT_COLS : im.nv <= QUARTER_COLS ? QUARTER_COLS : 0;      // columns from the accumulator of even products to that of odd ones
+                const uint32_t b_half = PAIR && !GATHER ? b_unit : b_step;
+                uint32_t first = gu % A_STAGES, turn = gu / A_STAGES;
                 int left = ksteps, units = 2 * nchunks;
 #pragma unroll 1
                 while (true) {
@@ -712,15 +767,16 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                             continue;
                         }
                         fence_after();
-                        if (left > 0) mma_step(lead, d, d + second, a, b, id, acc, acc | (second == 0));
+                        const uint32_t dh = by_chunk ? d + (s >> 1) * SPLIT_COLS : d;
+                        const uint32_t acc = left != ksteps && !(by_chunk && left == ksteps - 4);      // the first unit of an item, or of either half, overwrites
+                        if (left > 0) mma_step(lead, dh, dh + second, a, b, id, acc, acc | (second == 0));
                         if constexpr (!PAIR) {
                             mma_commit(lead, done + 16 * s);
                             if (!warp_wait(b_full + 8 * (sb + 1), (2 * turn + (s >> 1)) & 1u)) return false;
                             fence_after();
                         }
-                        if (left > 1) mma_step(lead, d, d + second, a + A_COLS / 2, b + b_half, id, 1, 1);
+                        if (left > 1) mma_step(lead, dh, dh + second, a + A_COLS / 2, b + b_half, id, 1, 1);
                         mma_commit(lead, done + 16 * s + 8);
-                        acc = 1;
                         left -= 2;
                         if (--units == 0) { mma_commit(lead, acc_full + 8 * h); return true; }
                     }
@@ -728,14 +784,16 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                     ++turn;
                 }
             };
-            if constexpr (EXACT) ok = ok && products(std::true_type{});
+            if constexpr (TWO) ok = ok && (me ? chunks(std::integral_constant<uint32_t, 1>{}) : chunks(std::integral_constant<uint32_t, 0>{}));
+            else if constexpr (EXACT) ok = ok && products(std::true_type{});
             else ok = ok && (p.b_pair ? products(std::true_type{}) : products(std::false_type{}));
             gu += 2 * nchunks;
         }
         if (!ok && lane == 0) give_up();
         // nothing may be in flight when the tensor memory is freed (after a clean run the epilogue has waited for all of it)
-        mma_commit(lead, drain);
-        warp_wait(drain, 0);
+        const uint32_t mine = me ? b_full + 8 * (MAX_B_STAGES - 1) : drain;      // (that many B stages come through the A stages' barriers)
+        mma_commit(lead, mine);
+        warp_wait(mine, 0);
     } else if (warp == RAW_WARP) {
         // ---- raw blocks ----
         constexpr int PARTS = chunk_parts<T>();
@@ -849,6 +907,7 @@ template <uint32_t T> bool gemm_fit(int experts, int cap_wanted, GemmArgs & a) {
             if (gemm_smem<T>(experts, o[0], o[1], s) <= GEMM_SMEM_LIMIT) {
                 a.cap = o[0]; a.cap_log2 = o[0] == 256 ? 8 : o[0] == 128 ? 7 : 6; a.b_stages = o[1]; a.raw_slots = s;
                 a.b_pair = o[1] == 2 * A_STAGES;
+                a.by_chunk = a.cap <= SPLIT_COLS && ceil_div(a.k, 256) % 2 == 0;
                 return true;
             }
     }
@@ -937,7 +996,8 @@ int32_t gemm_launch_t(GemmArgs a, long long live, const b2moe_bank * const * m, 
         if (m[i]) mapped = mapped && bank_map<T>(maps.w[i], m[i], MODE == 0 ? 4 : 8);
     if (!mapped) return B2MOE_ERR_CUDA;
     const size_t smem = gemm_smem<T>(a.experts, a.cap, a.b_stages, a.raw_slots);
-    auto kernel = a.out_dtype == B2MOE_F32 ? gemm_tc_k<T, MODE, true, false> : gemm_tc_k<T, MODE, false, false>;
+    auto kernel = a.by_chunk ? (a.out_dtype == B2MOE_F32 ? gemm_tc_k<T, MODE, true, false, 0, true> : gemm_tc_k<T, MODE, false, false, 0, true>)
+                             : a.out_dtype == B2MOE_F32 ? gemm_tc_k<T, MODE, true, false> : gemm_tc_k<T, MODE, false, false>;
     if constexpr (MODE == 0)
         if (!slots) {
             if (a.out_dtype != B2MOE_F32) return B2MOE_ERR_SHAPE;      // calls with 16-bit results bring scratch for the rows in slot order
