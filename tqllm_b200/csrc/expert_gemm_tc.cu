@@ -84,8 +84,12 @@ struct GemmArgs {
     int by_chunk;                           // items of up to SPLIT_COLS tokens split their K by chunks (and products), not by products: cap <= 64, an even number of chunks
     int b_pair;                             // 1: the B stages are filled and freed a unit at a time, beside the A stage of the unit and through its barriers (b_stages = 2 A_STAGES)
 };
-// x[i]: the activation rows, boxes of (i + 1) cap / 4 rows (a gathering launch: x[0], one row); w: banks (gate, up) or (down, -), then the shared expert's
-struct GemmMaps { CUtensorMap x[4], w[4]; };
+// The rows' boxes: sixteen rows and multiples of them, as many as the products take (32 in launches of items of up to 256 tokens). With boxes in quarters of
+// `cap` 80 tokens brought 96 rows. Layers, us: c3 prefill 626 -> 623.5, c4 prefill 974 -> 966, c5 prefill 2785 -> 2768
+constexpr int BOXES = 8;
+__host__ __device__ inline int box_log2(int cap) { return cap > 16 * BOXES ? 5 : 4; }
+// x[i]: the activation rows, boxes of i + 1 times 1 << box_log2(cap) rows (a gathering launch: x[0], one row; the exact form: x[0], x[1], and of the sub-block sums x[2], x[3]); w: banks (gate, up) or (down, -), then the shared expert's
+struct GemmMaps { CUtensorMap x[BOXES], w[4]; };
 
 template <uint32_t T> constexpr int chunk_tiles() { return 256 / Fmt<T>::KT; }
 template <uint32_t T> constexpr int chunk_bytes() { return chunk_tiles<T>() * Fmt<T>::TILE; }
@@ -405,9 +409,9 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
         return r;
     };
     auto x_row = [&](int a) { return MODE == 0 ? (a < p.A ? a / p.topk : a - p.A) : a; };
-    // the rows' boxes come in four sizes: the smallest that holds the item's tokens
-    auto b_class = [&](int nv) { return max(nv - 1, 0) >> (EXACT ? 4 : p.cap_log2 - 2); };
-    const int class_rows = EXACT ? 16 : p.cap / 4;
+    // the smallest box that holds the item's tokens
+    auto b_class = [&](int nv) { return max(nv - 1, 0) >> (EXACT ? 4 : box_log2(p.cap)); };
+    const int class_rows = EXACT ? 16 : 1 << box_log2(p.cap);
     auto give_up = [&]() { *abort_flag = 1; atomicExch(p.plan + PLAN_STATUS, 2); };
     int at = 0;
 
@@ -990,7 +994,7 @@ int32_t gemm_launch_t(GemmArgs a, long long live, const b2moe_bank * const * m, 
     a.inv_scale = inv;
     GemmMaps maps;
     bool mapped = true;
-    if (slots) for (int i = 0; i < 4; ++i) mapped = mapped && rows_map(maps.x[i], xb, rows, a.k, (i + 1) * a.cap / 4, a.b_pair ? 2 : 1);
+    if (slots) for (int i = 0; i < a.cap >> box_log2(a.cap); ++i) mapped = mapped && rows_map(maps.x[i], xb, rows, a.k, (i + 1) << box_log2(a.cap), a.b_pair ? 2 : 1);
     else mapped = gather_map(maps.x[0], xb, rows, a.k);
     for (int i = 0; i < 4; ++i)
         if (m[i]) mapped = mapped && bank_map<T>(maps.w[i], m[i], MODE == 0 ? 4 : 8);
