@@ -291,31 +291,24 @@ template <> struct Exact<T_IQ3S4> {
 
 // ---------------------------------------------------------------------------------------------------------------
 // The eight 4-bit codes of a word -> their kvalues (exact) times `scale`, in nibble order, through a 256-entry table byte ->
-// half2 in shared memory with a copy per lane (no bank conflicts: entry b of lane l at word 32 b + l). Per code byte: a byte
-// permute extracts it, a multiply-add makes the address, one load, one product by the scale. The integer pipe takes one of
-// the four: it is the one these formats fill (shift, mask and add take three: c5, 24 tokens, gate/up 332 us at 0.69 of that
-// pipe; byte permutes over a codebook in registers 23 instructions a word, fifteen of them there: 370 us).
+// half2 in shared memory with a copy per lane (no bank conflicts: entry b of lane l at word 32 b + l). Per code byte: a dot product
+// of the word's four bytes with 128 at that byte's place and 0 elsewhere makes the address (extraction, scaling and base in one instruction), one load, one product by
+// the scale. With a byte permute and a multiply-add for the address: c5, 24 tokens 277 -> 263.5 us a layer; with shift, mask and add gate/up was bound by the integer pipe (332 us, 0.69 of it), byte
+// permutes over a codebook in registers take 23 instructions a word, fifteen of them there (370 us).
 constexpr int LUT_BYTES = 256 * 32 * 4;
 __device__ inline void build_lut(void * tab, int tid, int nthreads) {
     uint32_t * lut = static_cast<uint32_t *>(tab);
     for (int i = tid; i < 256 * 32; i += nthreads) lut[i] = pack_h2(float(c_kvalues_iq4nl[(i >> 5) & 15]), float(c_kvalues_iq4nl[i >> 9]));
 }
-// the lane's copy: its shared-memory address and the 128 bytes between entries, opaque so that the address stays a multiply-add
-struct Lut { uint32_t base, stride; };
-__device__ __forceinline__ Lut lut_of(const void * tab, int lane) {
-    Lut l{uint32_t(__cvta_generic_to_shared(tab)) + 4u * uint32_t(lane), 0};
-    asm volatile("mov.b32 %0, 128;" : "=r"(l.stride));
-    return l;
-}
-__device__ __forceinline__ uint4 lut_word(const Lut & l, uint32_t w, __half2 scale) {
-    auto val = [&](uint32_t sel) {
-        uint32_t b, at, v;
-        asm("prmt.b32 %0, %1, 0, %2;" : "=r"(b) : "r"(w), "r"(sel));
-        asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(at) : "r"(b), "r"(l.stride), "r"(l.base));
-        asm("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(at));
+// the lane's copy: its shared-memory address
+__device__ __forceinline__ uint32_t lut_of(const void * tab, int lane) { return uint32_t(__cvta_generic_to_shared(tab)) + 4u * uint32_t(lane); }
+__device__ __forceinline__ uint4 lut_word(uint32_t base, uint32_t w, __half2 scale) {
+    auto val = [&](uint32_t entry_bytes) {                             // 128, the bytes of an entry, at the code byte's place
+        uint32_t v;
+        asm("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(__dp4a(w, entry_bytes, base)));
         return h2_bits(__hmul2(bits_h2(v), scale));
     };
-    return make_uint4(val(0x4440u), val(0x4441u), val(0x4442u), val(0x4443u));
+    return make_uint4(val(0x00000080u), val(0x00008000u), val(0x00800000u), val(0x80000000u));
 }
 
 template <> struct Dec<T_IQ4_XS> {
@@ -342,7 +335,7 @@ template <> struct Dec<T_IQ4_XS> {
     struct Raw { uint4 w; };
     template <int J> __device__ __forceinline__ static Raw load(const uint8_t * chunk, int lane, const uint8_t *) { return Raw{plane(chunk, J, lane)}; }
     template <int J> __device__ __forceinline__ static void step(const Raw & raw, int lane, const void * tab, const Pre & p, uint32_t (&f)[16]) {
-        const Lut lut = lut_of(tab, lane);
+        const uint32_t lut = lut_of(tab, lane);
         const int src = (lane & ~3) | (2 * (J & 1));
         const __half2 d0 = bits_h2(__shfl_sync(0xffffffffu, p.dl[J >> 1], src)), d1 = bits_h2(__shfl_sync(0xffffffffu, p.dl[J >> 1], src + 1));
         put(f, 0, 0, lut_word(lut, raw.w.x, __low2half2(d0)));
@@ -372,7 +365,7 @@ template <> struct Dec<T_IQ4_NL> {
         return raw;
     }
     template <int J> __device__ __forceinline__ static void step(const Raw & raw, int lane, const void * tab, const Pre &, uint32_t (&f)[16]) {
-        const Lut lut = lut_of(tab, lane);
+        const uint32_t lut = lut_of(tab, lane);
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
             put(f, 0, b, lut_word(lut, raw.w[b].x, __half2half2(raw.d[b][0])));
