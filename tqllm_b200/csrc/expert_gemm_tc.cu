@@ -67,11 +67,15 @@ constexpr int g_threads(bool gather) { return (LOAD_WARP0 + load_warps(gather) +
 static_assert(EPI_WARPS * 32 == MAX_CAP, "an epilogue thread looks one token up");
 static_assert(MAX_B_STAGES <= STEP_RING, "a B stage is freed by the barrier of the step that used it");
 // The exact form (TERMS > 0): items of up to X_CAP tokens at every density (an expert of 100 tokens is decoded four times: 1000 tokens on 60 experts 311 us,
-// 168 with the other form's items of 128); two sets of sums, a chunk's each: X_CAP columns per term of the activations, then X_CAP
-// of the mins; after both the mins' A operand of either chunk. X_RING: chunks whose row constants the epilogue may still need
-constexpr int X_CAP = 32, X_SET = 3 * X_CAP, X_MINS = 2 * X_CAP, X_AMINS = 2 * X_SET, X_RING = 4;
-static_assert(X_AMINS + 2 * 8 <= A_COL0, "two sets of sums and two operands of mins below the A stages");
-constexpr int N_BARS = 3 * RAW_SLOTS + A_STAGES + STEP_RING + MAX_B_STAGES + X_RING + 6;
+// 168 with the other form's items of 128); sets of sums, a chunk's each: X_CAP columns per term of the activations, then X_CAP
+// of the mins; after them the mins' A operand of either group's chunk. As many sets as fit: with two of them the products waited for the epilogue warps
+// (445 of 1140 cycles a unit): c2, 509 tokens 316.6 -> 313.4 us, c4, 600 tokens 670 -> 666.5. x_ring: chunks whose row constants the epilogue may still need: those are written when the products of
+// the chunk two before are done, so when the sums of the chunk x_sets + 2 before are read
+constexpr int X_CAP = 32;
+constexpr int x_sets(bool mins, int terms) { return !mins ? 4 : terms == 1 ? 3 : 2; }
+constexpr int x_set_cols(bool mins, int terms) { return X_CAP * (terms + (mins ? 1 : 0)); }
+constexpr int x_ring(bool mins, int terms) { return x_sets(mins, terms) > 2 ? 8 : 4; }
+constexpr int N_BARS = 3 * RAW_SLOTS + A_STAGES + STEP_RING + MAX_B_STAGES + 10;
 
 struct GemmArgs {
     const float * aux0, * aux1, * saux0, * saux1;      // row scales of the banks (gate, up) or (down, -) and of the shared expert's (may be null)
@@ -101,10 +105,12 @@ template <uint32_t T> constexpr int part_words() { return chunk_bytes<T>() / chu
 struct Info { int cum, e, cnt, off; };
 
 // what the exact form keeps beside the operands: the mins' B tiles (32 bytes a row) and the rows' constants
-constexpr size_t exact_smem(int terms) { return terms ? size_t(A_STAGES) * X_CAP * 32 + size_t(X_RING) * 128 * sizeof(float2) : 0; }
+constexpr size_t exact_smem(bool mins, int terms) {
+    return !terms ? 0 : mins ? size_t(A_STAGES) * X_CAP * 32 + size_t(x_ring(true, terms)) * 128 * sizeof(float2) : size_t(8192);      // (no mins: a float a row, 4 KB, would do)
+}
 template <uint32_t T>
 constexpr size_t gemm_smem(int experts, int cap, int b_stages, int raw_slots, int terms = 0) {
-    return 1024 + size_t(b_stages) * cap * 128 * (terms ? terms : 1) + exact_smem(terms) + size_t(8) * raw_slots * chunk_bytes<T>() + gdec::Dec<T>::TAB_BYTES +
+    return 1024 + size_t(b_stages) * cap * 128 * (terms ? terms : 1) + exact_smem(T == T_Q4_K, terms) + size_t(8) * raw_slots * chunk_bytes<T>() + gdec::Dec<T>::TAB_BYTES +
            DEC_WARPS * gdec::Dec<T>::SCRATCH + size_t(experts + 2) * sizeof(Info) + 2 * MAX_CAP * sizeof(int2) + size_t(N_BARS) * 8 + 16;
 }
 
@@ -310,9 +316,9 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
     // the block's shared memory became a generic load with 64-bit addresses
     uint8_t * smem = smem_raw + (-saddr(smem_raw) & 1023u);
     uint8_t * b_st = smem;                                            // [b_stages][cap][128 bytes], swizzled
-    uint8_t * mins_st = b_st + size_t(p.b_stages) * p.cap * 128 * PLANES;       // exact: [A stages][X_CAP][32 bytes], swizzled; then the row constants, [X_RING][128]
-    float2 * consts = reinterpret_cast<float2 *>(mins_st + A_STAGES * X_CAP * 32);
-    uint8_t * raw = mins_st + exact_smem(TERMS);                      // [raw_slots][8 row tiles][CB]
+    uint8_t * mins_st = b_st + size_t(p.b_stages) * p.cap * 128 * PLANES;       // exact: [A stages][X_CAP][32 bytes], swizzled (only with mins); then the row constants, [x_ring][128]
+    float2 * consts = reinterpret_cast<float2 *>(mins_st + (X::MINS ? A_STAGES * X_CAP * 32 : 0));
+    uint8_t * raw = mins_st + exact_smem(X::MINS, TERMS);                      // [raw_slots][8 row tiles][CB]
     uint8_t * dec_tab = raw + size_t(8) * p.raw_slots * CB;           // the decoder's lookup table
     uint8_t * dec_scratch = dec_tab + D::TAB_BYTES;                   // [decode warps][SCRATCH]
     Info * info = reinterpret_cast<Info *>(dec_scratch + DEC_WARPS * D::SCRATCH);   // [na + 1]
@@ -323,7 +329,12 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
     const int S = p.raw_slots, BS = p.b_stages;
     const uint32_t raw_full = saddr(bars), raw_empty = raw_full + 16 * RAW_SLOTS, a_full = raw_empty + 8 * RAW_SLOTS,
                    done = a_full + 8 * A_STAGES, b_full = done + 8 * STEP_RING, acc_full = b_full + 8 * MAX_B_STAGES, acc_empty = acc_full + 16,
-                   drain = acc_empty + 16, tok_bar = drain + 8, const_full = tok_bar + 8;
+                   drain = acc_empty + 16, tok_bar = drain + 8;
+    // the exact form: as many barriers as sets and chunks of constants, in place of those that it does not need (B stages come through the A stages' barriers)
+    constexpr int SETS = x_sets(X::MINS, TERMS), SET_COLS = x_set_cols(X::MINS, TERMS), MINS_COL = X_CAP * TERMS, AMINS = SETS * SET_COLS, CONSTS = x_ring(X::MINS, TERMS);
+    static_assert(!EXACT || AMINS + (X::MINS ? 2 * 8 : 0) <= A_COL0, "sets of sums and two operands of mins below the A stages");
+    static_assert(CONSTS <= MAX_B_STAGES && SETS <= 4 && CONSTS >= SETS + 2);
+    const uint32_t const_full = b_full, set_full = tok_bar + 8, set_empty = acc_full;
     // The warp's number as a shuffle's result: the compiler then knows it, and with it the roles' branches, their loops and addresses, to be the same in the whole warp, and
     // keeps them in uniform registers: fewer instructions in every role, and products issued without moving their operands there one by one.
     // c3 decode 8 73.0 -> 66.9 us, c5 decode 24 308 -> 292 (309 with the issuing branch taken by one lane), c2 509 tokens 351 -> 323, c4 600 745 -> 685
@@ -342,12 +353,12 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
 #pragma unroll 1
         for (int i = 0; i < STEP_RING; ++i) bar_init(done + 8 * i, 1);
 #pragma unroll 1
-        for (int i = 0; i < MAX_B_STAGES; ++i) bar_init(b_full + 8 * i, GATHER ? LOAD_WARPS : 1);
-        for (int i = 0; i < 2; ++i) { bar_init(acc_full + 8 * i, NARROW ? 2 : 1); bar_init(acc_empty + 8 * i, EPI_WARPS); }
+        for (int i = 0; i < MAX_B_STAGES; ++i) bar_init(b_full + 8 * i, EXACT ? 8 : GATHER ? LOAD_WARPS : 1);
+        for (int i = 0; i < 2; ++i) { bar_init(acc_full + 8 * i, EXACT ? EPI_WARPS : NARROW ? 2 : 1); bar_init(acc_empty + 8 * i, EPI_WARPS); }
         bar_init(drain, 1);
         bar_init(tok_bar, EPI_WARPS);
 #pragma unroll 1
-        for (int i = 0; i < X_RING; ++i) bar_init(const_full + 8 * i, 8);
+        for (int i = 0; EXACT && i < 4; ++i) bar_init(set_full + 8 * i, 1);
         *abort_flag = 0;
         bar_init_fence();
     }
@@ -481,10 +492,12 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                 for (int i = 0; i < 16; ++i) sum[i >> 3][i & 7] = 0.f;
 #pragma unroll 1
                 for (int c = 0; c < nchunks; ++c, ++uses0) {
-                    const uint32_t set = uses0 & 1u, at_set = tmem + (uint32_t(32 * q) << 16) + set * X_SET;
-                    if (!warp_wait(const_full + 8 * (uses0 % X_RING), (uses0 / X_RING) & 1u)) { ok = false; break; }
-                    const float2 k = consts[(uses0 % X_RING) * 128 + 32 * q + lane];
-                    if (!warp_wait(acc_full + 8 * set, (uses0 >> 1) & 1u)) { ok = false; break; }
+                    const uint32_t set = uses0 % SETS, at_set = tmem + (uint32_t(32 * q) << 16) + set * SET_COLS;
+                    if (!warp_wait(const_full + 8 * (uses0 % CONSTS), (uses0 / CONSTS) & 1u)) { ok = false; break; }
+                    float2 k;
+                    if constexpr (X::MINS) k = consts[(uses0 % CONSTS) * 128 + 32 * q + lane];
+                    else k.x = reinterpret_cast<const float *>(consts)[(uses0 % CONSTS) * 128 + 32 * q + lane];
+                    if (!warp_wait(set_full + 8 * set, (uses0 / SETS) & 1u)) { ok = false; break; }
                     fence_after();
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
@@ -492,7 +505,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                         uint32_t v[8], w[8], z[8];
                         tmem_ld8(at_set + g0 + 16 * i, v);
                         if constexpr (TERMS == 2) tmem_ld8(at_set + lo + g0 + 16 * i, w);
-                        if constexpr (X::MINS) tmem_ld8(at_set + X_MINS + g0 + 16 * i, z);
+                        if constexpr (X::MINS) tmem_ld8(at_set + MINS_COL + g0 + 16 * i, z);
                         tmem_ld_wait();
 #pragma unroll
                         for (int j = 0; j < 8; ++j) {
@@ -504,7 +517,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                     }
                     fence_before();
                     __syncwarp();
-                    if (lane == 0) bar_arrive(acc_empty + 8 * set);
+                    if (lane == 0) bar_arrive(set_empty + 8 * set);
                 }
                 if (!ok) break;
 #pragma unroll
@@ -632,7 +645,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                     __syncwarp();
                     if (lane == 0) {
                         bar_arrive(full + 8 * u);
-                        if (EXACT && u == 0) bar_arrive(const_full + 8 * (group + 2 * (turn & 1u)));
+                        if (EXACT && u == 0) bar_arrive(const_full + 8 * ((group + 2 * turn) % CONSTS));
                         if (u == 1) bar_arrive(raw_empty + 8 * slot);  // every lane is done with the slot (the syncwarp above)
                     }
                 };
@@ -646,13 +659,18 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                 if (!stage_free(0)) { ok = false; break; }
                 tmem_st_16x256b_x4(a_addr, f);
                 if constexpr (EXACT) {
-                    // the chunk's mins and row constants: what used their places belongs to chunks whose sums are read (the wait above)
+                    // the chunk's mins and row constants: what used their places belongs to products that are done, and to chunks whose sums are read (the wait above)
                     if constexpr (X::MINS) {
                         uint32_t mn[4];
                         X::mins(chunk, lane, mn);
-                        tmem_st_16x256b_x1(tmem + (uint32_t(32 * q + 16 * m) << 16) + X_AMINS + 8 * group, mn);
+                        tmem_st_16x256b_x1(tmem + (uint32_t(32 * q + 16 * m) << 16) + AMINS + 8 * group, mn);
                     }
-                    if (lane < 16) consts[(group + 2 * (turn & 1u)) * 128 + 32 * q + 16 * m + lane] = X::consts(chunk, lane);
+                    if (lane < 16) {
+                        const float2 k = X::consts(chunk, lane);
+                        const uint32_t place = ((group + 2 * turn) % CONSTS) * 128 + 32 * q + 16 * m + lane;
+                        if constexpr (X::MINS) consts[place] = k;
+                        else reinterpret_cast<float *>(consts)[place] = k.x;
+                    }
                 }
                 if constexpr (AHEAD) {
                     if constexpr (T == T_Q4_K) {                        // every lane has read the first unit's constants
@@ -718,18 +736,19 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                 for (uint32_t c = c0 + ((c0 ^ decltype(ME)::value) & 1u); c < c0 + uint32_t(nchunks); c += 2) {
                     const uint32_t turn = c >> 1;
                     const int left = ksteps - 4 * int(c - c0);
-                    if constexpr (EXACT) { if (turn > 0 && !warp_wait(acc_empty + 8 * decltype(ME)::value, (turn - 1) & 1u)) return false; }
+                    const uint32_t set = c % SETS;
+                    if constexpr (EXACT) { if (c >= uint32_t(SETS) && !warp_wait(set_empty + 8 * set, (c / SETS - 1) & 1u)) return false; }
 #pragma unroll
                     for (uint32_t u = 0; u < 2; ++u) {
                         const uint32_t s = s0 + u, a = tmem + A_COL0 + s * A_COLS, b = b_lo0 + 2 * s * b_step;
                         if (!warp_wait(a_full + 8 * s, turn & 1u)) return false;
                         fence_after();
                         if constexpr (EXACT) {
-                            const uint32_t ds = tmem + decltype(ME)::value * X_SET;
+                            const uint32_t ds = tmem + set * SET_COLS;
                             mma_step(lead, ds, ds, a, b, id, u, 1);
                             mma_step(lead, ds, ds, a + A_COLS / 2, b + b_unit, id, 1, 1);
                             if constexpr (X::MINS)
-                                if (u == 0) mma_f16<SW32_DESC_HI>(lead, ds + X_MINS, tmem + X_AMINS + 8 * decltype(ME)::value, sw128_desc_lo(saddr(mins_st) + s * (X_CAP * 32)), idesc(128, npad, 0), 0);
+                                if (u == 0) mma_f16<SW32_DESC_HI>(lead, ds + MINS_COL, tmem + AMINS + 8 * decltype(ME)::value, sw128_desc_lo(saddr(mins_st) + s * (X_CAP * 32)), idesc(128, npad, 0), 0);
                         } else {
                             if (left > 2 * int(u)) mma_step(lead, d0, d1, a, b, id, acc, acc | uint32_t(d1 == d0));
                             if (left > 2 * int(u) + 1) mma_step(lead, d0, d1, a + A_COLS / 2, b + b_unit, id, 1, 1);
@@ -737,7 +756,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                         }
                         mma_commit(lead, done + 16 * s + 8);
                     }
-                    if constexpr (EXACT) mma_commit(lead, acc_full + 8 * decltype(ME)::value);
+                    if constexpr (EXACT) mma_commit(lead, set_full + 8 * set);
                 }
                 if constexpr (!EXACT) mma_commit(lead, acc_full + 8 * h);
                 return true;
@@ -757,16 +776,16 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                         if (!warp_wait(a_full + 8 * s, turn & 1u)) return false;
                         if (!PAIR && !warp_wait(b_full + 8 * sb, (2 * turn + (s >> 1)) & 1u)) return false;      // with b_pair a_full stands for the unit's rows too
                         if constexpr (EXACT) {                         // a chunk's units are the stages 0, 1 or 2, 3, its sums a set of their own
-                            const uint32_t set = s >> 1, ds = tmem + set * X_SET;
-                            if ((s & 1) == 0 && turn > 0 && !warp_wait(acc_empty + 8 * set, (turn - 1) & 1u)) return false;
+                            const uint32_t c = 2 * turn + (s >> 1), set = c % SETS, ds = tmem + set * SET_COLS;
+                            if ((s & 1) == 0 && c >= uint32_t(SETS) && !warp_wait(set_empty + 8 * set, (c / SETS - 1) & 1u)) return false;
                             fence_after();
                             mma_step(lead, ds, ds, a, b, id, s & 1, 1);
                             mma_step(lead, ds, ds, a + A_COLS / 2, b + b_half, id, 1, 1);
                             if constexpr (X::MINS)
                                 if ((s & 1) == 0)
-                                    mma_f16<SW32_DESC_HI>(lead, ds + X_MINS, tmem + X_AMINS + 8 * set, sw128_desc_lo(saddr(mins_st) + s * (X_CAP * 32)), idesc(128, npad, 0), 0);
+                                    mma_f16<SW32_DESC_HI>(lead, ds + MINS_COL, tmem + AMINS + 8 * (s >> 1), sw128_desc_lo(saddr(mins_st) + s * (X_CAP * 32)), idesc(128, npad, 0), 0);
                             mma_commit(lead, done + 16 * s + 8);
-                            if (s & 1) mma_commit(lead, acc_full + 8 * set);
+                            if (s & 1) mma_commit(lead, set_full + 8 * set);
                             if (--units == 0) return true;
                             continue;
                         }
@@ -795,7 +814,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
         }
         if (!ok && lane == 0) give_up();
         // nothing may be in flight when the tensor memory is freed (after a clean run the epilogue has waited for all of it)
-        const uint32_t mine = me ? b_full + 8 * (MAX_B_STAGES - 1) : drain;      // (that many B stages come through the A stages' barriers)
+        const uint32_t mine = me ? done : drain;                       // (no step that is the first of a unit has a barrier where there are two issuers)
         mma_commit(lead, mine);
         warp_wait(mine, 0);
     } else if (warp == RAW_WARP) {
