@@ -123,9 +123,15 @@ __global__ void __launch_bounds__(RM_WARPS * 32) router_mma_k(const float * __re
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();                    // the gridDim.z blocks that split the hidden dimension
     grid_release();
-    grid_wait();                                                       // x may be the output of the launch before this one
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int r0 = blockIdx.x * 16, t0 = blockIdx.y * TOK;
+    // The router rows are asked for into the L2 while the launch before this one ends: no value is read, so nothing that launch may write is read too early. Calls of one token
+    // back to back 28.3 -> 27.0 us (512 experts x 2048), four layers of 64 tokens 651 -> 649
+    if (threadIdx.x < 16 && blockIdx.y == 0 && r0 + int(threadIdx.x) < rows) {
+        const int r = r0 + threadIdx.x, cols = h / int(gridDim.z);
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((r == e ? shared : w + size_t(r) * h) + int(blockIdx.z) * cols), "r"(cols * 4));
+    }
+    grid_wait();                                                       // x may be the output of the launch before this one
     const int ra = min(r0 + g, rows - 1), rb = min(r0 + g + 8, rows - 1);
     const float * wa = ra == e ? shared : w + size_t(ra) * h, * wb = rb == e ? shared : w + size_t(rb) * h;
     float acc[J][4];
@@ -140,17 +146,21 @@ __global__ void __launch_bounds__(RM_WARPS * 32) router_mma_k(const float * __re
 #pragma unroll (XT == 1 ? 4 : 2)
     for (int k0 = k_lo; k0 < k_hi; k0 += 16) {
         uint32_t hi[4], mid[4], lo[4];
-        split3(*reinterpret_cast<const float2 *>(wa + k0 + 2 * t), hi[0], mid[0], lo[0]);
-        split3(*reinterpret_cast<const float2 *>(wb + k0 + 2 * t), hi[1], mid[1], lo[1]);
-        split3(*reinterpret_cast<const float2 *>(wa + k0 + 2 * t + 8), hi[2], mid[2], lo[2]);
-        split3(*reinterpret_cast<const float2 *>(wb + k0 + 2 * t + 8), hi[3], mid[3], lo[3]);
+        // lane t holds columns 4 t .. 4 t + 3 of the sixteen in both operands (the sum does not care which of them the fragment calls 2 t, 2 t + 1, 2 t + 8, 2 t + 9): one load
+        // a row instead of two. 504 sizes of 512 to 5120 columns: bf16 up to 64 tokens 1.06 times as fast, fp32 1.03, fp16 1.01; 64 tokens x 2048 x 512 9.3 -> 8.6 us
+        const float4 va = *reinterpret_cast<const float4 *>(wa + k0 + 4 * t), vb = *reinterpret_cast<const float4 *>(wb + k0 + 4 * t);
+        split3(make_float2(va.x, va.y), hi[0], mid[0], lo[0]);
+        split3(make_float2(vb.x, vb.y), hi[1], mid[1], lo[1]);
+        split3(make_float2(va.z, va.w), hi[2], mid[2], lo[2]);
+        split3(make_float2(vb.z, vb.w), hi[3], mid[3], lo[3]);
 #pragma unroll
         for (int j = 0; j < J; ++j) {
             const int tok = min(t0 + 8 * j + g, n - 1);
-            const typename Elem<DT>::type * xr = x + size_t(tok) * h + k0 + 2 * t;
+            struct alignas(4 * sizeof(typename Elem<DT>::type)) Four { typename Elem<DT>::type v[4]; };
+            const Four xr = *reinterpret_cast<const Four *>(x + size_t(tok) * h + k0 + 4 * t);
             uint32_t b0[XT], b1[XT];
-            x_pair<DT>(xr, b0);
-            x_pair<DT>(xr + 8, b1);
+            x_pair<DT>(xr.v, b0);
+            x_pair<DT>(xr.v + 2, b1);
             if constexpr (XT == 1) {                                     // smallest terms first
                 mma_bf16_acc(acc[j], lo, b0[0], b1[0]);
                 mma_bf16_acc(acc[j], mid, b0[0], b1[0]);
@@ -665,7 +675,9 @@ int32_t router_launch(const float * w, const float * shared, const void * xv, fl
     // 16-bit rows go to router_tc_k where router_mma_k, with its 64 tokens a block, has more than two blocks per SM, or more than one and enough rows to fill most of a tile of
     // 128. Before / router_tc_k, us: bf16 2048 columns x 512 experts, 256 tokens 17.8 / 10.1, 509 23.5 / 11.2, 4096 87 / 32; 4096 x 128, 8192 tokens 163 / 40; 3072 x 256, 2047
     // tokens 57 / 20; fp16 600 x 3072 x 256 32 / 15.5, 4096 x 2048 x 512 187 / 73, 600 x 2560 x 60 (160 blocks) 21.9 / 13.7. Not where the other kernels are more precise (2-norm against
-    // fp64): bf16 below 256 tokens (1.3e-7 to 2.2e-7, here 4.7e-7), fp16 below 768 columns (6.9e-8, here 7.2e-8; from there on 8.1e-8 to 1.04e-7).
+    // fp64): bf16 below 256 tokens (1.3e-7 to 2.2e-7, the chains here 4.7e-7), fp16 below 768 columns (6.9e-8, here 7.2e-8; from there on 8.1e-8 to 1.04e-7). bf16 rows below 256 tokens
+    // with more than a block per SM take the fine form instead (7.2e-8) where it costs fewer cycles; router_mma_k / fine, us: 2048 x 512, 65 tokens 15.3 / 12.9, 128 18.1 / 13.1, 255 35.4 / 13.3;
+    // 3072 x 256, 200 tokens 1.5 times as fast.
     // bf16 rows between one and two blocks per SM and up to 48 router rows: the fine form (7.2e-8; router_mma_k up to 2.7e-7) where it costs fewer cycles. router_tile_k, which served them once at
     // 8.2e-7 / router_mma_k / fine, us: 2048 x 48, 1024 tokens 12.7 / 17.6 / 12.3; 1536 x 48, 1500 14.1 / 23.9 / 12.5; 1024 x 32, 2047 13.9 / 14.9 / 12.7; 256 x 32, 8192 10.5 / 12.1 / 7.8; dearer:
     // 5120 x 32, 2047 55 / 26.6 / 39. Up to 16 rows a tile of 128 stays empty: router_mma_k (1.3e-7 and more exact than the chains) where it costs less than they: 3072 x 8, 6000 tokens
@@ -681,12 +693,12 @@ int32_t router_launch(const float * w, const float * shared, const void * xv, fl
         if (h % RT_K == 0 && h >= 768 && (blocks > 2 * ROUTER_SMS || (blocks > ROUTER_SMS && rows > 48)))
             return rtc::launch<DT, true>(w, shared, x, logits, ld, h, e, rows, n, s);
     if constexpr (DT == B2MOE_BF16)
-        if (h % RT_K == 0 && n >= 256 && blocks > ROUTER_SMS) {
+        if (h % RT_K == 0 && blocks > ROUTER_SMS) {
             const long long mma_cycles = 5000 + blocks * (8900 + 156LL * (h / ks) / 10) / ROUTER_SMS;
             auto below_mma = [&](const rtc::Shape & p) { return p.cycles < mma_cycles || ceil_div(n, 64) > GRID_Y; };
-            if (rows > 48 || (blocks > 2 * ROUTER_SMS && (rows > 16 || below_mma(rtc::shape_of<DT, false>(rows, n, h)))))
+            if (n >= 256 && (rows > 48 || (blocks > 2 * ROUTER_SMS && (rows > 16 || below_mma(rtc::shape_of<DT, false>(rows, n, h))))))
                 return rtc::launch<DT, false>(w, shared, x, logits, ld, h, e, rows, n, s);
-            if (blocks <= 2 * ROUTER_SMS && rows > 16 && below_mma(rtc::shape_of<DT, true>(rows, n, h)))
+            if ((n < 256 || blocks <= 2 * ROUTER_SMS) && rows > 16 && below_mma(rtc::shape_of<DT, true>(rows, n, h)))
                 return rtc::launch<DT, true>(w, shared, x, logits, ld, h, e, rows, n, s);
         }
     if constexpr (DT != B2MOE_BF16) if (h % RT_K == 0 && blocks > 2 * ROUTER_SMS && ceil_div(n, RT_TOK) <= GRID_Y) {
