@@ -60,6 +60,11 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void * src, uint32_
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(bar) : "memory");
 }
+// the same for data that is read once (once_policy)
+__device__ __forceinline__ void bulk_g2s_once(uint32_t dst, const void * src, uint32_t bytes, uint32_t bar, uint64_t policy) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+                 ::"r"(dst), "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(bar), "l"(policy) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -423,6 +428,7 @@ __global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(c
         // ---- producer: lane w < 16 feeds consumer warp w (its ring, its barriers); lanes 16 .. 23 copy the activation rows ----
         const int w = lane & (CTA_WARPS - 1);
         const uint32_t my_full = full0 + 8 * w * MAX_STAGES, my_empty = empty0 + 8 * w * MAX_STAGES, my_ring = smem_addr(ring) + uint32_t(w) * S * SLOT;
+        [[maybe_unused]] const uint64_t policy = FEW ? 0 : once_policy();          // small launches gain nothing from it
         uint32_t slot = 0, issued = 0, xissued = 0;
         bool ok = true;
         // known = the caller has already located this pass (e_in, c0_in)
@@ -491,7 +497,8 @@ __global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(c
                             const uint8_t * src = ((NMAT == 2 && (j & 1)) ? b1 : b0) + size_t(ks) * SLOT;
                             const uint32_t bytes = uint32_t(min(SLOT_TILES, p.k_tiles - ks * SLOT_TILES)) * TILE;
                             mbar_expect_tx(my_full + 8 * slot, bytes);
-                            bulk_g2s(my_ring + slot * SLOT, src, bytes, my_full + 8 * slot);
+                            if constexpr (FEW) bulk_g2s(my_ring + slot * SLOT, src, bytes, my_full + 8 * slot);
+                            else bulk_g2s_once(my_ring + slot * SLOT, src, bytes, my_full + 8 * slot, policy);
                         }
                         ++issued;
                         slot = slot + 1 == uint32_t(S) ? 0 : slot + 1;

@@ -59,6 +59,10 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void * src, uint32_
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(bar) : "memory");
 }
+__device__ __forceinline__ void bulk_g2s_once(uint32_t dst, const void * src, uint32_t bytes, uint32_t bar, uint64_t policy) {      // data that is read once (once_policy)
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+                 ::"r"(dst), "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(bar), "l"(policy) : "memory");
+}
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile("{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
@@ -221,6 +225,7 @@ __global__ void __launch_bounds__(CTA_WARPS * 32, 1) iq3s_grouped_k(Iq3sArgs p) 
     uint32_t xissued = 0;                  // thread 0: activation stagings issued (their copies must land before the block leaves)
     if (threadIdx.x == 0 && int(blockIdx.x) < n_items) { stage_x(blockIdx.x, 0); ++xissued; }
 
+    const uint64_t policy = once_policy();
     int iter = 0;
     for (int it = blockIdx.x; it < n_items; it += gridDim.x, ++iter) {
         const int b = p.nbuf == 2 ? (iter & 1) : 0;
@@ -247,7 +252,7 @@ __global__ void __launch_bounds__(CTA_WARPS * 32, 1) iq3s_grouped_k(Iq3sArgs p) 
                 const uint32_t s = filled % STAGES;
                 const uint8_t * src = ((NMAT == 2 && (j & 1)) ? base1 : base0) + size_t(NMAT == 2 ? j >> 1 : j) * TILE;
                 mbar_expect_tx(bar0 + 8 * s, TILE);
-                bulk_g2s(ring0 + s * TILE, src, TILE, bar0 + 8 * s);
+                bulk_g2s_once(ring0 + s * TILE, src, TILE, bar0 + 8 * s, policy);
             };
             for (int j = 0; j < STAGES && j < ntiles; ++j) { if (lane == 0) issue(j); ++filled; }
             float acc[NMAT][NCH][4];
