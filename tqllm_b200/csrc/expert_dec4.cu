@@ -214,20 +214,20 @@ template <bool STAGER> constexpr int threads_of() { return (CTA_WARPS + (STAGER 
 template <bool STAGER> constexpr int bound_threads() { return STAGER ? 640 : threads_of<false>(); }
 
 // The prologue of a ROUTED block, all of its threads; returns its passes
-template <int GATING> __device__ __noinline__ void route_warp(const Dec4Route & r, int experts, int topk, int * ids, float * weights, float * shared_weights, int token, int lane) {
+template <int GATING> __device__ __noinline__ void route_warp(const Dec4Route & r, int experts, int topk, int * ids, float * weights, float * shared_weights, int token, int lane, Picked * list) {
     const float * bias = GATING == B2MOE_SOFTMAX ? nullptr : r.bias;
-    if (experts <= 128) route_token_regs<GATING, 4>(r.logits, r.ld, bias, ids, weights, shared_weights, experts, topk, r.norm, r.scale, token, lane);
-    else if (experts <= 256) route_token_regs<GATING, 8>(r.logits, r.ld, bias, ids, weights, shared_weights, experts, topk, r.norm, r.scale, token, lane);
-    else route_token_regs<GATING, 16>(r.logits, r.ld, bias, ids, weights, shared_weights, experts, topk, r.norm, r.scale, token, lane);
+    if (experts <= 128) route_token_regs<GATING, 4>(r.logits, r.ld, bias, ids, weights, shared_weights, experts, topk, r.norm, r.scale, token, lane, list);
+    else if (experts <= 256) route_token_regs<GATING, 8>(r.logits, r.ld, bias, ids, weights, shared_weights, experts, topk, r.norm, r.scale, token, lane, list);
+    else route_token_regs<GATING, 16>(r.logits, r.ld, bias, ids, weights, shared_weights, experts, topk, r.norm, r.scale, token, lane, list);
 }
-__device__ __forceinline__ int route_and_plan(const Dec4Args & p, const Dec4Route & in, Routed & r, uint8_t * rows, uint32_t xrow, int bits) {
+__device__ __forceinline__ int route_and_plan(const Dec4Args & p, const Dec4Route & in, Routed & r, Picked * list, uint8_t * rows, uint32_t xrow, int bits) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, A = p.A, e1 = p.experts + 1;
     int * counts = p.plan + PLAN_HDR, * offsets = counts + e1, * active = offsets + e1 + 1, * perm = active + e1;
     const bool lead = blockIdx.x == 0;                                 // writes what is not spread over the blocks
     if (warp < in.n) {                                                 // n <= PASS_TOKENS: warps 0 .. 7 route, 8 .. 15 stage
         float * sw = lead ? in.shared_weights : nullptr;
-        if (in.gating == B2MOE_SOFTMAX) route_warp<B2MOE_SOFTMAX>(in, p.experts, p.topk, r.ids, r.weights, sw, warp, lane);
-        else route_warp<B2MOE_SIGMOID>(in, p.experts, p.topk, r.ids, r.weights, nullptr, warp, lane);
+        if (in.gating == B2MOE_SOFTMAX) route_warp<B2MOE_SOFTMAX>(in, p.experts, p.topk, r.ids, r.weights, sw, warp, lane, list + 32 * warp);
+        else route_warp<B2MOE_SIGMOID>(in, p.experts, p.topk, r.ids, r.weights, nullptr, warp, lane, list + 32 * warp);
     } else if (warp >= PASS_TOKENS && warp < PASS_TOKENS + in.n) {
         const int row = warp - PASS_TOKENS, k = p.k_tiles * 256;
         const float inv = stage_row_lanes(in.x, in.x_dtype, size_t(row) * k, k, bits, rows + row * xrow, lane);
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(c
     const int * counts = p.plan + PLAN_HDR, * offsets = counts + e1, * active = offsets + e1 + 1, * perm = active + e1;
     __shared__ typename std::conditional<ROUTED, Routed, int>::type routed;
     int routed_passes = 0;
-    if constexpr (ROUTED) routed_passes = route_and_plan(p, route, routed, xs, xrow, F::BITS);
+    if constexpr (ROUTED) routed_passes = route_and_plan(p, route, routed, reinterpret_cast<Picked *>(ring), xs, xrow, F::BITS);      // (the rings are empty yet)
     const int * passes = ROUTED ? nullptr : perm + p.A + counts[p.experts];     // the plan's own count of always-on rows (a range of the tokens under expert parallelism)
     const int na = ROUTED ? routed_passes : p.plan[PLAN_NACTIVE], row_tiles = (p.rows + 15) >> 4;
     // the block's share of the launch: jobs [u_begin, u_end) of the pass-major list of (pass, row tile) jobs; it walks the

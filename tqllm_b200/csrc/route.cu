@@ -457,9 +457,9 @@ template <int GATING>
 __device__ __forceinline__ void route_token(const float * logits, int ld, const float * __restrict__ bias, int * __restrict__ ids,
                                             float * __restrict__ weights, float * __restrict__ shared_weights, int e, int k, int norm,
                                             float scale, int token, int lane, float * p, float * key) {
-    if (k <= 32 && e <= 128) return route_token_regs<GATING, 4>(logits, ld, bias, ids, weights, shared_weights, e, k, norm, scale, token, lane);
-    if (k <= 32 && e <= 256) return route_token_regs<GATING, 8>(logits, ld, bias, ids, weights, shared_weights, e, k, norm, scale, token, lane);
-    if (k <= 32 && e <= 512) return route_token_regs<GATING, 16>(logits, ld, bias, ids, weights, shared_weights, e, k, norm, scale, token, lane);
+    if (k <= 32 && e <= 128) return route_token_regs<GATING, 4>(logits, ld, bias, ids, weights, shared_weights, e, k, norm, scale, token, lane, reinterpret_cast<Picked *>(p));
+    if (k <= 32 && e <= 256) return route_token_regs<GATING, 8>(logits, ld, bias, ids, weights, shared_weights, e, k, norm, scale, token, lane, reinterpret_cast<Picked *>(p));
+    if (k <= 32 && e <= 512) return route_token_regs<GATING, 16>(logits, ld, bias, ids, weights, shared_weights, e, k, norm, scale, token, lane, reinterpret_cast<Picked *>(p));
     const float * x = logits + size_t(token) * ld;
     if (GATING == B2MOE_SOFTMAX) {
         float m = -CUDART_INF_F;
@@ -510,7 +510,7 @@ __device__ __forceinline__ void route_token(const float * logits, int ld, const 
 template <int GATING>
 __global__ void route_k(const float * logits, int ld, const float * __restrict__ bias, int * __restrict__ ids,
                         float * __restrict__ weights, float * __restrict__ shared_weights, int e, int k, int norm, float scale, int n) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int token = blockIdx.x * warps + warp;
     grid_release();
@@ -525,7 +525,7 @@ __global__ void route_k(const float * logits, int ld, const float * __restrict__
 struct RouteSet { const float * logits; int * ids; float * weights; float * shared_weights; };
 template <int GATING>
 __global__ void route2_k(const RouteSet a, const RouteSet b, int ld, const float * __restrict__ bias, int e, int k, int norm, float scale, int n) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int token = blockIdx.x * warps + warp;
     const RouteSet & t = blockIdx.y ? b : a;
@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(RD_THREADS) route_dispatch_k(const float * log
                                                          int * __restrict__ ids, float * __restrict__ weights,
                                                          float * __restrict__ shared_weights, int e, int k, int norm, float scale, int n,
                                                          int shared_first, int shared_count, int * __restrict__ plan) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float * p = smem + size_t(warp) * 2 * e;
     grid_release();
@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(RD_THREADS) route_cluster_k(const float * logi
                                                         int * __restrict__ ids, float * __restrict__ weights,
                                                         float * __restrict__ shared_weights, int e, int k, int norm, float scale, int n,
                                                         int shared_first, int shared_count, int * __restrict__ plan, const StageJob st) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
