@@ -293,6 +293,40 @@ __global__ void exact_rows_k(const typename Elem<DT>::type * x, const int * plan
     if (lane == 0) inv_scale[slot] = inv;
 }
 
+// The experts that have tokens, in order, and the items before each, into info (then the number of items): from the counts themselves, one scan by all threads of the block; returns how many.
+// By way of the plan's list of them (three dependent loads), scanned by one warp, a block asked for its first chunk 2.1 us after it had begun with 75 experts, 4.7 us with 513; now 1.6 and 1.7. A function
+// of its own: in the kernel it cost the decoders registers (IQ4, 24 tokens 261 -> 274 us). The caller synchronises after it.
+__device__ __noinline__ int find_experts(const int * counts, int e1, int row_blocks, int cap_log2, Info * info, int2 * sums) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, threads = blockDim.x, * offsets = counts + e1;
+    int na = 0, items = 0;
+#pragma unroll 1
+    for (int base = 0; base < e1; base += threads) {
+        const int e = base + int(threadIdx.x), cnt = e < e1 ? counts[e] : 0, off = e < e1 ? offsets[e] : 0, mine = ((cnt + (1 << cap_log2) - 1) >> cap_log2) * row_blocks;
+        int a = cnt > 0, v = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int oa = __shfl_up_sync(0xffffffffu, a, d), ov = __shfl_up_sync(0xffffffffu, v, d);
+            if (lane >= d) { a += oa; v += ov; }
+        }
+        if (base > 0) __syncthreads();                                 // the sums of the round before are read
+        if (lane == 31) sums[warp] = make_int2(a, v);
+        __syncthreads();
+        const int2 own = lane < threads / 32 ? sums[lane] : make_int2(0, 0);
+        int2 w = own;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int oa = __shfl_up_sync(0xffffffffu, w.x, d), ov = __shfl_up_sync(0xffffffffu, w.y, d);
+            if (lane >= d) { w.x += oa; w.y += ov; }
+        }
+        const int wa = __shfl_sync(0xffffffffu, w.x - own.x, warp), wv = __shfl_sync(0xffffffffu, w.y - own.y, warp);
+        if (cnt > 0) info[na + wa + a - 1] = Info{items + wv + v - mine, e, cnt, off};
+        na += __shfl_sync(0xffffffffu, w.x, 31);
+        items += __shfl_sync(0xffffffffu, w.y, 31);
+    }
+    if (threadIdx.x == 0) info[na].cum = items;
+    return na;
+}
+
 // MODE 0: act[a][r] = silu(gate_r . x_tok(a)) * (up_r . x_tok(a));  MODE 1: y[a][r] = down_r . act[a]
 // TERMS > 0: the exact form: no rounding but that of the activations to TERMS fp16 terms (16-bit ones: none above 2^-29 of the row's largest) and of the fp32 sums
 // F32_OUT: an instance for fp32 results and one for 16-bit ones, chosen by the call's output type. A branch at the stores, or two
@@ -340,60 +374,43 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
     // c3 decode 8 73.0 -> 66.9 us, c5 decode 24 308 -> 292 (309 with the issuing branch taken by one lane), c2 509 tokens 351 -> 323, c4 600 745 -> 685
     const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0);
     const int e1 = p.experts + 1;
-    const int * counts = p.plan + PLAN_HDR, * offsets = counts + e1, * active = offsets + e1 + 1, * perm = active + e1;
+    const int * counts = p.plan + PLAN_HDR, * offsets = counts + e1, * perm = offsets + e1 + 1 + e1;
     const int row_tiles = (p.rows + 15) >> 4, row_blocks = (row_tiles + ITEM_TILES - 1) / ITEM_TILES;
     const int ksteps = p.k / G_KS, nchunks = (ksteps + 3) >> 2;             // a last chunk may lack steps: they bring no products, but their barriers turn
 
-    D::init(dec_tab, threadIdx.x, G_THREADS);
-    if (threadIdx.x == 0) {
-#pragma unroll 1
-        for (int i = 0; i < RAW_SLOTS; ++i) { bar_init(raw_full + 8 * i, 1); bar_init(raw_full + 8 * (RAW_SLOTS + i), 1); bar_init(raw_empty + 8 * i, DEC_WARPS / 2); }
-#pragma unroll 1
-        for (int i = 0; i < A_STAGES; ++i) bar_init(a_full + 8 * i, p.b_pair ? 8 + (GATHER ? LOAD_WARPS : 1) : 8);
-#pragma unroll 1
-        for (int i = 0; i < STEP_RING; ++i) bar_init(done + 8 * i, 1);
-#pragma unroll 1
-        for (int i = 0; i < MAX_B_STAGES; ++i) bar_init(b_full + 8 * i, EXACT ? 8 : GATHER ? LOAD_WARPS : 1);
-        for (int i = 0; i < 2; ++i) { bar_init(acc_full + 8 * i, EXACT ? EPI_WARPS : NARROW ? 2 : 1); bar_init(acc_empty + 8 * i, EPI_WARPS); }
-        bar_init(drain, 1);
-        bar_init(tok_bar, EPI_WARPS);
-#pragma unroll 1
-        for (int i = 0; EXACT && i < 4; ++i) bar_init(set_full + 8 * i, 1);
-        *abort_flag = 0;
+    // A thread per barrier; two threads that know the tensor maps will be needed
+    if (threadIdx.x < N_BARS) {
+        const int i = threadIdx.x;
+        int at = 2 * RAW_SLOTS, count = 1;                             // raw_full; then the others in their order
+        auto next = [&](int n, int c) { if (i >= at) count = c; at += n; };
+        next(RAW_SLOTS, DEC_WARPS / 2);
+        next(A_STAGES, p.b_pair ? 8 + (GATHER ? LOAD_WARPS : 1) : 8);
+        next(STEP_RING, 1);
+        next(MAX_B_STAGES, EXACT ? 8 : GATHER ? LOAD_WARPS : 1);
+        next(2, EXACT ? EPI_WARPS : NARROW ? 2 : 1);
+        next(2, EPI_WARPS);
+        next(1, 1);
+        next(1, EPI_WARPS);
+        next(4, 1);
+        bar_init(saddr(bars) + 8 * i, count);
         bar_init_fence();
     }
+    if (threadIdx.x == 64) *abort_flag = 0;
+    if (warp == RAW_WARP && lane < (MODE == 0 ? 2 : 1)) prefetch_map(maps.w + lane);
+    if (warp == LOAD_WARP0 && lane == 0) prefetch_map(maps.x);
     if (warp == MMA_WARP) tmem_alloc(saddr(tmem_slot), 512);
     // The launch before this one converts the activation rows, and began to let this one in when the plan was complete (rows_begin): only the rows are awaited
-    // (grid_wait), by the warps that read them. The plan is looked through, and the first chunks are brought and decoded, meanwhile
-    const int na = p.plan[PLAN_NACTIVE];
-#pragma unroll 1
-    for (int i = threadIdx.x; i < na; i += G_THREADS) {
-        const int e = active[i];
-        info[i] = Info{0, e, counts[e], offsets[e]};
-    }
+    // (grid_wait), by the warps that read them. The plan is looked through, and the first chunks are brought and decoded, meanwhile.
+    auto tiles_of = [&](int cnt) { return (cnt + p.cap - 1) >> p.cap_log2; };      // an expert's tokens are spread evenly over the fewest tiles of at most `cap`
+    D::init(dec_tab, threadIdx.x, G_THREADS);
+    const int na = __shfl_sync(0xffffffffu, find_experts(counts, e1, row_blocks, p.cap_log2, info, tok), 0);    // (the table's first use comes later)
     fence_before();
     __syncthreads();
     fence_after();
-    // an expert's tokens are spread evenly over the fewest tiles of at most `cap`
-    auto tiles_of = [&](int cnt) { return (cnt + p.cap - 1) >> p.cap_log2; };
-    if (warp == 0) {                                                  // items before active expert i
-        int carry = 0;
-#pragma unroll 1
-        for (int base = 0; base < na; base += 32) {
-            const int i = base + lane;
-            const int mine = i < na ? tiles_of(info[i].cnt) * row_blocks : 0;
-            int v = mine;
-            for (int d = 1; d < 32; d <<= 1) { const int o = __shfl_up_sync(0xffffffffu, v, d); if (lane >= d) v += o; }
-            if (i < na) info[i].cum = carry + v - mine;
-            carry += __shfl_sync(0xffffffffu, v, 31);
-        }
-        if (lane == 0) info[na].cum = carry;
-    }
-    __syncthreads();
     // All 512 columns are this block's, so they begin at column 0 of lane 0. As a constant the base saves the issuing thread an addition and
     // a move into the uniform registers per product: c5 decode 24 gate/up 196.6 -> 194.5 us, down 119 -> 115
     constexpr uint32_t tmem = 0;
-    const int n_items = info[na].cum;
+    const int n_items = __shfl_sync(0xffffffffu, info[na].cum, 0);
 
     // item -> expert, first token slot, token count, row block; called by whole warps, with `at` = the active expert of the
     // warp's previous item (items only grow: usually one round of 32 probes)

@@ -66,6 +66,8 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void * map, int 
     asm volatile("cp.async.bulk.tensor.4d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
                  ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar) : "memory");
 }
+// a tensor map that copies will need soon
+__device__ __forceinline__ void prefetch_map(const void * map) { asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory"); }
 // one lane of a converged warp, the same every time
 __device__ __forceinline__ bool elect_one() {
     uint32_t ok;
