@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(THREADS, 1) router_tc_k(const float * w, const
                    acc_empty = acc_full + 16, drain = acc_empty + 16;
     uint32_t * tmem_slot = reinterpret_cast<uint32_t *>(gate + S * STEP) + 2 * N_BARS;
     volatile int * gave_up = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);      // uniform: as in gemm_tc_k
     const int r0 = blockIdx.y * ROWS, t0 = blockIdx.x * NT;                  // tokens on gridDim.x: any batch size
     const bool has_gate = rows > e && r0 + ROWS > e;                    // the tile holds row e
 
