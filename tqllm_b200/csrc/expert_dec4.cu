@@ -300,7 +300,7 @@ template <uint32_t T, int MODE, bool FEW, bool ROUTED = false>
 __global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(const Dec4Args p, const typename std::conditional<ROUTED, Dec4Route, NoRoute>::type route) {
     static_assert(!ROUTED || (FEW && MODE == 0));
     constexpr bool STAGER = FEW && MODE == 1;
-    using Job = typename std::conditional<FEW, int, long long>::type;
+    using Job = uint32_t;            // (a pass stands for up to eight of the output's rows: a GPU's memory holds fewer than 2^32 jobs)
     using F = D4<T>;
     constexpr int NMAT = MODE == 0 ? 2 : 1, TILE = F::TILE;
     // how the byte sums of a four-token pass meet: two shuffles and half of the fp32 steps, or four shuffles and no selects.
@@ -354,16 +354,14 @@ __global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(c
     // share as segments = runs of row tiles [r0, r1) of one pass
     const int n_pass = ROUTED ? routed_passes : p.plan[PLAN_NPASS];
     const Job n_jobs = Job(n_pass) * row_tiles;
-    Job u_begin, u_end;
+    // n_jobs b / blocks = q b + r b / blocks with n_jobs = q blocks + r: 32-bit divisions (64-bit ones in the large launches: own Q4_K, 77 tokens 97.2 -> 99.1 us)
+    const uint32_t blocks = gridDim.x, q = n_jobs / blocks, r = n_jobs - q * blocks;
+    Job u_begin = q * blockIdx.x + r * blockIdx.x / blocks, u_end = q * (blockIdx.x + 1) + r * (blockIdx.x + 1) / blocks;
     if constexpr (FEW) {
-        // n_jobs b / blocks = q b + r b / blocks with n_jobs = q blocks + r: 32-bit divisions
-        const int blocks = int(gridDim.x), q = n_jobs / blocks, r = n_jobs - q * blocks;
-        u_begin = q * int(blockIdx.x) + r * int(blockIdx.x) / blocks;
-        u_end = q * int(blockIdx.x + 1) + r * int(blockIdx.x + 1) / blocks;
         // Few passes: every pass on blocks of its own, where a block's share is then still one round of JW jobs. A share that runs into a
         // second pass waits for that one's plan entries, activation rows and products in turn: one token of 512 IQ3_S experts, gate/up: done after 9.2 us, blocks with one
         // pass after 6.6. Larger shares hide that behind their rounds, and whole passes leave them uneven (8 tokens, 75 passes: 73.5 us a layer with equal shares, 80).
-        const int per_pass = blocks / max(n_pass, 1);
+        const int per_pass = int(blocks) / max(n_pass, 1);
         if (per_pass > 0 && (row_tiles + per_pass - 1) / per_pass <= JW) {
             const int pass = int(blockIdx.x) / per_pass, part = int(blockIdx.x) - pass * per_pass;
             u_begin = u_end = 0;
@@ -372,14 +370,11 @@ __global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(c
                 u_end = pass * row_tiles + row_tiles * (part + 1) / per_pass;
             }
         }
-    } else {
-        u_begin = n_jobs * blockIdx.x / gridDim.x;
-        u_end = n_jobs * (blockIdx.x + 1) / gridDim.x;
     }
     auto segment = [&](Job u, int & pass, int & r0, int & r1) {
-        pass = int(u / row_tiles);
-        r0 = int(u - Job(pass) * row_tiles);
-        r1 = int(min(Job(row_tiles), r0 + (u_end - u)));
+        pass = int(u / uint32_t(row_tiles));
+        r0 = int(u) - pass * row_tiles;
+        r1 = int(min(uint32_t(row_tiles), r0 + (u_end - u)));
     };
 
     // pass w -> (expert, first token slot); the pass list runs over the active experts from the last to the first. Called by
@@ -540,8 +535,8 @@ __global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(c
     } else if (STAGER && warp == CTA_WARPS + 1) {
         {
         // ---- stager (down product): segment q's activation rows, fp32 in global memory -> staged form in buffer q % nbuf ----
-        const int pass_first = u_begin < u_end ? int(u_begin / row_tiles) : 0;
-        const int nseg = u_begin < u_end ? int((u_end - 1) / row_tiles) - pass_first + 1 : 0;
+        const int pass_first = u_begin < u_end ? int(u_begin / uint32_t(row_tiles)) : 0;
+        const int nseg = u_begin < u_end ? int((u_end - 1) / uint32_t(row_tiles)) - pass_first + 1 : 0;
         bool ok = true;
         if (early) grid_wait();
 #pragma unroll 1
