@@ -33,7 +33,7 @@
 // status word, and the block drains and leaves.
 // The exact form (TERMS > 0; Q4_K and IQ3_S codes, where the decode kernels' precision is asked for and their eight tokens a pass are too few): A
 // holds the integers sc q or (1 + 2 s)(2 n - 15), B the activations in one or two fp16 terms, every 256-column chunk has accumulators of
-// its own (two sets in turn), and the epilogue warps scale a chunk's sums by the rows' d in fp32 while the next one is multiplied. The mins of Q4_K
+// its own (sets in turn), and the epilogue warps scale a chunk's sums by the rows' d in fp32 while the next one is multiplied. The mins of Q4_K
 // meet the sub-block sums of the activations in one more product a chunk. Items have up to 32 tokens. Decoding costs two instructions
 // less a pair of weights than with the scales in the operand, reading the sums back about 150 a scheduler and chunk.
 //
