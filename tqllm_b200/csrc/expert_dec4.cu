@@ -228,6 +228,7 @@ __device__ __forceinline__ int route_and_plan(const Dec4Args & p, const Dec4Rout
         float * sw = lead ? in.shared_weights : nullptr;
         if (in.gating == B2MOE_SOFTMAX) route_warp<B2MOE_SOFTMAX>(in, p.experts, p.topk, r.ids, r.weights, sw, warp, lane, list + 32 * warp);
         else route_warp<B2MOE_SIGMOID>(in, p.experts, p.topk, r.ids, r.weights, nullptr, warp, lane, list + 32 * warp);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the list lies in the rings: its stores come before the copies into them
     } else if (warp >= PASS_TOKENS && warp < PASS_TOKENS + in.n) {
         const int row = warp - PASS_TOKENS, k = p.k_tiles * 256;
         const float inv = stage_row_lanes(in.x, in.x_dtype, size_t(row) * k, k, bits, rows + row * xrow, lane);
