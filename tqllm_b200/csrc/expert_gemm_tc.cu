@@ -21,7 +21,8 @@
 //   overlaps the products of the next; a wider item takes both. An item of up to 64 tokens splits its K over the two halves of
 //   its accumulator (products in turn), and the epilogue adds them: half as long a chain of truncated sums (NVFP4 gate/up, relative error against
 //   64 bits 3.7e-7 and 8.3e-7 in one chain); the products' pace is the same either way. In launches of narrow items (by_chunk) the halves take an even
-//   number of chunks in turn, and an item of up to 32 tokens has a quarter each for their even and odd products (NVFP4, K = 2048: 1.9e-7 in halves, 1.1e-7 in quarters).
+//   number of chunks in turn, and an item of up to 32 tokens has a quarter each for their even and odd products (NVFP4, K = 2048: 1.9e-7 in halves, 1.1e-7 in quarters); a wider one too, of both accumulators,
+//   where a last chunk that is not full would leave the halves uneven.
 // The control warps share their schedulers with six others, so what they execute per unit bounds the block: they walk uniform
 // loops, one elected lane issues, and the raw blocks and rows come in the largest boxes that fit. They are the first warps of the
 // block: as the last ones they were served last (c3 decode gate/up 110 us, as the first 78).
@@ -86,6 +87,10 @@ struct GemmArgs {
     int rows, k, experts, topk, A;
     int cap, cap_log2, b_stages, raw_slots; // most tokens of an item; B stages; raw chunks in the ring
     int by_chunk;                           // items of up to SPLIT_COLS tokens split their K by chunks (and products), not by products: cap <= 64, an even number of chunks
+    // by_chunk: an item of more tokens than this takes both accumulators, a quarter of 64 columns for each of its four sums. Rows that end inside a chunk: 32, as halves of whole chunks are uneven
+    // there (K = 384: 16 and 8 products), a longer chain of truncated sums than products in turn give. Relative error against 64 bits, 50 tokens, products in turn / halves of chunks / quarters: K = 384
+    // 6.90e-8 / 7.14e-8 / 6.37e-8, 896 1.03e-7 / 1.04e-7 / 7.9e-8, 1408 1.40e-7 / 1.41e-7 / 9.4e-8. Else 64: no item
+    int both_above;
     int b_pair;                             // 1: the B stages are filled and freed a unit at a time, beside the A stage of the unit and through its barriers (b_stages = 2 A_STAGES)
 };
 // The rows' boxes: sixteen rows and multiples of them, as many as the products take (32 in launches of items of up to 256 tokens). With boxes in quarters of
@@ -440,6 +445,8 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
     // the smallest box that holds the item's tokens
     auto b_class = [&](int nv) { return max(nv - 1, 0) >> (EXACT ? 4 : box_log2(p.cap)); };
     const int class_rows = EXACT ? 16 : 1 << box_log2(p.cap);
+    // an item that takes both accumulators
+    auto takes_both = [&](int nv) { return NARROW || (GATHER && p.by_chunk) ? nv > p.both_above : nv > ACC_COLS; };
     auto give_up = [&]() { *abort_flag = 1; atomicExch(p.plan + PLAN_STATUS, 2); };
     int at = 0;
 
@@ -474,8 +481,9 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
         if (int(blockIdx.x) < n_items) { im = locate(blockIdx.x, at); fetch(im); ok = put(0); }
 #pragma unroll 1
         for (int it = blockIdx.x; it < n_items && ok && !*abort_flag; it += gridDim.x, ++ic, im = after) {
-            const bool wide = im.nv > ACC_COLS;
-            const int parts = im.nv > SPLIT_COLS ? 1 : (NARROW || (GATHER && p.by_chunk)) && im.nv <= QUARTER_COLS ? 4 : 2;      // sums that an item's K is split into
+            const bool wide = takes_both(im.nv);
+            // sums that an item's K is split into, and the columns from one to the next
+            const int parts = !NARROW && im.nv > SPLIT_COLS ? 1 : (NARROW || (GATHER && p.by_chunk)) && (wide || im.nv <= QUARTER_COLS) ? 4 : 2, part_cols = wide || parts == 2 ? SPLIT_COLS : QUARTER_COLS;
             const uint32_t h = wide ? 0 : next;
             next = wide ? 0 : next ^ 1u;
             if (it + int(gridDim.x) < n_items) { after = locate(it + gridDim.x, at); fetch(after); }
@@ -568,7 +576,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                     for (int i = 0; i < 2; ++i) {
                         uint32_t w[4][8];
 #pragma unroll
-                        for (int q4 = 0; q4 < 4; ++q4) tmem_ld8(taddr + q4 * QUARTER_COLS + c + 8 * i, w[q4]);
+                        for (int q4 = 0; q4 < 4; ++q4) tmem_ld8(taddr + q4 * part_cols + c + 8 * i, w[q4]);
                         tmem_ld_wait();
 #pragma unroll
                         for (int j = 0; j < 8; ++j)
@@ -733,7 +741,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
 #pragma unroll 1
         for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x) {
             const Item im = locate(it, at);
-            const bool wide = im.nv > ACC_COLS;
+            const bool wide = takes_both(im.nv);
             const uint32_t h = wide ? 0 : next;
             next = wide ? 0 : next ^ 1u;
             const uint32_t npad = uint32_t(max(im.nv, 1) + 15) & ~15u, id = idesc(128, npad * PLANES, 0), d = tmem + h * ACC_COLS;
@@ -747,7 +755,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
             // this issuer's chunks of the item
             auto chunks = [&](auto ME) {
                 constexpr uint32_t s0 = 2 * decltype(ME)::value;
-                const uint32_t c0 = gu >> 1, d0 = d + decltype(ME)::value * SPLIT_COLS, d1 = im.nv <= QUARTER_COLS ? d0 + QUARTER_COLS : d0;
+                const uint32_t c0 = gu >> 1, part_cols = wide ? SPLIT_COLS : QUARTER_COLS, d0 = d + decltype(ME)::value * 2 * part_cols, d1 = wide || im.nv <= QUARTER_COLS ? d0 + part_cols : d0;
                 uint32_t acc = 0;
 #pragma unroll 1
                 for (uint32_t c = c0 + ((c0 ^ decltype(ME)::value) & 1u); c < c0 + uint32_t(nchunks); c += 2) {
@@ -780,7 +788,8 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
             };
             auto products = [&](auto PAIR) {
                 const bool by_chunk = GATHER && p.by_chunk && im.nv <= SPLIT_COLS;      // (rows in slot order: chunks())
-                const uint32_t second = im.nv > SPLIT_COLS ? 0 : !by_chunk ? SPLIT_COLS : im.nv <= QUARTER_COLS ? QUARTER_COLS : 0;      // columns from the accumulator of even products to that of odd ones
+                const uint32_t half = wide ? ACC_COLS : SPLIT_COLS;      // by_chunk: columns from the sums of one group's chunks to those of the other's
+                const uint32_t second = im.nv > SPLIT_COLS ? 0 : !by_chunk || wide ? SPLIT_COLS : im.nv <= QUARTER_COLS ? QUARTER_COLS : 0;      // columns from the accumulator of even products to that of odd ones
                 const uint32_t b_half = PAIR && !GATHER ? b_unit : b_step;
                 uint32_t first = gu % A_STAGES, turn = gu / A_STAGES;
                 int left = ksteps, units = 2 * nchunks;
@@ -807,7 +816,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                             continue;
                         }
                         fence_after();
-                        const uint32_t dh = by_chunk ? d + (s >> 1) * SPLIT_COLS : d;
+                        const uint32_t dh = by_chunk ? d + (s >> 1) * half : d;
                         const uint32_t acc = left != ksteps && !(by_chunk && left == ksteps - 4);      // the first unit of an item, or of either half, overwrites
                         if (left > 0) mma_step(lead, dh, dh + second, a, b, id, acc, acc | (second == 0));
                         if constexpr (!PAIR) {
@@ -955,6 +964,7 @@ template <uint32_t T> bool gemm_fit(int experts, int cap_wanted, GemmArgs & a) {
                 a.cap = o[0]; a.cap_log2 = o[0] == 256 ? 8 : o[0] == 128 ? 7 : 6; a.b_stages = o[1]; a.raw_slots = s;
                 a.b_pair = o[1] == 2 * A_STAGES;
                 a.by_chunk = a.cap <= SPLIT_COLS && ceil_div(a.k, 256) % 2 == 0;
+                a.both_above = a.k % 256 ? QUARTER_COLS : SPLIT_COLS;
                 return true;
             }
     }
