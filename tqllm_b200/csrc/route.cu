@@ -677,11 +677,14 @@ int32_t router_launch(const float * w, const float * shared, const void * xv, fl
     // tokens 57 / 20; fp16 600 x 3072 x 256 32 / 15.5, 4096 x 2048 x 512 187 / 73, 600 x 2560 x 60 (160 blocks) 21.9 / 13.7. Not where the other kernels are more precise (2-norm against
     // fp64): bf16 below 256 tokens (1.3e-7 to 2.2e-7, the chains here 4.7e-7), fp16 below 768 columns (6.9e-8, here 7.2e-8; from there on 8.1e-8 to 1.04e-7). bf16 rows below 256 tokens
     // with more than a block per SM take the fine form instead (7.2e-8) where it costs fewer cycles; router_mma_k / fine, us: 2048 x 512, 65 tokens 15.3 / 12.9, 128 18.1 / 13.1, 255 35.4 / 13.3;
-    // 3072 x 256, 200 tokens 1.5 times as fast.
+    // 3072 x 256, 200 tokens 1.5 times as fast; 2048 x 1024, 1 token 7.0 / 13.0, 16 8.0 / 14.4, 32 13.6 / 14.3, 64 18.1 / 14.8; 2048 x 4000, 1 token 20.6 / 13.9. What router_mma_k costs there is the cost of the instance that
+    // it would launch: with the 64-token one's for every batch 232 sizes of up to 64 tokens took 1.23 times the better kernel's time on average, 2.25 at most; now 1276 sizes take 1.002 and 1.20 (352 of 65 to 255 tokens: 1.0025, 1.17).
     // bf16 rows between one and two blocks per SM and up to 48 router rows: the fine form (7.2e-8; router_mma_k up to 2.7e-7) where it costs fewer cycles. router_tile_k, which served them once at
     // 8.2e-7 / router_mma_k / fine, us: 2048 x 48, 1024 tokens 12.7 / 17.6 / 12.3; 1536 x 48, 1500 14.1 / 23.9 / 12.5; 1024 x 32, 2047 13.9 / 14.9 / 12.7; 256 x 32, 8192 10.5 / 12.1 / 7.8; dearer:
     // 5120 x 32, 2047 55 / 26.6 / 39. Up to 16 rows a tile of 128 stays empty: router_mma_k (1.3e-7 and more exact than the chains) where it costs less than they: 3072 x 8, 6000 tokens
-    // 29 / 37, 5120 x 8, 4096 (256 blocks) 25 / 36, but 2048 x 16, 8192 35 / 19. Cycles of router_mma_k: fitted to 300 sizes of 256 to 5120 columns, to 10 % (2-norm).
+    // 29 / 37, 5120 x 8, 4096 (256 blocks) 25 / 36, but 2048 x 16, 8192 35 / 19. Cycles of router_mma_k: of 64 tokens a block as fitted to 300 sizes of 256 to 5120 columns
+    // when a lane loaded two columns (0.99 of 720 sizes' times since, 15 % spread), of fewer fitted to 957 sizes of 600 and more rows, on
+    // the scale of the fine form's cycles (1400 to 1500 a microsecond).
     // fp16 rows stay here with few rows too, as it is the most exact (8 rows x 3072, 8192 tokens: 70 us, router_mma_k 45 at 8.9e-8; router_tile_k 93 at 9.7e-8).
     // Rows of fp32, and short ones of fp16: tiles once router_mma_k has more than two blocks per SM. router_mma_k / tiles, us: 1024 columns x 32 experts, fp16,
     // 600 tokens 8.9 / 17.7, 2047 (256 blocks) 16.8 / 18.0, 4096 (512 blocks) 32 / 18; 2560 x 60, 600 tokens (160) 22.8 / 31, 2047 (512) 46 / 32;
@@ -689,12 +692,17 @@ int32_t router_launch(const float * w, const float * shared, const void * xv, fl
     // A grid holds 65,535 blocks of tokens; what is more than that many takes the scalar loop, as everything else that does not fit.
     constexpr int GRID_Y = 65535;
     const long long blocks = mma_blocks(64);
+    // the fewest tokens a block of router_mma_k that leave at most a block per SM: with 64, 64 tokens of 768 columns x 64 experts were 8 blocks
+    auto fits = [&](int tokens) { return n <= tokens || mma_blocks(tokens) <= ROUTER_SMS; };
+    const int mma_tokens = fits(8) ? 8 : fits(16) ? 16 : fits(32) ? 32 : 64;
     if constexpr (DT == B2MOE_F16)
         if (h % RT_K == 0 && h >= 768 && (blocks > 2 * ROUTER_SMS || (blocks > ROUTER_SMS && rows > 48)))
             return rtc::launch<DT, true>(w, shared, x, logits, ld, h, e, rows, n, s);
     if constexpr (DT == B2MOE_BF16)
         if (h % RT_K == 0 && blocks > ROUTER_SMS) {
-            const long long mma_cycles = 5000 + blocks * (8900 + 156LL * (h / ks) / 10) / ROUTER_SMS;
+            struct Cost { int launch, block, ten_columns; };
+            const Cost c = mma_tokens <= 16 ? Cost{3000, 3500, 27} : mma_tokens == 32 ? Cost{6700, 5500, 54} : Cost{5000, 8900, 156};
+            const long long mma_cycles = c.launch + mma_blocks(mma_tokens) * (c.block + (long long)c.ten_columns * (h / ks) / 10) / ROUTER_SMS;
             auto below_mma = [&](const rtc::Shape & p) { return p.cycles < mma_cycles || ceil_div(n, 64) > GRID_Y; };
             if (n >= 256 && (rows > 48 || (blocks > 2 * ROUTER_SMS && (rows > 16 || below_mma(rtc::shape_of<DT, false>(rows, n, h))))))
                 return rtc::launch<DT, false>(w, shared, x, logits, ld, h, e, rows, n, s);
@@ -717,9 +725,7 @@ int32_t router_launch(const float * w, const float * shared, const void * xv, fl
         auto launch = [&](auto kernel, int tokens) {
             return launch_cluster_z(kernel, dim3(ceil_div(rows, 16), ceil_div(n, tokens), ks), RM_WARPS * 32, 0, s, w, shared, x, logits, ld, h, e, rows, n, clear);
         };
-        // the fewest tokens a block that leave at most a block per SM: with 64, 64 tokens of 768 columns x 64 experts were 8 blocks
-        auto fits = [&](int tokens) { return n <= tokens || mma_blocks(tokens) <= ROUTER_SMS; };
-        return fits(8) ? launch(router_mma_k<DT, 1>, 8) : fits(16) ? launch(router_mma_k<DT, 2>, 16) : fits(32) ? launch(router_mma_k<DT, 4>, 32) : launch(router_mma_k<DT, 8>, 64);
+        return mma_tokens == 8 ? launch(router_mma_k<DT, 1>, 8) : mma_tokens == 16 ? launch(router_mma_k<DT, 2>, 16) : mma_tokens == 32 ? launch(router_mma_k<DT, 4>, 32) : launch(router_mma_k<DT, 8>, 64);
     }
     router_k<DT><<<dim3(ceil_div(rows, 8), std::min(ceil_div(n, ROUTER_TOK), 64)), 256, 0, s>>>(w, shared, x, logits, ld, h, e, rows, n);
     return launch_status();
