@@ -14,6 +14,16 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (run on the B200 box with -m gpu)")
 
 
+@pytest.fixture(scope="session", autouse=True)
+def current_test_kernels():
+    """Test kernels include the package's headers: one that was built before a header changed would test what the header was."""
+    import __graft_entry__ as entry
+    from tqllm_b200 import build
+    for name in entry.TEST_KERNELS:
+        if os.path.isfile(entry.kernel_path(name)) and not entry.kernel_is_current(name) and os.access(build.NVCC, os.X_OK):
+            entry.build_test_kernel(name)
+
+
 @pytest.fixture(scope="session")
 def orc():
     import oracle
