@@ -15,8 +15,11 @@ __device__ __forceinline__ uint32_t ordered_bits(float v) {          // monotoni
     const uint32_t u = __float_as_uint(v);
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
-// a / b with r = 1 / b, both rounded to nearest: the quotient's residual is exact and corrects it to the correctly rounded one (P. Markstein, Computation of elementary functions on the IBM RISC
-// System/6000 processor, 1990), unless all of b's mantissa bits are set or the residual underflows. Sixteen of them side by side take what one division with its special cases takes.
+// a / b to the bit with r = 1 / b rounded to nearest, where not all of b's mantissa bits are set and no residual underflows. Sixteen of them side by side take what one division with its special cases takes.
+// Mantissas in [1, 2), u = 2^-24. A first quotient within one ulp has a residual of at most 24 bits: it is exact, and corrects the quotient to the correctly rounded one (P. Markstein, Computation of
+// elementary functions on the IBM RISC System/6000 processor, 1990). The first quotient can be further off where a < b: by 1/2 ulp for its own rounding and a / 2 for r's; with a <= b - 2u <= 2 - 6u that
+// is at most 1.5 - 3u. Its residual takes 25 bits, whose rounding moves the corrected value by at most 1 / b's mantissa as a whole number (u to 2u) ulp, r's error by 1.5u: to be rounded the wrong way, a / b would have to lie
+// that near to the middle between two floats. Such an a / b, more than one ulp from the first quotient, is 1.5 ulp away but for as much, which takes a and b next to 2, where the two add up to less than 3u: it cannot be.
 __device__ __forceinline__ float quotient(float a, float b, float r) {
     const float q = a * r;
     return fmaf(fmaf(-q, b, a), r, q);
