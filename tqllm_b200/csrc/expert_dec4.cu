@@ -60,8 +60,8 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void * src, uint32_
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(bar) : "memory");
 }
-// the same for data that is read once (once_policy)
-__device__ __forceinline__ void bulk_g2s_once(uint32_t dst, const void * src, uint32_t bytes, uint32_t bar, uint64_t policy) {
+// the same with a policy (first_out_policy)
+__device__ __forceinline__ void bulk_g2s_first_out(uint32_t dst, const void * src, uint32_t bytes, uint32_t bar, uint64_t policy) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
                  ::"r"(dst), "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(bar), "l"(policy) : "memory");
 }
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(c
         // ---- producer: lane w < 16 feeds consumer warp w (its ring, its barriers); lanes 16 .. 23 copy the activation rows ----
         const int w = lane & (CTA_WARPS - 1);
         const uint32_t my_full = full0 + 8 * w * MAX_STAGES, my_empty = empty0 + 8 * w * MAX_STAGES, my_ring = smem_addr(ring) + uint32_t(w) * S * SLOT;
-        [[maybe_unused]] const uint64_t policy = FEW ? 0 : once_policy();          // small launches gain nothing from it
+        [[maybe_unused]] const uint64_t policy = FEW ? 0 : first_out_policy();          // small launches gain nothing from it
         uint32_t slot = 0, issued = 0, xissued = 0;
         bool ok = true;
         // known = the caller has already located this pass (e_in, c0_in)
@@ -494,7 +494,7 @@ __global__ void __launch_bounds__(bound_threads<FEW && MODE == 1>(), 1) dec4_k(c
                             const uint32_t bytes = uint32_t(min(SLOT_TILES, p.k_tiles - ks * SLOT_TILES)) * TILE;
                             mbar_expect_tx(my_full + 8 * slot, bytes);
                             if constexpr (FEW) bulk_g2s(my_ring + slot * SLOT, src, bytes, my_full + 8 * slot);
-                            else bulk_g2s_once(my_ring + slot * SLOT, src, bytes, my_full + 8 * slot, policy);
+                            else bulk_g2s_first_out(my_ring + slot * SLOT, src, bytes, my_full + 8 * slot, policy);
                         }
                         ++issued;
                         slot = slot + 1 == uint32_t(S) ? 0 : slot + 1;

@@ -847,8 +847,9 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
         // ---- raw blocks ----
         constexpr int PARTS = chunk_parts<T>();
         constexpr uint32_t BYTES = 8 * CB;
-        constexpr bool ONCE = NARROW || EXACT;                         // launches whose experts have one item each, nearly; others read their weights again (c5 prefill 2751 -> 2795 us)
-        [[maybe_unused]] const uint64_t policy = ONCE ? once_policy() : 0;
+        // Launches of narrow items, and the exact form at every density (first_out_policy); with items of 128 and 256 tokens it costs (c5 prefill 2751 -> 2795 us)
+        constexpr bool FIRST_OUT = NARROW || EXACT;
+        [[maybe_unused]] const uint64_t policy = FIRST_OUT ? first_out_policy() : 0;
         uint32_t issued = 0, slot = 0, phase = 1;                      // phase: of the empty barrier's wait (none in the first round)
         bool ok = true;
 #pragma unroll 1
@@ -862,9 +863,9 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
                 if (elect_one()) {
                     const uint32_t bar = raw_full + 8 * (issued % (2 * uint32_t(S))), dst = saddr(raw) + slot * BYTES;
                     bar_expect_tx(bar, BYTES);
-                    if constexpr (ONCE) {
-                        tma_load_3d_once(dst, map, 0, c * PARTS, rt, bar, policy);
-                        if (MODE == 0) tma_load_3d_once(dst + BYTES / 2, map + 1, 0, c * PARTS, rt, bar, policy);
+                    if constexpr (FIRST_OUT) {
+                        tma_load_3d_first_out(dst, map, 0, c * PARTS, rt, bar, policy);
+                        if (MODE == 0) tma_load_3d_first_out(dst + BYTES / 2, map + 1, 0, c * PARTS, rt, bar, policy);
                     } else {
                         tma_load_3d(dst, map, 0, c * PARTS, rt, bar);
                         if (MODE == 0) tma_load_3d(dst + BYTES / 2, map + 1, 0, c * PARTS, rt, bar);

@@ -59,7 +59,7 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void * src, uint32_
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void bulk_g2s_once(uint32_t dst, const void * src, uint32_t bytes, uint32_t bar, uint64_t policy) {      // data that is read once (once_policy)
+__device__ __forceinline__ void bulk_g2s_first_out(uint32_t dst, const void * src, uint32_t bytes, uint32_t bar, uint64_t policy) {      // the same with a policy (first_out_policy)
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
                  ::"r"(dst), "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(bar), "l"(policy) : "memory");
 }
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(CTA_WARPS * 32, 1) iq3s_grouped_k(Iq3sArgs p) 
     uint32_t xissued = 0;                  // thread 0: activation stagings issued (their copies must land before the block leaves)
     if (threadIdx.x == 0 && int(blockIdx.x) < n_items) { stage_x(blockIdx.x, 0); ++xissued; }
 
-    const uint64_t policy = once_policy();
+    const uint64_t policy = first_out_policy();
     int iter = 0;
     for (int it = blockIdx.x; it < n_items; it += gridDim.x, ++iter) {
         const int b = p.nbuf == 2 ? (iter & 1) : 0;
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(CTA_WARPS * 32, 1) iq3s_grouped_k(Iq3sArgs p) 
                 const uint32_t s = filled % STAGES;
                 const uint8_t * src = ((NMAT == 2 && (j & 1)) ? base1 : base0) + size_t(NMAT == 2 ? j >> 1 : j) * TILE;
                 mbar_expect_tx(bar0 + 8 * s, TILE);
-                bulk_g2s_once(ring0 + s * TILE, src, TILE, bar0 + 8 * s, policy);
+                bulk_g2s_first_out(ring0 + s * TILE, src, TILE, bar0 + 8 * s, policy);
             };
             for (int j = 0; j < STAGES && j < ntiles; ++j) { if (lane == 0) issue(j); ++filled; }
             float acc[NMAT][NCH][4];

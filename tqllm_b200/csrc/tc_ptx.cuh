@@ -57,8 +57,8 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const void * map, int 
     asm volatile("cp.async.bulk.tensor.3d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                  ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
 }
-// the same for data that is read once (once_policy)
-__device__ __forceinline__ void tma_load_3d_once(uint32_t dst, const void * map, int x, int y, int z, uint32_t bar, uint64_t policy) {
+// the same with a policy (first_out_policy)
+__device__ __forceinline__ void tma_load_3d_first_out(uint32_t dst, const void * map, int x, int y, int z, uint32_t bar, uint64_t policy) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cta.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4}], [%5], %6;"
                  ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar), "l"(policy) : "memory");
 }
