@@ -110,8 +110,9 @@ template <uint32_t T> constexpr int part_words() { return chunk_bytes<T>() / chu
 struct Info { int cum, e, cnt, off; };
 
 // what the exact form keeps beside the operands: the mins' B tiles (32 bytes a row) and the rows' constants
+// (no mins: 8 KB as ever, though a float a row takes 4: those would only move the numbers of experts, 2565 and 3637, from which a block's ring holds five chunks and four)
 constexpr size_t exact_smem(bool mins, int terms) {
-    return !terms ? 0 : mins ? size_t(A_STAGES) * X_CAP * 32 + size_t(x_ring(true, terms)) * 128 * sizeof(float2) : size_t(8192);      // (no mins: a float a row, 4 KB, would do)
+    return !terms ? 0 : mins ? size_t(A_STAGES) * X_CAP * 32 + size_t(x_ring(true, terms)) * 128 * sizeof(float2) : size_t(8192);
 }
 template <uint32_t T>
 constexpr size_t gemm_smem(int experts, int cap, int b_stages, int raw_slots, int terms = 0) {
@@ -571,7 +572,7 @@ __global__ void __launch_bounds__(g_threads(GATHER), 1) gemm_tc_k(const GemmArgs
             for (int c = first; c < im.nv; c += 32) {
                 uint32_t v[16];
                 if ((NARROW || GATHER) && parts == 4) {
-                    // pairs first: which of a block's chunks an item begins with must not show in the sum
+                    // the two sums of either issuer first, so that neither's place shows in the result
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
                         uint32_t w[4][8];
