@@ -38,7 +38,7 @@ inline void launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);       // the error, if any, is read by launch_status()
 }
 // The policy of the weight copies of decode-sized launches: the weights leave the L2 first, so that a stream several times its size leaves code, plan, activations and router rows there. With the default policy a
-// launch found nothing of its own but in HBM, its instructions included. us a layer call, default / this policy, on one box, runs 0.3 % apart: c4 16 tokens 188.5 / 177.0, 64 348.8 / 336.1, own Q4_K 77 tokens 106.8 / 97.4, c3 8 63.0 / 55.6,
+// launch found nothing of its own but in HBM, its instructions included. us a layer call, default / this policy, on one B200, runs 0.3 % apart: c4 16 tokens 188.5 / 177.0, 64 348.8 / 336.1, own Q4_K 77 tokens 106.8 / 97.4, c3 8 63.0 / 55.6,
 // c2 64 x 4 659.6 / 629.5, c5 24 239.7 / 232.1; first passes on new buffers gain as much. It costs nothing where a launch reads an expert's weights again, as that happens soon after: dec4_k with two and more passes an
 // expert (Q4_K of 60 experts at 6.4 per expert 94.8 / 90.1), iq3s_grouped_k (512 experts at 1.3 per expert 282.6 / 271.4, 10 589.5 / 586.0, 23 1121.9 / 1120.8; 60 at 51 384.7 / 379.3), the exact form of the grouped GEMM on small banks (60 experts of Q4_K at 40 per
 // expert 152.3 / 145.4, 100 260.4 / 257.5, 400 888.4 / 889.0; 32 at 125 172.4 / 170.3, 512 626.7 / 627.7; IQ3_S codes of 60 at 400 690.9 / 692.5; 39 shapes in all: 0.98 to 1.075 times as fast, 1.02 on average).
